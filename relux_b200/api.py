@@ -23,13 +23,11 @@ from . import lib as L
 
 
 def _ptr(a):
-    if a is None:
-        return None
+    if a is None or isinstance(a, int):
+        return a
     if isinstance(a, DeviceBuffer):
         return a.ptr
-    if isinstance(a, int):
-        return a
-    return a.ctypes.data
+    return a.__array_interface__["data"][0]
 
 
 def _mem(a):
@@ -312,39 +310,47 @@ class Pool:
         L.check(self.lib.relux_pool_kernel_ms_list(self.h, int(last_n), out.ctypes.data, C.byref(n)))
         return out[:n.value]
 
-    def _append_args(self, layer, a, b, n_seqs, seq_ids, n_new, layout, advance, dtype, pipelined=False):
+    def _pack_append(self, layer, a, b, n_seqs, seq_ids, n_new, layout, advance, dtype, pipelined=False):
+        """(relux_append_args as bytes, the arrays it points to)."""
         ids = None if seq_ids is None else np.ascontiguousarray(seq_ids, dtype=np.int32)
         nn = None if n_new is None else np.ascontiguousarray(n_new, dtype=np.int32)
-        self._keep = [ids, nn, a, b]
-        return L.AppendArgs(layer=layer, n_seqs=n_seqs, seq_ids=_ptr(ids), n_new=_ptr(nn), a=_ptr(a), b=_ptr(b),
-                            dtype=_dtype_flag(a, dtype), mem=_mem(a), layout=layout, advance=int(advance),
-                            flags=L.CALL_PIPELINED if pipelined else 0)
+        return L.pack_append(layer, n_seqs, _ptr(ids) or 0, _ptr(nn) or 0, _ptr(a) or 0, _ptr(b) or 0, _dtype_flag(a, dtype), _mem(a), layout,
+                             int(advance), L.CALL_PIPELINED if pipelined else 0), (ids, nn, a, b)
+
+    def _append_args(self, *args, **kw):
+        packed, keep = self._pack_append(*args, **kw)
+        self._keep = keep
+        return L.AppendArgs.from_buffer_copy(packed)
 
     def append(self, layer, a, b, n_seqs, seq_ids=None, n_new=None, layout=L.LAYOUT_TOKEN_MAJOR, advance=True, dtype=None,
                pipelined=False):
         """MLA: a = c_kv [rows, dC], b = k_rope [rows, dHR].  GQA: a = K, b = V.  pipelined: host inputs travel on the copy
         stream and the call returns once queued (see RELUX_CALL_PIPELINED in include/relux_cuda.h)."""
-        args = self._append_args(layer, a, b, n_seqs, seq_ids, n_new, layout, advance, dtype, pipelined)
-        fn = self.lib.relux_mla_append if self.kind == L.POOL_MLA else self.lib.relux_gqa_append
-        L.check(fn(self.h, C.byref(args)))
+        args, self._keep = self._pack_append(layer, a, b, n_seqs, seq_ids, n_new, layout, advance, dtype, pipelined)
+        L.check(self._fn("append")(self.h, args))
 
-    def _attn_args(self, layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, extra_tokens, causal, mode,
+    def _fn(self, call):
+        return L.packed[("mla_" if self.kind == L.POOL_MLA else "gqa_") + call]
+
+    def _pack_attn(self, layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, extra_tokens, causal, mode,
                    w_uk, w_uv, seq_ids, q_layout, out_layout, q_dtype, out_dtype, pipelined=False):
+        """(relux_attn_args as bytes, the arrays it points to)."""
         ids = None if seq_ids is None else np.ascontiguousarray(seq_ids, dtype=np.int32)
-        self._keep2 = [ids, q, q_rope, out]
-        return L.AttnArgs(layer=layer, n_seqs=n_seqs, seq_ids=_ptr(ids), q_tokens=q_tokens, extra_tokens=extra_tokens,
-                          causal=int(causal), num_heads=num_heads, head_dim=head_dim, scale=scale, q=_ptr(q), q_rope=_ptr(q_rope),
-                          q_dtype=_dtype_flag(q, q_dtype), q_mem=_mem(q), q_layout=q_layout, w_uk=_ptr(w_uk), w_uv=_ptr(w_uv),
-                          out=_ptr(out), out_dtype=_dtype_flag(out, out_dtype), out_mem=_mem(out), out_layout=out_layout, mode=mode,
-                          flags=L.CALL_PIPELINED if pipelined else 0)
+        return L.pack_attn(layer, n_seqs, _ptr(ids) or 0, q_tokens, extra_tokens, int(causal), num_heads, head_dim, scale, _ptr(q) or 0,
+                           _ptr(q_rope) or 0, _dtype_flag(q, q_dtype), _mem(q), q_layout, _ptr(w_uk) or 0, _ptr(w_uv) or 0, _ptr(out) or 0,
+                           _dtype_flag(out, out_dtype), _mem(out), out_layout, mode, L.CALL_PIPELINED if pipelined else 0), (ids, q, q_rope, out)
+
+    def _attn_args(self, *args, **kw):
+        packed, keep = self._pack_attn(*args, **kw)
+        self._keep2 = keep
+        return L.AttnArgs.from_buffer_copy(packed)
 
     def decode(self, layer, n_seqs, q, out, num_heads, head_dim, scale, q_rope=None, w_uk=None, w_uv=None, q_tokens=1,
                extra_tokens=0, causal=True, mode=L.ATTN_FAST, seq_ids=None, q_layout=L.LAYOUT_TOKEN_MAJOR,
                out_layout=L.LAYOUT_TOKEN_MAJOR, q_dtype=None, out_dtype=None, pipelined=False):
-        args = self._attn_args(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, extra_tokens, causal, mode,
-                               w_uk, w_uv, seq_ids, q_layout, out_layout, q_dtype, out_dtype, pipelined)
-        fn = self.lib.relux_mla_decode if self.kind == L.POOL_MLA else self.lib.relux_gqa_decode
-        L.check(fn(self.h, C.byref(args)))
+        args, self._keep2 = self._pack_attn(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, extra_tokens, causal, mode,
+                                            w_uk, w_uv, seq_ids, q_layout, out_layout, q_dtype, out_dtype, pipelined)
+        L.check(self._fn("decode")(self.h, args))
 
     def decode_noalloc(self, layer, n_seqs, q, out, num_heads, head_dim, scale, q_tokens=1, extra_tokens=0, causal=True,
                        seq_ids=None):
@@ -359,20 +365,18 @@ class Pool:
                kv_dtype=None, pipelined=False):
         """Speculative verify: draft rows are written past the cursor, q_tokens rows attend causally."""
         n_new = np.full(n_seqs, q_tokens, np.int32)
-        ap = self._append_args(layer, draft_a, draft_b, n_seqs, seq_ids, n_new, kv_layout, False, kv_dtype, pipelined)
-        at = self._attn_args(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, q_tokens, True, mode, w_uk, w_uv,
-                             seq_ids, L.LAYOUT_TOKEN_MAJOR, L.LAYOUT_TOKEN_MAJOR, q_dtype, out_dtype, pipelined)
-        fn = self.lib.relux_mla_verify if self.kind == L.POOL_MLA else self.lib.relux_gqa_verify
-        L.check(fn(self.h, C.byref(at), C.byref(ap)))
+        ap, self._keep = self._pack_append(layer, draft_a, draft_b, n_seqs, seq_ids, n_new, kv_layout, False, kv_dtype, pipelined)
+        at, self._keep2 = self._pack_attn(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, q_tokens, q_tokens, True, mode, w_uk,
+                                          w_uv, seq_ids, L.LAYOUT_TOKEN_MAJOR, L.LAYOUT_TOKEN_MAJOR, q_dtype, out_dtype, pipelined)
+        L.check(self._fn("verify")(self.h, at, ap))
 
     def step(self, layer, n_seqs, new_a, new_b, q, out, num_heads, head_dim, scale, q_rope=None, w_uk=None, w_uv=None, n_new=None,
              mode=L.ATTN_FAST, seq_ids=None, kv_layout=L.LAYOUT_TOKEN_MAJOR, q_dtype=None, out_dtype=None, kv_dtype=None, pipelined=False):
         """One decode step in one call: append the new rows, then attend (relux_mla_step / relux_gqa_step)."""
-        ap = self._append_args(layer, new_a, new_b, n_seqs, seq_ids, n_new, kv_layout, True, kv_dtype, pipelined)
-        at = self._attn_args(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, 1, 0, True, mode, w_uk, w_uv, seq_ids,
-                             L.LAYOUT_TOKEN_MAJOR, L.LAYOUT_TOKEN_MAJOR, q_dtype, out_dtype, pipelined)
-        fn = self.lib.relux_mla_step if self.kind == L.POOL_MLA else self.lib.relux_gqa_step
-        L.check(fn(self.h, C.byref(ap), C.byref(at)))
+        ap, self._keep = self._pack_append(layer, new_a, new_b, n_seqs, seq_ids, n_new, kv_layout, True, kv_dtype, pipelined)
+        at, self._keep2 = self._pack_attn(layer, n_seqs, q, q_rope, out, num_heads, head_dim, scale, 1, 0, True, mode, w_uk, w_uv, seq_ids,
+                                          L.LAYOUT_TOKEN_MAJOR, L.LAYOUT_TOKEN_MAJOR, q_dtype, out_dtype, pipelined)
+        L.check(self._fn("step")(self.h, ap, at))
 
     def spec_accept(self, n_seqs, k, vocab, draft_tokens, draft_logits, target_logits, draws, temperature=1.0, top_k=0,
                     top_p=1.0, min_p=0.0, mode=L.ATTN_FAST, commit=False, seq_ids=None):

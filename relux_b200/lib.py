@@ -6,6 +6,7 @@ is raised.
 """
 import ctypes as C
 import os
+import struct
 import subprocess
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -133,6 +134,25 @@ class SampleArgs(C.Structure):
                 ("prev_stride", C.c_int32), ("reserved", C.c_int32 * 3), ("tokens", C.c_void_p)]
 
 
+def _packer(cls, skip=("reserved",)):
+    """pack(*fields in order) -> bytes laid out as the struct `cls`, one C call (a keyword-built ctypes struct of 23 fields
+    costs six times as much host time); the reserved fields are zero."""
+    code = {C.c_int32: "i", C.c_int64: "q", C.c_float: "f", C.c_void_p: "P"}
+    fmt, at = "@", 0
+    for name, typ in cls._fields_:
+        if name in skip:
+            continue
+        fmt += "%dx" % (getattr(cls, name).offset - at) + code[typ]
+        at = getattr(cls, name).offset + C.sizeof(typ)
+    s = struct.Struct(fmt + "%dx" % (C.sizeof(cls) - at))
+    assert s.size == C.sizeof(cls)
+    return s.pack
+
+
+pack_append = _packer(AppendArgs)
+pack_attn = _packer(AttnArgs)
+
+
 class ReluxCudaError(RuntimeError):
     def __init__(self, code, msg):
         super().__init__("librelux_cuda status %d: %s" % (code, msg))
@@ -149,6 +169,7 @@ def build(force=False, verbose=False):
 
 
 _lib = None
+packed = {}
 
 
 def load():
@@ -213,6 +234,12 @@ def load():
         L.relux_pool_kernel_ms_mean.argtypes = [C.c_void_p, C.c_int32, C.POINTER(C.c_float), C.POINTER(C.c_int32)]
         L.relux_cuda_launch_count.argtypes = [C.c_void_p, C.POINTER(C.c_int64)]
         L.relux_cuda_stream.argtypes = [C.c_void_p, C.POINTER(C.c_void_p)]
+        # the per-token calls once more, taking their argument structs as packed bytes (pack_append, pack_attn)
+        for name, n_structs in (("mla_append", 1), ("gqa_append", 1), ("mla_decode", 1), ("gqa_decode", 1), ("mla_verify", 2), ("gqa_verify", 2),
+                                ("mla_step", 2), ("gqa_step", 2)):
+            f = L["relux_" + name]   # a function object of its own
+            f.restype, f.argtypes = C.c_int32, [C.c_void_p] + [C.c_char_p] * n_structs
+            packed[name] = f
         _lib = L
     return _lib
 
