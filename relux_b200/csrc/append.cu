@@ -123,10 +123,18 @@ __global__ void gqa_append_kernel(AppendGeom g, uint16_t* __restrict__ k_base, u
   advance_lengths_by_last_block(g);
 }
 
-__global__ void set_len_kernel(int32_t* len, const int32_t* seq_ids, const int32_t* new_len, int n_seqs) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_seqs) return;
-  len[seq_ids ? seq_ids[i] : i] = new_len[i];
+// New lengths travel as kernel arguments: no staging copy and its engine switch in front of the launch.
+constexpr int kSetLenMax = 256;
+struct SetLenParams {
+  int32_t* len;                 // first layer to set, [layers][stride]
+  int32_t layers, stride, n;
+  int32_t seq[kSetLenMax], val[kSetLenMax];
+};
+__global__ void set_len_kernel(const __grid_constant__ SetLenParams p) {
+  chain_release();
+  chain_wait();
+  for (int l = blockIdx.x; l < p.layers; l += gridDim.x)
+    for (int i = threadIdx.x; i < p.n; i += blockDim.x) p.len[(size_t)l * p.stride + p.seq[i]] = p.val[i];
 }
 
 static AppendGeom make_geom(Pool* p, const SeqBatch& sb, int layer, int advance) {
@@ -179,11 +187,21 @@ int32_t launch_gqa_append(Pool* p, const SeqBatch& sb, int layer, const void* k,
   return finish_append(p);
 }
 
-int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer, const int32_t* d_new_len) {
-  int32_t* len = p->d_len + (size_t)layer * p->prm.max_seqs;
-  set_len_kernel<<<(sb.n_seqs + 127) / 128, 128, 0, p->dev->stream>>>(len, sb.d_seq_ids, d_new_len, sb.n_seqs);
-  RELUX_CUDA_TRY(cudaGetLastError());
-  count_launch(p->dev);
+int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer0, int layers, const int32_t* new_len) {
+  SetLenParams k;
+  k.len = p->d_len + (size_t)layer0 * p->prm.max_seqs;
+  k.layers = layers;
+  k.stride = p->prm.max_seqs;
+  for (int i0 = 0; i0 < sb.n_seqs; i0 += kSetLenMax) {
+    k.n = std::min(kSetLenMax, sb.n_seqs - i0);
+    for (int i = 0; i < k.n; i++) {
+      k.seq[i] = sb.seq[i0 + i];
+      k.val[i] = new_len[i0 + i];
+    }
+    RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, set_len_kernel, dim3(std::min(layers, 128)), dim3(kSetLenMax), 0,
+                                  p->dev->stream, k));
+    count_launch(p->dev);
+  }
   return RELUX_OK;
 }
 

@@ -139,6 +139,32 @@ __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bu
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Device time of a launch without event records between it and its neighbours (two records cost the stream 2-4 us per
+// call and keep a chained launch from starting early): every block stamps its first and last moment into the call's slot.
+// `begin_inv` holds the complement, so that both words are maxima over zero-filled memory; the first block clears the
+// slot of the call after this one (whose stamps come after its chain_wait()).
+struct TimeSlot {
+  unsigned long long begin_inv, end;
+};
+struct TimeStamp {
+  TimeSlot* slot;    // nullptr: this call is not timed
+  TimeSlot* clear;
+};
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+// By one thread per block, after chain_wait().
+__device__ __forceinline__ void stamp_begin(const TimeStamp& ts) {
+  if (!ts.slot) return;
+  atomicMax(&ts.slot->begin_inv, ~global_ns());
+  if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) ts.clear->begin_inv = ts.clear->end = 0ull;
+}
+__device__ __forceinline__ void stamp_end(const TimeStamp& ts) {
+  if (ts.slot) atomicMax(&ts.slot->end, global_ns());
+}
+
 // Untiled bulk copy global -> shared through the TMA unit (not the load/store unit): both addresses 16-byte aligned,
 // `bytes` a multiple of 16; completion is counted in bytes on `bar`.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

@@ -1,13 +1,12 @@
-// GQA flash-decode / speculative verify over the paged bf16 K/V pool (RELUX_ATTN_FAST).
+// GQA attention on grid chunks (RELUX_ATTN_FAST): prompts whose group size does not tile the prefill kernel's 128 rows, as
+// grid slices of groups of query tokens, and the allocation-free entry point.  Decode and verify steps run on the
+// one-launch kernel of gqa_stream.cu.
 //
 // Bound: HBM bandwidth.  Every cached token costs Hkv * D * 2 (K,V) * 2 B = 4096 B at Hkv=8, D=128,
 // against about 16 flop/B of work, so the kernel is organised around keeping TMA loads in flight:
 //   * one CTA per (sequence chunk, kv head); warp 4 is the producer, warps 0-3 consume;
-//   * the producer streams each 64-token page of this head as four 8 KB TMA boxes (K and V, two 64-wide
-//     halves each, 128-byte swizzle) through a ring of kStages stages guarded by full/empty mbarriers;
-//   * the g query heads sharing the kv head times the S query tokens form the 16-row M dimension of
-//     mma.sync m16n8k16 (bf16 in, f32 accumulate); each consumer warp owns 16 tokens of every page and
-//     keeps its own online-softmax state, so warps never wait on each other inside the loop;
+//   * the producer streams each 64-token page of this head as four 8 KB TMA boxes through a ring of kStages stages
+//     guarded by full/empty mbarriers; the consumers' arithmetic is in gqa_parts.cuh;
 //   * at the end the four warps' (max, sum, O) are combined through shared memory and written as one
 //     split-KV partial; merge_splits_kernel combines the chunks of a sequence.
 // All mbarrier waits are bounded; a wait that runs out records RELUX_ERR_TIMEOUT and the CTA leaves.
@@ -16,6 +15,7 @@
 #include <mutex>
 #include <vector>
 #include "common.cuh"
+#include "gqa_parts.cuh"
 #include "internal.h"
 #include "splitkv.h"
 
@@ -24,11 +24,7 @@ namespace relux {
 namespace {
 
 constexpr int kStages = 5;
-constexpr int kPageTok = 64;
-constexpr int kD = 128;
-constexpr int kStageBytes = 4 * 8192;  // K lo, K hi, V lo, V hi
-constexpr int kQStride = kD + 8;       // bf16 elements per Q row in shared memory (272 B, conflict-free ldmatrix)
-constexpr int kConsumerWarps = 4;
+constexpr int kPageTok = kGqaPageTok, kD = kGqaD, kStageBytes = kGqaStageBytes, kQStride = kGqaQStride, kConsumerWarps = kGqaConsumerWarps;
 
 struct GqaParams {
   const WorkItem* items;
@@ -134,30 +130,11 @@ __global__ void __launch_bounds__(160, 1) gqa_decode_kernel(const __grid_constan
 
   // ---------------- consumers ----------------
   uint32_t qa[MT][8][4];
-#pragma unroll
-  for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-    for (int ks = 0; ks < 8; ks++) {
-      const int m = lane >> 3;
-      const int row = mt * 16 + (m & 1) * 8 + (lane & 7);
-      const int col = ks * 16 + (m >> 1) * 8;
-      ldmatrix_x4(qa[mt][ks][0], qa[mt][ks][1], qa[mt][ks][2], qa[mt][ks][3], smem_u32(qs + row * kQStride + col));
-    }
-
-  float oacc[MT][16][4];
-  float m_run[MT][2], l_run[MT][2];
-#pragma unroll
-  for (int mt = 0; mt < MT; mt++) {
-#pragma unroll
-    for (int nt = 0; nt < 16; nt++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) oacc[mt][nt][e] = 0.f;
-    m_run[mt][0] = m_run[mt][1] = -INFINITY;
-    l_run[mt][0] = l_run[mt][1] = 0.f;
-  }
+  gqa_load_q<MT>(qa, qs, lane);
+  GqaState<MT> state;
+  state.clear();
   const int tb = warp * 16;  // this warp's tokens inside every page
   bool alive = true;
-
   for (int it = 0; it < npages; it++) {
     const int st = it % kStages;
     if (!mbar_wait(&full[st], (it / kStages) & 1)) {
@@ -165,92 +142,8 @@ __global__ void __launch_bounds__(160, 1) gqa_decode_kernel(const __grid_constan
       alive = false;
       break;
     }
-    const uint32_t kt = smem_u32(stages + st * kStageBytes);
-    const uint32_t vt = kt + 16384;
-    float sacc[MT][2][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-      for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) sacc[mt][nt][e] = 0.f;
-#pragma unroll
-    for (int ks = 0; ks < 8; ks++) {
-      const int m = lane >> 3;
-      const uint32_t row = tb + (m >> 1) * 8 + (lane & 7);
-      const uint32_t chunk = (ks & 3) * 2 + (m & 1);
-      uint32_t b0, b1, b2, b3;
-      ldmatrix_x4(b0, b1, b2, b3, kt + (ks >> 2) * 8192 + swz128(row, chunk));
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++) {
-        mma_bf16_16816(sacc[mt][0], qa[mt][ks], b0, b1);
-        mma_bf16_16816(sacc[mt][1], qa[mt][ks], b2, b3);
-      }
-    }
-    // scale to the log2 domain, mask the tail of the sequence and the causal part of the draft
-    const int tok0 = (item.page_begin + it) * kPageTok + tb;
-    const bool need_mask = (tok0 + 16 > T - (prm.causal ? S : 0));
-    uint32_t pa[MT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++) {
-#pragma unroll
-      for (int hf = 0; hf < 2; hf++) {
-        const int row = mt * 16 + hf * 8 + (lane >> 2);
-        const int limit = prm.causal ? (T - S + row / prm.g) : (T - 1);  // last visible token
-        float mx = -INFINITY;
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            float v = sacc[mt][nt][hf * 2 + e] * prm.scale_log2;
-            if (need_mask) {
-              const int tok = tok0 + nt * 8 + 2 * (lane & 3) + e;
-              if (tok > limit || tok >= T) v = -INFINITY;
-            }
-            sacc[mt][nt][hf * 2 + e] = v;
-            mx = fmaxf(mx, v);
-          }
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float m_new = fmaxf(m_run[mt][hf], mx);
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-        const float alpha = exp2f(m_run[mt][hf] - m_use);
-        m_run[mt][hf] = m_new;
-        float ps = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const float pv = exp2f(sacc[mt][nt][hf * 2 + e] - m_use);
-            sacc[mt][nt][hf * 2 + e] = pv;
-            ps += pv;
-          }
-        l_run[mt][hf] = l_run[mt][hf] * alpha + ps;
-#pragma unroll
-        for (int nt = 0; nt < 16; nt++) {
-          oacc[mt][nt][hf * 2] *= alpha;
-          oacc[mt][nt][hf * 2 + 1] *= alpha;
-        }
-      }
-      pa[mt][0] = pack_bf16x2(sacc[mt][0][0], sacc[mt][0][1]);
-      pa[mt][1] = pack_bf16x2(sacc[mt][0][2], sacc[mt][0][3]);
-      pa[mt][2] = pack_bf16x2(sacc[mt][1][0], sacc[mt][1][1]);
-      pa[mt][3] = pack_bf16x2(sacc[mt][1][2], sacc[mt][1][3]);
-    }
-    // O += P V
-#pragma unroll
-    for (int n2 = 0; n2 < 8; n2++) {
-      const int m = lane >> 3;
-      const uint32_t row = tb + (m & 1) * 8 + (lane & 7);
-      const uint32_t chunk = n2 * 2 + (m >> 1);  // 16 chunks of 8 dims
-      uint32_t b0, b1, b2, b3;
-      ldmatrix_x4_trans(b0, b1, b2, b3, vt + (chunk >> 3) * 8192 + swz128(row, chunk & 7));
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++) {
-        mma_bf16_16816(oacc[mt][2 * n2], pa[mt], b0, b1);
-        mma_bf16_16816(oacc[mt][2 * n2 + 1], pa[mt], b2, b3);
-      }
-    }
+    gqa_consume_page<MT>(state, qa, smem_u32(stages + st * kStageBytes), tb, (item.page_begin + it) * kPageTok + tb, T, S, prm.g, prm.causal,
+                         prm.scale_log2, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[st]);
   }
@@ -258,27 +151,9 @@ __global__ void __launch_bounds__(160, 1) gqa_decode_kernel(const __grid_constan
   // ---------------- combine the four warps, write the split-KV partial ----------------
   // every load this CTA issued has completed once all consumers passed their last full-barrier wait
   asm volatile("bar.sync 1, 128;" ::: "memory");
-  constexpr int kMStride = kD + 2;
+  constexpr int kMStride = kGqaStateStride;
   float* mb = reinterpret_cast<float*>(stages);  // [4 warps][16*MT rows][kD + 2]
-#pragma unroll
-  for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-    for (int hf = 0; hf < 2; hf++) {
-      float l = l_run[mt][hf];
-      l += __shfl_xor_sync(0xffffffffu, l, 1);
-      l += __shfl_xor_sync(0xffffffffu, l, 2);
-      const int row = mt * 16 + hf * 8 + (lane >> 2);
-      float* dst = mb + ((size_t)warp * 16 * MT + row) * kMStride;
-#pragma unroll
-      for (int nt = 0; nt < 16; nt++) {
-        dst[nt * 8 + 2 * (lane & 3)] = oacc[mt][nt][hf * 2];
-        dst[nt * 8 + 2 * (lane & 3) + 1] = oacc[mt][nt][hf * 2 + 1];
-      }
-      if ((lane & 3) == 0) {
-        dst[kD] = alive ? m_run[mt][hf] : -INFINITY;
-        dst[kD + 1] = alive ? l : 0.f;
-      }
-    }
+  gqa_store_state<MT>(state, mb + (size_t)warp * 16 * MT * kMStride, 16 * MT, lane, alive);
   asm volatile("bar.sync 1, 128;" ::: "memory");
   const int d = threadIdx.x;  // 128 consumer threads, one output dim each
   for (int r = 0; r < R; r++) {
@@ -309,65 +184,6 @@ constexpr size_t gqa_smem_bytes() {
 }
 
 }  // namespace
-
-// One launch of the decode kernel + merge for query tokens [s0, s0 + Sg) of a call with a.q_tokens tokens.
-// With the causal mask a group of tokens sees the cache as if it ended with its own last token, so the group is
-// exactly a call with q_tokens = Sg on a cache shortened by the tokens that follow it (extra_g <= a.extra_tokens).
-static int32_t launch_gqa_group(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, void* d_out, int s0, int Sg) {
-  const relux_pool_params& prm = p->prm;
-  const int g = a.num_heads / prm.gqa_num_kv_heads, R = g * Sg;
-  const int extra_g = a.causal ? a.extra_tokens - (a.q_tokens - s0 - Sg) : a.extra_tokens;
-  SplitPlan plan;
-  int32_t rc = plan_splitkv(p, sb, a.layer, extra_g, prm.gqa_num_kv_heads, 2, 1, 0, &plan);
-  if (rc) return rc;
-  const int rows_total = Sg * a.num_heads;
-  rc = grow(p->dev, p->part_o, (size_t)plan.num_items * rows_total * kD * sizeof(float));
-  if (rc) return rc;
-  rc = grow(p->dev, p->part_ml, (size_t)plan.num_items * rows_total * 2 * sizeof(float));
-  if (rc) return rc;
-  GqaParams k{};
-  k.items = plan.items;
-  k.table = p->d_table;
-  k.table_stride = prm.max_pages_per_seq;
-  k.len = p->d_len + (size_t)a.layer * prm.max_seqs;
-  k.num_pages = prm.num_pages;
-  k.Hkv = prm.gqa_num_kv_heads;
-  k.H = a.num_heads;
-  k.g = g;
-  k.S = Sg;
-  k.R = R;
-  k.extra = extra_g;
-  k.causal = a.causal;
-  k.q_tokens_total = a.q_tokens;
-  k.q_token0 = s0;
-  const int64_t rows_per_block = (int64_t)prm.num_pages * prm.gqa_num_kv_heads * kPageTok;
-  k.krow0 = (int32_t)((int64_t)a.layer * 2 * rows_per_block);
-  k.vrow0 = (int32_t)((int64_t)a.layer * 2 * rows_per_block + rows_per_block);
-  k.scale_log2 = a.scale * 1.4426950408889634f;
-  k.q = d_q;
-  k.q_bf16 = a.q_dtype == RELUX_DTYPE_BF16;
-  k.part_o = (float*)p->part_o.p;
-  k.part_ml = (float*)p->part_ml.p;
-  k.rows_total = rows_total;
-  k.status = p->d_status;
-  dim3 grid(plan.num_items, prm.gqa_num_kv_heads);
-  cudaStream_t st = p->dev->stream;
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), st));
-  if (R <= 16) {
-    constexpr size_t smem = gqa_smem_bytes<1>();
-    RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gqa_decode_kernel<1><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
-  } else {
-    constexpr size_t smem = gqa_smem_bytes<2>();
-    RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gqa_decode_kernel<2><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
-  }
-  RELUX_CUDA_TRY(cudaGetLastError());
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), st));
-  p->timed_calls++;
-  count_launch(p->dev);
-  return launch_merge_rows(p, plan, sb.n_seqs, rows_total, kD, (float*)d_out, a.q_tokens * a.num_heads, s0 * a.num_heads);
-}
 
 // A multi-token call longer than one group (a prompt): one work list for the whole call, the groups of `per_group`
 // query tokens as z slices of the decode grid and of the merge grid.  Slice z sees the cache as if it ended with its own
@@ -419,18 +235,18 @@ static int32_t launch_gqa_prompt(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.rows_total = rows_total;
   k.status = p->d_status;
   cudaStream_t st = p->dev->stream;
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), st));
+  if (int32_t rct = time_events_begin(p, p->attn_times)) return rct;
   for (int z0 = 0; z0 < groups; z0 += zmax) {
     const int nz = std::min(zmax, groups - z0);
     k.group0 = z0;
     dim3 grid(plan.num_items, prm.gqa_num_kv_heads, nz);
     if (per_group * g <= 16) {
       constexpr size_t smem = gqa_smem_bytes<1>();
-      RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (int32_t rcs = allow_smem(p->dev, gqa_decode_kernel<1>, smem)) return rcs;
       gqa_decode_kernel<1><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
     } else {
       constexpr size_t smem = gqa_smem_bytes<2>();
-      RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (int32_t rcs = allow_smem(p->dev, gqa_decode_kernel<2>, smem)) return rcs;
       gqa_decode_kernel<2><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
     }
     RELUX_CUDA_TRY(cudaGetLastError());
@@ -439,8 +255,7 @@ static int32_t launch_gqa_prompt(Pool* p, const SeqBatch& sb, const relux_attn_a
                            (long long)group_rows);
     if (rc) return rc;
   }
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), st));
-  p->timed_calls++;
+  if (int32_t rct = time_events_end(p, p->attn_times)) return rct;
   return RELUX_OK;
 }
 
@@ -464,7 +279,7 @@ int32_t launch_gqa_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   // the kernel holds (num_heads / num_kv_heads) * q_tokens <= 32 query rows per kv head; longer multi-token calls
   // (a prompt) are cut into groups of tokens that run as the z slices of one grid
   const int per_group = std::max(1, 32 / g);
-  if (a.q_tokens <= per_group) return launch_gqa_group(p, sb, a, d_q, d_out, 0, a.q_tokens);
+  if (a.q_tokens <= per_group) return launch_gqa_stream(p, sb, a, d_q, d_out, false, nullptr);
   // a prompt: 128 query rows per CTA on the tcgen05 prefill kernel; the grid slices of the decode kernel serve the
   // group sizes that do not tile 128 rows, and stay selectable as a tuning knob
   if (a.q_dtype == RELUX_DTYPE_BF16 && gqa_prompt_wants_bf16(p, a)) return launch_gqa_prefill_sm100(p, sb, a, (const uint16_t*)d_q, (float*)d_out);
@@ -627,11 +442,11 @@ extern "C" __attribute__((visibility("default"))) int32_t relux_gqa_decode_noall
   dim3 grid((unsigned)items, prm.gqa_num_kv_heads);
   if (R <= 16) {
     constexpr size_t smem = gqa_smem_bytes<1>();
-    RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int32_t rcs = allow_smem(p->dev, gqa_decode_kernel<1>, smem)) return rcs;
     gqa_decode_kernel<1><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
   } else {
     constexpr size_t smem = gqa_smem_bytes<2>();
-    RELUX_CUDA_TRY(cudaFuncSetAttribute(gqa_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int32_t rcs = allow_smem(p->dev, gqa_decode_kernel<2>, smem)) return rcs;
     gqa_decode_kernel<2><<<grid, 160, smem, st>>>(p->tmap_gqa, k);
   }
   RELUX_CUDA_TRY(cudaGetLastError());

@@ -134,6 +134,7 @@ struct PrefillParams {
   float scale_log2;
   float* out;                 // [n][S][H][128] f32
   int32_t* status;
+  TimeStamp time;
 };
 
 // The order of the work.  Under the causal mask block pair p of a stream (a sequence's kv head) needs 2 (p + 1) key tiles:
@@ -250,6 +251,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     return;
   }
   if (threadIdx.x == 0) {
+    stamp_begin(prm.time);
     for (int s = 0; s < 2; s++) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
     for (int s = 0; s < kMaxDepth; s++) {
       mbar_init(&bars->k_full[s], 1);
@@ -611,6 +613,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   __syncwarp();
   tc_fence_before();
   cluster_sync();
+  if (threadIdx.x == 0) stamp_end(prm.time);
   if (warp == 0) tmem_dealloc<2>(tmem, kTmemCols);
 }
 
@@ -696,13 +699,11 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   cudaStream_t st = p->dev->stream;
   const int workers = std::min(prefill_workers<false>(p), k.n_couples);
   constexpr int kSmemTotal = Plan<false>::kSmemTotal;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(prefill_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal));
+  if (int32_t rcs = allow_smem(p->dev, prefill_sm100_kernel<false>, kSmemTotal)) return rcs;
+  k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), st));
   prefill_sm100_kernel<false><<<grid, kThreads, kSmemTotal, st>>>(p->tmap_gqa, tq, tq, p->tmap_gqa, k);
   RELUX_CUDA_TRY(cudaGetLastError());
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), st));
-  p->timed_calls++;
   count_launch(p->dev);
   return RELUX_OK;
 }
@@ -789,13 +790,11 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   cudaStream_t st = p->dev->stream;
   const int workers = std::min(prefill_workers<true>(p), k.n_couples);
   constexpr int kSmemTotal = Plan<true>::kSmemTotal;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(prefill_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal));
+  if (int32_t rcs = allow_smem(p->dev, prefill_sm100_kernel<true>, kSmemTotal)) return rcs;
+  k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), st));
   prefill_sm100_kernel<true><<<grid, kThreads, kSmemTotal, st>>>(tx, tq, tqr, p->tmap_mla, k);
   RELUX_CUDA_TRY(cudaGetLastError());
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), st));
-  p->timed_calls++;
   count_launch(p->dev);
   return RELUX_OK;
 }

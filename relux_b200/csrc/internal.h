@@ -12,6 +12,7 @@
 #include <utility>
 #include <vector>
 
+#include "common.cuh"
 #include "relux_cuda.h"
 
 namespace relux {
@@ -44,6 +45,7 @@ struct Device {
   bool copies_in_flight = false;
   std::mutex mu;
   int64_t launches = 0;
+  std::vector<std::pair<const void*, size_t>> smem_allowed;   // kernels that allow_smem has set, under mu
   void* flush_buf = nullptr;
   size_t flush_bytes = 0;
 };
@@ -74,6 +76,16 @@ struct PipeSlots {
   uint64_t next = 0;
 };
 
+// Times of the last kCalls calls.  A call is timed by stamps its kernel writes (one launch: time_stamp_next), or by an
+// event pair around several launches (time_events_begin / _end).
+struct TimeRing {
+  static constexpr int kCalls = 8192, kSlots = kCalls + 1;   // a call clears the slot of the one after it
+  TimeSlot* slots = nullptr;                                 // device [kSlots], zero-filled
+  cudaEvent_t ev[kCalls][2] = {};
+  uint8_t stamped[kCalls] = {};
+  uint64_t calls = 0;
+};
+
 struct Pool {
   uint32_t magic = kPoolMagic;
   Device* dev = nullptr;
@@ -83,6 +95,7 @@ struct Pool {
   size_t page_elems = 0;    // elements per page per tensor (MLA: P*(dC+dHR); GQA: Hkv*P*D for K, same for V)
   size_t layer_elems = 0;   // elements per layer (GQA: K then V)
   uint16_t* storage = nullptr;  // bf16 bits
+  void* meta = nullptr;         // one device block: table, lengths, status, ids, row offsets, time slots of the attention calls
   int32_t* d_table = nullptr;   // [max_seqs][max_pages_per_seq]
   int32_t* d_len = nullptr;     // [num_layers][max_seqs]
   int32_t* d_status = nullptr;   // [0] status word, [1] block counter of the append kernels
@@ -106,11 +119,11 @@ struct Pool {
   // Pinned staging for per-call id / row-offset / length arrays: a ring of slots, each guarded by its own event, so
   // that a call waits for a copy issued kStageSlots calls ago (long finished) instead of for the previous step's kernels.
   static constexpr int kStageSlots = 8;
-  int32_t* h_stage = nullptr;    // pinned [kStageSlots][2 * max_seqs + 1]
+  int32_t* h_stage = nullptr;    // pinned [kStageSlots][4 * (max_seqs + 1)]
   cudaEvent_t stage_ev[kStageSlots] = {};
   bool stage_busy[kStageSlots] = {};
   uint32_t stage_next = 0;
-  size_t stage_slot_ints() const { return 2 * (size_t)prm.max_seqs + 1; }
+  size_t stage_slot_ints() const { return 4 * ((size_t)prm.max_seqs + 1); }
   // staging of activations that arrive in host memory, and outputs that leave to it
   GrowBuf in_a, in_b, out_buf, q_conv;
   GrowBuf expand_buf;  // expanded keys / values of an MLA prompt (+ the sequences' first rows)
@@ -120,6 +133,8 @@ struct Pool {
   GrowBuf q_abs;     // MLA absorbed queries, bf16 [n][S][H][dC+dHR]
   GrowBuf part_o;    // split-KV partial accumulators, f32
   GrowBuf part_ml;   // split-KV partial (max, sum), f32 pairs
+  GrowBuf stream_done;   // GQA stream kernel: finished pieces per (sequence, kv head), zero between launches
+  GrowBuf seq_list;      // GQA stream kernel: the sequences of a call too long for kernel arguments
   GrowBuf work;      // int32 work list + per-sequence chunk offsets
   GrowBuf o_lat;     // MLA merged latent output, f32/bf16
   // TMA descriptors over the pool storage (built at create when the shape allows it)
@@ -131,22 +146,10 @@ struct Pool {
   GrowBuf rope_tab, layer_buf;
   int rope_dim = 0, rope_positions = 0;
   float rope_base = 0.f;
-  // timing of the dominant kernel: a ring of event pairs, one pair per attention call, so that a caller can read
-  // the device times of its last kTimeRing calls after the fact without a synchronisation between them.  The events
-  // of a slot are created the first time the slot is used.
-  static constexpr int kTimeRing = 8192;
-  cudaEvent_t ev_ring[kTimeRing][2] = {};
-  uint64_t timed_calls = 0;
+  // device times of the dominant kernel of the last kTimeRing attention calls, and of the input-projection GEMM of the
+  // layer steps, for a caller to read after the fact without a synchronisation between the calls
+  TimeRing attn_times, proj_times;
   uint64_t attn_calls = 0;   // MLA decode calls, timed or not (RELUX_TUNE_KERNEL_TIMING_STRIDE)
-  cudaEvent_t proj_ring[kTimeRing][2] = {};   // same, around the input-projection GEMM of the layer step
-  uint64_t proj_calls = 0;
-  static cudaEvent_t ring_event(cudaEvent_t (*ring)[2], uint64_t call, int which) {
-    cudaEvent_t& e = ring[call % kTimeRing][which];
-    if (!e && cudaEventCreate(&e) != cudaSuccess) { (void)cudaGetLastError(); e = nullptr; }
-    return e;
-  }
-  cudaEvent_t ev_begin() { return ring_event(ev_ring, timed_calls, 0); }
-  cudaEvent_t ev_end() { return ring_event(ev_ring, timed_calls, 1); }
 };
 
 inline Device* as_device(relux_device_t h) {
@@ -178,18 +181,29 @@ struct SeqBatch {
   std::vector<int32_t> rows; // host copy of rows per sequence
 };
 int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32_t* n_rows, int32_t uniform_rows,
-                    SeqBatch* out);
+                    SeqBatch* out, bool upload = true);
 
 // kernels (defined in the .cu files of this directory)
 int32_t launch_mla_append(Pool* p, const SeqBatch& sb, int layer, const void* ckv, const void* kr, int dtype, int advance);
 int32_t launch_gqa_append(Pool* p, const SeqBatch& sb, int layer, const void* k, const void* v, int dtype, int layout,
                           int advance);
-int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer, const int32_t* d_new_len);
+int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer0, int layers, const int32_t* new_len);   // new_len: host
 int32_t launch_gather_rows(Pool* p, int layer, int seq, int tok0, int n, uint16_t* d_a, uint16_t* d_b);
 int32_t launch_attn_reference_gqa(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const float* d_q, float* d_out);
 int32_t launch_attn_reference_mla(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const float* d_q, const float* d_qr,
                                   float* d_out);
 int32_t launch_gqa_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, void* d_out);
+// The new rows of a GQA decode or verify step that its attention launch appends itself (gqa_stream.cu).
+struct GqaAppend {
+  const void* k;
+  const void* v;
+  int dtype, layout, advance;
+  const int32_t* rows;   // host: new rows per sequence
+};
+bool gqa_stream_eligible(const Pool* p, const relux_attn_args& a);
+bool gqa_append_fusable(const Pool* p, const relux_attn_args& a, int max_new_rows, bool advance);
+int32_t launch_gqa_stream(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, void* d_out, bool out_bf16,
+                          const GqaAppend* app);
 // True when this call is a multi-token call that the tcgen05 prefill kernel serves (it takes bf16 queries).
 bool mla_expand_eligible(const Pool* p, int num_heads, int head_dim);
 int64_t mla_expand_rows(const Pool* p, const SeqBatch& sb, int layer, int extra);
@@ -206,7 +220,9 @@ struct StepAppend {
   const int32_t* d_row_off;   // device row offsets of the append batch (nullptr = one row per sequence)
 };
 int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, const void* d_qr,
-                               void* d_out, const StepAppend* step = nullptr);
+                               void* d_out, bool out_bf16 = false, const StepAppend* step = nullptr);
+// True when that path's last kernel can write its result as bf16 itself.
+bool mla_writes_bf16(const Pool* p, const SeqBatch& sb, const relux_attn_args& a);
 // True when launch_mla_decode_fast can take the step's append into its preparation launch.
 bool mla_step_fusable(Pool* p, const relux_attn_args& a, int n_seqs);
 
@@ -231,6 +247,15 @@ int32_t check_dev_align(const void* ptr, const char* what);
 bool make_tmap_2d(CUtensorMap* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
 bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint64_t cols, uint32_t box_cols, uint32_t box_mid,
                   uint32_t box_outer);
+
+TimeStamp time_stamp_next(Pool* p, TimeRing& r);
+int32_t time_events_begin(Pool* p, TimeRing& r);
+int32_t time_events_end(Pool* p, TimeRing& r);
+
+// Dynamic shared memory above 48 KB has to be allowed once per kernel and device, not per launch.
+int32_t allow_smem(Device* dev, const void* kernel, size_t bytes);
+template <typename... KArgs>
+inline int32_t allow_smem(Device* dev, void (*kernel)(KArgs...), size_t bytes) { return allow_smem(dev, (const void*)kernel, bytes); }
 
 inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 

@@ -45,6 +45,7 @@ struct GemmParams {
   int32_t M, K, n_total, split_k;
   float* part;                           // [split_k][M][n_total] f32
   int32_t* status;
+  TimeStamp time;                        // input projections only
 };
 
 struct GemmBars {
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
     return;
   }
   if (threadIdx.x == 0) {
+    stamp_begin(prm.time);
     for (int s = 0; s < kStages; s++) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
     mbar_init(&bars->done, 1);
     bars->abort_flag = 0;
@@ -173,6 +175,7 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) stamp_end(prm.time);
   if (warp == 0) tmem_dealloc<1>(tmem, 128);
 }
 
@@ -271,7 +274,7 @@ struct WeightRef {
 
 // part[split][M][n_total] = A[M][K] x [W_0 | W_1 | ...]; returns the number of splits used.
 int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const WeightRef* ws, int nw, float* part, size_t part_cap_bytes,
-                           int* split_out) {
+                           int* split_out, TimeStamp time = TimeStamp{nullptr, nullptr}) {
   GemmMaps maps;
   GemmParams g;
   memset(&g, 0, sizeof(g));
@@ -317,7 +320,8 @@ int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const 
   g.split_k = best;
   g.part = part;
   g.status = p->d_status;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(skinny_gemm_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem));
+  g.time = time;
+  if (int32_t rc = allow_smem(p->dev, skinny_gemm_sm100_kernel, kGemmSmem)) return rc;
   dim3 grid(tiles * best, mblocks);
   skinny_gemm_sm100_kernel<<<grid, 192, kGemmSmem, p->dev->stream>>>(maps, g);
   RELUX_CUDA_TRY(cudaGetLastError());
@@ -369,30 +373,26 @@ int32_t ensure_rope_table(Pool* p, int dHR, float base, int positions) {
 }
 
 // x [M][K] f32 -> every segment's buffer: cast + split-K tensor-core GEMM (or the reference-order GEMM), then the
-// finish kernel.  `proj_timing` records the event pair of the GEMM launch in the pool's projection ring.
+// finish kernel.  The GEMM's device time goes to the pool's projection ring.
 int32_t project_and_finish(Pool* p, const SeqBatch& sb, int layer, const float* dx, int M, int K, int S, const WeightRef* ws,
                            const ProjSeg* segs, int nw, bool mma, uint16_t* a_bf16, float* part, size_t part_cap, bool same_pos = false) {
   cudaStream_t st = p->dev->stream;
   int n_total = 0;
   for (int j = 0; j < nw; j++) n_total += ws[j].n;
   int split = 1;
-  cudaEvent_t evs[2] = {Pool::ring_event(p->proj_ring, p->proj_calls, 0), Pool::ring_event(p->proj_ring, p->proj_calls, 1)};
   if (mma) {
     const size_t n8 = (size_t)M * K / 8;
     cast_bf16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(dx, a_bf16, n8);
     RELUX_CUDA_TRY(cudaGetLastError());
     count_launch(p->dev);
-    if (evs[0]) RELUX_CUDA_TRY(cudaEventRecord(evs[0], st));
-    int32_t rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &split);
+    int32_t rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &split, time_stamp_next(p, p->proj_times));
     if (rc) return rc;
   } else {
-    if (evs[0]) RELUX_CUDA_TRY(cudaEventRecord(evs[0], st));
-    int32_t rc = launch_gemm_reference(p, dx, M, K, ws, nw, part, n_total);
+    int32_t rc = time_events_begin(p, p->proj_times);
     if (rc) return rc;
-  }
-  if (evs[0]) {
-    RELUX_CUDA_TRY(cudaEventRecord(evs[1], st));
-    p->proj_calls++;
+    rc = launch_gemm_reference(p, dx, M, K, ws, nw, part, n_total);
+    if (rc) return rc;
+    if ((rc = time_events_end(p, p->proj_times))) return rc;
   }
   FinishParams f;
   memset(&f, 0, sizeof(f));
@@ -593,7 +593,7 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   aa.w_uv = w.w_uv;
   aa.mode = a->mode;
   const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr};   // one row per sequence
-  rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, d_attn, fused_append ? &step : nullptr)
+  rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, d_attn, false, fused_append ? &step : nullptr)
             : launch_attn_reference_mla(p, sb, aa, (const float*)d_qc, (const float*)d_qr, d_attn);
   if (rc) return rc;
   // 5. output projection
@@ -657,30 +657,37 @@ int32_t do_gqa_layer(Pool* p, const relux_gqa_layer_args* a) {
   const ProjSeg segs[3] = {{H * hd, rd, d_q, fast ? 1 : 0}, {Hkv * hd, rd, d_k, 0}, {Hkv * hd, 0, d_v, 0}};
   rc = project_and_finish(p, sb, a->layer, (const float*)dx, M, D, S, proj, segs, 3, mma, sc.a_bf16, sc.part, sc.part_cap, faithful);
   if (rc) return rc;
-  // append: the GEMM rows are token-major [row][Hkv][hd]; advance = 0 leaves the rows past the cursor (verify)
-  rc = launch_gqa_append(p, sb, a->layer, d_k, d_v, RELUX_DTYPE_F32, RELUX_LAYOUT_TOKEN_MAJOR, a->advance);
-  if (rc) return rc;
+  // append: the GEMM rows are token-major [row][Hkv][hd]; advance = 0 leaves the rows past the cursor (verify).  A short
+  // step leaves the append to the attention launch.
+  relux_attn_args aa;
+  memset(&aa, 0, sizeof(aa));
+  aa.mode = a->mode;
+  aa.num_heads = H;
+  aa.q_tokens = S;
+  aa.extra_tokens = a->advance ? 0 : S;
+  const bool fused_append = fast && gqa_append_fusable(p, aa, S, a->advance != 0);
+  if (!fused_append) {
+    rc = launch_gqa_append(p, sb, a->layer, d_k, d_v, RELUX_DTYPE_F32, RELUX_LAYOUT_TOKEN_MAJOR, a->advance);
+    if (rc) return rc;
+  }
   if (a->advance)
     for (int i = 0; i < sb.n_seqs; i++) {
       int32_t& len = p->h_len[(size_t)a->layer * prm.max_seqs + sb.seq[i]];
       note_append(p, a->layer, sb.seq[i], len, S);
       len += S;
     }
-  relux_attn_args aa;
-  memset(&aa, 0, sizeof(aa));
   aa.layer = a->layer;
   aa.n_seqs = sb.n_seqs;
   aa.seq_ids = a->seq_ids;
-  aa.q_tokens = S;
-  aa.extra_tokens = a->advance ? 0 : S;
   aa.causal = a->causal;
-  aa.num_heads = H;
   aa.head_dim = hd;
   aa.scale = (float)(1.0 / std::sqrt((double)hd));   // mha.go:319
   aa.q_dtype = fast ? RELUX_DTYPE_BF16 : RELUX_DTYPE_F32;
   aa.q_layout = RELUX_LAYOUT_TOKEN_MAJOR;
-  aa.mode = a->mode;
-  rc = fast ? launch_gqa_decode_fast(p, sb, aa, d_q, d_attn) : launch_attn_reference_gqa(p, sb, aa, (const float*)d_q, d_attn);
+  const GqaAppend app{d_k, d_v, RELUX_DTYPE_F32, RELUX_LAYOUT_TOKEN_MAJOR, a->advance ? 1 : 0, sb.rows.data()};
+  rc = fused_append ? launch_gqa_stream(p, sb, aa, d_q, d_attn, false, &app)
+       : fast       ? launch_gqa_decode_fast(p, sb, aa, d_q, d_attn)
+                    : launch_attn_reference_gqa(p, sb, aa, (const float*)d_q, d_attn);
   if (rc) return rc;
   return output_projection(p, d_attn, M, H * hd, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
 }

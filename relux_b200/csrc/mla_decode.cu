@@ -18,7 +18,8 @@
 
 namespace relux {
 
-int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs);
+int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
+                                TimeStamp time);
 bool mla_sm100_eligible(const Pool* p, const relux_attn_args& a);
 int mla_sm100_workers(Pool* p, int q_tokens);
 bool mla_proj_mma_eligible(int Dh, int dC);
@@ -30,7 +31,7 @@ int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rop
                               int rows, int H, int dC, int dHR);
 int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W_UV, float* out, int rows, int H, int dC);
 int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
-                                 float* out, int rows, int S, int H, int dC, int32_t* status, bool chained);
+                                 void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
 
 namespace {
 
@@ -249,8 +250,13 @@ bool mla_step_fusable(Pool* p, const relux_attn_args& a, int n_seqs) {
          mla_proj_mma_eligible(a.head_dim, prm.mla_dc) && mla_prep_fits(n_seqs, a.num_heads, prm.mla_dc);
 }
 
+// The merge + up-projection kernel rounds its own result; the unfused up-projections and the prefill kernel write float32.
+bool mla_writes_bf16(const Pool* p, const SeqBatch& sb, const relux_attn_args& a) {
+  return mla_proj_mma_eligible(a.head_dim, p->prm.mla_dc) && p->prm.mla_dc <= 512 && !mla_prefill_eligible(p, sb, a);
+}
+
 int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, const void* d_qr,
-                               void* d_out, const StepAppend* step) {
+                               void* d_out, bool out_bf16, const StepAppend* step) {
   const relux_pool_params& prm = p->prm;
   const int H = a.num_heads, Dh = a.head_dim, dC = prm.mla_dc, dHR = prm.mla_dhr, S = a.q_tokens;
   const int rows = sb.n_seqs * S, rows_total = S * H, roww = dC + dHR;
@@ -345,15 +351,15 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));
     if (rc) return rc;
   }
-  // the event pair around the decode kernel: on every call, or on every Nth (the records are not free: they sit
-  // between this launch and its neighbours)
+  // the decode kernel is timed on every call, or on every Nth (RELUX_TUNE_KERNEL_TIMING_STRIDE)
   const int stride = std::max(1, p->tune.get(RELUX_TUNE_KERNEL_TIMING_STRIDE));
   const bool timed = (p->attn_calls++ % (uint64_t)stride) == 0;
-  if (timed) RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), st));
   if (sm100) {
-    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p);
+    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p,
+                                 timed ? time_stamp_next(p, p->attn_times) : TimeStamp{nullptr, nullptr});
     if (rc) return rc;
   } else {
+    if (timed && (rc = time_events_begin(p, p->attn_times))) return rc;
     MlaGenParams k;
     k.items = plan.items;
     k.table = p->d_table;
@@ -381,16 +387,13 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
       default: rc = launch_generic<512>(p, k, plan.num_items, st); break;
     }
     if (rc) return rc;
-  }
-  if (timed) {
-    RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), st));
-    p->timed_calls++;
+    if (timed && (rc = time_events_end(p, p->attn_times))) return rc;
   }
   count_launch(p->dev);
   if (fused_merge) {
     // split-KV merge fused into the up-projection: the merged latent output never touches HBM
     rc = launch_mla_merge_vup_mma(p->dev, (const float*)p->part_o.p, (const float*)p->part_ml.p, plan.chunk_off, (const uint16_t*)a.w_uv,
-                                  (float*)d_out, rows, S, H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
+                                  d_out, out_bf16, rows, S, H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
     if (rc) return rc;
   } else if (proj_mma) {
     // merged latent output goes to the up-projection as bf16 (tensor-core operand)

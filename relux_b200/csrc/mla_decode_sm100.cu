@@ -86,6 +86,7 @@ struct MlaSm100Params {
   float* part_ml;
   int32_t rows_total;
   int32_t* status;
+  TimeStamp time;
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -146,6 +147,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     return;
   }
   if (threadIdx.x == 0) {
+    stamp_begin(prm.time);
     for (int i = 0; i < kKGroups; i++) { mbar_init(&bars->k_full[i], 1); mbar_init(&bars->k_empty[i], 1); }
     for (int i = 0; i < 4; i++) { mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1); }
     mbar_init(&bars->s_full[0], 1);
@@ -487,6 +489,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   }
   tc_fence_before();
   cluster_sync();
+  if (threadIdx.x == 0) stamp_end(prm.time);
   if (warp == 0) tmem_dealloc<2>(tmem, kTmemCols);
 }
 
@@ -536,7 +539,8 @@ int mla_sm100_workers(Pool* p, int q_tokens) {
   return std::max(1, mc / q_tokens);
 }
 
-int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs) {
+int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
+                                TimeStamp time) {
   const relux_pool_params& prm = p->prm;
   if (plan.num_items == 0) return RELUX_OK;   // every sequence is empty: the merge writes zeros
   CUtensorMap tq;   // the absorbed queries [rows][576], 64 x 64 boxes
@@ -561,7 +565,8 @@ int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_ar
   k.rows_total = a.q_tokens * a.num_heads;
   k.H = a.num_heads;
   k.status = p->d_status;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_decode_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal));
+  k.time = time;
+  if (int32_t rc = allow_smem(p->dev, mla_decode_sm100_kernel, kSmemTotal)) return rc;
   dim3 grid(2 * plan.num_workers * sx, a.q_tokens / sx);
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, mla_decode_sm100_kernel, grid, dim3(192), (size_t)kSmemTotal,
                                 p->dev->stream, p->tmap_mla, tq, k));

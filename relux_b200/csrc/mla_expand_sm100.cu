@@ -415,7 +415,7 @@ int32_t launch_mla_expand_sm100(Pool* p, const SeqBatch& sb, int layer, int extr
   k.row0 = (int64_t)layer * prm.num_pages * k.blocks_per_page * kPage;
   k.Ttot = Ttot;
   k.status = p->d_status;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_expand_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal));
+  if (int32_t rcs = allow_smem(p->dev, mla_expand_sm100_kernel, kSmemTotal)) return rcs;
   const int launched = (int)((units + k.span - 1) / k.span);
   mla_expand_sm100_kernel<<<dim3(2 * launched), kThreads, kSmemTotal, st>>>(p->tmap_mla, t_uk, t_uv, t_out, k);
   RELUX_CUDA_TRY(cudaGetLastError());

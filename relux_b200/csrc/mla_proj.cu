@@ -355,7 +355,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
 // grid (H, ceil(rows/64)), 512 threads, row = seq_index * S + query token.  dC = 128 * nk, nk <= 4.
 __global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                                 const int32_t* __restrict__ chunk_off, const uint16_t* __restrict__ W_UV,
-                                                                float* __restrict__ out, int rows, int S, int H, int dC,
+                                                                void* __restrict__ out, int out_bf16, int rows, int S, int H, int dC,
                                                                 int32_t* __restrict__ status) {
   extern __shared__ __align__(16) uint16_t sm[];
   __shared__ __align__(8) uint64_t w_full[kMaxChunks];   // chunk k of W_UV has landed (bytes counted by the bulk copies)
@@ -398,10 +398,13 @@ __global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(con
   for (int hf = 0; hf < 2; hf++) {
     const int r = r0 + (warp & 3) * 16 + hf * 8 + (lane >> 2);
     if (r >= rows) continue;
-    float* dst = out + ((size_t)r * H + h) * kDh + (warp >> 2) * 64;
+    const size_t off = ((size_t)r * H + h) * kDh + (warp >> 2) * 64 + 2 * (lane & 3);
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++)
-      *reinterpret_cast<float2*>(dst + nt * 8 + 2 * (lane & 3)) = make_float2(acc[nt][hf * 2], acc[nt][hf * 2 + 1]);
+    for (int nt = 0; nt < 8; nt++) {
+      const float x = acc[nt][hf * 2], y = acc[nt][hf * 2 + 1];
+      if (out_bf16) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + off + nt * 8) = pack_bf16x2(x, y);
+      else *reinterpret_cast<float2*>(reinterpret_cast<float*>(out) + off + nt * 8) = make_float2(x, y);
+    }
   }
 }
 
@@ -413,7 +416,7 @@ int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rop
                               int rows, int H, int dC, int dHR) {
   dim3 grid(H, dC / 128, (rows + 63) / 64);
   const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_absorb_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int32_t rc = allow_smem(dev, mla_absorb_mma_kernel, smem)) return rc;
   mla_absorb_mma_kernel<<<grid, 128, smem, dev->stream>>>(q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(dev);
@@ -428,7 +431,7 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
   const int z_absorb = (rows + 63) / 64;
   dim3 grid(H, dC / 128, z_absorb + 1);
   const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int32_t rc = allow_smem(dev, mla_prep_kernel, smem)) return rc;
   RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, grid, dim3(128), smem, dev->stream, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC,
                                 dHR, z_absorb, ap, pl));
   count_launch(dev);
@@ -438,7 +441,7 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
 int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W_UV, float* out, int rows, int H, int dC) {
   dim3 grid(H, (rows + 63) / 64);
   const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_vup_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int32_t rc = allow_smem(dev, mla_vup_mma_kernel, smem)) return rc;
   mla_vup_mma_kernel<<<grid, 128, smem, dev->stream>>>(o_lat, W_UV, out, rows, H, dC);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(dev);
@@ -446,12 +449,12 @@ int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W
 }
 
 int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
-                                 float* out, int rows, int S, int H, int dC, int32_t* status, bool chained) {
+                                 void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
   dim3 grid(H, (rows + 63) / 64);
   const size_t smem = (size_t)(dC / 128) * (64 + 128) * kStride * 2;
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(mla_merge_vup_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int32_t rc = allow_smem(dev, mla_merge_vup_mma_kernel, smem)) return rc;
   RELUX_CUDA_TRY(launch_chained(chained, mla_merge_vup_mma_kernel, grid, dim3(32 * kMergeWarps), smem, dev->stream, part_o, part_ml, chunk_off,
-                                W_UV, out, rows, S, H, dC, status));
+                                W_UV, out, out_bf16, rows, S, H, dC, status));
   count_launch(dev);
   return RELUX_OK;
 }

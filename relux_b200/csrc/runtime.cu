@@ -38,6 +38,50 @@ int32_t grow(Device* dev, GrowBuf& b, size_t bytes) {
   return RELUX_OK;
 }
 
+int32_t allow_smem(Device* dev, const void* kernel, size_t bytes) {
+  for (auto& e : dev->smem_allowed)
+    if (e.first == kernel) {
+      if (e.second >= bytes) return RELUX_OK;
+      RELUX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      e.second = bytes;
+      return RELUX_OK;
+    }
+  RELUX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  dev->smem_allowed.emplace_back(kernel, bytes);
+  return RELUX_OK;
+}
+
+// The slot of the next timed call, for its kernel to stamp; null when the slots could not be allocated (the call is then
+// not timed).
+TimeStamp time_stamp_next(Pool* p, TimeRing& r) {
+  if (!r.slots) {
+    if (cudaMalloc((void**)&r.slots, sizeof(TimeSlot) * TimeRing::kSlots) != cudaSuccess) {
+      (void)cudaGetLastError();
+      r.slots = nullptr;
+      return TimeStamp{nullptr, nullptr};
+    }
+    cudaMemsetAsync(r.slots, 0, sizeof(TimeSlot) * TimeRing::kSlots, p->dev->stream);
+  }
+  const uint64_t c = r.calls++;
+  r.stamped[c % TimeRing::kCalls] = 1;
+  return TimeStamp{r.slots + c % TimeRing::kSlots, r.slots + (c + 1) % TimeRing::kSlots};
+}
+static int32_t time_event(Pool* p, TimeRing& r, int which) {
+  cudaEvent_t& e = r.ev[r.calls % TimeRing::kCalls][which];
+  if (!e) RELUX_CUDA_TRY(cudaEventCreate(&e));
+  RELUX_CUDA_TRY(cudaEventRecord(e, p->dev->stream));
+  return RELUX_OK;
+}
+int32_t time_events_begin(Pool* p, TimeRing& r) { return time_event(p, r, 0); }
+int32_t time_events_end(Pool* p, TimeRing& r) {
+  int32_t rc = time_event(p, r, 1);
+  if (rc) return rc;
+  r.stamped[r.calls++ % TimeRing::kCalls] = 0;
+  if (r.slots)   // the slot of the call after this one
+    RELUX_CUDA_TRY(cudaMemsetAsync(r.slots + r.calls % TimeRing::kSlots, 0, sizeof(TimeSlot), p->dev->stream));
+  return RELUX_OK;
+}
+
 int32_t stage_acquire(Pool* p, int32_t** slot, int* slot_index) {
   const int i = (int)(p->stage_next++ % Pool::kStageSlots);
   if (p->stage_busy[i]) {
@@ -56,8 +100,9 @@ int32_t stage_release(Pool* p, int slot_index) {
 
 // Copies the call's sequence ids / rows-per-sequence to the device when they are not the
 // trivial (identity, uniform) case, through one pinned staging block guarded by an event.
+// upload = false: only the host half (the caller's kernel takes the sequences as arguments).
 int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32_t* n_rows, int32_t uniform_rows,
-                    SeqBatch* out) {
+                    SeqBatch* out, bool upload) {
   const relux_pool_params& prm = p->prm;
   if (n_seqs <= 0 || n_seqs > prm.max_seqs) {
     set_error("n_seqs=%d outside [1, max_seqs=%d]", n_seqs, prm.max_seqs);
@@ -101,7 +146,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
   }
   out->d_seq_ids = nullptr;
   out->d_row_off = nullptr;
-  if (!seq_ids && uniform) return RELUX_OK;
+  if (!upload || (!seq_ids && uniform)) return RELUX_OK;
   Device* dev = p->dev;
   int32_t* slot = nullptr;
   int slot_index = 0;
@@ -189,18 +234,18 @@ static void pool_free_all(Pool* p) {
       if (ps->ready[i]) cudaEventDestroy(ps->ready[i]);
       if (ps->freed[i]) cudaEventDestroy(ps->freed[i]);
     }
-  fr(p->storage); fr(p->d_table); fr(p->d_len); fr(p->d_status); fr(p->d_seq_ids); fr(p->d_row_off);
-  fr(p->in_a.p); fr(p->in_b.p); fr(p->out_buf.p); fr(p->q_abs.p); fr(p->part_o.p); fr(p->part_ml.p); fr(p->work.p);
+  fr(p->storage); fr(p->meta);
+  fr(p->in_a.p); fr(p->in_b.p); fr(p->out_buf.p); fr(p->q_abs.p); fr(p->part_o.p); fr(p->part_ml.p); fr(p->work.p); fr(p->stream_done.p); fr(p->seq_list.p);
   fr(p->o_lat.p); fr(p->q_conv.p); fr(p->rope_tab.p); fr(p->layer_buf.p); fr(p->shadow_f32); fr(p->chunk_tab.p); fr(p->step_rows.p); fr(p->expand_buf.p);
   if (p->h_stage) cudaFreeHost(p->h_stage);
   for (cudaEvent_t ev : p->stage_ev)
     if (ev) cudaEventDestroy(ev);
-  for (auto& pair : p->ev_ring)
-    for (cudaEvent_t ev : pair)
-      if (ev) cudaEventDestroy(ev);
-  for (auto& pair : p->proj_ring)
-    for (cudaEvent_t ev : pair)
-      if (ev) cudaEventDestroy(ev);
+  fr(p->proj_times.slots);   // those of the attention calls are part of `meta`
+  for (TimeRing* r : {&p->attn_times, &p->proj_times}) {
+    for (auto& pair : r->ev)
+      for (cudaEvent_t ev : pair)
+        if (ev) cudaEventDestroy(ev);
+  }
   p->magic = 0;
   delete p;
 }
@@ -359,7 +404,7 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
 int32_t convert_layout(Device* dev, const void* src, void* dst, int n, int S, int H, int D, int src_dtype, int dst_dtype,
                        int src_layout, int dst_layout);
 
-static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const StepAppend* step = nullptr) {
+static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const StepAppend* step = nullptr, const GqaAppend* gstep = nullptr) {
   if (!a) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
   if (p->prm.kind != kind) { set_error("pool kind does not match this attention call"); return RELUX_ERR_INVALID_ARG; }
   int32_t rc = check_layer(p, a->layer);
@@ -395,7 +440,8 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   if (a->out_mem == RELUX_MEM_DEVICE && (rc = check_dev_align(a->out, "out"))) return rc;
   if (kind == RELUX_POOL_MLA && ((rc = check_dev_align(a->w_uk, "w_uk")) || (rc = check_dev_align(a->w_uv, "w_uv")))) return rc;
   SeqBatch sb;
-  rc = stage_batch(p, a->n_seqs, a->seq_ids, nullptr, a->q_tokens, &sb);
+  const bool gqa_stream = kind == RELUX_POOL_GQA && a->mode == RELUX_ATTN_FAST && gqa_stream_eligible(p, *a);
+  rc = stage_batch(p, a->n_seqs, a->seq_ids, nullptr, a->q_tokens, &sb, !gqa_stream);
   if (rc) return rc;
   for (int i = 0; i < sb.n_seqs; i++) {
     int s = sb.seq[i];
@@ -445,15 +491,19 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
       dqr = b2;
     }
   }
-  // kernels write f32 token-major into `kout`; deliver converts if the caller wants otherwise
+  // The kernels write token-major rows into `kout`: float32, or bf16 where the last kernel of the path can round its own
+  // result (the same rounding as the conversion it saves); deliver converts if the caller wants otherwise
   const size_t out_elems = (size_t)n * S * H * D;
-  const bool direct = a->out_mem == RELUX_MEM_DEVICE && a->out_dtype == RELUX_DTYPE_F32 &&
-                      (a->out_layout == RELUX_LAYOUT_TOKEN_MAJOR || S == 1);
-  float* kout;
+  const bool out_tm = a->out_layout == RELUX_LAYOUT_TOKEN_MAJOR || S == 1;
+  const bool k_bf16 = a->out_dtype == RELUX_DTYPE_BF16 && out_tm &&
+                      (gqa_stream || (kind == RELUX_POOL_MLA && a->mode == RELUX_ATTN_FAST && mla_writes_bf16(p, sb, *a)));
+  const int k_dtype = k_bf16 ? RELUX_DTYPE_BF16 : RELUX_DTYPE_F32;
+  const bool direct = a->out_mem == RELUX_MEM_DEVICE && a->out_dtype == k_dtype && out_tm;
+  void* kout;
   const bool piped_out = piped && a->out_mem == RELUX_MEM_HOST;
   int slot_out = -1;
-  char* out_block = nullptr;   // [kernel output f32 | converted output]
-  if (direct) kout = (float*)a->out;
+  char* out_block = nullptr;   // [kernel output | converted output]
+  if (direct) kout = a->out;
   else if (piped_out) {
     PipeSlots& po = p->pipe_out;
     slot_out = (int)(po.next++ % PipeSlots::kSlots);
@@ -462,27 +512,29 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
     // the copy that last read this slot (two pipelined calls ago) must have finished before the kernels overwrite it
     if (po.used[slot_out]) RELUX_CUDA_TRY(cudaStreamWaitEvent(p->dev->stream, po.freed[slot_out], 0));
     out_block = (char*)po.buf[slot_out].p;
-    kout = (float*)out_block;
+    kout = out_block;
   } else {
     rc = grow(p->dev, p->out_buf, out_elems * 4 + out_elems * dtype_size(a->out_dtype));
     if (rc) return rc;
     out_block = (char*)p->out_buf.p;
-    kout = (float*)out_block;
+    kout = out_block;
   }
   relux_attn_args aa = *a;
   aa.q_dtype = want_dtype;
   aa.q_layout = RELUX_LAYOUT_TOKEN_MAJOR;
   if (a->mode != RELUX_ATTN_FAST) {
-    rc = (kind == RELUX_POOL_MLA) ? launch_attn_reference_mla(p, sb, aa, (const float*)dq, (const float*)dqr, kout)
-                                  : launch_attn_reference_gqa(p, sb, aa, (const float*)dq, kout);
+    rc = (kind == RELUX_POOL_MLA) ? launch_attn_reference_mla(p, sb, aa, (const float*)dq, (const float*)dqr, (float*)kout)
+                                  : launch_attn_reference_gqa(p, sb, aa, (const float*)dq, (float*)kout);
+  } else if (gqa_stream) {
+    rc = launch_gqa_stream(p, sb, aa, dq, kout, k_bf16, gstep);
   } else {
-    rc = (kind == RELUX_POOL_MLA) ? launch_mla_decode_fast(p, sb, aa, dq, dqr, kout, step) : launch_gqa_decode_fast(p, sb, aa, dq, kout);
+    rc = (kind == RELUX_POOL_MLA) ? launch_mla_decode_fast(p, sb, aa, dq, dqr, kout, k_bf16, step) : launch_gqa_decode_fast(p, sb, aa, dq, kout);
   }
   if (rc) return rc;
   if ((rc = pipe_release(p, p->pipe_in_a, slot_q)) || (rc = pipe_release(p, p->pipe_in_b, slot_qr))) return rc;
   if (!direct) {
     void* conv = out_block + out_elems * 4;
-    const bool need_conv = a->out_dtype != RELUX_DTYPE_F32 || (a->out_layout == RELUX_LAYOUT_HEAD_MAJOR && S > 1);
+    const bool need_conv = a->out_dtype != k_dtype || !out_tm;
     const void* src = kout;
     if (need_conv) {
       void* dst = (a->out_mem == RELUX_MEM_DEVICE) ? a->out : conv;
@@ -792,23 +844,29 @@ API int32_t relux_pool_create(relux_device_t h, const relux_pool_params* prm, re
   cudaError_t e = cudaSuccess;
   auto A = [&](void** q, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(q, bytes); };
   A((void**)&p->storage, storage_bytes);
-  A((void**)&p->d_table, table_n * 4);
-  A((void**)&p->d_len, len_n * 4);
-  A((void**)&p->d_status, 8);   // [0] status word, [1] block counter of the append kernels
-  A((void**)&p->d_seq_ids, (size_t)prm->max_seqs * 4);
-  A((void**)&p->d_row_off, ((size_t)prm->max_seqs + 1) * 4);
+  // the small arrays in one block: [table | lengths, status (word, block counter of the append kernels), time slots |
+  // sequence ids | row offsets]; the middle part starts as zeros
+  auto pad = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t off_len = pad(table_n * 4), off_status = off_len + pad(len_n * 4), off_slots = off_status + 256,
+               off_ids = off_slots + pad(sizeof(TimeSlot) * TimeRing::kSlots), off_row = off_ids + pad((size_t)prm->max_seqs * 4);
+  A(&p->meta, off_row + pad(((size_t)prm->max_seqs + 1) * 4));
+  p->d_table = (int32_t*)p->meta;
+  p->d_len = (int32_t*)((char*)p->meta + off_len);
+  p->d_status = (int32_t*)((char*)p->meta + off_status);
+  p->attn_times.slots = (TimeSlot*)((char*)p->meta + off_slots);
+  p->d_seq_ids = (int32_t*)((char*)p->meta + off_ids);
+  p->d_row_off = (int32_t*)((char*)p->meta + off_row);
   p->compat = (prm->flags & RELUX_POOL_FLAG_REFERENCE_COMPAT) != 0;
   if (p->compat && prm->kind == RELUX_POOL_MLA) {
     const size_t shadow_bytes = p->layer_elems * prm->num_layers * sizeof(float);
     A((void**)&p->shadow_f32, shadow_bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(p->shadow_f32, 0, shadow_bytes, dev->stream);
   }
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&p->h_stage, Pool::kStageSlots * (2 * (size_t)prm->max_seqs + 1) * 4);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&p->h_stage, Pool::kStageSlots * p->stage_slot_ints() * 4);
   for (cudaEvent_t& ev : p->stage_ev)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMemsetAsync(p->d_table, 0xFF, table_n * 4, dev->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->d_len, 0, len_n * 4, dev->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(p->d_status, 0, 8, dev->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p->d_len, 0, off_ids - off_len, dev->stream);
   // The reference zero-fills new caches (kvcache.go:73-84, mla_cache.go:46-52).
   if (e == cudaSuccess) e = cudaMemsetAsync(p->storage, 0, storage_bytes, dev->stream);
   if (e != cudaSuccess) {
@@ -1000,30 +1058,20 @@ API int32_t relux_seq_set_len(relux_pool_t h, int32_t layer, int32_t n_seqs, con
 
 // The caller holds the device guard.
 int32_t relux::seq_set_len(Pool* p, int32_t layer, int32_t n_seqs, const int32_t* seq_ids, const int32_t* new_len) {
-  Device* dev = p->dev;
   const relux_pool_params& prm = p->prm;
   if (!new_len || layer >= prm.num_layers) { set_error("set_len: bad arguments"); return RELUX_ERR_INVALID_ARG; }
   SeqBatch sb;
-  int32_t rc = stage_batch(p, n_seqs, seq_ids, nullptr, 1, &sb);
+  int32_t rc = stage_batch(p, n_seqs, seq_ids, nullptr, 1, &sb, false);
   if (rc) return rc;
   for (int i = 0; i < n_seqs; i++)
     if (new_len[i] < 0 || new_len[i] > p->seq_pages[sb.seq[i]] * prm.page_tokens) {
       set_error("set_len: length %d outside the capacity of sequence %d", new_len[i], sb.seq[i]);
       return RELUX_ERR_OVERFLOW;
     }
-  // lengths travel through the row-offset staging block
-  int32_t* hs = nullptr;
-  int slot_index = 0;
-  rc = stage_acquire(p, &hs, &slot_index);
-  if (rc) return rc;
-  memcpy(hs, new_len, sizeof(int32_t) * n_seqs);
-  RELUX_CUDA_TRY(cudaMemcpyAsync(p->d_row_off, hs, sizeof(int32_t) * n_seqs, cudaMemcpyHostToDevice, dev->stream));
-  rc = stage_release(p, slot_index);
-  if (rc) return rc;
   int l0 = layer < 0 ? 0 : layer, l1 = layer < 0 ? prm.num_layers : layer + 1;
+  rc = launch_set_len(p, sb, l0, l1 - l0, new_len);
+  if (rc) return rc;
   for (int l = l0; l < l1; l++) {
-    rc = launch_set_len(p, sb, l, p->d_row_off);
-    if (rc) return rc;
     for (int i = 0; i < n_seqs; i++) {
       int32_t& len = p->h_len[(size_t)l * prm.max_seqs + sb.seq[i]];
       note_set_len(p, l, sb.seq[i], len, new_len[i]);
@@ -1105,11 +1153,74 @@ API int32_t relux_gqa_decode(relux_pool_t h, const relux_attn_args* a) {
   return do_attention(p, a, RELUX_POOL_GQA);
 }
 
+// The rows of a GQA decode (advance) or verify step ride in the attention launch: validated and staged exactly as do_append
+// does.  An attention call that is refused leaves the rows appended, as the two calls one after the other would.
+static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_attn_args* attn) {
+  const relux_pool_params& prm = p->prm;
+  SeqBatch sb;
+  int32_t rc = stage_batch(p, kv->n_seqs, kv->seq_ids, kv->n_new, 1, &sb, false);
+  if (rc) return rc;
+  const int adv = kv->advance ? 1 : 0;
+  int32_t* hl = &p->h_len[(size_t)kv->layer * prm.max_seqs];
+  for (int i = 0; i < sb.n_seqs; i++) {
+    const int s = sb.seq[i], cap = p->seq_pages[s] * prm.page_tokens;
+    if (hl[s] + sb.rows[i] > cap) {
+      set_error("Append: layer %d overflow: total=%d + newLen=%d > capacity=%d (sequence %d)", kv->layer, hl[s], sb.rows[i], cap, s);
+      return RELUX_ERR_OVERFLOW;
+    }
+  }
+  if (sb.total_rows == 0 || !gqa_append_fusable(p, *attn, sb.max_rows, adv)) {
+    rc = do_append(p, kv, RELUX_POOL_GQA);
+    return rc ? rc : do_attention(p, attn, RELUX_POOL_GQA);
+  }
+  if (kv->mem == RELUX_MEM_DEVICE && ((rc = check_dev_align(kv->a, "append input a")) || (rc = check_dev_align(kv->b, "append input b")))) return rc;
+  const size_t bytes = (size_t)sb.total_rows * prm.gqa_num_kv_heads * prm.gqa_head_dim * dtype_size(kv->dtype);
+  const bool piped = (kv->flags & RELUX_CALL_PIPELINED) && kv->mem == RELUX_MEM_HOST && p->dev->h2d_stream;
+  const void *da = kv->a, *db = kv->b;
+  int slot_a = -1, slot_b = -1;
+  if (piped) {
+    if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes, &da, &slot_a))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes, &db, &slot_b))) return rc;
+  } else if (kv->mem == RELUX_MEM_HOST) {
+    // the attention call stages q in in_a: the step's rows get a block of their own
+    const size_t off_b = (bytes + 255) & ~(size_t)255;
+    if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
+    da = p->step_rows.p;
+    db = (char*)p->step_rows.p + off_b;
+    RELUX_CUDA_TRY(cudaMemcpyAsync((void*)da, kv->a, bytes, cudaMemcpyHostToDevice, p->dev->stream));
+    RELUX_CUDA_TRY(cudaMemcpyAsync((void*)db, kv->b, bytes, cudaMemcpyHostToDevice, p->dev->stream));
+  }
+  const GqaAppend app{da, db, kv->dtype, kv->layout, adv, sb.rows.data()};
+  if (adv)   // the host lengths count the new rows from here on
+    for (int i = 0; i < sb.n_seqs; i++) hl[sb.seq[i]] += sb.rows[i];
+  rc = do_attention(p, attn, RELUX_POOL_GQA, nullptr, &app);
+  if (rc) {
+    if (adv)
+      for (int i = 0; i < sb.n_seqs; i++) hl[sb.seq[i]] -= sb.rows[i];
+    char why[512];
+    relux_cuda_last_error(why, sizeof(why));
+    do_append(p, kv, RELUX_POOL_GQA);
+    set_error("%s", why);
+    return rc;
+  }
+  if ((rc = pipe_release(p, p->pipe_app_a, slot_a)) || (rc = pipe_release(p, p->pipe_app_b, slot_b))) return rc;
+  return RELUX_OK;
+}
+static bool gqa_fuse_args_ok(const Pool* p, const relux_append_args* kv, const relux_attn_args* attn) {
+  const bool same_ids = (!kv->seq_ids && !attn->seq_ids) ||
+                        (kv->seq_ids && attn->seq_ids && memcmp(kv->seq_ids, attn->seq_ids, sizeof(int32_t) * (size_t)std::max(0, kv->n_seqs)) == 0);
+  return p->prm.kind == RELUX_POOL_GQA && !p->compat && same_ids && kv->n_seqs > 0 && kv->n_seqs <= p->prm.max_seqs && kv->a && kv->b &&
+         attn->mode == RELUX_ATTN_FAST && attn->num_heads > 0 && gqa_stream_eligible(p, *attn) &&
+         (kv->dtype == RELUX_DTYPE_F32 || kv->dtype == RELUX_DTYPE_BF16) && (kv->mem == RELUX_MEM_HOST || kv->mem == RELUX_MEM_DEVICE) &&
+         !(kv->flags & ~RELUX_CALL_PIPELINED) && kv->layer >= 0 && kv->layer < p->prm.num_layers;
+}
+
 static int32_t do_verify(Pool* p, const relux_attn_args* attn, const relux_append_args* kv, int kind) {
   if (!attn || !kv) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
   if (kv->advance != 0) { set_error("verify: draft rows must be appended with advance=0"); return RELUX_ERR_INVALID_ARG; }
   if (kv->layer != attn->layer || kv->n_seqs != attn->n_seqs) { set_error("verify: append and attention arguments disagree"); return RELUX_ERR_INVALID_ARG; }
   if (attn->extra_tokens != attn->q_tokens) { set_error("verify: extra_tokens must equal q_tokens"); return RELUX_ERR_INVALID_ARG; }
+  if (kind == RELUX_POOL_GQA && gqa_fuse_args_ok(p, kv, attn)) return do_gqa_fused(p, kv, attn);
   int32_t rc = do_append(p, kv, kind);
   if (rc) return rc;
   return do_attention(p, attn, kind);
@@ -1117,11 +1228,13 @@ static int32_t do_verify(Pool* p, const relux_attn_args* attn, const relux_appen
 // One decode step: append the new rows (advance = 1), then attend over the cache that now includes them
 // (MLA.forwardCached steps 4-6, mla.go:309-377; MHA.forwardCached steps 5-8, mha.go:283-348).  For the MLA tensor-core
 // path the append rides in the attention call's preparation launch (absorb + append + stream partition: one kernel
-// instead of three); every other case is the two calls one after the other.
+// instead of three), and for the GQA decode kernel in the attention launch itself; every other case is the two calls one
+// after the other.
 static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_args* attn, int kind) {
   if (!attn || !kv) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
   if (kv->advance != 1) { set_error("step: the new rows must be appended with advance=1 (use relux_*_verify for draft rows)"); return RELUX_ERR_INVALID_ARG; }
   if (kv->layer != attn->layer || kv->n_seqs != attn->n_seqs) { set_error("step: append and attention arguments disagree"); return RELUX_ERR_INVALID_ARG; }
+  if (kind == RELUX_POOL_GQA && gqa_fuse_args_ok(p, kv, attn)) return do_gqa_fused(p, kv, attn);
   const bool same_ids = (!kv->seq_ids && !attn->seq_ids) ||
                         (kv->seq_ids && attn->seq_ids && memcmp(kv->seq_ids, attn->seq_ids, sizeof(int32_t) * (size_t)std::max(0, kv->n_seqs)) == 0);
   const bool fuse = kind == RELUX_POOL_MLA && p->prm.kind == RELUX_POOL_MLA && same_ids && kv->n_seqs > 0 && kv->n_seqs <= p->prm.max_seqs &&
@@ -1265,36 +1378,36 @@ API int32_t relux_pool_selftest_wait(relux_pool_t h, int32_t polls) {
   return do_selftest_wait(p, polls);
 }
 
-API int32_t relux_pool_last_kernel_ms(relux_pool_t h, float* ms) {
-  GET_POOL(h);
-  if (!ms) return RELUX_ERR_INVALID_ARG;
-  if (!p->timed_calls) { set_error("no attention kernel has been timed on this pool yet"); return RELUX_ERR_INVALID_ARG; }
-  const auto& pair = p->ev_ring[(p->timed_calls - 1) % Pool::kTimeRing];
-  if (!pair[0] || !pair[1]) { set_error("the last call recorded no timing events"); return RELUX_ERR_CUDA; }
-  RELUX_CUDA_TRY(cudaEventSynchronize(pair[1]));
-  RELUX_CUDA_TRY(cudaEventElapsedTime(ms, pair[0], pair[1]));
-  return RELUX_OK;
-}
-
-// Times of the last n calls of a ring, oldest first; slots whose events were never recorded are skipped.
-static int32_t ring_list(cudaEvent_t (*ring)[2], uint64_t calls, int32_t last_n, float* out, int32_t* counted) {
-  const uint64_t n = std::min<uint64_t>(std::min<uint64_t>((uint64_t)last_n, calls), Pool::kTimeRing);
+// Times of the last n calls of a ring, oldest first; calls whose launch failed are skipped.
+static int32_t ring_list(Pool* p, TimeRing& r, int32_t last_n, float* out, int32_t* counted) {
+  const uint64_t n = std::min<uint64_t>(std::min<uint64_t>((uint64_t)last_n, r.calls), TimeRing::kCalls);
+  std::vector<TimeSlot> slots;
+  if (r.slots) {
+    slots.resize(TimeRing::kSlots);
+    RELUX_CUDA_TRY(cudaMemcpyAsync(slots.data(), r.slots, sizeof(TimeSlot) * slots.size(), cudaMemcpyDeviceToHost, p->dev->stream));
+  }
+  RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
   int32_t k = 0;
   for (uint64_t i = n; i-- > 0;) {
-    cudaEvent_t* pair = ring[(calls - 1 - i) % Pool::kTimeRing];
+    const uint64_t c = r.calls - 1 - i;
+    if (r.stamped[c % TimeRing::kCalls]) {
+      const TimeSlot& t = slots[c % TimeRing::kSlots];
+      if (t.begin_inv && t.end) out[k++] = (float)((double)(t.end - ~t.begin_inv) * 1e-6);
+      continue;
+    }
+    cudaEvent_t* pair = r.ev[c % TimeRing::kCalls];
     if (!pair[0] || !pair[1]) continue;
     float ms = 0.f;
-    RELUX_CUDA_TRY(cudaEventSynchronize(pair[1]));
     RELUX_CUDA_TRY(cudaEventElapsedTime(&ms, pair[0], pair[1]));
     out[k++] = ms;
   }
   *counted = k;
   return RELUX_OK;
 }
-static int32_t ring_mean(cudaEvent_t (*ring)[2], uint64_t calls, int32_t last_n, float* mean_ms, int32_t* counted) {
-  std::vector<float> ms((size_t)std::min<int64_t>(last_n, Pool::kTimeRing));
+static int32_t ring_mean(Pool* p, TimeRing& r, int32_t last_n, float* mean_ms, int32_t* counted) {
+  std::vector<float> ms((size_t)std::min<int64_t>(last_n, TimeRing::kCalls));
   int32_t n = 0;
-  int32_t rc = ring_list(ring, calls, last_n, ms.data(), &n);
+  int32_t rc = ring_list(p, r, last_n, ms.data(), &n);
   if (rc) return rc;
   double sum = 0.0;
   for (int i = 0; i < n; i++) sum += ms[i];
@@ -1303,22 +1416,33 @@ static int32_t ring_mean(cudaEvent_t (*ring)[2], uint64_t calls, int32_t last_n,
   return RELUX_OK;
 }
 
+API int32_t relux_pool_last_kernel_ms(relux_pool_t h, float* ms) {
+  GET_POOL(h);
+  if (!ms) return RELUX_ERR_INVALID_ARG;
+  if (!p->attn_times.calls) { set_error("no attention kernel has been timed on this pool yet"); return RELUX_ERR_INVALID_ARG; }
+  int32_t n = 0;
+  int32_t rc = ring_list(p, p->attn_times, 1, ms, &n);
+  if (rc) return rc;
+  if (!n) { set_error("the last call recorded no times"); return RELUX_ERR_CUDA; }
+  return RELUX_OK;
+}
+
 API int32_t relux_pool_kernel_ms_list(relux_pool_t h, int32_t last_n, float* ms_out, int32_t* counted) {
   GET_POOL(h);
   if (!ms_out || !counted || last_n <= 0) return RELUX_ERR_INVALID_ARG;
-  return ring_list(p->ev_ring, p->timed_calls, last_n, ms_out, counted);
+  return ring_list(p, p->attn_times, last_n, ms_out, counted);
 }
 
 API int32_t relux_pool_kernel_ms_mean(relux_pool_t h, int32_t last_n, float* mean_ms, int32_t* counted) {
   GET_POOL(h);
   if (!mean_ms || last_n <= 0) return RELUX_ERR_INVALID_ARG;
-  if (!p->timed_calls) { set_error("no attention kernel has been timed on this pool yet"); return RELUX_ERR_INVALID_ARG; }
-  return ring_mean(p->ev_ring, p->timed_calls, last_n, mean_ms, counted);
+  if (!p->attn_times.calls) { set_error("no attention kernel has been timed on this pool yet"); return RELUX_ERR_INVALID_ARG; }
+  return ring_mean(p, p->attn_times, last_n, mean_ms, counted);
 }
 
 API int32_t relux_pool_projection_ms_mean(relux_pool_t h, int32_t last_n, float* mean_ms, int32_t* counted) {
   GET_POOL(h);
   if (!mean_ms || last_n <= 0) return RELUX_ERR_INVALID_ARG;
-  if (!p->proj_calls) { set_error("no layer step has run on this pool yet"); return RELUX_ERR_INVALID_ARG; }
-  return ring_mean(p->proj_ring, p->proj_calls, last_n, mean_ms, counted);
+  if (!p->proj_times.calls) { set_error("no layer step has run on this pool yet"); return RELUX_ERR_INVALID_ARG; }
+  return ring_mean(p, p->proj_times, last_n, mean_ms, counted);
 }

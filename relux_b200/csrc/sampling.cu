@@ -1042,7 +1042,7 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
     if (rc) return rc;
   }
   // device time of the selection kernel, readable through relux_pool_kernel_ms_mean like the attention kernels'
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_begin(), dev->stream));
+  if (int32_t rct = time_events_begin(p, p->attn_times)) return rct;
   if (mode == RELUX_ATTN_REFERENCE) {
     spec_accept_reference_kernel<<<(n + 31) / 32, 32, 0, dev->stream>>>(prm, n, (float*)p->part_o.p, (int32_t*)p->part_ml.p);
   } else {
@@ -1091,8 +1091,7 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
     RELUX_CUDA_TRY(cudaLaunchKernelEx(&cfg, spec_accept_kernel, prm));
   }
   RELUX_CUDA_TRY(cudaGetLastError());
-  RELUX_CUDA_TRY(cudaEventRecord(p->ev_end(), dev->stream));
-  p->timed_calls++;
+  if (int32_t rct = time_events_end(p, p->attn_times)) return rct;
   count_launch(dev);
   host.resize((size_t)2 * n);
   RELUX_CUDA_TRY(cudaMemcpyAsync(host.data(), p->out_buf.p, sizeof(int32_t) * 2 * (size_t)n, cudaMemcpyDeviceToHost, dev->stream));
