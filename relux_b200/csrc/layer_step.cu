@@ -27,14 +27,26 @@ int32_t stage_in(Pool* p, GrowBuf& buf, const void* src, size_t bytes, int mem, 
 namespace {
 
 constexpr int kMaxWeights = 4;   // weight matrices that share one activation matrix in a launch
-constexpr int kTileN = 128, kTileM = 128, kTileK = 64;
-constexpr int kStages = 6;
-constexpr int kStageA = kTileM * kTileK * 2;   // 16 KB: [128 rows][64 k] bf16, 128-byte swizzle, K-major
-constexpr int kStageB = kTileK * kTileN * 2;   // 16 KB: two [64 k][64 n] blocks, 128-byte swizzle, MN-major
-constexpr int kGemmSmem = kStages * (kStageA + kStageB) + 1024;
+constexpr int kTileN = 128, kTileK = 64;
+constexpr int kStageW = kTileK * kTileN * 2;   // 16 KB of weights: two [64 k][64 n] blocks, 128-byte swizzle, MN-major
+constexpr int kMaxTok = 256;                   // activation rows of one block
+
+// A launch's work: the K steps of all 128-column tiles laid end to end, cut into `workers` ranges that differ by at most
+// one step.  A PIECE is the part of a tile inside one range; piece j of a tile (in range order) is split j of the result.
+struct GemmRanges {
+  int32_t steps, range, more;   // K steps per tile; steps per worker, one more for the first `more` of them.  steps = 0: one piece
+  __host__ __device__ int begin(int w) const { return w * range + (w < more ? w : more); }
+  __host__ __device__ int worker_of(int u) const {
+    const int big = more * (range + 1);
+    return u < big ? (int)((unsigned)u / (unsigned)(range + 1)) : more + (int)((unsigned)(u - big) / (unsigned)range);
+  }
+  __host__ __device__ int pieces(int tile) const {
+    return steps ? worker_of((tile + 1) * steps - 1) - worker_of(tile * steps) + 1 : 1;
+  }
+};
 
 struct GemmMaps {
-  CUtensorMap a;                 // activations [M][K] bf16
+  CUtensorMap a;                 // activations [M][K] bf16, box: 64 k x NT rows
   CUtensorMap w[kMaxWeights];    // weights [K][N_j] bf16
 };
 struct GemmParams {
@@ -42,17 +54,29 @@ struct GemmParams {
   int32_t tile_first[kMaxWeights + 1];   // first 128-column tile of every weight
   int32_t n_cols[kMaxWeights];           // N_j
   int32_t col_first[kMaxWeights];        // first output column of weight j in the concatenated result
-  int32_t M, K, n_total, split_k;
-  float* part;                           // [split_k][M][n_total] f32
+  int32_t M, n_total;
+  GemmRanges rg;
+  float* part;                           // [piece][M][n_total] f32
   int32_t* status;
   TimeStamp time;                        // input projections only
 };
 
+// NT: activation rows of a block (the N of the MMA).  As many stages as shared memory holds.
+template <int NT>
+struct GemmShape {
+  static constexpr int kStageX = NT * kTileK * 2;   // [NT rows][64 k] bf16, 128-byte swizzle, K-major
+  static constexpr int kStage = kStageW + kStageX;
+  static constexpr int kStages = (232448 - 1024) / kStage;
+  static constexpr int kSmem = kStages * kStage + 1024;
+  static constexpr int kAcc = NT < 32 ? 32 : NT;    // columns of one of the two accumulators
+};
+
 struct GemmBars {
-  uint64_t full[kStages], empty[kStages], done;
+  uint64_t full[12], empty[12], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   volatile int32_t abort_flag;
 };
+static_assert(GemmShape<16>::kStages <= 12 && sizeof(GemmBars) <= 1024, "barrier block too small");
 
 __device__ __noinline__ void gemm_wait_slow(uint64_t* bar, uint32_t parity, GemmBars* b, int32_t* status) {
   for (uint32_t i = 0; i < kSpinLimit; i++) {
@@ -68,36 +92,47 @@ __device__ __forceinline__ void gemm_wait(uint64_t* bar, uint32_t parity, GemmBa
   if (!mbar_try_wait(bar, parity)) gemm_wait_slow(bar, parity, b, status);
 }
 
-// grid (tiles * split_k, ceil(M / 128)), 192 threads: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer.
-// Unit = (128-column tile of one weight, K split): D[128 x 128] f32 in tensor memory accumulates
-// A[128 x 64] (K-major) x W[64 x 128] (MN-major: the row-major weight rows as they lie in HBM) per pipeline stage.
-__global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_constant__ GemmMaps maps, const GemmParams prm) {
+// part[piece][m][n] = x [M][K] x [W_0 | W_1 | ...] over the piece's K steps.  Bound: HBM, every weight is read once.
+// grid (workers, ceil(M / NT)), 192 threads: warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer.
+//   * The WEIGHTS are the M = 128 operand (MN-major: the row-major rows as they lie in HBM) and the activations, 16 to 256
+//     rows, the N operand, so that a stage is 16 KB of weights and no more activations than there are: with the
+//     activations as the M = 128 operand a stage of 16 rows was half padding, read from L2 for every step.
+//   * One CTA per SM walks an equal share of the steps of all tiles without draining its pipeline in between (two
+//     accumulators: a piece is written out while the next one's MMAs run).
+//   * The weights do not depend on the launches before this one, whose tail and launch gap they hide: the producer
+//     fills its stages with them before chain_wait().  The first kernel of a layer step (cast_bf16_kernel) releases its
+//     successors only when everything before the step is complete, so that weights written earlier in the stream are there.
+// Measured with the chained launches around it (a layer step, before -> now): 16 rows of d_model 16384, 1.36 GB of weights,
+// 308 -> 286 us; 24 rows of d_model 4096, 84 MB, 82.8 -> 67.3 us.
+template <int NT>
+__global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams prm) {
+  using SH = GemmShape<NT>;
+  constexpr int kStages = SH::kStages;
   extern __shared__ __align__(1024) uint8_t smem[];
-  GemmBars* bars = reinterpret_cast<GemmBars*>(smem + kStages * (kStageA + kStageB));
+  GemmBars* bars = reinterpret_cast<GemmBars*>(smem + kStages * SH::kStage);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x / prm.split_k, split = blockIdx.x % prm.split_k;
-  const int m0 = blockIdx.y * kTileM;
-  int j = 0;
-  while (j + 1 < prm.n_weights && tile >= prm.tile_first[j + 1]) j++;
-  const int n0 = (tile - prm.tile_first[j]) * kTileN;
-  const int steps_total = (prm.K + kTileK - 1) / kTileK;
-  const int step0 = (int)((long long)steps_total * split / prm.split_k);
-  const int step1 = (int)((long long)steps_total * (split + 1) / prm.split_k);
-  const int nsteps = step1 - step0;
-
+  const int m0 = blockIdx.y * NT;
+  const int u0 = prm.rg.begin(blockIdx.x), u1 = prm.rg.begin(blockIdx.x + 1);
+  auto weight_of = [&](int tile) -> int {
+    int j = 0;
+    while (j + 1 < prm.n_weights && tile >= prm.tile_first[j + 1]) j++;
+    return j;
+  };
+  chain_release();
   if ((smem_u32(smem) & 1023u) != 0) {
+    chain_wait();
     if (threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     return;
   }
   if (threadIdx.x == 0) {
-    stamp_begin(prm.time);
+    stamp_begin(prm.time);   // the launch that cleared the slot is complete: see cast_bf16_kernel
     for (int s = 0; s < kStages; s++) { mbar_init(&bars->full[s], 1); mbar_init(&bars->empty[s], 1); }
-    mbar_init(&bars->done, 1);
+    for (int b = 0; b < 2; b++) { mbar_init(&bars->acc_full[b], 1); mbar_init(&bars->acc_empty[b], 4); }
     bars->abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 0) {
-    tmem_alloc<1>(&bars->tmem_base, 128);
+    tmem_alloc<1>(&bars->tmem_base, 2 * SH::kAcc);
     tmem_relinquish<1>();
   }
   tc_fence_before();
@@ -107,76 +142,99 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
 
   if (warp == 4) {
     const bool el = elect_one();
-    const CUtensorMap* wmap = &maps.w[j];
-    if (el) {
-      tma_prefetch_desc(&maps.a);
-      tma_prefetch_desc(wmap);
-    }
-    for (int i = 0; i < nsteps; i++) {
-      const int s = i % kStages, use = i / kStages;
-      if (use > 0) gemm_wait(&bars->empty[s], (use - 1) & 1, bars, prm.status);
+    if (el) tma_prefetch_desc(&maps.a);
+    int tile = u0 / prm.rg.steps, k = u0 - tile * prm.rg.steps, j = weight_of(tile);
+    auto load_w = [&](int g) {   // the weights of step g of this range; arms the stage for both operands
+      const int s = g % kStages;
       if (el) {
-        uint8_t* sa = smem + s * (kStageA + kStageB);
-        uint8_t* sb = sa + kStageA;
-        const int k0 = (step0 + i) * kTileK;
-        mbar_expect_tx(&bars->full[s], kStageA + kStageB);   // out-of-range parts of a box are zero-filled and still counted
-        tma_load_2d(sa, &maps.a, k0, m0, &bars->full[s]);
-        tma_load_2d(sb, wmap, n0, k0, &bars->full[s]);
-        tma_load_2d(sb + kStageB / 2, wmap, n0 + 64, k0, &bars->full[s]);
+        uint8_t* sw = smem + s * SH::kStage;
+        const int n0 = (tile - prm.tile_first[j]) * kTileN;
+        mbar_expect_tx(&bars->full[s], SH::kStage);   // out-of-range parts of a box are zero-filled and still counted
+        tma_load_2d(sw, &maps.w[j], n0, k * kTileK, &bars->full[s]);
+        tma_load_2d(sw + kStageW / 2, &maps.w[j], n0 + 64, k * kTileK, &bars->full[s]);
       }
       __syncwarp();
+      if (++k == prm.rg.steps) {
+        k = 0;
+        j = weight_of(++tile);
+      }
+    };
+    auto load_x = [&](int g, int kx) {
+      const int s = g % kStages;
+      if (el) tma_load_2d(smem + s * SH::kStage + kStageW, &maps.a, kx * kTileK, m0, &bars->full[s]);
+      __syncwarp();
+    };
+    const int n = u1 - u0, ahead = min(n, kStages);
+    int kx = k;
+    for (int g = 0; g < ahead; g++) load_w(g);
+    chain_wait();
+    for (int g = 0; g < n; g++) {
+      if (g >= ahead) {
+        gemm_wait(&bars->empty[g % kStages], (g / kStages - 1) & 1, bars, prm.status);
+        load_w(g);
+      }
+      load_x(g, kx);
+      if (++kx == prm.rg.steps) kx = 0;
     }
   } else if (warp == 5) {
+    chain_wait();
     const bool el = elect_one();
-    const uint32_t idesc = make_idesc_bf16(kTileM, kTileN, false, true);
-    for (int i = 0; i < nsteps; i++) {
-      const int s = i % kStages, use = i / kStages;
-      gemm_wait(&bars->full[s], use & 1, bars, prm.status);
+    const uint32_t idesc = make_idesc_bf16(kTileN, NT, true, false);
+    int g = 0;
+    for (int u = u0, piece = 0; u < u1; piece++) {
+      const int end = min(u1, (u / prm.rg.steps + 1) * prm.rg.steps);
+      const uint32_t d = tmem + (piece & 1) * SH::kAcc;
+      if (piece >= 2) gemm_wait(&bars->acc_empty[piece & 1], ((piece >> 1) - 1) & 1, bars, prm.status);
       tc_fence_after();
-      if (el) {
-        const uint32_t sa = smem_u32(smem + s * (kStageA + kStageB));
-        const uint64_t dA = make_desc_kmajor_sw128(sa);
-        const uint64_t dB = make_desc_mnmajor_sw128(sa + kStageA, kStageB / 2);
+      for (bool first = true; u < end; u++, g++, first = false) {
+        const int s = g % kStages;
+        gemm_wait(&bars->full[s], (g / kStages) & 1, bars, prm.status);
+        tc_fence_after();
+        if (el) {
+          const uint32_t sw = smem_u32(smem + s * SH::kStage);
+          const uint64_t dW = make_desc_mnmajor_sw128(sw, kStageW / 2);
+          const uint64_t dX = make_desc_kmajor_sw128(sw + kStageW);
 #pragma unroll
-        for (int kk = 0; kk < kTileK / 16; kk++)
-          umma_ss<1>(tmem, dA + ((uint32_t)(kk * 32) >> 4), dB + ((uint32_t)(kk * 2048) >> 4), idesc, (i | kk) != 0);
-        umma_commit<1>(&bars->empty[s]);
+          for (int kk = 0; kk < kTileK / 16; kk++)
+            umma_ss<1>(d, dW + ((uint32_t)(kk * 2048) >> 4), dX + ((uint32_t)(kk * 32) >> 4), idesc, !first || kk != 0);
+          umma_commit<1>(&bars->empty[s]);
+        }
+        __syncwarp();
       }
+      if (el) umma_commit<1>(&bars->acc_full[piece & 1]);
       __syncwarp();
     }
-    if (el) umma_commit<1>(&bars->done);
-    __syncwarp();
   } else {
-    // epilogue: thread = accumulator row
-    gemm_wait(&bars->done, 0, bars, prm.status);
-    tc_fence_after();
-    const int row = m0 + warp * 32 + lane;
-    const int ncols = min(kTileN, prm.n_cols[j] - n0);   // a multiple of 8
-    const bool ok = !bars->abort_flag && nsteps > 0;
-    float* dst = prm.part + ((size_t)split * prm.M + row) * prm.n_total + prm.col_first[j] + n0;
+    // epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once
+    chain_wait();
+    for (int u = u0, piece = 0; u < u1; piece++) {
+      const int tile = u / prm.rg.steps, j = weight_of(tile);
+      u = min(u1, (tile + 1) * prm.rg.steps);
+      const int split = (int)blockIdx.x - prm.rg.worker_of(tile * prm.rg.steps);
+      const int n = (tile - prm.tile_first[j]) * kTileN + warp * 32 + lane;
+      const int m_end = min(NT, prm.M - m0);
+      float* dst = prm.part + ((size_t)split * prm.M + m0) * prm.n_total + prm.col_first[j] + n;
+      gemm_wait(&bars->acc_full[piece & 1], (piece >> 1) & 1, bars, prm.status);
+      tc_fence_after();
+      const bool ok = !bars->abort_flag, mine = n < prm.n_cols[j];
 #pragma unroll 1
-    for (int c = 0; c < kTileN; c += 32) {
-      uint32_t v[32];
-      if (ok) {
-        tmem_ld_32x32b_x32(tmem + ((uint32_t)(warp * 32) << 16) + c, v);
+      for (int c = 0; c < m_end; c += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem + ((uint32_t)(warp * 32) << 16) + (piece & 1) * SH::kAcc + c, v);
         tmem_ld_wait();
-      } else {
 #pragma unroll
-        for (int q = 0; q < 32; q++) v[q] = 0u;
+        for (int q = 0; q < 32; q++)
+          if (mine && c + q < m_end) dst[(size_t)(c + q) * prm.n_total] = ok ? __uint_as_float(v[q]) : 0.f;
       }
-      if (row < prm.M) {
-#pragma unroll
-        for (int q = 0; q < 32; q += 4)
-          if (c + q < ncols)
-            *reinterpret_cast<float4*>(dst + c + q) = make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]),
-                                                                  __uint_as_float(v[q + 2]), __uint_as_float(v[q + 3]));
-      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->acc_empty[piece & 1]);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0) stamp_end(prm.time);
-  if (warp == 0) tmem_dealloc<1>(tmem, 128);
+  if (warp == 0) tmem_dealloc<1>(tmem, 2 * SH::kAcc);
 }
 
 // The reference's matmulBatched3D in its own operation order: out[m][n] = sum over k ascending of x[m][k] * w[k][n],
@@ -191,7 +249,11 @@ __global__ void gemm_reference_kernel(const float* __restrict__ x, const uint16_
   out[(size_t)m * out_stride + col_first + n] = acc;
 }
 
+// The first kernel of a layer step.  It waits before it releases the launch after it, which may therefore rely on
+// everything that was queued before the step without a wait of its own.
 __global__ void cast_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, size_t n8) {
+  chain_wait();
+  chain_release();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const float4 a = reinterpret_cast<const float4*>(src)[2 * i], b = reinterpret_cast<const float4*>(src)[2 * i + 1];
@@ -210,7 +272,9 @@ struct ProjSeg {
 };
 struct FinishParams {
   const float* part;
-  int32_t split_k, M, n_total, S, n_segs;
+  GemmRanges rg;
+  int32_t tile_first[kMaxWeights];   // first 128-column tile of every segment
+  int32_t M, n_total, S, n_segs;
   ProjSeg seg[kMaxWeights];
   const int32_t* len;              // this layer's lengths BEFORE the append
   const int32_t* seq_ids;
@@ -223,17 +287,21 @@ struct FinishParams {
 __global__ void proj_finish_kernel(const FinishParams p) {
   const int pair = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
   const int col = 2 * pair;
+  chain_release();
+  chain_wait();
   if (col >= p.n_total || m >= p.M) return;
-  float v0 = 0.f, v1 = 0.f;
-  for (int s = 0; s < p.split_k; s++) {
-    const float2 t = *reinterpret_cast<const float2*>(p.part + ((size_t)s * p.M + m) * p.n_total + col);
-    v0 += t.x;
-    v1 += t.y;
-  }
   int c = col, j = 0;
   while (j + 1 < p.n_segs && c >= p.seg[j].n) {
     c -= p.seg[j].n;
     j++;
+  }
+  const int pieces = p.rg.pieces(p.tile_first[j] + c / kTileN);
+  float v0 = 0.f, v1 = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < pieces; s++) {
+    const float2 t = *reinterpret_cast<const float2*>(p.part + ((size_t)s * p.M + m) * p.n_total + col);
+    v0 += t.x;
+    v1 += t.y;
   }
   const ProjSeg sg = p.seg[j];
   if (sg.rope_dim > 0) {
@@ -256,11 +324,16 @@ __global__ void proj_finish_kernel(const FinishParams p) {
   else *reinterpret_cast<float2*>(reinterpret_cast<float*>(sg.dst) + (size_t)m * sg.n + c) = make_float2(v0, v1);
 }
 
-__global__ void sum_splits_kernel(const float* __restrict__ part, int split_k, size_t n4, float* __restrict__ out) {
+// out [M][N] = sum over the pieces of one weight's tiles; a thread sums four adjacent columns.
+__global__ void sum_splits_kernel(const float* __restrict__ part, GemmRanges rg, int N, size_t n4, float* __restrict__ out) {
+  chain_release();
+  chain_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
+  const int pieces = rg.pieces((int)(4 * i % (unsigned)N) / kTileN);
   float4 acc = reinterpret_cast<const float4*>(part)[i];
-  for (int s = 1; s < split_k; s++) {
+#pragma unroll 4
+  for (int s = 1; s < pieces; s++) {
     const float4 t = reinterpret_cast<const float4*>(part)[(size_t)s * n4 + i];
     acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
   }
@@ -272,13 +345,24 @@ struct WeightRef {
   int n;
 };
 
-// part[split][M][n_total] = A[M][K] x [W_0 | W_1 | ...]; returns the number of splits used.
+template <int NT>
+int32_t launch_skinny_gemm_rows(Pool* p, const GemmMaps& maps, const GemmParams& g, int workers) {
+  if (int32_t rc = allow_smem(p->dev, skinny_gemm_sm100_kernel<NT>, GemmShape<NT>::kSmem)) return rc;
+  RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, skinny_gemm_sm100_kernel<NT>, dim3(workers, (g.M + NT - 1) / NT),
+                                dim3(192), (size_t)GemmShape<NT>::kSmem, p->dev->stream, maps, g));
+  count_launch(p->dev);
+  return RELUX_OK;
+}
+
+// part[piece][M][n_total] = A[M][K] x [W_0 | W_1 | ...]; returns the ranges, which say how many pieces every tile has.
 int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const WeightRef* ws, int nw, float* part, size_t part_cap_bytes,
-                           int* split_out, TimeStamp time = TimeStamp{nullptr, nullptr}) {
+                           GemmRanges* ranges, TimeStamp time = TimeStamp{nullptr, nullptr}) {
   GemmMaps maps;
   GemmParams g;
   memset(&g, 0, sizeof(g));
-  if (!make_tmap_2d(&maps.a, (void*)a_bf16, (uint64_t)M, (uint64_t)K, kTileK, kTileM)) {
+  int nt = 16;   // rows of a block: the smallest tile that holds them all (padding costs L2 reads and shared memory)
+  while (nt < M && nt < kMaxTok) nt *= 2;
+  if (!make_tmap_2d(&maps.a, (void*)a_bf16, (uint64_t)M, (uint64_t)K, kTileK, nt)) {
     set_error("tensor map for the activations could not be encoded");
     return RELUX_ERR_CUDA;
   }
@@ -298,36 +382,32 @@ int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const 
   g.tile_first[nw] = tiles;
   g.n_weights = nw;
   g.M = M;
-  g.K = K;
   g.n_total = cols;
-  const int mblocks = (M + kTileM - 1) / kTileM;
+  const int mblocks = (M + nt - 1) / nt;
   const int steps = (K + kTileK - 1) / kTileK;
-  const int sms = std::max(1, p->dev->sm_count);
-  // split K so that the units fill whole waves of SMs: cost = waves x (steps per unit + fixed cost per unit)
-  int best = 1;
-  double best_cost = 1e300;
-  const int max_split = std::min(std::min(steps, 32), (int)std::max<size_t>(1, part_cap_bytes / ((size_t)M * cols * 4)));
-  for (int s = 1; s <= max_split; s++) {
-    const long units = (long)tiles * mblocks * s;
-    const long waves = (units + sms - 1) / sms;
-    const double cost = (double)waves * ((double)(steps + s - 1) / s + 6.0);
-    if (cost < best_cost - 1e-9) {
-      best_cost = cost;
-      best = s;
-    }
+  if ((int64_t)tiles * steps >= (int64_t)1 << 31) { set_error("a projection of more than 2^31 steps"); return RELUX_ERR_UNSUPPORTED; }
+  const int units = tiles * steps;
+  // One range per SM, the rows' blocks side by side; ranges of fewer than four steps do not pay for their piece of the
+  // result.  The pieces have to fit the scratch: one worker always does.
+  int workers = std::max(1, std::min(std::max(1, p->dev->sm_count) / mblocks, units / 4));
+  if (const int ov = p->tune.get(RELUX_TUNE_GEMM_SPLIT)) workers = std::max(1, std::min(units, tiles * ov));   // tuning knob
+  for (;; workers = (workers + 1) / 2) {
+    g.rg = GemmRanges{steps, units / workers, units % workers};
+    int most = 0;
+    for (int t = 0; t < tiles; t++) most = std::max(most, g.rg.pieces(t));
+    if (workers == 1 || (size_t)most * M * cols * 4 <= part_cap_bytes) break;
   }
-  if (const int ov = p->tune.get(RELUX_TUNE_GEMM_SPLIT)) best = std::max(1, std::min(max_split, ov));   // tuning knob
-  g.split_k = best;
   g.part = part;
   g.status = p->d_status;
   g.time = time;
-  if (int32_t rc = allow_smem(p->dev, skinny_gemm_sm100_kernel, kGemmSmem)) return rc;
-  dim3 grid(tiles * best, mblocks);
-  skinny_gemm_sm100_kernel<<<grid, 192, kGemmSmem, p->dev->stream>>>(maps, g);
-  RELUX_CUDA_TRY(cudaGetLastError());
-  count_launch(p->dev);
-  *split_out = best;
-  return RELUX_OK;
+  *ranges = g.rg;
+  switch (nt) {
+    case 16: return launch_skinny_gemm_rows<16>(p, maps, g, workers);
+    case 32: return launch_skinny_gemm_rows<32>(p, maps, g, workers);
+    case 64: return launch_skinny_gemm_rows<64>(p, maps, g, workers);
+    case 128: return launch_skinny_gemm_rows<128>(p, maps, g, workers);
+    default: return launch_skinny_gemm_rows<kMaxTok>(p, maps, g, workers);
+  }
 }
 
 bool gemm_sm100_eligible(int K, const WeightRef* ws, int nw) {
@@ -372,20 +452,25 @@ int32_t ensure_rope_table(Pool* p, int dHR, float base, int positions) {
   return RELUX_OK;
 }
 
+int32_t launch_cast(Pool* p, const float* src, uint16_t* dst, size_t n) {
+  RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, cast_bf16_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0,
+                                p->dev->stream, src, dst, n / 8));
+  count_launch(p->dev);
+  return RELUX_OK;
+}
+
 // x [M][K] f32 -> every segment's buffer: cast + split-K tensor-core GEMM (or the reference-order GEMM), then the
 // finish kernel.  The GEMM's device time goes to the pool's projection ring.
 int32_t project_and_finish(Pool* p, const SeqBatch& sb, int layer, const float* dx, int M, int K, int S, const WeightRef* ws,
                            const ProjSeg* segs, int nw, bool mma, uint16_t* a_bf16, float* part, size_t part_cap, bool same_pos = false) {
   cudaStream_t st = p->dev->stream;
+  const bool chained = p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0;
   int n_total = 0;
   for (int j = 0; j < nw; j++) n_total += ws[j].n;
-  int split = 1;
+  GemmRanges ranges{};
   if (mma) {
-    const size_t n8 = (size_t)M * K / 8;
-    cast_bf16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(dx, a_bf16, n8);
-    RELUX_CUDA_TRY(cudaGetLastError());
-    count_launch(p->dev);
-    int32_t rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &split, time_stamp_next(p, p->proj_times));
+    int32_t rc = launch_cast(p, dx, a_bf16, (size_t)M * K);
+    if (!rc) rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &ranges, time_stamp_next(p, p->proj_times));
     if (rc) return rc;
   } else {
     int32_t rc = time_events_begin(p, p->proj_times);
@@ -397,7 +482,8 @@ int32_t project_and_finish(Pool* p, const SeqBatch& sb, int layer, const float* 
   FinishParams f;
   memset(&f, 0, sizeof(f));
   f.part = part;
-  f.split_k = split;
+  f.rg = ranges;
+  for (int j = 1; j < nw; j++) f.tile_first[j] = f.tile_first[j - 1] + (ws[j - 1].n + kTileN - 1) / kTileN;
   f.M = M;
   f.n_total = n_total;
   f.S = S;
@@ -415,13 +501,13 @@ int32_t project_and_finish(Pool* p, const SeqBatch& sb, int layer, const float* 
   f.same_pos = same_pos ? 1 : 0;
   f.status = p->d_status;
   dim3 grid((n_total / 2 + 255) / 256, M);
-  proj_finish_kernel<<<grid, 256, 0, st>>>(f);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  RELUX_CUDA_TRY(launch_chained(chained, proj_finish_kernel, grid, dim3(256), 0, st, f));
   count_launch(p->dev);
   return RELUX_OK;
 }
 
-// out [M][N] f32 = attn [M][K] f32 x W_O [K][N]; `out` is the caller's buffer (host or device).
+// out [M][N] f32 = attn [M][K] x W_O [K][N]; `out` is the caller's buffer (host or device).  d_attn: float32, or nullptr when
+// the rows are in a_bf16 already (mma).
 int32_t output_projection(Pool* p, const float* d_attn, int M, int K, const void* w_o, int N, bool mma, uint16_t* a_bf16, float* part,
                           size_t part_cap, void* out, int out_mem) {
   cudaStream_t st = p->dev->stream;
@@ -434,16 +520,13 @@ int32_t output_projection(Pool* p, const float* d_attn, int M, int K, const void
   }
   const WeightRef outp[1] = {{w_o, N}};
   if (mma) {
-    const size_t n8 = (size_t)M * K / 8;
-    cast_bf16_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(d_attn, a_bf16, n8);
-    RELUX_CUDA_TRY(cudaGetLastError());
-    count_launch(p->dev);
-    int split = 1;
-    int32_t rc = launch_skinny_gemm(p, a_bf16, M, K, outp, 1, part, part_cap, &split);
+    GemmRanges ranges{};
+    int32_t rc = d_attn ? launch_cast(p, d_attn, a_bf16, (size_t)M * K) : RELUX_OK;
+    if (!rc) rc = launch_skinny_gemm(p, a_bf16, M, K, outp, 1, part, part_cap, &ranges);
     if (rc) return rc;
     const size_t n4 = (size_t)M * N / 4;
-    sum_splits_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(part, split, n4, d_out);
-    RELUX_CUDA_TRY(cudaGetLastError());
+    RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, sum_splits_kernel, dim3((unsigned)((n4 + 255) / 256)), dim3(256), 0, st,
+                                  (const float*)part, ranges, N, n4, d_out));
     count_launch(p->dev);
   } else {
     int32_t rc = launch_gemm_reference(p, d_attn, M, K, outp, 1, d_out, N);
@@ -593,11 +676,12 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   aa.w_uv = w.w_uv;
   aa.mode = a->mode;
   const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr};   // one row per sequence
-  rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, d_attn, false, fused_append ? &step : nullptr)
+  const bool o_bf16 = mma && mla_writes_bf16(p, sb, aa);   // the output projection's operand, rounded by the kernel that makes it
+  rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, fused_append ? &step : nullptr)
             : launch_attn_reference_mla(p, sb, aa, (const float*)d_qc, (const float*)d_qr, d_attn);
   if (rc) return rc;
   // 5. output projection
-  return output_projection(p, d_attn, M, H * Dh, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
+  return output_projection(p, o_bf16 ? nullptr : d_attn, M, H * Dh, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
 }
 
 // MHA.forwardCached (mha.go:245-369) for a batch of independent sequences: projections with Wq / Wk / Wv, RoPE on q
@@ -685,11 +769,12 @@ int32_t do_gqa_layer(Pool* p, const relux_gqa_layer_args* a) {
   aa.q_dtype = fast ? RELUX_DTYPE_BF16 : RELUX_DTYPE_F32;
   aa.q_layout = RELUX_LAYOUT_TOKEN_MAJOR;
   const GqaAppend app{d_k, d_v, RELUX_DTYPE_F32, RELUX_LAYOUT_TOKEN_MAJOR, a->advance ? 1 : 0, sb.rows.data()};
-  rc = fused_append ? launch_gqa_stream(p, sb, aa, d_q, d_attn, false, &app)
+  const bool o_bf16 = mma && fused_append;   // the output projection's operand, rounded by the kernel that makes it
+  rc = fused_append ? launch_gqa_stream(p, sb, aa, d_q, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, &app)
        : fast       ? launch_gqa_decode_fast(p, sb, aa, d_q, d_attn)
                     : launch_attn_reference_gqa(p, sb, aa, (const float*)d_q, d_attn);
   if (rc) return rc;
-  return output_projection(p, d_attn, M, H * hd, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
+  return output_projection(p, o_bf16 ? nullptr : d_attn, M, H * hd, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
 }
 
 // ComputeBackend.MatMulFloat32 as matmulBatched3D uses it (interface.go:25-29, mha.go:759-785): C = A x B with A, C float32
