@@ -218,13 +218,14 @@ struct StepAppend {
   const void* kr;
   int dtype;
   const int32_t* d_row_off;   // device row offsets of the append batch (nullptr = one row per sequence)
+  bool weights_ready = false; // a launch before this one in the call has waited for everything older (launch_mla_prep)
 };
 int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, const void* d_qr,
                                void* d_out, bool out_bf16 = false, const StepAppend* step = nullptr);
 // True when that path's last kernel can write its result as bf16 itself.
 bool mla_writes_bf16(const Pool* p, const SeqBatch& sb, const relux_attn_args& a);
 // True when launch_mla_decode_fast can take the step's append into its preparation launch.
-bool mla_step_fusable(Pool* p, const relux_attn_args& a, int n_seqs);
+bool mla_step_fusable(Pool* p, const relux_attn_args& a);
 
 int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a);
 int32_t do_gqa_layer(Pool* p, const relux_gqa_layer_args* a);

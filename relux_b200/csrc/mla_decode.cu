@@ -23,10 +23,9 @@ int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_ar
 bool mla_sm100_eligible(const Pool* p, const relux_attn_args& a);
 int mla_sm100_workers(Pool* p, int q_tokens);
 bool mla_proj_mma_eligible(int Dh, int dC);
-bool mla_prep_fits(int n_seqs, int H, int dC);
 int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const uint16_t* d_q, const uint16_t* d_qr, float* d_out);
 int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows,
-                        int H, int dC, int dHR, const PrepAppend& ap, const PrepPlan& pl, bool chained);
+                        int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained);
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
                               int rows, int H, int dC, int dHR);
 int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W_UV, float* out, int rows, int H, int dC);
@@ -244,10 +243,10 @@ int32_t launch_generic(Pool* p, const MlaGenParams& k, int items, cudaStream_t s
 
 }  // namespace
 
-bool mla_step_fusable(Pool* p, const relux_attn_args& a, int n_seqs) {
+bool mla_step_fusable(Pool* p, const relux_attn_args& a) {
   const relux_pool_params& prm = p->prm;
   return !p->compat && a.mode == RELUX_ATTN_FAST && a.extra_tokens == 0 && mla_sm100_eligible(p, a) &&
-         mla_proj_mma_eligible(a.head_dim, prm.mla_dc) && mla_prep_fits(n_seqs, a.num_heads, prm.mla_dc);
+         mla_proj_mma_eligible(a.head_dim, prm.mla_dc);
 }
 
 // The merge + up-projection kernel rounds its own result; the unfused up-projections and the prefill kernel write float32.
@@ -307,7 +306,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     pl.items = plan.stream_items;
     pl.chunk_off = plan.chunk_off;
     pl.worker_first = plan.worker_first;
-    rc = launch_mla_prep(p->dev, d_q, d_qr, a.q_dtype == RELUX_DTYPE_BF16, (const uint16_t*)a.w_uk, (uint16_t*)p->q_abs.p, rows, H, dC, dHR, ap,
+    rc = launch_mla_prep(p->dev, d_q, d_qr, a.q_dtype == RELUX_DTYPE_BF16, (const uint16_t*)a.w_uk, (uint16_t*)p->q_abs.p, rows, H, dC, dHR, step->weights_ready, ap,
                          pl, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
     if (rc) return rc;
   }

@@ -138,16 +138,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   const int worker = cluster / prm.sx;
   const int sq = blockIdx.y * prm.sx + cluster % prm.sx;   // query token of this worker
   chain_release();
-  chain_wait();   // the ranges, the absorbed queries and the step's new rows come from the kernel before this one
-  const int it0 = prm.worker_first[worker], it1 = prm.worker_first[worker + 1];
-  if (it0 >= it1 || sq >= prm.S) return;   // an empty range: both CTAs of the pair leave before any pair-wide step
-
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled layouts need a 1024-byte aligned base
+    chain_wait();
     if (threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     return;
   }
+  // the set-up needs nothing of the kernel before this one, whose tail hides it
   if (threadIdx.x == 0) {
-    stamp_begin(prm.time);
     for (int i = 0; i < kKGroups; i++) { mbar_init(&bars->k_full[i], 1); mbar_init(&bars->k_empty[i], 1); }
     for (int i = 0; i < 4; i++) { mbar_init(&bars->v_full[i], 1); mbar_init(&bars->v_empty[i], 1); }
     mbar_init(&bars->s_full[0], 1);
@@ -157,6 +154,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     mbar_init(&bars->q_full, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
+    tma_prefetch_desc(&tmap_kv);
+    tma_prefetch_desc(&tmap_q);
   }
   if (warp == 0) {
     tmem_alloc<2>(&bars->tmem_base, kTmemCols);
@@ -166,17 +165,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  chain_wait();   // the ranges, the absorbed queries and the step's new rows come from the kernel before this one
+  int it0 = prm.worker_first[worker], it1 = prm.worker_first[worker + 1];
+  if (sq >= prm.S) it1 = it0;   // an empty range: nothing to do, and the CTA pair still meets at the end
+  if (threadIdx.x == 0 && it0 < it1) stamp_begin(prm.time);
 
-  if (warp == 4) {
+  if (it0 >= it1) {
+  } else if (warp == 4) {
     // =============================== producer: TMA loads into this CTA's slots ===============================
     // The whole warp stays converged and one elected lane issues: operands that every lane computes identically
     // live in uniform registers, which is what keeps the issue rate of TMA / tcgen05 instructions high.
     const bool el = elect_one();
     const uint32_t lead_q = mapa_u32(smem_u32(&bars->q_full), 0);
-    if (el) {
-      tma_prefetch_desc(&tmap_kv);
-      tma_prefetch_desc(&tmap_q);
-    }
     auto win_load = [&](const StreamItem& it, int blk) -> int32_t {
       const int lp = min(32 * blk + lane, it.page_end - it.page_begin - 1);
       int32_t pg = __ldg(prm.table + (size_t)it.seq * prm.table_stride + it.page_begin + lp);
@@ -489,7 +489,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   }
   tc_fence_before();
   cluster_sync();
-  if (threadIdx.x == 0) stamp_end(prm.time);
+  if (threadIdx.x == 0 && it0 < it1) stamp_end(prm.time);
   if (warp == 0) tmem_dealloc<2>(tmem, kTmemCols);
 }
 

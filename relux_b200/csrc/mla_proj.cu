@@ -63,7 +63,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // sources), the result leaves through shared memory as 16-byte row-contiguous stores.
 __device__ __forceinline__ void absorb_block(uint16_t* sm, const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
                                              const uint16_t* __restrict__ W_UK, uint16_t* __restrict__ q_abs, int rows, int H, int dC,
-                                             int dHR, int bx, int by, int bz) {
+                                             int dHR, int bx, int by, int bz, bool wait_for_queries = false) {
   uint16_t* As = sm;                  // [64][kStride]
   uint16_t* Bs = sm + 64 * kStride;   // [128][kStride]   rows = latent index c, cols = d
   const int h = bx, c0 = by * 128, r0 = bz * 64;
@@ -73,6 +73,7 @@ __device__ __forceinline__ void absorb_block(uint16_t* sm, const void* __restric
     const int c = e / (kDh / 8), v = e % (kDh / 8);
     cp_async16(Bs + c * kStride + v * 8, W_UK + (size_t)(c0 + c) * H * kDh + (size_t)h * kDh + (size_t)v * 8);
   }
+  if (wait_for_queries) chain_wait();
   // A: 64 rows x 128 d, 8 elements per thread per step
 #pragma unroll 4
   for (int e = threadIdx.x; e < 64 * (kDh / 8); e += blockDim.x) {
@@ -141,22 +142,27 @@ __global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const void* __restr
   absorb_block(sm, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// The preparation of one MLA decode step in ONE launch: the absorb grid (H, dC/128, ceil(rows/64)) plus one extra z
-// slice whose blocks append the step's new rows (block e < n_seqs: sequence e) and build the stream partition (block
-// e == n_seqs).  The three jobs are independent of one another: the append reads the lengths before it writes, the
-// partition counts every sequence's new rows itself, and the last of those blocks to finish advances the lengths.
+// The preparation of one MLA decode step in ONE launch: blocks 0 .. n_seqs - 1 append the step's new rows (a sequence
+// each), block n_seqs builds the stream partition, and the blocks after them are the absorb grid (head fastest, then the
+// dC / 128 latent slices, then 64 rows each).  The three jobs are independent of one another: the append reads the lengths
+// before it writes, the partition counts every sequence's new rows itself, and the last of those blocks to finish advances
+// the lengths.  They come first because theirs is the longer chain of dependent reads.
+// The kernel releases the launches after it only when everything before it is complete (the up-projection fetches its
+// weights without a wait of its own), unless the launches before it in the call have seen to that (weights_ready): its own
+// weights are then fetched ahead of its wait too.
 __global__ void __launch_bounds__(128) mla_prep_kernel(const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
                                                        const uint16_t* __restrict__ W_UK, uint16_t* __restrict__ q_abs, int rows, int H,
-                                                       int dC, int dHR, int z_absorb, const PrepAppend ap, const PrepPlan pl) {
+                                                       int dC, int dHR, int weights_ready, const PrepAppend ap, const PrepPlan pl) {
   extern __shared__ __align__(16) uint16_t sm[];
+  const int e = blockIdx.x;
+  if (!weights_ready) chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
   chain_release();
-  chain_wait();   // the kernel before this one in the stream may still be reading what this one overwrites
-  if ((int)blockIdx.z < z_absorb) {
-    absorb_block(sm, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z);
+  if (e > ap.n_seqs) {
+    const int a = e - ap.n_seqs - 1, slices = dC / 128;
+    absorb_block(sm, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, weights_ready != 0);
     return;
   }
-  const int e = blockIdx.y * gridDim.x + blockIdx.x;
-  if (e > ap.n_seqs) return;
+  if (weights_ready) chain_wait();
   if (e < ap.n_seqs) prep_append_seq(ap, e);
   else prep_build_stream(ap, pl);
   prep_arrive_and_advance(ap, (uint32_t)ap.n_seqs + 1u);
@@ -202,27 +208,23 @@ __global__ void __launch_bounds__(128) mla_vup_mma_kernel(const uint16_t* __rest
   }
 }
 
-// 64 x 128 x 128 tile for eight warps: warp w owns rows 16 (w & 3) .. +15 and the 64 columns of half (w >> 2).
-// Bs is [k][n] (n contiguous) -> ldmatrix.trans.
-__device__ __forceinline__ void tile_mma_64x64x128_bt(const uint16_t* As, const uint16_t* Bs, float (&acc)[8][4], int warp, int lane) {
-  const int wr = warp & 3, wn = warp >> 2;
+// 16 rows x 16 * nj columns of a warp, over one 128-wide k chunk: A rows at As (kStride), B [128 k][128 n] at Bs as two 64-column
+// blocks with the 128-byte swizzle (n contiguous -> ldmatrix.trans).
+__device__ __forceinline__ void tile_mma_16xn(const uint16_t* As, uint32_t Bs, float (&acc)[4][4], int col0, int nj, int lane) {
+  const int m = lane >> 3;
 #pragma unroll
   for (int ks = 0; ks < 8; ks++) {
     uint32_t a[4];
-    const int m = lane >> 3;
-    {
-      const int row = wr * 16 + (m & 1) * 8 + (lane & 7);
-      const int col = ks * 16 + (m >> 1) * 8;
-      ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + row * kStride + col));
-    }
+    ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + ((m & 1) * 8 + (lane & 7)) * kStride + ks * 16 + (m >> 1) * 8));
+    const int krow = ks * 16 + (m & 1) * 8 + (lane & 7);
 #pragma unroll
-    for (int n2 = 0; n2 < 4; n2++) {
+    for (int j = 0; j < 2; j++) {
+      if (j >= nj) break;
+      const int col = col0 + j * 16 + (m >> 1) * 8;
       uint32_t b0, b1, b2, b3;
-      const int krow = ks * 16 + (m & 1) * 8 + (lane & 7);
-      const int ncol = wn * 64 + n2 * 16 + (m >> 1) * 8;
-      ldmatrix_x4_trans(b0, b1, b2, b3, smem_u32(Bs + krow * kStride + ncol));
-      mma_bf16_16816(acc[2 * n2], a, b0, b1);
-      mma_bf16_16816(acc[2 * n2 + 1], a, b2, b3);
+      ldmatrix_x4_trans(b0, b1, b2, b3, Bs + (col >> 6) * 16384 + swz128(krow, (col & 63) >> 3));
+      mma_bf16_16816(acc[2 * j], a, b0, b1);
+      mma_bf16_16816(acc[2 * j + 1], a, b2, b3);
     }
   }
 }
@@ -231,17 +233,21 @@ __device__ __forceinline__ void tile_mma_64x64x128_bt(const uint16_t* As, const 
 // same 4 of every 128 latent columns, so every load instruction of a warp is 512 contiguous bytes of one partial row
 // (four threads per row with 128 bytes each, the first layout, put 32 different cache lines into every load
 // instruction: the kernel spent most of its time in the load unit's address stage).  The weights of a row's items come
-// from one round trip: lane j reads (max, sum) of item j, the warp reduces.  Four items are in flight per lane.
+// from one round trip: lane j reads (max, sum) of item j, the warp reduces.
+// kChunks: 128-column chunks of a warp, 4 / kChunks warps share a row; 16 / kChunks items are in flight per lane.  A call of
+// up to four rows has more warps than rows, and its rows the most items (each worker holds a piece of some sequence).
 // Rows past the batch are zero rows of the MMA tile.
 constexpr int kMergeWarps = 16;
-// `after_first_requests` runs once per thread, after the loads of the warp's first row have been issued: work that
-// stalls the thread for its own reasons goes there, under the shadow of that round trip.
-template <typename Hook>
+template <int kChunks>
 __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                const int32_t* __restrict__ chunk_off, int r0, int rows, int S, int H, int h, int dC, int nk,
-                                                int rows_total, Hook&& after_first_requests) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  bool hook_due = true;
+                                                const int32_t* __restrict__ chunk_off, int r0, int rows, int tile_rows, int S, int H, int h, int dC, int nk_all,
+                                                int rows_total) {
+  constexpr int kParts = kMaxChunks / kChunks, kItems = 16 / kChunks, kRowStep = kMergeWarps / kParts;
+  const int warp = (int)(threadIdx.x >> 5) / kParts, lane = threadIdx.x & 31;   // the warp's first row of the tile
+  const int k0 = (int)(threadIdx.x >> 5) % kParts * kChunks, nk = min(kChunks, nk_all - k0);
+  if (nk <= 0) return;
+  part_o += k0 * 128;
+  As += (size_t)k0 * 64 * kStride;
   // The item range of a row is the first of two dependent round trips to L2, so it is requested one row ahead.
   int c0_next = 0, c1_next = 0;
   if (r0 + warp < rows) {
@@ -249,40 +255,36 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
     c0_next = __ldg(chunk_off + i);
     c1_next = __ldg(chunk_off + i + 1);
   }
-  for (int row = warp; row < 64; row += kMergeWarps) {
+  for (int row = warp; row < tile_rows; row += kRowStep) {
     const int r = r0 + row;
     const int c0 = c0_next, c1 = c1_next;
     c0_next = c1_next = 0;
-    if (row + kMergeWarps < 64 && r + kMergeWarps < rows) {
-      const int i = (r + kMergeWarps) / S;
+    if (row + kRowStep < tile_rows && r + kRowStep < rows) {
+      const int i = (r + kRowStep) / S;
       c0_next = __ldg(chunk_off + i);
       c1_next = __ldg(chunk_off + i + 1);
     }
-    float4 acc[kMaxChunks];
+    float4 acc[kChunks];
 #pragma unroll
-    for (int k = 0; k < kMaxChunks; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < kChunks; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) {
       const size_t prow = (size_t)(r % S) * H + h;
-      // (max, sum) of this lane's item of every group of 32, and at the same time the partial rows of the first four
+      // (max, sum) of this lane's item of every group of 32, and at the same time the partial rows of the first
       // items: one memory round trip serves the common case of a sequence cut into a handful of items
       const int n_items = c1 - c0;
       if (n_items <= 0) goto store_row;   // no partial to merge: a zero row
       float2 ml = make_float2(-INFINITY, 0.f);
       if (lane < n_items) ml = __ldg(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
-      float4 x[4][kMaxChunks];
+      float4 x[kItems][kChunks];
       const int ng0 = min(32, n_items);
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
+      for (int u = 0; u < kItems; u++) {
         // a slot past the group's last item stays zero (its weight is zero too): the load unit's data path, 128 bytes
         // per clock for all 16 warps, is what a row's requests queue on, so no load is spent on padding
         const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(c0 + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
-        for (int k = 0; k < kMaxChunks; k++)
+        for (int k = 0; k < kChunks; k++)
           if (k < nk) x[u][k] = (u < ng0) ? __ldg(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      if (hook_due) {
-        after_first_requests();
-        hook_due = false;
       }
       // global maximum and normaliser over all items of the sequence
       float M = ml.x;
@@ -298,7 +300,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
       for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
       const float inv = (L > 0.f) ? 1.0f / L : 0.f;
       for (int cb = c0; cb < c1; cb += 32) {
-        // this lane's item of the group of 32: its weight; then four items at a time, weights by shuffle
+        // this lane's item of the group of 32: its weight; then kItems at a time, weights by shuffle
         float w_mine = 0.f;
         if (cb == c0) {
           w_mine = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M) * inv;
@@ -307,22 +309,22 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
           w_mine = (m == -INFINITY) ? 0.f : exp2f(m - M) * inv;
         }
         const int ng = min(32, c1 - cb);
-        for (int j = 0; j < ng; j += 4) {
-          if (cb != c0 || j != 0) {   // the first four items of the row are in flight already
+        for (int j = 0; j < ng; j += kItems) {
+          if (cb != c0 || j != 0) {   // the first items of the row are in flight already
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < kItems; u++) {
               const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(cb + j + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
-              for (int k = 0; k < kMaxChunks; k++)
+              for (int k = 0; k < kChunks; k++)
                 if (k < nk) x[u][k] = (j + u < ng) ? __ldg(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
+          for (int u = 0; u < kItems; u++) {
             float w = __shfl_sync(0xffffffffu, w_mine, min(j + u, 31));
             if (j + u >= ng) w = 0.f;
 #pragma unroll
-            for (int k = 0; k < kMaxChunks; k++)
+            for (int k = 0; k < kChunks; k++)
               if (k < nk) {
                 acc[k].x = fmaf(x[u][k].x, w, acc[k].x);
                 acc[k].y = fmaf(x[u][k].y, w, acc[k].y);
@@ -334,12 +336,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
       }
     }
   store_row:
-    if (hook_due) {
-      after_first_requests();
-      hook_due = false;
-    }
 #pragma unroll
-    for (int k = 0; k < kMaxChunks; k++)
+    for (int k = 0; k < kChunks; k++)
       if (k < nk)
         *reinterpret_cast<uint2*>(As + ((size_t)k * 64 + row) * kStride + lane * 4) =
             make_uint2(pack_bf16x2(acc[k].x, acc[k].y), pack_bf16x2(acc[k].z, acc[k].w));
@@ -349,58 +347,61 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
 // Split-KV merge fused into the value up-projection: the A operand (the merged, normalised latent output of
 // 64 rows of one head, as bf16) is built straight from the per-item partials
 //   part_o [item][S * H][dC] f32 (unnormalised), part_ml [item][S * H][2] = (max in the log2 domain, sum),
-// items of sequence i = [chunk_off[i], chunk_off[i + 1]).  All of W_UV's slice for this head (dC x 128 bf16) streams
-// into shared memory as bulk copies while the partials are combined by 16 warps (merge_rows_warp); the first 8 warps
-// then run the MMAs, chunk by chunk as the copies land.
+// items of sequence i = [chunk_off[i], chunk_off[i + 1]).
+// All of W_UV's slice for this head (dC x 128 bf16) is fetched by one thread as 2 * nk TMA boxes before chain_wait(): the
+// weights do not depend on the decode kernel, and the launches before it have waited for everything older (as 512 bulk
+// copies of a row each, issued behind the merge's first loads, they took 2-3 us to be accepted).  The MMAs of the row
+// groups that hold a row are shared by all 16 warps (8 for up to 16 rows), chunk by chunk as the boxes land.
 // grid (H, ceil(rows/64)), 512 threads, row = seq_index * S + query token.  dC = 128 * nk, nk <= 4.
-__global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                                const int32_t* __restrict__ chunk_off, const uint16_t* __restrict__ W_UV,
+__global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const float* __restrict__ part_o,
+                                                                const float* __restrict__ part_ml, const int32_t* __restrict__ chunk_off,
                                                                 void* __restrict__ out, int out_bf16, int rows, int S, int H, int dC,
                                                                 int32_t* __restrict__ status) {
-  extern __shared__ __align__(16) uint16_t sm[];
-  __shared__ __align__(8) uint64_t w_full[kMaxChunks];   // chunk k of W_UV has landed (bytes counted by the bulk copies)
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t w_full[kMaxChunks];   // chunk k of W_UV has landed (bytes counted by the TMA loads)
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int nk = dC / 128;
-  uint16_t* As = sm;                             // [nk][64][kStride]
-  uint16_t* Bs = sm + (size_t)nk * 64 * kStride;  // [nk][128][kStride]
+  const uint32_t Bs = smem_u32(smem);                                       // [nk][2 halves of 64 columns][128][64], swizzled
+  uint16_t* As = reinterpret_cast<uint16_t*>(smem + (size_t)nk * 32768);    // [nk][64][kStride]
   const int h = blockIdx.x, r0 = blockIdx.y * 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows_total = S * H;
   chain_release();
-  chain_wait();   // the partial results come from the kernel before this one
-  // W_UV's slice comes in as one 256-byte bulk copy per latent row, through the TMA unit: as 16-byte cp.async requests
-  // the same 128 KB sat in the load/store unit's queue ahead of the merge's own loads, whose round trips then took
-  // 1.0-1.6 us each.
   if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmap_w);
     for (int k = 0; k < nk; k++) mbar_init(&w_full[k], 1);
     fence_mbar_init();
+    for (int k = 0; k < nk; k++) {
+      mbar_expect_tx(&w_full[k], 32768);
+      tma_load_2d(smem + (size_t)k * 32768, &tmap_w, h * kDh, k * 128, &w_full[k]);
+      tma_load_2d(smem + (size_t)k * 32768 + 16384, &tmap_w, h * kDh + 64, k * 128, &w_full[k]);
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < nk; k++) mbar_expect_tx(&w_full[k], 128u * kDh * 2u);
-  // 512 bulk copies queue up in the TMA unit (2-3 us until the last is accepted), so each thread issues its own after the
-  // loads of its first row are on their way
-  merge_rows_warp(As, part_o, part_ml, chunk_off, r0, rows, S, H, h, dC, nk, rows_total, [&]() {
-    for (int e = threadIdx.x; e < nk * 128; e += blockDim.x)
-      bulk_load_1d(Bs + (size_t)e * kStride, W_UV + (size_t)e * H * kDh + (size_t)h * kDh, kDh * 2, &w_full[e >> 7]);
-  });
-  float acc[8][4];
+  chain_wait();   // the partial results come from the kernel before this one
+  const int rows_here = min(64, rows - r0), groups = rows_here <= 16 ? 1 : rows_here <= 32 ? 2 : 4;
+  if (rows_here <= 4) merge_rows_warp<1>(As, part_o, part_ml, chunk_off, r0, rows, groups * 16, S, H, h, dC, nk, rows_total);
+  else if (rows_here <= 8) merge_rows_warp<2>(As, part_o, part_ml, chunk_off, r0, rows, groups * 16, S, H, h, dC, nk, rows_total);
+  else merge_rows_warp<4>(As, part_o, part_ml, chunk_off, r0, rows, groups * 16, S, H, h, dC, nk, rows_total);
+  float acc[4][4];
 #pragma unroll
-  for (int i = 0; i < 8; i++)
+  for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-  __syncthreads();   // the merged A tiles are complete
-  if (warp >= 8) return;
+  __syncthreads();   // the merged A tiles are complete, and the barriers visible
+  const int nj = groups == 4 ? 2 : 1, row_w = (warp % groups) * 16, col0 = (warp / groups) * 16 * nj;
+  if (col0 >= kDh) return;   // up to 16 rows: eight warps have all columns
   for (int k = 0; k < nk; k++) {
     if (!mbar_wait(&w_full[k], 0)) set_status(status, RELUX_ERR_TIMEOUT);   // bounded: a copy that never lands is reported, not waited for
-    tile_mma_64x64x128_bt(As + (size_t)k * 64 * kStride, Bs + (size_t)k * 128 * kStride, acc, warp, lane);
+    tile_mma_16xn(As + ((size_t)k * 64 + row_w) * kStride, Bs + k * 32768, acc, col0, nj, lane);
   }
 #pragma unroll
   for (int hf = 0; hf < 2; hf++) {
-    const int r = r0 + (warp & 3) * 16 + hf * 8 + (lane >> 2);
+    const int r = r0 + row_w + hf * 8 + (lane >> 2);
     if (r >= rows) continue;
-    const size_t off = ((size_t)r * H + h) * kDh + (warp >> 2) * 64 + 2 * (lane & 3);
+    const size_t off = ((size_t)r * H + h) * kDh + col0 + 2 * (lane & 3);
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
+    for (int nt = 0; nt < 4; nt++) {
+      if (nt >= 2 * nj) break;
       const float x = acc[nt][hf * 2], y = acc[nt][hf * 2 + 1];
       if (out_bf16) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + off + nt * 8) = pack_bf16x2(x, y);
       else *reinterpret_cast<float2*>(reinterpret_cast<float*>(out) + off + nt * 8) = make_float2(x, y);
@@ -423,17 +424,14 @@ int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rop
   return RELUX_OK;
 }
 
-// One launch: absorb + append of the step's rows + stream partition (see mla_prep_kernel).  n_seqs + 1 extra blocks
-// must fit one z slice of the absorb grid.
-bool mla_prep_fits(int n_seqs, int H, int dC) { return n_seqs + 1 <= H * (dC / 128); }
+// One launch: absorb + append of the step's rows + stream partition (see mla_prep_kernel).
 int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows,
-                        int H, int dC, int dHR, const PrepAppend& ap, const PrepPlan& pl, bool chained) {
-  const int z_absorb = (rows + 63) / 64;
-  dim3 grid(H, dC / 128, z_absorb + 1);
+                        int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained) {
+  const unsigned blocks = (unsigned)ap.n_seqs + 1u + (unsigned)H * (unsigned)(dC / 128) * (unsigned)((rows + 63) / 64);
   const size_t smem = (size_t)(64 + 128) * kStride * 2;
   if (int32_t rc = allow_smem(dev, mla_prep_kernel, smem)) return rc;
-  RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, grid, dim3(128), smem, dev->stream, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC,
-                                dHR, z_absorb, ap, pl));
+  RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, dim3(blocks), dim3(128), smem, dev->stream, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H,
+                                dC, dHR, weights_ready ? 1 : 0, ap, pl));
   count_launch(dev);
   return RELUX_OK;
 }
@@ -451,10 +449,15 @@ int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W
 int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
                                  void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
   dim3 grid(H, (rows + 63) / 64);
-  const size_t smem = (size_t)(dC / 128) * (64 + 128) * kStride * 2;
+  const size_t smem = (size_t)(dC / 128) * (32768 + 64 * kStride * 2) + 1024;
+  CUtensorMap tw;   // W_UV [dC][H * 128], 128 x 64 boxes
+  if (!make_tmap_2d(&tw, (void*)W_UV, (uint64_t)dC, (uint64_t)H * kDh, 64, 128)) {
+    set_error("tensor map for w_uv could not be encoded");
+    return RELUX_ERR_CUDA;
+  }
   if (int32_t rc = allow_smem(dev, mla_merge_vup_mma_kernel, smem)) return rc;
-  RELUX_CUDA_TRY(launch_chained(chained, mla_merge_vup_mma_kernel, grid, dim3(32 * kMergeWarps), smem, dev->stream, part_o, part_ml, chunk_off,
-                                W_UV, out, out_bf16, rows, S, H, dC, status));
+  RELUX_CUDA_TRY(launch_chained(chained, mla_merge_vup_mma_kernel, grid, dim3(32 * kMergeWarps), smem, dev->stream, tw, part_o, part_ml, chunk_off,
+                                out, out_bf16, rows, S, H, dC, status));
   count_launch(dev);
   return RELUX_OK;
 }

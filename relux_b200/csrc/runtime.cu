@@ -1238,7 +1238,7 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   const bool same_ids = (!kv->seq_ids && !attn->seq_ids) ||
                         (kv->seq_ids && attn->seq_ids && memcmp(kv->seq_ids, attn->seq_ids, sizeof(int32_t) * (size_t)std::max(0, kv->n_seqs)) == 0);
   const bool fuse = kind == RELUX_POOL_MLA && p->prm.kind == RELUX_POOL_MLA && same_ids && kv->n_seqs > 0 && kv->n_seqs <= p->prm.max_seqs &&
-                    kv->a && kv->b && attn->num_heads > 0 && attn->head_dim > 0 && mla_step_fusable(p, *attn, kv->n_seqs) &&
+                    kv->a && kv->b && attn->num_heads > 0 && attn->head_dim > 0 && mla_step_fusable(p, *attn) &&
                     (kv->dtype == RELUX_DTYPE_F32 || kv->dtype == RELUX_DTYPE_BF16) && (kv->mem == RELUX_MEM_HOST || kv->mem == RELUX_MEM_DEVICE) &&
                     !(kv->flags & ~RELUX_CALL_PIPELINED) && kv->layer >= 0 && kv->layer < p->prm.num_layers;
   if (!fuse) {
