@@ -31,17 +31,53 @@ constexpr int kTileN = 128, kTileK = 64;
 constexpr int kStageW = kTileK * kTileN * 2;   // 16 KB of weights: two [64 k][64 n] blocks, 128-byte swizzle, MN-major
 constexpr int kMaxTok = 256;                   // activation rows of one block
 
-// A launch's work: the K steps of all 128-column tiles laid end to end, cut into `workers` ranges that differ by at most
-// one step.  A PIECE is the part of a tile inside one range; piece j of a tile (in range order) is split j of the result.
+// How a launch's 128-column tiles are dealt out.  `full` rounds of whole tiles, neighbouring tiles side by side: the workers
+// then walk K in step and together read whole weight rows, which DRAM serves faster than 256-byte pieces of rows that lie far
+// apart (0.54 GB: 86.8 us so, 90.1 us with every worker somewhere else in K; 0.82 GB: 128.5 against 130.8 us).  The tiles that
+// are left are cut along K, `split` equal parts each (also in step) where that keeps five of six workers busy; otherwise
+// (split = 0) their K steps, laid end to end, are cut into ranges that differ by at most one step.  A PIECE is the part of a
+// tile that one worker does; piece j of a tile (in K order) is split j of the result.
 struct GemmRanges {
-  int32_t steps, range, more;   // K steps per tile; steps per worker, one more for the first `more` of them.  steps = 0: one piece
-  __host__ __device__ int begin(int w) const { return w * range + (w < more ? w : more); }
-  __host__ __device__ int worker_of(int u) const {
+  int32_t workers, steps, full, split;   // steps: K steps per tile.  steps = 0: one piece per tile
+  int32_t range, more;                   // split = 0: steps per worker, one more for the first `more` of them
+  int32_t rest;                          // tiles that are left after the full rounds
+  __host__ __device__ int begin(int w) const {   // in steps of the tiles that are left
+    if (!split) return w * range + (w < more ? w : more);
+    return w < rest * split ? w / split * steps + w % split * steps / split : rest * steps;
+  }
+  __host__ __device__ int worker_of(int u) const {   // split = 0
     const int big = more * (range + 1);
     return u < big ? (int)((unsigned)u / (unsigned)(range + 1)) : more + (int)((unsigned)(u - big) / (unsigned)range);
   }
   __host__ __device__ int pieces(int tile) const {
-    return steps ? worker_of((tile + 1) * steps - 1) - worker_of(tile * steps) + 1 : 1;
+    const int t = tile - full * workers;
+    if (!steps || t < 0) return 1;
+    return split ? split : worker_of((t + 1) * steps - 1) - worker_of(t * steps) + 1;
+  }
+};
+// The pieces of one worker: GemmWalk walk(rg, w); while (walk.next()) ... walk.tile, steps [k0, k1), split.
+struct GemmWalk {
+  const GemmRanges& g;
+  int w, n, u, u1, tile, k0, k1, split;
+  __device__ GemmWalk(const GemmRanges& rg, int worker)
+      : g(rg), w(worker), n(0), u(rg.begin(worker)), u1(rg.begin(worker + 1)), tile(0), k0(0), k1(0), split(0) {}
+  __device__ int total() const { return g.full * g.steps + g.begin(w + 1) - g.begin(w); }
+  __device__ bool next() {
+    split = 0;
+    if (n < g.full) {
+      tile = n++ * g.workers + w;
+      k0 = 0;
+      k1 = g.steps;
+      return true;
+    }
+    if (u >= u1) return false;
+    const int t = u / g.steps;
+    tile = g.full * g.workers + t;
+    k0 = u - t * g.steps;
+    u = min(u1, (t + 1) * g.steps);
+    k1 = u - t * g.steps;
+    split = g.split ? w - t * g.split : w - g.worker_of(t * g.steps);
+    return true;
   }
 };
 
@@ -97,13 +133,13 @@ __device__ __forceinline__ void gemm_wait(uint64_t* bar, uint32_t parity, GemmBa
 //   * The WEIGHTS are the M = 128 operand (MN-major: the row-major rows as they lie in HBM) and the activations, 16 to 256
 //     rows, the N operand, so that a stage is 16 KB of weights and no more activations than there are: with the
 //     activations as the M = 128 operand a stage of 16 rows was half padding, read from L2 for every step.
-//   * One CTA per SM walks an equal share of the steps of all tiles without draining its pipeline in between (two
-//     accumulators: a piece is written out while the next one's MMAs run).
+//   * One CTA per SM walks its pieces (GemmRanges) without draining its pipeline in between (two accumulators: a piece is
+//     written out while the next one's MMAs run).
 //   * The weights do not depend on the launches before this one, whose tail and launch gap they hide: the producer
 //     fills its stages with them before chain_wait().  The first kernel of a layer step (cast_bf16_kernel) releases its
 //     successors only when everything before the step is complete, so that weights written earlier in the stream are there.
 // Measured with the chained launches around it (a layer step, before -> now): 16 rows of d_model 16384, 1.36 GB of weights,
-// 308 -> 286 us; 24 rows of d_model 4096, 84 MB, 82.8 -> 67.3 us.
+// 308 -> 272 us; 24 rows of d_model 4096, 84 MB, 82.8 -> 67.0 us.
 template <int NT>
 __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmParams prm) {
   using SH = GemmShape<NT>;
@@ -112,7 +148,7 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
   GemmBars* bars = reinterpret_cast<GemmBars*>(smem + kStages * SH::kStage);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * NT;
-  const int u0 = prm.rg.begin(blockIdx.x), u1 = prm.rg.begin(blockIdx.x + 1);
+  GemmWalk walk(prm.rg, blockIdx.x);
   auto weight_of = [&](int tile) -> int {
     int j = 0;
     while (j + 1 < prm.n_weights && tile >= prm.tile_first[j + 1]) j++;
@@ -143,29 +179,32 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
   if (warp == 4) {
     const bool el = elect_one();
     if (el) tma_prefetch_desc(&maps.a);
-    int tile = u0 / prm.rg.steps, k = u0 - tile * prm.rg.steps, j = weight_of(tile);
-    auto load_w = [&](int g) {   // the weights of step g of this range; arms the stage for both operands
+    const int n = walk.total(), ahead = min(n, kStages);
+    GemmWalk wx = walk;   // the activations' place, up to kStages steps behind
+    walk.next();
+    wx.next();
+    int k = walk.k0, kx = wx.k0, j = weight_of(walk.tile);
+    auto load_w = [&](int g) {   // the weights of step g of this worker; arms the stage for both operands
       const int s = g % kStages;
       if (el) {
         uint8_t* sw = smem + s * SH::kStage;
-        const int n0 = (tile - prm.tile_first[j]) * kTileN;
+        const int n0 = (walk.tile - prm.tile_first[j]) * kTileN;
         mbar_expect_tx(&bars->full[s], SH::kStage);   // out-of-range parts of a box are zero-filled and still counted
         tma_load_2d(sw, &maps.w[j], n0, k * kTileK, &bars->full[s]);
         tma_load_2d(sw + kStageW / 2, &maps.w[j], n0 + 64, k * kTileK, &bars->full[s]);
       }
       __syncwarp();
-      if (++k == prm.rg.steps) {
-        k = 0;
-        j = weight_of(++tile);
+      if (++k == walk.k1 && walk.next()) {
+        k = walk.k0;
+        j = weight_of(walk.tile);
       }
     };
-    auto load_x = [&](int g, int kx) {
+    auto load_x = [&](int g) {
       const int s = g % kStages;
       if (el) tma_load_2d(smem + s * SH::kStage + kStageW, &maps.a, kx * kTileK, m0, &bars->full[s]);
       __syncwarp();
+      if (++kx == wx.k1 && wx.next()) kx = wx.k0;
     };
-    const int n = u1 - u0, ahead = min(n, kStages);
-    int kx = k;
     for (int g = 0; g < ahead; g++) load_w(g);
     chain_wait();
     for (int g = 0; g < n; g++) {
@@ -173,20 +212,18 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
         gemm_wait(&bars->empty[g % kStages], (g / kStages - 1) & 1, bars, prm.status);
         load_w(g);
       }
-      load_x(g, kx);
-      if (++kx == prm.rg.steps) kx = 0;
+      load_x(g);
     }
   } else if (warp == 5) {
     chain_wait();
     const bool el = elect_one();
     const uint32_t idesc = make_idesc_bf16(kTileN, NT, true, false);
     int g = 0;
-    for (int u = u0, piece = 0; u < u1; piece++) {
-      const int end = min(u1, (u / prm.rg.steps + 1) * prm.rg.steps);
+    for (int piece = 0; walk.next(); piece++) {
       const uint32_t d = tmem + (piece & 1) * SH::kAcc;
       if (piece >= 2) gemm_wait(&bars->acc_empty[piece & 1], ((piece >> 1) - 1) & 1, bars, prm.status);
       tc_fence_after();
-      for (bool first = true; u < end; u++, g++, first = false) {
+      for (int k = walk.k0; k < walk.k1; k++, g++) {
         const int s = g % kStages;
         gemm_wait(&bars->full[s], (g / kStages) & 1, bars, prm.status);
         tc_fence_after();
@@ -196,7 +233,7 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
           const uint64_t dX = make_desc_kmajor_sw128(sw + kStageW);
 #pragma unroll
           for (int kk = 0; kk < kTileK / 16; kk++)
-            umma_ss<1>(d, dW + ((uint32_t)(kk * 2048) >> 4), dX + ((uint32_t)(kk * 32) >> 4), idesc, !first || kk != 0);
+            umma_ss<1>(d, dW + ((uint32_t)(kk * 2048) >> 4), dX + ((uint32_t)(kk * 32) >> 4), idesc, k != walk.k0 || kk != 0);
           umma_commit<1>(&bars->empty[s]);
         }
         __syncwarp();
@@ -207,13 +244,11 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
   } else {
     // epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once
     chain_wait();
-    for (int u = u0, piece = 0; u < u1; piece++) {
-      const int tile = u / prm.rg.steps, j = weight_of(tile);
-      u = min(u1, (tile + 1) * prm.rg.steps);
-      const int split = (int)blockIdx.x - prm.rg.worker_of(tile * prm.rg.steps);
-      const int n = (tile - prm.tile_first[j]) * kTileN + warp * 32 + lane;
+    for (int piece = 0; walk.next(); piece++) {
+      const int j = weight_of(walk.tile);
+      const int n = (walk.tile - prm.tile_first[j]) * kTileN + warp * 32 + lane;
       const int m_end = min(NT, prm.M - m0);
-      float* dst = prm.part + ((size_t)split * prm.M + m0) * prm.n_total + prm.col_first[j] + n;
+      float* dst = prm.part + ((size_t)walk.split * prm.M + m0) * prm.n_total + prm.col_first[j] + n;
       gemm_wait(&bars->acc_full[piece & 1], (piece >> 1) & 1, bars, prm.status);
       tc_fence_after();
       const bool ok = !bars->abort_flag, mine = n < prm.n_cols[j];
@@ -387,14 +422,22 @@ int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const 
   const int steps = (K + kTileK - 1) / kTileK;
   if ((int64_t)tiles * steps >= (int64_t)1 << 31) { set_error("a projection of more than 2^31 steps"); return RELUX_ERR_UNSUPPORTED; }
   const int units = tiles * steps;
-  // One range per SM, the rows' blocks side by side; ranges of fewer than four steps do not pay for their piece of the
+  // One worker per SM, the rows' blocks side by side; pieces of fewer than four steps do not pay for their share of the
   // result.  The pieces have to fit the scratch: one worker always does.
   int workers = std::max(1, std::min(std::max(1, p->dev->sm_count) / mblocks, units / 4));
   if (const int ov = p->tune.get(RELUX_TUNE_GEMM_SPLIT)) workers = std::max(1, std::min(units, tiles * ov));   // tuning knob
   for (;; workers = (workers + 1) / 2) {
-    g.rg = GemmRanges{steps, units / workers, units % workers};
-    int most = 0;
-    for (int t = 0; t < tiles; t++) most = std::max(most, g.rg.pieces(t));
+    GemmRanges& r = g.rg;
+    r = GemmRanges{workers, steps, tiles / workers, 0, 0, 0, tiles % workers};
+    int most = 1;
+    if (r.rest) {
+      const int fits = workers / r.rest, most_split = std::max(1, steps / 4);
+      if (fits >= most_split) r.split = most_split;
+      else if (6 * fits * r.rest >= 5 * workers) r.split = fits;
+      r.range = r.rest * steps / workers;
+      r.more = r.rest * steps % workers;
+      for (int t = r.full * workers; t < tiles; t++) most = std::max(most, r.pieces(t));
+    }
     if (workers == 1 || (size_t)most * M * cols * 4 <= part_cap_bytes) break;
   }
   g.part = part;
