@@ -134,6 +134,8 @@ struct Pool {
   GrowBuf part_o;    // split-KV partial accumulators, f32
   GrowBuf part_ml;   // split-KV partial (max, sum), f32 pairs
   GrowBuf stream_done;   // GQA stream kernel: finished pieces per (sequence, kv head), zero between launches
+  int32_t* sel_host = nullptr;   // page-locked result words of the selection kernels
+  size_t sel_words = 0;
   GrowBuf seq_list;      // GQA stream kernel: the sequences of a call too long for kernel arguments
   GrowBuf work;      // int32 work list + per-sequence chunk offsets
   GrowBuf o_lat;     // MLA merged latent output, f32/bf16

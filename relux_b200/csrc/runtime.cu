@@ -238,6 +238,7 @@ static void pool_free_all(Pool* p) {
   fr(p->in_a.p); fr(p->in_b.p); fr(p->out_buf.p); fr(p->q_abs.p); fr(p->part_o.p); fr(p->part_ml.p); fr(p->work.p); fr(p->stream_done.p); fr(p->seq_list.p);
   fr(p->o_lat.p); fr(p->q_conv.p); fr(p->rope_tab.p); fr(p->layer_buf.p); fr(p->shadow_f32); fr(p->chunk_tab.p); fr(p->step_rows.p); fr(p->expand_buf.p);
   if (p->h_stage) cudaFreeHost(p->h_stage);
+  if (p->sel_host) cudaFreeHost(p->sel_host);
   for (cudaEvent_t ev : p->stage_ev)
     if (ev) cudaEventDestroy(ev);
   fr(p->proj_times.slots);   // those of the attention calls are part of `meta`

@@ -11,6 +11,7 @@
 // instead of sequential), so a decision can only differ when a draw falls within rounding distance of a boundary.
 // REFERENCE: one thread per sequence walks the reference's loops in the reference's order (bit-exact, slow).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdint>
 #include <cstdlib>
@@ -46,6 +47,7 @@ struct SelParams {
   float top_p, min_p;
   int32_t lookahead;             // accept loop: take the next position's maxima in the pass that sums this one's
   int32_t batched;               // accept loop: maxima of all positions' rows in one stage, all sums in a second
+  TimeStamp time;
 };
 
 // Shared memory of one CTA: exchange slots read by the other CTAs of the cluster.
@@ -370,11 +372,10 @@ __device__ bool radix_select(Ctx& c, const float* __restrict__ row, KeyF key_wei
 // Inverse-CDF search: the first index whose running sum of prob(index, value) exceeds r (Sampler.Sample step 8,
 // sampler.go:200-209; resampleRejected, speculative.go:271-291), or `dflt` when the sum never does.  Sums run per
 // warp segment, then in segment order; the segment that crosses is walked again in index order.
-template <class ProbF>
-__device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, float r, int dflt, int32_t* out) {
-  float part = 0.0f;
-  for_segment(c, row, [&](int i, float v) { part += prob(i, v); });
-  part = warp_sum(part);
+// sum_segment(): this lane's share of the sum over the warp's segment.
+template <class ProbF, class SumF>
+__device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, float r, int dflt, int32_t* out, SumF sum_segment) {
+  const float part = warp_sum(sum_segment());
   if (c.lane == 0) c.sh->warp_seg[c.warp] = part;
   __syncthreads();
   float tot = 0.0f;
@@ -450,6 +451,14 @@ __device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, floa
       if (c.lane == 0) *out = hit_idx;
     }
   }
+}
+template <class ProbF>
+__device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, float r, int dflt, int32_t* out) {
+  cdf_find(c, row, prob, r, dflt, out, [&]() {
+    float part = 0.0f;
+    for_segment(c, row, [&](int i, float v) { part += prob(i, v); });
+    return part;
+  });
 }
 
 // Sampler.Sample with a small top-k, finished on a list: after top-k only the k largest logits (and their ties) carry
@@ -696,6 +705,7 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
   c.wlo = min(c.hi, c.lo + c.warp * wper);
   c.whi = min(c.hi, c.wlo + wper);
   const int b = blockIdx.x / c.csize;
+  if (threadIdx.x == 0) stamp_begin(prm.time);
   const float* draws = prm.draws + (size_t)b * (k + 1);
   int32_t* out_tok = prm.next_token + b;
   const bool writer = c.rank == 0 && threadIdx.x == 0;
@@ -788,22 +798,24 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     const float u = draws[used++];
     if (u < ap) continue;
     // rejected at i: resample from norm(max(0, p_target - p_draft))   speculative.go:256-295
-    auto adj = [&](int j, float tv) {
+    auto adj = [&](float tv, float dv) {
       float tp = __fmul_rn(fastexp32_ref(__fsub_rn(tv, mt)), invt);
-      float dp = __fmul_rn(fastexp32_ref(__fsub_rn(__ldg(drow + j), md)), invd);
+      float dp = __fmul_rn(fastexp32_ref(__fsub_rn(dv, md)), invd);
       float diff = __fsub_rn(tp, dp);
       return diff < 0.0f ? 0.0f : diff;
     };
     v4[0] = v4[1] = v4[2] = v4[3] = 0.0f;
-    for_segment2(c, drow, trow, [&](int, float dv, float tv) {
-      float diff = __fsub_rn(__fmul_rn(fastexp32_ref(__fsub_rn(tv, mt)), invt), __fmul_rn(fastexp32_ref(__fsub_rn(dv, md)), invd));
-      v4[0] += diff < 0.0f ? 0.0f : diff;
-    });
+    for_segment2(c, drow, trow, [&](int, float dv, float tv) { v4[0] += adj(tv, dv); });
     cluster_reduce4<0>(c, v4);
     const float r = draws[used++];
     if (v4[0] > 0.0f) {
       const float inv = __fdiv_rn(1.0f, v4[0]);
-      cdf_find(c, trow, [&](int j, float tv) { return __fmul_rn(adj(j, tv), inv); }, r, 0, out_tok);
+      // the sums read both rows as vectors (through prob, the draft row came as single floats)
+      cdf_find(c, trow, [&](int j, float tv) { return __fmul_rn(adj(tv, __ldg(drow + j)), inv); }, r, 0, out_tok, [&]() {
+        float part = 0.0f;
+        for_segment2(c, drow, trow, [&](int, float dv, float tv) { part += __fmul_rn(adj(tv, dv), inv); });
+        return part;
+      });
     } else {
       cdf_find(c, trow, [&](int, float tv) { return __fmul_rn(fastexp32_ref(__fsub_rn(tv, mt)), invt); }, r, 0, out_tok);
     }
@@ -813,6 +825,7 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
   if (!done) sample_row(c, prm, prm.target_logits + ((size_t)b * (k + 1) + k) * V, draws[used++], out_tok);
   if (writer && prm.n_accepted) prm.n_accepted[b] = n_acc;
   cl.sync();   // no CTA leaves while another may still read its exchange buffers
+  if (threadIdx.x == 0) stamp_end(prm.time);
 }
 
 // ---- REFERENCE: one thread per sequence, the reference's loops in the reference's order ------------------------
@@ -1007,15 +1020,27 @@ __global__ void repetition_penalty_kernel(const float* __restrict__ src, float* 
   }
 }
 
-// Launches the selection kernel on device-resident inputs (prm holds the input pointers, k and vocab) and brings the
-// 2 n result words (accepted counts, then tokens) to the host; synchronises the stream.
-static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_sampler_params& sp, int mode, std::vector<int32_t>& host) {
+// Launches the selection kernel on device-resident inputs (prm holds the input pointers, k and vocab) and synchronises the
+// stream.  *host: the 2 n result words (accepted counts, then tokens), which the kernel writes to page-locked host memory
+// itself (one word each per row, nothing reads them back), and it stamps its own time: the copy, two event records and a
+// memset around it took 12 us of a 200 us call.
+static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_sampler_params& sp, int mode, const int32_t** host) {
   Device* dev = p->dev;
   const int V = prm.vocab;
   int32_t rc;
-  rc = grow(dev, p->out_buf, sizeof(int32_t) * 2 * (size_t)n);
-  if (rc) return rc;
-  prm.n_accepted = (int32_t*)p->out_buf.p;
+  if (p->sel_words < 2 * (size_t)n) {
+    if (p->sel_host) {
+      RELUX_CUDA_TRY(cudaStreamSynchronize(dev->stream));   // an earlier call that failed may have left its kernel running
+      int32_t* old = p->sel_host;
+      p->sel_host = nullptr;
+      p->sel_words = 0;
+      RELUX_CUDA_TRY(cudaFreeHost(old));
+    }
+    const size_t words = std::max<size_t>(512, 2 * (size_t)n);
+    RELUX_CUDA_TRY(cudaMallocHost((void**)&p->sel_host, words * sizeof(int32_t)));
+    p->sel_words = words;
+  }
+  prm.n_accepted = p->sel_host;
   prm.next_token = prm.n_accepted + n;
   prm.status = p->d_status;
   prm.temperature = sp.temperature;
@@ -1042,10 +1067,13 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
     if (rc) return rc;
   }
   // device time of the selection kernel, readable through relux_pool_kernel_ms_mean like the attention kernels'
-  if (int32_t rct = time_events_begin(p, p->attn_times)) return rct;
   if (mode == RELUX_ATTN_REFERENCE) {
+    if (int32_t rct = time_events_begin(p, p->attn_times)) return rct;
     spec_accept_reference_kernel<<<(n + 31) / 32, 32, 0, dev->stream>>>(prm, n, (float*)p->part_o.p, (int32_t*)p->part_ml.p);
+    RELUX_CUDA_TRY(cudaGetLastError());
+    if (int32_t rct = time_events_end(p, p->attn_times)) return rct;
   } else {
+    prm.time = time_stamp_next(p, p->attn_times);
     // Cluster size: slices should stay long enough to keep 512 threads busy, and all sequences should be resident at
     // once -- a second wave of clusters doubles the latency of the whole chain, which costs more than longer slices.
     const int by_vocab = V >= 32768 ? 8 : V >= 8192 ? 4 : V >= 2048 ? 2 : 1;
@@ -1090,12 +1118,9 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
     cfg.numAttrs = 1;
     RELUX_CUDA_TRY(cudaLaunchKernelEx(&cfg, spec_accept_kernel, prm));
   }
-  RELUX_CUDA_TRY(cudaGetLastError());
-  if (int32_t rct = time_events_end(p, p->attn_times)) return rct;
   count_launch(dev);
-  host.resize((size_t)2 * n);
-  RELUX_CUDA_TRY(cudaMemcpyAsync(host.data(), p->out_buf.p, sizeof(int32_t) * 2 * (size_t)n, cudaMemcpyDeviceToHost, dev->stream));
   RELUX_CUDA_TRY(cudaStreamSynchronize(dev->stream));
+  *host = p->sel_host;
   return RELUX_OK;
 }
 
@@ -1154,8 +1179,8 @@ int32_t do_spec_accept(Pool* p, const relux_spec_accept_args* a) {
   prm.draws = (const float*)d;
   prm.k = k;
   prm.vocab = V;
-  std::vector<int32_t> host;
-  rc = launch_selection(p, prm, n, a->sampler, a->mode, host);
+  const int32_t* host = nullptr;
+  rc = launch_selection(p, prm, n, a->sampler, a->mode, &host);
   if (rc) return rc;
   for (int i = 0; i < n; i++) {
     if (a->n_accepted) a->n_accepted[i] = host[i];
@@ -1227,8 +1252,8 @@ int32_t do_sample(Pool* p, const relux_sample_args* a) {
   }
   prm.k = 0;
   prm.vocab = V;
-  std::vector<int32_t> host;
-  rc = launch_selection(p, prm, n, a->sampler, a->mode, host);
+  const int32_t* host = nullptr;
+  rc = launch_selection(p, prm, n, a->sampler, a->mode, &host);
   if (rc) return rc;
   for (int i = 0; i < n; i++) a->tokens[i] = host[(size_t)n + i];
   return RELUX_OK;
