@@ -5,7 +5,7 @@
 //   up-proj: out[row][h][:]    = O_lat[row][h][:] . W_UV[:, h*Dh:(h+1)*Dh]          M = rows, N = Dh,  K = dC
 // Both are about 1 GFLOP per step at batch 64 (1.5 % of the decode's work) and move ~30 MB; they are written to stay
 // out of the way of the decode kernel, not to chase the tensor peak: one CTA per (head, 128-wide slice, 64 rows),
-// operands staged in padded shared memory (cp.async, every load of a CTA in flight at once), fragments through
+// operands staged in shared memory by a few TMA boxes (every load of a CTA in flight at once), fragments through
 // ldmatrix.  The up-projection also performs the split-KV merge while it builds its A operand.
 // Shapes: Dh = 128, dC a multiple of 128.  Other shapes use the scalar kernels in mla_decode.cu.
 #include "common.cuh"
@@ -20,85 +20,71 @@ constexpr int kDh = 128;
 constexpr int kStride = kDh + 8;  // bf16 elements per shared-memory row (272 B: conflict-free ldmatrix)
 constexpr int kMaxChunks = 4;     // the fused merge + up-projection keeps at most 4 x 128 latent columns in shared memory
 
-// 64 x 128 A tile (rows x k) and 128 x 128 B tile; warp w owns rows 16w..16w+15 and all 128 columns.
-// kBTrans = false: Bs is [n][k] (k contiguous)  -> ldmatrix;  true: Bs is [k][n] (n contiguous) -> ldmatrix.trans
-template <bool kBTrans>
+// 64 x 128 A tile (rows x k) and 128 x 128 B tile [k][n] (n contiguous -> ldmatrix.trans); warp w owns rows 16w..16w+15 and all
+// 128 columns.
 __device__ __forceinline__ void tile_mma_64x128x128(const uint16_t* As, const uint16_t* Bs, float (&acc)[16][4], int warp, int lane) {
 #pragma unroll
   for (int ks = 0; ks < 8; ks++) {
     uint32_t a[4];
-    {
-      const int m = lane >> 3;
-      const int row = warp * 16 + (m & 1) * 8 + (lane & 7);
-      const int col = ks * 16 + (m >> 1) * 8;
-      ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + row * kStride + col));
-    }
+    const int m = lane >> 3;
+    ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + (warp * 16 + (m & 1) * 8 + (lane & 7)) * kStride + ks * 16 + (m >> 1) * 8));
 #pragma unroll
     for (int n2 = 0; n2 < 8; n2++) {
       uint32_t b0, b1, b2, b3;
-      const int m = lane >> 3;
-      if (!kBTrans) {
-        const int nrow = n2 * 16 + (m >> 1) * 8 + (lane & 7);
-        const int kcol = ks * 16 + (m & 1) * 8;
-        ldmatrix_x4(b0, b1, b2, b3, smem_u32(Bs + nrow * kStride + kcol));
-      } else {
-        const int krow = ks * 16 + (m & 1) * 8 + (lane & 7);
-        const int ncol = n2 * 16 + (m >> 1) * 8;
-        ldmatrix_x4_trans(b0, b1, b2, b3, smem_u32(Bs + krow * kStride + ncol));
-      }
+      ldmatrix_x4_trans(b0, b1, b2, b3, smem_u32(Bs + (ks * 16 + (m & 1) * 8 + (lane & 7)) * kStride + n2 * 16 + (m >> 1) * 8));
       mma_bf16_16816(acc[2 * n2], a, b0, b1);
       mma_bf16_16816(acc[2 * n2 + 1], a, b2, b3);
     }
   }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// grid (H, dC/128, ceil(rows/64)), 128 threads.  Every load of the CTA is in flight at once (cp.async for bf16
-// sources), the result leaves through shared memory as 16-byte row-contiguous stores.
-__device__ __forceinline__ void absorb_block(uint16_t* sm, const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
-                                             const uint16_t* __restrict__ W_UK, uint16_t* __restrict__ q_abs, int rows, int H, int dC,
-                                             int dHR, int bx, int by, int bz, bool wait_for_queries = false) {
-  uint16_t* As = sm;                  // [64][kStride]
-  uint16_t* Bs = sm + 64 * kStride;   // [128][kStride]   rows = latent index c, cols = d
+// 64 rows x 128 latent columns of the absorb for one head, by 128 threads.  W_UK's tile [128 c][128 d] and (bf16) the query
+// tile [64 rows][128 d] come as four TMA boxes from one thread: as 3072 cp.async of 16 bytes they took 2.2 us to issue.  Both
+// lie as two 64-column blocks with the 128-byte swizzle.  Up to 32 rows, the warps share the row groups that hold a row.
+// Measured (the whole preparation launch, before -> now): 3 rows 8.1 -> 4.7 us, 64 rows 12.6 -> 12.0 us.
+// The result leaves through shared memory as 16-byte row-contiguous stores.
+constexpr int kAbsorbSmem = 32768 + 16384 + 1024;
+__device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const void* __restrict__ q_nope,
+                                             const void* __restrict__ q_rope, int q_bf16, uint16_t* __restrict__ q_abs, int rows, int H, int dC,
+                                             int dHR, int bx, int by, int bz, int32_t* status, bool wait_for_queries) {
+  __shared__ __align__(8) uint64_t landed;
+  uint8_t* sm = (uint8_t*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* Bs = sm;             // [2 halves of d][128 c][64], swizzled
+  uint8_t* As = sm + 32768;     // [2 halves of d][64 rows][64], swizzled
   const int h = bx, c0 = by * 128, r0 = bz * 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll 4
-  for (int e = threadIdx.x; e < 128 * (kDh / 8); e += blockDim.x) {
-    const int c = e / (kDh / 8), v = e % (kDh / 8);
-    cp_async16(Bs + c * kStride + v * 8, W_UK + (size_t)(c0 + c) * H * kDh + (size_t)h * kDh + (size_t)v * 8);
+  const int rows_here = min(64, rows - r0), groups = rows_here <= 16 ? 1 : rows_here <= 32 ? 2 : 4;
+  if (threadIdx.x == 0) {
+    mbar_init(&landed, 1);
+    fence_mbar_init();
+    mbar_expect_tx(&landed, 32768 + (q_bf16 ? 16384 : 0));
+    tma_load_2d(Bs, tmap_w, h * kDh, c0, &landed);
+    tma_load_2d(Bs + 16384, tmap_w, h * kDh + 64, c0, &landed);
   }
   if (wait_for_queries) chain_wait();
-  // A: 64 rows x 128 d, 8 elements per thread per step
-#pragma unroll 4
-  for (int e = threadIdx.x; e < 64 * (kDh / 8); e += blockDim.x) {
-    const int r = e / (kDh / 8), v = e % (kDh / 8);
-    uint16_t* dst = As + r * kStride + v * 8;
-    if (r0 + r >= rows) {
-      *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-      continue;
+  if (q_bf16) {
+    if (threadIdx.x == 0) {   // rows past the batch are zero-filled
+      tma_load_2d(As, tmap_q, h * kDh, r0, &landed);
+      tma_load_2d(As + 8192, tmap_q, h * kDh + 64, r0, &landed);
     }
-    const size_t off = ((size_t)(r0 + r) * H + h) * kDh + (size_t)v * 8;
-    if (q_bf16) {
-      cp_async16(dst, reinterpret_cast<const uint16_t*>(q_nope) + off);
-    } else {
-      const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_nope) + off);
-      const float4 x = s[0], y = s[1];
-      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
+  } else {
+#pragma unroll 4
+    for (int e = threadIdx.x; e < groups * 16 * (kDh / 8); e += blockDim.x) {
+      const int r = e / (kDh / 8), v = e % (kDh / 8);
+      uint4 w = make_uint4(0, 0, 0, 0);
+      if (r < rows_here) {
+        const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_nope) + ((size_t)(r0 + r) * H + h) * kDh + (size_t)v * 8);
+        const float4 x = s[0], y = s[1];
+        w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
+      }
+      *reinterpret_cast<uint4*>(As + (v >> 3) * 8192 + swz128(r, v & 7)) = w;
     }
   }
-  cp_async_commit();
   const int roww = dC + dHR;
   if (by == 0) {   // the rope part of q~ is a copy (with the same rounding when the source is float32)
     const int vecs = dHR / 8;
-    for (int e = threadIdx.x; e < 64 * vecs; e += blockDim.x) {
+    for (int e = threadIdx.x; e < rows_here * vecs; e += blockDim.x) {
       const int r = e / vecs, v = e % vecs;
-      if (r0 + r >= rows) continue;
       const size_t off = ((size_t)(r0 + r) * H + h) * dHR + (size_t)v * 8;
       uint4 w;
       if (q_bf16) w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_rope) + off);
@@ -110,36 +96,54 @@ __device__ __forceinline__ void absorb_block(uint16_t* sm, const void* __restric
       *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + dC + (size_t)v * 8) = w;
     }
   }
-  cp_async_wait<0>();
-  __syncthreads();
+  __syncthreads();   // the barrier and the float32 rows are visible
+  if (!mbar_wait(&landed, 0)) set_status(status, RELUX_ERR_TIMEOUT);   // bounded: a load that never lands is reported
+  // warp: 16 rows x 32 * groups columns
+  const int m = lane >> 3, row_w = (warp % groups) * 16, col_w = (warp / groups) * 32 * groups;
+  const uint32_t a_base = smem_u32(As), b_base = smem_u32(Bs);
   float acc[16][4];
 #pragma unroll
   for (int i = 0; i < 16; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-  tile_mma_64x128x128<false>(As, Bs, acc, warp, lane);
-  __syncthreads();   // every warp is done with As / Bs: Bs becomes the 64 x 128 output staging tile
-  uint16_t* Os = Bs;
+#pragma unroll
+  for (int ks = 0; ks < 8; ks++) {
+    uint32_t a[4];
+    const int ka = ks * 2 + (m >> 1), kb = ks * 2 + (m & 1);   // 16-byte chunk of the row
+    ldmatrix_x4(a[0], a[1], a[2], a[3], a_base + (ka >> 3) * 8192 + swz128(row_w + (m & 1) * 8 + (lane & 7), ka & 7));
+#pragma unroll
+    for (int n2 = 0; n2 < 8; n2++) {
+      if (n2 >= 2 * groups) break;
+      uint32_t b0, b1, b2, b3;
+      ldmatrix_x4(b0, b1, b2, b3, b_base + (kb >> 3) * 16384 + swz128(col_w + n2 * 16 + (m >> 1) * 8 + (lane & 7), kb & 7));
+      mma_bf16_16816(acc[2 * n2], a, b0, b1);
+      mma_bf16_16816(acc[2 * n2 + 1], a, b2, b3);
+    }
+  }
+  __syncthreads();   // every warp is done with As / Bs: Bs becomes the output staging tile
+  uint16_t* Os = reinterpret_cast<uint16_t*>(Bs);
 #pragma unroll
   for (int hf = 0; hf < 2; hf++) {
-    const int r = warp * 16 + hf * 8 + (lane >> 2);
+    const int r = row_w + hf * 8 + (lane >> 2);
 #pragma unroll
-    for (int nt = 0; nt < 16; nt++)
-      *reinterpret_cast<uint32_t*>(Os + r * kStride + nt * 8 + 2 * (lane & 3)) = pack_bf16x2(acc[nt][hf * 2], acc[nt][hf * 2 + 1]);
+    for (int nt = 0; nt < 16; nt++) {
+      if (nt >= 4 * groups) break;
+      *reinterpret_cast<uint32_t*>(Os + r * kStride + col_w + nt * 8 + 2 * (lane & 3)) = pack_bf16x2(acc[nt][hf * 2], acc[nt][hf * 2 + 1]);
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < 64 * 16; e += blockDim.x) {
+  for (int e = threadIdx.x; e < rows_here * 16; e += blockDim.x) {
     const int r = e / 16, v = e % 16;
-    if (r0 + r >= rows) continue;
     *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + c0 + v * 8) = *reinterpret_cast<const uint4*>(Os + r * kStride + v * 8);
   }
 }
 
-__global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
-                                                             const uint16_t* __restrict__ W_UK, uint16_t* __restrict__ q_abs, int rows,
-                                                             int H, int dC, int dHR) {
-  extern __shared__ __align__(16) uint16_t sm[];
-  absorb_block(sm, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z);
+// grid (H, dC/128, ceil(rows/64)), 128 threads.
+__global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
+                                                             const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
+                                                             uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int32_t* status) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z, status, false);
 }
 
 // The preparation of one MLA decode step in ONE launch: blocks 0 .. n_seqs - 1 append the step's new rows (a sequence
@@ -150,16 +154,18 @@ __global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const void* __restr
 // The kernel releases the launches after it only when everything before it is complete (the up-projection fetches its
 // weights without a wait of its own), unless the launches before it in the call have seen to that (weights_ready): its own
 // weights are then fetched ahead of its wait too.
-__global__ void __launch_bounds__(128) mla_prep_kernel(const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
-                                                       const uint16_t* __restrict__ W_UK, uint16_t* __restrict__ q_abs, int rows, int H,
-                                                       int dC, int dHR, int weights_ready, const PrepAppend ap, const PrepPlan pl) {
-  extern __shared__ __align__(16) uint16_t sm[];
+__global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
+                                                       const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
+                                                       uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int weights_ready,
+                                                       const __grid_constant__ PrepAppend ap, const __grid_constant__ PrepPlan pl) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int e = blockIdx.x;
   if (!weights_ready) chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
   chain_release();
   if (e > ap.n_seqs) {
     const int a = e - ap.n_seqs - 1, slices = dC / 128;
-    absorb_block(sm, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, weights_ready != 0);
+    absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, ap.status,
+                 weights_ready != 0);
     return;
   }
   if (weights_ready) chain_wait();
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(128) mla_vup_mma_kernel(const uint16_t* __rest
       *reinterpret_cast<uint4*>(Bs + c * kStride + v * 8) = w;
     }
     __syncthreads();
-    tile_mma_64x128x128<true>(As, Bs, acc, warp, lane);
+    tile_mma_64x128x128(As, Bs, acc, warp, lane);
   }
 #pragma unroll
   for (int hf = 0; hf < 2; hf++) {
@@ -413,12 +419,24 @@ __global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(con
 
 bool mla_proj_mma_eligible(int Dh, int dC) { return Dh == kDh && dC % 128 == 0; }
 
+// W_UK [dC][H * 128] in 128 x 64 boxes; bf16 queries [rows][H * 128] in 64 x 64 boxes.
+static int32_t absorb_maps(const uint16_t* W_UK, const void* q_nope, int q_bf16, int rows, int H, int dC, CUtensorMap* tw, CUtensorMap* tq) {
+  if (!make_tmap_2d(tw, (void*)W_UK, (uint64_t)dC, (uint64_t)H * kDh, 64, 128) ||
+      (q_bf16 && !make_tmap_2d(tq, (void*)q_nope, (uint64_t)rows, (uint64_t)H * kDh, 64, 64))) {
+    set_error("tensor map for w_uk or the queries could not be encoded");
+    return RELUX_ERR_CUDA;
+  }
+  if (!q_bf16) *tq = *tw;
+  return RELUX_OK;
+}
+
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
-                              int rows, int H, int dC, int dHR) {
+                              int rows, int H, int dC, int dHR, int32_t* status) {
   dim3 grid(H, dC / 128, (rows + 63) / 64);
-  const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  if (int32_t rc = allow_smem(dev, mla_absorb_mma_kernel, smem)) return rc;
-  mla_absorb_mma_kernel<<<grid, 128, smem, dev->stream>>>(q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR);
+  CUtensorMap tw, tq;
+  if (int32_t rc = absorb_maps(W_UK, q_nope, q_bf16, rows, H, dC, &tw, &tq)) return rc;
+  if (int32_t rc = allow_smem(dev, mla_absorb_mma_kernel, kAbsorbSmem)) return rc;
+  mla_absorb_mma_kernel<<<grid, 128, kAbsorbSmem, dev->stream>>>(tw, tq, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, status);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(dev);
   return RELUX_OK;
@@ -428,10 +446,11 @@ int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rop
 int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows,
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained) {
   const unsigned blocks = (unsigned)ap.n_seqs + 1u + (unsigned)H * (unsigned)(dC / 128) * (unsigned)((rows + 63) / 64);
-  const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  if (int32_t rc = allow_smem(dev, mla_prep_kernel, smem)) return rc;
-  RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, dim3(blocks), dim3(128), smem, dev->stream, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H,
-                                dC, dHR, weights_ready ? 1 : 0, ap, pl));
+  CUtensorMap tw, tq;
+  if (int32_t rc = absorb_maps(W_UK, q_nope, q_bf16, rows, H, dC, &tw, &tq)) return rc;
+  if (int32_t rc = allow_smem(dev, mla_prep_kernel, kAbsorbSmem)) return rc;
+  RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, dim3(blocks), dim3(128), (size_t)kAbsorbSmem, dev->stream, tw, tq, q_nope, q_rope, q_bf16,
+                                q_abs, rows, H, dC, dHR, weights_ready ? 1 : 0, ap, pl));
   count_launch(dev);
   return RELUX_OK;
 }
