@@ -176,7 +176,8 @@ int32_t stage_release(Pool* p, int slot_index);
 struct SeqBatch {
   int32_t n_seqs = 0;
   const int32_t* d_seq_ids = nullptr;  // nullptr = identity
-  const int32_t* d_row_off = nullptr;  // nullptr = one row per sequence
+  const int32_t* d_row_off = nullptr;  // nullptr = rows_each rows per sequence
+  int32_t rows_each = 1;
   int32_t total_rows = 0;
   int32_t max_rows = 0;
   std::vector<int32_t> seq;  // host copy of ids
@@ -219,7 +220,8 @@ struct StepAppend {
   const void* ckv;
   const void* kr;
   int dtype;
-  const int32_t* d_row_off;   // device row offsets of the append batch (nullptr = one row per sequence)
+  const int32_t* d_row_off;   // device row offsets of the append batch (nullptr = rows_each rows per sequence)
+  int32_t rows_each = 1;
   bool weights_ready = false; // a launch before this one in the call has waited for everything older (launch_mla_prep)
 };
 int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, const void* d_qr,

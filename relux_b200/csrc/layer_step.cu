@@ -582,8 +582,7 @@ int32_t output_projection(Pool* p, const float* d_attn, int M, int K, const void
   return RELUX_OK;
 }
 
-// Validation shared by the two layer entry points; fills the batch with explicit rows per sequence (the append
-// kernels read "no row offsets" as one row per sequence).
+// Validation shared by the two layer entry points; fills the batch with S rows per sequence.
 int32_t layer_batch(Pool* p, int layer, int n_seqs, const int32_t* seq_ids, int S, const char* what, SeqBatch* sb) {
   const relux_pool_params& prm = p->prm;
   if (layer < 0 || layer >= prm.num_layers) {
@@ -594,8 +593,7 @@ int32_t layer_batch(Pool* p, int layer, int n_seqs, const int32_t* seq_ids, int 
     set_error("n_seqs=%d outside [1, max_seqs=%d]", n_seqs, prm.max_seqs);
     return RELUX_ERR_INVALID_ARG;
   }
-  const std::vector<int32_t> rows_per_seq((size_t)n_seqs, S);
-  int32_t rc = stage_batch(p, n_seqs, seq_ids, rows_per_seq.data(), 1, sb);
+  int32_t rc = stage_batch(p, n_seqs, seq_ids, nullptr, S, sb);
   if (rc) return rc;
   for (int i = 0; i < sb->n_seqs; i++) {   // the reference panics on overflow (kvcache.go:282-285, mla_cache.go:160-164)
     const int s = sb->seq[i];
@@ -718,7 +716,7 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   aa.w_uk = w.w_uk;
   aa.w_uv = w.w_uv;
   aa.mode = a->mode;
-  const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr, mma};   // one row per sequence
+  const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr, 1, mma};   // one row per sequence
   const bool o_bf16 = mma && mla_writes_bf16(p, sb, aa);   // the output projection's operand, rounded by the kernel that makes it
   rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, fused_append ? &step : nullptr)
             : launch_attn_reference_mla(p, sb, aa, (const float*)d_qc, (const float*)d_qr, d_attn);

@@ -286,6 +286,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     ap.len = p->d_len + (size_t)a.layer * prm.max_seqs;
     ap.seq_ids = sb.d_seq_ids;
     ap.row_off = step->d_row_off;
+    ap.rows_each = step->rows_each;
     ap.num_pages = prm.num_pages;
     ap.page_tokens = prm.page_tokens;
     ap.max_pages_per_seq = prm.max_pages_per_seq;

@@ -13,7 +13,8 @@ struct PrepAppend {
   int32_t table_stride;
   int32_t* len;                // this layer's [max_seqs]
   const int32_t* seq_ids;
-  const int32_t* row_off;      // nullptr = one new row per sequence
+  const int32_t* row_off;      // nullptr = rows_each new rows per sequence
+  int32_t rows_each;
   int32_t num_pages, page_tokens, max_pages_per_seq, n_seqs;
   int32_t* status;
   uint32_t* done;              // zero between launches; counts the blocks that have finished with the lengths
@@ -53,7 +54,7 @@ __device__ __forceinline__ void prep_arrive_and_advance(const PrepAppend& g, uin
   if (!s_last) return;
   for (int i = threadIdx.x; i < g.n_seqs; i += blockDim.x) {
     const int seq = g.seq_ids ? g.seq_ids[i] : i;
-    g.len[seq] += g.row_off ? g.row_off[i + 1] - g.row_off[i] : 1;
+    g.len[seq] += g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each;
   }
   if (threadIdx.x == 0) *g.done = 0u;
 }
@@ -61,8 +62,8 @@ __device__ __forceinline__ void prep_arrive_and_advance(const PrepAppend& g, uin
 // All new rows of sequence i (MLA row = [dC | dHR] fused; 16-byte stores).
 __device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i) {
   const int seq = g.seq_ids ? g.seq_ids[i] : i;
-  const int r0 = g.row_off ? g.row_off[i] : i;
-  const int nrows = g.row_off ? g.row_off[i + 1] - r0 : 1;
+  const int r0 = g.row_off ? g.row_off[i] : i * g.rows_each;
+  const int nrows = g.row_off ? g.row_off[i + 1] - r0 : g.rows_each;
   const int base_len = g.len[seq];
   const int row_elems = g.dC + g.dHR, vec_per_row = row_elems / 8, vc = g.dC / 8;
   for (int r = 0; r < nrows; r++) {
@@ -113,7 +114,7 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
     int seq = 0, pages = 0, tokens = 0;
     if (i < g.n_seqs) {
       seq = g.seq_ids ? g.seq_ids[i] : i;
-      tokens = g.len[seq] + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : 1) + pl.extra;
+      tokens = g.len[seq] + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
       pages = (tokens + g.page_tokens - 1) / g.page_tokens;
     }
     int tot_pages, tot_items;

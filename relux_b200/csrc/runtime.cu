@@ -99,7 +99,7 @@ int32_t stage_release(Pool* p, int slot_index) {
 }
 
 // Copies the call's sequence ids / rows-per-sequence to the device when they are not the
-// trivial (identity, uniform) case, through one pinned staging block guarded by an event.
+// trivial case (all sequences in order, the same number of rows each), through one pinned staging block guarded by an event.
 // upload = false: only the host half (the caller's kernel takes the sequences as arguments).
 int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32_t* n_rows, int32_t uniform_rows,
                     SeqBatch* out, bool upload) {
@@ -125,7 +125,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
       set_error("negative row count for sequence %d", s);
       return RELUX_ERR_INVALID_ARG;
     }
-    if (r != uniform_rows) uniform = false;
+    if (i > 0 && r != out->rows[0]) uniform = false;
     out->seq[i] = s;
     out->rows[i] = r;
     out->total_rows += r;
@@ -146,6 +146,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
   }
   out->d_seq_ids = nullptr;
   out->d_row_off = nullptr;
+  out->rows_each = out->rows[0];
   if (!upload || (!seq_ids && uniform)) return RELUX_OK;
   Device* dev = p->dev;
   int32_t* slot = nullptr;
@@ -1285,7 +1286,7 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   }
   // the host lengths count the new rows from here on: the attention call plans with them
   for (int i = 0; i < sb.n_seqs; i++) p->h_len[(size_t)kv->layer * prm.max_seqs + sb.seq[i]] += sb.rows[i];
-  StepAppend step{da, db, kv->dtype, sb.d_row_off};
+  StepAppend step{da, db, kv->dtype, sb.d_row_off, sb.rows_each};
   rc = do_attention(p, attn, kind, &step);
   if (rc) {   // nothing was launched for the append: take the rows back
     for (int i = 0; i < sb.n_seqs; i++) p->h_len[(size_t)kv->layer * prm.max_seqs + sb.seq[i]] -= sb.rows[i];
