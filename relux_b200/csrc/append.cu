@@ -53,7 +53,7 @@ __device__ __forceinline__ void advance_lengths_by_last_block(const AppendGeom& 
   if (!s_last) return;
   for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
     const int seq = g.seq_ids ? g.seq_ids[i] : i;
-    g.len[seq] += g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each;
+    g.len[seq] = load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each);
   }
   if (threadIdx.x == 0) *g.done = 0u;
 }
@@ -90,11 +90,13 @@ __device__ __forceinline__ void pages_of_rows(const AppendGeom& g, int seq, int 
 template <bool kF32>
 __global__ void mla_append_kernel(AppendGeom g, uint16_t* __restrict__ layer_base, const void* __restrict__ ckv,
                                   const void* __restrict__ kr, int dC, int dHR, int blocked, float* __restrict__ shadow) {
+  chain_release();
+  chain_wait();
   const int i = blockIdx.x;
   const int seq = g.seq_ids ? g.seq_ids[i] : i;
   const int r0 = g.row_off ? g.row_off[i] : i * g.rows_each;
   const int nrows = g.row_off ? g.row_off[i + 1] - r0 : g.rows_each;
-  const int base_len = g.len[seq];
+  const int base_len = load_chained(g.len + seq);
   const int row_elems = dC + dHR, vec_per_row = row_elems / 8, vc = dC / 8;
   constexpr int kN = kAhead;
   for (int r = blockIdx.y * kN; r < nrows; r += gridDim.y * kN) {
@@ -131,11 +133,13 @@ __global__ void mla_append_kernel(AppendGeom g, uint16_t* __restrict__ layer_bas
 template <bool kF32>
 __global__ void gqa_append_kernel(AppendGeom g, uint16_t* __restrict__ k_base, uint16_t* __restrict__ v_base,
                                   const void* __restrict__ ksrc, const void* __restrict__ vsrc, int Hkv, int D, int head_major) {
+  chain_release();
+  chain_wait();
   const int i = blockIdx.x;
   const int seq = g.seq_ids ? g.seq_ids[i] : i;
   const int r0 = g.row_off ? g.row_off[i] : i * g.rows_each;
   const int nrows = g.row_off ? g.row_off[i + 1] - r0 : g.rows_each;
-  const int base_len = g.len[seq];
+  const int base_len = load_chained(g.len + seq);
   const int vec_per_head = D / 8, vec_per_tok = Hkv * vec_per_head;
   constexpr int kN = kAhead;
   for (int r = blockIdx.y * kN; r < nrows; r += gridDim.y * kN) {
@@ -198,8 +202,9 @@ static int row_slices(const SeqBatch& sb) {
   return std::min(std::max((sb.max_rows + kAhead - 1) / kAhead, 1), std::max(1, kBlocks / sb.n_seqs));
 }
 
-static int32_t finish_append(Pool* p) {
-  RELUX_CUDA_TRY(cudaGetLastError());
+template <typename Kernel, typename... Args>
+static int32_t launch_append(Pool* p, Kernel kernel, dim3 grid, int threads, Args... args) {
+  RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, kernel, grid, dim3(threads), 0, p->dev->stream, args...));
   count_launch(p->dev);
   return RELUX_OK;
 }
@@ -210,11 +215,8 @@ int32_t launch_mla_append(Pool* p, const SeqBatch& sb, int layer, const void* ck
   dim3 grid(sb.n_seqs, row_slices(sb));
   int threads = 96;  // 72 vectors per 576-element row
   float* shadow = p->shadow_f32 ? p->shadow_f32 + (size_t)layer * p->layer_elems : nullptr;
-  if (dtype == RELUX_DTYPE_F32)
-    mla_append_kernel<true><<<grid, threads, 0, p->dev->stream>>>(g, base, ckv, kr, p->prm.mla_dc, p->prm.mla_dhr, p->mla_blocked, shadow);
-  else
-    mla_append_kernel<false><<<grid, threads, 0, p->dev->stream>>>(g, base, ckv, kr, p->prm.mla_dc, p->prm.mla_dhr, p->mla_blocked, shadow);
-  return finish_append(p);
+  return launch_append(p, dtype == RELUX_DTYPE_F32 ? mla_append_kernel<true> : mla_append_kernel<false>, grid, threads, g, base, ckv, kr,
+                       p->prm.mla_dc, p->prm.mla_dhr, (int)p->mla_blocked, shadow);
 }
 
 int32_t launch_gqa_append(Pool* p, const SeqBatch& sb, int layer, const void* k, const void* v, int dtype, int layout,
@@ -225,11 +227,8 @@ int32_t launch_gqa_append(Pool* p, const SeqBatch& sb, int layer, const void* k,
   dim3 grid(sb.n_seqs, row_slices(sb));
   int threads = 256;
   int hm = layout == RELUX_LAYOUT_HEAD_MAJOR;
-  if (dtype == RELUX_DTYPE_F32)
-    gqa_append_kernel<true><<<grid, threads, 0, p->dev->stream>>>(g, kb, vb, k, v, p->prm.gqa_num_kv_heads, p->prm.gqa_head_dim, hm);
-  else
-    gqa_append_kernel<false><<<grid, threads, 0, p->dev->stream>>>(g, kb, vb, k, v, p->prm.gqa_num_kv_heads, p->prm.gqa_head_dim, hm);
-  return finish_append(p);
+  return launch_append(p, dtype == RELUX_DTYPE_F32 ? gqa_append_kernel<true> : gqa_append_kernel<false>, grid, threads, g, kb, vb, k, v,
+                       p->prm.gqa_num_kv_heads, p->prm.gqa_head_dim, hm);
 }
 
 int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer0, int layers, const int32_t* new_len) {

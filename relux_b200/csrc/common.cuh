@@ -116,10 +116,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// Brings one box of a tiled tensor into L2 without touching shared memory (no mbarrier, fire and forget).
-__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* map, int32_t x, int32_t y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
 // 2-D tiled TMA store shared -> global of one box (bulk async-group completion).  The shared tile must have been made
 // visible to the async proxy (fence_proxy_async) by the threads that wrote it.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int32_t x, int32_t y, const void* smem_src) {
@@ -165,13 +161,9 @@ __device__ __forceinline__ void stamp_end(const TimeStamp& ts) {
   if (ts.slot) atomicMax(&ts.slot->end, global_ns());
 }
 
-// Untiled bulk copy global -> shared through the TMA unit (not the load/store unit): both addresses 16-byte aligned,
-// `bytes` a multiple of 16; completion is counted in bytes on `bar`.
-__device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(gsrc),
-               "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
+// A value that the launch before this one may have changed after this launch began (a length, a plan): read from L2, so that a
+// line which another block of this SM brought into L1 meanwhile is not taken for it.
+__device__ __forceinline__ int32_t load_chained(const int32_t* p) { return __ldcg(p); }
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -165,14 +165,14 @@ __device__ __forceinline__ Item item_of(const PrefillParams& prm, Cursor u) {
   it.hk = stream % prm.Hkv;
   it.bi = stream / prm.Hkv;
   it.seq = prm.seq_ids ? __ldg(prm.seq_ids + it.bi) : it.bi;
-  it.T = __ldg(prm.len + it.seq) + prm.extra;
+  it.T = load_chained(prm.len + it.seq) + prm.extra;
   // keys the PAIR needs: all T without the mask, else up to the position of its last real token
   const int last_tok = min(prm.S, (2 * it.pair + 2) * prm.bq) - 1;
   const int kmax = prm.causal ? (it.T - prm.S + last_tok + 1) : it.T;
   it.ntiles = max(1, (kmax + kTile - 1) / kTile);
   it.last_slot = (it.T + kPage - 1) / kPage - 1;   // last page slot of the sequence that holds a row
   it.base = 0;
-  if constexpr (kMla) it.base = __ldg(prm.seq_base + it.bi);
+  if constexpr (kMla) it.base = load_chained(prm.seq_base + it.bi);
   return it;
 }
 
@@ -244,14 +244,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int worker = blockIdx.x >> 1, n_workers = gridDim.x >> 1;
+  chain_release();
   if (worker >= prm.n_couples) return;   // both CTAs of the pair leave before any pair-wide step
 
   if ((smem_u32(smem) & 1023u) != 0) {   // the swizzled layouts need a 1024-byte aligned base (same in both CTAs of the pair)
+    chain_wait();
     if (threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     return;
   }
   if (threadIdx.x == 0) {
-    stamp_begin(prm.time);
     for (int s = 0; s < 2; s++) { mbar_init(&bars->q_full[s], 1); mbar_init(&bars->q_empty[s], 1); }
     for (int s = 0; s < kMaxDepth; s++) {
       mbar_init(&bars->k_full[s], 1);
@@ -281,6 +282,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  chain_wait();   // the set-up needs nothing of the launch before this one, whose tail hides it
+  if (threadIdx.x == 0) stamp_begin(prm.time);
 
   if (warp == kSoftmaxWarps) {
     // =============================== producer: TMA loads into this CTA's slots ===============================
@@ -702,8 +705,8 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   if (int32_t rcs = allow_smem(p->dev, prefill_sm100_kernel<false>, kSmemTotal)) return rcs;
   k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
-  prefill_sm100_kernel<false><<<grid, kThreads, kSmemTotal, st>>>(p->tmap_gqa, tq, tq, p->tmap_gqa, k);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<false>, grid, dim3(kThreads), (size_t)kSmemTotal, st,
+                                p->tmap_gqa, tq, tq, p->tmap_gqa, k));
   count_launch(p->dev);
   return RELUX_OK;
 }
@@ -793,8 +796,8 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   if (int32_t rcs = allow_smem(p->dev, prefill_sm100_kernel<true>, kSmemTotal)) return rcs;
   k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
-  prefill_sm100_kernel<true><<<grid, kThreads, kSmemTotal, st>>>(tx, tq, tqr, p->tmap_mla, k);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<true>, grid, dim3(kThreads), (size_t)kSmemTotal, st, tx,
+                                tq, tqr, p->tmap_mla, k));
   count_launch(p->dev);
   return RELUX_OK;
 }

@@ -342,7 +342,7 @@ __global__ void proj_finish_kernel(const FinishParams p) {
   if (sg.rope_dim > 0) {
     const int i = m / p.S, s = m % p.S;
     const int seq = p.seq_ids ? p.seq_ids[i] : i;
-    const int len0 = p.len[seq];
+    const int len0 = load_chained(p.len + seq);
     const int pos = (p.same_pos && len0 > 0) ? len0 : len0 + s;
     if (pos >= p.rope_positions) {
       set_status(p.status, RELUX_ERR_OVERFLOW);   // the reference panics: position >= maxSeqLen (rope.go:160-162)

@@ -100,9 +100,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const uint32_t rank = cluster_ctarank();
   const int worker = blockIdx.x >> 1;
   const int u0 = worker * prm.span, u1 = min(prm.units, u0 + prm.span);
+  chain_release();
   if (u0 >= u1) return;   // both CTAs of the pair leave before any pair-wide step
 
   if ((smem_u32(smem) & 1023u) != 0) {
+    chain_wait();
     if (threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     return;
   }
@@ -124,6 +126,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  chain_wait();
 
   if (warp == kEpiWarps) {
     // =============================== producer ===============================
@@ -141,13 +144,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         int lo = 0, hi = prm.n_seqs - 1;
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (__ldg(prm.seq_base + mid) <= tt * kTokTile) lo = mid;
+          if (load_chained(prm.seq_base + mid) <= tt * kTokTile) lo = mid;
           else hi = mid - 1;
         }
         const int seq = prm.seq_ids ? __ldg(prm.seq_ids + lo) : lo;
-        const int T = __ldg(prm.len + seq) + prm.extra;
+        const int T = load_chained(prm.len + seq) + prm.extra;
         const int last_slot = max(0, (T + kPage - 1) / kPage - 1);
-        const int tok0 = tt * kTokTile - __ldg(prm.seq_base + lo) + 128 * (int)rank;   // this CTA's first token in the sequence
+        const int tok0 = tt * kTokTile - load_chained(prm.seq_base + lo) + 128 * (int)rank;   // this CTA's first token in the sequence
         int64_t y[2];
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++) {
@@ -315,12 +318,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 __global__ void mla_expand_plan_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
                                        int32_t* __restrict__ seq_base) {
   __shared__ int32_t s_warp[32];
+  chain_release();
+  chain_wait();
   int base = 0;
   for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     int rows = 0;
     if (i < n_seqs) {
-      const int T = len[seq_ids ? seq_ids[i] : i] + extra;
+      const int T = load_chained(len + (seq_ids ? seq_ids[i] : i)) + extra;
       rows = (T + kTokTile - 1) / kTokTile * kTokTile;
     }
     int total;
@@ -391,8 +396,8 @@ int32_t launch_mla_expand_sm100(Pool* p, const SeqBatch& sb, int layer, int extr
     return RELUX_ERR_CUDA;
   }
   const int32_t* len = p->d_len + (size_t)layer * prm.max_seqs;
-  mla_expand_plan_kernel<<<1, 256, 0, st>>>(len, sb.d_seq_ids, sb.n_seqs, extra, seq_base);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  const bool chained = p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0;
+  RELUX_CUDA_TRY(launch_chained(chained, mla_expand_plan_kernel, dim3(1), dim3(256), 0, st, len, sb.d_seq_ids, sb.n_seqs, extra, seq_base));
   count_launch(p->dev);
   ExpandParams k{};
   k.table = p->d_table;
@@ -417,8 +422,8 @@ int32_t launch_mla_expand_sm100(Pool* p, const SeqBatch& sb, int layer, int extr
   k.status = p->d_status;
   if (int32_t rcs = allow_smem(p->dev, mla_expand_sm100_kernel, kSmemTotal)) return rcs;
   const int launched = (int)((units + k.span - 1) / k.span);
-  mla_expand_sm100_kernel<<<dim3(2 * launched), kThreads, kSmemTotal, st>>>(p->tmap_mla, t_uk, t_uv, t_out, k);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  RELUX_CUDA_TRY(launch_chained(chained, mla_expand_sm100_kernel, dim3(2 * launched), dim3(kThreads), (size_t)kSmemTotal, st, p->tmap_mla, t_uk, t_uv,
+                                t_out, k));
   count_launch(p->dev);
   return RELUX_OK;
 }

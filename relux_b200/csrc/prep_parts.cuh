@@ -54,7 +54,7 @@ __device__ __forceinline__ void prep_arrive_and_advance(const PrepAppend& g, uin
   if (!s_last) return;
   for (int i = threadIdx.x; i < g.n_seqs; i += blockDim.x) {
     const int seq = g.seq_ids ? g.seq_ids[i] : i;
-    g.len[seq] += g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each;
+    g.len[seq] = load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each);
   }
   if (threadIdx.x == 0) *g.done = 0u;
 }
@@ -64,7 +64,7 @@ __device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i) {
   const int seq = g.seq_ids ? g.seq_ids[i] : i;
   const int r0 = g.row_off ? g.row_off[i] : i * g.rows_each;
   const int nrows = g.row_off ? g.row_off[i + 1] - r0 : g.rows_each;
-  const int base_len = g.len[seq];
+  const int base_len = load_chained(g.len + seq);
   const int row_elems = g.dC + g.dHR, vec_per_row = row_elems / 8, vc = g.dC / 8;
   for (int r = 0; r < nrows; r++) {
     const int pos = base_len + r;
@@ -114,7 +114,7 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
     int seq = 0, pages = 0, tokens = 0;
     if (i < g.n_seqs) {
       seq = g.seq_ids ? g.seq_ids[i] : i;
-      tokens = g.len[seq] + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
+      tokens = load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
       pages = (tokens + g.page_tokens - 1) / g.page_tokens;
     }
     int tot_pages, tot_items;
