@@ -640,7 +640,7 @@ def run_gqa(args, w, world, rank, local, dist):
                   "what": "the first repeat of the timed region (boost clocks, before the power cap settles)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": alg_bytes * TRAFFIC_RATIO["gqa"],
-                     "peak_source": peak_src, "kernel": "gqa_decode_kernel", "kernel_ms": kernel_ms, "launches_timed": counted,
+                     "peak_source": peak_src, "kernel": "gqa_stream_kernel", "kernel_ms": kernel_ms, "launches_timed": counted,
                      "algorithmic_bytes_per_launch": alg_bytes, "frac_of_nominal_8TBs": achieved / 8000.0,
                      "kernel_ms_x_sm_mhz": (kernel_ms * sm_mhz) if sm_mhz else None},
         "e2e": {"value": acc_per_step * K * world / (ms_e2e * 1e-3), "unit": "tokens/s",
