@@ -27,7 +27,9 @@ def _ptr(a):
         return a
     if isinstance(a, DeviceBuffer):
         return a.ptr
-    return a.__array_interface__["data"][0]
+    if isinstance(a, np.ndarray):
+        return a.__array_interface__["data"][0]   # a.ctypes.data without building the ctypes helper, 1 us
+    return a.ctypes.data   # refuses NumPy's integer scalars: their own __array_interface__ is the scalar object's address
 
 
 def _mem(a):
