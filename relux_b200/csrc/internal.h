@@ -45,7 +45,7 @@ struct Device {
   bool copies_in_flight = false;
   std::mutex mu;
   int64_t launches = 0;
-  std::vector<std::pair<const void*, size_t>> smem_allowed;   // kernels that allow_smem has set, under mu
+  std::vector<std::pair<const void*, size_t>> smem_allowed;   // what allow_smem knows of the kernels' limits, under mu
   void* flush_buf = nullptr;
   size_t flush_bytes = 0;
 };
@@ -257,7 +257,7 @@ TimeStamp time_stamp_next(Pool* p, TimeRing& r);
 int32_t time_events_begin(Pool* p, TimeRing& r);
 int32_t time_events_end(Pool* p, TimeRing& r);
 
-// Dynamic shared memory above 48 KB has to be allowed once per kernel and device, not per launch.
+// Dynamic shared memory above 48 KB has to be allowed once per kernel and context, not per launch.
 int32_t allow_smem(Device* dev, const void* kernel, size_t bytes);
 template <typename... KArgs>
 inline int32_t allow_smem(Device* dev, void (*kernel)(KArgs...), size_t bytes) { return allow_smem(dev, (const void*)kernel, bytes); }

@@ -38,16 +38,30 @@ int32_t grow(Device* dev, GrowBuf& b, size_t bytes) {
   return RELUX_OK;
 }
 
+// The limit belongs to the kernel in the device's context, not to a handle: several handles of one GPU share it.  So it is
+// only ever raised, to the most that any handle has asked for.
 int32_t allow_smem(Device* dev, const void* kernel, size_t bytes) {
+  std::pair<const void*, size_t>* mine = nullptr;
   for (auto& e : dev->smem_allowed)
     if (e.first == kernel) {
       if (e.second >= bytes) return RELUX_OK;
-      RELUX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-      e.second = bytes;
-      return RELUX_OK;
+      mine = &e;
     }
-  RELUX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  dev->smem_allowed.emplace_back(kernel, bytes);
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, size_t>> most;   // under mu, like the attribute itself
+  std::lock_guard<std::mutex> lk(mu);
+  size_t want = bytes;
+  size_t* known = nullptr;
+  for (auto& e : most)
+    if (e.first == kernel) {
+      want = std::max(want, e.second);
+      known = &e.second;
+    }
+  RELUX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want));
+  if (known) *known = want;
+  else most.emplace_back(kernel, want);
+  if (mine) mine->second = want;
+  else dev->smem_allowed.emplace_back(kernel, want);
   return RELUX_OK;
 }
 
