@@ -238,6 +238,9 @@ int32_t do_sample(Pool* p, const relux_sample_args* a);
 int32_t do_matmul(Pool* p, const relux_matmul_args* a);
 int32_t do_import_mla(Pool* p, const relux_mla_import_args* a);
 int32_t do_selftest_wait(Pool* p, int32_t polls);
+// After a fused call that counted sb's rows and failed: the lengths before it, on the host and, whatever the call had queued
+// by then, on the device.  The error text of the call stays.
+void take_rows_back(Pool* p, const SeqBatch& sb, int layer);
 int32_t seq_set_len(Pool* p, int32_t layer, int32_t n_seqs, const int32_t* seq_ids, const int32_t* new_len);
 // Chunk bookkeeping of reference-compat pools (no-ops otherwise): an append of n rows at old_len, a length change.
 void note_append(Pool* p, int layer, int seq, int old_len, int n);

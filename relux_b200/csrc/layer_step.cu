@@ -720,7 +720,10 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   const bool o_bf16 = mma && mla_writes_bf16(p, sb, aa);   // the output projection's operand, rounded by the kernel that makes it
   rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, fused_append ? &step : nullptr)
             : launch_attn_reference_mla(p, sb, aa, (const float*)d_qc, (const float*)d_qr, d_attn);
-  if (rc) return rc;
+  if (rc) {
+    if (fused_append) take_rows_back(p, sb, a->layer);   // nobody appended them
+    return rc;
+  }
   // 5. output projection
   return output_projection(p, o_bf16 ? nullptr : d_attn, M, H * Dh, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
 }
@@ -814,7 +817,10 @@ int32_t do_gqa_layer(Pool* p, const relux_gqa_layer_args* a) {
   rc = fused_append ? launch_gqa_stream(p, sb, aa, d_q, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, &app)
        : fast       ? launch_gqa_decode_fast(p, sb, aa, d_q, d_attn)
                     : launch_attn_reference_gqa(p, sb, aa, (const float*)d_q, d_attn);
-  if (rc) return rc;
+  if (rc) {
+    if (fused_append && a->advance) take_rows_back(p, sb, a->layer);   // nobody appended them
+    return rc;
+  }
   return output_projection(p, o_bf16 ? nullptr : d_attn, M, H * hd, w.w_o, D, mma, sc.a_bf16, sc.part, sc.part_cap, a->out, a->out_mem);
 }
 

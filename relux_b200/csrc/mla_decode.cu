@@ -241,6 +241,11 @@ int32_t launch_generic(Pool* p, const MlaGenParams& k, int items, cudaStream_t s
   return RELUX_OK;
 }
 
+int32_t grow_partials(Pool* p, const SplitPlan& plan, int rows_total, int dC) {
+  const int32_t rc = grow(p->dev, p->part_o, (size_t)plan.num_items * rows_total * dC * sizeof(float));
+  return rc ? rc : grow(p->dev, p->part_ml, (size_t)plan.num_items * rows_total * 2 * sizeof(float));
+}
+
 }  // namespace
 
 bool mla_step_fusable(Pool* p, const relux_attn_args& a) {
@@ -279,6 +284,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   if (fused_prep) {
     // one launch: absorb + the step's append + the stream partition (the host lengths already count the new rows)
     rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, st, false);
+    if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
     if (rc) return rc;
     PrepAppend ap;
     ap.table = p->d_table;
@@ -342,10 +348,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   else
     rc = plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
   if (rc) return rc;
-  rc = grow(p->dev, p->part_o, (size_t)plan.num_items * rows_total * dC * sizeof(float));
-  if (rc) return rc;
-  rc = grow(p->dev, p->part_ml, (size_t)plan.num_items * rows_total * 2 * sizeof(float));
-  if (rc) return rc;
+  if ((rc = grow_partials(p, plan, rows_total, dC))) return rc;
   const bool fused_merge = proj_mma && dC <= 512;
   if (!fused_merge) {   // the unfused paths hand the merged latent output to the up-projection through this buffer
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));

@@ -1169,6 +1169,18 @@ API int32_t relux_gqa_decode(relux_pool_t h, const relux_attn_args* a) {
   return do_attention(p, a, RELUX_POOL_GQA);
 }
 
+// The caller holds the device guard.
+void relux::take_rows_back(Pool* p, const SeqBatch& sb, int layer) {
+  char why[512];
+  relux_cuda_last_error(why, sizeof(why));
+  int32_t* hl = &p->h_len[(size_t)layer * p->prm.max_seqs];
+  std::vector<int32_t> len(sb.n_seqs);
+  for (int i = 0; i < sb.n_seqs; i++) len[i] = hl[sb.seq[i]] -= sb.rows[i];
+  (void)cudaGetLastError();   // the call's own; a context that is lost refuses the launch as well
+  (void)launch_set_len(p, sb, layer, 1, len.data());
+  set_error("%s", why);
+}
+
 // The rows of a GQA decode (advance) or verify step ride in the attention launch: validated and staged exactly as do_append
 // does.  An attention call that is refused leaves the rows appended, as the two calls one after the other would.
 static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_attn_args* attn) {
@@ -1211,10 +1223,9 @@ static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_at
     for (int i = 0; i < sb.n_seqs; i++) hl[sb.seq[i]] += sb.rows[i];
   rc = do_attention(p, attn, RELUX_POOL_GQA, nullptr, &app);
   if (rc) {
-    if (adv)
-      for (int i = 0; i < sb.n_seqs; i++) hl[sb.seq[i]] -= sb.rows[i];
     char why[512];
     relux_cuda_last_error(why, sizeof(why));
+    if (adv) take_rows_back(p, sb, kv->layer);
     do_append(p, kv, RELUX_POOL_GQA);
     set_error("%s", why);
     return rc;
@@ -1302,8 +1313,8 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   for (int i = 0; i < sb.n_seqs; i++) p->h_len[(size_t)kv->layer * prm.max_seqs + sb.seq[i]] += sb.rows[i];
   StepAppend step{da, db, kv->dtype, sb.d_row_off, sb.rows_each};
   rc = do_attention(p, attn, kind, &step);
-  if (rc) {   // nothing was launched for the append: take the rows back
-    for (int i = 0; i < sb.n_seqs; i++) p->h_len[(size_t)kv->layer * prm.max_seqs + sb.seq[i]] -= sb.rows[i];
+  if (rc) {
+    take_rows_back(p, sb, kv->layer);
     return rc;
   }
   if ((rc = pipe_release(p, p->pipe_app_a, slot_a)) || (rc = pipe_release(p, p->pipe_app_b, slot_b))) return rc;
