@@ -18,6 +18,7 @@ void set_error(const char* fmt, ...) {
 }
 int32_t cuda_fail(cudaError_t e, const char* what) {
   set_error("CUDA error %d (%s) in %s", (int)e, cudaGetErrorString(e), what);
+  (void)cudaGetLastError();   // reported here: the check behind a later call's launch must not find it again
   if (e == cudaErrorMemoryAllocation) return RELUX_ERR_OUT_OF_MEMORY;
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return RELUX_ERR_NO_DEVICE;
   return RELUX_ERR_CUDA;
@@ -1176,7 +1177,6 @@ void relux::take_rows_back(Pool* p, const SeqBatch& sb, int layer) {
   int32_t* hl = &p->h_len[(size_t)layer * p->prm.max_seqs];
   std::vector<int32_t> len(sb.n_seqs);
   for (int i = 0; i < sb.n_seqs; i++) len[i] = hl[sb.seq[i]] -= sb.rows[i];
-  (void)cudaGetLastError();   // the call's own; a context that is lost refuses the launch as well
   (void)launch_set_len(p, sb, layer, 1, len.data());
   set_error("%s", why);
 }

@@ -40,7 +40,7 @@ def _world(dev, oracle, kind):
 
     ctx = rng.standard_normal((B * CTX,) + wa, dtype=np.float32), rng.standard_normal((B * CTX,) + wb, dtype=np.float32)
     pool.append(0, *ctx, B, n_new=np.full(B, CTX, np.int32))
-    if kind.endswith("step"):
+    if kind.endswith(("step", "verify")):
         more = dict(w_uk=up((DC, H * DH), 0.05), w_uv=up((DC, H * DH), 0.05)) if mla else {}
         out = dev.alloc(B * H * DH * 4, L.DTYPE_F32)
         bufs.append(out)
@@ -48,6 +48,10 @@ def _world(dev, oracle, kind):
 
         def step(i):
             off = lambda x, n: x.ptr + 2 * i * B * n   # noqa: E731
+            if kind == "gqa_verify":
+                pool.verify(0, B, off(q, H * DH), out, off(a, int(np.prod(wa))), off(b, int(np.prod(wb))), H, DH, 0.07, 1, q_dtype=L.DTYPE_BF16,
+                            kv_dtype=L.DTYPE_BF16)
+                return out.download((B, H, DH), np.float32)
             if mla:
                 more["q_rope"] = off(qr, H * DHR)
             pool.step(0, B, off(a, int(np.prod(wa))), off(b, int(np.prod(wb))), off(q, H * DH), out, H, DH, 0.07, q_dtype=L.DTYPE_BF16,
@@ -78,7 +82,7 @@ def _world(dev, oracle, kind):
     return pool, step, close
 
 
-@pytest.mark.parametrize("kind", ["mla_step", "gqa_step", "mla_layer", "gqa_layer"])
+@pytest.mark.parametrize("kind", ["mla_step", "gqa_step", "gqa_verify", "mla_layer", "gqa_layer"])
 def test_call_without_memory(oracle, kind):
     import relux_b200 as rb
     from relux_b200 import lib as L
@@ -93,7 +97,7 @@ def test_call_without_memory(oracle, kind):
         for b in held:
             b.free()
     # a GQA step keeps its rows when its attention is refused, as the two calls one after the other do; the other calls leave
-    # the cache as it was
+    # the lengths as they were.  No later call meets the error again.
     if kind == "gqa_step":
         step2(1)
     n = [other.seq_len(0, s) for s in range(B)]
@@ -101,7 +105,7 @@ def test_call_without_memory(oracle, kind):
     for i in (2, 3):   # the device's lengths: where these rows land, and what they see
         assert np.array_equal(step(i), step2(i))
     for s in (0, B - 1):
-        for x, y in zip(pool.read_rows(0, s, CTX - 2, n[s] + 4 - CTX), other.read_rows(0, s, CTX - 2, n[s] + 4 - CTX)):
+        for x, y in zip(pool.read_rows(0, s, CTX - 2, n[s] + 3 - CTX), other.read_rows(0, s, CTX - 2, n[s] + 3 - CTX)):
             assert np.array_equal(x, y)
     assert pool.status() == 0
     close(); close2()
