@@ -1,5 +1,5 @@
 """The tcgen05 projection GEMM at the sizes where its row blocks (16 to 256), its 128-column tiles and its ranges of K steps
-can go wrong, against float64 on the same bf16 operands."""
+can go wrong, and where its row blocks fill the SMs in turns, against float64 on the same bf16 operands."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 # (M, K, N): row blocks exactly full, one over, several; K below a step, ragged, many steps; N below a tile, ragged, a tile and
 # a bit; pieces that begin and end inside a tile (units that are no multiple of the SMs)
 CASES = [(1, 8, 8), (16, 64, 128), (17, 72, 136), (32, 4096, 64), (33, 1000, 264), (64, 2048, 4096), (65, 16384, 200), (128, 520, 1032),
-         (129, 4096, 384), (256, 192, 72), (257, 640, 520), (700, 328, 1160), (5, 4096, 19200)]
+         (129, 4096, 384), (256, 192, 72), (257, 640, 520), (700, 328, 1160), (5, 4096, 19200),
+         (200, 4096, 1024), (300, 4096, 6144), (520, 2048, 1160), (2049, 520, 264), (4700, 264, 1032), (12801, 328, 136), (19200, 136, 640),
+         (40001, 72, 72)]
 
 
 @pytest.mark.parametrize("M,K,N", CASES)
