@@ -16,10 +16,10 @@ template <bool kF32>
 __device__ __forceinline__ uint4 load8_as_bf16(const void* src, size_t elem_off) {
   if constexpr (kF32) {
     const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) + elem_off);
-    float4 a = s[0], b = s[1];
+    const float4 a = load_chained(s), b = load_chained(s + 1);
     return make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
   } else {
-    return *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(src) + elem_off);
+    return load_chained(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(src) + elem_off));
   }
 }
 
@@ -120,7 +120,8 @@ __global__ void mla_append_kernel(AppendGeom g, uint16_t* __restrict__ layer_bas
           const size_t so = (v < vc) ? (size_t)(r0 + r + q) * dC + (size_t)v * 8 : (size_t)(r0 + r + q) * dHR + (size_t)(v - vc) * 8;
 #pragma unroll
           for (int e = 0; e < 8; e++)
-            srow[e] = kF32 ? reinterpret_cast<const float*>(sp)[so + e] : f32_from_bf16_bits(reinterpret_cast<const uint16_t*>(sp)[so + e]);
+            srow[e] = kF32 ? load_chained(reinterpret_cast<const float*>(sp) + so + e)
+                           : f32_from_bf16_bits(load_chained(reinterpret_cast<const uint16_t*>(sp) + so + e));
         }
       }
     }

@@ -161,9 +161,12 @@ __device__ __forceinline__ void stamp_end(const TimeStamp& ts) {
   if (ts.slot) atomicMax(&ts.slot->end, global_ns());
 }
 
-// A value that the launch before this one may have changed after this launch began (a length, a plan): read from L2, so that a
-// line which another block of this SM brought into L1 meanwhile is not taken for it.
-__device__ __forceinline__ int32_t load_chained(const int32_t* p) { return __ldcg(p); }
+// What the launch before this one may have written after this launch began (lengths, plans, activations, partial results): read
+// from L2, so that a line which another block of this SM brought into L1 meanwhile is not taken for it.  Never by __ldg, nor
+// through a const __restrict__ pointer without this: such loads may become ld.global.nc, which wants data that nobody writes
+// while the kernel exists, and which the compiler may move ahead of chain_wait().
+template <typename T>
+__device__ __forceinline__ T load_chained(const T* p) { return __ldcg(p); }
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

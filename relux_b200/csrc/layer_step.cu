@@ -309,7 +309,7 @@ __global__ void cast_bf16_kernel(const float* __restrict__ src, uint16_t* __rest
   chain_release();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
-  const float4 a = reinterpret_cast<const float4*>(src)[2 * i], b = reinterpret_cast<const float4*>(src)[2 * i + 1];
+  const float4 a = load_chained(reinterpret_cast<const float4*>(src) + 2 * i), b = load_chained(reinterpret_cast<const float4*>(src) + 2 * i + 1);
   reinterpret_cast<uint4*>(dst)[i] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
 }
 
@@ -354,7 +354,7 @@ __global__ void proj_finish_kernel(const FinishParams p) {
   float v0 = 0.f, v1 = 0.f;
 #pragma unroll 4
   for (int s = 0; s < pieces; s++) {
-    const float2 t = *reinterpret_cast<const float2*>(p.part + ((size_t)s * p.M + m) * p.n_total + col);
+    const float2 t = load_chained(reinterpret_cast<const float2*>(p.part + ((size_t)s * p.M + m) * p.n_total + col));
     v0 += t.x;
     v1 += t.y;
   }
@@ -388,10 +388,10 @@ __global__ void sum_splits_kernel(const float* __restrict__ part, GemmRanges rg,
   if (i >= n4) return;
   const int col_tile = (int)(4 * i % (unsigned)N) / kTileN;
   const int pieces = rg.pieces(kTurns ? rg.tile_of(col_tile, (int)(4 * i / (unsigned)N)) : col_tile);
-  float4 acc = reinterpret_cast<const float4*>(part)[i];
+  float4 acc = load_chained(reinterpret_cast<const float4*>(part) + i);
 #pragma unroll 4
   for (int s = 1; s < pieces; s++) {
-    const float4 t = reinterpret_cast<const float4*>(part)[(size_t)s * n4 + i];
+    const float4 t = load_chained(reinterpret_cast<const float4*>(part) + (size_t)s * n4 + i);
     acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
   }
   reinterpret_cast<float4*>(out)[i] = acc;

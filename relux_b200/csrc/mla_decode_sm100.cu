@@ -113,8 +113,8 @@ __device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, Bars* b
 }
 
 __device__ __forceinline__ StreamItem load_item(const StreamItem* p) {
-  const int4 a = __ldg(reinterpret_cast<const int4*>(p));
-  const int4 b = __ldg(reinterpret_cast<const int4*>(p) + 1);
+  const int4 a = load_chained(reinterpret_cast<const int4*>(p));
+  const int4 b = load_chained(reinterpret_cast<const int4*>(p) + 1);
   StreamItem it;
   it.seq_index = a.x; it.seq = a.y; it.page_begin = a.z; it.page_end = a.w;
   it.tokens = b.x; it.pad[0] = it.pad[1] = it.pad[2] = 0;
@@ -166,7 +166,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   chain_wait();   // the ranges, the absorbed queries and the step's new rows come from the kernel before this one
-  int it0 = prm.worker_first[worker], it1 = prm.worker_first[worker + 1];
+  int it0 = load_chained(prm.worker_first + worker), it1 = load_chained(prm.worker_first + worker + 1);
   if (sq >= prm.S) it1 = it0;   // an empty range: nothing to do, and the CTA pair still meets at the end
   if (threadIdx.x == 0 && it0 < it1) stamp_begin(prm.time);
 
@@ -323,7 +323,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         __syncwarp();
       };
       auto tiles_of = [&](int it) -> int {
-        const int4 a = __ldg(reinterpret_cast<const int4*>(prm.items + it));
+        const int4 a = load_chained(reinterpret_cast<const int4*>(prm.items + it));
         return (a.w - a.z + 1) >> 1;
       };
       int ntiles = tiles_of(it0);

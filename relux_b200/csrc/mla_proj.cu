@@ -74,7 +74,7 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
       uint4 w = make_uint4(0, 0, 0, 0);
       if (r < rows_here) {
         const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_nope) + ((size_t)(r0 + r) * H + h) * kDh + (size_t)v * 8);
-        const float4 x = s[0], y = s[1];
+        const float4 x = load_chained(s), y = load_chained(s + 1);
         w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
       }
       *reinterpret_cast<uint4*>(As + (v >> 3) * 8192 + swz128(r, v & 7)) = w;
@@ -87,10 +87,10 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
       const int r = e / vecs, v = e % vecs;
       const size_t off = ((size_t)(r0 + r) * H + h) * dHR + (size_t)v * 8;
       uint4 w;
-      if (q_bf16) w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_rope) + off);
+      if (q_bf16) w = load_chained(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_rope) + off));
       else {
         const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_rope) + off);
-        const float4 x = s[0], y = s[1];
+        const float4 x = load_chained(s), y = load_chained(s + 1);
         w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
       }
       *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + dC + (size_t)v * 8) = w;
@@ -258,8 +258,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
   int c0_next = 0, c1_next = 0;
   if (r0 + warp < rows) {
     const int i = (r0 + warp) / S;
-    c0_next = __ldg(chunk_off + i);
-    c1_next = __ldg(chunk_off + i + 1);
+    c0_next = load_chained(chunk_off + i);
+    c1_next = load_chained(chunk_off + i + 1);
   }
   for (int row = warp; row < tile_rows; row += kRowStep) {
     const int r = r0 + row;
@@ -267,8 +267,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
     c0_next = c1_next = 0;
     if (row + kRowStep < tile_rows && r + kRowStep < rows) {
       const int i = (r + kRowStep) / S;
-      c0_next = __ldg(chunk_off + i);
-      c1_next = __ldg(chunk_off + i + 1);
+      c0_next = load_chained(chunk_off + i);
+      c1_next = load_chained(chunk_off + i + 1);
     }
     float4 acc[kChunks];
 #pragma unroll
@@ -280,7 +280,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
       const int n_items = c1 - c0;
       if (n_items <= 0) goto store_row;   // no partial to merge: a zero row
       float2 ml = make_float2(-INFINITY, 0.f);
-      if (lane < n_items) ml = __ldg(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
+      if (lane < n_items) ml = load_chained(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
       float4 x[kItems][kChunks];
       const int ng0 = min(32, n_items);
 #pragma unroll
@@ -290,16 +290,16 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
         const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(c0 + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
         for (int k = 0; k < kChunks; k++)
-          if (k < nk) x[u][k] = (u < ng0) ? __ldg(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < nk) x[u][k] = (u < ng0) ? load_chained(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       // global maximum and normaliser over all items of the sequence
       float M = ml.x;
-      for (int c = c0 + 32 + lane; c < c1; c += 32) M = fmaxf(M, __ldg(part_ml + ((size_t)c * rows_total + prow) * 2));
+      for (int c = c0 + 32 + lane; c < c1; c += 32) M = fmaxf(M, load_chained(part_ml + ((size_t)c * rows_total + prow) * 2));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
       float L = (ml.x != -INFINITY) ? ml.y * exp2f(ml.x - M) : 0.f;
       for (int c = c0 + 32 + lane; c < c1; c += 32) {
-        const float2 t = __ldg(reinterpret_cast<const float2*>(part_ml + ((size_t)c * rows_total + prow) * 2));
+        const float2 t = load_chained(reinterpret_cast<const float2*>(part_ml + ((size_t)c * rows_total + prow) * 2));
         if (t.x != -INFINITY) L += t.y * exp2f(t.x - M);
       }
 #pragma unroll
@@ -311,7 +311,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
         if (cb == c0) {
           w_mine = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M) * inv;
         } else if (cb + lane < c1) {
-          const float m = __ldg(part_ml + ((size_t)(cb + lane) * rows_total + prow) * 2);
+          const float m = load_chained(part_ml + ((size_t)(cb + lane) * rows_total + prow) * 2);
           w_mine = (m == -INFINITY) ? 0.f : exp2f(m - M) * inv;
         }
         const int ng = min(32, c1 - cb);
@@ -322,7 +322,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
               const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(cb + j + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
               for (int k = 0; k < kChunks; k++)
-                if (k < nk) x[u][k] = (j + u < ng) ? __ldg(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k < nk) x[u][k] = (j + u < ng) ? load_chained(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
 #pragma unroll

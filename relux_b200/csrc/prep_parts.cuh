@@ -35,10 +35,10 @@ struct PrepPlan {
 __device__ __forceinline__ uint4 prep_load8(const void* src, size_t elem_off, bool f32) {
   if (f32) {
     const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) + elem_off);
-    const float4 a = s[0], b = s[1];
+    const float4 a = load_chained(s), b = load_chained(s + 1);
     return make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
   }
-  return *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(src) + elem_off);
+  return load_chained(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(src) + elem_off));
 }
 
 // Every block that reads the lengths arrives here once it is done with them; the last one to arrive advances all
