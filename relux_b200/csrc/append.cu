@@ -126,6 +126,7 @@ __global__ void mla_append_kernel(AppendGeom g, uint16_t* __restrict__ layer_bas
       }
     }
   }
+  fence_chained_writes();
   advance_lengths_by_last_block(g);
 }
 
@@ -164,6 +165,7 @@ __global__ void gqa_append_kernel(AppendGeom g, uint16_t* __restrict__ k_base, u
       }
     }
   }
+  fence_chained_writes();
   advance_lengths_by_last_block(g);
 }
 

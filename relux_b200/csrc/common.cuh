@@ -161,6 +161,12 @@ __device__ __forceinline__ void stamp_end(const TimeStamp& ts) {
   if (ts.slot) atomicMax(&ts.slot->end, global_ns());
 }
 
+// By every thread that wrote with ordinary stores what a later launch of the chain reads by TMA (cached rows, bf16 activations,
+// queries), behind its last store: TMA reads through the async proxy, and it is nowhere stated that chain_wait() alone orders that
+// proxy after another launch's generic writes, as the end of a plain launch does.  On this side because nothing is in flight here; behind the readers' wait the same fence waited for their weights (67.0 -> 69.4 us of
+// a GQA layer step).
+__device__ __forceinline__ void fence_chained_writes() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
 // What the launch before this one may have written after this launch began (lengths, plans, activations, partial results): read
 // from L2, so that a line which another block of this SM brought into L1 meanwhile is not taken for it.  Never by __ldg, nor
 // through a const __restrict__ pointer without this: such loads may become ld.global.nc, which wants data that nobody writes

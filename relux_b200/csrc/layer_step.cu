@@ -311,6 +311,7 @@ __global__ void cast_bf16_kernel(const float* __restrict__ src, uint16_t* __rest
   if (i >= n8) return;
   const float4 a = load_chained(reinterpret_cast<const float4*>(src) + 2 * i), b = load_chained(reinterpret_cast<const float4*>(src) + 2 * i + 1);
   reinterpret_cast<uint4*>(dst)[i] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+  fence_chained_writes();
 }
 
 // Sums the K splits of the projection result (fixed order, so the result does not depend on scheduling), applies
@@ -375,8 +376,12 @@ __global__ void proj_finish_kernel(const FinishParams p) {
       v1 = r1;
     }
   }
-  if (sg.bf16) reinterpret_cast<uint32_t*>(sg.dst)[((size_t)m * sg.n + c) >> 1] = pack_bf16x2(v0, v1);
-  else *reinterpret_cast<float2*>(reinterpret_cast<float*>(sg.dst) + (size_t)m * sg.n + c) = make_float2(v0, v1);
+  if (sg.bf16) {
+    reinterpret_cast<uint32_t*>(sg.dst)[((size_t)m * sg.n + c) >> 1] = pack_bf16x2(v0, v1);
+    fence_chained_writes();
+  } else {
+    *reinterpret_cast<float2*>(reinterpret_cast<float*>(sg.dst) + (size_t)m * sg.n + c) = make_float2(v0, v1);
+  }
 }
 
 // out [M][N] = sum over the pieces of one weight's tiles; a thread sums four adjacent columns.

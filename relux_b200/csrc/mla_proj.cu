@@ -136,6 +136,7 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
     const int r = e / 16, v = e % 16;
     *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + c0 + v * 8) = *reinterpret_cast<const uint4*>(Os + r * kStride + v * 8);
   }
+  fence_chained_writes();
 }
 
 // grid (H, dC/128, ceil(rows/64)), 128 threads.
@@ -413,6 +414,7 @@ __global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(con
       else *reinterpret_cast<float2*>(reinterpret_cast<float*>(out) + off + nt * 8) = make_float2(x, y);
     }
   }
+  if (out_bf16) fence_chained_writes();   // a projection's operand
 }
 
 }  // namespace

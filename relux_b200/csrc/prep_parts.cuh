@@ -81,6 +81,7 @@ __device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i) {
       *reinterpret_cast<uint4*>(page + mla_page_off(g.blocked != 0, g.page_tokens, row_elems, pos % g.page_tokens, v * 8)) = w;
     }
   }
+  fence_chained_writes();
 }
 
 // Exclusive prefix sum over a block of up to 1024 threads; *total receives the block's sum.
