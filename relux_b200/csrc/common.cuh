@@ -130,8 +130,8 @@ __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bu
 
 // Programmatic dependent launch.  A kernel launched with the stream-serialization attribute may be scheduled while the
 // kernel before it in the stream still runs; chain_wait() returns once that kernel has completed and its writes are
-// visible, so it stands before the first access to global memory.  chain_release() lets the kernel after this one be
-// scheduled (it blocks in its own chain_wait() until this grid is complete).  Both are no-ops in a plain launch.
+// visible.  chain_release() lets the kernel after this one be scheduled.  Both are no-ops in a plain launch.  The rules of a
+// chain (who writes these launches, who may read before the wait) stand at launch_chained in internal.h.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -163,8 +163,8 @@ __device__ __forceinline__ void stamp_end(const TimeStamp& ts) {
 
 // By every thread that wrote with ordinary stores what a later launch of the chain reads by TMA (cached rows, bf16 activations,
 // queries), behind its last store: TMA reads through the async proxy, and it is nowhere stated that chain_wait() alone orders that
-// proxy after another launch's generic writes, as the end of a plain launch does.  On this side because nothing is in flight here; behind the readers' wait the same fence waited for their weights (67.0 -> 69.4 us of
-// a GQA layer step).
+// proxy after another launch's generic writes, as the end of a plain launch does.  On this side because nothing is in flight
+// here; behind the readers' wait the same fence waited for their weights (67.0 -> 69.4 us of a GQA layer step).
 __device__ __forceinline__ void fence_chained_writes() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 // What the launch before this one may have written after this launch began (lengths, plans, activations, partial results): read

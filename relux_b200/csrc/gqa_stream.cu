@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
   for (int e = threadIdx.x; e < kQBufs * SM::kQBytes / 4; e += kThreads) reinterpret_cast<uint32_t*>(smem + SM::kQ)[e] = 0u;   // rows >= R stay zero
   __syncthreads();
   chain_release();
+  if (c.seqs) chain_wait();   // the list is a copy that was queued just before this launch
   Piece p = first_piece();
 
   if (warp == kConsumers + kFinishers) {

@@ -268,8 +268,22 @@ inline int32_t allow_smem(Device* dev, void (*kernel)(KArgs...), size_t bytes) {
 inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 
 // Launches `kern`; with `chained` the launch carries the programmatic stream-serialization attribute, so the grid may be
-// scheduled while the kernel before it in the stream still runs.  Such a kernel calls chain_wait() (common.cuh) before
-// its first access to global memory, which is what keeps the stream's order of results.
+// scheduled as soon as every block of the kernel before it in the stream has called chain_release() (common.cuh) or ended,
+// whatever that kernel itself still waits for.  What keeps the stream's order of results:
+//   1. Every such kernel calls chain_wait() in the threads that write, and in those that read what a launch of the chain
+//      writes, before they do.  A kernel is complete only when all its threads are, so "the launch before me is complete" holds
+//      back to the first launch of the chain.
+//   2. What a launch of the chain writes is read by load_chained() or plain loads of pointers that are not const __restrict__, and
+//      by TMA only where the writer has called fence_chained_writes().
+//   3. Before its wait a kernel may read what was complete before the HEAD of its chain began.  A head is a plain launch, a launch
+//      behind a copy or an event, or one whose blocks all wait before they release: cast_bf16_kernel, and mla_prep_kernel
+//      without weights_ready.  Those who read early, and why they may:
+//        - page tables, everywhere: the host calls that change them wait for the stream and for their copy;
+//        - skinny_gemm_sm100_kernel, the weights: the first launch of a layer step or matmul is cast_bf16_kernel, the
+//          second GEMM of a layer follows it, a plain absorb launch, or a cast of its own;
+//        - mla_prep_kernel with weights_ready, W_UK: only behind the projections of the same call (do_mla_layer);
+//        - mla_merge_vup_mma_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.
+//      A new early read names its head here; a new launch in front of one of these keeps a head between.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(bool chained, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                   Args&&... args) {
