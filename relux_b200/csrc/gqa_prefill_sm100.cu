@@ -707,6 +707,7 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<false>, grid, dim3(kThreads), (size_t)kSmemTotal, st,
                                 p->tmap_gqa, tq, tq, p->tmap_gqa, k));
+  time_stamp_done(p->attn_times, k.time);
   count_launch(p->dev);
   return RELUX_OK;
 }
@@ -798,6 +799,7 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<true>, grid, dim3(kThreads), (size_t)kSmemTotal, st, tx,
                                 tq, tqr, p->tmap_mla, k));
+  time_stamp_done(p->attn_times, k.time);
   count_launch(p->dev);
   return RELUX_OK;
 }

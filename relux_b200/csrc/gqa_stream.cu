@@ -475,6 +475,7 @@ int32_t launch(Pool* p, const GqaStreamCommon& c, const GqaSeq* seqs, int worker
   if (int32_t rc = allow_smem(p->dev, gqa_stream_kernel<MT, RS, N>, SM::kTotal)) return rc;
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, gqa_stream_kernel<MT, RS, N>, dim3(workers), dim3(kThreads),
                                 (size_t)SM::kTotal, p->dev->stream, p->tmap_gqa, prm));
+  time_stamp_done(p->attn_times, c.time);
   count_launch(p->dev);
   return RELUX_OK;
 }

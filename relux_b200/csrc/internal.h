@@ -257,6 +257,7 @@ bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint
                   uint32_t box_outer);
 
 TimeStamp time_stamp_next(Pool* p, TimeRing& r);
+void time_stamp_done(TimeRing& r, const TimeStamp& ts);
 int32_t time_events_begin(Pool* p, TimeRing& r);
 int32_t time_events_end(Pool* p, TimeRing& r);
 

@@ -581,8 +581,10 @@ int32_t project_and_finish(Pool* p, const SeqBatch& sb, int layer, const float* 
   GemmRanges ranges{};
   if (mma) {
     int32_t rc = launch_cast(p, dx, a_bf16, (size_t)M * K);
-    if (!rc) rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &ranges, time_stamp_next(p, p->proj_times));
+    const TimeStamp time = time_stamp_next(p, p->proj_times);
+    if (!rc) rc = launch_skinny_gemm(p, a_bf16, M, K, ws, nw, part, part_cap, &ranges, time);
     if (rc) return rc;
+    time_stamp_done(p->proj_times, time);
   } else {
     int32_t rc = time_events_begin(p, p->proj_times);
     if (rc) return rc;

@@ -570,6 +570,7 @@ int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_ar
   dim3 grid(2 * plan.num_workers * sx, a.q_tokens / sx);
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, mla_decode_sm100_kernel, grid, dim3(192), (size_t)kSmemTotal,
                                 p->dev->stream, p->tmap_mla, tq, k));
+  time_stamp_done(p->attn_times, time);
   return RELUX_OK;
 }
 

@@ -67,7 +67,8 @@ int32_t allow_smem(Device* dev, const void* kernel, size_t bytes) {
 }
 
 // The slot of the next timed call, for its kernel to stamp; null when the slots could not be allocated (the call is then
-// not timed).
+// not timed).  The call counts once time_stamp_done says that its kernel is queued: that kernel clears the slot after it, so a call
+// that fails in between must leave its own slot, cleared already, to the next one.
 TimeStamp time_stamp_next(Pool* p, TimeRing& r) {
   if (!r.slots) {
     if (cudaMalloc((void**)&r.slots, sizeof(TimeSlot) * TimeRing::kSlots) != cudaSuccess) {
@@ -77,9 +78,10 @@ TimeStamp time_stamp_next(Pool* p, TimeRing& r) {
     }
     cudaMemsetAsync(r.slots, 0, sizeof(TimeSlot) * TimeRing::kSlots, p->dev->stream);
   }
-  const uint64_t c = r.calls++;
-  r.stamped[c % TimeRing::kCalls] = 1;
-  return TimeStamp{r.slots + c % TimeRing::kSlots, r.slots + (c + 1) % TimeRing::kSlots};
+  return TimeStamp{r.slots + r.calls % TimeRing::kSlots, r.slots + (r.calls + 1) % TimeRing::kSlots};
+}
+void time_stamp_done(TimeRing& r, const TimeStamp& ts) {
+  if (ts.slot) r.stamped[r.calls++ % TimeRing::kCalls] = 1;
 }
 static int32_t time_event(Pool* p, TimeRing& r, int which) {
   cudaEvent_t& e = r.ev[r.calls % TimeRing::kCalls][which];
@@ -1405,7 +1407,7 @@ API int32_t relux_pool_selftest_wait(relux_pool_t h, int32_t polls) {
   return do_selftest_wait(p, polls);
 }
 
-// Times of the last n calls of a ring, oldest first; calls whose launch failed are skipped.
+// Times of the last n calls of a ring, oldest first; calls that recorded none are skipped.
 static int32_t ring_list(Pool* p, TimeRing& r, int32_t last_n, float* out, int32_t* counted) {
   const uint64_t n = std::min<uint64_t>(std::min<uint64_t>((uint64_t)last_n, r.calls), TimeRing::kCalls);
   std::vector<TimeSlot> slots;

@@ -1117,6 +1117,7 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     RELUX_CUDA_TRY(cudaLaunchKernelEx(&cfg, spec_accept_kernel, prm));
+    time_stamp_done(p->attn_times, prm.time);
   }
   count_launch(dev);
   RELUX_CUDA_TRY(cudaStreamSynchronize(dev->stream));
