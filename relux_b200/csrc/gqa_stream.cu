@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
   uint64_t* state_full = q_full + kQBufs;           // the consumers' states of a piece are in shared memory
   uint64_t* state_empty = state_full + 1;      // and have been read
   uint64_t* merge_go = state_empty + 2;        // the finishers know which rows are to be merged here
-  uint32_t* merge_flags = (uint32_t*)(state_empty + 3);   // [kFinishers]
+  uint32_t* merge_flags = (uint32_t*)(state_empty + 3);   // [kFinishers], and the warps that are done with the merge
   uint64_t* rows_done = state_empty + 1;       // the new rows of this CTA's pieces are in their pages
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     mbar_init(state_empty, kFinishers);
     mbar_init(rows_done, kFinishers);
     mbar_init(merge_go, kFinishers);
+    merge_flags[kFinishers] = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap);
   }
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     if (merge_flags[r % kFinishers] >> k & 1u) merge_row(k ? p_last : p_first, r);
   }
   if (c.out_bf16) fence_chained_writes();   // a projection's operand
-  if (warp == kConsumers && lane == 0) stamp_end(c.time);
+  if (lane == 0 && atomicAdd(&merge_flags[kFinishers], 1u) == kConsumers + kFinishers - 1) stamp_end(c.time);   // the last of them
 }
 
 
