@@ -28,7 +28,6 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained);
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
                               int rows, int H, int dC, int dHR, int32_t* status);
-int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W_UV, float* out, int rows, int H, int dC);
 int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
                                  void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
 
@@ -254,7 +253,7 @@ bool mla_step_fusable(Pool* p, const relux_attn_args& a) {
          mla_proj_mma_eligible(a.head_dim, prm.mla_dc);
 }
 
-// The merge + up-projection kernel rounds its own result; the unfused up-projections and the prefill kernel write float32.
+// The merge + up-projection kernel rounds its own result; the unfused up-projection and the prefill kernel write float32.
 bool mla_writes_bf16(const Pool* p, const SeqBatch& sb, const relux_attn_args& a) {
   return mla_proj_mma_eligible(a.head_dim, p->prm.mla_dc) && p->prm.mla_dc <= 512 && !mla_prefill_eligible(p, sb, a);
 }
@@ -349,8 +348,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     rc = plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
   if (rc) return rc;
   if ((rc = grow_partials(p, plan, rows_total, dC))) return rc;
-  const bool fused_merge = proj_mma && dC <= 512;
-  if (!fused_merge) {   // the unfused paths hand the merged latent output to the up-projection through this buffer
+  if (!proj_mma) {   // the unfused path hands the merged latent output to the up-projection through this buffer
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));
     if (rc) return rc;
   }
@@ -393,19 +391,13 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     if (timed && (rc = time_events_end(p, p->attn_times))) return rc;
   }
   count_launch(p->dev);
-  if (fused_merge) {
+  if (proj_mma) {
     // split-KV merge fused into the up-projection: the merged latent output never touches HBM
     rc = launch_mla_merge_vup_mma(p->dev, (const float*)p->part_o.p, (const float*)p->part_ml.p, plan.chunk_off, (const uint16_t*)a.w_uv,
                                   d_out, out_bf16, rows, S, H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
     if (rc) return rc;
-  } else if (proj_mma) {
-    // merged latent output goes to the up-projection as bf16 (tensor-core operand)
-    rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, nullptr, (uint16_t*)p->o_lat.p);
-    if (rc) return rc;
-    rc = launch_mla_vup_mma(p->dev, (const uint16_t*)p->o_lat.p, (const uint16_t*)a.w_uv, (float*)d_out, rows, H, dC);
-    if (rc) return rc;
   } else {
-    rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, (float*)p->o_lat.p, nullptr);
+    rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, (float*)p->o_lat.p);
     if (rc) return rc;
     dim3 grid(H, (rows + 7) / 8);
     size_t smem = (size_t)8 * dC * 4;

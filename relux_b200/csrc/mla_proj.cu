@@ -20,24 +20,6 @@ constexpr int kDh = 128;
 constexpr int kStride = kDh + 8;  // bf16 elements per shared-memory row (272 B: conflict-free ldmatrix)
 constexpr int kMaxChunks = 4;     // the fused merge + up-projection keeps at most 4 x 128 latent columns in shared memory
 
-// 64 x 128 A tile (rows x k) and 128 x 128 B tile [k][n] (n contiguous -> ldmatrix.trans); warp w owns rows 16w..16w+15 and all
-// 128 columns.
-__device__ __forceinline__ void tile_mma_64x128x128(const uint16_t* As, const uint16_t* Bs, float (&acc)[16][4], int warp, int lane) {
-#pragma unroll
-  for (int ks = 0; ks < 8; ks++) {
-    uint32_t a[4];
-    const int m = lane >> 3;
-    ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + (warp * 16 + (m & 1) * 8 + (lane & 7)) * kStride + ks * 16 + (m >> 1) * 8));
-#pragma unroll
-    for (int n2 = 0; n2 < 8; n2++) {
-      uint32_t b0, b1, b2, b3;
-      ldmatrix_x4_trans(b0, b1, b2, b3, smem_u32(Bs + (ks * 16 + (m & 1) * 8 + (lane & 7)) * kStride + n2 * 16 + (m >> 1) * 8));
-      mma_bf16_16816(acc[2 * n2], a, b0, b1);
-      mma_bf16_16816(acc[2 * n2 + 1], a, b2, b3);
-    }
-  }
-}
-
 // 64 rows x 128 latent columns of the absorb for one head, by 128 threads.  W_UK's tile [128 c][128 d] and (bf16) the query
 // tile [64 rows][128 d] come as four TMA boxes from one thread: as 3072 cp.async of 16 bytes they took 2.2 us to issue.  Both
 // lie as two 64-column blocks with the 128-byte swizzle.  Up to 32 rows, the warps share the row groups that hold a row.
@@ -173,46 +155,6 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ C
   if (e < ap.n_seqs) prep_append_seq(ap, e);
   else prep_build_stream(ap, pl);
   prep_arrive_and_advance(ap, (uint32_t)ap.n_seqs + 1u);
-}
-
-// grid (H, ceil(rows/64)), 128 threads.  o_lat bf16 [rows][H][dC]; out f32 [rows][H][128].
-__global__ void __launch_bounds__(128) mla_vup_mma_kernel(const uint16_t* __restrict__ o_lat, const uint16_t* __restrict__ W_UV,
-                                                          float* __restrict__ out, int rows, int H, int dC) {
-  extern __shared__ __align__(16) uint16_t sm[];
-  uint16_t* As = sm;                  // [64][kStride]   rows x 128 latent columns of this k chunk
-  uint16_t* Bs = sm + 64 * kStride;   // [128][kStride]  rows = latent index c of the chunk, cols = d
-  const int h = blockIdx.x, r0 = blockIdx.y * 64;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float acc[16][4];
-#pragma unroll
-  for (int i = 0; i < 16; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-  for (int kc = 0; kc < dC; kc += 128) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < 64 * 16; e += blockDim.x) {
-      const int r = e / 16, v = e % 16;
-      uint4 w = make_uint4(0, 0, 0, 0);
-      if (r0 + r < rows) w = *reinterpret_cast<const uint4*>(o_lat + ((size_t)(r0 + r) * H + h) * dC + kc + (size_t)v * 8);
-      *reinterpret_cast<uint4*>(As + r * kStride + v * 8) = w;
-    }
-    for (int e = threadIdx.x; e < 128 * 16; e += blockDim.x) {
-      const int c = e / 16, v = e % 16;
-      const uint4 w = *reinterpret_cast<const uint4*>(W_UV + (size_t)(kc + c) * H * kDh + (size_t)h * kDh + (size_t)v * 8);
-      *reinterpret_cast<uint4*>(Bs + c * kStride + v * 8) = w;
-    }
-    __syncthreads();
-    tile_mma_64x128x128(As, Bs, acc, warp, lane);
-  }
-#pragma unroll
-  for (int hf = 0; hf < 2; hf++) {
-    const int r = r0 + warp * 16 + hf * 8 + (lane >> 2);
-    if (r >= rows) continue;
-    float* dst = out + ((size_t)r * H + h) * kDh;
-#pragma unroll
-    for (int nt = 0; nt < 16; nt++)
-      *reinterpret_cast<float2*>(dst + nt * 8 + 2 * (lane & 3)) = make_float2(acc[nt][hf * 2], acc[nt][hf * 2 + 1]);
-  }
 }
 
 // 16 rows x 16 * nj columns of a warp, over one 128-wide k chunk: A rows at As (kStride), B [128 k][128 n] at Bs as two 64-column
@@ -453,16 +395,6 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
   if (int32_t rc = allow_smem(dev, mla_prep_kernel, kAbsorbSmem)) return rc;
   RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, dim3(blocks), dim3(128), (size_t)kAbsorbSmem, dev->stream, tw, tq, q_nope, q_rope, q_bf16,
                                 q_abs, rows, H, dC, dHR, weights_ready ? 1 : 0, ap, pl));
-  count_launch(dev);
-  return RELUX_OK;
-}
-
-int32_t launch_mla_vup_mma(Device* dev, const uint16_t* o_lat, const uint16_t* W_UV, float* out, int rows, int H, int dC) {
-  dim3 grid(H, (rows + 63) / 64);
-  const size_t smem = (size_t)(64 + 128) * kStride * 2;
-  if (int32_t rc = allow_smem(dev, mla_vup_mma_kernel, smem)) return rc;
-  mla_vup_mma_kernel<<<grid, 128, smem, dev->stream>>>(o_lat, W_UV, out, rows, H, dC);
-  RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(dev);
   return RELUX_OK;
 }

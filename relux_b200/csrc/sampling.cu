@@ -500,7 +500,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
     int32_t* k_idx = l_idx + 4 * kCandCap;
     float* k_p = l_val + 6 * kCandCap;
     int32_t* k_ord = l_idx + 6 * kCandCap;
-    __shared__ int s_n, s_cut, s_tok;
+    __shared__ int s_n, s_cut;
     __shared__ float s_thr, s_scale;
     // gather the lists of all CTAs (rank order)
     int n_c = 0;
@@ -1160,7 +1160,6 @@ int32_t do_spec_accept(Pool* p, const relux_spec_accept_args* a) {
         set_error("spec_accept: draft token %d outside the vocabulary of %d", a->draft_tokens[i], V);
         return RELUX_ERR_INVALID_ARG;
       }
-  Device* dev = p->dev;
   SelParams prm{};
   const void* d = nullptr;
   int32_t rc;
