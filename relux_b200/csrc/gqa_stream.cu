@@ -462,8 +462,8 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     const int k = e >= c.R, r = k ? e - c.R : e;
     if (merge_flags[r % kFinishers] >> k & 1u) merge_row(k ? p_last : p_first, r);
   }
-  if (c.out_bf16) fence_chained_writes();   // a projection's operand
   if (lane == 0 && atomicAdd(&merge_flags[kFinishers], 1u) == kConsumers + kFinishers - 1) stamp_end(c.time);   // the last of them
+  if (c.out_bf16) fence_chained_writes();   // a projection's operand
 }
 
 

@@ -323,6 +323,7 @@ struct ProjSeg {
   int32_t rope_dim;   // 0: no rotation; else the per-head width the rotation works on
   void* dst;          // [M][n], f32 or bf16
   int32_t bf16;
+  int32_t by_tma;     // the next launch reads it by TMA
 };
 struct FinishParams {
   const float* part;
@@ -378,7 +379,7 @@ __global__ void proj_finish_kernel(const FinishParams p) {
   }
   if (sg.bf16) {
     reinterpret_cast<uint32_t*>(sg.dst)[((size_t)m * sg.n + c) >> 1] = pack_bf16x2(v0, v1);
-    fence_chained_writes();
+    if (sg.by_tma) fence_chained_writes();
   } else {
     *reinterpret_cast<float2*>(reinterpret_cast<float*>(sg.dst) + (size_t)m * sg.n + c) = make_float2(v0, v1);
   }
@@ -748,7 +749,7 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   float* d_kr = (float*)(sc.rest + b_qc + b_qr + b_c);
   float* d_attn = (float*)(sc.rest + b_qc + b_qr + b_c + b_kr);
   // 1 + 2. projections, RoPE on q^R and k^R
-  const ProjSeg segs[4] = {{H * Dh, 0, d_qc, fast ? 1 : 0}, {H * dHR, dHR, d_qr, fast ? 1 : 0}, {dC, 0, d_c, 0}, {dHR, dHR, d_kr, 0}};
+  const ProjSeg segs[4] = {{H * Dh, 0, d_qc, fast ? 1 : 0, 1}, {H * dHR, dHR, d_qr, fast ? 1 : 0, S > 1}, {dC, 0, d_c, 0, 0}, {dHR, dHR, d_kr, 0, 0}};
   rc = project_and_finish(p, sb, a->layer, (const float*)dx, M, D, S, proj, segs, 4, mma, sc.a_bf16, sc.part, sc.part_cap, faithful);
   if (rc) return rc;
   // 3. append (advances the cursors).  A one-token step on the tensor-core path leaves the append to the attention's
@@ -852,7 +853,7 @@ int32_t do_gqa_layer(Pool* p, const relux_gqa_layer_args* a) {
   float* d_v = (float*)(sc.rest + b_q + b_kv);
   float* d_attn = (float*)(sc.rest + b_q + 2 * b_kv);
   const int rd = a->rope ? hd : 0;
-  const ProjSeg segs[3] = {{H * hd, rd, d_q, fast ? 1 : 0}, {Hkv * hd, rd, d_k, 0}, {Hkv * hd, 0, d_v, 0}};
+  const ProjSeg segs[3] = {{H * hd, rd, d_q, fast ? 1 : 0, S > 1}, {Hkv * hd, rd, d_k, 0, 0}, {Hkv * hd, 0, d_v, 0, 0}};
   rc = project_and_finish(p, sb, a->layer, (const float*)dx, M, D, S, proj, segs, 3, mma, sc.a_bf16, sc.part, sc.part_cap, faithful);
   if (rc) return rc;
   // append: the GEMM rows are token-major [row][Hkv][hd]; advance = 0 leaves the rows past the cursor (verify).  A short
