@@ -28,7 +28,7 @@ constexpr int kMaxChunks = 4;     // the fused merge + up-projection keeps at mo
 constexpr int kAbsorbSmem = 32768 + 16384 + 1024;
 __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const void* __restrict__ q_nope,
                                              const void* __restrict__ q_rope, int q_bf16, uint16_t* __restrict__ q_abs, int rows, int H, int dC,
-                                             int dHR, int bx, int by, int bz, int32_t* status, bool wait_for_queries) {
+                                             int dHR, int bx, int by, int bz, int32_t* status, bool chained, bool wait_for_queries) {
   __shared__ __align__(8) uint64_t landed;
   uint8_t* sm = (uint8_t*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* Bs = sm;             // [2 halves of d][128 c][64], swizzled
@@ -118,15 +118,16 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
     const int r = e / 16, v = e % 16;
     *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + c0 + v * 8) = *reinterpret_cast<const uint4*>(Os + r * kStride + v * 8);
   }
-  fence_chained_writes();
+  if (chained) fence_chained_writes();
 }
 
-// grid (H, dC/128, ceil(rows/64)), 128 threads.
+// grid (H, dC/128, ceil(rows/64)), 128 threads.  A plain launch that releases nobody early: the decode kernel reads its rows by TMA
+// behind its end.
 __global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
                                                              const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
                                                              uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int32_t* status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z, status, false);
+  absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z, status, false, false);
 }
 
 // The preparation of one MLA decode step in ONE launch: blocks 0 .. n_seqs - 1 append the step's new rows (a sequence
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ C
   if (e > ap.n_seqs) {
     const int a = e - ap.n_seqs - 1, slices = dC / 128;
     absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, ap.status,
-                 weights_ready != 0);
+                 true, weights_ready != 0);
     return;
   }
   if (weights_ready) chain_wait();
@@ -185,11 +186,11 @@ __device__ __forceinline__ void tile_mma_16xn(const uint16_t* As, uint32_t Bs, f
 // from one round trip: lane j reads (max, sum) of item j, the warp reduces.
 // kChunks: 128-column chunks of a warp, 4 / kChunks warps share a row; 16 / kChunks items are in flight per lane.  A call of
 // up to four rows has more warps than rows, and its rows the most items (each worker holds a piece of some sequence).
-// Rows past the batch are zero rows of the MMA tile.
+// Rows past the batch are zero rows of the MMA tile.  The pointers have come through behind_wait().
 constexpr int kMergeWarps = 16;
 template <int kChunks>
-__device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                                const int32_t* __restrict__ chunk_off, int r0, int rows, int tile_rows, int S, int H, int h, int dC, int nk_all,
+__device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* part_o, const float* part_ml, const int32_t* chunk_off,
+                                                int r0, int rows, int tile_rows, int S, int H, int h, int dC, int nk_all,
                                                 int rows_total) {
   constexpr int kParts = kMaxChunks / kChunks, kItems = 16 / kChunks, kRowStep = kMergeWarps / kParts;
   const int warp = (int)(threadIdx.x >> 5) / kParts, lane = threadIdx.x & 31;   // the warp's first row of the tile
@@ -201,8 +202,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
   int c0_next = 0, c1_next = 0;
   if (r0 + warp < rows) {
     const int i = (r0 + warp) / S;
-    c0_next = load_chained(chunk_off + i);
-    c1_next = load_chained(chunk_off + i + 1);
+    c0_next = load_settled(chunk_off + i);
+    c1_next = load_settled(chunk_off + i + 1);
   }
   for (int row = warp; row < tile_rows; row += kRowStep) {
     const int r = r0 + row;
@@ -210,8 +211,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
     c0_next = c1_next = 0;
     if (row + kRowStep < tile_rows && r + kRowStep < rows) {
       const int i = (r + kRowStep) / S;
-      c0_next = load_chained(chunk_off + i);
-      c1_next = load_chained(chunk_off + i + 1);
+      c0_next = load_settled(chunk_off + i);
+      c1_next = load_settled(chunk_off + i + 1);
     }
     float4 acc[kChunks];
 #pragma unroll
@@ -223,7 +224,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
       const int n_items = c1 - c0;
       if (n_items <= 0) goto store_row;   // no partial to merge: a zero row
       float2 ml = make_float2(-INFINITY, 0.f);
-      if (lane < n_items) ml = load_chained(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
+      if (lane < n_items) ml = load_settled(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
       float4 x[kItems][kChunks];
       const int ng0 = min(32, n_items);
 #pragma unroll
@@ -233,16 +234,16 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
         const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(c0 + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
         for (int k = 0; k < kChunks; k++)
-          if (k < nk) x[u][k] = (u < ng0) ? load_chained(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < nk) x[u][k] = (u < ng0) ? load_settled(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       // global maximum and normaliser over all items of the sequence
       float M = ml.x;
-      for (int c = c0 + 32 + lane; c < c1; c += 32) M = fmaxf(M, load_chained(part_ml + ((size_t)c * rows_total + prow) * 2));
+      for (int c = c0 + 32 + lane; c < c1; c += 32) M = fmaxf(M, load_settled(part_ml + ((size_t)c * rows_total + prow) * 2));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
       float L = (ml.x != -INFINITY) ? ml.y * exp2f(ml.x - M) : 0.f;
       for (int c = c0 + 32 + lane; c < c1; c += 32) {
-        const float2 t = load_chained(reinterpret_cast<const float2*>(part_ml + ((size_t)c * rows_total + prow) * 2));
+        const float2 t = load_settled(reinterpret_cast<const float2*>(part_ml + ((size_t)c * rows_total + prow) * 2));
         if (t.x != -INFINITY) L += t.y * exp2f(t.x - M);
       }
 #pragma unroll
@@ -254,7 +255,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
         if (cb == c0) {
           w_mine = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M) * inv;
         } else if (cb + lane < c1) {
-          const float m = load_chained(part_ml + ((size_t)(cb + lane) * rows_total + prow) * 2);
+          const float m = load_settled(part_ml + ((size_t)(cb + lane) * rows_total + prow) * 2);
           w_mine = (m == -INFINITY) ? 0.f : exp2f(m - M) * inv;
         }
         const int ng = min(32, c1 - cb);
@@ -265,7 +266,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
               const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(cb + j + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
               for (int k = 0; k < kChunks; k++)
-                if (k < nk) x[u][k] = (j + u < ng) ? load_chained(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k < nk) x[u][k] = (j + u < ng) ? load_settled(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
 #pragma unroll
@@ -302,8 +303,8 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* __res
 // copies of a row each, issued behind the merge's first loads, they took 2-3 us to be accepted).  The MMAs of the row
 // groups that hold a row are shared by all 16 warps (8 for up to 16 rows), chunk by chunk as the boxes land.
 // grid (H, ceil(rows/64)), 512 threads, row = seq_index * S + query token.  dC = 128 * nk, nk <= 4.
-__global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const float* __restrict__ part_o,
-                                                                const float* __restrict__ part_ml, const int32_t* __restrict__ chunk_off,
+__global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const float* part_o,
+                                                                const float* part_ml, const int32_t* chunk_off,
                                                                 void* __restrict__ out, int out_bf16, int rows, int S, int H, int dC,
                                                                 int32_t* __restrict__ status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -327,6 +328,9 @@ __global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(con
     }
   }
   chain_wait();   // the partial results come from the kernel before this one
+  part_o = behind_wait(part_o);
+  part_ml = behind_wait(part_ml);
+  chunk_off = behind_wait(chunk_off);
   const int rows_here = min(64, rows - r0), groups = rows_here <= 16 ? 1 : rows_here <= 32 ? 2 : 4;
   if (rows_here <= 4) merge_rows_warp<1>(As, part_o, part_ml, chunk_off, r0, rows, groups * 16, S, H, h, dC, nk, rows_total);
   else if (rows_here <= 8) merge_rows_warp<2>(As, part_o, part_ml, chunk_off, r0, rows, groups * 16, S, H, h, dC, nk, rows_total);

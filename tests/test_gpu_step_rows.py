@@ -9,7 +9,7 @@ from tests.test_gpu_attention import EDGE_MAX, EDGE_MEAN, build_mla, dev  # noqa
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B", [1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("B", [1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 150])
 @pytest.mark.parametrize("q_bf16", [False, True])
 def test_mla_step_rows(dev, oracle, B, q_bf16):  # noqa: F811
     H, Dh, dC, dHR = 16, 128, 512, 64
