@@ -195,9 +195,15 @@ __device__ __forceinline__ float2 load_settled(const float2* p) {
   asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(__cvta_generic_to_global(p)));
   return v;
 }
-__device__ __forceinline__ float4 load_settled(const float4* p) {
+// The float4 at p, or zeros without a load where `there` is false: a predicate, not a branch around every load.
+__device__ __forceinline__ float4 load_settled_if(const float4* p, bool there) {
   float4 v;
-  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(__cvta_generic_to_global(p)));
+  asm("{\n\t.reg .pred t;\n\t"
+      "setp.ne.s32 t, %5, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
+      "@t ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
+      : "l"(__cvta_generic_to_global(p)), "r"((int)there));
   return v;
 }
 

@@ -234,7 +234,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* part_
         const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(c0 + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
         for (int k = 0; k < kChunks; k++)
-          if (k < nk) x[u][k] = (u < ng0) ? load_settled(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < nk) x[u][k] = load_settled_if(src + k * 32, u < ng0);
       }
       // global maximum and normaliser over all items of the sequence
       float M = ml.x;
@@ -266,7 +266,7 @@ __device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* part_
               const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(cb + j + u) * rows_total + prow) * dC) + lane;
 #pragma unroll
               for (int k = 0; k < kChunks; k++)
-                if (k < nk) x[u][k] = (j + u < ng) ? load_settled(src + k * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k < nk) x[u][k] = load_settled_if(src + k * 32, j + u < ng);
             }
           }
 #pragma unroll
