@@ -204,7 +204,8 @@ int32_t relux_pool_read_rows(relux_pool_t pool, const relux_read_rows_args* args
 #define RELUX_TUNE_MLA_WORKERS 1        /* RELUX_MLA_WORKERS: ranges the stream of pages is cut into (0 = resident pairs)   */
 #define RELUX_TUNE_CHUNK_PAGES 2        /* RELUX_CHUNK_PAGES: chunk length of the split-KV planner (0 = chosen per call)    */
 #define RELUX_TUNE_GEMM_GENERIC 3       /* RELUX_GEMM_GENERIC: 1 = projections on the plain kernel                          */
-#define RELUX_TUNE_GEMM_SPLIT 4         /* RELUX_GEMM_SPLIT: split-K factor of the tcgen05 GEMM (0 = chosen per call)       */
+#define RELUX_TUNE_GEMM_SPLIT 4         /* RELUX_GEMM_SPLIT: workers per tile (128 weight columns x a block of rows) of the tcgen05
+                                           GEMM (0 = one worker per SM, the split along K chosen per call)                 */
 #define RELUX_TUNE_GQA_PROMPT_PARTIAL_MB 5 /* RELUX_GQA_PROMPT_PARTIAL_MB: partial-buffer budget of a GQA prompt (256)      */
 #define RELUX_TUNE_SEL_CLUSTER 6        /* RELUX_SEL_CLUSTER: cluster size of the selection kernel, 1/2/4/8 (0 = per call) */
 #define RELUX_TUNE_SEL_LOOKAHEAD 7      /* RELUX_SEL_LOOKAHEAD: 0/1 (-1 = per call)                                         */
@@ -214,11 +215,12 @@ int32_t relux_pool_read_rows(relux_pool_t pool, const relux_read_rows_args* args
 #define RELUX_TUNE_MLA_PROMPT_MIN_TOKENS 10 /* RELUX_MLA_PROMPT_MIN_TOKENS: query tokens per sequence from which an MLA call expands
                                            K / V and runs the tcgen05 prefill kernel (128; a huge value turns the path off) */
 #define RELUX_TUNE_MLA_PROMPT_SCRATCH_MB 11 /* RELUX_MLA_PROMPT_SCRATCH_MB: most device memory the expanded K / V may take (16384) */
-#define RELUX_TUNE_KERNEL_TIMING_STRIDE 12 /* RELUX_KERNEL_TIMING_STRIDE: the MLA decode kernel's event pair is recorded on every
-                                           Nth call (1); the pairs are what relux_pool_kernel_ms_* read */
-#define RELUX_TUNE_CHAINED_LAUNCHES 13 /* RELUX_CHAINED_LAUNCHES: 1 = the kernels of an MLA decode step are launched with
-                                           programmatic stream serialization, so each is scheduled while the one before it
-                                           still runs and waits on the device for its results (1); 0 = plain launches */
+#define RELUX_TUNE_KERNEL_TIMING_STRIDE 12 /* RELUX_KERNEL_TIMING_STRIDE: the MLA decode kernel is timed on every Nth call (1);
+                                           relux_pool_kernel_ms_* read the times */
+#define RELUX_TUNE_CHAINED_LAUNCHES 13 /* RELUX_CHAINED_LAUNCHES: 1 = the kernels of decode and verify steps, layer steps, matmuls
+                                           and prompts, and relux_seq_set_len, are launched with programmatic stream
+                                           serialization, so each is scheduled while the one before it still runs and waits
+                                           on the device for its results (1); 0 = plain launches */
 #define RELUX_TUNE_COUNT 14
 /* Changes one tuning knob of a pool (see RELUX_TUNE_*).  A pool takes its defaults once, when it is created, from the
  * environment variables named beside the knobs; no call reads the environment afterwards.  value < 0 restores the
@@ -304,8 +306,11 @@ int32_t relux_gqa_decode(relux_pool_t pool, const relux_attn_args* args);
 /* One decode step in one call: append the new rows (append->advance must be 1), then attend over the cache that now
  * includes them -- MLA.forwardCached steps 4-6 (mla.go:309-377), MHA.forwardCached steps 5-8 (mha.go:283-348).  Same
  * results as relux_*_append followed by relux_*_decode.  On the MLA tensor-core path the append and the stream partition
- * ride in the launch that absorbs W_UK into the queries (one kernel instead of three); other shapes and modes run the two
- * calls one after the other.  Both argument structs must name the same layer and sequences. */
+ * ride in the launch that absorbs W_UK into the queries (one kernel instead of three).  A GQA step of up to 32 query rows
+ * per kv head (64-token pages, 128-wide heads, FAST mode) is one launch: append, attention and the merge of its splits; so
+ * is relux_gqa_verify.  Other shapes and modes run the two calls one after the other.  Both argument structs must name the
+ * same layer and sequences.  Where the attention is refused, the rows of a GQA step and of a step run as two calls stay
+ * appended, as by two calls; a fused MLA step leaves the lengths as they were. */
 int32_t relux_mla_step(relux_pool_t pool, const relux_append_args* append, const relux_attn_args* attn);
 int32_t relux_gqa_step(relux_pool_t pool, const relux_append_args* append, const relux_attn_args* attn);
 
@@ -514,22 +519,26 @@ typedef struct relux_stream_partition_args {
 } relux_stream_partition_args;
 int32_t relux_stream_partition(const relux_stream_partition_args* args);
 
-/* Device-time of the dominant attention kernel of the most recent relux_*_decode / verify call on this
- * pool, measured with CUDA events around that one launch.  Synchronises the stream.  Measurement aid: no counterpart
- * in the reference. */
+/* Device time of the dominant attention kernel of the most recent relux_*_decode / verify / step call on this pool (for
+ * token selection, of the selection kernel).  The tensor-core kernels stamp %globaltimer themselves: from the first block
+ * that has its inputs (the kernel before it in the stream complete) to the end of the last block; launch overhead is not in
+ * it, and for a GQA step the append and the merge are.  The reference-mode and generic kernels, and GQA prompts as grid
+ * slices, are timed by CUDA events around their launches.  Synchronises the stream.  Measurement aid: no counterpart in
+ * the reference. */
 int32_t relux_pool_last_kernel_ms(relux_pool_t pool, float* ms);
 
 /* Mean device time of that kernel over the most recent `last_n` decode / verify calls on this pool (at most
- * 8192 are kept); `counted` receives how many calls went into the mean.  The event pairs are recorded by the
- * calls themselves, so reading them after a timed loop does not disturb the loop.  Synchronises the stream.
+ * 8192 are kept); `counted` receives how many calls went into the mean.  The times are recorded by the calls
+ * themselves, so reading them after a timed loop does not disturb the loop.  Synchronises the stream.
  * Measurement aid: no counterpart in the reference. */
 int32_t relux_pool_kernel_ms_mean(relux_pool_t pool, int32_t last_n, float* mean_ms, int32_t* counted);
 /* The same times one by one: ms_out [last_n] receives the device time of each of the most recent calls, oldest first;
  * `counted` how many were written.  Measurement aid: no counterpart in the reference. */
 int32_t relux_pool_kernel_ms_list(relux_pool_t pool, int32_t last_n, float* ms_out, int32_t* counted);
 
-/* Same for the input-projection launch (x . [W_Q | W_QR | W_DKV | W_KR]) of the most recent
- * relux_mla_forward_cached calls on this pool.  Measurement aid: no counterpart in the reference. */
+/* Same for the input-projection launch (x . [W_Q | W_QR | W_DKV | W_KR], or x . [W_Q | W_K | W_V]) of the most recent
+ * relux_*_forward_cached calls on this pool; its blocks stamp their begin before they wait for the rounded x, when their
+ * weights begin to load.  Measurement aid: no counterpart in the reference. */
 int32_t relux_pool_projection_ms_mean(relux_pool_t pool, int32_t last_n, float* mean_ms, int32_t* counted);
 
 /* ---- the matmul of the compute backend ---------------------------------------------------------
