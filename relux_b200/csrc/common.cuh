@@ -122,6 +122,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int32_t x, 
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, int32_t x, int32_t y, int32_t z, int32_t w, const void* smem_src) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map), "r"(smem_u32(smem_src)), "r"(x),
+               "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // All committed stores of this thread have finished READING their shared tiles (the tiles may be written again).
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -243,5 +248,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // Byte offset of element (row, col16B chunk) inside a tile whose rows are 128 bytes and which was
 // written by TMA with CU_TENSOR_MAP_SWIZZLE_128B: the 16-byte chunk index is XORed with (row & 7).
 __device__ __forceinline__ uint32_t swz128(uint32_t row, uint32_t chunk16) { return row * 128u + ((chunk16 ^ (row & 7u)) << 4); }
+// The same for rows of 64 bytes and CU_TENSOR_MAP_SWIZZLE_64B.
+__device__ __forceinline__ uint32_t swz64(uint32_t row, uint32_t chunk16) { return row * 64u + ((chunk16 ^ ((row >> 1) & 3u)) << 4); }
 
 }  // namespace relux

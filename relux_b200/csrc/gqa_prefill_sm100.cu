@@ -70,10 +70,11 @@ constexpr int kMaxDepth = 4;
 
 // Shared-memory plan of the two variants.
 //   GQA (kMla = false): score width 128.  Q tile [dims 0-63 | dims 64-127] x 2 buffers (items in turn), K stage = own
-//     page [dims 0-63 | dims 64-127] (16 KB), four K and four V stages: 64 + 64 + 64 = 192 KB.
+//     page [dims 0-63 | dims 64-127] (16 KB), four K and four V stages, 4 KB of output staging per read-out warp:
+//     64 + 64 + 64 + 16 = 208 KB.
 //   MLA (kMla = true): score width 192 = 128 expanded key dims + 64 shared RoPE dims.  Q tile [nope 0-63 | nope 64-127 |
 //     rope] (48 KB) x 2 buffers, K stage = own 64 keys [nope 0-63 | nope 64-127 | rope] (24 KB), three K and three V
-//     stages: 96 + 72 + 48 = 216 KB.
+//     stages, 2 KB of output staging per read-out warp: 96 + 72 + 48 + 8 = 224 KB.
 // P never touches shared memory: the softmax warps write it, packed to bf16, over the first 64 columns of the S tile they
 // have just read, and PV takes its A operand from tensor memory.
 template <bool kMla>
@@ -87,7 +88,10 @@ struct Plan {
   static constexpr int kSmemQ = 0;
   static constexpr int kSmemK = kSmemQ + kQBufs * kQBytes;
   static constexpr int kSmemV = kSmemK + kDepthK * kKBytes;
-  static constexpr int kSmemBar = kSmemV + kDepthV * kVBytes;
+  static constexpr int kSmemOut = kSmemV + kDepthV * kVBytes;
+  static constexpr int kOutCols = kMla ? 16 : 32;           // output columns a read-out warp stages at a time (float32)
+  static constexpr int kOutTile = 32 * kOutCols * 4;
+  static constexpr int kSmemBar = kSmemOut + 4 * kOutTile;
   static constexpr int kSmemTotal = kSmemBar + 3072;
   static_assert(kSmemTotal <= 232448, "more shared memory than a CTA may use");
 };
@@ -132,7 +136,6 @@ struct PrefillParams {
   int32_t Ttot, rope_block, blocks_per_page;
   int64_t pool_row0;
   float scale_log2;
-  float* out;                 // [n][S][H][128] f32
   int32_t* status;
   TimeStamp time;
 };
@@ -231,11 +234,12 @@ __device__ __forceinline__ void tma_load_3d_2sm(void* smem_dst, const CUtensorMa
 }
 
 // tmap_kv: GQA the pool's K / V rows; MLA the expanded keys / values.  tmap_q: the queries (MLA: their nope part).
-// tmap_qr, tmap_rope (MLA only): the queries' RoPE part, and the pool's 64-column blocks.
+// tmap_qr, tmap_rope (MLA only): the queries' RoPE part, and the pool's 64-column blocks.  tmap_out: [n][S][H][128] float32.
 template <bool kMla>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_q,
-                         const __grid_constant__ CUtensorMap tmap_qr, const __grid_constant__ CUtensorMap tmap_rope, const PrefillParams prm) {
+                         const __grid_constant__ CUtensorMap tmap_qr, const __grid_constant__ CUtensorMap tmap_rope,
+                         const __grid_constant__ CUtensorMap tmap_out, const PrefillParams prm) {
   using PL = Plan<kMla>;
   constexpr int kQBytes = PL::kQBytes, kQBufs = PL::kQBufs, kKBytes = PL::kKBytes, kDepthK = PL::kDepthK, kDepthV = PL::kDepthV;
   constexpr int kSmemQ = PL::kSmemQ, kSmemK = PL::kSmemK, kSmemV = PL::kSmemV;
@@ -574,17 +578,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // =============================== read-out: O / l -> out ===============================
     // One warp per TMEM lane quarter; item n's accumulator is O buffer n & 1, handed over by the commit behind the
     // item's last PV and handed back (to the first PV of item n + 2) when the row has been read.
+    // The rows leave through a swizzled tile in shared memory and by TMA, as whole lines; rows past the prompt's last token
+    // lie outside the tensor map and are not written.  Stores from registers, a row per lane (32 half sectors an
+    // instruction), held up the warps that share the load/store unit: @@
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
-    const int tq = r / prm.g, hq = r % prm.g;       // token in block, head in group
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const uint32_t o_empty_lead[2] = {mapa_u32(smem_u32(&bars->o_empty[0]), 0), mapa_u32(smem_u32(&bars->o_empty[1]), 0)};
+    constexpr int kOutCols = PL::kOutCols;
+    uint8_t* tile = smem + PL::kSmemOut + wq * PL::kOutTile;
+    if (lane == 0) tma_prefetch_desc(&tmap_out);
     int n = 0;
     for (Cursor cu{worker, 0}; cursor_valid(prm, cu); cu = cursor_next(prm, cu, n_workers), n++) {
       const Item it = item_of<kMla>(prm, cu);
-      const int t0 = (2 * it.pair + (int)rank) * prm.bq;          // first query token of this CTA's block
-      const int ntok = max(0, min(prm.bq, prm.S - t0));           // its real tokens (0: the odd block of the last pair)
-      const bool real = tq < ntok;                                 // rows past the prompt's last token are padding: computed, never written
+      const int t0 = (2 * it.pair + (int)rank) * prm.bq + wq * 32 / prm.g;   // first query token of the warp's rows
       wait_bar(&bars->l_full, n & 1, bars, prm.status);
       const float l_row = bars->lsum[r];
       __syncwarp();
@@ -594,24 +601,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       tc_fence_after();
       const bool ok = !__any_sync(0xffffffffu, bars->abort_flag != 0);
       const float inv = (ok && l_row > 0.f) ? 1.f / l_row : 0.f;
-      float* orow = prm.out + (((size_t)it.bi * prm.S + t0 + (real ? tq : 0)) * prm.H + (size_t)it.hk * prm.g + hq) * kD;
 #pragma unroll 1
       for (int c = 0; c < kD; c += 32) {
         uint32_t ov[32];
         tmem_ld_32x32b_x32(tmem + lane_addr + kTmemO + (n & 1) * 128 + c, ov);
         tmem_ld_wait();
-        if (real) {
-          float4* dst = reinterpret_cast<float4*>(orow + c);
 #pragma unroll
-          for (int i = 0; i < 8; i++)
-            dst[i] = make_float4(__uint_as_float(ov[4 * i]) * inv, __uint_as_float(ov[4 * i + 1]) * inv, __uint_as_float(ov[4 * i + 2]) * inv,
-                                 __uint_as_float(ov[4 * i + 3]) * inv);
+        for (int h = 0; h < 32; h += kOutCols) {
+          if (lane == 0) tma_store_wait_read();   // the tile's last store has read it
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < kOutCols / 4; i++)
+            *reinterpret_cast<float4*>(tile + (kOutCols == 32 ? swz128(lane, i) : swz64(lane, i))) =
+                make_float4(__uint_as_float(ov[h + 4 * i]) * inv, __uint_as_float(ov[h + 4 * i + 1]) * inv,
+                            __uint_as_float(ov[h + 4 * i + 2]) * inv, __uint_as_float(ov[h + 4 * i + 3]) * inv);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0 && t0 < prm.S) {
+            tma_store_4d(&tmap_out, c + h, it.hk * prm.g, t0, it.bi, tile);
+            tma_store_commit();
+          }
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster((n & 1) ? o_empty_lead[1] : o_empty_lead[0]);
     }
+    if (lane == 0) tma_store_wait_all();
   }
   __syncwarp();
   tc_fence_before();
@@ -653,6 +669,14 @@ int prefill_workers(Pool* p) {
   return max_clusters;
 }
 
+// Output [n][S][H][128] float32: a box is kOutCols columns of the rows of one read-out warp, g heads of 32 / g tokens of a sequence.
+template <bool kMla>
+bool make_tmap_out(CUtensorMap* m, float* out, int n, int S, int H, int g) {
+  const uint64_t dims[4] = {(uint64_t)kD, (uint64_t)H, (uint64_t)S, (uint64_t)n};
+  const uint32_t box[4] = {(uint32_t)Plan<kMla>::kOutCols, (uint32_t)g, (uint32_t)(32 / g), 1};
+  return make_tmap_4d_f32(m, out, dims, box);
+}
+
 }  // namespace
 
 // g query heads per kv head must tile the 128 rows of the block exactly.
@@ -667,6 +691,11 @@ bool gqa_prefill_eligible(const Pool* p, const relux_attn_args& a) {
 int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const uint16_t* d_q, float* d_out) {
   const relux_pool_params& prm = p->prm;
   const int g = a.num_heads / prm.gqa_num_kv_heads, bq = 128 / g, S = a.q_tokens, H = a.num_heads;
+  CUtensorMap tout;
+  if (!make_tmap_out<false>(&tout, d_out, sb.n_seqs, S, H, g)) {
+    set_error("tensor map for the prompt's output could not be encoded");
+    return RELUX_ERR_CUDA;
+  }
   CUtensorMap tq;   // queries [n * S][H][128]: a box is the g heads of one KV head for bq tokens
   if (!make_tmap_3d(&tq, (void*)d_q, (uint64_t)sb.n_seqs * S, (uint64_t)H, kD, 64, (uint32_t)g, (uint32_t)bq)) {
     set_error("tensor map for the prompt's queries could not be encoded");
@@ -697,7 +726,6 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.krow0 = (int32_t)((int64_t)a.layer * 2 * rows_per_block);
   k.vrow0 = (int32_t)((int64_t)a.layer * 2 * rows_per_block + rows_per_block);
   k.scale_log2 = a.scale * 1.4426950408889634f;
-  k.out = d_out;
   k.status = p->d_status;
   cudaStream_t st = p->dev->stream;
   const int workers = std::min(prefill_workers<false>(p), k.n_couples);
@@ -706,7 +734,7 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<false>, grid, dim3(kThreads), (size_t)kSmemTotal, st,
-                                p->tmap_gqa, tq, tq, p->tmap_gqa, k));
+                                p->tmap_gqa, tq, tq, p->tmap_gqa, tout, k));
   time_stamp_done(p->attn_times, k.time);
   count_launch(p->dev);
   return RELUX_OK;
@@ -749,7 +777,11 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   int32_t* seq_base = (int32_t*)((char*)p->expand_buf.p + ((x_bytes + 255) & ~(size_t)255));
   rc = launch_mla_expand_sm100(p, sb, a.layer, a.extra_tokens, H, (const uint16_t*)a.w_uk, (const uint16_t*)a.w_uv, Ttot, kx, vx, seq_base);
   if (rc) return rc;
-  CUtensorMap tq, tqr, tx;
+  CUtensorMap tq, tqr, tx, tout;
+  if (!make_tmap_out<true>(&tout, d_out, sb.n_seqs, S, H, 1)) {
+    set_error("tensor map for the prompt's output could not be encoded");
+    return RELUX_ERR_CUDA;
+  }
   // queries [n * S][H][128] and their rope parts [n * S][H][64]: a box is one head for 128 tokens
   if (!make_tmap_3d(&tq, (void*)d_q, (uint64_t)sb.n_seqs * S, (uint64_t)H, kD, 64, 1, 128) ||
       !make_tmap_3d(&tqr, (void*)d_qr, (uint64_t)sb.n_seqs * S, (uint64_t)H, 64, 64, 1, 128)) {
@@ -789,7 +821,6 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.rope_block = prm.mla_dc / 64;
   k.pool_row0 = (int64_t)a.layer * prm.num_pages * k.blocks_per_page * kPage;
   k.scale_log2 = a.scale * 1.4426950408889634f;
-  k.out = d_out;
   k.status = p->d_status;
   cudaStream_t st = p->dev->stream;
   const int workers = std::min(prefill_workers<true>(p), k.n_couples);
@@ -798,7 +829,7 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.time = time_stamp_next(p, p->attn_times);
   dim3 grid(2 * workers, 1, 1);   // CTA pairs
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, prefill_sm100_kernel<true>, grid, dim3(kThreads), (size_t)kSmemTotal, st, tx,
-                                tq, tqr, p->tmap_mla, k));
+                                tq, tqr, p->tmap_mla, tout, k));
   time_stamp_done(p->attn_times, k.time);
   count_launch(p->dev);
   return RELUX_OK;

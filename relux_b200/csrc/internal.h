@@ -253,6 +253,8 @@ int32_t check_dev_align(const void* ptr, const char* what);
 //   2-D: [rows][cols], cols contiguous, box = box_cols x box_rows.
 //   3-D: [outer][mid][cols], cols contiguous and mid rows adjacent, box = box_cols x box_mid x box_outer.
 bool make_tmap_2d(CUtensorMap* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
+//   4-D, float32, for stores: dims and box innermost first, box[0] = 16 or 32 columns (swizzled by the row length).
+bool make_tmap_4d_f32(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]);
 bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint64_t cols, uint32_t box_cols, uint32_t box_mid,
                   uint32_t box_outer);
 

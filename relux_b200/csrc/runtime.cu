@@ -240,6 +240,17 @@ bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint
   return r == CUDA_SUCCESS;
 }
 
+// Float32, for stores; box[0] is 16 or 32 columns, the swizzle that of the box's row length.
+bool make_tmap_4d_f32(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return false;
+  const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]};
+  const cuuint64_t strides[3] = {d[0] * 4, d[1] * d[0] * 4, d[2] * d[1] * d[0] * 4};
+  const cuuint32_t b[4] = {box[0], box[1], box[2], box[3]}, estr[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, d, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 void tuning_defaults(Tuning* t);
 
 static void pool_free_all(Pool* p) {
