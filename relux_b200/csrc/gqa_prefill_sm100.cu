@@ -580,7 +580,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // item's last PV and handed back (to the first PV of item n + 2) when the row has been read.
     // The rows leave through a swizzled tile in shared memory and by TMA, as whole lines; rows past the prompt's last token
     // lie outside the tensor map and are not written.  Stores from registers, a row per lane (32 half sectors an
-    // instruction), held up the warps that share the load/store unit: @@
+    // instruction), held up the warps that share the load/store unit: 343 -> 317 us (8 x 2048 tokens,
+    // 32 heads over 8), 274 -> 251 us (MLA, 4 x 1000).
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
