@@ -31,7 +31,7 @@ namespace {
 constexpr int kSelThreads = 512;
 constexpr int kSelWarps = kSelThreads / 32;
 constexpr int kMaxCluster = 8;
-constexpr int kStatMax = 16;     // batched statistics: two rows for each of up to 8 draft positions
+constexpr int kStatMax = 32;     // batched statistics: two sums and two maxima for each of up to 8 draft positions
 
 struct SelParams {
   const int32_t* draft_tokens;   // [n][k] or nullptr (plain sampling)
@@ -45,8 +45,7 @@ struct SelParams {
   float temperature;
   int32_t top_k;
   float top_p, min_p;
-  int32_t lookahead;             // accept loop: take the next position's maxima in the pass that sums this one's
-  int32_t batched;               // accept loop: maxima of all positions' rows in one stage, all sums in a second
+  int32_t batched;               // accept loop: the rows of all positions in one stage
   TimeStamp time;
 };
 
@@ -57,11 +56,12 @@ struct SelShared {
   float hist_sum[256];
   uint32_t hist_cnt[256];
   float warp_seg[kSelWarps];  // per-warp segment sums of the search pass
-  uint32_t warp_hist[kSelWarps][256];   // radix selection: one histogram per warp (counts, or float sums)
-  uint32_t list_count;        // candidate list of the small-top-k path (the list itself reuses warp_hist)
+  alignas(16) uint32_t warp_hist[kSelWarps][256];   // radix selection: one histogram per warp (counts, or float sums)
+  uint32_t list_count, list_bound;      // candidate list of the small-top-k path (the list itself reuses warp_hist), and its bound
+  alignas(16) uint32_t grp_key[kSelThreads];        // keys of the largest element of every thread (or pair of threads)
   float red_n[2][kStatMax];   // cluster_reduce_n: per-CTA partials, double-buffered like red
   float warp_part_n[kSelWarps][kStatMax];
-  float stat[2][kStatMax];    // [0] maxima, [1] sums of exponentials of all draft positions' rows (batched statistics)
+  float stat[kStatMax];       // batched statistics: of draft position i the sums (draft, target) at 4 i, the maxima at 4 i + 2
 };
 
 __device__ __forceinline__ uint32_t order_key(float x) {
@@ -129,27 +129,28 @@ __device__ void cluster_reduce4(Ctx& c, float (&v)[4]) {
   c.round++;
 }
 
-// The same for `count` <= kStatMax values per thread (acc[]); the results land in dst[] in this CTA's shared memory.
-template <bool kMax>
+// The same for `count` <= kStatMax values per thread (acc[]), sums where bit 1 of the index is clear and maxima where it is
+// set; the results land in dst[] in this CTA's shared memory.
 __device__ void cluster_reduce_n(Ctx& c, const float* acc, int count, float* dst) {
   cg::cluster_group cl = cg::this_cluster();
   for (int j = 0; j < count; j++) {
-    const float r = kMax ? warp_max(acc[j]) : warp_sum(acc[j]);
+    const float r = (j & 2) ? warp_max(acc[j]) : warp_sum(acc[j]);
     if (c.lane == 0) c.sh->warp_part_n[c.warp][j] = r;
   }
   __syncthreads();
   const int buf = c.round & 1;
+  const bool mx = threadIdx.x & 2;
   if ((int)threadIdx.x < count) {
     float a = c.sh->warp_part_n[0][threadIdx.x];
-    for (int w = 1; w < kSelWarps; w++) a = kMax ? fmaxf(a, c.sh->warp_part_n[w][threadIdx.x]) : a + c.sh->warp_part_n[w][threadIdx.x];
+    for (int w = 1; w < kSelWarps; w++) a = mx ? fmaxf(a, c.sh->warp_part_n[w][threadIdx.x]) : a + c.sh->warp_part_n[w][threadIdx.x];
     c.sh->red_n[buf][threadIdx.x] = a;
   }
   cl.sync();
   if ((int)threadIdx.x < count) {
-    float a = kMax ? -INFINITY : 0.0f;
+    float a = mx ? -INFINITY : 0.0f;
     for (int r = 0; r < c.csize; r++) {
       const float x = *cl.map_shared_rank(&c.sh->red_n[buf][threadIdx.x], r);
-      a = kMax ? fmaxf(a, x) : a + x;
+      a = mx ? fmaxf(a, x) : a + x;
     }
     dst[threadIdx.x] = a;
   }
@@ -369,104 +370,121 @@ __device__ bool radix_select(Ctx& c, const float* __restrict__ row, KeyF key_wei
   return true;
 }
 
-// Inverse-CDF search: the first index whose running sum of prob(index, value) exceeds r (Sampler.Sample step 8,
-// sampler.go:200-209; resampleRejected, speculative.go:271-291), or `dflt` when the sum never does.  Sums run per
-// warp segment, then in segment order; the segment that crosses is walked again in index order.
-// sum_segment(): this lane's share of the sum over the warp's segment.
-template <class ProbF, class SumF>
-__device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, float r, int dflt, int32_t* out, SumF sum_segment) {
-  const float part = warp_sum(sum_segment());
+// Inverse-CDF search: the first index whose running sum of probabilities exceeds r (Sampler.Sample step 8, sampler.go:200-209;
+// resampleRejected, speculative.go:271-291), or `dflt` when the sum never does.  Two calls, so that a pass which sums the row
+// anyway (for its normalisation) is not made twice: segment_sums() takes this lane's share of the sum over the warp's
+// segment, leaves the sums of the warps in shared memory and those of the CTAs in all[], and returns the row's; cdf_search()
+// finds the segment that crosses (its sums times `factor`) and walks that one in index order.
+__device__ float segment_sums(Ctx& c, float part, float (&all)[kMaxCluster]) {
+  part = warp_sum(part);
   if (c.lane == 0) c.sh->warp_seg[c.warp] = part;
   __syncthreads();
   float tot = 0.0f;
   for (int w = 0; w < kSelWarps; w++) tot += c.sh->warp_seg[w];
-  float all[kMaxCluster];
   cluster_gather1(c, tot, all);
-  float base = 0.0f;
+  float sum = 0.0f;
+#pragma unroll
+  for (int q = 0; q < kMaxCluster; q++)
+    if (q < c.csize) sum += all[q];
+  return sum;
+}
+// Four neighbouring elements of a row from index i; what lies at or past hi is 0 (and must not be used).
+__device__ __forceinline__ float4 load4(const Ctx& c, const float* __restrict__ row, int i, int hi) {
+  if (c.vec) return i < hi ? __ldg(reinterpret_cast<const float4*>(row + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(i < hi ? __ldg(row + i) : 0.f, i + 1 < hi ? __ldg(row + i + 1) : 0.f, i + 2 < hi ? __ldg(row + i + 2) : 0.f,
+                     i + 3 < hi ? __ldg(row + i + 3) : 0.f);
+}
+// prob(value, value of row2 at the same index); row2 may be nullptr.
+template <class ProbF>
+__device__ void cdf_search(Ctx& c, const float* __restrict__ row, const float* __restrict__ row2, ProbF prob, float r, int dflt, int32_t* out,
+                           const float (&all)[kMaxCluster], float factor) {
+  float base = 0.0f, run = 0.0f;
   int cross = -1;
-  float run = 0.0f;
-  for (int q = 0; q < c.csize; q++) {
+#pragma unroll
+  for (int q = 0; q < kMaxCluster; q++) {
+    if (q >= c.csize) break;
     if (q == c.rank) base = run;
-    run += all[q];
+    run += __fmul_rn(all[q], factor);
     if (cross < 0 && run > r) cross = q;
   }
   // No path below leaves early with the cluster's exchange still in use: the caller ends with a cluster barrier.
   if (cross < 0) {
     if (c.rank == 0 && threadIdx.x == 0) *out = dflt;
-  } else if (cross == c.rank) {
-    // this CTA holds the crossing: pick the warp, then walk its segment in order
-    int wsel = kSelWarps - 1;
-    float wbase = base;
-    float acc = base;
-    for (int w = 0; w < kSelWarps; w++) {
-      float nxt = acc + c.sh->warp_seg[w];
-      wbase = acc;
-      if (nxt > r) { wsel = w; break; }
-      acc = nxt;
+    return;
+  }
+  if (cross != c.rank) return;
+  // this CTA holds the crossing: pick the warp, then walk its segment in order
+  int wsel = kSelWarps - 1;
+  float acc = base, wbase = base;
+  for (int w = 0; w < kSelWarps; w++) {
+    const float nxt = acc + __fmul_rn(c.sh->warp_seg[w], factor);
+    wbase = acc;
+    if (nxt > r) { wsel = w; break; }
+    acc = nxt;
+  }
+  if (c.warp != wsel) return;
+  // The segment in blocks of 128 elements, four neighbours per lane, four blocks' loads in flight.  The first block in which
+  // the running sum crosses is searched lane by lane, and the lane that crosses element by element.  (Lanes that each summed a
+  // contiguous chunk of the segment paid for 16 dependent rounds of scattered loads.)
+  acc = wbase;
+  int hit = -1, last_pos = -1;
+  for (int b0 = c.wlo; b0 < c.whi && hit < 0; b0 += 512) {
+    float4 p[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int i = b0 + 128 * u + 4 * c.lane;
+      const float4 v = load4(c, row, i, c.whi), v2 = row2 ? load4(c, row2, i, c.whi) : v;
+      p[u] = v;
+      p[u].x = i < c.whi ? prob(v.x, v2.x) : 0.0f;
+      p[u].y = i + 1 < c.whi ? prob(v.y, v2.y) : 0.0f;
+      p[u].z = i + 2 < c.whi ? prob(v.z, v2.z) : 0.0f;
+      p[u].w = i + 3 < c.whi ? prob(v.w, v2.w) : 0.0f;
     }
-    if (c.warp == wsel) {
-      // Two levels, so that the walk costs two memory latencies instead of one per 32 elements: every lane sums a
-      // contiguous chunk of the segment, a scan over the lanes finds the chunk that crosses, and that chunk alone is
-      // walked in index order.
-      const int seglen = c.whi - c.wlo;
-      const int chunk = (((seglen + 31) >> 5) + 3) & ~3;
-      const int l0 = min(c.whi, c.wlo + c.lane * chunk), l1 = min(c.whi, l0 + chunk);
-      float mine = 0.0f;
-#pragma unroll 4
-      for (int i = l0; i < l1; i++) mine += prob(i, __ldg(row + i));
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const float mine = p[u].x + p[u].y + p[u].z + p[u].w;
       float x = mine;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        float y = __shfl_up_sync(0xffffffffu, x, o);
+        const float y = __shfl_up_sync(0xffffffffu, x, o);
         if (c.lane >= o) x += y;
       }
-      const uint32_t over = __ballot_sync(0xffffffffu, wbase + x > r);
-      const uint32_t carry = __ballot_sync(0xffffffffu, mine > 0.0f);
-      int hit_idx = -1;
-      if (over || carry) {
-        const int lsel = over ? __ffs(over) - 1 : 31 - __clz(carry);
-        const float before = __shfl_up_sync(0xffffffffu, x, 1);
-        float acc2 = wbase + __shfl_sync(0xffffffffu, c.lane > 0 ? before : 0.0f, lsel);
-        const int c0 = __shfl_sync(0xffffffffu, l0, lsel), c1 = __shfl_sync(0xffffffffu, l1, lsel);
-        int last_pos = -1;
-        for (int j = c0; j < c1 && hit_idx < 0; j += 32) {
-          const int i = j + c.lane;
-          const float pv = i < c1 ? prob(i, __ldg(row + i)) : 0.0f;
-          float z = pv;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            float y = __shfl_up_sync(0xffffffffu, z, o);
-            if (c.lane >= o) z += y;
-          }
-          const uint32_t hit = __ballot_sync(0xffffffffu, i < c1 && acc2 + z > r);
-          if (hit) hit_idx = j + __ffs(hit) - 1;
-          const uint32_t pos = __ballot_sync(0xffffffffu, pv > 0.0f);
-          if (pos) last_pos = j + 31 - __clz(pos);
-          acc2 += __shfl_sync(0xffffffffu, z, 31);
+      const int i = b0 + 128 * u + 4 * c.lane;
+      // the last element so far that carries probability: what is taken when rounding puts the crossing past the end
+      const int lp = p[u].w > 0.0f ? i + 3 : p[u].z > 0.0f ? i + 2 : p[u].y > 0.0f ? i + 1 : p[u].x > 0.0f ? i : -1;
+      const uint32_t pos = __ballot_sync(0xffffffffu, lp >= 0), over = __ballot_sync(0xffffffffu, acc + x > r);
+      if (hit < 0) {
+        if (over) {
+          const float before = __shfl_up_sync(0xffffffffu, x, 1);
+          float a = acc + (c.lane > 0 ? before : 0.0f);
+          int h = -1;
+          a += p[u].x; if (h < 0 && a > r) h = i;
+          a += p[u].y; if (h < 0 && a > r) h = i + 1;
+          a += p[u].z; if (h < 0 && a > r) h = i + 2;
+          a += p[u].w; if (h < 0 && a > r) h = i + 3;
+          if (h < 0) h = lp;                     // the lane's own sum rounds differently from its four steps
+          const int src = __ffs(over) - 1;
+          hit = __shfl_sync(0xffffffffu, h, src);
+          if (hit < 0) hit = b0 + 128 * u + 4 * src;
         }
-        // when rounding put the crossing past the end of the chunk: its last element that carries probability
-        if (hit_idx < 0) hit_idx = last_pos;
+        if (pos) last_pos = __shfl_sync(0xffffffffu, lp, 31 - __clz(pos));
+        acc += __shfl_sync(0xffffffffu, x, 31);
       }
-      if (hit_idx < 0) hit_idx = c.whi > c.wlo ? c.whi - 1 : dflt;
-      if (c.lane == 0) *out = hit_idx;
     }
   }
-}
-template <class ProbF>
-__device__ void cdf_find(Ctx& c, const float* __restrict__ row, ProbF prob, float r, int dflt, int32_t* out) {
-  cdf_find(c, row, prob, r, dflt, out, [&]() {
-    float part = 0.0f;
-    for_segment(c, row, [&](int i, float v) { part += prob(i, v); });
-    return part;
-  });
+  if (hit < 0) hit = last_pos >= 0 ? last_pos : c.whi > c.wlo ? c.whi - 1 : dflt;
+  if (c.lane == 0) *out = min(hit, c.whi - 1);
 }
 
 // Sampler.Sample with a small top-k, finished on a list: after top-k only the k largest logits (and their ties) carry
-// probability, so once the radix walk has narrowed the row down to at most kCandCap elements the CTAs collect them,
-// CTA 0 sorts them by index and walks the rest of the reference's chain (softmax, nucleus, min-p, draw) over the list.
-// Every float32 sum runs in index order over the kept elements -- the elements the reference adds zeros for are
-// skipped -- so this path gives the reference's token bit for bit.  Returns false (nothing written) when the list
-// would not fit; the caller then takes the pass-per-step path.
+// probability.  Two looks at the row put them on a list.  Every thread keeps the largest element it has read; with m = k / CTAs
+// (rounded up), the m-th largest of a CTA's is a bound that at least m of its elements reach, so the smallest of the CTAs'
+// bounds is one that at least k of the row's reach, and hardly more do (about 70 of 131072 for k = 50).  The few threads that
+// hold one read their elements again.  (A radix walk over the row for the bound took a histogram round or two, each 3-5 us.)
+// Rank 0 gathers the lists and walks the rest of the reference's chain (softmax, nucleus, min-p, draw) over what is on them.
+// Every float32 sum runs in index order over the kept elements -- the elements the reference adds zeros for are skipped -- so
+// this path gives the reference's token bit for bit.  Lists that would not fit (plateaus of ties, tiny rows) are narrowed down
+// by the radix walk; returns false (nothing written) when not even that fits, and the caller takes the pass-per-step path.
 constexpr int kCandTopK = 128;   // largest top-k that takes this path
 constexpr int kCandCap = 512;    // list capacity
 
@@ -474,129 +492,215 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
                                       int32_t* out) {
   cg::cluster_group cl = cg::this_cluster();
   const int V = prm.vocab;
-  uint32_t key_lo = 0, n_ge = 0;
-  radix_select<false>(c, row, [&](float v, uint32_t& k, float& w) { k = order_key(d.scaled(v)); w = 0.0f; }, (uint32_t)topk, 0.0f, &key_lo,
-                      (uint32_t)kCandCap, &n_ge);
-  if (n_ge > (uint32_t)kCandCap) return false;     // more ties at the threshold than the list holds (uniform over the cluster)
-  // the list lives in the histogram block: words [0,512) values, [512,1024) indices
-  float* l_val = reinterpret_cast<float*>(&c.sh->warp_hist[0][0]);
-  int32_t* l_idx = reinterpret_cast<int32_t*>(&c.sh->warp_hist[0][0]) + kCandCap;
-  uint32_t* l_cnt = &c.sh->list_count;
-  if (threadIdx.x == 0) *l_cnt = 0;
+  SelShared& sh = *c.sh;
+  // the lists live in the histogram block: words [0,512) values, [512,1024) indices of this CTA's
+  float* l_val = reinterpret_cast<float*>(&sh.warp_hist[0][0]);
+  int32_t* l_idx = reinterpret_cast<int32_t*>(&sh.warp_hist[0][0]) + kCandCap;
+  auto collect = [&](uint32_t key_lo) {
+    for_segment(c, row, [&](int i, float v) {
+      const float x = d.scaled(v);
+      if (order_key(x) >= key_lo) {
+        const uint32_t pos = atomicAdd(&sh.list_count, 1u);
+        if (pos < (uint32_t)kCandCap) { l_val[pos] = x; l_idx[pos] = i; }
+      }
+    });
+  };
+  // The largest element per thread, as a key (the division by the temperature keeps the order, so it is made once, behind the
+  // pass).  Of long slices, pairs of threads: half as many keys to rank.
+  uint32_t key = 0;
+  for_segment(c, row, [&](int, float v) { key = max(key, order_key(v)); });
+  if (key) {
+    const uint32_t u = (key & 0x80000000u) ? (key & 0x7fffffffu) : ~key;
+    key = order_key(d.scaled(__uint_as_float(u)));
+  }
+  const bool pairs = c.hi - c.lo > 8 * kSelThreads;
+  const int m = (topk + c.csize - 1) / c.csize;
+  const int n_grp = pairs ? kSelThreads / 2 : kSelThreads;
+  uint32_t grp = key;
+  if (pairs) grp = max(grp, __shfl_xor_sync(0xffffffffu, grp, 1));
+  if (!pairs) sh.grp_key[threadIdx.x] = grp;
+  else if (!(c.lane & 1)) sh.grp_key[threadIdx.x >> 1] = grp;
+  if (threadIdx.x == 0) sh.list_count = 0;
   __syncthreads();
-  for_segment(c, row, [&](int i, float v) {
-    const float x = d.scaled(v);
-    if (order_key(x) >= key_lo) {
-      const uint32_t pos = atomicAdd(l_cnt, 1u);
-      if (pos < (uint32_t)kCandCap) { l_val[pos] = x; l_idx[pos] = i; }
+  if ((int)threadIdx.x < n_grp) {
+    const uint32_t mine = sh.grp_key[threadIdx.x];
+    int gt = 0, ge = 0;
+#pragma unroll 4
+    for (int j = 0; j < n_grp; j += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&sh.grp_key[j]);
+      gt += (q.x > mine) + (q.y > mine) + (q.z > mine) + (q.w > mine);
+      ge += (q.x >= mine) + (q.y >= mine) + (q.z >= mine) + (q.w >= mine);
     }
-  });
+    if (gt < m && m <= ge) sh.list_bound = mine;   // several threads with the same key write the same value
+  }
   __syncthreads();
   cl.sync();
+  uint32_t bound = 0xffffffffu;
+  for (int q = 0; q < c.csize; q++) bound = min(bound, *cl.map_shared_rank(&sh.list_bound, q));
+  if (key >= bound) collect(bound);
+  __syncthreads();
+  cl.sync();
+  uint32_t total = 0;
+  for (int q = 0; q < c.csize; q++) total += *cl.map_shared_rank(&sh.list_count, q);
+  if (total > (uint32_t)kCandCap) {   // uniform over the cluster
+    cl.sync();                        // everyone has read the counts
+    uint32_t key_lo = 0, n_ge = 0;
+    radix_select<false>(c, row, [&](float v, uint32_t& k, float& w) { k = order_key(d.scaled(v)); w = 0.0f; }, (uint32_t)topk, 0.0f, &key_lo,
+                        (uint32_t)kCandCap, &n_ge);
+    if (n_ge > (uint32_t)kCandCap) return false;     // more ties at the threshold than the list holds
+    if (threadIdx.x == 0) sh.list_count = 0;
+    __syncthreads();
+    collect(key_lo);
+    __syncthreads();
+    cl.sync();
+  }
   if (c.rank == 0) {
-    float* a_val = l_val + 2 * kCandCap;            // all candidates, then (sorted by index) the kept ones and their probabilities
+    float* a_val = l_val + 2 * kCandCap;            // all candidates, then the kept ones by index and their probabilities
     int32_t* a_idx = l_idx + 2 * kCandCap;
-    float* k_val = l_val + 4 * kCandCap;
+    float* k_p = l_val + 4 * kCandCap;
     int32_t* k_idx = l_idx + 4 * kCandCap;
-    float* k_p = l_val + 6 * kCandCap;
     int32_t* k_ord = l_idx + 6 * kCandCap;
-    __shared__ int s_n, s_cut;
-    __shared__ float s_thr, s_scale;
-    // gather the lists of all CTAs (rank order)
-    int n_c = 0;
-    for (int q = 0; q < c.csize; q++) {
-      const uint32_t cnt = min(*cl.map_shared_rank(l_cnt, q), (uint32_t)kCandCap);
+    __shared__ int s_n, s_c, s_cut;
+    __shared__ float s_thr, s_scale, s_max;
+    if (threadIdx.x == 0) { s_n = 0; s_c = 0; }
+    __syncthreads();
+    {   // gather: the warps share the lists out among them
+      const int q = c.warp % c.csize, per = kSelWarps / c.csize;
+      const int cnt = (int)*cl.map_shared_rank(&sh.list_count, q);
       const float* rv = cl.map_shared_rank(l_val, q);
       const int32_t* ri = cl.map_shared_rank(l_idx, q);
-      for (int t = threadIdx.x; t < (int)cnt; t += kSelThreads)
-        if (n_c + t < kCandCap) { a_val[n_c + t] = rv[t]; a_idx[n_c + t] = ri[t]; }
-      n_c += (int)cnt;
+      for (int t = (c.warp / c.csize) * 32 + c.lane; t < cnt; t += per * 32) {
+        const float v = rv[t];
+        const int32_t i = ri[t];
+        const int pos = atomicAdd(&s_c, 1);
+        a_val[pos] = v;
+        a_idx[pos] = i;
+      }
     }
-    n_c = min(n_c, kCandCap);
     __syncthreads();
+    const int n_c = s_c;
     // kthLargest (sampler.go:283-300): the value with fewer than topk elements above it and at least topk at or above
-    if (threadIdx.x < n_c) {
-      const float v = a_val[threadIdx.x];
+    for (int t = threadIdx.x; t < n_c; t += kSelThreads) {
+      const float v = a_val[t];
       int gt = 0, ge = 0;
+#pragma unroll 4
       for (int j = 0; j < n_c; j++) { gt += a_val[j] > v; ge += a_val[j] >= v; }
       if (gt < topk && topk <= ge) s_thr = v;
+      if (gt == 0) s_max = v;
     }
-    if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
-    const float thr = s_thr;
-    // keep what the mask leaves (not below the threshold), in index order
-    if (threadIdx.x < n_c && !(a_val[threadIdx.x] < thr)) {
+    const float thr = s_thr, maxV = s_max;
+    // keep what the mask leaves (not below the threshold), in index order, with its exponential (sampler.go:118-137)
+    for (int t = threadIdx.x; t < n_c; t += kSelThreads) {
+      const float v = a_val[t];
+      if (v < thr) continue;
+      const int i = a_idx[t];
       int pos = 0;
-      for (int j = 0; j < n_c; j++) pos += (!(a_val[j] < thr)) && a_idx[j] < a_idx[threadIdx.x];
-      k_val[pos] = a_val[threadIdx.x];
-      k_idx[pos] = a_idx[threadIdx.x];
+#pragma unroll 4
+      for (int j = 0; j < n_c; j++) pos += (!(a_val[j] < thr)) && a_idx[j] < i;
+      k_idx[pos] = i;
+      k_p[pos] = fastexp32_ref(__fsub_rn(v, maxV));
       atomicAdd(&s_n, 1);
     }
     __syncthreads();
     const int n_k = s_n;
-    // softmax over the kept logits (sampler.go:118-137)
-    if (threadIdx.x == 0) {
-      float maxV = k_val[0];
-      for (int j = 1; j < n_k; j++) if (k_val[j] > maxV) maxV = k_val[j];
-      float sum = 0.0f;
-      for (int j = 0; j < n_k; j++) { k_p[j] = fastexp32_ref(__fsub_rn(k_val[j], maxV)); sum = __fadd_rn(sum, k_p[j]); }
-      s_scale = sum > 0.0f ? __fdiv_rn(1.0f, sum) : 1.0f;
-    }
-    __syncthreads();
-    if (threadIdx.x < n_k) k_p[threadIdx.x] = __fmul_rn(k_p[threadIdx.x], s_scale);
-    __syncthreads();
+    // sums in index order: one thread, four elements a load (what is padded adds zeros)
+    auto sum_in_order = [&]() {
+      if (threadIdx.x == 0) {
+        for (int j = n_k; j < ((n_k + 3) & ~3); j++) k_p[j] = 0.0f;
+        float sum = 0.0f;
+#pragma unroll 4
+        for (int j = 0; j < n_k; j += 4) {
+          const float4 q = *reinterpret_cast<const float4*>(k_p + j);
+          sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, q.x), q.y), q.z), q.w);
+        }
+        s_scale = sum > 0.0f ? __fdiv_rn(1.0f, sum) : 1.0f;
+      }
+      __syncthreads();
+    };
+    auto rescale = [&]() {
+      for (int t = threadIdx.x; t < n_k; t += kSelThreads) k_p[t] = __fmul_rn(k_p[t], s_scale);
+      __syncthreads();
+    };
+    sum_in_order();
+    rescale();
     float topP = prm.top_p;
     if (topP <= 0.0f || topP > 1.0f) topP = 1.0f;
     if (topP < 1.0f) {
-      // argsortDescF32 (sampler.go:268-281) followed only as far as the cut: a selection sort over all indices whose
-      // step i swaps the first largest remaining entry with whatever sits at position i.  Entries without probability
-      // are interchangeable, so only the positions of the kept elements are tracked (k_ord: position in the reference's
-      // index array, -1 once selected, -2 selected and kept); which of two equal probabilities comes first follows
-      // from the swaps, exactly as in the reference.
-      if (threadIdx.x < n_k) k_ord[threadIdx.x] = k_idx[threadIdx.x];
-      __syncthreads();
-      if (c.warp == 0) {   // one warp: the search of every step is spread over its lanes, the running sum stays sequential
-        float cum = 0.0f;
-        bool cut = false;
-        for (int step = 0; step < n_k && !cut; step++) {
-          float bp = -1.0f;
-          int bpos = 0x7fffffff, bj = -1, at_i = -1;
-          for (int j = c.lane; j < n_k; j += 32) {
-            const int pj = k_ord[j];
-            if (pj < 0) continue;
-            if (pj == step) at_i = j;
-            const float pv = k_p[j];
-            if (pv > bp || (pv == bp && pj < bpos)) { bp = pv; bpos = pj; bj = j; }
-          }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            const float op = __shfl_xor_sync(0xffffffffu, bp, o);
-            const int opos = __shfl_xor_sync(0xffffffffu, bpos, o), oj = __shfl_xor_sync(0xffffffffu, bj, o);
-            at_i = max(at_i, __shfl_xor_sync(0xffffffffu, at_i, o));
-            if (op > bp || (op == bp && opos < bpos)) { bp = op; bpos = opos; bj = oj; }
-          }
-          if (bj < 0 || !(bp > 0.0f)) break;      // only zeros are left: the running sum stays below top-p
-          if (c.lane == 0) {
-            if (at_i >= 0 && at_i != bj) k_ord[at_i] = bpos;   // what sat at position `step` moves to the winner's place
-            k_ord[bj] = -2;
-          }
-          __syncwarp();
-          cum = __fadd_rn(cum, bp);
-          if (cum >= topP) cut = true;
-        }
-        if (c.lane == 0) s_cut = cut ? 1 : 0;
+      // The reference sorts by probability (argsortDescF32, sampler.go:268-281) and cuts where the running sum reaches topP.
+      // Which of equal probabilities comes first does not change the sums, so any order by rank gives the cut; only when it
+      // falls between equals does it matter which of them are kept, and then the sort is followed step by step (below).
+      float* ranked = a_val;
+      for (int t = threadIdx.x; t < n_k; t += kSelThreads) {
+        const float v = k_p[t];
+        int rank = 0;
+#pragma unroll 4
+        for (int j = 0; j < n_k; j++) rank += k_p[j] > v || (k_p[j] == v && j < t);
+        ranked[rank] = v;
+        k_ord[t] = rank;
       }
-      __syncthreads();
-      if (s_cut && threadIdx.x < n_k && k_ord[threadIdx.x] != -2) k_p[threadIdx.x] = 0.0f;
       __syncthreads();
       if (threadIdx.x == 0) {
-        float s2 = 0.0f;
-        for (int j = 0; j < n_k; j++) s2 = __fadd_rn(s2, k_p[j]);
-        s_scale = s2 > 0.0f ? __fdiv_rn(1.0f, s2) : 1.0f;
+        float cum = 0.0f;
+        int cut = n_k;
+        for (int j = 0; j < n_k; j++) {
+          cum = __fadd_rn(cum, ranked[j]);
+          if (cum >= topP) { cut = j + 1; break; }
+        }
+        s_cut = cut < n_k && ranked[cut] == ranked[cut - 1] ? -1 : cut;
       }
       __syncthreads();
-      if (threadIdx.x < n_k) k_p[threadIdx.x] = __fmul_rn(k_p[threadIdx.x], s_scale);
-      __syncthreads();
+      const int cut = s_cut;
+      if (cut >= 0) {
+        for (int t = threadIdx.x; t < n_k; t += kSelThreads)
+          if (k_ord[t] >= cut) k_p[t] = 0.0f;
+        __syncthreads();
+      } else {
+        // argsortDescF32 followed as far as the cut: a selection sort over all indices whose step i swaps the first largest
+        // remaining entry with whatever sits at position i.  Entries without probability are interchangeable, so only the
+        // positions of the kept elements are tracked (k_ord: position in the reference's index array, -2 once selected);
+        // which of two equal probabilities comes first follows from the swaps, exactly as in the reference.
+        for (int t = threadIdx.x; t < n_k; t += kSelThreads) k_ord[t] = k_idx[t];
+        __syncthreads();
+        if (c.warp == 0) {   // one warp: the search of every step is spread over its lanes, the running sum stays sequential
+          float cum = 0.0f;
+          bool done = false;
+          for (int step = 0; step < n_k && !done; step++) {
+            float bp = -1.0f;
+            int bpos = 0x7fffffff, bj = -1, at_i = -1;
+            for (int j = c.lane; j < n_k; j += 32) {
+              const int pj = k_ord[j];
+              if (pj < 0) continue;
+              if (pj == step) at_i = j;
+              const float pv = k_p[j];
+              if (pv > bp || (pv == bp && pj < bpos)) { bp = pv; bpos = pj; bj = j; }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+              const float op = __shfl_xor_sync(0xffffffffu, bp, o);
+              const int opos = __shfl_xor_sync(0xffffffffu, bpos, o), oj = __shfl_xor_sync(0xffffffffu, bj, o);
+              at_i = max(at_i, __shfl_xor_sync(0xffffffffu, at_i, o));
+              if (op > bp || (op == bp && opos < bpos)) { bp = op; bpos = opos; bj = oj; }
+            }
+            if (bj < 0 || !(bp > 0.0f)) break;      // only zeros are left: the running sum stays below top-p
+            if (c.lane == 0) {
+              if (at_i >= 0 && at_i != bj) k_ord[at_i] = bpos;   // what sat at position `step` moves to the winner's place
+              k_ord[bj] = -2;
+            }
+            __syncwarp();
+            cum = __fadd_rn(cum, bp);
+            if (cum >= topP) done = true;
+          }
+          if (c.lane == 0) s_cut = done ? 1 : 0;
+        }
+        __syncthreads();
+        if (s_cut)
+          for (int t = threadIdx.x; t < n_k; t += kSelThreads)
+            if (k_ord[t] != -2) k_p[t] = 0.0f;
+        __syncthreads();
+      }
+      sum_in_order();
+      rescale();
     }
     if (prm.min_p > 0.0f) {
       if (threadIdx.x == 0) {
@@ -605,20 +709,16 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
         s_thr = __fmul_rn(maxProb, prm.min_p);
       }
       __syncthreads();
-      if (threadIdx.x < n_k && k_p[threadIdx.x] < s_thr) k_p[threadIdx.x] = 0.0f;
+      for (int t = threadIdx.x; t < n_k; t += kSelThreads)
+        if (k_p[t] < s_thr) k_p[t] = 0.0f;
       __syncthreads();
-      if (threadIdx.x == 0) {
-        float s3 = 0.0f;
-        for (int j = 0; j < n_k; j++) s3 = __fadd_rn(s3, k_p[j]);
-        s_scale = s3 > 0.0f ? __fdiv_rn(1.0f, s3) : 1.0f;
-      }
-      __syncthreads();
-      if (threadIdx.x < n_k) k_p[threadIdx.x] = __fmul_rn(k_p[threadIdx.x], s_scale);
-      __syncthreads();
+      sum_in_order();
+      rescale();
     }
     if (threadIdx.x == 0) {
       float cum = 0.0f;
       int tok = V - 1;
+#pragma unroll 4
       for (int j = 0; j < n_k; j++) {
         cum = __fadd_rn(cum, k_p[j]);
         if (r < cum) { tok = k_idx[j]; break; }
@@ -650,10 +750,10 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
   cluster_reduce4<1>(c, v4);
   d.m = v4[0];
   d.inv1 = 1.0f;
-  v4[0] = v4[1] = v4[2] = v4[3] = 0.0f;
-  for_segment(c, row, [&](int, float v) { v4[0] += d.p1(v); });
-  cluster_reduce4<0>(c, v4);
-  if (v4[0] > 0.0f) d.inv1 = __fdiv_rn(1.0f, v4[0]);
+  float all[kMaxCluster], part = 0.0f;
+  for_segment(c, row, [&](int, float v) { part += d.p1(v); });
+  const float sum = segment_sums(c, part, all);
+  if (sum > 0.0f) d.inv1 = __fdiv_rn(1.0f, sum);
   float topP = prm.top_p;
   if (topP <= 0.0f || topP > 1.0f) topP = 1.0f;
   if (topP < 1.0f) {
@@ -682,8 +782,15 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
     d.minp_thr = thr;
     d.inv3 = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
   }
-  auto p3 = [&](int, float v) { float p = p2(v); if (minp) p = p < d.minp_thr ? 0.0f : __fmul_rn(p, d.inv3); return p; };
-  cdf_find(c, row, p3, r, V - 1, out);
+  auto p3 = [&](float v, float) { float p = p2(v); if (minp) p = p < d.minp_thr ? 0.0f : __fmul_rn(p, d.inv3); return p; };
+  float factor = d.inv1;   // without a filter behind the sum, its segments are the search's
+  if (nucleus || minp) {
+    factor = 1.0f;
+    part = 0.0f;
+    for_segment(c, row, [&](int, float v) { part += p3(v, 0.0f); });
+    segment_sums(c, part, all);
+  }
+  cdf_search(c, row, nullptr, p3, r, V - 1, out, all, factor);
 }
 
 __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams prm) {
@@ -712,42 +819,67 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
   int used = 0;
   int n_acc = k;
   bool done = false;
-  // Few sequences: the chain's length is what costs, not the bytes.  The maxima of the rows of ALL draft positions are
-  // taken in one stage and all sums of exponentials in a second, so the accept loop below runs without a pass of its own
-  // per position (rows after a rejection are read in vain).
-  const bool batched = prm.batched && k >= 2 && 2 * k <= kStatMax;
+  // Maximum and sum of exponentials of a draft and a target row in ONE pass: the sum needs the maximum first (fastexp32 is not
+  // multiplicative), so it is taken against a guess, the logit of the draft token -- the draft's largest where the draft model
+  // decodes greedily, and the target's where the two agree -- and made again, out of L2, for a row whose maximum turns out to
+  // be another.
+  auto drow_of = [&](int i) { return prm.draft_logits + ((size_t)b * k + i) * V; };
+  auto trow_of = [&](int i) { return prm.target_logits + ((size_t)b * (k + 1) + i) * V; };
+  auto pair_pass = [&](int i, float& sd, float& st, float& md, float& mt) {
+    const float *drow = drow_of(i), *trow = trow_of(i);
+    const int tok = min(max(prm.draft_tokens[(size_t)b * k + i], 0), V - 1);
+    const float gd = __ldg(drow + tok), gt = __ldg(trow + tok);
+    float a = 0.0f, t = 0.0f, ma = -INFINITY, mb = -INFINITY;
+    for_segment2(c, drow, trow, [&](int, float dv, float tv) {
+      ma = fmaxf(ma, dv);
+      mb = fmaxf(mb, tv);
+      a += fastexp32_ref(__fsub_rn(dv, gd));
+      t += fastexp32_ref(__fsub_rn(tv, gt));
+    });
+    sd = a; st = t; md = ma; mt = mb;
+  };
+  // the sums again where the guess was not the maximum; whether there is anything to do
+  auto pair_again = [&](int i, float md, float mt, float& sd, float& st) {
+    const float *drow = drow_of(i), *trow = trow_of(i);
+    const int tok = min(max(prm.draft_tokens[(size_t)b * k + i], 0), V - 1);
+    const bool bad_d = __ldg(drow + tok) != md, bad_t = __ldg(trow + tok) != mt;
+    float a = 0.0f, t = 0.0f;
+    if (bad_d && bad_t)
+      for_segment2(c, drow, trow, [&](int, float dv, float tv) { a += fastexp32_ref(__fsub_rn(dv, md)); t += fastexp32_ref(__fsub_rn(tv, mt)); });
+    else if (bad_d)
+      for_segment(c, drow, [&](int, float dv) { a += fastexp32_ref(__fsub_rn(dv, md)); });
+    else if (bad_t)
+      for_segment(c, trow, [&](int, float tv) { t += fastexp32_ref(__fsub_rn(tv, mt)); });
+    sd = a; st = t;
+    return (bad_d ? 1 : 0) | (bad_t ? 2 : 0);
+  };
+  // Few sequences: the chain's length is what costs, not the bytes.  The rows of ALL draft positions are read in one stage
+  // (and the sums to be made again in a second), so the accept loop below runs without a pass of its own per position (rows
+  // after a rejection are read in vain).
+  const bool batched = prm.batched && k >= 2 && 4 * k <= kStatMax;
   if (batched) {
     float acc[kStatMax];
+    for (int i = 0; i < k; i++) pair_pass(i, acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+    cluster_reduce_n(c, acc, 4 * k, c.sh->stat);
+    int any = 0;
     for (int i = 0; i < k; i++) {
-      float a = -INFINITY, t = -INFINITY;
-      for_segment2(c, prm.draft_logits + ((size_t)b * k + i) * V, prm.target_logits + ((size_t)b * (k + 1) + i) * V,
-                   [&](int, float dv, float tv) { a = fmaxf(a, dv); t = fmaxf(t, tv); });
-      acc[2 * i] = a;
-      acc[2 * i + 1] = t;
+      const int bad = pair_again(i, c.sh->stat[4 * i + 2], c.sh->stat[4 * i + 3], acc[4 * i], acc[4 * i + 1]);
+      // a row whose sum stands brings it along from one thread of the cluster
+      const bool first = c.rank == 0 && threadIdx.x == 0;
+      if (!(bad & 1)) acc[4 * i] = first ? c.sh->stat[4 * i] : 0.0f;
+      if (!(bad & 2)) acc[4 * i + 1] = first ? c.sh->stat[4 * i + 1] : 0.0f;
+      acc[4 * i + 2] = c.sh->stat[4 * i + 2];
+      acc[4 * i + 3] = c.sh->stat[4 * i + 3];
+      any |= bad;
     }
-    cluster_reduce_n<true>(c, acc, 2 * k, c.sh->stat[0]);
-    for (int i = 0; i < k; i++) {
-      const float md = c.sh->stat[0][2 * i], mt = c.sh->stat[0][2 * i + 1];
-      float a = 0.0f, t = 0.0f;
-      for_segment2(c, prm.draft_logits + ((size_t)b * k + i) * V, prm.target_logits + ((size_t)b * (k + 1) + i) * V,
-                   [&](int, float dv, float tv) { a += fastexp32_ref(__fsub_rn(dv, md)); t += fastexp32_ref(__fsub_rn(tv, mt)); });
-      acc[2 * i] = a;
-      acc[2 * i + 1] = t;
+    if (any) {   // uniform over the cluster: everyone looked at the same logits and maxima
+      __syncthreads();
+      cluster_reduce_n(c, acc, 4 * k, c.sh->stat);
     }
-    cluster_reduce_n<false>(c, acc, 2 * k, c.sh->stat[1]);
-  }
-  float next_md = 0.0f, next_mt = 0.0f;
-  if (k > 0 && prm.lookahead && !batched) {
-    float v4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    for_segment2(c, prm.draft_logits + (size_t)b * k * V, prm.target_logits + (size_t)b * (k + 1) * V,
-                 [&](int, float dv, float tv) { v4[0] = fmaxf(v4[0], dv); v4[1] = fmaxf(v4[1], tv); });
-    cluster_reduce4<1>(c, v4);
-    next_md = v4[0];
-    next_mt = v4[1];
   }
   for (int i = 0; i < k && !done; i++) {
-    const float* drow = prm.draft_logits + ((size_t)b * k + i) * V;
-    const float* trow = prm.target_logits + ((size_t)b * (k + 1) + i) * V;
+    const float* drow = drow_of(i);
+    const float* trow = trow_of(i);
     const int tok = prm.draft_tokens[(size_t)b * k + i];
     if (tok < 0 || tok >= V) {   // uniform over the cluster: every thread reads the same token
       if (writer) { set_status(prm.status, RELUX_ERR_INVALID_ARG); *out_tok = -1; }
@@ -755,39 +887,24 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
       done = true;
       break;
     }
-    // With look-ahead the maxima of this position's rows came with the previous position's sums (or from the pass
-    // before the loop): the pass below adds up the exponentials and already takes the maxima of the next position's
-    // rows, one barrier per draft position, at the price of two rows read in vain when this position rejects.  That
-    // pays while the chain is bound by latency (few sequences); with many sequences the passes are bound by bytes and
-    // the maxima get a pass of their own.
-    float v4[4];
-    float md, mt;
+    float v4[4], md, mt;
     if (batched) {
-      md = c.sh->stat[0][2 * i];
-      mt = c.sh->stat[0][2 * i + 1];
-      v4[0] = c.sh->stat[1][2 * i];
-      v4[1] = c.sh->stat[1][2 * i + 1];
+      v4[0] = c.sh->stat[4 * i];
+      v4[1] = c.sh->stat[4 * i + 1];
+      md = c.sh->stat[4 * i + 2];
+      mt = c.sh->stat[4 * i + 3];
     } else {
-      if (!prm.lookahead) {
-        v4[0] = v4[1] = v4[2] = v4[3] = -INFINITY;
-        for_segment2(c, drow, trow, [&](int, float dv, float tv) { v4[0] = fmaxf(v4[0], dv); v4[1] = fmaxf(v4[1], tv); });
-        cluster_reduce4<1>(c, v4);
-        next_md = v4[0];
-        next_mt = v4[1];
-      }
-      md = next_md;
-      mt = next_mt;
-      v4[0] = v4[1] = 0.0f;
-      v4[2] = v4[3] = -INFINITY;
-      for_segment2(c, drow, trow, [&](int, float dv, float tv) {
-        v4[0] += fastexp32_ref(__fsub_rn(dv, md));
-        v4[1] += fastexp32_ref(__fsub_rn(tv, mt));
-      });
-      if (prm.lookahead && i + 1 < k)
-        for_segment2(c, drow + V, trow + V, [&](int, float dv, float tv) { v4[2] = fmaxf(v4[2], dv); v4[3] = fmaxf(v4[3], tv); });
+      pair_pass(i, v4[0], v4[1], v4[2], v4[3]);
       cluster_reduce4<2>(c, v4);
-      next_md = v4[2];
-      next_mt = v4[3];
+      md = v4[2];
+      mt = v4[3];
+      float w4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const int bad = pair_again(i, md, mt, w4[0], w4[1]);
+      if (bad) {
+        cluster_reduce4<0>(c, w4);
+        if (bad & 1) v4[0] = w4[0];
+        if (bad & 2) v4[1] = w4[1];
+      }
     }
     const float invd = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
     const float invt = v4[1] > 0.0f ? __fdiv_rn(1.0f, v4[1]) : 1.0f;
@@ -804,20 +921,19 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
       float diff = __fsub_rn(tp, dp);
       return diff < 0.0f ? 0.0f : diff;
     };
-    v4[0] = v4[1] = v4[2] = v4[3] = 0.0f;
-    for_segment2(c, drow, trow, [&](int, float dv, float tv) { v4[0] += adj(tv, dv); });
-    cluster_reduce4<0>(c, v4);
+    float all[kMaxCluster], part = 0.0f;
+    for_segment2(c, drow, trow, [&](int, float dv, float tv) { part += adj(tv, dv); });
+    const float sum = segment_sums(c, part, all);
     const float r = draws[used++];
-    if (v4[0] > 0.0f) {
-      const float inv = __fdiv_rn(1.0f, v4[0]);
-      // the sums read both rows as vectors (through prob, the draft row came as single floats)
-      cdf_find(c, trow, [&](int j, float tv) { return __fmul_rn(adj(tv, __ldg(drow + j)), inv); }, r, 0, out_tok, [&]() {
-        float part = 0.0f;
-        for_segment2(c, drow, trow, [&](int, float dv, float tv) { part += __fmul_rn(adj(tv, dv), inv); });
-        return part;
-      });
+    if (sum > 0.0f) {
+      const float inv = __fdiv_rn(1.0f, sum);
+      cdf_search(c, trow, drow, [&](float tv, float dv) { return __fmul_rn(adj(tv, dv), inv); }, r, 0, out_tok, all, inv);
     } else {
-      cdf_find(c, trow, [&](int, float tv) { return __fmul_rn(fastexp32_ref(__fsub_rn(tv, mt)), invt); }, r, 0, out_tok);
+      auto tprob = [&](float tv, float) { return __fmul_rn(fastexp32_ref(__fsub_rn(tv, mt)), invt); };
+      part = 0.0f;
+      for_segment(c, trow, [&](int, float tv) { part += tprob(tv, 0.0f); });
+      segment_sums(c, part, all);
+      cdf_search(c, trow, nullptr, tprob, r, 0, out_tok, all, 1.0f);
     }
     n_acc = i;
     done = true;
@@ -1049,8 +1165,6 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
   prm.min_p = sp.min_p;
   prm.batched = n <= 16 ? 1 : 0;
   if (p->tune.get(RELUX_TUNE_SEL_BATCHED) >= 0) prm.batched = p->tune.get(RELUX_TUNE_SEL_BATCHED) ? 1 : 0;       // tuning knob
-  prm.lookahead = n <= 32 ? 1 : 0;   // measured: 6 % faster at 4-16 sequences, even at 32, 1 % slower at 64
-  if (p->tune.get(RELUX_TUNE_SEL_LOOKAHEAD) >= 0) prm.lookahead = p->tune.get(RELUX_TUNE_SEL_LOOKAHEAD) ? 1 : 0;   // tuning knob
   if (mode == RELUX_ATTN_REFERENCE) {
     // One thread per sequence repeats the reference's selection sorts: quadratic in the vocabulary for the nucleus cut,
     // top_k x vocabulary for kthLargest.  Refuse sizes that would keep the device busy for many seconds.
