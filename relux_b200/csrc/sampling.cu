@@ -1163,7 +1163,7 @@ static int32_t launch_selection(Pool* p, SelParams& prm, int n, const relux_samp
   prm.top_k = sp.top_k;
   prm.top_p = sp.top_p;
   prm.min_p = sp.min_p;
-  prm.batched = n <= 16 ? 1 : 0;
+  prm.batched = n <= 24 ? 1 : 0;
   if (p->tune.get(RELUX_TUNE_SEL_BATCHED) >= 0) prm.batched = p->tune.get(RELUX_TUNE_SEL_BATCHED) ? 1 : 0;       // tuning knob
   if (mode == RELUX_ATTN_REFERENCE) {
     // One thread per sequence repeats the reference's selection sorts: quadratic in the vocabulary for the nucleus cut,
