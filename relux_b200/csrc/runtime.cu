@@ -130,7 +130,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
   out->rows.resize(n_seqs);
   out->total_rows = 0;
   out->max_rows = 0;
-  bool uniform = true;
+  bool uniform = true, in_order = true;   // in_order: sequences 0, 1, ..., named or not
   for (int i = 0; i < n_seqs; i++) {
     int s = seq_ids ? seq_ids[i] : i;
     if (s < 0 || s >= prm.max_seqs || p->seq_pages[s] == 0) {
@@ -143,6 +143,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
       return RELUX_ERR_INVALID_ARG;
     }
     if (i > 0 && r != out->rows[0]) uniform = false;
+    if (s != i) in_order = false;
     out->seq[i] = s;
     out->rows[i] = r;
     out->total_rows += r;
@@ -164,7 +165,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
   out->d_seq_ids = nullptr;
   out->d_row_off = nullptr;
   out->rows_each = out->rows[0];
-  if (!upload || (!seq_ids && uniform)) return RELUX_OK;
+  if (!upload || (in_order && uniform)) return RELUX_OK;
   Device* dev = p->dev;
   int32_t* slot = nullptr;
   int slot_index = 0;
@@ -172,7 +173,7 @@ int32_t stage_batch(Pool* p, int32_t n_seqs, const int32_t* seq_ids, const int32
   if (rc_stage) return rc_stage;
   int32_t* h_ids = slot;
   int32_t* h_off = slot + prm.max_seqs;
-  if (seq_ids) {
+  if (!in_order) {
     memcpy(h_ids, out->seq.data(), sizeof(int32_t) * n_seqs);
     RELUX_CUDA_TRY(cudaMemcpyAsync(p->d_seq_ids, h_ids, sizeof(int32_t) * n_seqs, cudaMemcpyHostToDevice, dev->stream));
     out->d_seq_ids = p->d_seq_ids;
@@ -528,12 +529,19 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   const bool k_bf16 = a->out_dtype == RELUX_DTYPE_BF16 && out_tm &&
                       (gqa_stream || (kind == RELUX_POOL_MLA && a->mode == RELUX_ATTN_FAST && mla_writes_bf16(p, sb, *a)));
   const int k_dtype = k_bf16 ? RELUX_DTYPE_BF16 : RELUX_DTYPE_F32;
-  const bool direct = a->out_mem == RELUX_MEM_DEVICE && a->out_dtype == k_dtype && out_tm;
+  const bool need_conv = a->out_dtype != k_dtype || !out_tm;
+  const bool direct = a->out_mem == RELUX_MEM_DEVICE && !need_conv;
   void* kout;
   const bool piped_out = piped && a->out_mem == RELUX_MEM_HOST;
+  // A small result for host memory: the last kernel writes it to page-locked memory itself (write-only there: the prompt
+  // kernels' TMA stores and the reference kernels keep to device memory)
+  const size_t out_bytes = out_elems * dtype_size(a->out_dtype);
+  const bool by_kernel = a->out_mem == RELUX_MEM_HOST && !piped_out && out_bytes <= Device::kHostOutBytes && p->dev->host_out &&
+                         (need_conv || (a->mode == RELUX_ATTN_FAST && (gqa_stream || (kind == RELUX_POOL_MLA && !mla_prefill_eligible(p, sb, *a)))));
   int slot_out = -1;
   char* out_block = nullptr;   // [kernel output | converted output]
   if (direct) kout = a->out;
+  else if (by_kernel && !need_conv) kout = p->dev->host_out;
   else if (piped_out) {
     PipeSlots& po = p->pipe_out;
     slot_out = (int)(po.next++ % PipeSlots::kSlots);
@@ -563,11 +571,9 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   if (rc) return rc;
   if ((rc = pipe_release(p, p->pipe_in_a, slot_q)) || (rc = pipe_release(p, p->pipe_in_b, slot_qr))) return rc;
   if (!direct) {
-    void* conv = out_block + out_elems * 4;
-    const bool need_conv = a->out_dtype != k_dtype || !out_tm;
     const void* src = kout;
     if (need_conv) {
-      void* dst = (a->out_mem == RELUX_MEM_DEVICE) ? a->out : conv;
+      void* dst = (a->out_mem == RELUX_MEM_DEVICE) ? a->out : by_kernel ? p->dev->host_out : out_block + out_elems * 4;
       rc = convert_layout(p->dev, kout, dst, n, S, H, D, RELUX_DTYPE_F32, a->out_dtype, RELUX_LAYOUT_TOKEN_MAJOR, a->out_layout);
       if (rc) return rc;
       src = dst;
@@ -581,8 +587,11 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
       RELUX_CUDA_TRY(cudaEventRecord(po.freed[slot_out], dev->d2h_stream));
       po.used[slot_out] = true;
       dev->copies_in_flight = true;
+    } else if (by_kernel) {
+      RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
+      memcpy(a->out, p->dev->host_out, out_bytes);
     } else if (a->out_mem == RELUX_MEM_HOST) {
-      RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_elems * dtype_size(a->out_dtype), cudaMemcpyDeviceToHost, p->dev->stream));
+      RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_bytes, cudaMemcpyDeviceToHost, p->dev->stream));
       RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
     }
   }
@@ -675,6 +684,10 @@ API int32_t relux_cuda_device_open(int32_t device_index, relux_device_t* out) {
     (void)cudaGetLastError();   // without copy streams pipelined calls behave like ordinary ones
     d->h2d_stream = d->d2h_stream = nullptr;
   }
+  if (cudaMallocHost(&d->host_out, Device::kHostOutBytes) != cudaSuccess) {
+    (void)cudaGetLastError();   // without it results are copied
+    d->host_out = nullptr;
+  }
   *out = d;
   return RELUX_OK;
 }
@@ -687,6 +700,7 @@ API int32_t relux_cuda_device_close(relux_device_t h) {
     if (g.rc) return g.rc;
     cudaStreamSynchronize(dev->stream);
     if (dev->flush_buf) cudaFree(dev->flush_buf);
+    if (dev->host_out) cudaFreeHost(dev->host_out);
     if (dev->side_stream) { cudaStreamSynchronize(dev->side_stream); cudaStreamDestroy(dev->side_stream); }
     if (dev->ev_fork) cudaEventDestroy(dev->ev_fork);
     if (dev->ev_join) cudaEventDestroy(dev->ev_join);
