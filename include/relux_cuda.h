@@ -208,7 +208,7 @@ int32_t relux_pool_read_rows(relux_pool_t pool, const relux_read_rows_args* args
                                            GEMM (0 = one worker per SM, the split along K chosen per call)                 */
 #define RELUX_TUNE_GQA_PROMPT_PARTIAL_MB 5 /* RELUX_GQA_PROMPT_PARTIAL_MB: partial-buffer budget of a GQA prompt (256)      */
 #define RELUX_TUNE_SEL_CLUSTER 6        /* RELUX_SEL_CLUSTER: cluster size of the selection kernel, 1/2/4/8 (0 = per call) */
-#define RELUX_TUNE_SEL_LOOKAHEAD 7      /* RELUX_SEL_LOOKAHEAD: 0/1 (-1 = per call)                                         */
+#define RELUX_TUNE_SEL_LOOKAHEAD 7      /* RELUX_SEL_LOOKAHEAD: accepted, without effect (one pass per position either way)    */
 #define RELUX_TUNE_SEL_BATCHED 8        /* RELUX_SEL_BATCHED: 0/1 (-1 = per call)                                           */
 #define RELUX_TUNE_GQA_PROMPT_SLICES 9  /* RELUX_GQA_PROMPT_SLICES: 1 = GQA prompts as grid slices of the decode kernel instead
                                            of the tcgen05 prefill kernel                                                  */

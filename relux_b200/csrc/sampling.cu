@@ -31,6 +31,7 @@ namespace {
 constexpr int kSelThreads = 512;
 constexpr int kSelWarps = kSelThreads / 32;
 constexpr int kMaxCluster = 8;
+constexpr int kAhead = 32;
 constexpr int kStatMax = 32;     // batched statistics: two sums and two maxima for each of up to 8 draft positions
 
 struct SelParams {
@@ -61,12 +62,21 @@ struct SelShared {
   alignas(16) uint32_t grp_key[kSelThreads];        // keys of the largest element of every thread (or pair of threads)
   float red_n[2][kStatMax];   // cluster_reduce_n: per-CTA partials, double-buffered like red
   float warp_part_n[kSelWarps][kStatMax];
+  int32_t tok[kAhead];        // what the accept loop needs of the first positions, fetched at once: draft tokens, their logits in
+  float guess[2][kAhead];     // the draft and the target row, and the draws
+  float draw[kAhead + 1];
   float stat[kStatMax];       // batched statistics: of draft position i the sums (draft, target) at 4 i, the maxima at 4 i + 2
 };
 
 __device__ __forceinline__ uint32_t order_key(float x) {
   uint32_t u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// fastexp32 of what is at most 0 (or NaN): a difference to a maximum.  Above 0 its result means nothing.
+__device__ __forceinline__ float fastexp32_below(float x) {
+  const float t = __fadd_rn(__fmul_rn(12102203.0f, x), 1064948224.0f);
+  return x < -87.0f ? 0.0f : __uint_as_float((uint32_t)__float2int_rz(t));
 }
 
 // Everything the passes need to evaluate the reference's probability of one logit on the fly.
@@ -746,9 +756,9 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
     d.topk_key = key;
   }
   float v4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  for_segment(c, row, [&](int, float v) { v4[0] = fmaxf(v4[0], d.scaled(v)); });
+  for_segment(c, row, [&](int, float v) { v4[0] = fmaxf(v4[0], v); });
   cluster_reduce4<1>(c, v4);
-  d.m = v4[0];
+  d.m = d.scaled(v4[0]);   // the division keeps the order: one of it instead of one an element
   d.inv1 = 1.0f;
   float all[kMaxCluster], part = 0.0f;
   for_segment(c, row, [&](int, float v) { part += d.p1(v); });
@@ -761,11 +771,11 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
     uint32_t key = 0;
     bool cut = radix_select<true>(c, row, [&](float v, uint32_t& k, float& w) { w = d.p1(v); k = __float_as_uint(w); }, 0u, topP, &key);
     const float tau = cut ? __uint_as_float(key) : 0.0f;
-    v4[0] = v4[1] = v4[2] = v4[3] = 0.0f;
-    for_segment(c, row, [&](int, float v) { float p = d.p1(v); if (p >= tau) v4[0] += p; });
-    cluster_reduce4<0>(c, v4);
+    part = 0.0f;
+    for_segment(c, row, [&](int, float v) { float p = d.p1(v); if (p >= tau) part += p; });
+    const float kept = segment_sums(c, part, all);
     d.tau = tau;
-    d.inv2 = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
+    d.inv2 = kept > 0.0f ? __fdiv_rn(1.0f, kept) : 1.0f;
   }
   // Dist::p2 drops below tau only when tau > 0; the renormalisation applies whenever the nucleus step ran
   auto p2 = [&](float v) { float p = d.p1(v); if (nucleus) p = p < d.tau ? 0.0f : __fmul_rn(p, d.inv2); return p; };
@@ -783,8 +793,8 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
     d.inv3 = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
   }
   auto p3 = [&](float v, float) { float p = p2(v); if (minp) p = p < d.minp_thr ? 0.0f : __fmul_rn(p, d.inv3); return p; };
-  float factor = d.inv1;   // without a filter behind the sum, its segments are the search's
-  if (nucleus || minp) {
+  float factor = nucleus ? d.inv2 : d.inv1;   // the segments of the last normalisation are the search's
+  if (minp) {
     factor = 1.0f;
     part = 0.0f;
     for_segment(c, row, [&](int, float v) { part += p3(v, 0.0f); });
@@ -825,33 +835,59 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
   // be another.
   auto drow_of = [&](int i) { return prm.draft_logits + ((size_t)b * k + i) * V; };
   auto trow_of = [&](int i) { return prm.target_logits + ((size_t)b * (k + 1) + i) * V; };
+  auto fetch = [&](int i, int32_t& tok, float& gd, float& gt) {   // tok as it is, possibly outside the vocabulary
+    if (i < kAhead) {
+      tok = sh.tok[i];
+      gd = sh.guess[0][i];
+      gt = sh.guess[1][i];
+    } else {
+      tok = prm.draft_tokens[(size_t)b * k + i];
+      const int j = min(max(tok, 0), V - 1);
+      gd = __ldg(drow_of(i) + j);
+      gt = __ldg(trow_of(i) + j);
+    }
+  };
+  if ((int)threadIdx.x < min(k, kAhead)) {
+    const int i = threadIdx.x, tok = prm.draft_tokens[(size_t)b * k + i], j = min(max(tok, 0), V - 1);
+    sh.tok[i] = tok;
+    sh.guess[0][i] = __ldg(drow_of(i) + j);
+    sh.guess[1][i] = __ldg(trow_of(i) + j);
+  } else if (threadIdx.x >= 64 && (int)threadIdx.x - 64 <= min(k, kAhead)) {
+    sh.draw[threadIdx.x - 64] = draws[threadIdx.x - 64];
+  }
+  __syncthreads();
+  auto next_draw = [&]() {
+    const int j = used++;
+    return j <= kAhead ? sh.draw[j] : draws[j];
+  };
   auto pair_pass = [&](int i, float& sd, float& st, float& md, float& mt) {
-    const float *drow = drow_of(i), *trow = trow_of(i);
-    const int tok = min(max(prm.draft_tokens[(size_t)b * k + i], 0), V - 1);
-    const float gd = __ldg(drow + tok), gt = __ldg(trow + tok);
+    int32_t tok;
+    float gd, gt;
+    fetch(i, tok, gd, gt);
     float a = 0.0f, t = 0.0f, ma = -INFINITY, mb = -INFINITY;
-    for_segment2(c, drow, trow, [&](int, float dv, float tv) {
+    for_segment2(c, drow_of(i), trow_of(i), [&](int, float dv, float tv) {
       ma = fmaxf(ma, dv);
       mb = fmaxf(mb, tv);
-      a += fastexp32_ref(__fsub_rn(dv, gd));
-      t += fastexp32_ref(__fsub_rn(tv, gt));
+      a += fastexp32_below(__fsub_rn(dv, gd));
+      t += fastexp32_below(__fsub_rn(tv, gt));
     });
     sd = a; st = t; md = ma; mt = mb;
   };
-  // the sums again where the guess was not the maximum; whether there is anything to do
+  // the sums again where the guess was not the maximum; which they are (bit 0: draft, bit 1: target)
   auto pair_again = [&](int i, float md, float mt, float& sd, float& st) {
-    const float *drow = drow_of(i), *trow = trow_of(i);
-    const int tok = min(max(prm.draft_tokens[(size_t)b * k + i], 0), V - 1);
-    const bool bad_d = __ldg(drow + tok) != md, bad_t = __ldg(trow + tok) != mt;
+    int32_t tok;
+    float gd, gt;
+    fetch(i, tok, gd, gt);
+    const int bad = (gd != md ? 1 : 0) | (gt != mt ? 2 : 0);
     float a = 0.0f, t = 0.0f;
-    if (bad_d && bad_t)
-      for_segment2(c, drow, trow, [&](int, float dv, float tv) { a += fastexp32_ref(__fsub_rn(dv, md)); t += fastexp32_ref(__fsub_rn(tv, mt)); });
-    else if (bad_d)
-      for_segment(c, drow, [&](int, float dv) { a += fastexp32_ref(__fsub_rn(dv, md)); });
-    else if (bad_t)
-      for_segment(c, trow, [&](int, float tv) { t += fastexp32_ref(__fsub_rn(tv, mt)); });
+    if (bad == 3)
+      for_segment2(c, drow_of(i), trow_of(i), [&](int, float dv, float tv) { a += fastexp32_below(__fsub_rn(dv, md)); t += fastexp32_below(__fsub_rn(tv, mt)); });
+    else if (bad == 1)
+      for_segment(c, drow_of(i), [&](int, float dv) { a += fastexp32_below(__fsub_rn(dv, md)); });
+    else if (bad == 2)
+      for_segment(c, trow_of(i), [&](int, float tv) { t += fastexp32_below(__fsub_rn(tv, mt)); });
     sd = a; st = t;
-    return (bad_d ? 1 : 0) | (bad_t ? 2 : 0);
+    return bad;
   };
   // Few sequences: the chain's length is what costs, not the bytes.  The rows of ALL draft positions are read in one stage
   // (and the sums to be made again in a second), so the accept loop below runs without a pass of its own per position (rows
@@ -880,7 +916,9 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
   for (int i = 0; i < k && !done; i++) {
     const float* drow = drow_of(i);
     const float* trow = trow_of(i);
-    const int tok = prm.draft_tokens[(size_t)b * k + i];
+    int32_t tok;
+    float tok_d, tok_t;   // the token's logits
+    fetch(i, tok, tok_d, tok_t);
     if (tok < 0 || tok >= V) {   // uniform over the cluster: every thread reads the same token
       if (writer) { set_status(prm.status, RELUX_ERR_INVALID_ARG); *out_tok = -1; }
       n_acc = -1;
@@ -908,11 +946,11 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     }
     const float invd = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
     const float invt = v4[1] > 0.0f ? __fdiv_rn(1.0f, v4[1]) : 1.0f;
-    const float dP = __fmul_rn(fastexp32_ref(__fsub_rn(__ldg(drow + tok), md)), invd);
-    const float tP = __fmul_rn(fastexp32_ref(__fsub_rn(__ldg(trow + tok), mt)), invt);
+    const float dP = __fmul_rn(fastexp32_ref(__fsub_rn(tok_d, md)), invd);
+    const float tP = __fmul_rn(fastexp32_ref(__fsub_rn(tok_t, mt)), invt);
     float ap = __fdiv_rn(tP, dP > 1e-10f ? dP : 1e-10f);
     if (ap > 1.0f) ap = 1.0f;
-    const float u = draws[used++];
+    const float u = next_draw();
     if (u < ap) continue;
     // rejected at i: resample from norm(max(0, p_target - p_draft))   speculative.go:256-295
     auto adj = [&](float tv, float dv) {
@@ -924,7 +962,7 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     float all[kMaxCluster], part = 0.0f;
     for_segment2(c, drow, trow, [&](int, float dv, float tv) { part += adj(tv, dv); });
     const float sum = segment_sums(c, part, all);
-    const float r = draws[used++];
+    const float r = next_draw();
     if (sum > 0.0f) {
       const float inv = __fdiv_rn(1.0f, sum);
       cdf_search(c, trow, drow, [&](float tv, float dv) { return __fmul_rn(adj(tv, dv), inv); }, r, 0, out_tok, all, inv);
@@ -938,7 +976,7 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     n_acc = i;
     done = true;
   }
-  if (!done) sample_row(c, prm, prm.target_logits + ((size_t)b * (k + 1) + k) * V, draws[used++], out_tok);
+  if (!done) sample_row(c, prm, prm.target_logits + ((size_t)b * (k + 1) + k) * V, next_draw(), out_tok);
   if (writer && prm.n_accepted) prm.n_accepted[b] = n_acc;
   cl.sync();   // no CTA leaves while another may still read its exchange buffers
   if (threadIdx.x == 0) stamp_end(prm.time);
