@@ -82,7 +82,9 @@ struct Piece {
   int32_t i, kvh, us, pb, pe, pages;   // sequence of the call, kv head, first unit of the stream, logical pages [pb, pe) of `pages`
 };
 
-// RS: rows of one warp's state in shared memory (16: all of MT = 1, a warp's half for MT = 2).  The number
+// RS: rows of one warp's state in shared memory (8 or 16: all of MT = 1, a warp's half for MT = 2).  Up to 8 rows there is room
+// for two pieces' states, so the consumers go on while the finishers read: streams of a page or two are as fast as the
+// finishers then, not as both in turn.  The number
 // of stages is even, so that with alternating pages a stage belongs to one group of warps for good: a group that waited
 // on a stage it had skipped for a lap would take that lap's phase for its own (mbarrier phases are told apart by parity).
 // Four stages, 128 KB in flight per SM: with six, the SMs' shares of the bandwidth drift apart (28 to 41 us for equal
@@ -94,9 +96,11 @@ struct StreamSmem {
   static_assert(kStages % 2 == 0, "see above");
   static constexpr int kQBytes = 16 * MT * kGqaQStride * 2;
   static constexpr int kQ = kStages * kGqaStageBytes;                       // kQBufs buffers, pieces in turn
-  static constexpr int kState = kQ + kQBufs * kQBytes;                           // [8 warps][RS][kGqaStateStride] f32
-  static constexpr int kBar = kState + kConsumers * RS * kGqaStateStride * 4;
-  static constexpr int kTotal = 1024 + kBar + (2 * kStages + kQBufs + 4) * 8 + 16;
+  static constexpr int kState = kQ + kQBufs * kQBytes;                           // [kStateBufs][8 warps][RS][kGqaStateStride] f32
+  static constexpr int kStateBufs = RS == 8 ? 2 : 1;
+  static constexpr int kStateFloats = kConsumers * RS * kGqaStateStride;
+  static constexpr int kBar = kState + kStateBufs * kStateFloats * 4;
+  static constexpr int kTotal = 1024 + kBar + (2 * kStages + kQBufs + 6) * 8 + 16;
   static_assert(kTotal <= 232448, "more shared memory than a CTA may use");
 };
 
@@ -113,11 +117,12 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
   uint64_t* full = (uint64_t*)(smem + SM::kBar);
   uint64_t* empty = full + kStages;
   uint64_t* q_full = empty + kStages;          // [kQBufs]: the queries of piece n are in buffer n % kQBufs
-  uint64_t* state_full = q_full + kQBufs;           // the consumers' states of a piece are in shared memory
-  uint64_t* state_empty = state_full + 1;      // and have been read
-  uint64_t* merge_go = state_empty + 2;        // the finishers know which rows are to be merged here
-  uint32_t* merge_flags = (uint32_t*)(state_empty + 3);   // [kFinishers], and the warps that are done with the merge
-  uint64_t* rows_done = state_empty + 1;       // the new rows of this CTA's pieces are in their pages
+  constexpr int kStateBufs = SM::kStateBufs;
+  uint64_t* state_full = q_full + kQBufs;      // [2]: the consumers' states of piece n are in buffer n % kStateBufs
+  uint64_t* state_empty = state_full + 2;      // [2]: and have been read
+  uint64_t* rows_done = state_empty + 2;       // the new rows of this CTA's pieces are in their pages
+  uint64_t* merge_go = rows_done + 1;          // the finishers know which rows are to be merged here
+  uint32_t* merge_flags = (uint32_t*)(merge_go + 1);   // [kFinishers], and the warps that are done with the merge
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   auto seq_of = [&](int i) -> GqaSeq { return c.seqs ? c.seqs[i] : prm.seqs[i]; };
@@ -166,9 +171,11 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
       mbar_init(&empty[s], MT == 1 ? 4 : 8);   // the warps that read the page
     }
     for (int b = 0; b < kQBufs; b++) mbar_init(&q_full[b], kFinishers);
-    mbar_init(state_full, kConsumers);
-    mbar_init(state_empty, kFinishers);
-    mbar_init(rows_done, kFinishers);
+    for (int b = 0; b < kStateBufs; b++) {
+      mbar_init(&state_full[b], kConsumers);
+      mbar_init(&state_empty[b], kFinishers);
+    }
+    mbar_init(rows_done, kConsumers + kFinishers);
     mbar_init(merge_go, kFinishers);
     merge_flags[kFinishers] = 0;
     fence_mbar_init();
@@ -254,12 +261,50 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     if (c.out_bf16) *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(c.out) + off) = make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
     else *reinterpret_cast<float4*>(reinterpret_cast<float*>(c.out) + off) = o;
   };
+  // All new rows of this CTA's pieces, a piece per warp in turn: 16 lanes write a K row, 16 the V row, 16 bytes each.  By every
+  // warp that would wait for the first page now: the loads of a stream's last page wait for all of them, and three warps took
+  // 5 us over the pieces of a range of short streams.  (Written by the producer when it reached their page, every short stream
+  // cost it two memory latencies.)
+  auto write_new_rows = [&]() {
+    if (!c.k_new) return;
+    int k = 0;
+    for (Piece q = p; q.us < u_end; q = next_piece(q), k++) {
+      if (k % (kConsumers + kFinishers) != warp) continue;
+      const GqaSeq sq = seq_of(q.i);
+      const int n_new = (c.seqs ? c.seqs[q.i + 1].row0 : prm.seqs[q.i + 1].row0) - sq.row0;
+      const int v = lane >> 4, ch = (lane & 15) * 8;
+      const void* from = v ? c.v_new : c.k_new;
+      const int r_hi = min(sq.len0 + n_new, q.pe * kGqaPageTok);
+      for (int pos = max(sq.len0, q.pb * kGqaPageTok); pos < r_hi; pos++) {
+        const int32_t pg = __ldg(c.table + (size_t)sq.seq * c.table_stride + pos / kGqaPageTok);
+        const int idx = pos - sq.len0;
+        const size_t src = c.head_major ? (size_t)sq.row0 * c.Hkv * kGqaD + ((size_t)q.kvh * n_new + idx) * kGqaD + ch
+                                        : ((size_t)(sq.row0 + idx) * c.Hkv + q.kvh) * kGqaD + ch;
+        uint4 w;
+        if (c.new_f32) {
+          const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(from) + src);
+          const float4 a = s[0], b = s[1];
+          w = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+        } else {
+          w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(from) + src);
+        }
+        if (pg < 0 || pg >= c.num_pages) continue;   // reported by the producer
+        uint16_t* dst = (v ? c.v_base : c.k_base) + (((size_t)pg * c.Hkv + q.kvh) * kGqaPageTok + (pos & (kGqaPageTok - 1))) * kGqaD + ch;
+        *reinterpret_cast<uint4*>(dst) = w;
+      }
+    }
+    fence_proxy_async_all();   // the rows are read back by the producer's TMA loads
+    __syncwarp();
+    if (lane == 0) mbar_arrive(rows_done);
+  };
   const Piece p_first = p;
   Piece p_last = p;
   if (warp < kConsumers) {
     // ---------------- consumers ----------------
     const int grp = warp >> 2, tb = (warp & 3) * 16;   // this warp's tokens inside a page
     const int row0 = MT == 1 ? 0 : grp * 16;           // first query row of this warp
+    chain_wait();
+    write_new_rows();
     int g = 0, n = 0;
     bool alive = true;
     for (; p.us < u_end; p_last = p, p = next_piece(p), n++) {
@@ -282,10 +327,11 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
           if (lane == 0) mbar_arrive(&empty[st]);
         }
       }
-      if (n > 0 && alive) alive = timed_wait(state_empty, (n - 1) & 1);
-      gqa_store_state<1>(state, mb + (size_t)warp * RS * kGqaStateStride, RS, lane, alive);
+      const int sb = n % kStateBufs;
+      if (n >= kStateBufs && alive) alive = timed_wait(&state_empty[sb], (n / kStateBufs - 1) & 1);
+      gqa_store_state<1>(state, mb + sb * SM::kStateFloats + (size_t)warp * RS * kGqaStateStride, RS, lane, alive);
       __syncwarp();
-      if (lane == 0) mbar_arrive(state_full);
+      if (lane == 0) mbar_arrive(&state_full[sb]);
     }
   } else {
     // ---------------- finishers ----------------
@@ -293,19 +339,30 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     // Q rows of a piece's kv head as bf16 into buffer b; row r = s * g + head in group
     auto load_queries = [&](const Piece& q, int b) {
       uint16_t* qs = reinterpret_cast<uint16_t*>(smem + SM::kQ + b * SM::kQBytes);
-      for (int e = ft; e < c.R * (kGqaD / 8); e += 32 * kFinishers) {
-        const int r = e >> 4, ch = (e & 15) * 8;
-        const int s = r / c.g, hq = r - s * c.g;
-        const size_t off = (((size_t)q.i * c.S + s) * c.H + (size_t)q.kvh * c.g + hq) * kGqaD + ch;
-        uint4 w;
-        if (c.q_bf16) {
-          w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(c.q) + off);
-        } else {
-          const float4* f = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(c.q) + off);
-          const float4 a = f[0], b2 = f[1];
-          w = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b2.x, b2.y), pack_bf16x2(b2.z, b2.w));
+      constexpr int kAtOnce = 3;   // loads in flight per thread
+      const int total = c.R * (kGqaD / 8);
+      for (int e0 = ft; e0 < total; e0 += kAtOnce * 32 * kFinishers) {
+        uint4 w[kAtOnce];
+#pragma unroll
+        for (int k = 0; k < kAtOnce; k++) {
+          const int e = e0 + k * 32 * kFinishers;
+          if (e >= total) break;
+          const int r = e >> 4, ch = (e & 15) * 8;
+          const int s = r / c.g, hq = r - s * c.g;
+          const size_t off = (((size_t)q.i * c.S + s) * c.H + (size_t)q.kvh * c.g + hq) * kGqaD + ch;
+          if (c.q_bf16) {
+            w[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(c.q) + off);
+          } else {
+            const float4* f = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(c.q) + off);
+            const float4 a = f[0], b2 = f[1];
+            w[k] = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b2.x, b2.y), pack_bf16x2(b2.z, b2.w));
+          }
         }
-        *reinterpret_cast<uint4*>(qs + r * kGqaQStride + ch) = w;
+#pragma unroll
+        for (int k = 0; k < kAtOnce; k++) {
+          const int e = e0 + k * 32 * kFinishers;
+          if (e < total) *reinterpret_cast<uint4*>(qs + (e >> 4) * kGqaQStride + (e & 15) * 8) = w[k];
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&q_full[b]);
@@ -314,40 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
     if (ft == 0) stamp_begin(c.time);
     Piece p_ahead = p;   // the next piece whose queries have not been requested
     for (int b = 0; b < 2 && p_ahead.us < u_end; b++, p_ahead = next_piece(p_ahead)) load_queries(p_ahead, b);
-    if (c.k_new) {
-      // All new rows of this CTA's pieces, a piece per warp in turn: 16 lanes write a K row, 16 the V row, 16 bytes each.
-      // (Written by the producer when it reached their page, every short stream cost it two memory latencies.)
-      int k = 0;
-      for (Piece q = p; q.us < u_end; q = next_piece(q), k++) {
-        if (k % kFinishers == fw) {
-          const GqaSeq sq = seq_of(q.i);
-          const int n_new = (c.seqs ? c.seqs[q.i + 1].row0 : prm.seqs[q.i + 1].row0) - sq.row0;
-          const int v = lane >> 4, ch = (lane & 15) * 8;
-          const void* from = v ? c.v_new : c.k_new;
-          const int r_hi = min(sq.len0 + n_new, q.pe * kGqaPageTok);
-          for (int pos = max(sq.len0, q.pb * kGqaPageTok); pos < r_hi; pos++) {
-            const int32_t pg = __ldg(c.table + (size_t)sq.seq * c.table_stride + pos / kGqaPageTok);
-            if (pg < 0 || pg >= c.num_pages) continue;   // reported by the producer
-            const int idx = pos - sq.len0;
-            const size_t src = c.head_major ? (size_t)sq.row0 * c.Hkv * kGqaD + ((size_t)q.kvh * n_new + idx) * kGqaD + ch
-                                            : ((size_t)(sq.row0 + idx) * c.Hkv + q.kvh) * kGqaD + ch;
-            uint4 w;
-            if (c.new_f32) {
-              const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(from) + src);
-              const float4 a = s[0], b = s[1];
-              w = make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
-            } else {
-              w = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(from) + src);
-            }
-            uint16_t* dst = (v ? c.v_base : c.k_base) + (((size_t)pg * c.Hkv + q.kvh) * kGqaPageTok + (pos & (kGqaPageTok - 1))) * kGqaD + ch;
-            *reinterpret_cast<uint4*>(dst) = w;
-          }
-        }
-      }
-      fence_proxy_async_all();   // the rows are read back by the producer's TMA loads
-      __syncwarp();
-      if (lane == 0) mbar_arrive(rows_done);
-    }
+    write_new_rows();
     // The pieces of a stream are one each of the workers w0 .. w1, and a row belongs to the same finisher warp in all of
     // them: each warp counts for itself (no block-wide barrier), and the warp that counts last merges its own rows of all of
     // them.  (The fence takes up to 10 us under full load; the query buffers cover it.)
@@ -370,41 +394,67 @@ __global__ void __launch_bounds__(kThreads, 1) gqa_stream_kernel(const __grid_co
         load_queries(p_ahead, (n + 2) % kQBufs);
         p_ahead = next_piece(p_ahead);
       }
-      if (alive) alive = timed_wait(state_full, n & 1);
+      if (alive) alive = timed_wait(&state_full[n % kStateBufs], (n / kStateBufs) & 1);
       // combine the warps' states: a warp per row, four dims per lane
       const bool whole = p.pb == 0 && p.pe == p.pages;
       const int slot = 2 * (int)blockIdx.x + (p.us + p.pb == u_begin ? 0 : 1);
       constexpr int kW = MT == 1 ? 8 : 4;   // warps that hold a state of a row
+      // two rows at a time: a row is a chain of shuffles, about 1.1 us whatever its loads
+      const float* states = mb + (n % kStateBufs) * SM::kStateFloats;
 #pragma unroll 1
-      for (int r = fw; r < c.R; r += kFinishers) {
-        const float* src = mb + ((size_t)(MT == 1 ? 0 : (r >> 4) * 4) * RS + (MT == 1 ? r : (r & 15))) * kGqaStateStride;
-        // lane k (mod kW) weighs warp k's state
-        const float2 ml = *reinterpret_cast<const float2*>(src + (size_t)(lane & (kW - 1)) * RS * kGqaStateStride + kGqaD);
-        float M = ml.x;
+      for (int r0 = fw; r0 < c.R; r0 += 2 * kFinishers) {
+        const int r1 = r0 + kFinishers < c.R ? r0 + kFinishers : r0;   // the same row twice where there is no second
+        const float* src[2];
+        float M[2], L[2], wgt[2];
+        float4 o[2];
 #pragma unroll
-        for (int i = 1; i < kW; i <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, i));
-        const float wgt = (ml.x == -INFINITY) ? 0.f : gqa_ex2(ml.x - M);
-        float L = ml.y * wgt;
-#pragma unroll
-        for (int i = 1; i < kW; i <<= 1) L += __shfl_xor_sync(0xffffffffu, L, i);
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < kW; w++) {
-          const float f = __shfl_sync(0xffffffffu, wgt, w);
-          const float4 x = *reinterpret_cast<const float4*>(src + (size_t)w * RS * kGqaStateStride + lane * 4);
-          o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+        for (int k = 0; k < 2; k++) {
+          const int r = k ? r1 : r0;
+          src[k] = states + ((size_t)(MT == 1 ? 0 : (r >> 4) * 4) * RS + (MT == 1 ? r : (r & 15))) * kGqaStateStride;
+          // lane j (mod kW) weighs warp j's state
+          const float2 ml = *reinterpret_cast<const float2*>(src[k] + (size_t)(lane & (kW - 1)) * RS * kGqaStateStride + kGqaD);
+          M[k] = ml.x;
+          L[k] = ml.y;
+          wgt[k] = ml.x;
+          o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (whole) {
-          const float inv = (L > 0.f) ? 1.f / L : 0.f;
-          store_out(p, r, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
-        } else {
-          const size_t row = (size_t)slot * c.R + r;
-          __stcg(reinterpret_cast<float4*>(c.part_o + row * kGqaD + lane * 4), o);
-          if (lane == 0) __stcg(reinterpret_cast<float2*>(c.part_ml + row * 2), make_float2(M, L));
+#pragma unroll
+        for (int i = 1; i < kW; i <<= 1)
+#pragma unroll
+          for (int k = 0; k < 2; k++) M[k] = fmaxf(M[k], __shfl_xor_sync(0xffffffffu, M[k], i));
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          wgt[k] = wgt[k] == -INFINITY ? 0.f : gqa_ex2(wgt[k] - M[k]);
+          L[k] *= wgt[k];
+        }
+#pragma unroll
+        for (int i = 1; i < kW; i <<= 1)
+#pragma unroll
+          for (int k = 0; k < 2; k++) L[k] += __shfl_xor_sync(0xffffffffu, L[k], i);
+#pragma unroll
+        for (int w = 0; w < kW; w++)
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const float f = __shfl_sync(0xffffffffu, wgt[k], w);
+            const float4 x = *reinterpret_cast<const float4*>(src[k] + (size_t)w * RS * kGqaStateStride + lane * 4);
+            o[k].x = fmaf(x.x, f, o[k].x); o[k].y = fmaf(x.y, f, o[k].y); o[k].z = fmaf(x.z, f, o[k].z); o[k].w = fmaf(x.w, f, o[k].w);
+          }
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const int r = k ? r1 : r0;
+          if (k && r1 == r0) break;
+          if (whole) {
+            const float inv = (L[k] > 0.f) ? 1.f / L[k] : 0.f;
+            store_out(p, r, make_float4(o[k].x * inv, o[k].y * inv, o[k].z * inv, o[k].w * inv));
+          } else {
+            const size_t row = (size_t)slot * c.R + r;
+            __stcg(reinterpret_cast<float4*>(c.part_o + row * kGqaD + lane * 4), o[k]);
+            if (lane == 0) __stcg(reinterpret_cast<float2*>(c.part_ml + row * 2), make_float2(M[k], L[k]));
+          }
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(state_empty);
+      if (lane == 0) mbar_arrive(&state_empty[n % kStateBufs]);
       if (!whole && publish(p)) due |= p.us + p.pb == p_first.us + p_first.pb ? 1u : 2u;
     }
     if (lane == 0) {
@@ -482,6 +532,7 @@ int32_t launch(Pool* p, const GqaStreamCommon& c, const GqaSeq* seqs, int worker
 }
 template <int N>
 int32_t launch_rows(Pool* p, const GqaStreamCommon& c, const GqaSeq* seqs, int workers) {
+  if (c.R <= 8) return launch<1, 8, N>(p, c, seqs, workers);
   if (c.R <= 16) return launch<1, 16, N>(p, c, seqs, workers);
   return launch<2, 16, N>(p, c, seqs, workers);
 }
