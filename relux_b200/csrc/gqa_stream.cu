@@ -74,10 +74,11 @@ struct GqaStreamParams {
   GqaSeq seqs[N + 1];
 };
 
-// A stream (sequence, kv head) is its pages and kStreamUnits units of fixed cost: what a piece costs its consumers beyond
-// its pages (queries, states) is about a page's time.  Without them the workers with the shortest streams finished last
-// (47 against 39 us at 32 sequences of 100 to 3000 tokens).
-constexpr int kStreamUnits = 1;
+// A stream (sequence, kv head) is its pages and kStreamUnits units of fixed cost: what a piece costs its consumers and finishers
+// beyond its pages (queries, states, the rows' sums), 2-3 us against 0.74 us a page.  Measured with 0, 1, 4 and 6 units: 32
+// sequences of 100 to 3000 tokens 47, 45.4, 44.8, 44.8 us; 100 of 22 to 700 tokens -, 45.3, 36.3, 36.3; 64 of 50 to 1500 -, 46.9,
+// 44.2, 44.5.  (Too few, and the workers with the shortest streams finish last.)
+constexpr int kStreamUnits = 4;
 struct Piece {
   int32_t i, kvh, us, pb, pe, pages;   // sequence of the call, kv head, first unit of the stream, logical pages [pb, pe) of `pages`
 };
