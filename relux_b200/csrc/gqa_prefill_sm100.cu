@@ -95,11 +95,9 @@ struct Plan {
   static constexpr int kSmemTotal = kSmemBar + 3072;
   static_assert(kSmemTotal <= 232448, "more shared memory than a CTA may use");
 };
-constexpr int kSplit = 2;                                     // threads per query row: each takes 128 / kSplit keys and output dims
-constexpr int kCols = 128 / kSplit;
-constexpr int kSoftmaxWarps = 4 * kSplit;
+constexpr int kSoftmaxWarps = 8;                              // 16 query rows each
 constexpr int kEpiWarps = 4;                                  // read-out warps: one per TMEM lane quarter
-constexpr int kSoftmaxThreads = 32 * kSoftmaxWarps, kThreads = kSoftmaxThreads + 64 + 32 * kEpiWarps;
+constexpr int kThreads = 32 * kSoftmaxWarps + 64 + 32 * kEpiWarps;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemS = 0, kTmemO = 256;                  // S(g) at kTmemS + 128 (g & 1); O of item n at kTmemO + 128 (n & 1)
 constexpr float kRescaleThreshold = 8.0f;
@@ -109,12 +107,10 @@ constexpr float kRescaleThreshold = 8.0f;
 constexpr int kPolyPairsOf8 = RELUX_PREFILL_POLY_PAIRS;   // score pairs out of every eight whose exponential runs on the FMA pipe
 
 struct Bars {
-  uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full, pv_done;
+  uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full[2], pv_done;
   uint64_t o_full[2], o_empty[2], l_full, l_empty, drain;
   uint32_t tmem_base;
   volatile int32_t abort_flag;
-  float rowmax[2][kSplit][128];   // [tile parity][key slice][row]; at the end of an item the buffer of the tile that follows
-                                  // carries the row sums of the key slices from one slice's thread to the other's
   float lsum[128];                // an item's row sums, handed to the read-out warps
 };
 static_assert(sizeof(Bars) <= 3072, "barrier block too large");
@@ -145,69 +141,93 @@ struct PrefillParams {
 // long member first.  Couples are numbered stream by stream and worker w takes couples w, w + W, ...: every worker gets
 // the same amount of work, and the workers that run at the same time read the keys and values of a few streams only,
 // which then come out of L2 (with 128 heads and long prompts the streams of one call are far larger than L2 together).
-struct Cursor {
-  int32_t c, m;   // couple, member (0: pair n_pairs - 1 - k, 1: pair k, for couple k of its stream)
-};
-__device__ __forceinline__ bool cursor_valid(const PrefillParams& prm, Cursor u) { return u.c < prm.n_couples; }
-__device__ __forceinline__ Cursor cursor_next(const PrefillParams& prm, Cursor u, int n_workers) {
-  const int k = u.c % prm.n_half;
-  if (u.m == 0 && prm.n_pairs - 1 - k != k) return Cursor{u.c, 1};
-  return Cursor{u.c + n_workers, 0};
-}
-
-// One item as every warp of the pair derives it from the cursor.
 struct Item {
-  int32_t bi, seq, hk, pair;
+  int32_t bi, seq, hk, pair;      // sequence of the call, sequence of the pool, kv head, block pair
   int32_t T, ntiles, last_slot, base;
 };
+// A worker's items in order, as every warp of the pair derives them.  Between two items lies no division (the couple's place is
+// advanced by the digits of the step) and no load that is waited for (lengths are loaded an item ahead): together they had the
+// softmax warps pause 1300 clocks there, most of a tile's time.
 template <bool kMla>
-__device__ __forceinline__ Item item_of(const PrefillParams& prm, Cursor u) {
+struct Walk {
+  const PrefillParams& prm;
+  int32_t step_k, step_hk, step_bi;                // the number of workers, in digits of (couples per stream, kv heads)
+  int32_t k, hk, bi, m;                            // couple of the stream, stream, and member (0: pair n_pairs - 1 - k, 1: pair k)
+  int32_t next_seq, next_len, next_base;           // of the next item: nothing is computed from these before it begins
   Item it;
-  const int stream = u.c / prm.n_half, k = u.c % prm.n_half;
-  it.pair = u.m ? k : prm.n_pairs - 1 - k;
-  it.hk = stream % prm.Hkv;
-  it.bi = stream / prm.Hkv;
-  it.seq = prm.seq_ids ? __ldg(prm.seq_ids + it.bi) : it.bi;
-  it.T = load_chained(prm.len + it.seq) + prm.extra;
-  // keys the PAIR needs: all T without the mask, else up to the position of its last real token
-  const int last_tok = min(prm.S, (2 * it.pair + 2) * prm.bq) - 1;
-  const int kmax = prm.causal ? (it.T - prm.S + last_tok + 1) : it.T;
-  it.ntiles = max(1, (kmax + kTile - 1) / kTile);
-  it.last_slot = (it.T + kPage - 1) / kPage - 1;   // last page slot of the sequence that holds a row
-  it.base = 0;
-  if constexpr (kMla) it.base = load_chained(prm.seq_base + it.bi);
-  return it;
-}
-
-// exp2(score * scale - max) for this thread's kCols scores of one row: bf16 P values, two per 32-bit word in key order,
-// into pw; returns the two partial row sums.  (The caller stores pw to tensor memory: that store is warp-collective and
-// this function is called under a per-row condition.)
-template <bool kPoly>
-__device__ __forceinline__ uint64_t exp_rows(const uint32_t (&sv)[kCols], uint64_t scale2, uint64_t neg_m2, uint32_t (&pw)[kCols / 2]) {
-  static_assert(kCols == 64, "one 32-column store per thread");
-  uint64_t ps2 = pack2(0.f, 0.f);
-#pragma unroll
-  for (int q2 = 0; q2 < kCols / 32; q2++) {
-    uint32_t* pk = pw + 16 * q2;
-#pragma unroll
-    for (int c = 0; c < 32; c += 2) {
-      const uint64_t x2 = fma2(pack2(__uint_as_float(sv[q2 * 32 + c]), __uint_as_float(sv[q2 * 32 + c + 1])), scale2, neg_m2);
-      uint64_t p2;
-      if (kPoly && ((c >> 1) & 7) < kPolyPairsOf8) {
-        p2 = ex2_poly2(x2);
-      } else {
-        float x0, x1;
-        unpack2(x2, x0, x1);
-        p2 = pack2(ex2_approx(x0), ex2_approx(x1));
-      }
-      ps2 = add2(ps2, p2);
-      float p0, p1;
-      unpack2(p2, p0, p1);
-      __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
-      pk[c >> 1] = *reinterpret_cast<uint32_t*>(&b2);
-    }
+  int n;
+  __device__ __forceinline__ Walk(const PrefillParams& p, int worker, int workers) : prm(p), m(0), n(0) {
+    step_k = workers % p.n_half;
+    step_hk = workers / p.n_half % p.Hkv;
+    step_bi = workers / p.n_half / p.Hkv;
+    k = worker % p.n_half;
+    hk = worker / p.n_half % p.Hkv;
+    bi = worker / p.n_half / p.Hkv;
+    load();
+    enter();
   }
-  return ps2;
+  __device__ __forceinline__ bool valid() const { return bi < prm.n_seqs; }
+  __device__ __forceinline__ void load() {   // for the item the place points to
+    if (!valid()) return;
+    next_seq = prm.seq_ids ? __ldg(prm.seq_ids + bi) : bi;
+    next_len = load_chained(prm.len + next_seq);
+    next_base = kMla ? load_chained(prm.seq_base + bi) : 0;
+  }
+  __device__ __forceinline__ void enter() {   // takes the item at the place, and moves the place on
+    it.bi = bi;
+    it.hk = hk;
+    it.pair = m ? k : prm.n_pairs - 1 - k;
+    it.seq = next_seq;
+    it.base = next_base;
+    it.T = next_len + prm.extra;
+    // keys the PAIR needs: all T without the mask, else up to the position of its last real token
+    const int last_tok = min(prm.S, (2 * it.pair + 2) * prm.bq) - 1;
+    const int kmax = prm.causal ? (it.T - prm.S + last_tok + 1) : it.T;
+    it.ntiles = max(1, (kmax + kTile - 1) / kTile);
+    it.last_slot = (it.T + kPage - 1) / kPage - 1;   // last page slot of the sequence that holds a row
+    if (m == 0 && prm.n_pairs - 1 - k != k) {
+      m = 1;
+    } else {
+      m = 0;
+      k += step_k;
+      hk += step_hk;
+      bi += step_bi;
+      if (k >= prm.n_half) { k -= prm.n_half; hk++; }
+      if (hk >= prm.Hkv) { hk -= prm.Hkv; bi++; }
+    }
+    more = valid();
+    load();
+  }
+  bool more;                                       // the place points to an item
+  __device__ __forceinline__ bool next() {         // false: that was the last item
+    n++;
+    if (!more) return false;
+    enter();
+    return true;
+  }
+};
+
+// exp2(score * scale - max) for a thread's 2 x 32 scores of a tile (tmem_ld_16x256b_x16: pairs of neighbouring keys of rows a and
+// b in turn): bf16 P values in the order of tmem_st_16x128b_x16; the partial row sums are added to ps2.
+template <bool kPoly>
+__device__ __forceinline__ void exp_quads(const uint32_t (&sv)[64], uint64_t scale2, const uint64_t (&neg_m2)[2], uint32_t (&pw)[32], uint64_t (&ps2)[2]) {
+#pragma unroll
+  for (int i = 0; i < 32; i++) {   // pair i: row i & 1
+    const uint64_t x2 = fma2(pack2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, neg_m2[i & 1]);
+    uint64_t p2;
+    if (kPoly && (i & 7) < kPolyPairsOf8) {
+      p2 = ex2_poly2(x2);
+    } else {
+      float x0, x1;
+      unpack2(x2, x0, x1);
+      p2 = pack2(ex2_approx(x0), ex2_approx(x1));
+    }
+    ps2[i & 1] = add2(ps2[i & 1], p2);
+    float p0, p1;
+    unpack2(p2, p0, p1);
+    __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
+    pw[i] = *reinterpret_cast<uint32_t*>(&b2);
+  }
 }
 
 __device__ __noinline__ void wait_slow(uint64_t* bar, uint32_t parity, Bars* b, int32_t* status) {
@@ -266,13 +286,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     mbar_init(&bars->s_full[0], 1);
     mbar_init(&bars->s_full[1], 1);
-    mbar_init(&bars->p_full, 2 * kSoftmaxWarps);   // one arrival per softmax warp of each CTA of the pair
+    for (int s = 0; s < 2; s++) mbar_init(&bars->p_full[s], 2 * kSoftmaxWarps);   // one arrival per softmax warp of each CTA of the pair
     mbar_init(&bars->pv_done, 1);
     for (int s = 0; s < 2; s++) {
       mbar_init(&bars->o_full[s], 1);
       mbar_init(&bars->o_empty[s], 2 * kEpiWarps);   // the read-out warps of both CTAs (leader's copy is the one waited on)
     }
-    mbar_init(&bars->l_full, kSoftmaxWarps / kSplit);
+    mbar_init(&bars->l_full, kSoftmaxWarps);
     mbar_init(&bars->l_empty, kEpiWarps);
     mbar_init(&bars->drain, 1);
     bars->abort_flag = 0;
@@ -317,36 +337,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       }
       __syncwarp();
     };
-    int g = 0, n = 0;
-    Cursor cu{worker, 0};
-    Item cur = item_of<kMla>(prm, cu);
-    load_q(cur, 0);
-    for (; cursor_valid(prm, cu); n++) {
+    int g = 0;
+    Walk<kMla> w(prm, worker, n_workers);
+    load_q(w.it, 0);
+    for (bool go = true; go;) {
+      const Item cur = w.it;
+      const int32_t* row = prm.table + (size_t)cur.seq * prm.table_stride;
+      int32_t ids = 0;   // lane l: page id of slot 32 k + l
       for (int j = 0; j < cur.ntiles; j++, g++) {
+        if ((j & 15) == 0) ids = __ldg(row + min(2 * j + lane, cur.last_slot));   // a tile's second page may lie past the sequence: its keys are masked
         // rows of the tile's two 64-key halves in tmap_kv (relative to krow0 / vrow0), and for MLA the pool row of the
         // RoPE block of this CTA's half
         int32_t y[2], y_rope = 0;
+        auto page_of = [&](int h2) {
+          const int32_t pg = __shfl_sync(0xffffffffu, ids, (2 * j + h2) & 31);
+          if (pg >= 0 && pg < prm.num_pages) return pg;
+          set_status(prm.status, RELUX_ERR_BAD_PAGE);   // reported, and replaced by page 0 so that no load leaves the pool
+          return 0;
+        };
         if constexpr (kMla) {
           y[0] = cur.hk * prm.Ttot + cur.base + j * kTile;
           y[1] = y[0] + kPage;
-          const int slot = min(2 * j + (int)rank, cur.last_slot);
-          int32_t pg = __ldg(prm.table + (size_t)cur.seq * prm.table_stride + slot);
-          if (pg < 0 || pg >= prm.num_pages) {
-            set_status(prm.status, RELUX_ERR_BAD_PAGE);
-            pg = 0;
-          }
-          y_rope = (int32_t)(prm.pool_row0 + ((int64_t)pg * prm.blocks_per_page + prm.rope_block) * kPage);
+          y_rope = (int32_t)(prm.pool_row0 + ((int64_t)page_of((int)rank) * prm.blocks_per_page + prm.rope_block) * kPage);
         } else {
-#pragma unroll
-          for (int h2 = 0; h2 < 2; h2++) {
-            const int slot = min(2 * j + h2, cur.last_slot);   // a tile's second page may lie past the sequence: its keys are masked
-            int32_t pg = __ldg(prm.table + (size_t)cur.seq * prm.table_stride + slot);
-            if (pg < 0 || pg >= prm.num_pages) {               // reported, and replaced by page 0 so that no load leaves the pool
-              set_status(prm.status, RELUX_ERR_BAD_PAGE);
-              pg = 0;
-            }
-            y[h2] = (pg * prm.Hkv + cur.hk) * kPage;
-          }
+          y[0] = (page_of(0) * prm.Hkv + cur.hk) * kPage;
+          y[1] = (page_of(1) * prm.Hkv + cur.hk) * kPage;
         }
         const int32_t y_own = rank ? y[1] : y[0];
         {   // K: this CTA's 64 keys of the tile, every 64-dim block of the score contraction
@@ -375,11 +390,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           __syncwarp();
         }
       }
-      cu = cursor_next(prm, cu, n_workers);
-      if (cursor_valid(prm, cu)) {   // the next item's Q, while this item's last tiles are still in flight
-        cur = item_of<kMla>(prm, cu);
-        load_q(cur, n + 1);
-      }
+      go = w.next();
+      if (go) load_q(w.it, w.n);   // the next item's Q, while this item's last tiles are still in flight
     }
   } else if (warp == kSoftmaxWarps + 1) {
     // =============================== MMA issuer (leader CTA only; converged warp + elected lane) ===============================
@@ -417,7 +429,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       auto issue_pv = [&](int g, int n, bool first, bool last) {
         const int st = g % kDepthV;
         if (first && n >= 2) wait_bar(&bars->o_empty[n & 1], ((n >> 1) - 1) & 1, bars, prm.status);
-        wait_bar(&bars->p_full, g & 1, bars, prm.status);
+        wait_bar(&bars->p_full[g & 1], (g >> 1) & 1, bars, prm.status);
         wait_bar(&bars->v_full[st], (g / kDepthV) & 1, bars, prm.status);
         tc_fence_after();   // P rows, a possible O rescale and the previous item's O read-out were done by the softmax warps of both CTAs
         if (el) {
@@ -432,27 +444,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         __syncwarp();
       };
-      int g = 0, n = 0;
-      Cursor cu{worker, 0};
-      int ntiles = item_of<kMla>(prm, cu).ntiles;
+      Walk<kMla> w(prm, worker, n_workers);
+      int g = 0, ntiles = w.it.ntiles;
       issue_qk(0, 0, true, ntiles == 1);
-      for (; cursor_valid(prm, cu); n++) {
-        cu = cursor_next(prm, cu, n_workers);
-        const bool has_next = cursor_valid(prm, cu);
-        const int next_tiles = has_next ? item_of<kMla>(prm, cu).ntiles : 0;
+      while (ntiles > 0) {
+        const int n = w.n, next_tiles = w.next() ? w.it.ntiles : 0;
         for (int i = 0; i < ntiles; i++, g++) {
-          if (i + 1 < ntiles) {
-            issue_qk(g + 1, n, false, i + 2 == ntiles);
-            issue_pv(g, n, i == 0, false);
-          } else if (has_next && kQBufs > 1) {
-            issue_qk(g + 1, n + 1, true, next_tiles == 1);
-            issue_pv(g, n, i == 0, true);
-          } else {
-            // one Q buffer: the next item's Q is requested when this item's last QK^T has completed, so its first QK^T
-            // goes behind this item's last PV instead of waiting for the load in front of it
-            issue_pv(g, n, i == 0, true);
-            if (has_next) issue_qk(g + 1, n + 1, true, next_tiles == 1);
-          }
+          if (i + 1 < ntiles) issue_qk(g + 1, n, false, i + 2 == ntiles);
+          else if (next_tiles > 0) issue_qk(g + 1, n + 1, true, next_tiles == 1);
+          issue_pv(g, n, i == 0, i + 1 == ntiles);
         }
         ntiles = next_tiles;
       }
@@ -464,116 +464,137 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
   } else if (warp < kSoftmaxWarps) {
     // =============================== softmax / correction ===============================
-    // Warp w reads TMEM lanes 32 (w & 3) .. +31 (the hardware's rule); the kSplit warps that share a lane quarter take
-    // one slice of kCols keys (and output dims) each.
-    const int wq = warp & 3, hb = warp >> 2;
-    const int r = wq * 32 + lane;                   // TMEM lane = query row
-    const int tq = r / prm.g;                       // token in block
-    const uint32_t lane_addr = ((uint32_t)(wq * 32) << 16) + (uint32_t)(hb * kCols);
-    const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full), 0);
-    int g = 0, n = 0;
-    for (Cursor cu{worker, 0}; cursor_valid(prm, cu); cu = cursor_next(prm, cu, n_workers), n++) {
-      const Item it = item_of<kMla>(prm, cu);
+    // Warp w reads TMEM lanes 32 (w & 3) .. +31 (the hardware's rule), of which warps w and w + 4 take 16 rows each.  The loads
+    // give four lanes a row (two neighbouring keys of every eight each), so a row's maximum and sum meet by shuffles and no warp
+    // waits for another: with a row shared by two warps the maxima went through shared memory and a barrier in every tile, and
+    // shared memory answers slowly while the MMAs read their operands from it.
+    const int r16 = (warp & 3) * 32 + (warp >> 2) * 16;
+    const uint32_t lane_addr = (uint32_t)r16 << 16;
+    const int row[2] = {r16 + (lane >> 2), r16 + (lane >> 2) + 8};   // this lane's two query rows
+    const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full[0]), 0);
+    const int tq[2] = {row[0] / prm.g, row[1] / prm.g};              // token in block
+    const uint64_t scale2 = pack2(prm.scale_log2, prm.scale_log2);
+#ifdef STAG
+    if (warp >= 4) { const long long c0 = clock64(); while (clock64() - c0 < STAG) {} __syncwarp(); }
+#endif
+    int g = 0;
+    Walk<kMla> w(prm, worker, n_workers);
+    do {
+      const Item it = w.it;
+      const int n = w.n;
       const int t0 = (2 * it.pair + (int)rank) * prm.bq;          // first query token of this CTA's block
-      // keys [0, t_eff) are visible to this row
-      const int t_eff = prm.causal ? min(it.T, it.T - prm.S + t0 + tq + 1) : it.T;
+      // keys [0, t_eff) are visible to a row; counted from this lane's first key of a tile
+      int t_lane[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) t_lane[k] = (prm.causal ? min(it.T, it.T - prm.S + t0 + tq[k] + 1) : it.T) - 2 * (lane & 3);
       const uint32_t tmem_o = tmem + lane_addr + kTmemO + (n & 1) * 128;
-      float m_used = -INFINITY, l_run = 0.f;
+      float m_used[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
       for (int j = 0; j < it.ntiles; j++, g++) {
+        const uint32_t tmem_s = tmem + lane_addr + kTmemS + (g & 1) * 128;
         wait_bar(&bars->s_full[g & 1], (g >> 1) & 1, bars, prm.status);
         __syncwarp();   // the TMEM loads below are warp-collective
         tc_fence_after();
-        uint32_t sv[kCols];
-#pragma unroll
-        for (int c = 0; c < kCols; c += 32)
-          tmem_ld_32x32b_x32(tmem + lane_addr + kTmemS + (g & 1) * 128 + c, *reinterpret_cast<uint32_t(*)[32]>(&sv[c]));
+        uint32_t sv[64];
+        tmem_ld_16x256b_x16(tmem_s, sv);
         tmem_ld_wait();
-        const int nvalid = max(0, min(kCols, t_eff - j * kTile - hb * kCols));
-        if (nvalid < kCols) {
+        const int nv0 = t_lane[0] - j * kTile, nv1 = t_lane[1] - j * kTile;   // row 1 sees no fewer keys than row 0
+        const bool whole = __all_sync(0xffffffffu, nv0 >= kTile);
+        if (!whole) {
+          // bit 2 i + e: key 8 i + e of this lane's (of its first key on) lies at or past the row's limit
 #pragma unroll
-          for (int c = 0; c < kCols; c++)
-            if (c >= nvalid) sv[c] = 0xFF800000u;   // -inf
+          for (int k = 0; k < 2; k++) {
+            const int nv = k ? nv1 : nv0;
+            const int keys = nv <= 0 ? 0 : 2 * (nv >> 3) + min(nv & 7, 2);   // of the lane's 32 keys of the tile, how many the row sees
+            const uint32_t hidden = keys >= 32 ? 0u : 0xffffffffu << keys;
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+              if (hidden & (1u << i)) sv[4 * (i >> 1) + 2 * k + (i & 1)] = 0xFF800000u;   // -inf
+          }
         }
         // row max of the raw scores (the softmax scale is positive, so it commutes with max); four chains of three-input
         // maxima, two scores per instruction
-        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float mx4[2][4];
 #pragma unroll
-        for (int c = 0; c < kCols; c += 8)
+        for (int k = 0; k < 2; k++)
 #pragma unroll
-          for (int k = 0; k < 4; k++) mx4[k] = max3(mx4[k], __uint_as_float(sv[c + 2 * k]), __uint_as_float(sv[c + 2 * k + 1]));
-        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * prm.scale_log2;
-        bars->rowmax[g & 1][hb][r] = mx;
-        asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
+          for (int c = 0; c < 4; c++) mx4[k][c] = -INFINITY;
 #pragma unroll
-        for (int k = 0; k < kSplit; k++) mx = fmaxf(mx, bars->rowmax[g & 1][k][r]);
-        // lazily updated running max: all threads of a row take the same decision
-        float alpha = 1.f;
+        for (int i = 0; i < 16; i++)
+#pragma unroll
+          for (int k = 0; k < 2; k++)
+            mx4[k][i & 3] = max3(mx4[k][i & 3], __uint_as_float(sv[4 * i + 2 * k]), __uint_as_float(sv[4 * i + 2 * k + 1]));
+        float mx[2], alpha[2] = {1.f, 1.f};
+#pragma unroll
+        for (int k = 0; k < 2; k++) mx[k] = fmaxf(fmaxf(mx4[k][0], mx4[k][1]), fmaxf(mx4[k][2], mx4[k][3]));
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+          for (int k = 0; k < 2; k++) mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+        // lazily updated running max: all lanes of a row take the same decision
         bool rescale = false;
-        if (mx > m_used + kRescaleThreshold) {   // also true on the first tile with a visible key (m_used = -inf)
-          alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
-          rescale = (m_used != -INFINITY);
-          m_used = mx;
+        uint64_t neg_m2[2], ps2[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const float m = mx[k] * prm.scale_log2;
+          if (m > m_used[k] + kRescaleThreshold) {   // also true on the first tile with a visible key (m_used = -inf)
+            if (m_used[k] != -INFINITY) {
+              alpha[k] = exp2f(m_used[k] - m);
+              rescale = true;
+            }
+            m_used[k] = m;
+          }
+          const float neg_m = (m_used[k] == -INFINITY) ? 0.f : -m_used[k];
+          neg_m2[k] = pack2(neg_m, neg_m);
+          ps2[k] = pack2(0.f, 0.f);
         }
-        const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
-        const uint64_t scale2 = pack2(prm.scale_log2, prm.scale_log2), neg_m2 = pack2(neg_m, neg_m);
-        // P(g), packed to bf16, goes over the first 64 columns of S(g): every slice of the row has read its S columns (the
-        // barrier above came after the loads), and QK(g+2), which writes this S buffer again, is issued behind PV(g).
-        // kPolyPairsOf8 pairs of every eight take the polynomial; a thread with a masked key in its slice (the diagonal
-        // tiles only) keeps to ex2(-inf) = 0 exactly.
-        uint32_t pw[kCols / 2];
-        uint64_t ps2;
-        if (nvalid == kCols) ps2 = exp_rows<true>(sv, scale2, neg_m2, pw);
-        else ps2 = exp_rows<false>(sv, scale2, neg_m2, pw);
+        // P(g), packed to bf16, goes over the first 64 columns of S(g): the rows' scores are in registers, and QK(g+2), which
+        // writes this S buffer again, is issued behind PV(g).  kPolyPairsOf8 pairs of every eight take the polynomial; a warp
+        // with a masked key in the tile (the diagonal tiles only) keeps to ex2(-inf) = 0 exactly.
+        uint32_t pw[32];
+        if (whole) exp_quads<true>(sv, scale2, neg_m2, pw, ps2);
+        else exp_quads<false>(sv, scale2, neg_m2, pw, ps2);
         __syncwarp();   // the store is warp-collective
-        tmem_st_32x32b_x32(tmem + ((uint32_t)(wq * 32) << 16) + kTmemS + (g & 1) * 128 + hb * (kCols / 2), pw);
-        float ps0, ps1;
-        unpack2(ps2, ps0, ps1);
-        l_run = l_run * alpha + (ps0 + ps1);
-        // O may be rescaled only after PV(g-1) has completed.  The wait is made on an item's first tile too (PV(g-1) is then
-        // the previous item's last one): PV(g-1) was issued behind the completion of p_full's phase g-1, so no warp arrives
-        // for tile g before every warp OF BOTH CTAs has arrived for tile g-1.  Without it the softmax warps of one CTA,
-        // which after an item's last tile wait for nothing but S of the next item's first tile (computed ahead), could
-        // arrive twice while a warp of the other CTA was still writing P(g-1): p_full's phase g-1 completed early and the
-        // item's last PV read an unfinished P.
-        if (g > 0) wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
-        __syncwarp();
+        tmem_st_16x128b_x16(tmem_s, pw);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          float ps0, ps1;
+          unpack2(ps2[k], ps0, ps1);
+          l_run[k] = l_run[k] * alpha[k] + (ps0 + ps1);
+        }
         // The TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep
-        // their maximum multiply by one.  This thread's slice of the row: output dims kCols hb .. +kCols-1.
-        if (j > 0 && __any_sync(0xffffffffu, rescale)) {
-          const float a_row = rescale ? alpha : 1.f;
+        // their maximum multiply by one.  O may be rescaled only after PV(g-1) has completed; PV(g-2) has: QK(g), whose scores
+        // are in, was issued behind it.
+        if (__any_sync(0xffffffffu, rescale)) {
+          wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
+          __syncwarp();
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < kCols; c += 32) {
+          for (int c = 0; c < kD; c += 64) {
             uint32_t ov[32];
-            tmem_ld_32x32b_x32(tmem_o + c, ov);
+            tmem_ld_16x256b_x8(tmem_o + c, ov);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; i++) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * a_row);
-            tmem_st_32x32b_x32(tmem_o + c, ov);
+            for (int i = 0; i < 32; i++) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha[(i >> 1) & 1]);
+            tmem_st_16x256b_x8(tmem_o + c, ov);
           }
-          tmem_st_wait();
         }
         tmem_st_wait();   // P, and a rescaled O
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(p_full_lead);
+        // P(g) is complete when every warp of both CTAs has arrived.  A barrier per tile parity: a warp may be a tile ahead of
+        // another, never two (S(g+2) is computed behind PV(g)).
+        if (lane == 0) mbar_arrive_cluster(p_full_lead + (g & 1) * 8);
       }
-      // ---- end of the item: the row sum (the sum of its key slices) goes to the read-out warps ----
-      // The slices meet in the row-maximum buffer of the tile that follows; nobody writes it before the second barrier.
-      float(*lx)[128] = bars->rowmax[g & 1];
-      lx[hb][r] = l_run;
-      asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
-      if (hb == 0) {
-        float l = 0.f;
+      // ---- end of the item: the row sums go to the read-out warps ----
 #pragma unroll
-        for (int k = 0; k < kSplit; k++) l += lx[k][r];
-        if (n > 0) wait_bar(&bars->l_empty, (n - 1) & 1, bars, prm.status);   // the read-out of the previous item has taken its sums
-        bars->lsum[r] = l;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->l_full);
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxThreads) : "memory");
-    }
+      for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < 2; k++) l_run[k] += __shfl_xor_sync(0xffffffffu, l_run[k], o);
+      if (n > 0) wait_bar(&bars->l_empty, (n - 1) & 1, bars, prm.status);   // the read-out of the previous item has taken its sums
+      if ((lane & 3) < 2) bars->lsum[row[lane & 1]] = (lane & 1) ? l_run[1] : l_run[0];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->l_full);
+    } while (w.next());
   } else {
     // =============================== read-out: O / l -> out ===============================
     // One warp per TMEM lane quarter; item n's accumulator is O buffer n & 1, handed over by the commit behind the
@@ -589,9 +610,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     constexpr int kOutCols = PL::kOutCols;
     uint8_t* tile = smem + PL::kSmemOut + wq * PL::kOutTile;
     if (lane == 0) tma_prefetch_desc(&tmap_out);
-    int n = 0;
-    for (Cursor cu{worker, 0}; cursor_valid(prm, cu); cu = cursor_next(prm, cu, n_workers), n++) {
-      const Item it = item_of<kMla>(prm, cu);
+    Walk<kMla> w(prm, worker, n_workers);
+    do {
+      const Item it = w.it;
+      const int n = w.n;
       const int t0 = (2 * it.pair + (int)rank) * prm.bq + wq * 32 / prm.g;   // first query token of the warp's rows
       wait_bar(&bars->l_full, n & 1, bars, prm.status);
       const float l_row = bars->lsum[r];
@@ -627,7 +649,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster((n & 1) ? o_empty_lead[1] : o_empty_lead[0]);
-    }
+    } while (w.next());
     if (lane == 0) tma_store_wait_all();
   }
   __syncwarp();
