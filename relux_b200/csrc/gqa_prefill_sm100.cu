@@ -102,7 +102,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemS = 0, kTmemO = 256;                  // S(g) at kTmemS + 128 (g & 1); O of item n at kTmemO + 128 (n & 1)
 constexpr float kRescaleThreshold = 8.0f;
 #ifndef RELUX_PREFILL_POLY_PAIRS
-#define RELUX_PREFILL_POLY_PAIRS 3
+#define RELUX_PREFILL_POLY_PAIRS 2
 #endif
 constexpr int kPolyPairsOf8 = RELUX_PREFILL_POLY_PAIRS;   // score pairs out of every eight whose exponential runs on the FMA pipe
 
@@ -523,26 +523,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int k = 0; k < 2; k++)
             mx4[k][i & 3] = max3(mx4[k][i & 3], __uint_as_float(sv[4 * i + 2 * k]), __uint_as_float(sv[4 * i + 2 * k + 1]));
-        float mx[2], alpha[2] = {1.f, 1.f};
+        float mx[2];
 #pragma unroll
-        for (int k = 0; k < 2; k++) mx[k] = fmaxf(fmaxf(mx4[k][0], mx4[k][1]), fmaxf(mx4[k][2], mx4[k][3]));
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1)
-#pragma unroll
-          for (int k = 0; k < 2; k++) mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        // lazily updated running max: all lanes of a row take the same decision
+        for (int k = 0; k < 2; k++) mx[k] = fmaxf(fmaxf(mx4[k][0], mx4[k][1]), fmaxf(mx4[k][2], mx4[k][3])) * prm.scale_log2;
+        // Lazily updated running max.  The lanes of a row meet only in a tile that raises some row's (the first tile with a
+        // visible key does, m_used = -inf); all lanes of a row take the same decision.
         bool rescale = false;
+        float alpha[2] = {1.f, 1.f};
+        if (__any_sync(0xffffffffu, mx[0] > m_used[0] + kRescaleThreshold || mx[1] > m_used[1] + kRescaleThreshold)) {
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < 2; k++) mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+#pragma unroll
+          for (int k = 0; k < 2; k++)
+            if (mx[k] > m_used[k] + kRescaleThreshold) {
+              if (m_used[k] != -INFINITY) {
+                alpha[k] = exp2f(m_used[k] - mx[k]);
+                rescale = true;
+                l_run[k] *= alpha[k];
+              }
+              m_used[k] = mx[k];
+            }
+        }
         uint64_t neg_m2[2], ps2[2];
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-          const float m = mx[k] * prm.scale_log2;
-          if (m > m_used[k] + kRescaleThreshold) {   // also true on the first tile with a visible key (m_used = -inf)
-            if (m_used[k] != -INFINITY) {
-              alpha[k] = exp2f(m_used[k] - m);
-              rescale = true;
-            }
-            m_used[k] = m;
-          }
           const float neg_m = (m_used[k] == -INFINITY) ? 0.f : -m_used[k];
           neg_m2[k] = pack2(neg_m, neg_m);
           ps2[k] = pack2(0.f, 0.f);
@@ -559,7 +565,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         for (int k = 0; k < 2; k++) {
           float ps0, ps1;
           unpack2(ps2[k], ps0, ps1);
-          l_run[k] = l_run[k] * alpha[k] + (ps0 + ps1);
+          l_run[k] += ps0 + ps1;
         }
         // The TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep
         // their maximum multiply by one.  O may be rescaled only after PV(g-1) has completed; PV(g-2) has: QK(g), whose scores
