@@ -367,6 +367,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       for (int i = 0; i < ntiles; i++, g++) {
         // no thread leaves this loop early: every thread must reach the same named barriers
         wait_bar(&bars->s_full[g & 1], (g >> 1) & 1, bars, prm.status);
+        __syncwarp();   // the TMEM loads below are warp-collective
         tc_fence_after();
         uint32_t sv[2][32];
         tmem_ld_32x32b_x32(tmem + lane_addr + kTmemS + (g & 1) * 64, sv[0]);
@@ -417,7 +418,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         l_run = l_run * alpha + psum;
         // P(g) may overwrite the buffer, and O may be rescaled, only after PV(g-1) has completed
         if (g > 0) wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
-        if (rescale && i > 0) {
+        // TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep their
+        // maximum multiply by one
+        if (__any_sync(0xffffffffu, rescale && i > 0)) {
+          const float a_row = rescale ? alpha : 1.f;
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < 256; c += 32) {
@@ -425,7 +429,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
             tmem_ld_32x32b_x32(tmem + lane_addr + kTmemO + c, ov);
             tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; j++) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * alpha);
+            for (int j = 0; j < 32; j++) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * a_row);
             tmem_st_32x32b_x32(tmem + lane_addr + kTmemO + c, ov);
           }
           tmem_st_wait();
@@ -442,7 +446,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       }
       // ---- item epilogue: O (unnormalised), running max and sum -> split-KV partial of this item ----
       wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
-      const bool ok = !bars->abort_flag;
+      const bool ok = !__any_sync(0xffffffffu, bars->abort_flag != 0);   // the TMEM loads below are warp-collective
       tc_fence_after();
       if (hf == 1) bars->lsum[row] = l_run;
       asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -463,10 +467,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 #pragma unroll 1
         for (int c = 0; c < 128; c += 32) {
           uint32_t ov[32];
-          if (ok && m_used != -INFINITY) {
-            tmem_ld_32x32b_x32(tmem + lane_addr + kTmemO + nb * 128 + c, ov);
-            tmem_ld_wait();
-          } else {
+          tmem_ld_32x32b_x32(tmem + lane_addr + kTmemO + nb * 128 + c, ov);
+          tmem_ld_wait();
+          if (!ok || m_used == -INFINITY) {
 #pragma unroll
             for (int j = 0; j < 32; j++) ov[j] = 0u;
           }
