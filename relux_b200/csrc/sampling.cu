@@ -889,29 +889,13 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     sd = a; st = t;
     return bad;
   };
-  // Few sequences: the chain's length is what costs, not the bytes.  The rows of ALL draft positions are read in one stage
-  // (and the sums to be made again in a second), so the accept loop below runs without a pass of its own per position (rows
-  // after a rejection are read in vain).
+  // Few sequences: the chain's length is what costs, not the bytes.  The rows of ALL draft positions are read in one stage, so
+  // the accept loop below runs without a pass of its own per position (rows after a rejection are read in vain).
   const bool batched = prm.batched && k >= 2 && 4 * k <= kStatMax;
   if (batched) {
     float acc[kStatMax];
     for (int i = 0; i < k; i++) pair_pass(i, acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
     cluster_reduce_n(c, acc, 4 * k, c.sh->stat);
-    int any = 0;
-    for (int i = 0; i < k; i++) {
-      const int bad = pair_again(i, c.sh->stat[4 * i + 2], c.sh->stat[4 * i + 3], acc[4 * i], acc[4 * i + 1]);
-      // a row whose sum stands brings it along from one thread of the cluster
-      const bool first = c.rank == 0 && threadIdx.x == 0;
-      if (!(bad & 1)) acc[4 * i] = first ? c.sh->stat[4 * i] : 0.0f;
-      if (!(bad & 2)) acc[4 * i + 1] = first ? c.sh->stat[4 * i + 1] : 0.0f;
-      acc[4 * i + 2] = c.sh->stat[4 * i + 2];
-      acc[4 * i + 3] = c.sh->stat[4 * i + 3];
-      any |= bad;
-    }
-    if (any) {   // uniform over the cluster: everyone looked at the same logits and maxima
-      __syncthreads();
-      cluster_reduce_n(c, acc, 4 * k, c.sh->stat);
-    }
   }
   for (int i = 0; i < k && !done; i++) {
     const float* drow = drow_of(i);
@@ -936,13 +920,23 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
       cluster_reduce4<2>(c, v4);
       md = v4[2];
       mt = v4[3];
+    }
+    const float u = next_draw();
+    if (tok_d != md || tok_t != mt) {
+      // A sum against a guess says most of what the one against the maximum would: fastexp32 is e^x but for a factor between
+      // 0.967 and 1.027, so the two differ from e^(guess - maximum) by a factor below 1.062.  A draw that is accepted with that
+      // much to spare needs no second pass (the usual case); everything else gets the sums as the reference has them.
+      constexpr float kSpare = 1.07f;
+      const float est_d = v4[0] * expf(tok_d - md), est_t = v4[1] * expf(tok_t - mt);
+      const float dP = fastexp32_ref(__fsub_rn(tok_d, md)) / est_d * (tok_d != md ? kSpare : 1.0001f);
+      const float tP = fastexp32_ref(__fsub_rn(tok_t, mt)) / est_t / (tok_t != mt ? kSpare : 1.0001f);
+      const bool sound = md - tok_d < 80.0f && mt - tok_t < 80.0f && v4[0] < 1e38f && v4[1] < 1e38f;   // false for NaN too
+      if (sound && u < fminf(tP / fmaxf(dP, 1e-10f), 1.0f)) continue;
       float w4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       const int bad = pair_again(i, md, mt, w4[0], w4[1]);
-      if (bad) {
-        cluster_reduce4<0>(c, w4);
-        if (bad & 1) v4[0] = w4[0];
-        if (bad & 2) v4[1] = w4[1];
-      }
+      cluster_reduce4<0>(c, w4);
+      if (bad & 1) v4[0] = w4[0];
+      if (bad & 2) v4[1] = w4[1];
     }
     const float invd = v4[0] > 0.0f ? __fdiv_rn(1.0f, v4[0]) : 1.0f;
     const float invt = v4[1] > 0.0f ? __fdiv_rn(1.0f, v4[1]) : 1.0f;
@@ -950,7 +944,6 @@ __global__ void __launch_bounds__(kSelThreads, 2) spec_accept_kernel(SelParams p
     const float tP = __fmul_rn(fastexp32_ref(__fsub_rn(tok_t, mt)), invt);
     float ap = __fdiv_rn(tP, dP > 1e-10f ? dP : 1e-10f);
     if (ap > 1.0f) ap = 1.0f;
-    const float u = next_draw();
     if (u < ap) continue;
     // rejected at i: resample from norm(max(0, p_target - p_draft))   speculative.go:256-295
     auto adj = [&](float tv, float dv) {
