@@ -19,7 +19,7 @@
 //     O[256 x 128] += P V       8 MMAs M256 N128 K16; A = P from tensor memory; B = V as it lies (MN-major), split by
 //                               output dims: CTA r holds dims [64 r, 64 r + 64) of both pages (16 KB)
 // Persistent workers.  As many CTA pairs as fit on the GPU are launched once and walk a static list of items (see
-// Cursor below for its order).  One launch per block measured 16k cycles (8 us) of fixed cost per CTA pair -- launch,
+// Walk below for its order).  One launch per block measured 16k cycles (8 us) of fixed cost per CTA pair -- launch,
 // tensor-memory allocation, the latency of the first Q / K loads, pipeline fill, drain and the epilogue -- against
 // 2.1k cycles per tile: at 2048-token prompts (9 tiles per item on average) that was half of the kernel.  Here the tile
 // pipeline does not drain at an item boundary: tiles are numbered over the worker's whole life, Q has two buffers (the
@@ -30,12 +30,19 @@
 // TMEM per CTA: S double-buffered (2 x 128 columns, P over the first 64 of each), O double-buffered (2 x 128 columns);
 // rows = TMEM lanes.  Issue order QK(g+1), PV(g): QK(g+2), which overwrites the S / P buffer of tile g, is issued behind
 // PV(g), and the tensor pipe executes in issue order.
-// Warp roles per CTA: 8 softmax warps -- a query row (TMEM lane) is shared by two threads, 64 keys (and 64 output dims
-// of a rescale) each --, 1 TMA producer, 1 MMA issuer (leader CTA only), both converged with one elected lane, 4 read-out
-// warps.  The softmax warps are the busiest part: per tile and SM 16384 scores through max, scale, exp2, sum and pack.
-// The special-function unit delivers 16 exponentials per clock and SM (1024 clocks per tile, as long as the tile's
-// MMAs), so three pairs of every eight take a cubic on the FMA pipe instead, arithmetic runs two lanes per instruction
-// (fma.f32x2, add.f32x2) and the row maximum takes two scores per instruction (three-input max).
+// Warp roles per CTA: 8 softmax warps of 16 query rows (TMEM lanes) each, four lanes to a row, 1 TMA producer, 1 MMA issuer
+// (leader CTA only), both converged with one elected lane, 4 read-out warps.  The softmax warps are the busiest part: per tile
+// and SM 16384 scores through max, scale, exp2, sum and pack.  The special-function unit delivers 16 exponentials per clock and
+// SM (1024 clocks per tile, as long as the tile's MMAs), so two pairs of every eight take a cubic on the FMA pipe instead
+// (three: the same within 1 %, four: 2 % slower), arithmetic runs two lanes per instruction (fma.f32x2, add.f32x2) and the row
+// maximum takes two scores per instruction (three-input max).
+// What bounds it (clock stamps, 8 x 2048 tokens, 32 heads over 8): a tile takes 1740 clocks, 1000 of them exponentials of two
+// warps per scheduler in step, 330 the maxima, the rest waits and tensor-memory round trips; between two items 1000-2400 more.
+// Measured, 8 x 2048 GQA and 4 x 1000 MLA tokens (this launch): rows shared by two warps, stored a row per lane 343 and 274 us;
+// output by TMA 317 and 251; 16 rows per warp without a barrier, items walked by digits 307 and 235; the vote before the
+// shuffles and two pairs of eight 303 and 229.  Not kept: the two halves of the softmax warps on alternate tiles, a whole row
+// per thread (8 % slower or worse with two, three S buffers, one O): the diagonal tiles and the item ends, serial there, cost
+// more than the overlap gave.  Holding one warp of a scheduler back by half a phase changed nothing.
 // Barriers: full barriers live in the leader CTA and count the bytes of both CTAs' loads; empty / s_full / pv_done /
 // o_full barriers live in each CTA and are armed by tcgen05.commit with mbarrier multicast (not a TMA load); p_full and
 // o_empty live in the leader and count warps of both CTAs.  No TMA multicast anywhere.

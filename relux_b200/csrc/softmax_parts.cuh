@@ -60,28 +60,4 @@ __device__ __forceinline__ uint64_t ex2_poly2(uint64_t x2) {
   return pack2(p0, p1);
 }
 
-// exp2(score * scale - max) for 32 consecutive scores of one row: bf16 P values, two per 32-bit word in key order, into
-// pw; the two partial row sums are added to ps2.  kPoly: kPolyPairs pairs of every eight take the polynomial (a row with
-// masked keys among the 32 must not: ex2(-inf) = 0 exactly, the polynomial clamps).
-template <bool kPoly, int kPolyPairs>
-__device__ __forceinline__ void exp_chunk32(const uint32_t (&sv)[32], uint64_t scale2, uint64_t neg_m2, uint32_t (&pw)[16], uint64_t& ps2) {
-#pragma unroll
-  for (int c = 0; c < 32; c += 2) {
-    const uint64_t x2 = fma2(pack2(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), scale2, neg_m2);
-    uint64_t p2;
-    if (kPoly && ((c >> 1) & 7) < kPolyPairs) {
-      p2 = ex2_poly2(x2);
-    } else {
-      float x0, x1;
-      unpack2(x2, x0, x1);
-      p2 = pack2(ex2_approx(x0), ex2_approx(x1));
-    }
-    ps2 = add2(ps2, p2);
-    float p0, p1;
-    unpack2(p2, p0, p1);
-    __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
-    pw[c >> 1] = *reinterpret_cast<uint32_t*>(&b2);
-  }
-}
-
 }  // namespace relux
