@@ -12,19 +12,21 @@
 //
 // Shape: a TOKEN TILE is 256 consecutive tokens of one sequence (4 pages), an OUTPUT TILE 128 columns (one head of K or
 // of V).  A worker is a CTA pair (tcgen05 cta_group::2, M = 256, N = 128): CTA r holds tokens [128 r, 128 r + 128) of the
-// token tile -- 8 latent blocks of [128 tokens x 64 columns], 128 KB, straight out of the blocked pages -- and columns
+// token tile -- 8 latent blocks of [128 tokens x 64 columns], straight out of the blocked pages -- and columns
 // [64 r, 64 r + 64) of every weight stage ([128 latent rows x 64 columns], MN-major as the weights lie).  Worker w takes a
 // contiguous run of (token tile, output tile) units in token-tile-major order, so the latent tile is loaded once per run
-// (twice when the run crosses a token tile) and the 32 MB of weights stream from L2 through a four-stage ring.
-// The latent tile is the A operand of every MMA of a run: it is copied once from shared memory into tensor memory (lane =
-// token, two latents per 32-bit column, 256 columns), so that the MMAs read only the weight stages from shared memory.
-// The accumulator is double-buffered in tensor memory: four epilogue warps convert unit n while the MMAs of unit n + 1
-// run (they also make the copy of the latent tile, between two runs of units), and the bf16 rows leave through a
-// swizzled shared tile and TMA stores (whole 128-byte lines instead of 16 bytes per lane at a 256-byte pitch).
-// What bounds the kernel is neither of those: every token tile streams all of W_UK and W_UV (32 MB at 128 heads), 256
-// flop per weight byte at 256 tokens per pair, and the L2 -> SM traffic measured 4.2 TB/s: 1.0-1.06 PFLOP/s with the latent
-// tile in shared or in tensor memory, with rows stored from registers or by TMA alike.
-// Warp roles per CTA: 4 epilogue warps, 1 TMA producer, 1 MMA issuer (leader CTA only).
+// (twice when the run crosses a token tile) and the 32 MB of weights stream from L2 through an eight-stage ring.
+// The latent tile is the A operand of every MMA of a run: it is copied once through shared memory, in two rounds of 64 KB, into
+// tensor memory (lane = token, two latents per 32-bit column, 256 columns), so that the MMAs read only the weight stages from
+// shared memory.
+// The accumulator is double-buffered in tensor memory: eight epilogue warps convert unit n while the MMAs of unit n + 1
+// run (they also make the copy of the latent tile, between two runs of units), and the bf16 rows leave through swizzled
+// shared tiles and TMA stores (whole 128-byte lines instead of 16 bytes per lane at a 256-byte pitch).
+// What bounds it: a unit is 2048 clocks of MMAs.  Four warps that converted its 128 columns in turn, behind the read of the
+// unit before, and a ring of one unit's weights (a window of 1500 clocks, an L2 round trip) made it 4100; two groups of four
+// warps, 64 columns and a shared tile each, and a ring of two units brought a 4 x 1000 token prompt's call from 397 to 375 us.
+// Every token tile streams all of W_UK and W_UV (32 MB at 128 heads) from L2, and 512 B per token and head are written.
+// Warp roles per CTA: 8 epilogue warps, 1 TMA producer, 1 MMA issuer (leader CTA only).
 // No TMA multicast.  The weight stages' full barriers live in the leader and count both CTAs' bytes; the latent tile's
 // full barrier is each CTA's own (its epilogue warps wait on it).  Every wait is bounded, and the MMA issuer sees its
 // last MMA complete before the pair frees its tensor memory.
@@ -43,15 +45,16 @@ namespace {
 constexpr int kDC = 512, kPage = 64, kTokTile = 256;
 constexpr int kBlk = 8192;                          // one [64 rows x 64 cols] bf16 box, 128-byte swizzled
 constexpr int kABlock = 2 * kBlk;                   // [128 tokens x 64 latent columns]
-constexpr int kABytes = (kDC / 64) * kABlock;       // 131072
+constexpr int kARounds = 2, kABlocks = kDC / 64 / kARounds;   // a latent tile passes through shared memory in two rounds
+constexpr int kABytes = kABlocks * kABlock;         // 65536
 constexpr int kStageBytes = 2 * kBlk;               // [128 latent rows x 64 output columns]
-constexpr int kStages = 4, kStagesPerUnit = kDC / 128;
+constexpr int kStages = 8, kStagesPerUnit = kDC / 128;
 constexpr int kSmemRing = kABytes;
 constexpr int kSmemOut = kSmemRing + kStages * kStageBytes;   // one output tile [128 tokens x (cols 0-63 | cols 64-127)] bf16, swizzled
 constexpr int kOutBytes = 4 * kBlk;
 constexpr int kSmemBar = kSmemOut + kOutBytes;                // 229376
 constexpr int kSmemTotal = kSmemBar + 1024;
-constexpr int kEpiWarps = 4, kThreads = 32 * (kEpiWarps + 2);
+constexpr int kEpiWarps = 8, kThreads = 32 * (kEpiWarps + 2);
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemA = 256;                    // accumulators at columns [0, 256), the latent tile at [256, 512)
 
@@ -137,6 +140,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       tma_prefetch_desc(&tmap_wuv);
     }
     int cur_tt = -1, na = 0, gs = 0;
+    // Every CTA's latent tile reports to its OWN barrier: its epilogue warps copy it to tensor memory.  The second round goes
+    // behind the weights of the tile's first unit, which do not wait for it.
+    int64_t y[2] = {0, 0};
+    bool pending = false;
+    auto load_a = [&](const int64_t (&y)[2], int round) {
+      if (na > 0) wait_bar(&bars->a_empty, (na - 1) & 1, bars, prm.status);
+      const uint32_t own = mapa_u32(smem_u32(&bars->a_full), rank);
+      if (el) {
+        mbar_expect_tx(&bars->a_full, kABytes);
+#pragma unroll 1
+        for (int j = 0; j < kABlocks; j++) {
+          const int kb = round * kABlocks + j;
+          tma_load_2d_2sm(smem + j * kABlock, &tmap_pool, 0, (int32_t)(y[0] + kb * kPage), own);
+          tma_load_2d_2sm(smem + j * kABlock + kBlk, &tmap_pool, 0, (int32_t)(y[1] + kb * kPage), own);
+        }
+      }
+      __syncwarp();
+      na++;
+    };
     for (int u = u0; u < u1; u++) {
       const int tt = u / prm.n_out, nt = u % prm.n_out;
       if (tt != cur_tt) {
@@ -151,7 +173,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const int T = load_chained(prm.len + seq) + prm.extra;
         const int last_slot = max(0, (T + kPage - 1) / kPage - 1);
         const int tok0 = tt * kTokTile - load_chained(prm.seq_base + lo) + 128 * (int)rank;   // this CTA's first token in the sequence
-        int64_t y[2];
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++) {
           const int slot = min(tok0 / kPage + h2, last_slot);
@@ -162,20 +183,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
           y[h2] = prm.row0 + (int64_t)pg * prm.blocks_per_page * kPage;
         }
-        if (na > 0) wait_bar(&bars->a_empty, (na - 1) & 1, bars, prm.status);
-        // every CTA's latent tile reports to its OWN barrier: its epilogue warps copy it to tensor memory
-        const uint32_t lead = mapa_u32(smem_u32(&bars->a_full), rank);
-        if (el) {
-          mbar_expect_tx(&bars->a_full, kABytes);
-#pragma unroll 1
-          for (int kb = 0; kb < kDC / 64; kb++) {
-            tma_load_2d_2sm(smem + kb * kABlock, &tmap_pool, 0, (int32_t)(y[0] + kb * kPage), lead);
-            tma_load_2d_2sm(smem + kb * kABlock + kBlk, &tmap_pool, 0, (int32_t)(y[1] + kb * kPage), lead);
-          }
-        }
-        __syncwarp();
-        na++;
         cur_tt = tt;
+        load_a(y, 0);
+        pending = true;
       }
       const CUtensorMap* wm = nt < prm.H ? &tmap_wuk : &tmap_wuv;
       const int x = (nt < prm.H ? nt : nt - prm.H) * 128 + 64 * (int)rank;
@@ -189,6 +199,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           tma_load_2d_2sm(smem + kSmemRing + st * kStageBytes, wm, x, s * 128, lead);
         }
         __syncwarp();
+      }
+      if (pending) {
+        load_a(y, 1);
+        pending = false;
       }
     }
   } else if (warp == kEpiWarps + 1) {
@@ -232,40 +246,46 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
   } else {
     // =============================== epilogue: accumulator -> bf16 rows ===============================
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    // Warp w reads TMEM lanes 32 (w & 3) .. +31 (the hardware's rule); warps w < 4 take columns 0-63 of a unit, the others 64-127:
+    // two groups, each with a barrier, a shared tile and a thread that stores of its own.
+    const int half = warp >> 2;
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t lead_empty0 = mapa_u32(smem_u32(&bars->acc_empty[0]), 0), lead_empty1 = mapa_u32(smem_u32(&bars->acc_empty[1]), 0);
     const uint32_t lead_ready = mapa_u32(smem_u32(&bars->a_ready), 0);
-    const int row = warp * 32 + lane;
+    const int row = (warp & 3) * 32 + lane;
+    const bool storer = (warp & 3) == 0 && lane == 0;
     int n = 0, na = 0, cur_tt = -1;
     for (int u = u0; u < u1; u++, n++) {
       const int tt = u / prm.n_out, nt = u % prm.n_out;
       if (tt != cur_tt) {
         // A new latent tile.  The MMAs that read the previous one have completed (this warp has seen acc_full of the last
         // unit that used it).  Row `row` of every 64-column block -> 32 columns of this thread's lane.
-        wait_bar(&bars->a_full, na & 1, bars, prm.status);
-        __syncwarp();
 #pragma unroll 1
-        for (int kb = 0; kb < kDC / 64; kb++) {
-          uint32_t w[32];
-          const uint8_t* src = smem + kb * kABlock + row * 128;
+        for (int round = 0; round < kARounds; round++, na++) {
+          wait_bar(&bars->a_full, na & 1, bars, prm.status);
+          __syncwarp();
+#pragma unroll 1
+          for (int j2 = half * (kABlocks / 2); j2 < (half + 1) * (kABlocks / 2); j2++) {
+            uint32_t w[32];
+            const uint8_t* src = smem + j2 * kABlock + row * 128;
 #pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const uint4 v = *reinterpret_cast<const uint4*>(src + ((j ^ (row & 7)) << 4));
-            w[4 * j] = v.x;
-            w[4 * j + 1] = v.y;
-            w[4 * j + 2] = v.z;
-            w[4 * j + 3] = v.w;
+            for (int j = 0; j < 8; j++) {
+              const uint4 v = *reinterpret_cast<const uint4*>(src + ((j ^ (row & 7)) << 4));
+              w[4 * j] = v.x;
+              w[4 * j + 1] = v.y;
+              w[4 * j + 2] = v.z;
+              w[4 * j + 3] = v.w;
+            }
+            tmem_st_32x32b_x32(tmem + lane_addr + kTmemA + (round * kABlocks + j2) * 32, w);
           }
-          tmem_st_32x32b_x32(tmem + lane_addr + kTmemA + kb * 32, w);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&bars->a_empty);      // the producer may fetch the next round into the shared tile
+            if (round + 1 == kARounds) mbar_arrive_cluster(lead_ready);
+          }
         }
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&bars->a_empty);        // the producer may fetch the next token tile into the shared tile
-          mbar_arrive_cluster(lead_ready);
-        }
-        na++;
         cur_tt = tt;
       }
       const int buf = n & 1;
@@ -273,40 +293,38 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       __syncwarp();   // the TMEM loads below are warp-collective
       tc_fence_after();
       // the stores of the previous unit have read the shared tile
-      if (threadIdx.x == 0) tma_store_wait_read();
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-      uint8_t* orow = smem + kSmemOut + row * 128;
-#pragma unroll 1
-      for (int c = 0; c < 128; c += 32) {
+      if (storer) tma_store_wait_read();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+      uint8_t* orow = smem + kSmemOut + half * 2 * kBlk + row * 128;
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + buf * 128 + c, v);
+        tmem_ld_32x32b_x32(tmem + lane_addr + buf * 128 + half * 64 + c, v);
         tmem_ld_wait();
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) pk[i] = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-        // columns c .. c + 31 = 16-byte chunks (c & 63) / 8 .. + 3 of the 64-column half c / 64
+        // columns c .. c + 31 of the half = 16-byte chunks c / 8 .. + 3
 #pragma unroll
         for (int i = 0; i < 4; i++)
-          *reinterpret_cast<uint4*>(orow + (c >> 6) * 2 * kBlk + (((((c & 63) >> 3) + i) ^ (row & 7)) << 4)) =
+          *reinterpret_cast<uint4*>(orow + ((((c >> 3) + i) ^ (row & 7)) << 4)) =
               make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(buf ? lead_empty1 : lead_empty0);   // the accumulator is free again
       fence_proxy_async();
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-      if (threadIdx.x == 0) {
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+      if (storer) {
         // first row of this CTA's 128 tokens in the [2 H Ttot][128] array of expanded keys and values
         const int32_t y = (int32_t)((int64_t)nt * prm.Ttot + (int64_t)tt * kTokTile + 128 * (int)rank);
 #pragma unroll
-        for (int h2 = 0; h2 < 2; h2++)
-#pragma unroll
-          for (int r2 = 0; r2 < 2; r2++) tma_store_2d(&tmap_out, 64 * h2, y + 64 * r2, smem + kSmemOut + h2 * 2 * kBlk + r2 * kBlk);
+        for (int r2 = 0; r2 < 2; r2++) tma_store_2d(&tmap_out, 64 * half, y + 64 * r2, smem + kSmemOut + half * 2 * kBlk + r2 * kBlk);
         tma_store_commit();
       }
     }
+    if (storer) tma_store_wait_all();
   }
-  if (threadIdx.x == 0) tma_store_wait_all();
   __syncwarp();
   tc_fence_before();
   cluster_sync();
