@@ -38,6 +38,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "splitkv.h"
+#include "softmax_parts.cuh"
 #include "umma.cuh"
 
 namespace relux {
@@ -89,10 +90,16 @@ struct MlaSm100Params {
   TimeStamp time;
 };
 
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+// Barrier of the 128 softmax threads that tells all of them whether any brought `yes`.
+__device__ __forceinline__ bool softmax_any(bool yes) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.or.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any)
+      : "r"((uint32_t)yes)
+      : "memory");
+  return any != 0;
 }
 
 // Bounded wait.  The common case (phase already complete) is a single try_wait.  When the bound runs out the
@@ -383,44 +390,54 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
             for (int j = 0; j < 32; j++)
               if (h2 * 32 + j >= nvalid) sv[h2][j] = 0xFF800000u;  // -inf
         }
-        // row max of the raw scores (the softmax scale is positive, so it commutes with max)
-        float mx = -INFINITY;
+        // row max of the raw scores (the softmax scale is positive, so it commutes with max); four chains of three-input maxima
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++)
 #pragma unroll
-          for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(sv[h2][j]));
-        mx *= prm.scale_log2;
-        bars->rowmax[g & 1][hf][row] = mx;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        mx = fmaxf(mx, bars->rowmax[g & 1][hf ^ 1][row]);
-        // lazily updated running max: both threads of a row take the same decision
+          for (int j = 0; j < 32; j += 8)
+#pragma unroll
+            for (int k = 0; k < 4; k++) mx4[k] = max3(mx4[k], __uint_as_float(sv[h2][j + 2 * k]), __uint_as_float(sv[h2][j + 2 * k + 1]));
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * prm.scale_log2;
+        // Lazily updated running max.  The two threads of a row meet only in a tile that raises some row's (the first one with a
+        // visible token does, m_used = -inf): in all others the barrier itself says that there is none.  Both take the same decision.
         float alpha = 1.f;
         bool rescale = false;
-        if (mx > m_used + kRescaleThreshold) {   // also true on the first tile with a visible token (m_used = -inf)
-          alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
-          rescale = (m_used != -INFINITY);
-          m_used = mx;
+        const bool raised = softmax_any(mx > m_used + kRescaleThreshold);
+        if (raised) {
+          bars->rowmax[g & 1][hf][row] = mx;
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          mx = fmaxf(mx, bars->rowmax[g & 1][hf ^ 1][row]);
+          if (mx > m_used + kRescaleThreshold) {
+            alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
+            rescale = (m_used != -INFINITY);
+            m_used = mx;
+          }
         }
-        // p = 2^(s * scale_log2 - m): one FFMA and one MUFU.EX2 per score
+        // p = 2^(s * scale_log2 - m), two scores an instruction but for the exponentials
         const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
-        float psum = 0.f;
+        const uint64_t scale2 = pack2(prm.scale_log2, prm.scale_log2), neg_m2 = pack2(neg_m, neg_m);
+        uint64_t ps2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
         uint32_t pk[32];
 #pragma unroll
         for (int h2 = 0; h2 < 2; h2++)
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float p0 = ex2_approx(fmaf(__uint_as_float(sv[h2][j]), prm.scale_log2, neg_m));
-            const float p1 = ex2_approx(fmaf(__uint_as_float(sv[h2][j + 1]), prm.scale_log2, neg_m));
-            psum += p0 + p1;
+            float x0, x1;
+            unpack2(fma2(pack2(__uint_as_float(sv[h2][j]), __uint_as_float(sv[h2][j + 1])), scale2, neg_m2), x0, x1);
+            const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
+            ps2[(j >> 1) & 1] = add2(ps2[(j >> 1) & 1], pack2(p0, p1));
             __nv_bfloat162 b2 = __floats2bfloat162_rn(p0, p1);
             pk[h2 * 16 + j / 2] = *reinterpret_cast<uint32_t*>(&b2);
           }
-        l_run = l_run * alpha + psum;
+        float ps0, ps1;
+        unpack2(add2(ps2[0], ps2[1]), ps0, ps1);
+        l_run = l_run * alpha + (ps0 + ps1);
         // P(g) may overwrite the buffer, and O may be rescaled, only after PV(g-1) has completed
         if (g > 0) wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
         // TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep their
         // maximum multiply by one
-        if (__any_sync(0xffffffffu, rescale && i > 0)) {
+        if (raised && __any_sync(0xffffffffu, rescale && i > 0)) {
           const float a_row = rescale ? alpha : 1.f;
           tc_fence_after();
 #pragma unroll 1
