@@ -423,13 +423,15 @@ __device__ void cdf_search(Ctx& c, const float* __restrict__ row, const float* _
     return;
   }
   if (cross != c.rank) return;
-  // this CTA holds the crossing: pick the warp, then walk its segment in order
+  // This CTA holds the crossing: pick the warp, then walk its segment in order.  The warps' sums are scaled one by one and round
+  // differently from the CTA's: where none of them crosses, it is the last one that carries probability (the warps behind it
+  // may have none, or no elements at all).
   int wsel = kSelWarps - 1;
   float acc = base, wbase = base;
   for (int w = 0; w < kSelWarps; w++) {
-    const float nxt = acc + __fmul_rn(c.sh->warp_seg[w], factor);
-    wbase = acc;
-    if (nxt > r) { wsel = w; break; }
+    const float seg = c.sh->warp_seg[w], nxt = acc + __fmul_rn(seg, factor);
+    if (seg > 0.0f) { wsel = w; wbase = acc; }
+    if (nxt > r) break;
     acc = nxt;
   }
   if (c.warp != wsel) return;
