@@ -474,10 +474,12 @@ __device__ void cdf_search(Ctx& c, const float* __restrict__ row, const float* _
           a += p[u].y; if (h < 0 && a > r) h = i + 1;
           a += p[u].z; if (h < 0 && a > r) h = i + 2;
           a += p[u].w; if (h < 0 && a > r) h = i + 3;
-          if (h < 0) h = lp;                     // the lane's own sum rounds differently from its four steps
           const int src = __ffs(over) - 1;
           hit = __shfl_sync(0xffffffffu, h, src);
-          if (hit < 0) hit = b0 + 128 * u + 4 * src;
+          if (hit < 0) {   // the scan rounds differently from the lane's steps: the last element up to here that carries probability
+            const uint32_t upto = pos & (0xffffffffu >> (31 - src));
+            hit = upto ? __shfl_sync(0xffffffffu, lp, 31 - __clz(upto)) : last_pos;
+          }
         }
         if (pos) last_pos = __shfl_sync(0xffffffffu, lp, 31 - __clz(pos));
         acc += __shfl_sync(0xffffffffu, x, 31);

@@ -107,3 +107,46 @@ def test_resampled_token_between_the_sums_of_a_cta_and_its_warps(pool, V):  # no
     assert n_acc.tolist() == [0] * n
     assert np.isfinite(rows[np.arange(n), got]).all(), "a token without probability: %s" % got
     assert got.tolist() == want.tolist()
+
+
+def lanes_that_cross_without_probability(n, seed, V, per_lane):
+    """Rows of V <= 128 (one warp) whose scan over the lanes rounds up at a lane without probability, and the draws below that."""
+    rng = np.random.default_rng(seed)
+    rows, draws, want = np.full((n, V), -np.inf, F), np.zeros(n, F), np.zeros(n, np.int32)
+    lanes = V // 4
+    for b in range(n):
+        while True:
+            has = rng.random(lanes) < 0.6
+            at = 4 * np.flatnonzero(has) + rng.integers(0, 4, has.sum())
+            logit = (-3.0 * rng.random(len(at))).astype(F)
+            e = fastexp(logit - logit.max())
+            part = np.zeros(32, F)      # the warp's sum, a butterfly over what its lanes have read
+            if per_lane == 4:
+                part[np.flatnonzero(has)] = e
+            else:
+                for j in range(0, V, 32):
+                    inside = (at >= j) & (at < j + 32)
+                    part[at[inside] - j] = (part[at[inside] - j] + e[inside]).astype(F)
+            for o in (16, 8, 4, 2, 1):
+                part = (part + part[np.arange(32) ^ o]).astype(F)
+            factor = F(F(1.0) / part[0])
+            x = np.zeros(32, F)
+            x[np.flatnonzero(has)] = (e * factor).astype(F)
+            for o in (1, 2, 4, 8, 16):
+                x = np.concatenate([x[:o], (x[o:] + x[:-o]).astype(F)])
+            top = np.maximum.accumulate(x)
+            odd = [j for j in range(1, lanes - 1) if not has[j] and x[j] > top[j - 1] > 0 and top[-1] > x[j]]
+            if odd:
+                break
+        rows[b, at] = logit
+        draws[b], want[b] = top[odd[0] - 1], at[at < 4 * odd[0]].max()
+    return rows, draws, want
+
+
+@pytest.mark.parametrize("V,per_lane", [(128, 4), (127, 1)])     # vectors, and single loads
+def test_sampled_token_where_a_lane_without_probability_crosses(pool, V, per_lane):  # noqa: F811
+    rows, draws, want = lanes_that_cross_without_probability(16, V, V - V % 4, per_lane)
+    rows = np.concatenate([rows, np.full((16, V % 4), -np.inf, F)], axis=1)
+    got = pool.sample(rows, draws)
+    assert np.isfinite(rows[np.arange(len(got)), got]).all(), "a token without probability: %s" % got
+    assert got.tolist() == want.tolist()
