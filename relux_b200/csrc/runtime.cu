@@ -435,6 +435,16 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
 int32_t convert_layout(Device* dev, const void* src, void* dst, int n, int S, int H, int D, int src_dtype, int dst_dtype,
                        int src_layout, int dst_layout);
 
+// A pointer that a caller gave as host memory but the host cannot write: the runtime's copies find out by themselves, memcpy not.
+static bool is_device_memory(const void* ptr) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice;
+}
+
 static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const StepAppend* step = nullptr, const GqaAppend* gstep = nullptr) {
   if (!a) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
   if (p->prm.kind != kind) { set_error("pool kind does not match this attention call"); return RELUX_ERR_INVALID_ARG; }
@@ -537,7 +547,8 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   // kernels' TMA stores and the reference kernels keep to device memory)
   const size_t out_bytes = out_elems * dtype_size(a->out_dtype);
   const bool by_kernel = a->out_mem == RELUX_MEM_HOST && !piped_out && out_bytes <= Device::kHostOutBytes && p->dev->host_out &&
-                         (need_conv || (a->mode == RELUX_ATTN_FAST && (gqa_stream || (kind == RELUX_POOL_MLA && !mla_prefill_eligible(p, sb, *a)))));
+                         (need_conv || (a->mode == RELUX_ATTN_FAST && (gqa_stream || (kind == RELUX_POOL_MLA && !mla_prefill_eligible(p, sb, *a))))) &&
+                         !is_device_memory(a->out);
   int slot_out = -1;
   char* out_block = nullptr;   // [kernel output | converted output]
   if (direct) kout = a->out;

@@ -44,3 +44,28 @@ def test_gqa_result_in_host_memory_equals_the_one_in_device_memory(dev, B, S, ou
     assert np.abs(want.astype(np.float32)).max() > 0 and pool.status() == 0
     buf.free()
     pool.destroy()
+
+
+def test_device_memory_given_as_host_memory_is_copied_to(dev):
+    """The copy behind a kernel takes whatever address it is given; a result by way of page-locked memory does too."""
+    import ctypes as C
+
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    rng = np.random.default_rng(3)
+    pool = rb.Pool(dev, L.POOL_GQA, 1, 3, 64, 1, 3, num_kv_heads=HKV, head_dim=D)
+    pool.set_tables(np.arange(3, dtype=np.int32).reshape(1, 3))
+    pool.append(0, rng.standard_normal((100, HKV, D)).astype(np.float32), rng.standard_normal((100, HKV, D)).astype(np.float32), 1,
+                n_new=np.asarray([100], np.int32))
+    q = rng.standard_normal((1, 1, H, D)).astype(np.float32)
+    out = np.zeros_like(q)
+    pool.decode(0, 1, q, out, H, D, D ** -0.5)
+    buf = dev.alloc(out.nbytes, L.DTYPE_F32)
+    args = pool._attn_args(0, 1, q, None, out, H, D, D ** -0.5, 1, 0, True, L.ATTN_FAST, None, None, None, L.LAYOUT_TOKEN_MAJOR,
+                           L.LAYOUT_TOKEN_MAJOR, None, None)
+    args.out = buf.ptr
+    assert args.out_mem == L.MEM_HOST
+    L.check(pool.lib.relux_gqa_decode(pool.h, C.byref(args)))
+    assert np.array_equal(buf.download(out.shape, np.float32), out) and pool.status() == 0
+    buf.free()
+    pool.destroy()
