@@ -43,9 +43,10 @@
 // shuffles and two pairs of eight 303 and 229.  Not kept: the two halves of the softmax warps on alternate tiles, a whole row
 // per thread (8 % slower or worse with two, three S buffers, one O): the diagonal tiles and the item ends, serial there, cost
 // more than the overlap gave.  Holding one warp of a scheduler back by half a phase changed nothing.
-// Barriers: full barriers live in the leader CTA and count the bytes of both CTAs' loads; empty / s_full / pv_done /
+// Barriers: full barriers live in the leader CTA and count the bytes of both CTAs' loads; empty / s_full /
 // o_full barriers live in each CTA and are armed by tcgen05.commit with mbarrier multicast (not a TMA load); p_full and
-// o_empty live in the leader and count warps of both CTAs.  No TMA multicast anywhere.
+// o_empty live in the leader and count warps of both CTAs.  s_full of a tile counts its QK^T and the PV two tiles before it, so
+// that every phase of it is waited for.  No TMA multicast anywhere.
 // No split-KV: the output is normalised in the read-out and written once.
 // Every wait is bounded (status RELUX_ERR_TIMEOUT, shared abort flag, all warps still reach the end and free TMEM).
 //
@@ -114,7 +115,7 @@ constexpr float kRescaleThreshold = 8.0f;
 constexpr int kPolyPairsOf8 = RELUX_PREFILL_POLY_PAIRS;   // score pairs out of every eight whose exponential runs on the FMA pipe
 
 struct Bars {
-  uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full[2], pv_done;
+  uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full[2];
   uint64_t o_full[2], o_empty[2], l_full, l_empty, drain;
   uint32_t tmem_base;
   volatile int32_t abort_flag;
@@ -291,10 +292,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       mbar_init(&bars->v_full[s], 1);
       mbar_init(&bars->v_empty[s], 1);
     }
-    mbar_init(&bars->s_full[0], 1);
-    mbar_init(&bars->s_full[1], 1);
+    for (int s = 0; s < 2; s++) mbar_init(&bars->s_full[s], 2);                  // QK of this tile and PV of the tile two before it
     for (int s = 0; s < 2; s++) mbar_init(&bars->p_full[s], 2 * kSoftmaxWarps);   // one arrival per softmax warp of each CTA of the pair
-    mbar_init(&bars->pv_done, 1);
     for (int s = 0; s < 2; s++) {
       mbar_init(&bars->o_full[s], 1);
       mbar_init(&bars->o_empty[s], 2 * kEpiWarps);   // the read-out warps of both CTAs (leader's copy is the one waited on)
@@ -304,6 +303,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     mbar_init(&bars->drain, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
+    for (int s = 0; s < 2; s++) mbar_arrive(&bars->s_full[s]);   // no PV before the first two tiles
   }
   if (warp == 0) {
     tmem_alloc<2>(&bars->tmem_base, kTmemCols);
@@ -446,7 +446,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           for (int ks = 0; ks < 8; ks++)
             umma_ts<2>(tmem + kTmemO + (n & 1) * 128, tP + ks * 8, dV + ((uint32_t)(ks * 2048) >> 4), idesc_pv, !first || ks != 0);
           umma_commit_mc<2>(&bars->v_empty[st], 0x3);
-          umma_commit_mc<2>(&bars->pv_done, 0x3);
+          umma_commit_mc<2>(&bars->s_full[g & 1], 0x3);   // the other half of s_full(g+2)
           if (last) umma_commit_mc<2>(&bars->o_full[n & 1], 0x3);
         }
         __syncwarp();
@@ -459,6 +459,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         for (int i = 0; i < ntiles; i++, g++) {
           if (i + 1 < ntiles) issue_qk(g + 1, n, false, i + 2 == ntiles);
           else if (next_tiles > 0) issue_qk(g + 1, n + 1, true, next_tiles == 1);
+          else if (el) umma_commit_mc<2>(&bars->s_full[(g + 1) & 1], 0x3);   // no tile behind the worker's last: what it waits for is PV(g-1)
           issue_pv(g, n, i == 0, i + 1 == ntiles);
         }
         ntiles = next_tiles;
@@ -575,10 +576,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           l_run[k] += ps0 + ps1;
         }
         // The TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep
-        // their maximum multiply by one.  O may be rescaled only after PV(g-1) has completed; PV(g-2) has: QK(g), whose scores
-        // are in, was issued behind it.
+        // their maximum multiply by one.  O may be rescaled only after PV(g-1) has completed: s_full(g+1) says so, and QK(g+1),
+        // issued right behind it, is as good as done by now.  (Phases are told apart by parity alone, so a barrier of its own for PV
+        // would have to be waited for in every tile, 1.3 % of a prompt's time; s_full is.)
         if (__any_sync(0xffffffffu, rescale)) {
-          wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
+          wait_bar(&bars->s_full[(g + 1) & 1], ((g + 1) >> 1) & 1, bars, prm.status);
           __syncwarp();
           tc_fence_after();
 #pragma unroll 1
