@@ -500,7 +500,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       for (int j = 0; j < it.ntiles; j++, g++) {
         const uint32_t tmem_s = tmem + lane_addr + kTmemS + (g & 1) * 128;
         wait_bar(&bars->s_full[g & 1], (g >> 1) & 1, bars, prm.status);
-        __syncwarp();   // the TMEM loads below are warp-collective
         tc_fence_after();
         uint32_t sv[64];
         tmem_ld_16x256b_x16(tmem_s, sv);
@@ -567,7 +566,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         uint32_t pw[32];
         if (whole) exp_quads<true>(sv, scale2, neg_m2, pw, ps2);
         else exp_quads<false>(sv, scale2, neg_m2, pw, ps2);
-        __syncwarp();   // the store is warp-collective
         tmem_st_16x128b_x16(tmem_s, pw);
 #pragma unroll
         for (int k = 0; k < 2; k++) {
@@ -581,7 +579,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         // would have to be waited for in every tile, 1.3 % of a prompt's time; s_full is.)
         if (__any_sync(0xffffffffu, rescale)) {
           wait_bar(&bars->s_full[(g + 1) & 1], ((g + 1) >> 1) & 1, bars, prm.status);
-          __syncwarp();
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < kD; c += 64) {
@@ -635,7 +632,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->l_empty);
       wait_bar(&bars->o_full[n & 1], (n >> 1) & 1, bars, prm.status);
-      __syncwarp();   // the TMEM loads below are warp-collective
       tc_fence_after();
       const bool ok = !__any_sync(0xffffffffu, bars->abort_flag != 0);
       const float inv = (ok && l_row > 0.f) ? 1.f / l_row : 0.f;
@@ -667,7 +663,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     } while (w.next());
     if (lane == 0) tma_store_wait_all();
   }
-  __syncwarp();
   tc_fence_before();
   cluster_sync();
   if (threadIdx.x == 0) stamp_end(prm.time);

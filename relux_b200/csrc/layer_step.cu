@@ -268,7 +268,6 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
       const int m_end = min(NT, prm.M - m0);
       float* dst = prm.part + ((size_t)walk.split * prm.M + m0) * prm.n_total + prm.col_first[j] + n;
       gemm_wait(&bars->acc_full[piece & 1], (piece >> 1) & 1, bars, prm.status);
-      __syncwarp();   // the TMEM loads below are warp-collective
       tc_fence_after();
       const bool ok = !bars->abort_flag, mine = n < prm.n_cols[j];
 #pragma unroll 1

@@ -374,7 +374,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       for (int i = 0; i < ntiles; i++, g++) {
         // no thread leaves this loop early: every thread must reach the same named barriers
         wait_bar(&bars->s_full[g & 1], (g >> 1) & 1, bars, prm.status);
-        __syncwarp();   // the TMEM loads below are warp-collective
         tc_fence_after();
         uint32_t sv[2][32];
         tmem_ld_32x32b_x32(tmem + lane_addr + kTmemS + (g & 1) * 64, sv[0]);

@@ -263,7 +263,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll 1
         for (int round = 0; round < kARounds; round++, na++) {
           wait_bar(&bars->a_full, na & 1, bars, prm.status);
-          __syncwarp();
 #pragma unroll 1
           for (int j2 = half * (kABlocks / 2); j2 < (half + 1) * (kABlocks / 2); j2++) {
             uint32_t w[32];
@@ -290,7 +289,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       }
       const int buf = n & 1;
       wait_bar(&bars->acc_full[buf], (n >> 1) & 1, bars, prm.status);
-      __syncwarp();   // the TMEM loads below are warp-collective
       tc_fence_after();
       // the stores of the previous unit have read the shared tile
       if (storer) tma_store_wait_read();
@@ -325,7 +323,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
     if (storer) tma_store_wait_all();
   }
-  __syncwarp();
   tc_fence_before();
   cluster_sync();
   if (warp == 0) tmem_dealloc<2>(tmem, kTmemCols);

@@ -23,6 +23,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Address of the same shared-memory variable in CTA `cta` of this cluster (shared::cluster window).
@@ -65,9 +66,12 @@ __device__ __forceinline__ void tma_load_2d_2sm(void* smem_dst, const CUtensorMa
 }
 
 // ---- tensor memory -------------------------------------------------------------------------------
+// These instructions are collective over the warp (.sync.aligned): all lanes must execute the same one together.  Each wrapper
+// that may follow a lane's branch (a wait, an elected lane's store) therefore brings the warp together itself.
 // kGroup = 1: one CTA; kGroup = 2: CTA pair (one warp of EACH CTA executes the call with the same slot offset).
 template <int kGroup>
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot_smem, uint32_t ncols) {
+  __syncwarp();
   if constexpr (kGroup == 1)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_smem)), "r"(ncols) : "memory");
   else
@@ -80,6 +84,7 @@ __device__ __forceinline__ void tmem_relinquish() {
 }
 template <int kGroup>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+  __syncwarp();
   if constexpr (kGroup == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
   else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
@@ -90,6 +95,7 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 
 // Warp w of a warpgroup reads TMEM lanes 32w..32w+31; thread t gets lane 32w+t, 32 consecutive 32-bit columns.
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -102,6 +108,7 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -116,6 +123,7 @@ __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_
 // 16 TMEM lanes (either half of the warp's 32) x 8 kNum columns, four lanes to a row: lane l gets columns 8 i + 2 (l & 3) + {0, 1}
 // of row l / 4 in v[4 i], v[4 i + 1] and of row l / 4 + 8 in v[4 i + 2], v[4 i + 3].
 __device__ __forceinline__ void tmem_ld_16x256b_x16(uint32_t taddr, uint32_t (&v)[64]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -134,6 +142,7 @@ __device__ __forceinline__ void tmem_ld_16x256b_x16(uint32_t taddr, uint32_t (&v
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&v)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -146,6 +155,7 @@ __device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&v)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_16x256b_x8(uint32_t taddr, const uint32_t (&v)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -159,6 +169,7 @@ __device__ __forceinline__ void tmem_st_16x256b_x8(uint32_t taddr, const uint32_
 // The same rows, one column per lane of every four: lane l writes column 4 i + (l & 3) of row l / 4 from v[2 i] and of row
 // l / 4 + 8 from v[2 i + 1].
 __device__ __forceinline__ void tmem_st_16x128b_x16(uint32_t taddr, const uint32_t (&v)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.16x128b.x16.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
