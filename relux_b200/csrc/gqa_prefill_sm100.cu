@@ -109,10 +109,7 @@ constexpr int kThreads = 32 * kSoftmaxWarps + 64 + 32 * kEpiWarps;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemS = 0, kTmemO = 256;                  // S(g) at kTmemS + 128 (g & 1); O of item n at kTmemO + 128 (n & 1)
 constexpr float kRescaleThreshold = 8.0f;
-#ifndef RELUX_PREFILL_POLY_PAIRS
-#define RELUX_PREFILL_POLY_PAIRS 2
-#endif
-constexpr int kPolyPairsOf8 = RELUX_PREFILL_POLY_PAIRS;   // score pairs out of every eight whose exponential runs on the FMA pipe
+constexpr int kPolyPairsOf8 = 2;   // score pairs out of every eight whose exponential runs on the FMA pipe
 
 struct Bars {
   uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full[2];
@@ -131,7 +128,7 @@ struct PrefillParams {
   int32_t num_pages, Hkv, H, g, S, extra, causal;
   int32_t bq;                 // query tokens per block = 128 / g
   int32_t n_qblocks, n_pairs; // blocks and block pairs per (sequence, kv head)
-  int32_t n_seqs, n_items;    // items = n_pairs * Hkv * n_seqs
+  int32_t n_seqs;
   int32_t n_half, n_couples;  // couples per (sequence, kv head) = ceil(n_pairs / 2), and in all
   int32_t krow0, vrow0;       // first TMA row of this layer's K block / V block (MLA: of the expanded keys / values)
   // MLA only: expanded rows are dense, row = head * Ttot + seq_base[sequence] + token; the RoPE part of a key is read from
@@ -482,9 +479,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full[0]), 0);
     const int tq[2] = {row[0] / prm.g, row[1] / prm.g};              // token in block
     const uint64_t scale2 = pack2(prm.scale_log2, prm.scale_log2);
-#ifdef STAG
-    if (warp >= 4) { const long long c0 = clock64(); while (clock64() - c0 < STAG) {} __syncwarp(); }
-#endif
     int g = 0;
     Walk<kMla> w(prm, worker, n_workers);
     do {
@@ -752,7 +746,6 @@ int32_t launch_gqa_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.n_seqs = sb.n_seqs;
   const int64_t items = (int64_t)k.n_pairs * prm.gqa_num_kv_heads * sb.n_seqs;
   if (items > ((int64_t)1 << 30)) { set_error("prompt too long for one prefill launch"); return RELUX_ERR_UNSUPPORTED; }
-  k.n_items = (int32_t)items;
   k.n_half = (k.n_pairs + 1) / 2;
   k.n_couples = k.n_half * prm.gqa_num_kv_heads * sb.n_seqs;
   const int64_t rows_per_block = (int64_t)prm.num_pages * prm.gqa_num_kv_heads * kPage;
@@ -843,7 +836,6 @@ int32_t launch_mla_prefill_sm100(Pool* p, const SeqBatch& sb, const relux_attn_a
   k.n_seqs = sb.n_seqs;
   const int64_t items = (int64_t)k.n_pairs * H * sb.n_seqs;
   if (items > ((int64_t)1 << 30)) { set_error("prompt too long for one prefill launch"); return RELUX_ERR_UNSUPPORTED; }
-  k.n_items = (int32_t)items;
   k.n_half = (k.n_pairs + 1) / 2;
   k.n_couples = k.n_half * H * sb.n_seqs;
   k.krow0 = 0;
