@@ -68,10 +68,13 @@ struct SelShared {
   float stat[kStatMax];       // batched statistics: of draft position i the sums (draft, target) at 4 i, the maxima at 4 i + 2
 };
 
-__device__ __forceinline__ uint32_t order_key(float x) {
+// Keys that order like the values, by their bits alone (-0 below 0) ...
+__device__ __forceinline__ uint32_t bit_key(float x) {
   uint32_t u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+// ... and with both zeros equal, as the reference's comparisons have them: what a threshold is compared with.
+__device__ __forceinline__ uint32_t order_key(float x) { return bit_key(__fadd_rn(x, 0.0f)); }
 
 // fastexp32 of what is at most 0 (or NaN): a difference to a maximum.  Above 0 its result means nothing.
 __device__ __forceinline__ float fastexp32_below(float x) {
@@ -522,7 +525,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   // The largest element per thread, as a key (the division by the temperature keeps the order, so it is made once, behind the
   // pass).  Of long slices, pairs of threads: half as many keys to rank.
   uint32_t key = 0;
-  for_segment(c, row, [&](int, float v) { key = max(key, order_key(v)); });
+  for_segment(c, row, [&](int, float v) { key = max(key, bit_key(v)); });
   if (key) {
     const uint32_t u = (key & 0x80000000u) ? (key & 0x7fffffffu) : ~key;
     key = order_key(d.scaled(__uint_as_float(u)));
