@@ -90,18 +90,6 @@ struct MlaSm100Params {
   TimeStamp time;
 };
 
-// Barrier of the 128 softmax threads that tells all of them whether any brought `yes`.
-__device__ __forceinline__ bool softmax_any(bool yes) {
-  uint32_t any;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
-      "barrier.cta.red.or.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(any)
-      : "r"((uint32_t)yes)
-      : "memory");
-  return any != 0;
-}
-
 // Bounded wait.  The common case (phase already complete) is a single try_wait.  When the bound runs out the
 // waiter records RELUX_ERR_TIMEOUT, raises the CTA's abort flag and RETURNS: nobody leaves a loop early, every
 // later wait sees the flag on its first failed poll and returns at once, so all warps still reach the named
@@ -398,20 +386,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 #pragma unroll
             for (int k = 0; k < 4; k++) mx4[k] = max3(mx4[k], __uint_as_float(sv[h2][j + 2 * k]), __uint_as_float(sv[h2][j + 2 * k + 1]));
         float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * prm.scale_log2;
-        // Lazily updated running max.  The two threads of a row meet only in a tile that raises some row's (the first one with a
-        // visible token does, m_used = -inf): in all others the barrier itself says that there is none.  Both take the same decision.
+        // (a barrier that votes first, with the exchange only behind a yes, took as long per tile and 1 % longer per item: every
+        // item's first tile is one)
+        bars->rowmax[g & 1][hf][row] = mx;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        mx = fmaxf(mx, bars->rowmax[g & 1][hf ^ 1][row]);
+        // lazily updated running max: both threads of a row take the same decision
         float alpha = 1.f;
         bool rescale = false;
-        const bool raised = softmax_any(mx > m_used + kRescaleThreshold);
-        if (raised) {
-          bars->rowmax[g & 1][hf][row] = mx;
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          mx = fmaxf(mx, bars->rowmax[g & 1][hf ^ 1][row]);
-          if (mx > m_used + kRescaleThreshold) {
-            alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
-            rescale = (m_used != -INFINITY);
-            m_used = mx;
-          }
+        if (mx > m_used + kRescaleThreshold) {   // also true on the first tile with a visible token (m_used = -inf)
+          alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
+          rescale = (m_used != -INFINITY);
+          m_used = mx;
         }
         // p = 2^(s * scale_log2 - m), two scores an instruction but for the exponentials
         const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
@@ -436,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         if (g > 0) wait_bar(&bars->pv_done, (g - 1) & 1, bars, prm.status);
         // TMEM loads and stores are warp-collective: the decision is taken for the whole warp, and the rows that keep their
         // maximum multiply by one
-        if (raised && __any_sync(0xffffffffu, rescale && i > 0)) {
+        if (__any_sync(0xffffffffu, rescale && i > 0)) {
           const float a_row = rescale ? alpha : 1.f;
           tc_fence_after();
 #pragma unroll 1
