@@ -547,8 +547,7 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   // kernels' TMA stores and the reference kernels keep to device memory)
   const size_t out_bytes = out_elems * dtype_size(a->out_dtype);
   const bool by_kernel = a->out_mem == RELUX_MEM_HOST && !piped_out && out_bytes <= Device::kHostOutBytes && p->dev->host_out &&
-                         (need_conv || (a->mode == RELUX_ATTN_FAST && (gqa_stream || (kind == RELUX_POOL_MLA && !mla_prefill_eligible(p, sb, *a))))) &&
-                         !is_device_memory(a->out);
+                         (need_conv || (a->mode == RELUX_ATTN_FAST && (gqa_stream || (kind == RELUX_POOL_MLA && !mla_prefill_eligible(p, sb, *a)))));
   int slot_out = -1;
   char* out_block = nullptr;   // [kernel output | converted output]
   if (direct) kout = a->out;
@@ -599,8 +598,10 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
       po.used[slot_out] = true;
       dev->copies_in_flight = true;
     } else if (by_kernel) {
+      const bool dev_mem = is_device_memory(a->out);   // asked while the kernels run: 0.7 us of host time before them
+      if (dev_mem) RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, p->dev->host_out, out_bytes, cudaMemcpyDefault, p->dev->stream));
       RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
-      memcpy(a->out, p->dev->host_out, out_bytes);
+      if (!dev_mem) memcpy(a->out, p->dev->host_out, out_bytes);
     } else if (a->out_mem == RELUX_MEM_HOST) {
       RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_bytes, cudaMemcpyDeviceToHost, p->dev->stream));
       RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
