@@ -73,10 +73,13 @@ __device__ __forceinline__ uint32_t bit_key(float x) {
   uint32_t u = __float_as_uint(x);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-// ... and with both zeros equal, as the reference's comparisons have them: what a threshold is compared with.
+// ... and with both zeros equal, as the reference's comparisons have them: what is counted for a threshold.  A threshold at 0 then lets
+// the keys by bits of both pass, so that the passes compare these (an addition per element cost 1 % of a nucleus call).
 __device__ __forceinline__ uint32_t order_key(float x) { return bit_key(__fadd_rn(x, 0.0f)); }
+__device__ __forceinline__ uint32_t with_both_zeros(uint32_t threshold) { return threshold == 0x80000000u ? 0x7fffffffu : threshold; }
 
-// fastexp32 of what is at most 0 (or NaN): a difference to a maximum.  Above 0 its result means nothing.
+// fastexp32 without its upper cut: good up to 88, past which the bits are those of no finite number.  Arguments are differences to a
+// row's maximum, or to a guess of it; a sum against a guess is used only where that lies less than 80 below.
 __device__ __forceinline__ float fastexp32_below(float x) {
   const float t = __fadd_rn(__fmul_rn(12102203.0f, x), 1064948224.0f);
   return x < -87.0f ? 0.0f : __uint_as_float((uint32_t)__float2int_rz(t));
@@ -92,7 +95,7 @@ struct Dist {
   __device__ __forceinline__ float scaled(float v) const { return temp == 1.0f ? v : __fdiv_rn(v, temp); }
   __device__ __forceinline__ float p1(float v) const {
     float x = scaled(v);
-    if (order_key(x) < topk_key) return 0.0f;
+    if (bit_key(x) < topk_key) return 0.0f;
     return __fmul_rn(fastexp32_ref(__fsub_rn(x, m)), inv1);
   }
 };
@@ -467,22 +470,19 @@ __device__ void cdf_search(Ctx& c, const float* __restrict__ row, const float* _
       const int i = b0 + 128 * u + 4 * c.lane;
       // the last element so far that carries probability: what is taken when rounding puts the crossing past the end
       const int lp = p[u].w > 0.0f ? i + 3 : p[u].z > 0.0f ? i + 2 : p[u].y > 0.0f ? i + 1 : p[u].x > 0.0f ? i : -1;
-      const uint32_t pos = __ballot_sync(0xffffffffu, lp >= 0), over = __ballot_sync(0xffffffffu, acc + x > r);
+      // (lanes without probability do not count: their x is a sum in another order, and may lie above the lane's before them)
+      const uint32_t pos = __ballot_sync(0xffffffffu, lp >= 0), over = __ballot_sync(0xffffffffu, lp >= 0 && acc + x > r);
       if (hit < 0) {
         if (over) {
           const float before = __shfl_up_sync(0xffffffffu, x, 1);
           float a = acc + (c.lane > 0 ? before : 0.0f);
           int h = -1;
-          a += p[u].x; if (h < 0 && a > r) h = i;
-          a += p[u].y; if (h < 0 && a > r) h = i + 1;
-          a += p[u].z; if (h < 0 && a > r) h = i + 2;
-          a += p[u].w; if (h < 0 && a > r) h = i + 3;
-          const int src = __ffs(over) - 1;
-          hit = __shfl_sync(0xffffffffu, h, src);
-          if (hit < 0) {   // the scan rounds differently from the lane's steps: the last element up to here that carries probability
-            const uint32_t upto = pos & (0xffffffffu >> (31 - src));
-            hit = upto ? __shfl_sync(0xffffffffu, lp, 31 - __clz(upto)) : last_pos;
-          }
+          a += p[u].x; if (h < 0 && a > r && p[u].x > 0.0f) h = i;
+          a += p[u].y; if (h < 0 && a > r && p[u].y > 0.0f) h = i + 1;
+          a += p[u].z; if (h < 0 && a > r && p[u].z > 0.0f) h = i + 2;
+          a += p[u].w; if (h < 0 && a > r && p[u].w > 0.0f) h = i + 3;
+          if (h < 0) h = lp;                     // the lane's own sum rounds differently from its four steps
+          hit = __shfl_sync(0xffffffffu, h, __ffs(over) - 1);
         }
         if (pos) last_pos = __shfl_sync(0xffffffffu, lp, 31 - __clz(pos));
         acc += __shfl_sync(0xffffffffu, x, 31);
@@ -516,7 +516,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   auto collect = [&](uint32_t key_lo) {
     for_segment(c, row, [&](int i, float v) {
       const float x = d.scaled(v);
-      if (order_key(x) >= key_lo) {
+      if (bit_key(x) >= key_lo) {
         const uint32_t pos = atomicAdd(&sh.list_count, 1u);
         if (pos < (uint32_t)kCandCap) { l_val[pos] = x; l_idx[pos] = i; }
       }
@@ -528,7 +528,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   for_segment(c, row, [&](int, float v) { key = max(key, bit_key(v)); });
   if (key) {
     const uint32_t u = (key & 0x80000000u) ? (key & 0x7fffffffu) : ~key;
-    key = order_key(d.scaled(__uint_as_float(u)));
+    key = bit_key(d.scaled(__uint_as_float(u)));
   }
   const bool pairs = c.hi - c.lo > 8 * kSelThreads;
   const int m = (topk + c.csize - 1) / c.csize;
@@ -554,6 +554,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   cl.sync();
   uint32_t bound = 0xffffffffu;
   for (int q = 0; q < c.csize; q++) bound = min(bound, *cl.map_shared_rank(&sh.list_bound, q));
+  bound = with_both_zeros(bound);
   if (key >= bound) collect(bound);
   __syncthreads();
   cl.sync();
@@ -567,7 +568,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
     if (n_ge > (uint32_t)kCandCap) return false;     // more ties at the threshold than the list holds
     if (threadIdx.x == 0) sh.list_count = 0;
     __syncthreads();
-    collect(key_lo);
+    collect(with_both_zeros(key_lo));
     __syncthreads();
     cl.sync();
   }
@@ -760,7 +761,7 @@ __device__ void sample_row(Ctx& c, const SelParams& prm, const float* __restrict
   if (topk > 0) {
     uint32_t key = 0;
     radix_select<false>(c, row, [&](float v, uint32_t& k, float& w) { k = order_key(d.scaled(v)); w = 0.0f; }, (uint32_t)topk, 0.0f, &key);
-    d.topk_key = key;
+    d.topk_key = with_both_zeros(key);
   }
   float v4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   for_segment(c, row, [&](int, float v) { v4[0] = fmaxf(v4[0], v); });

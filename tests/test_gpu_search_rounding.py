@@ -1,6 +1,6 @@
 """The inverse-CDF search where its levels round differently: the sums of CTAs, warps, lanes and elements are float32 sums of the same
 probabilities in different orders, so a draw can lie between two of them.  Whatever level says that the draw is crossed, the token
-returned is the last one at or before that point that carries probability, never one with none.
+returned is a neighbour of that point that carries probability, never one with none.
 
 The rows hold one finite logit per warp (or lane), everything else is -inf, so that each sum can be repeated on the host in float32."""
 import numpy as np
@@ -139,7 +139,7 @@ def lanes_that_cross_without_probability(n, seed, V, per_lane):
             if odd:
                 break
         rows[b, at] = logit
-        draws[b], want[b] = top[odd[0] - 1], at[at < 4 * odd[0]].max()
+        draws[b], want[b] = top[odd[0] - 1], at[at > 4 * odd[0]].min()   # the next one adds what takes the sum past the draw
     return rows, draws, want
 
 
