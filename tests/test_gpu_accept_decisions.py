@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [3, 30])           # all positions in one stage, and one by one
-@pytest.mark.parametrize("V", [777, 4096])       # single loads, and vectors
+@pytest.mark.parametrize("V", [777, 4096, 9001, 50256])       # single loads, and vectors; clusters of one, two, four and eight CTAs
 @pytest.mark.parametrize("tokens", ["largest", "drawn", "far"])
 def test_decisions_next_to_the_boundary(pool, oracle, n, V, tokens):  # noqa: F811
     rng = np.random.default_rng(V + n + len(tokens))

@@ -69,3 +69,38 @@ def test_device_memory_given_as_host_memory_is_copied_to(dev):
     assert np.array_equal(buf.download(out.shape, np.float32), out) and pool.status() == 0
     buf.free()
     pool.destroy()
+
+
+# 512 KB is 8 rows of 128 heads x 128 float32; three query tokens of head-major rows go through the conversion
+@pytest.mark.parametrize("B,S", [(1, 1), (8, 1), (9, 1), (2, 3), (3, 3)])
+@pytest.mark.parametrize("out_dtype", [np.float32, np.uint16])
+@pytest.mark.parametrize("head_major", [False, True])
+@pytest.mark.parametrize("generic", [0, 1])    # the merge that projects up, and the kernels for other shapes
+def test_latent_result_in_host_memory_equals_the_one_in_device_memory(dev, B, S, out_dtype, head_major, generic):
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    from oracle import binding as orc
+    H, DC, DHR = 128, 512, 64
+    rng = np.random.default_rng(B * 17 + S)
+    lens = rng.integers(S, 150, B).astype(np.int32)
+    pool = rb.Pool(dev, L.POOL_MLA, 1, B * 3, 64, B, 3, dC=DC, dHR=DHR)
+    pool.set_tables(rng.permutation(B * 3).astype(np.int32).reshape(B, 3))
+    pool.tune(L.TUNE_MLA_GENERIC, generic)
+    rows = int(lens.sum())
+    pool.append(0, rng.standard_normal((rows, DC)).astype(np.float32), rng.standard_normal((rows, DHR)).astype(np.float32), B, n_new=lens)
+    w = [dev.upload(orc.bf16_from_f32(0.02 * rng.standard_normal((DC, H * D)).astype(np.float32))) for _ in range(2)]
+    shape = (B, H, S, D) if head_major else (B, S, H, D)
+    q = rng.standard_normal(shape).astype(np.float32)
+    qr = rng.standard_normal(shape[:3] + (DHR,)).astype(np.float32)
+    lay = L.LAYOUT_HEAD_MAJOR if head_major else L.LAYOUT_TOKEN_MAJOR
+    kw = dict(q_rope=qr, w_uk=w[0], w_uv=w[1], q_tokens=S, q_layout=lay, out_layout=lay)
+    out = np.zeros(shape, out_dtype)
+    pool.decode(0, B, q, out, H, D, (D + DHR) ** -0.5, **kw)
+    buf = dev.alloc(out.nbytes, L.DTYPE_F32 if out_dtype == np.float32 else L.DTYPE_BF16)
+    pool.decode(0, B, q, buf, H, D, (D + DHR) ** -0.5, **kw)
+    dev.sync()
+    assert np.array_equal(out, buf.download(shape, out_dtype))
+    assert out.any() and pool.status() == 0
+    for x in (buf, *w):
+        x.free()
+    pool.destroy()

@@ -42,3 +42,43 @@ def test_gqa_prompt_with_rising_scores(dev, oracle, H, Hkv, S, cached, rise):  #
     check_attention(out, ref, "rising scores", max_tol=EDGE_MAX, mean_tol=EDGE_MEAN)
     assert pool.status() == 0
     pool.destroy()
+
+
+# the 192-wide kernel over expanded rows: one block pair, several, rows past the last token, a cached part before
+@pytest.mark.parametrize("S,cached", [(128, 0), (300, 64), (131, 517), (1100, 0)])
+@pytest.mark.parametrize("rise", [3.0, 14.0])
+def test_mla_prompt_with_rising_scores(dev, oracle, S, cached, rise):  # noqa: F811
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    rng = np.random.default_rng(S)
+    H, DH, DC, DHR, P, B = 16, 128, 512, 64, 64, 2
+    scale = (DH + DHR) ** -0.5
+    ctx = np.asarray([cached + S, cached + S + 37], np.int32)
+    T = int(ctx.max())
+    pages = (T + P - 1) // P
+    pool = rb.Pool(dev, L.POOL_MLA, 1, B * pages, P, B, pages, dC=DC, dHR=DHR)
+    pool.set_tables(rng.permutation(B * pages).astype(np.int32).reshape(B, pages))
+    c = 0.3 * rng.standard_normal((B, T, DC)).astype(np.float32)
+    r = 0.3 * rng.standard_normal((B, T, DHR)).astype(np.float32)
+    r[..., 0] = np.arange(T, dtype=np.float32)[None] / 16.0
+    cb, rb_ = oracle.bf16_from_f32(c), oracle.bf16_from_f32(r)
+    pool.append(0, np.concatenate([cb[i, :ctx[i]] for i in range(B)]), np.concatenate([rb_[i, :ctx[i]] for i in range(B)]), B, n_new=ctx)
+    q = oracle.bf16_from_f32(0.3 * rng.standard_normal((B, S, H, DH)).astype(np.float32))
+    qr = 0.3 * rng.standard_normal((B, S, H, DHR)).astype(np.float32)
+    qr[..., 0] = rise * np.log(2.0) / (scale * 128 / 16.0) * rng.uniform(0.4, 1.0, (B, S, H))
+    qr = oracle.bf16_from_f32(qr)
+    wuk, wuv = (oracle.bf16_from_f32(rng.standard_normal((DC, H * DH)).astype(np.float32) * 0.02) for _ in range(2))
+    d_uk, d_uv = dev.upload(wuk), dev.upload(wuv)
+    out = np.full(q.shape, np.nan, np.float32)
+    pool.decode(0, B, q, out, H, DH, scale, q_rope=qr, w_uk=d_uk, w_uv=d_uv, q_tokens=S)
+    for i in range(B):
+        cb[i, ctx[i]:] = 0
+        rb_[i, ctx[i]:] = 0
+    with oracle.exact_exp():
+        ref = oracle.mla_attend(cb, rb_, ctx, oracle.f32_from_bf16(q), oracle.f32_from_bf16(qr), wuk, wuv, scale, causal=True,
+                                absorbed=False)
+    check_attention(out, ref, "rising scores, expanded", max_tol=EDGE_MAX, mean_tol=EDGE_MEAN)
+    assert pool.status() == 0
+    pool.destroy()
+    d_uk.free()
+    d_uv.free()
