@@ -350,6 +350,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     const int hf = L >> 6;            // token half of the tile (= which CTA's page)
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full), 0);
+    // The partial results (36 MB at 64 sequences) wait for the merge while cached rows stream through L2, and came back from HBM:
+    // stored to be evicted last, a step of 64 x 4096 takes 98.9 us instead of 101.1, 16 x <= 32k 97.7 instead of 99.9.  (Cached rows
+    // loaded to be evicted first were gone before their second load, as values: 114 -> 127 us.)
+    const uint64_t evict_last = make_evict_last_policy();
     StreamItem cur = load_item(prm.items + it0);
     int g = 0;
     for (int it = it0; it < it1; ++it) {
@@ -484,7 +488,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
           for (int k = 0; k < 8; k++) {
             const int seg = k * 16 + (L >> 3), r = seg >> 1, h2 = seg & 1, j = L & 7;
             const uint4 v = *reinterpret_cast<const uint4*>(stage + seg * 128 + ((j ^ (r & 7)) << 4));
-            if (r < heads_here) *reinterpret_cast<uint4*>(obase + (size_t)r * kDC + 256 * nb + 128 * h2 + c + 4 * j) = v;
+            if (r < heads_here) store_hint(obase + (size_t)r * kDC + 256 * nb + 128 * h2 + c + 4 * j, v, evict_last);
           }
           asm volatile("bar.sync 1, 128;" ::: "memory");
         }
@@ -493,7 +497,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     }
   }
   tc_fence_before();
-  cluster_sync();
+  cluster_sync_relaxed();   // nothing is handed over: the pair's barriers and tensor memory outlive what the other CTA does with them
   if (threadIdx.x == 0 && it0 < it1) stamp_end(prm.time);
   if (warp == 0) tmem_dealloc<2>(tmem, kTmemCols);
 }
