@@ -290,7 +290,7 @@ inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 //        - skinny_gemm_sm100_kernel, the weights: the first launch of a layer step or matmul is cast_bf16_kernel, the
 //          second GEMM of a layer follows it, a plain absorb launch, or a cast of its own;
 //        - mla_prep_kernel with weights_ready, W_UK: only behind the projections of the same call (do_mla_layer);
-//        - mla_merge_vup_mma_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.
+//        - mla_merge_vup_mma_kernel, mla_merge_vup_sm100_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.
 //      A new early read names its head here; a new launch in front of one of these keeps a head between.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(bool chained, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
