@@ -513,14 +513,27 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   // the lists live in the histogram block: words [0,512) values, [512,1024) indices of this CTA's
   float* l_val = reinterpret_cast<float*>(&sh.warp_hist[0][0]);
   int32_t* l_idx = reinterpret_cast<int32_t*>(&sh.warp_hist[0][0]) + kCandCap;
-  auto collect = [&](uint32_t key_lo) {
-    for_segment(c, row, [&](int i, float v) {
+  // Puts what reaches key_lo of the elements that the lanes in `lanes` read in for_segment() on the list.  A warp goes through one lane's
+  // elements together: a trip to L2 and a few instructions each, where the lane by itself, 64 elements unrolled, took 10 us, most of
+  // them its own instructions' way into the cache.
+  auto collect = [&](uint32_t key_lo, uint32_t lanes) {
+    auto put = [&](int i, float v) {
       const float x = d.scaled(v);
       if (bit_key(x) >= key_lo) {
         const uint32_t pos = atomicAdd(&sh.list_count, 1u);
         if (pos < (uint32_t)kCandCap) { l_val[pos] = x; l_idx[pos] = i; }
       }
-    });
+    };
+    const int width = c.vec ? 4 : 1;
+#pragma unroll 1
+    for (; lanes; lanes &= lanes - 1) {
+#pragma unroll 1
+      for (int i = c.wlo + (__ffs(lanes) - 1 + 32 * c.lane) * width; i < c.whi; i += 1024 * width) {
+        const float4 v = load4(c, row, i, c.whi);
+#pragma unroll 1
+        for (int e = 0; e < width; e++) put(i + e, e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w);
+      }
+    }
   };
   // The largest element per thread, as a key (the division by the temperature keeps the order, so it is made once, behind the
   // pass).  Of long slices, pairs of threads: half as many keys to rank.
@@ -555,7 +568,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   uint32_t bound = 0xffffffffu;
   for (int q = 0; q < c.csize; q++) bound = min(bound, *cl.map_shared_rank(&sh.list_bound, q));
   bound = with_both_zeros(bound);
-  if (key >= bound) collect(bound);
+  collect(bound, __ballot_sync(0xffffffffu, key >= bound));
   __syncthreads();
   cl.sync();
   uint32_t total = 0;
@@ -568,7 +581,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
     if (n_ge > (uint32_t)kCandCap) return false;     // more ties at the threshold than the list holds
     if (threadIdx.x == 0) sh.list_count = 0;
     __syncthreads();
-    collect(with_both_zeros(key_lo));
+    collect(with_both_zeros(key_lo), 0xffffffffu);
     __syncthreads();
     cl.sync();
   }
