@@ -513,10 +513,11 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   // the lists live in the histogram block: words [0,512) values, [512,1024) indices of this CTA's
   float* l_val = reinterpret_cast<float*>(&sh.warp_hist[0][0]);
   int32_t* l_idx = reinterpret_cast<int32_t*>(&sh.warp_hist[0][0]) + kCandCap;
-  // Puts what reaches key_lo of the elements that the lanes in `lanes` read in for_segment() on the list.  A warp goes through one lane's
-  // elements together: a trip to L2 and a few instructions each, where the lane by itself, 64 elements unrolled, took 10 us, most of
-  // them its own instructions' way into the cache.
-  auto collect = [&](uint32_t key_lo, uint32_t lanes) {
+  // Puts what reaches key_lo of the elements that the threads with `mine` read in for_segment() on the list.  Where a thread has read
+  // eight times or more, a warp goes through one such lane's elements together: a trip to L2 and a few instructions each, where the
+  // lane by itself, 64 elements unrolled, took 10 us, most of them its own instructions' way into the cache (131072 logits, 64
+  // sequences: 109 -> 103.5 us a call).  Fewer reads are one trip for all the lanes (32000 logits: 39.5 us so, 42.5 lane by lane).
+  auto collect = [&](uint32_t key_lo, bool mine) {
     auto put = [&](int i, float v) {
       const float x = d.scaled(v);
       if (bit_key(x) >= key_lo) {
@@ -525,8 +526,12 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
       }
     };
     const int width = c.vec ? 4 : 1;
+    if (c.whi - c.wlo < 8 * 32 * width) {
+      if (mine) for_segment(c, row, put);
+      return;
+    }
 #pragma unroll 1
-    for (; lanes; lanes &= lanes - 1) {
+    for (uint32_t lanes = __ballot_sync(0xffffffffu, mine); lanes; lanes &= lanes - 1) {
 #pragma unroll 1
       for (int i = c.wlo + (__ffs(lanes) - 1 + 32 * c.lane) * width; i < c.whi; i += 1024 * width) {
         const float4 v = load4(c, row, i, c.whi);
@@ -568,7 +573,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   uint32_t bound = 0xffffffffu;
   for (int q = 0; q < c.csize; q++) bound = min(bound, *cl.map_shared_rank(&sh.list_bound, q));
   bound = with_both_zeros(bound);
-  collect(bound, __ballot_sync(0xffffffffu, key >= bound));
+  collect(bound, key >= bound);
   __syncthreads();
   cl.sync();
   uint32_t total = 0;
@@ -581,7 +586,7 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
     if (n_ge > (uint32_t)kCandCap) return false;     // more ties at the threshold than the list holds
     if (threadIdx.x == 0) sh.list_count = 0;
     __syncthreads();
-    collect(with_both_zeros(key_lo), 0xffffffffu);
+    collect(with_both_zeros(key_lo), true);
     __syncthreads();
     cl.sync();
   }
@@ -674,9 +679,12 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
       if (threadIdx.x == 0) {
         float cum = 0.0f;
         int cut = n_k;
-        for (int j = 0; j < n_k; j++) {
-          cum = __fadd_rn(cum, ranked[j]);
-          if (cum >= topP) { cut = j + 1; break; }
+        for (int j = 0; j < n_k; j += 4) {   // four sums a load: what lies past the end follows the last sum that counts
+          const float4 q = *reinterpret_cast<const float4*>(ranked + j);
+          const float c0 = __fadd_rn(cum, q.x), c1 = __fadd_rn(c0, q.y), c2 = __fadd_rn(c1, q.z);
+          cum = __fadd_rn(c2, q.w);
+          const int at = c0 >= topP ? j : c1 >= topP ? j + 1 : c2 >= topP ? j + 2 : cum >= topP ? j + 3 : n_k;
+          if (at < n_k) { cut = at + 1; break; }
         }
         s_cut = cut < n_k && ranked[cut] == ranked[cut - 1] ? -1 : cut;
       }
@@ -749,10 +757,12 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
     if (threadIdx.x == 0) {
       float cum = 0.0f;
       int tok = V - 1;
-#pragma unroll 4
-      for (int j = 0; j < n_k; j++) {
-        cum = __fadd_rn(cum, k_p[j]);
-        if (r < cum) { tok = k_idx[j]; break; }
+      for (int j = 0; j < n_k; j += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(k_p + j);
+        const float c0 = __fadd_rn(cum, q.x), c1 = __fadd_rn(c0, q.y), c2 = __fadd_rn(c1, q.z);
+        cum = __fadd_rn(c2, q.w);
+        const int at = r < c0 ? j : r < c1 ? j + 1 : r < c2 ? j + 2 : r < cum ? j + 3 : n_k;
+        if (at < n_k) { tok = k_idx[at]; break; }
       }
       *out = tok;
     }
