@@ -514,6 +514,7 @@ class KVCache:
         self.pool = Pool(dev, L.POOL_GQA, num_layers, pages, page_tokens, 1, pages, num_kv_heads=num_kv_heads, head_dim=head_dim,
                          reference_compat=reference_compat)
         self.seq = self.pool.seq_alloc(max_len)
+        self._ids, self._one_row = np.array([self.seq], np.int32), np.array([1], np.int32)   # as the calls take them
         self.num_layers, self.max_len, self.num_kv_heads, self.head_dim = num_layers, max_len, num_kv_heads, head_dim
 
     def DType(self):
@@ -533,7 +534,8 @@ class KVCache:
             raise ValueError("KVCache.Append: K rank=%d, want >= 3 [batch, heads, seq, headDim]" % new_k.ndim)
         n_new = new_k.shape[-2]
         try:
-            self.pool.append(layer, new_k, new_v, 1, seq_ids=[self.seq], n_new=[n_new], layout=L.LAYOUT_HEAD_MAJOR)
+            self.pool.append(layer, new_k, new_v, 1, seq_ids=self._ids, n_new=self._one_row if n_new == 1 else [n_new],
+                             layout=L.LAYOUT_HEAD_MAJOR)
         except L.ReluxCudaError as e:
             if e.code == L.ERR_OVERFLOW:
                 raise OverflowError(str(e))
@@ -559,7 +561,7 @@ class KVCache:
         _, H, S, D = q.shape
         out = np.empty_like(q)
         self.pool.decode(layer, 1, q, out, H, D, scale, q_tokens=S, extra_tokens=extra_tokens, causal=causal, mode=mode,
-                         seq_ids=[self.seq], q_layout=L.LAYOUT_HEAD_MAJOR, out_layout=L.LAYOUT_HEAD_MAJOR)
+                         seq_ids=self._ids, q_layout=L.LAYOUT_HEAD_MAJOR, out_layout=L.LAYOUT_HEAD_MAJOR)
         return out
 
     def close(self):

@@ -289,6 +289,33 @@ static int32_t check_layer(Pool* p, int layer) {
   return RELUX_OK;
 }
 
+// A pointer that a caller gave as host memory but the host cannot read or write: the runtime's copies find out by themselves, memcpy not.
+static bool is_device_memory(const void* ptr) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice;
+}
+
+// A small input that arrives in host memory, for kernels that read it once, by ordinary loads, on the device's stream: *dptr is a copy
+// in page-locked memory.  False: it is not small, or not the host's.
+static bool stage_small(Pool* p, const void* src, size_t bytes, int mem, const void** dptr) {
+  Device* dev = p->dev;
+  if (mem != RELUX_MEM_HOST || bytes > Device::kHostInMax || !dev->host_in || is_device_memory(src)) return false;
+  const size_t need = (bytes + 255) & ~(size_t)255;
+  if (dev->host_in_used + need > Device::kHostInBytes) {
+    if (cudaStreamSynchronize(dev->stream) != cudaSuccess) return false;
+    dev->host_in_used = 0;
+  }
+  char* at = dev->host_in + dev->host_in_used;
+  memcpy(at, src, bytes);
+  dev->host_in_used += need;
+  *dptr = at;
+  return true;
+}
+
 // Moves an activation that arrives in host memory to the device staging block.
 int32_t stage_in(Pool* p, GrowBuf& buf, const void* src, size_t bytes, int mem, const void** dptr) {
   if (mem == RELUX_MEM_DEVICE) {
@@ -414,8 +441,8 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
     if ((rc = pipe_stage_in(p, p->pipe_app_a, a->a, bytes_a, &da, &slot_a))) return rc;
     if ((rc = pipe_stage_in(p, p->pipe_app_b, a->b, bytes_b, &db, &slot_b))) return rc;
   } else {
-    if ((rc = stage_in(p, p->in_a, a->a, bytes_a, a->mem, &da))) return rc;
-    if ((rc = stage_in(p, p->in_b, a->b, bytes_b, a->mem, &db))) return rc;
+    if (!stage_small(p, a->a, bytes_a, a->mem, &da) && (rc = stage_in(p, p->in_a, a->a, bytes_a, a->mem, &da))) return rc;
+    if (!stage_small(p, a->b, bytes_b, a->mem, &db) && (rc = stage_in(p, p->in_b, a->b, bytes_b, a->mem, &db))) return rc;
   }
   if (kind == RELUX_POOL_MLA) rc = launch_mla_append(p, sb, a->layer, da, db, a->dtype, a->advance);
   else rc = launch_gqa_append(p, sb, a->layer, da, db, a->dtype, a->layout, a->advance);
@@ -434,16 +461,6 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
 // Converts q to the kernels' canonical device form and runs the attention, then delivers `out`.
 int32_t convert_layout(Device* dev, const void* src, void* dst, int n, int S, int H, int D, int src_dtype, int dst_dtype,
                        int src_layout, int dst_layout);
-
-// A pointer that a caller gave as host memory but the host cannot write: the runtime's copies find out by themselves, memcpy not.
-static bool is_device_memory(const void* ptr) {
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  return at.type == cudaMemoryTypeDevice;
-}
 
 static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const StepAppend* step = nullptr, const GqaAppend* gstep = nullptr) {
   if (!a) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
@@ -601,6 +618,7 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
       const bool dev_mem = is_device_memory(a->out);   // asked while the kernels run: 0.7 us of host time before them
       if (dev_mem) RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, p->dev->host_out, out_bytes, cudaMemcpyDefault, p->dev->stream));
       RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
+      p->dev->host_in_used = 0;
       if (!dev_mem) memcpy(a->out, p->dev->host_out, out_bytes);
     } else if (a->out_mem == RELUX_MEM_HOST) {
       RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_bytes, cudaMemcpyDeviceToHost, p->dev->stream));
@@ -700,6 +718,10 @@ API int32_t relux_cuda_device_open(int32_t device_index, relux_device_t* out) {
     (void)cudaGetLastError();   // without it results are copied
     d->host_out = nullptr;
   }
+  if (cudaMallocHost((void**)&d->host_in, Device::kHostInBytes) != cudaSuccess) {
+    (void)cudaGetLastError();   // without it inputs are copied
+    d->host_in = nullptr;
+  }
   *out = d;
   return RELUX_OK;
 }
@@ -713,6 +735,7 @@ API int32_t relux_cuda_device_close(relux_device_t h) {
     cudaStreamSynchronize(dev->stream);
     if (dev->flush_buf) cudaFree(dev->flush_buf);
     if (dev->host_out) cudaFreeHost(dev->host_out);
+    if (dev->host_in) cudaFreeHost(dev->host_in);
     if (dev->side_stream) { cudaStreamSynchronize(dev->side_stream); cudaStreamDestroy(dev->side_stream); }
     if (dev->ev_fork) cudaEventDestroy(dev->ev_fork);
     if (dev->ev_join) cudaEventDestroy(dev->ev_join);
@@ -1251,11 +1274,16 @@ static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_at
   } else if (kv->mem == RELUX_MEM_HOST) {
     // the attention call stages q in in_a: the step's rows get a block of their own
     const size_t off_b = (bytes + 255) & ~(size_t)255;
-    if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
-    da = p->step_rows.p;
-    db = (char*)p->step_rows.p + off_b;
-    RELUX_CUDA_TRY(cudaMemcpyAsync((void*)da, kv->a, bytes, cudaMemcpyHostToDevice, p->dev->stream));
-    RELUX_CUDA_TRY(cudaMemcpyAsync((void*)db, kv->b, bytes, cudaMemcpyHostToDevice, p->dev->stream));
+    if (!stage_small(p, kv->a, bytes, kv->mem, &da)) {
+      if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
+      da = p->step_rows.p;
+      RELUX_CUDA_TRY(cudaMemcpyAsync((void*)da, kv->a, bytes, cudaMemcpyHostToDevice, p->dev->stream));
+    }
+    if (!stage_small(p, kv->b, bytes, kv->mem, &db)) {
+      if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
+      db = (char*)p->step_rows.p + off_b;
+      RELUX_CUDA_TRY(cudaMemcpyAsync((void*)db, kv->b, bytes, cudaMemcpyHostToDevice, p->dev->stream));
+    }
   }
   const GqaAppend app{da, db, kv->dtype, kv->layout, adv, sb.rows.data()};
   if (adv)   // the host lengths count the new rows from here on
