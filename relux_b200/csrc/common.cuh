@@ -223,6 +223,9 @@ __device__ __forceinline__ void store_hint(void* p, const uint4& v, uint64_t pol
                "l"(policy)
                : "memory");
 }
+__device__ __forceinline__ void store_hint(float* p, float v, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(__cvta_generic_to_global(p)), "f"(v), "l"(policy) : "memory");
+}
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -260,7 +260,11 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
       __syncwarp();
     }
   } else {
-    // epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once
+    // Epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once.  The result of
+    // more than 32 rows, some MB that the next launch sums and the next GEMM overwrites, is stored to stay in L2 meanwhile (layer
+    // steps: 100 x 1000 of d_model 4096 113 -> 107.6 us, 60 x 1000 of 16384 281 -> 278; up to 32 rows 1 % slower so).
+    constexpr bool kKeep = NT >= 64;
+    const uint64_t evict_last = kKeep ? make_evict_last_policy() : 0;
     chain_wait();
     for (int piece = 0; walk.next(); piece++) {
       const int j = weight_of(walk.col), m0 = kBlocks ? walk.block * NT : 0;
@@ -277,7 +281,12 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
         tmem_ld_wait();
 #pragma unroll
         for (int q = 0; q < 32; q++)
-          if (mine && c + q < m_end) dst[(size_t)(c + q) * prm.n_total] = ok ? __uint_as_float(v[q]) : 0.f;
+          if (mine && c + q < m_end) {
+            float* to = dst + (size_t)(c + q) * prm.n_total;
+            const float x = ok ? __uint_as_float(v[q]) : 0.f;
+            if constexpr (kKeep) store_hint(to, x, evict_last);
+            else *to = x;
+          }
       }
       tc_fence_before();
       __syncwarp();
