@@ -308,6 +308,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     PrepPlan pl;
     pl.extra = a.extra_tokens;
     pl.G = plan.chunk_pages;
+    pl.by_item = plan.by_item ? 1 : 0;
     pl.workers = plan.num_workers;
     pl.items = plan.stream_items;
     pl.chunk_off = plan.chunk_off;

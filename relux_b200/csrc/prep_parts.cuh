@@ -25,7 +25,7 @@ struct PrepAppend {
 };
 
 struct PrepPlan {
-  int32_t extra, G, workers;
+  int32_t extra, G, workers, by_item;
   StreamItem* items;
   int32_t* chunk_off;
   int32_t* worker_first;
@@ -120,13 +120,14 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
     }
     int tot_pages, tot_items;
     const int start = page_base + prep_block_excl_scan(pages, s_warp, &tot_pages);
-    const int w0 = start / pl.G;
-    const int nc = pages > 0 ? (start + pages - 1) / pl.G - w0 + 1 : 0;
+    const int w0 = pl.by_item ? 0 : start / pl.G;
+    const int nc = pages > 0 ? (pl.by_item ? (pages + pl.G - 1) / pl.G : (start + pages - 1) / pl.G - w0 + 1) : 0;
     const int c0 = item_base + prep_block_excl_scan(nc, s_warp, &tot_items);
     if (i < g.n_seqs) {
       pl.chunk_off[i] = c0;
       for (int c = 0; c < nc; c++) {
-        const int lo = max(start, (w0 + c) * pl.G), hi = min(start + pages, (w0 + c + 1) * pl.G);
+        const int from = pl.by_item ? start + c * pl.G : (w0 + c) * pl.G;
+        const int lo = max(start, from), hi = min(start + pages, from + pl.G);
         StreamItem w;
         w.seq_index = i;
         w.seq = seq;
@@ -135,7 +136,8 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
         w.tokens = tokens;
         w.pad[0] = w.pad[1] = w.pad[2] = 0;
         pl.items[c0 + c] = w;
-        if (lo == (w0 + c) * pl.G) pl.worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
+        if (pl.by_item) pl.worker_first[c0 + c] = c0 + c;
+        else if (lo == from) pl.worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
       }
     }
     page_base += tot_pages;
@@ -143,7 +145,7 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
   }
   if (threadIdx.x == 0) pl.chunk_off[g.n_seqs] = item_base;
   // ranges past the end of the stream are empty
-  for (int w = (page_base + pl.G - 1) / pl.G + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;
+  for (int w = (pl.by_item ? item_base : (page_base + pl.G - 1) / pl.G) + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;
 }
 
 }  // namespace relux

@@ -143,8 +143,8 @@ __device__ __forceinline__ int block_excl_scan(int v, int32_t* s_warp, int* tota
 // is cut at every multiple of G; items are numbered in stream order, so the items of a sequence and the items of
 // a worker are both contiguous.
 __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
-                                    int page_tokens, int G, int workers, StreamItem* __restrict__ items, int32_t* __restrict__ chunk_off,
-                                    int32_t* __restrict__ worker_first) {
+                                    int page_tokens, int G, int workers, int by_item, StreamItem* __restrict__ items,
+                                    int32_t* __restrict__ chunk_off, int32_t* __restrict__ worker_first) {
   __shared__ int32_t s_warp[8];
   int page_base = 0, item_base = 0;
   for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
@@ -157,13 +157,14 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
     }
     int tot_pages, tot_items;
     const int start = page_base + block_excl_scan(pages, s_warp, &tot_pages);
-    const int w0 = start / G;
-    const int nc = pages > 0 ? (start + pages - 1) / G - w0 + 1 : 0;
+    const int w0 = by_item ? 0 : start / G;
+    const int nc = pages > 0 ? (by_item ? (pages + G - 1) / G : (start + pages - 1) / G - w0 + 1) : 0;
     const int c0 = item_base + block_excl_scan(nc, s_warp, &tot_items);
     if (i < n_seqs) {
       chunk_off[i] = c0;
       for (int c = 0; c < nc; c++) {
-        const int lo = max(start, (w0 + c) * G), hi = min(start + pages, (w0 + c + 1) * G);
+        const int from = by_item ? start + c * G : (w0 + c) * G;
+        const int lo = max(start, from), hi = min(start + pages, from + G);
         StreamItem w;
         w.seq_index = i;
         w.seq = seq;
@@ -172,7 +173,8 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
         w.tokens = tokens;
         w.pad[0] = w.pad[1] = w.pad[2] = 0;
         items[c0 + c] = w;
-        if (lo == (w0 + c) * G) worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
+        if (by_item) worker_first[c0 + c] = c0 + c;
+        else if (lo == from) worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
       }
     }
     page_base += tot_pages;
@@ -180,7 +182,7 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
   }
   if (threadIdx.x == 0) chunk_off[n_seqs] = item_base;
   // ranges past the end of the stream are empty
-  for (int w = (page_base + G - 1) / G + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
+  for (int w = (by_item ? item_base : (page_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
 }
 
 // Host statement of the stream partition: range length G and the counts that follow from it.  The device builder
@@ -205,6 +207,63 @@ void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_
   *items_out = items;
 }
 
+// What a plan costs, in tiles of two pages (about 2 us): its slowest worker's tiles and two for every item (start and write-out), 0.08 for
+// every partial that a row of the merge adds up, and 0.035 for every partial of the call.  From steps of 1 to 30 short sequences with
+// ranges of one and of two tiles (1 x 1300 tokens 19.9 against 21.5 us, 1 x 2600 21.5 and 21.4, 1 x 6000 26.8 and 24.0, 4 x 1200 24.0 and
+// 23.3, 25 x 200 27.4 and 28.3).
+static double plan_cost(double worst, int most_items, int items) { return worst + 0.08 * most_items + 0.035 * items; }
+
+// Cuts every sequence into pieces of 2 t pages, a worker each, so that no worker has a second item to start and write out, where that
+// costs less than ranges of G pages.  Returns the pages of a piece, 0: ranges.  Measured, ranges -> pieces: 3 x <= 1500 tokens 26.4 ->
+// 21.9 us, 16 x 300 28.0 -> 24.4, 64 x 300 48.7 -> 38.4, 40 x <= 2500 51.4 -> 45.3, 64 x 4096 95.5 -> 91.3, 8 x 20000 74.9 -> 61.0;
+// 64 x 32768 has 222 tiles a worker in ranges and 257 in pieces and keeps the ranges.
+static int plan_by_item(const std::vector<int>& pages, int workers, long G, int* items_out) {
+  int longest = 0, n_items = 0, most = 0, live = 0;
+  for (int n : pages) {
+    longest = std::max(longest, n);
+    live += n > 0;
+  }
+  if (live == 0 || live > workers) return 0;
+  auto items_of = [&](int t) {
+    int items = 0;
+    for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
+    return items;
+  };
+  long start = 0;
+  double worst = 0, here = 0;   // of the ranges: walked as the workers walk them
+  for (int n : pages) {
+    int of_seq = 0;
+    for (long at = start; at < start + n; of_seq++) {
+      const long end = std::min(start + n, (at / G + 1) * G);
+      if (at % G == 0) here = 0;
+      here += (end - at + 1) / 2 + 2;
+      worst = std::max(worst, here);
+      at = end;
+    }
+    most = std::max(most, of_seq);
+    n_items += of_seq;
+    start += n;
+  }
+  double best = plan_cost(worst, most, n_items);
+  int lo = 1, hi = (longest + 1) / 2;   // the smallest t whose pieces find a worker each: one piece a sequence does
+  while (lo < hi) {
+    const int t = (lo + hi) / 2;
+    if (items_of(t) <= workers) hi = t;
+    else lo = t + 1;
+  }
+  int piece = 0;
+  for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
+    const int items = items_of(t);
+    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
+    if (cost < best) {
+      best = cost;
+      piece = 2 * t;
+      *items_out = items;
+    }
+  }
+  return piece;
+}
+
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
                     bool launch_builder) {
   const relux_pool_params& prm = p->prm;
@@ -215,7 +274,16 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   }
   long G = 0;
   int items = 0;
+  const int resident = workers;
   stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, (long)p->tune.get(RELUX_TUNE_CHUNK_PAGES), &G, &workers, &items);
+  plan->by_item = false;
+  if (!p->tune.get(RELUX_TUNE_CHUNK_PAGES) && page_multiple == 2) {
+    if (const int piece = plan_by_item(pages, resident, G, &items)) {
+      plan->by_item = true;
+      G = piece;
+      workers = items;
+    }
+  }
   plan->chunk_pages = (int)G;
   plan->num_items = items;
   plan->num_workers = workers;
@@ -230,7 +298,7 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   if (!launch_builder) return RELUX_OK;
   const int32_t* len = p->d_len + (size_t)layer * prm.max_seqs;
   build_stream_kernel<<<1, 256, 0, st>>>(len, sb.d_seq_ids, sb.n_seqs, extra, prm.page_tokens, (int)G, workers,
-                                                     plan->stream_items, plan->chunk_off, plan->worker_first);
+                                                     plan->by_item ? 1 : 0, plan->stream_items, plan->chunk_off, plan->worker_first);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(p->dev);
   return RELUX_OK;

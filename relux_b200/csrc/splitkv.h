@@ -30,6 +30,7 @@ struct SplitPlan {
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]
   // stream plans only (plan_stream): worker w owns items [worker_first[w], worker_first[w + 1])
   int num_workers = 0;
+  bool by_item = false;                // every worker has one item: chunk_pages pages of a sequence (plan_stream)
   StreamItem* stream_items = nullptr;  // device [num_items]
   int32_t* worker_first = nullptr;     // device [num_workers + 1]
 };
@@ -40,7 +41,8 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
                      int max_chunk_pages, SplitPlan* plan);
 // Stream partition for persistent kernels: the pages of all sequences of the call, laid end to end, are cut into
 // `workers` equal ranges of `chunk_pages` pages (a multiple of `page_multiple`); one item = the part of one sequence
-// inside one range, so a worker meets an item boundary only where a sequence ends inside its range.
+// inside one range, so a worker meets an item boundary only where a sequence ends inside its range.  Short calls are cut sequence by
+// sequence instead, one item of chunk_pages pages a worker (by_item).
 // `st`: the stream the builder kernel is launched on (the pool's main stream, or the device's side stream).
 // launch_builder = false: only the host half (counts, buffers); the caller builds the lists itself (the fused decode-step
 // preparation of mla_proj.cu does it inside its own launch).
