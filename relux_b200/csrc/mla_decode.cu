@@ -309,6 +309,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     pl.extra = a.extra_tokens;
     pl.G = plan.chunk_pages;
     pl.by_item = plan.by_item ? 1 : 0;
+    pl.start_units = plan.start_units;
     pl.workers = plan.num_workers;
     pl.items = plan.stream_items;
     pl.chunk_off = plan.chunk_off;

@@ -25,7 +25,7 @@ struct PrepAppend {
 };
 
 struct PrepPlan {
-  int32_t extra, G, workers, by_item;
+  int32_t extra, G, workers, by_item, start_units;
   StreamItem* items;
   int32_t* chunk_off;
   int32_t* worker_first;
@@ -109,7 +109,7 @@ __device__ __forceinline__ int prep_block_excl_scan(int v, int32_t* s_warp, int*
 // yet: every sequence counts its cached rows + its new rows + extra).  Same arithmetic as build_stream_kernel.
 __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const PrepPlan& pl) {
   __shared__ int32_t s_warp[32];
-  int page_base = 0, item_base = 0;
+  int unit_base = 0, item_base = 0;
   for (int i0 = 0; i0 < g.n_seqs; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     int seq = 0, pages = 0, tokens = 0;
@@ -118,34 +118,31 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
       tokens = load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
       pages = (tokens + g.page_tokens - 1) / g.page_tokens;
     }
-    int tot_pages, tot_items;
-    const int start = page_base + prep_block_excl_scan(pages, s_warp, &tot_pages);
-    const int w0 = pl.by_item ? 0 : start / pl.G;
-    const int nc = pages > 0 ? (pl.by_item ? (pages + pl.G - 1) / pl.G : (start + pages - 1) / pl.G - w0 + 1) : 0;
-    const int c0 = item_base + prep_block_excl_scan(nc, s_warp, &tot_items);
+    int tot_units, tot_items;
+    const int at = unit_base + prep_block_excl_scan(SeqCut(pl.by_item, pl.G, pl.start_units, 0, pages).units, s_warp, &tot_units);
+    const SeqCut cut(pl.by_item, pl.G, pl.start_units, at, pages);
+    const int c0 = item_base + prep_block_excl_scan(cut.n, s_warp, &tot_items);
     if (i < g.n_seqs) {
       pl.chunk_off[i] = c0;
-      for (int c = 0; c < nc; c++) {
-        const int from = pl.by_item ? start + c * pl.G : (w0 + c) * pl.G;
-        const int lo = max(start, from), hi = min(start + pages, from + pl.G);
+      for (int c = 0; c < cut.n; c++) {
         StreamItem w;
         w.seq_index = i;
         w.seq = seq;
-        w.page_begin = lo - start;
-        w.page_end = hi - start;
+        w.page_begin = cut.begin(c);
+        w.page_end = cut.end(c);
         w.tokens = tokens;
         w.pad[0] = w.pad[1] = w.pad[2] = 0;
         pl.items[c0 + c] = w;
         if (pl.by_item) pl.worker_first[c0 + c] = c0 + c;
-        else if (lo == from) pl.worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
+        else if (cut.leads(c, at)) pl.worker_first[cut.first + c] = c0 + c;
       }
     }
-    page_base += tot_pages;
+    unit_base += tot_units;
     item_base += tot_items;
   }
   if (threadIdx.x == 0) pl.chunk_off[g.n_seqs] = item_base;
   // ranges past the end of the stream are empty
-  for (int w = (pl.by_item ? item_base : (page_base + pl.G - 1) / pl.G) + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;
+  for (int w = (pl.by_item ? item_base : (unit_base + pl.G - 1) / pl.G) + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;
 }
 
 }  // namespace relux

@@ -143,10 +143,10 @@ __device__ __forceinline__ int block_excl_scan(int v, int32_t* s_warp, int* tota
 // is cut at every multiple of G; items are numbered in stream order, so the items of a sequence and the items of
 // a worker are both contiguous.
 __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
-                                    int page_tokens, int G, int workers, int by_item, StreamItem* __restrict__ items,
-                                    int32_t* __restrict__ chunk_off, int32_t* __restrict__ worker_first) {
+                                    int page_tokens, int G, int workers, int by_item, int start_units,
+                                    StreamItem* __restrict__ items, int32_t* __restrict__ chunk_off, int32_t* __restrict__ worker_first) {
   __shared__ int32_t s_warp[8];
-  int page_base = 0, item_base = 0;
+  int unit_base = 0, item_base = 0;
   for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     int seq = 0, pages = 0, tokens = 0;
@@ -155,34 +155,31 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
       tokens = len[seq] + extra;
       pages = (tokens + page_tokens - 1) / page_tokens;
     }
-    int tot_pages, tot_items;
-    const int start = page_base + block_excl_scan(pages, s_warp, &tot_pages);
-    const int w0 = by_item ? 0 : start / G;
-    const int nc = pages > 0 ? (by_item ? (pages + G - 1) / G : (start + pages - 1) / G - w0 + 1) : 0;
-    const int c0 = item_base + block_excl_scan(nc, s_warp, &tot_items);
+    int tot_units, tot_items;
+    const int at = unit_base + block_excl_scan(SeqCut(by_item, G, start_units, 0, pages).units, s_warp, &tot_units);
+    const SeqCut cut(by_item, G, start_units, at, pages);
+    const int c0 = item_base + block_excl_scan(cut.n, s_warp, &tot_items);
     if (i < n_seqs) {
       chunk_off[i] = c0;
-      for (int c = 0; c < nc; c++) {
-        const int from = by_item ? start + c * G : (w0 + c) * G;
-        const int lo = max(start, from), hi = min(start + pages, from + G);
+      for (int c = 0; c < cut.n; c++) {
         StreamItem w;
         w.seq_index = i;
         w.seq = seq;
-        w.page_begin = lo - start;
-        w.page_end = hi - start;
+        w.page_begin = cut.begin(c);
+        w.page_end = cut.end(c);
         w.tokens = tokens;
         w.pad[0] = w.pad[1] = w.pad[2] = 0;
         items[c0 + c] = w;
         if (by_item) worker_first[c0 + c] = c0 + c;
-        else if (lo == from) worker_first[w0 + c] = c0 + c;   // the item that holds the first page of a range
+        else if (cut.leads(c, at)) worker_first[cut.first + c] = c0 + c;
       }
     }
-    page_base += tot_pages;
+    unit_base += tot_units;
     item_base += tot_items;
   }
   if (threadIdx.x == 0) chunk_off[n_seqs] = item_base;
   // ranges past the end of the stream are empty
-  for (int w = (by_item ? item_base : (page_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
+  for (int w = (by_item ? item_base : (unit_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
 }
 
 // Host statement of the stream partition: range length G and the counts that follow from it.  The device builder
@@ -213,55 +210,63 @@ void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_
 // 23.3, 25 x 200 27.4 and 28.3).
 static double plan_cost(double worst, int most_items, int items) { return worst + 0.08 * most_items + 0.035 * items; }
 
-// Cuts every sequence into pieces of 2 t pages, a worker each, so that no worker has a second item to start and write out, where that
-// costs less than ranges of G pages.  Returns the pages of a piece, 0: ranges.  Measured, ranges -> pieces: 3 x <= 1500 tokens 26.4 ->
-// 21.9 us, 16 x 300 28.0 -> 24.4, 64 x 300 48.7 -> 38.4, 40 x <= 2500 51.4 -> 45.3, 64 x 4096 95.5 -> 91.3, 8 x 20000 74.9 -> 61.0;
-// 64 x 32768 has 222 tiles a worker in ranges and 257 in pieces and keeps the ranges.
-static int plan_by_item(const std::vector<int>& pages, int workers, long G, int* items_out) {
-  int longest = 0, n_items = 0, most = 0, live = 0;
+// The cheapest plan of a call: equal ranges of the sequences laid end to end, each counted as its pages and kStartUnits, for a worker
+// that starts it has a second item to start and to write out; or every sequence cut by itself into pieces of 2 t pages, a worker each.
+// Measured, ranges of pages alone -> this: in ranges, 16 x <= 32768 tokens 99.3 -> 97.3 us, 64 x 32768 611 -> 591, 20 x 16000 80.5 -> 72.3;
+// in pieces, 3 x <= 1500 26.4 -> 21.9, 16 x 300 28.0 -> 24.4, 64 x 300 48.7 -> 38.4, 40 x <= 2500 51.4 -> 45.3, 64 x 4096 95.5 -> 91.3.
+constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for an item
+struct StreamShape {
+  int G, workers, items, start_units;
+  bool by_item;
+};
+static StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
+  int longest = 0, live = 0;
+  int64_t units = 0;
   for (int n : pages) {
     longest = std::max(longest, n);
     live += n > 0;
+    units += SeqCut(0, 1, kStartUnits, 0, n).units;
   }
-  if (live == 0 || live > workers) return 0;
+  StreamShape r{};
+  r.start_units = kStartUnits;
+  r.G = std::max((int)((units + workers - 1) / workers + 1) / 2 * 2, 2 * kStartUnits);
+  r.workers = std::max(1, (int)((units + r.G - 1) / r.G));
+  int at = 0, most = 0, of_worker = -1;
+  double worst = 0, here = 0;   // of the ranges, walked as the workers walk them
+  for (int n : pages) {
+    const SeqCut cut(0, r.G, kStartUnits, at, n);
+    for (int c = 0; c < cut.n; c++) {
+      if (cut.first + c != of_worker) here = 0;
+      of_worker = cut.first + c;
+      here += (cut.end(c) - cut.begin(c) + 1) / 2 + 2;
+      worst = std::max(worst, here);
+    }
+    most = std::max(most, cut.n);
+    r.items += cut.n;
+    at += cut.units;
+  }
+  if (live == 0 || live > workers) return r;
+  double best = plan_cost(worst, most, r.items);
   auto items_of = [&](int t) {
     int items = 0;
     for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
     return items;
   };
-  long start = 0;
-  double worst = 0, here = 0;   // of the ranges: walked as the workers walk them
-  for (int n : pages) {
-    int of_seq = 0;
-    for (long at = start; at < start + n; of_seq++) {
-      const long end = std::min(start + n, (at / G + 1) * G);
-      if (at % G == 0) here = 0;
-      here += (end - at + 1) / 2 + 2;
-      worst = std::max(worst, here);
-      at = end;
-    }
-    most = std::max(most, of_seq);
-    n_items += of_seq;
-    start += n;
-  }
-  double best = plan_cost(worst, most, n_items);
   int lo = 1, hi = (longest + 1) / 2;   // the smallest t whose pieces find a worker each: one piece a sequence does
   while (lo < hi) {
     const int t = (lo + hi) / 2;
     if (items_of(t) <= workers) hi = t;
     else lo = t + 1;
   }
-  int piece = 0;
   for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
     const int items = items_of(t);
     const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
     if (cost < best) {
       best = cost;
-      piece = 2 * t;
-      *items_out = items;
+      r = StreamShape{2 * t, items, items, 0, true};
     }
   }
-  return piece;
+  return r;
 }
 
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
@@ -272,19 +277,19 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
     const int T = p->h_len[(size_t)layer * prm.max_seqs + sb.seq[i]] + extra;
     pages[i] = (T + prm.page_tokens - 1) / prm.page_tokens;
   }
-  long G = 0;
-  int items = 0;
-  const int resident = workers;
-  stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, (long)p->tune.get(RELUX_TUNE_CHUNK_PAGES), &G, &workers, &items);
-  plan->by_item = false;
-  if (!p->tune.get(RELUX_TUNE_CHUNK_PAGES) && page_multiple == 2) {
-    if (const int piece = plan_by_item(pages, resident, G, &items)) {
-      plan->by_item = true;
-      G = piece;
-      workers = items;
-    }
+  StreamShape shape{};
+  if (const int chunk = p->tune.get(RELUX_TUNE_CHUNK_PAGES)) {   // tuning knob: ranges of that many pages
+    long G = 0;
+    stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, chunk, &G, &shape.workers, &shape.items);
+    shape.G = (int)G;
+  } else {
+    shape = cheapest_plan(pages, workers);
   }
-  plan->chunk_pages = (int)G;
+  const int G = shape.G, items = shape.items;
+  workers = shape.workers;
+  plan->by_item = shape.by_item;
+  plan->start_units = shape.start_units;
+  plan->chunk_pages = G;
   plan->num_items = items;
   plan->num_workers = workers;
   const size_t off_chunk = sizeof(StreamItem) * (size_t)items;
@@ -297,8 +302,8 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   plan->worker_first = (int32_t*)((char*)p->work.p + off_worker);
   if (!launch_builder) return RELUX_OK;
   const int32_t* len = p->d_len + (size_t)layer * prm.max_seqs;
-  build_stream_kernel<<<1, 256, 0, st>>>(len, sb.d_seq_ids, sb.n_seqs, extra, prm.page_tokens, (int)G, workers,
-                                                     plan->by_item ? 1 : 0, plan->stream_items, plan->chunk_off, plan->worker_first);
+  build_stream_kernel<<<1, 256, 0, st>>>(len, sb.d_seq_ids, sb.n_seqs, extra, prm.page_tokens, G, workers,
+                                                     plan->by_item ? 1 : 0, plan->start_units, plan->stream_items, plan->chunk_off, plan->worker_first);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(p->dev);
   return RELUX_OK;
@@ -306,8 +311,9 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
 
 }  // namespace relux
 
-// The stream partition computed on the host from page counts (no device involved): what the persistent MLA decode
-// kernel's planner produces for sequences of pages[i] pages.  items_out receives n_items x {seq_index, page_begin,
+// The stream partition computed on the host from page counts (no device involved): equal ranges of whole tiles over the
+// sequences laid end to end, as the persistent MLA decode kernel walks them (its own planner also counts what the start
+// of a sequence costs, see cheapest_plan).  items_out receives n_items x {seq_index, page_begin,
 // page_end, worker}; worker_first [workers_out + 1]; chunk_off [n_seqs + 1].  Returns the number of items, or -1 when
 // `cap` items are not enough.  Scheduling aid for callers and tests; no counterpart in the reference.
 extern "C" __attribute__((visibility("default"))) int32_t relux_stream_partition(const relux_stream_partition_args* args) {

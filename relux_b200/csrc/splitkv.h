@@ -23,14 +23,41 @@ struct __align__(16) StreamItem {
   int32_t pad[3];
 };
 
+// The items of a sequence of `pages` pages that begins at unit `at` of the stream: item c is its pages [begin(c), end(c)), and belongs to
+// worker first + c, or (by_item) to a worker of its own.  What the host counts and the device builds from.
+struct SeqCut {
+  int by_item, G, at0, pages, units, first, n;
+  __host__ __device__ SeqCut(int by_item_, int G_, int start_units, int at, int pages_) : by_item(by_item_), G(G_), pages(pages_) {
+    // with units of fixed cost, all in twos: ranges then begin on whole tiles of their sequences
+    units = pages <= 0 ? 0 : by_item ? pages : start_units ? start_units + (pages + 1) / 2 * 2 : pages;
+    at0 = at + (by_item ? 0 : start_units);
+    first = by_item ? 0 : at0 / G;
+    n = pages <= 0 ? 0 : by_item ? (pages + G - 1) / G : (at0 + pages - 1) / G - first + 1;
+  }
+  __host__ __device__ int begin(int c) const {
+    const int b = by_item ? c * G : (first + c) * G - at0;
+    return b > 0 ? b : 0;
+  }
+  __host__ __device__ int end(int c) const {
+    const int e = by_item ? (c + 1) * G : (first + c + 1) * G - at0;
+    return e < pages ? e : pages;
+  }
+  // of a range's items, is this the one with its first page?  (`at`: as above; a range that begins before the sequence holds pages of
+  // the one before it)
+  __host__ __device__ bool leads(int c, int at) const { return (first + c) * G >= at; }
+};
+
 struct SplitPlan {
-  int chunk_pages = 0;
+  int chunk_pages = 0;                 // of a stream plan: pages of a piece, or units of a range
   int num_items = 0;
   WorkItem* items = nullptr;    // device
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]
   // stream plans only (plan_stream): worker w owns items [worker_first[w], worker_first[w + 1])
   int num_workers = 0;
-  bool by_item = false;                // every worker has one item: chunk_pages pages of a sequence (plan_stream)
+  // every worker has one item, chunk_pages pages of a sequence; or ranges of chunk_pages units, a sequence's pages (an even number of
+  // units) behind `start_units` units of fixed cost (plan_stream)
+  bool by_item = false;
+  int start_units = 0;
   StreamItem* stream_items = nullptr;  // device [num_items]
   int32_t* worker_first = nullptr;     // device [num_workers + 1]
 };
@@ -39,10 +66,10 @@ struct Pool;
 struct SeqBatch;
 int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas_per_item, int min_chunk_pages, int chunk_multiple,
                      int max_chunk_pages, SplitPlan* plan);
-// Stream partition for persistent kernels: the pages of all sequences of the call, laid end to end, are cut into
-// `workers` equal ranges of `chunk_pages` pages (a multiple of `page_multiple`); one item = the part of one sequence
-// inside one range, so a worker meets an item boundary only where a sequence ends inside its range.  Short calls are cut sequence by
-// sequence instead, one item of chunk_pages pages a worker (by_item).
+// Stream partition for persistent kernels: the sequences of the call, laid end to end, are cut into at most `workers` equal ranges;
+// one item = the part of one sequence inside one range, so a worker meets an item boundary only where a sequence ends inside its
+// range.  Where that is cheaper they are cut sequence by sequence instead, one item a worker (cheapest_plan).  With the tuning knob
+// CHUNK_PAGES: ranges of that many pages, rounded up to `page_multiple`.
 // `st`: the stream the builder kernel is launched on (the pool's main stream, or the device's side stream).
 // launch_builder = false: only the host half (counts, buffers); the caller builds the lists itself (the fused decode-step
 // preparation of mla_proj.cu does it inside its own launch).
