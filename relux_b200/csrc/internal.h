@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_ring.h"
 #include "relux_cuda.h"
 
 namespace relux {
@@ -56,11 +57,11 @@ struct Device {
   // Page-locked memory for a call's new rows when they arrive in host memory, read by the kernel that caches them: a copy from pageable
   // memory costs the host 2-3 us and the stream a trip to the copy engine and back (one token through the cache object, 700 cached:
   // 44.2 -> 40.6 us; a step of one sequence 35.3 -> 33.0).  Queries are still copied: every CTA that works on a stream reads them, and
-  // over PCIe that cost more (44.2 -> 46.8).  Calls take pieces one behind another; the stream is waited for where they start again, and a
-  // call that waits for it anyway starts again at its end.  Used under `mu`.
+  // over PCIe that cost more (44.2 -> 46.8).  Calls take their places one behind another; the stream is waited for where they start again,
+  // and a call that waits for it anyway starts again at its end.  Used under `mu`.
   static constexpr size_t kHostInBytes = 1 << 20, kHostInMax = 32 << 10;
   char* host_in = nullptr;
-  size_t host_in_used = 0;
+  HostRing host_in_ring{kHostInBytes};
 };
 
 // A device buffer that grows on demand (never shrinks) for inputs that arrive in host memory

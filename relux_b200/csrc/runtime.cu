@@ -299,21 +299,21 @@ static bool is_device_memory(const void* ptr) {
   return at.type == cudaMemoryTypeDevice;
 }
 
-// A small input that arrives in host memory, for kernels that read it once, by ordinary loads, on the device's stream: *dptr is a copy
-// in page-locked memory.  False: it is not small, or not the host's.
-static bool stage_small(Pool* p, const void* src, size_t bytes, int mem, const void** dptr) {
+// A call's new rows, two tensors, where they arrive in host memory, for kernels that read them once, by ordinary loads, on the device's
+// stream: dst[i] is a copy of src[i] in page-locked memory.  One that is not small, or not the host's, leaves its dst[i] null.
+static void stage_small(Pool* p, const void* const (&src)[2], const size_t (&bytes)[2], int mem, const void* (&dst)[2]) {
   Device* dev = p->dev;
-  if (mem != RELUX_MEM_HOST || bytes > Device::kHostInMax || !dev->host_in || is_device_memory(src)) return false;
-  const size_t need = (bytes + 255) & ~(size_t)255;
-  if (dev->host_in_used + need > Device::kHostInBytes) {
-    if (cudaStreamSynchronize(dev->stream) != cudaSuccess) return false;
-    dev->host_in_used = 0;
-  }
-  char* at = dev->host_in + dev->host_in_used;
-  memcpy(at, src, bytes);
-  dev->host_in_used += need;
-  *dptr = at;
-  return true;
+  dst[0] = dst[1] = nullptr;
+  if (mem != RELUX_MEM_HOST || !dev->host_in) return;
+  int which[2], n = 0;
+  size_t len[2], at[2];
+  for (int i = 0; i < 2; i++)
+    if (bytes[i] <= Device::kHostInMax && !is_device_memory(src[i])) {
+      which[n] = i;
+      len[n++] = bytes[i];
+    }
+  if (!n || !dev->host_in_ring.take(len, n, at, [&] { return cudaStreamSynchronize(dev->stream) == cudaSuccess; })) return;
+  for (int k = 0; k < n; k++) dst[which[k]] = memcpy(dev->host_in + at[k], src[which[k]], len[k]);
 }
 
 // Moves an activation that arrives in host memory to the device staging block.
@@ -441,8 +441,10 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
     if ((rc = pipe_stage_in(p, p->pipe_app_a, a->a, bytes_a, &da, &slot_a))) return rc;
     if ((rc = pipe_stage_in(p, p->pipe_app_b, a->b, bytes_b, &db, &slot_b))) return rc;
   } else {
-    if (!stage_small(p, a->a, bytes_a, a->mem, &da) && (rc = stage_in(p, p->in_a, a->a, bytes_a, a->mem, &da))) return rc;
-    if (!stage_small(p, a->b, bytes_b, a->mem, &db) && (rc = stage_in(p, p->in_b, a->b, bytes_b, a->mem, &db))) return rc;
+    const void* staged[2];
+    stage_small(p, {a->a, a->b}, {bytes_a, bytes_b}, a->mem, staged);
+    if (!(da = staged[0]) && (rc = stage_in(p, p->in_a, a->a, bytes_a, a->mem, &da))) return rc;
+    if (!(db = staged[1]) && (rc = stage_in(p, p->in_b, a->b, bytes_b, a->mem, &db))) return rc;
   }
   if (kind == RELUX_POOL_MLA) rc = launch_mla_append(p, sb, a->layer, da, db, a->dtype, a->advance);
   else rc = launch_gqa_append(p, sb, a->layer, da, db, a->dtype, a->layout, a->advance);
@@ -618,7 +620,7 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
       const bool dev_mem = is_device_memory(a->out);   // asked while the kernels run: 0.7 us of host time before them
       if (dev_mem) RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, p->dev->host_out, out_bytes, cudaMemcpyDefault, p->dev->stream));
       RELUX_CUDA_TRY(cudaStreamSynchronize(p->dev->stream));
-      p->dev->host_in_used = 0;
+      p->dev->host_in_ring.restart();
       if (!dev_mem) memcpy(a->out, p->dev->host_out, out_bytes);
     } else if (a->out_mem == RELUX_MEM_HOST) {
       RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_bytes, cudaMemcpyDeviceToHost, p->dev->stream));
@@ -1274,12 +1276,14 @@ static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_at
   } else if (kv->mem == RELUX_MEM_HOST) {
     // the attention call stages q in in_a: the step's rows get a block of their own
     const size_t off_b = (bytes + 255) & ~(size_t)255;
-    if (!stage_small(p, kv->a, bytes, kv->mem, &da)) {
+    const void* staged[2];
+    stage_small(p, {kv->a, kv->b}, {bytes, bytes}, kv->mem, staged);
+    if (!(da = staged[0])) {
       if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
       da = p->step_rows.p;
       RELUX_CUDA_TRY(cudaMemcpyAsync((void*)da, kv->a, bytes, cudaMemcpyHostToDevice, p->dev->stream));
     }
-    if (!stage_small(p, kv->b, bytes, kv->mem, &db)) {
+    if (!(db = staged[1])) {
       if ((rc = grow(p->dev, p->step_rows, off_b + bytes))) return rc;
       db = (char*)p->step_rows.p + off_b;
       RELUX_CUDA_TRY(cudaMemcpyAsync((void*)db, kv->b, bytes, cudaMemcpyHostToDevice, p->dev->stream));

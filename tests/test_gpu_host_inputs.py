@@ -68,3 +68,45 @@ def test_a_device_address_given_as_host_memory(dev, oracle):  # noqa: F811
     pool.destroy()
     d_k.free()
     d_v.free()
+
+
+def check_rows(dev, oracle, seed, per_call):  # noqa: F811
+    n = sum(per_call)
+    pool = gqa_pool(dev, n)
+    rows = np.random.default_rng(seed).standard_normal((2, n, HKV, D)).astype(np.float32)
+    at = 0
+    for m in per_call:
+        k, v = rows[:, at:at + m].copy()        # gone as soon as the call returns
+        pool.append(0, k, v, 1, n_new=[m])
+        k[:], v[:] = np.nan, np.nan
+        at += m
+    got_k, got_v = pool.read_rows(0, 0, 0, n)
+    assert np.array_equal(got_k, oracle.bf16_from_f32(rows[0])) and np.array_equal(got_v, oracle.bf16_from_f32(rows[1]))
+    assert pool.status() == 0
+    pool.destroy()
+
+
+@pytest.mark.parametrize("rows", [3, 5])        # 12 and 20 KB a tensor: the block's end falls between a call's two tensors
+def test_pairs_that_do_not_divide_the_block(dev, oracle, rows):  # noqa: F811
+    check_rows(dev, oracle, rows, [rows] * 180)  # four and seven turns of the block
+
+
+def test_mixed_sizes_over_several_turns_of_the_block(dev, oracle):  # noqa: F811
+    check_rows(dev, oracle, 9, [int(m) for m in np.random.default_rng(9).integers(1, 11, 200)])   # past the limit (8 rows) too
+
+
+def test_latent_rows_over_several_turns_of_the_block(dev, oracle):  # noqa: F811
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    calls, m, dc, dhr = 180, 8, 512, 64         # 16 KB + 2 KB a call
+    n = calls * m
+    pages = (n + PAGE - 1) // PAGE
+    pool = rb.Pool(dev, L.POOL_MLA, 1, pages, PAGE, 1, pages, dC=dc, dHR=dhr)
+    pool.set_tables(np.arange(pages, dtype=np.int32).reshape(1, pages))
+    rng = np.random.default_rng(4)
+    c, r = (rng.standard_normal((n, w)).astype(np.float32) for w in (dc, dhr))
+    for i in range(0, n, m):
+        pool.append(0, c[i:i + m].copy(), r[i:i + m].copy(), 1, n_new=[m])
+    got_c, got_r = pool.read_rows(0, 0, 0, n)
+    assert np.array_equal(got_c, oracle.bf16_from_f32(c)) and np.array_equal(got_r, oracle.bf16_from_f32(r))
+    pool.destroy()
