@@ -516,7 +516,10 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
   // Puts what reaches key_lo of the elements that the threads with `mine` read in for_segment() on the list.  Where a thread has read
   // eight times or more, a warp goes through one such lane's elements together: a trip to L2 and a few instructions each, where the
   // lane by itself, 64 elements unrolled, took 10 us, most of them its own instructions' way into the cache (131072 logits, 64
-  // sequences: 109 -> 103.5 us a call).  Fewer reads are one trip for all the lanes (32000 logits: 39.5 us so, 42.5 lane by lane).
+  // sequences: 109 -> 103.5 us a call).  Fewer reads are one trip for all the lanes (32000 logits: 39.5 us so, 42.5 lane by lane), and
+  // so are many lanes of a warp, which ties at the bound bring: a lane's turn costs about what 256 elements of a whole look do (128 of rows
+  // that are read one by one).  131072 equal logits, lane by lane -> now: 177 -> 145 us a call of one row, 301 -> 270 of 64; 40 finite ones
+  // among -inf 244 -> 199; 700 ties at the top, 16 rows, 159 -> 152.  (Four lanes as the limit: 64 ordinary rows 41.4 -> 42.3.)
   auto collect = [&](uint32_t key_lo, bool mine) {
     auto put = [&](int i, float v) {
       const float x = d.scaled(v);
@@ -526,12 +529,13 @@ __device__ bool sample_row_candidates(Ctx& c, const SelParams& prm, const float*
       }
     };
     const int width = c.vec ? 4 : 1;
-    if (c.whi - c.wlo < 8 * 32 * width) {
+    uint32_t lanes = __ballot_sync(0xffffffffu, mine);
+    if (c.whi - c.wlo < 8 * 32 * width || __popc(lanes) * (c.vec ? 256 : 128) > c.whi - c.wlo) {
       if (mine) for_segment(c, row, put);
       return;
     }
 #pragma unroll 1
-    for (uint32_t lanes = __ballot_sync(0xffffffffu, mine); lanes; lanes &= lanes - 1) {
+    for (; lanes; lanes &= lanes - 1) {
 #pragma unroll 1
       for (int i = c.wlo + (__ffs(lanes) - 1 + 32 * c.lane) * width; i < c.whi; i += 1024 * width) {
         const float4 v = load4(c, row, i, c.whi);
