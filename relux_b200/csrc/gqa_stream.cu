@@ -38,11 +38,6 @@ namespace relux {
 
 namespace {
 
-// A page is read once.  The pages of a call of more than half of L2 are loaded to be evicted first, so that they push out each other and
-// not what the next launches read, nor, in turn after turn, all of themselves: 32 sequences of 100 to 3000 tokens 45.0 -> 43.2 us, 100 of
-// 22 to 700 (64 heads) 42.0 -> 36.5, 16 x 2000 29.2 -> 26.6, a layer of 24 x 2048 66.8 -> 65.9.  Smaller ones may stay in L2 from step to
-// step, which 32 x <= 1000 with 4 kv heads, 34 MB, did less so (16.0 -> 16.65).
-constexpr int64_t kResidentBytes = (int64_t)63 << 20;
 constexpr int kInlineSmall = 32, kInlineLarge = 256;   // sequences carried as kernel arguments (0.5 KB / 4 KB)
 
 struct GqaSeq {
@@ -57,7 +52,11 @@ struct GqaStreamCommon {
   const int32_t* table;
   int32_t table_stride, num_pages, n_seqs, range, range_more, Hkv, H, g, S, R, extra, causal;
   int32_t krow0, vrow0;    // first TMA row of this layer's K block / V block
-  int32_t streams;         // the call's pages stream through L2 (kResidentBytes)
+  // A page is read once.  The pages of a call of more than half of L2 are loaded to be evicted first, so that they push out each other
+  // and not what the next launches read, nor, in turn after turn, all of themselves: 32 sequences of 100 to 3000 tokens 45.0 -> 43.2 us,
+  // 100 of 22 to 700 (64 heads) 42.0 -> 36.5, 16 x 2000 29.2 -> 26.6, a layer of 24 x 2048 66.8 -> 65.9.  Smaller ones may stay in L2 from
+  // step to step, which 32 x <= 1000 with 4 kv heads, 34 MB, did less so (16.0 -> 16.65).
+  int32_t streams;
   float scale_log2;
   const void* q;
   int32_t q_bf16, out_bf16;

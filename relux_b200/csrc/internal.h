@@ -30,6 +30,8 @@ int32_t cuda_fail(cudaError_t e, const char* what);
     if (e__ != cudaSuccess) return ::relux::cuda_fail(e__, #expr); \
   } while (0)
 
+constexpr int64_t kResidentBytes = (int64_t)63 << 20;   // half of L2: what a launch may count on finding there again
+
 struct Device {
   uint32_t magic = kDeviceMagic;
   int index = 0;

@@ -116,6 +116,10 @@ struct GemmParams {
   // 84 MB, with the cached rows loaded so too, 66.6 -> 65.1 (24 x 2048), 76.4 -> 73.3 (128 x 300), 35.2 -> 34.3 (2 x 400).  Fewer may stay
   // in L2 from call to call.
   int32_t streams;
+  // The result of more than 32 rows, in all its pieces no more than half of L2, is stored to stay there until it is summed (layer steps:
+  // 100 x 1000 of d_model 4096 113 -> 107.6 us, 60 x 1000 of 16384 281 -> 278; up to 32 rows 1 % slower so).  More cannot stay, and would
+  // push out what can (layer prompts of 2 x 2048 and 4 x 2048 tokens, 100 and 201 MB: 523 and 1013 us so, 521 and 1007 without).
+  int32_t keeps;
   int32_t* status;
   TimeStamp time;                        // input projections only
 };
@@ -266,11 +270,9 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
       __syncwarp();
     }
   } else {
-    // Epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once.  The result of
-    // more than 32 rows, some MB that the next launch sums and the next GEMM overwrites, is stored to stay in L2 meanwhile (layer
-    // steps: 100 x 1000 of d_model 4096 113 -> 107.6 us, 60 x 1000 of 16384 281 -> 278; up to 32 rows 1 % slower so).
+    // epilogue: thread = weight column, accumulator column = activation row; a warp writes 128 bytes of a row at once
     constexpr bool kKeep = NT >= 64;
-    const uint64_t evict_last = kKeep ? make_evict_last_policy() : 0;
+    const uint64_t stay = !kKeep ? 0 : prm.keeps ? make_evict_last_policy() : make_evict_normal_policy();
     chain_wait();
     for (int piece = 0; walk.next(); piece++) {
       const int j = weight_of(walk.col), m0 = kBlocks ? walk.block * NT : 0;
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(192, 1) skinny_gemm_sm100_kernel(const __grid_
           if (mine && c + q < m_end) {
             float* to = dst + (size_t)(c + q) * prm.n_total;
             const float x = ok ? __uint_as_float(v[q]) : 0.f;
-            if constexpr (kKeep) store_hint(to, x, evict_last);
+            if constexpr (kKeep) store_hint(to, x, stay);
             else *to = x;
           }
       }
@@ -526,6 +528,9 @@ int32_t launch_skinny_gemm(Pool* p, const uint16_t* a_bf16, int M, int K, const 
   const int workers = g.rg.workers * g.rg.beside;
   g.part = part;
   g.streams = g.rg.row_blocks == 1 && (int64_t)K * cols * 2 > ((int64_t)16 << 20);
+  const int tiles_of_block = g.rg.full * g.rg.workers + g.rg.rest;
+  const int pieces_of_block = g.rg.full * g.rg.workers + (g.rg.split ? g.rg.rest * g.rg.split : g.rg.rest ? g.rg.rest + g.rg.workers : 0);
+  g.keeps = (int64_t)M * cols * 4 * pieces_of_block / tiles_of_block <= kResidentBytes;
   g.status = p->d_status;
   g.time = time;
   *ranges = g.rg;

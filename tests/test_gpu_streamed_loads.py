@@ -48,3 +48,22 @@ def test_cached_pages_around_half_of_l2(dev, oracle, B):  # noqa: F811
     assert np.linalg.norm(out - ref) <= 1e-2 * np.linalg.norm(ref)     # probabilities rounded to bf16
     assert pool.status() == 0
     pool.destroy()
+
+
+# results of half of L2 (63 MB) and more are not stored to stay there: 2730 rows of 6144 columns are 67 MB, 2500 are 61
+@pytest.mark.parametrize("m", [2500, 2730])
+def test_a_result_that_does_not_fit_in_l2(dev, oracle, m):  # noqa: F811
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    k, n = 256, 6144
+    rng = np.random.default_rng(m)
+    pool = rb.Pool(dev, L.POOL_MLA, 1, 2, 64, 1, 2, dC=64, dHR=16)
+    a = oracle.f32_from_bf16(oracle.bf16_from_f32(rng.standard_normal((m, k)).astype(np.float32)))
+    w = oracle.bf16_from_f32(rng.standard_normal((k, n)).astype(np.float32))
+    d_w = dev.upload(w)
+    got = pool.matmul(a, d_w, n)
+    ref = a.astype(np.float64) @ oracle.f32_from_bf16(w).astype(np.float64)
+    assert np.abs(got - ref).max() <= k * 2.0 ** -24 * 0.64 * k
+    assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
+    d_w.free()
+    pool.destroy()
