@@ -499,9 +499,11 @@ int32_t relux_gqa_decode_noalloc(relux_pool_t pool, const relux_attn_args* args)
 int32_t relux_seq_save_file(relux_pool_t pool, int32_t seq_id, const char* path, int32_t max_len);
 int32_t relux_seq_load_file(relux_pool_t pool, int32_t seq_id, const char* path, int32_t max_len, const int32_t* layer_len);
 
-/* The stream partition the persistent MLA decode kernel works on, computed on the host from page counts (no device
- * needed): the pages of all sequences, laid end to end, are cut into ranges of *range_pages_out pages (a multiple of
- * page_multiple), one range per worker; an item is the part of one sequence inside one range.
+/* A partition of cached pages into equal ranges, computed on the host from page counts (no device needed): the pages of
+ * all sequences, laid end to end, are cut into ranges of *range_pages_out pages (a multiple of page_multiple), one range
+ * per worker; an item is the part of one sequence inside one range.  It is what the persistent MLA decode kernel works on
+ * under RELUX_TUNE_CHUNK_PAGES = *range_pages_out; by default that kernel also counts what an item costs to start and to
+ * write out, and cuts short calls sequence by sequence.
  * items_out: n x {seq_index, page_begin, page_end, worker} (cap items of room), worker_first [*workers_out + 1],
  * chunk_off [n_seqs + 1]; any of the three may be NULL.  Returns the number of items, -1 on bad arguments or when cap
  * is too small.  Scheduling aid: no counterpart in the reference. */

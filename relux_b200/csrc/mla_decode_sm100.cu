@@ -9,7 +9,7 @@
 // the two CTAs' shared memories and read by both tensor cores.  No TMA multicast is used anywhere: each CTA
 // issues its own loads (`.cta_group::2` only routes the completion bytes to the leader's mbarrier).
 //
-// Persistent workers over a stream partition (or, short calls, a piece of one sequence each: cheapest_plan in splitkv.cu).  The pages of all sequences of the call, laid end to end, are cut
+// Persistent workers over a stream partition (or, short calls, a piece of one sequence each: cheapest_plan in stream_plan.h).  The pages of all sequences of the call, laid end to end, are cut
 // into as many equal ranges as CTA pairs fit on the GPU; a worker (one pair) walks its range once.  An ITEM is
 // the part of one sequence inside one range, so a worker changes item (new Q~, new accumulator, one split-KV
 // partial written) only where a sequence ends inside its range.  The tile pipeline does not drain at an item

@@ -182,8 +182,7 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
   for (int w = (by_item ? item_base : (unit_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
 }
 
-// Host statement of the stream partition: range length G and the counts that follow from it.  The device builder
-// (build_stream_kernel) applies the same arithmetic to the device-resident lengths.
+// Equal ranges of pages (the tuning knob CHUNK_PAGES, relux_stream_partition): range length G and the counts that follow from it.
 void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_multiple, long chunk_override, long* G_out,
                             int* workers_out, int* items_out) {
   long total = 0;
@@ -202,71 +201,6 @@ void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_
   *G_out = G;
   *workers_out = (int)std::max<long>(1, (total + G - 1) / G);
   *items_out = items;
-}
-
-// What a plan costs, in tiles of two pages (about 2 us): its slowest worker's tiles and two for every item (start and write-out), 0.08 for
-// every partial that a row of the merge adds up, and 0.035 for every partial of the call.  From steps of 1 to 30 short sequences with
-// ranges of one and of two tiles (1 x 1300 tokens 19.9 against 21.5 us, 1 x 2600 21.5 and 21.4, 1 x 6000 26.8 and 24.0, 4 x 1200 24.0 and
-// 23.3, 25 x 200 27.4 and 28.3).
-static double plan_cost(double worst, int most_items, int items) { return worst + 0.08 * most_items + 0.035 * items; }
-
-// The cheapest plan of a call: equal ranges of the sequences laid end to end, each counted as its pages and kStartUnits, for a worker
-// that starts it has a second item to start and to write out; or every sequence cut by itself into pieces of 2 t pages, a worker each.
-// Measured, ranges of pages alone -> this: in ranges, 16 x <= 32768 tokens 99.3 -> 97.3 us, 64 x 32768 611 -> 591, 20 x 16000 80.5 -> 72.3;
-// in pieces, 3 x <= 1500 26.4 -> 21.9, 16 x 300 28.0 -> 24.4, 64 x 300 48.7 -> 38.4, 40 x <= 2500 51.4 -> 45.3, 64 x 4096 95.5 -> 91.3.
-constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for an item
-struct StreamShape {
-  int G, workers, items, start_units;
-  bool by_item;
-};
-static StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
-  int longest = 0, live = 0;
-  int64_t units = 0;
-  for (int n : pages) {
-    longest = std::max(longest, n);
-    live += n > 0;
-    units += SeqCut(0, 1, kStartUnits, 0, n).units;
-  }
-  StreamShape r{};
-  r.start_units = kStartUnits;
-  r.G = std::max((int)((units + workers - 1) / workers + 1) / 2 * 2, 2 * kStartUnits);
-  r.workers = std::max(1, (int)((units + r.G - 1) / r.G));
-  int at = 0, most = 0, of_worker = -1;
-  double worst = 0, here = 0;   // of the ranges, walked as the workers walk them
-  for (int n : pages) {
-    const SeqCut cut(0, r.G, kStartUnits, at, n);
-    for (int c = 0; c < cut.n; c++) {
-      if (cut.first + c != of_worker) here = 0;
-      of_worker = cut.first + c;
-      here += (cut.end(c) - cut.begin(c) + 1) / 2 + 2;
-      worst = std::max(worst, here);
-    }
-    most = std::max(most, cut.n);
-    r.items += cut.n;
-    at += cut.units;
-  }
-  if (live == 0 || live > workers) return r;
-  double best = plan_cost(worst, most, r.items);
-  auto items_of = [&](int t) {
-    int items = 0;
-    for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
-    return items;
-  };
-  int lo = 1, hi = (longest + 1) / 2;   // the smallest t whose pieces find a worker each: one piece a sequence does
-  while (lo < hi) {
-    const int t = (lo + hi) / 2;
-    if (items_of(t) <= workers) hi = t;
-    else lo = t + 1;
-  }
-  for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
-    const int items = items_of(t);
-    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
-    if (cost < best) {
-      best = cost;
-      r = StreamShape{2 * t, items, items, 0, true};
-    }
-  }
-  return r;
 }
 
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
@@ -311,9 +245,8 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
 
 }  // namespace relux
 
-// The stream partition computed on the host from page counts (no device involved): equal ranges of whole tiles over the
-// sequences laid end to end, as the persistent MLA decode kernel walks them (its own planner also counts what the start
-// of a sequence costs, see cheapest_plan).  items_out receives n_items x {seq_index, page_begin,
+// The equal ranges of the tuning knob CHUNK_PAGES computed on the host from page counts (no device involved); without the knob
+// the persistent MLA decode kernel walks cheapest_plan (stream_plan.h).  items_out receives n_items x {seq_index, page_begin,
 // page_end, worker}; worker_first [workers_out + 1]; chunk_off [n_seqs + 1].  Returns the number of items, or -1 when
 // `cap` items are not enough.  Scheduling aid for callers and tests; no counterpart in the reference.
 extern "C" __attribute__((visibility("default"))) int32_t relux_stream_partition(const relux_stream_partition_args* args) {

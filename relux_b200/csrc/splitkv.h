@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "stream_plan.h"
+
 namespace relux {
 
 struct WorkItem {
@@ -21,30 +23,6 @@ struct __align__(16) StreamItem {
   int32_t page_end;
   int32_t tokens;      // cached length of the sequence + the call's extra tokens
   int32_t pad[3];
-};
-
-// The items of a sequence of `pages` pages that begins at unit `at` of the stream: item c is its pages [begin(c), end(c)), and belongs to
-// worker first + c, or (by_item) to a worker of its own.  What the host counts and the device builds from.
-struct SeqCut {
-  int by_item, G, at0, pages, units, first, n;
-  __host__ __device__ SeqCut(int by_item_, int G_, int start_units, int at, int pages_) : by_item(by_item_), G(G_), pages(pages_) {
-    // with units of fixed cost, all in twos: ranges then begin on whole tiles of their sequences
-    units = pages <= 0 ? 0 : by_item ? pages : start_units ? start_units + (pages + 1) / 2 * 2 : pages;
-    at0 = at + (by_item ? 0 : start_units);
-    first = by_item ? 0 : at0 / G;
-    n = pages <= 0 ? 0 : by_item ? (pages + G - 1) / G : (at0 + pages - 1) / G - first + 1;
-  }
-  __host__ __device__ int begin(int c) const {
-    const int b = by_item ? c * G : (first + c) * G - at0;
-    return b > 0 ? b : 0;
-  }
-  __host__ __device__ int end(int c) const {
-    const int e = by_item ? (c + 1) * G : (first + c + 1) * G - at0;
-    return e < pages ? e : pages;
-  }
-  // of a range's items, is this the one with its first page?  (`at`: as above; a range that begins before the sequence holds pages of
-  // the one before it)
-  __host__ __device__ bool leads(int c, int at) const { return (first + c) * G >= at; }
 };
 
 struct SplitPlan {

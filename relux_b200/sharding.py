@@ -34,8 +34,9 @@ def aggregate_throughput(units_per_rank, ms_per_rank):
 
 
 def stream_partition(pages, workers, page_multiple=2):
-    """The stream partition of the persistent MLA decode kernel for sequences of pages[i] pages (computed by the
-    library on the host; no GPU needed).  Returns (range_pages, n_workers, items, worker_first, chunk_off) with items an
+    """Equal ranges over the pages of sequences of pages[i] pages laid end to end (computed by the library on the host; no
+    GPU needed): what the persistent MLA decode kernel works on under the tuning knob CHUNK_PAGES = range_pages (its default
+    plan also counts what an item costs to start and to write out, and cuts short calls sequence by sequence).  Returns (range_pages, n_workers, items, worker_first, chunk_off) with items an
     int32 array [n, 4] of {seq_index, page_begin, page_end, worker}."""
     import ctypes as C
 

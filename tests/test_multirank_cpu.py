@@ -78,7 +78,8 @@ def test_two_gloo_ranks_shard_and_reduce_timings():
 
 
 def test_stream_partition_properties():
-    """The partition the persistent MLA decode kernel walks (host statement of the same arithmetic): every page of every
+    """The equal ranges of relux_stream_partition, which the persistent MLA decode kernel walks under the tuning knob CHUNK_PAGES
+    (its default plan: test_stream_plan.py): every page of every
     sequence is in exactly one item, items of a sequence and of a worker are contiguous, no worker holds more than one
     range, ranges are whole tiles."""
     import __graft_entry__ as g
