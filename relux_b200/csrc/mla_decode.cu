@@ -241,8 +241,9 @@ int32_t launch_generic(Pool* p, const MlaGenParams& k, int items, cudaStream_t s
 }
 
 int32_t grow_partials(Pool* p, const SplitPlan& plan, int rows_total, int dC) {
-  const int32_t rc = grow(p->dev, p->part_o, (size_t)plan.num_items * rows_total * dC * sizeof(float));
-  return rc ? rc : grow(p->dev, p->part_ml, (size_t)plan.num_items * rows_total * 2 * sizeof(float));
+  const size_t rows = (size_t)std::max(plan.num_items, plan.room_items) * rows_total;
+  const int32_t rc = grow(p->dev, p->part_o, rows * dC * sizeof(float));
+  return rc ? rc : grow(p->dev, p->part_ml, rows * 2 * sizeof(float));
 }
 
 }  // namespace

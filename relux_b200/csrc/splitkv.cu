@@ -216,19 +216,21 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
     long G = 0;
     stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, chunk, &G, &shape.workers, &shape.items);
     shape.G = (int)G;
+    shape.room = shape.items;
   } else {
     shape = cheapest_plan(pages, workers);
   }
-  const int G = shape.G, items = shape.items;
+  const int G = shape.G, items = shape.items, most_workers = workers;
   workers = shape.workers;
   plan->by_item = shape.by_item;
   plan->start_units = shape.start_units;
   plan->chunk_pages = G;
   plan->num_items = items;
+  plan->room_items = shape.room;
   plan->num_workers = workers;
-  const size_t off_chunk = sizeof(StreamItem) * (size_t)items;
+  const size_t off_chunk = sizeof(StreamItem) * (size_t)shape.room;
   const size_t off_worker = (off_chunk + sizeof(int32_t) * ((size_t)sb.n_seqs + 1) + 15) & ~(size_t)15;
-  int32_t rc = grow(p->dev, p->work, off_worker + sizeof(int32_t) * ((size_t)workers + 1) + 64);
+  int32_t rc = grow(p->dev, p->work, off_worker + sizeof(int32_t) * ((size_t)std::max(workers, most_workers) + 1) + 64);
   if (rc) return rc;
   plan->items = nullptr;
   plan->stream_items = (StreamItem*)p->work.p;

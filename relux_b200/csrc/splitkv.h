@@ -28,6 +28,7 @@ struct __align__(16) StreamItem {
 struct SplitPlan {
   int chunk_pages = 0;                 // of a stream plan: pages of a piece, or units of a range
   int num_items = 0;
+  int room_items = 0;           // partials are given room for as many (num_items, where that is more): StreamShape::room
   WorkItem* items = nullptr;    // device
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]
   // stream plans only (plan_stream): worker w owns items [worker_first[w], worker_first[w + 1])

@@ -52,6 +52,7 @@ constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for 
 struct StreamShape {
   int G, workers, items, start_units;
   bool by_item;
+  int room;   // items of the larger of the plans compared: scratch for as many serves the call on either side of their border
 };
 inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   int longest = 0, live = 0;
@@ -79,6 +80,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
     r.items += cut.n;
     at += cut.units;
   }
+  r.room = r.items;
   if (live == 0 || live > workers) return r;
   double best = plan_cost(worst, most, r.items);
   auto items_of = [&](int t) {
@@ -95,9 +97,10 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
     const int items = items_of(t);
     const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
+    r.room = std::max(r.room, items);
     if (cost < best) {
       best = cost;
-      r = StreamShape{2 * t, items, items, 0, true};
+      r = StreamShape{2 * t, items, items, 0, true, r.room};
     }
   }
   return r;

@@ -51,7 +51,7 @@ static bool check(const std::vector<int>& pages, int workers) {
     if (s.by_item) CHECK(worker_first[w + 1] == worker_first[w] + 1);
   }
   CHECK(worker_first[s.workers] == s.items && (live == 0) == (s.items == 0));
-  CHECK(s.items <= std::max(1, workers) + live);           // what scratch is sized for
+  CHECK(s.room >= s.items && s.room <= std::max(1, workers) + live);   // what scratch is sized for
   return true;
 }
 
@@ -60,7 +60,7 @@ int main(int argc, char** argv) {
     std::vector<int> pages;
     for (int i = 2; i < argc; i++) pages.push_back(atoi(argv[i]));
     const StreamShape s = cheapest_plan(pages, atoi(argv[1]));
-    printf("%s %d %d %d\n", s.by_item ? "pieces" : "ranges", s.G, s.workers, s.items);
+    printf("%s %d %d %d %d\n", s.by_item ? "pieces" : "ranges", s.G, s.workers, s.items, s.room);
     return 0;
   }
   std::mt19937 rng(3);

@@ -28,3 +28,16 @@ def test_which_plan_a_call_gets(exe, tokens, workers, plan):
     pages = [str((t + 63) // 64) for t in tokens]
     out = subprocess.run([exe, str(workers)] + pages, capture_output=True, text=True, timeout=60)
     assert out.returncode == 0 and out.stdout.split()[0] == plan, out.stdout
+
+
+def test_scratch_serves_both_plans(exe):
+    """64 sequences that grow from one plan into the other: what the call after the change needs is there already, but for the few items
+    by which ranges change from length to length."""
+    plans = []
+    for pages in range(20, 560, 4):
+        out = subprocess.run([exe, "74"] + [str(pages)] * 64, capture_output=True, text=True, timeout=60).stdout.split()
+        plans.append((out[0], int(out[3]), int(out[4])))
+    borders = [(a, b) for a, b in zip(plans, plans[1:]) if a[0] != b[0]]
+    assert borders
+    for (_, _, room), (_, items, _) in borders:
+        assert items <= room + 10
