@@ -56,10 +56,10 @@ struct Device {
   // 15 us at 512 KB; at 1 MB and more the driver's own copy is as fast or faster.
   static constexpr size_t kHostOutBytes = 512 << 10;
   void* host_out = nullptr;
-  // Page-locked memory for a call's new rows when they arrive in host memory, read by the kernel that caches them: a copy from pageable
-  // memory costs the host 2-3 us and the stream a trip to the copy engine and back (one token through the cache object, 700 cached:
+  // Page-locked memory for the new rows of an append or a GQA step that arrive in pageable memory, read by the kernel that caches them: a
+  // copy costs the host 2-3 us and the stream a trip to the copy engine and back (one token through the cache object, 700 cached:
   // 44.2 -> 40.6 us; a step of one sequence 35.3 -> 33.0).  Queries are still copied: every CTA that works on a stream reads them, and
-  // over PCIe that cost more (44.2 -> 46.8).  Calls take their places one behind another; the stream is waited for where they start again,
+  // over PCIe that cost more (44.2 -> 46.8); so are a latent step's rows.  Calls take their places one behind another; the stream is waited for where they start again,
   // and a call that waits for it anyway starts again at its end.  Used under `mu`.
   static constexpr size_t kHostInBytes = 1 << 20, kHostInMax = 32 << 10;
   char* host_in = nullptr;

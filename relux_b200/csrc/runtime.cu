@@ -298,17 +298,29 @@ static bool is_device_memory(const void* ptr) {
   }
   return at.type == cudaMemoryTypeDevice;
 }
+// Memory that the runtime reads before a copy from it returns.  Page-locked and managed memory it reads in the order of the stream: what
+// is queued there may still be writing it.
+static bool is_pageable(const void* ptr) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
 
-// A call's new rows, two tensors, where they arrive in host memory, for kernels that read them once, by ordinary loads, on the device's
-// stream: dst[i] is a copy of src[i] in page-locked memory.  One that is not small, or not the host's, leaves its dst[i] null.
+// A call's new rows, two tensors, where they arrive in pageable host memory, for kernels that read them once, by ordinary loads, on the
+// device's stream: dst[i] is a copy of src[i] in page-locked memory.  One that is not small or not pageable leaves its dst[i] null, and
+// so do both while the stream is captured: a graph reads its inputs when it is launched.
 static void stage_small(Pool* p, const void* const (&src)[2], const size_t (&bytes)[2], int mem, const void* (&dst)[2]) {
   Device* dev = p->dev;
   dst[0] = dst[1] = nullptr;
-  if (mem != RELUX_MEM_HOST || !dev->host_in) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (mem != RELUX_MEM_HOST || !dev->host_in || cudaStreamIsCapturing(dev->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
   int which[2], n = 0;
   size_t len[2], at[2];
   for (int i = 0; i < 2; i++)
-    if (bytes[i] <= Device::kHostInMax && !is_device_memory(src[i])) {
+    if (bytes[i] <= Device::kHostInMax && is_pageable(src[i])) {
       which[n] = i;
       len[n++] = bytes[i];
     }
