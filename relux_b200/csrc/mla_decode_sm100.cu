@@ -350,9 +350,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     const int hf = L >> 6;            // token half of the tile (= which CTA's page)
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full), 0);
-    // The partial results (36 MB at 64 sequences) wait for the merge while cached rows stream through L2, and came back from HBM:
-    // stored to be evicted last, a step of 64 x 4096 takes 98.9 us instead of 101.1, 16 x <= 32k 97.7 instead of 99.9.  (Cached rows
-    // loaded to be evicted first were gone before their second load, as values: 114 -> 127 us.)
+    // The partial results (256 KB an item at 128 heads: 17 MB in 64 pieces, 36 MB in 138 items of ranges) wait for the merge while cached
+    // rows stream through L2, and came back from HBM: stored to be evicted last, a step of 64 x 4096 takes 89.2 us instead of 90.5, 40 x
+    // <= 2500 45.2 instead of 46.2, 20 x 16000 94.5 instead of 95.8; shorter ones the same.  They stay while the pool is in use: a program's
+    // own pass over 96 MB behind a step of 64 x 1000 then takes 40 us instead of 37.5 (48 MB: no difference), and no less with a merge that
+    // reads them to be evicted first, which itself takes 1 us longer.  (Cached rows loaded to be evicted first were gone before their second
+    // load, as values: 114 -> 127 us.)
     const uint64_t evict_last = make_evict_last_policy();
     StreamItem cur = load_item(prm.items + it0);
     int g = 0;

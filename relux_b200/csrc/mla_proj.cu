@@ -469,8 +469,10 @@ __device__ __forceinline__ void merge_rows_piped(uint8_t* As, const float* part_
 // and D[128 output dims x rows] = W_UV^T O on tcgen05: the weights are the M = 128 operand as they lie (MN-major), the rows the N
 // operand (16, 32 or 64, K-major blocks of 64 columns), one tensor-memory column per row.  Rows of the tile past the batch hold
 // whatever shared memory held: their columns of D are not read.
-// Clock stamps at 64 sequences of 4096 tokens, 64 rows: merge 15-16.5 k (17-22 k with one row's round trips after another), MMAs
-// 4.5 k (7 k with mma.sync, whose fragments come from shared memory four times each), the outputs 2.5 k.
+// Clock stamps at 64 sequences of 4096 tokens, 64 rows of one item each: merge 15-16 k, MMAs 3.2 k, of which their issue is 2.8 k, the
+// outputs 1.5 k.  (With two items a row, the plan of equal ranges: merge 15-16.5 k, 17-22 k with one row's round trips after another; MMAs
+// by mma.sync, whose fragments come from shared memory four times each, 7 k.)  The code runs once and waits for its own instructions: an
+// operand more, for what the rows' rounding leaves, took 2-3 us of the launch, not the 0.4 of its MMAs, and one MMA a turn 3.
 // All of W_UV's slice for this head (dC x 128 bf16) is fetched by one thread as 2 * nk TMA boxes before chain_wait(): the
 // weights do not depend on the decode kernel, and the launches before it have waited for everything older (as 512 bulk
 // copies of a row each, issued behind the merge's first loads, they took 2-3 us to be accepted).

@@ -46,8 +46,11 @@ inline double plan_cost(double worst, int most_items, int items) { return worst 
 
 // The cheapest plan of a call: equal ranges of the sequences laid end to end, each counted as its pages and kStartUnits, for a worker
 // that starts it has a second item to start and to write out; or every sequence cut by itself into pieces of 2 t pages, a worker each.
-// Measured, ranges of pages alone -> this: in ranges, 16 x <= 32768 tokens 99.3 -> 97.3 us, 64 x 32768 611 -> 591, 20 x 16000 80.5 -> 72.3;
-// in pieces, 3 x <= 1500 26.4 -> 21.9, 16 x 300 28.0 -> 24.4, 64 x 300 48.7 -> 38.4, 40 x <= 2500 51.4 -> 45.3, 64 x 4096 95.5 -> 91.3.
+// Measured, ranges of pages alone -> this, one build: in pieces, 1 x 1300 tokens 21.8 -> 20.2 us, 3 x <= 1500 26.9 -> 22.3, 16 x 300 28.6 ->
+// 25.1, 64 x 300 41.0 -> 40.5, 40 x <= 2500 51.1 -> 45.1, 64 x 4096 93.8 -> 89.4, with 32 heads 64 x 500 42.5 -> 35.7; in ranges, 20 x 16000
+// 97.3 -> 95.5, and no difference beyond the runs' own at 16 x <= 32768 (97) and 64 x 32768 (565-585).  The fit is to one query token and
+// 128 heads; elsewhere: verify of 3 x <= 1500 with 4 tokens 39.1 -> 34.0, 16 x 300 with 2 43.2 -> 37.9, 32 x 1000 with 4 87.6 -> 79.3, 30 x
+// <= 800 with 3 and 32 heads 52.1 -> 46.2, the other way 64 x 300 with 2 and 32 heads 48.5 -> 50.1.
 constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for an item
 struct StreamShape {
   int G, workers, items, start_units;

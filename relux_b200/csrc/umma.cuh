@@ -26,7 +26,8 @@ __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same without ordering memory: at a kernel's end, where the release waited up to 1200 clocks for stores on their way.
+// The same without ordering memory: at a kernel's end, where the release waited up to 1200 clocks for stores on their way.  (What follows
+// it may run while they still are; the next launch waits for the grid's completion, and with it for them.)
 __device__ __forceinline__ void cluster_sync_relaxed() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
