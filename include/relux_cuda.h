@@ -524,7 +524,7 @@ int32_t relux_stream_partition(const relux_stream_partition_args* args);
 /* Device time of the dominant attention kernel of the most recent relux_*_decode / verify / step call on this pool (for
  * token selection, of the selection kernel).  The tensor-core kernels stamp %globaltimer themselves: from the first block
  * that has its inputs (the kernel before it in the stream complete) to the end of the last block; launch overhead is not in
- * it, nor is the way to L2 of results that the latent decode kernel and the projections have just stored (up to 0.7 us), and
+ * it, nor is the way to L2 of results that the latent decode kernel (up to 0.7 us) and the projections have just stored, and
  * for a GQA step the append and the merge are.  The reference-mode and generic kernels, and GQA prompts as grid
  * slices, are timed by CUDA events around their launches.  Synchronises the stream.  Measurement aid: no counterpart in
  * the reference. */
