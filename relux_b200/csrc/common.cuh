@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <stdint.h>
 
 #include "relux_cuda.h"
@@ -30,6 +31,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+
+__device__ __forceinline__ uint32_t round_bf16x2(float lo, float hi) {   // to nearest, by the conversion instruction (pack_bf16x2: the reference's rule)
+  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&b);
+}
 
 // fastexp32 of internal/transformer/mha.go:823-833 with its operations kept unfused.
 __device__ __forceinline__ float fastexp32_ref(float x) {
@@ -133,6 +139,14 @@ __device__ __forceinline__ uint64_t make_evict_normal_policy() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
+}
+// A box of a 5-D map (a reordered view of a matrix).
+__device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z, int32_t u, int32_t w, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(
+          smem_u32(smem_dst)),
+      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u), "r"(w)
+      : "memory");
 }
 // 2-D tiled TMA store shared -> global of one box (bulk async-group completion).  The shared tile must have been made
 // visible to the async proxy (fence_proxy_async) by the threads that wrote it.
@@ -241,8 +255,20 @@ __device__ __forceinline__ void store_hint(void* p, const uint4& v, uint64_t pol
                "l"(policy)
                : "memory");
 }
+// A store by a predicate, not behind a branch.
+__device__ __forceinline__ void store_if(float* p, float v, bool there) {
+  asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.s32 t, %2, 0;\n\t@t st.global.f32 [%0], %1;\n\t}" ::"l"(__cvta_generic_to_global(p)), "f"(v), "r"((int)there) : "memory");
+}
+__device__ __forceinline__ void store_if(uint16_t* p, uint16_t v, bool there) {
+  asm volatile("{\n\t.reg .pred t;\n\tsetp.ne.s32 t, %2, 0;\n\t@t st.global.u16 [%0], %1;\n\t}" ::"l"(__cvta_generic_to_global(p)), "h"(v), "r"((int)there) : "memory");
+}
 __device__ __forceinline__ void store_hint(float* p, float v, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(__cvta_generic_to_global(p)), "f"(v), "l"(policy) : "memory");
+}
+
+// Brings [p, p + bytes) into L2 (both multiples of 16).
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {

@@ -248,16 +248,6 @@ __device__ __forceinline__ void wait_bar(uint64_t* bar, uint32_t parity, Bars* b
   if (!mbar_try_wait(bar, parity)) wait_slow(bar, parity, b, status);
 }
 
-// 3-D tiled TMA load issued by either CTA of a pair into ITS OWN shared memory; the completion bytes go to an mbarrier
-// given as a shared::cluster address (the pair leader's).  No multicast.
-__device__ __forceinline__ void tma_load_3d_2sm(void* smem_dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z, uint32_t bar_cluster_addr) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
-          smem_u32(smem_dst)),
-      "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
-
 // tmap_kv: GQA the pool's K / V rows; MLA the expanded keys / values.  tmap_q: the queries (MLA: their nope part).
 // tmap_qr, tmap_rope (MLA only): the queries' RoPE part, and the pool's 64-column blocks.  tmap_out: [n][S][H][128] float32.
 template <bool kMla>

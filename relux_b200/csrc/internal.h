@@ -157,6 +157,7 @@ struct Pool {
   GrowBuf o_lat;     // MLA merged latent output, f32/bf16
   // TMA descriptors over the pool storage (built at create when the shape allows it)
   CUtensorMap tmap_mla{};   // 2-D [rows][dC+dHR], box 64 x 64, 128-byte swizzle
+  CUtensorMap tmap_mla_2{}, tmap_mla_3{};   // the same in boxes of two and of three neighbouring blocks of a page
   CUtensorMap tmap_gqa{};   // 2-D [rows][D],      box 64 x 64, 128-byte swizzle
   bool has_tmap = false;
   bool mla_blocked = false;   // MLA pages stored as 64-column blocks (see mla_page_off)
@@ -269,6 +270,8 @@ int32_t check_dev_align(const void* ptr, const char* what);
 //   2-D: [rows][cols], cols contiguous, box = box_cols x box_rows.
 //   3-D: [outer][mid][cols], cols contiguous and mid rows adjacent, box = box_cols x box_mid x box_outer.
 bool make_tmap_2d(CUtensorMap* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows);
+//   view: any of up to five dims, innermost first, strides of dims 1 .. in elements.
+bool make_tmap_view(CUtensorMap* m, void* base, int rank, const uint64_t* dims, const uint64_t* stride_elems, const uint32_t* box);
 //   4-D, float32, for stores: dims and box innermost first, box[0] = 16 or 32 columns (swizzled by the row length).
 bool make_tmap_4d_f32(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]);
 bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint64_t cols, uint32_t box_cols, uint32_t box_mid,
@@ -301,7 +304,8 @@ inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 //        - skinny_gemm_sm100_kernel, the weights: the first launch of a layer step or matmul is cast_bf16_kernel, the
 //          second GEMM of a layer follows it, a plain absorb launch, or a cast of its own;
 //        - mla_prep_kernel with weights_ready, W_UK: only behind the projections of the same call (do_mla_layer);
-//        - mla_merge_vup_mma_kernel, mla_merge_vup_sm100_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.
+//        - mla_vup_pieces_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.  (It also reads part_ml there,
+//          whatever it holds, and makes no use of it: mla_proj.cu.)
 //      A new early read names its head here; a new launch in front of one of these keeps a head between.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(bool chained, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

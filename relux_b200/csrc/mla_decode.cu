@@ -19,7 +19,7 @@
 namespace relux {
 
 int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
-                                TimeStamp time);
+                                int form, TimeStamp time);
 bool mla_sm100_eligible(const Pool* p, const relux_attn_args& a);
 int mla_sm100_workers(Pool* p, int q_tokens);
 bool mla_proj_mma_eligible(int Dh, int dC);
@@ -28,8 +28,8 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained);
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
                               int rows, int H, int dC, int dHR, int32_t* status);
-int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
-                                 void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
+int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, int form, bool natural, const uint16_t* W_UV,
+                              void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
 
 namespace {
 
@@ -115,7 +115,8 @@ struct MlaGenParams {
   const uint16_t* base;
   const uint16_t* q_abs;
   float scale_log2;
-  float* part_o;
+  const int32_t* halves;   // chunk_off where partial rows are two bf16 halves for the up-projection (mla_vup_pieces_kernel), else nullptr
+  void* part_o;
   float* part_ml;
   int32_t rows_total;
   int32_t* status;
@@ -213,17 +214,28 @@ __global__ void __launch_bounds__(256) mla_decode_generic_kernel(const MlaGenPar
   for (int r = 0; r < kRpw; r++) {
     const int grow = row_base + warp * kRpw + r;
     if (grow >= prm.rows_total) continue;
-    const size_t prow = (size_t)blockIdx.x * prm.rows_total + grow;
+    size_t prow = (size_t)blockIdx.x * prm.rows_total + grow;
+    if (prm.halves) {
+      const int first = prm.halves[item.seq_index], n = prm.halves[item.seq_index + 1] - first, q = grow / prm.H;
+      prow = ((size_t)first * prm.S + (size_t)q * n + ((int)blockIdx.x - first)) * prm.H + (grow - q * prm.H);
+    }
 #pragma unroll
     for (int i = 0; i < kPerLane / 2; i++) {
-      float2 v = make_float2(o[r][2 * i], o[r][2 * i + 1]);
-      *reinterpret_cast<float2*>(prm.part_o + prow * DC + 2 * (lane + 32 * i)) = v;
+      const float x = o[r][2 * i], y = o[r][2 * i + 1];
+      if (prm.halves) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(prm.part_o) + prow * DC + lane + 32 * i;   // [DC hi | DC lo], infinite less infinite is no number
+        dst[0] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+        dst[DC / 2] = round_bf16x2(isinf(x) ? 0.f : x - bf16_hi(__float_as_uint(x)), isinf(y) ? 0.f : y - bf16_hi(__float_as_uint(y)));
+      } else {
+        *reinterpret_cast<float2*>(reinterpret_cast<float*>(prm.part_o) + prow * DC + 2 * (lane + 32 * i)) = make_float2(x, y);
+      }
     }
     if (lane == 0) {
       prm.part_ml[prow * 2] = m_run[r];
       prm.part_ml[prow * 2 + 1] = l_run[r];
     }
   }
+  if (prm.halves) fence_chained_writes();
 }
 
 template <int DC>
@@ -355,11 +367,18 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));
     if (rc) return rc;
   }
+  // rows of one piece each are rounded where they are written
+  const bool split = !sm100 || plan.num_items > sb.n_seqs || [&] {
+    for (int i = 0; i < sb.n_seqs; i++)
+      if (plan.first[i + 1] - plan.first[i] > 1) return true;
+    return false;
+  }();
+  const int form = !proj_mma ? kPartialFloat32 : split ? kPartialHalves : kPartialOne;
   // the decode kernel is timed on every call, or on every Nth (RELUX_TUNE_KERNEL_TIMING_STRIDE)
   const int stride = std::max(1, p->tune.get(RELUX_TUNE_KERNEL_TIMING_STRIDE));
   const bool timed = (p->attn_calls++ % (uint64_t)stride) == 0;
   if (sm100) {
-    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p,
+    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p, form,
                                  timed ? time_stamp_next(p, p->attn_times) : TimeStamp{nullptr, nullptr});
     if (rc) return rc;
   } else {
@@ -380,7 +399,8 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     k.base = p->storage + (size_t)a.layer * p->layer_elems;
     k.q_abs = (const uint16_t*)p->q_abs.p;
     k.scale_log2 = a.scale * 1.4426950408889634f;
-    k.part_o = (float*)p->part_o.p;
+    k.halves = proj_mma ? plan.chunk_off : nullptr;
+    k.part_o = p->part_o.p;
     k.part_ml = (float*)p->part_ml.p;
     k.rows_total = rows_total;
     k.status = p->d_status;
@@ -395,9 +415,9 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   }
   count_launch(p->dev);
   if (proj_mma) {
-    // split-KV merge fused into the up-projection: the merged latent output never touches HBM
-    rc = launch_mla_merge_vup_mma(p->dev, (const float*)p->part_o.p, (const float*)p->part_ml.p, plan.chunk_off, (const uint16_t*)a.w_uv,
-                                  d_out, out_bf16, rows, S, H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
+    // the split-KV merge is part of the up-projection: the merged latent output never touches memory
+    rc = launch_mla_vup_pieces(p->dev, p->part_o.p, (const float*)p->part_ml.p, plan, form, !sm100, (const uint16_t*)a.w_uv, d_out, out_bf16, rows, S,
+                               H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
     if (rc) return rc;
   } else {
     rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, (float*)p->o_lat.p);

@@ -59,6 +59,7 @@ constexpr int kKGroups = 3, kKPerGroup = kNumKB / kKGroups;  // K slots are arme
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemO = 0, kTmemS = 256;          // O: 2 x 128 columns; S: 2 buffers x 64 columns
 constexpr float kRescaleThreshold = 8.0f;             // log2 units: rescale O only when the max grew by > 2^8
+constexpr int kPrefetchTiles = 2;                     // of a worker's end, before which it asks for its share of W_UV
 constexpr int kMaxInterleavedQ = 8;                   // up to this many query tokens work side by side on one range
 
 struct Bars {
@@ -83,9 +84,11 @@ struct MlaSm100Params {
                                       // (finite values, computed and thrown away; rows past the end of q~ are zero-filled by TMA)
   int32_t layer_row0;
   float scale_log2;
-  float* part_o;
+  int32_t form;                       // of the partial rows (PartialForm)
+  void* part_o;
   float* part_ml;
-  int32_t rows_total;
+  const uint8_t* w_uv;                // brought into L2 while the last tiles run, w_uv_each bytes a CTA (0: they will be there)
+  uint32_t w_uv_bytes, w_uv_each;
   int32_t* status;
   TimeStamp time;
 };
@@ -112,7 +115,7 @@ __device__ __forceinline__ StreamItem load_item(const StreamItem* p) {
   const int4 b = load_chained(reinterpret_cast<const int4*>(p) + 1);
   StreamItem it;
   it.seq_index = a.x; it.seq = a.y; it.page_begin = a.z; it.page_end = a.w;
-  it.tokens = b.x; it.pad[0] = it.pad[1] = it.pad[2] = 0;
+  it.tokens = b.x; it.first = b.y; it.n = b.z; it.pad = 0;
   return it;
 }
 
@@ -122,9 +125,102 @@ struct PageWin {
   int32_t cur, nxt, blk;
 };
 
+// The partial result of a warp: its 32 rows (heads) x 256 of the 512 latent columns of O, in eight chunks of 16 rows x 64 columns.  The
+// 16x256b loads give four lanes a row.  What a row is, kForm says.  The bf16 forms are operands of the up-projection: every 32 columns in
+// the order in which a lane holds them, column 8 i + 2 q + e at place 8 q + 2 i + e (mla_vup_pieces_kernel loads W_UV's rows in that
+// order), and a chunk passes through 4 KB of the P tile that belong to the warp, so that its stores are whole lines and no warp waits for
+// another.  Two halves (hi = the upper 16 bits of x, lo = bf16(x - hi), which is off by less than 2^-16 of x) where rows have several
+// pieces; where every row has one, what would be rounded to bf16 behind the merge is rounded here.  merge_splits_kernel reads float32.
+// Bound: an SM writes 32 bytes a clock, whether by stores of whole lines (128 KB in 4.0 k clocks, one CTA or all) or by TMA (4.3-5.2 k);
+// stores of 64 bytes a row take twice as long, and so did 64 TMA stores of 2 KB.  An
+// item takes 3.1 us as two halves, as it did in float32, and 1.8 in one.
+template <int kForm>
+__device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, void* part_o, int H, int piece, int head0, float m_used, bool ok) {
+  constexpr int kRowElems = kForm == kPartialOne ? kDC : 2 * kDC;   // bf16 forms
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+  // The partial results (256 KB an item at 128 heads: 17 MB in 64 pieces, 36 MB in 138 items of ranges) wait for the merge while cached
+  // rows stream through L2, and came back from HBM: stored to be evicted last, a step of 64 x 4096 takes 89.2 us instead of 90.5, 40 x
+  // <= 2500 45.2 instead of 46.2, 20 x 16000 94.5 instead of 95.8; shorter ones the same.  They stay while the pool is in use: a program's
+  // own pass over 96 MB behind a step of 64 x 1000 then takes 40 us instead of 37.5 (48 MB: no difference), and no less with a merge that
+  // reads them to be evicted first, which itself takes 1 us longer.  (Cached rows loaded to be evicted first were gone before their second
+  // load, as values: 114 -> 127 us.)
+  const uint64_t policy = make_evict_last_policy();
+  uint8_t* stage = smem + kSmemP + warp * 4096;
+  // two rows of 64 bytes to every eight lanes that write, one of 128 to every eight that read: no bank twice either way
+  auto place = [](int row, int chunk16) { return (uint32_t)(row * 128 + ((chunk16 ^ ((row & 1) << 2 | (row >> 1 & 3))) << 4)); };
+  uint32_t v[32];
+  auto load = [&](int u) { tmem_ld_16x256b_x8(tmem_o + ((uint32_t)(warp * 32 + (u >> 2) * 16) << 16) + (u & 3) * 64, v); };
+  load(0);
+#pragma unroll 1
+  for (int u = 0; u < 8; u++) {   // 4 * (half of the rows) + 64-column chunk
+    tmem_ld_wait_for(v);
+    const int dim = 128 * (warp >> 1) + 256 * ((u & 3) >> 1) + 64 * (u & 1);
+    const int head = head0 + (warp & 1) * 32 + (u >> 2) * 16;   // the chunk's first
+    if constexpr (kForm == kPartialFloat32) {
+      const int r32 = (u >> 2) * 16 + (lane >> 2);              // of the warp's 32 rows, the first of this lane's two
+      const bool seen[2] = {ok && __shfl_sync(0xffffffffu, m_used, r32) != -INFINITY,   // a row without a visible key is zero
+                            ok && __shfl_sync(0xffffffffu, m_used, r32 + 8) != -INFINITY};
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int r = head + (lane >> 2) + 8 * k;
+        if (r >= H) continue;
+        float* dst = reinterpret_cast<float*>(part_o) + ((size_t)piece * H + r) * kDC + dim + 2 * q;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          *reinterpret_cast<uint2*>(dst + 8 * i) = seen[k] ? make_uint2(v[4 * i + 2 * k], v[4 * i + 2 * k + 1]) : make_uint2(0u, 0u);
+      }
+      if (u < 7) load(u + 1);
+    } else {
+      // A row without a visible key may hold anything: the up-projection leaves it out by its maximum.
+      uint32_t hi[16], lo[16];   // [row of two][32 columns of two][4]
+      float big[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int w = 0; w < 16; w++) {
+        const uint32_t x = v[4 * (w & 7) + 2 * (w >> 3)], y = v[4 * (w & 7) + 2 * (w >> 3) + 1];
+        if constexpr (kForm == kPartialOne) {
+          hi[w] = round_bf16x2(__uint_as_float(x), __uint_as_float(y));
+        } else {
+          hi[w] = __byte_perm(x, y, 0x7632);
+          lo[w] = round_bf16x2(__uint_as_float(x) - bf16_hi(x), __uint_as_float(y) - bf16_hi(y));
+          big[w & 3] = max3(big[w & 3], fabsf(__uint_as_float(x)), fabsf(__uint_as_float(y)));
+        }
+      }
+      if (kForm == kPartialHalves && fmaxf(fmaxf(big[0], big[1]), fmaxf(big[2], big[3])) == INFINITY) {   // infinite less infinite is no number
+#pragma unroll
+        for (int w = 0; w < 16; w++) lo[w] &= ((hi[w] & 0x7fffu) == 0x7f80u ? 0u : 0xffffu) | ((hi[w] & 0x7fff0000u) == 0x7f800000u ? 0u : 0xffff0000u);
+      }
+      if (u < 7) load(u + 1);   // under the stores of this one
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint32_t at = place((lane >> 2) + 8 * k, 4 * h + q);
+          const int w = 8 * k + 4 * h;
+          *reinterpret_cast<uint4*>(stage + at) = make_uint4(hi[w], hi[w + 1], hi[w + 2], hi[w + 3]);
+          if constexpr (kForm == kPartialHalves) *reinterpret_cast<uint4*>(stage + 2048 + at) = make_uint4(lo[w], lo[w + 1], lo[w + 2], lo[w + 3]);
+        }
+      __syncwarp();
+      uint16_t* dst = reinterpret_cast<uint16_t*>(part_o) + ((size_t)piece * H + head + (lane >> 3)) * kRowElems + dim + (lane & 7) * 8;
+      uint4 a[4], b[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {   // eight lanes a row
+        a[k] = *reinterpret_cast<const uint4*>(stage + place(4 * k + (lane >> 3), lane & 7));
+        if constexpr (kForm == kPartialHalves) b[k] = *reinterpret_cast<const uint4*>(stage + 2048 + place(4 * k + (lane >> 3), lane & 7));
+      }
+      __syncwarp();   // before the next chunk
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (head + 4 * k + (lane >> 3) < H) {
+          store_hint(dst + (size_t)(4 * k) * kRowElems, a[k], policy);
+          if constexpr (kForm == kPartialHalves) store_hint(dst + (size_t)(4 * k) * kRowElems + kDC, b[k], policy);
+        }
+    }
+  }
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
-    mla_decode_sm100_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid_constant__ CUtensorMap tmap_q,
-                            const MlaSm100Params prm) {
+    mla_decode_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_q,
+                            const __grid_constant__ MlaSm100Params prm) {
   extern __shared__ __align__(1024) uint8_t smem[];
   Bars* bars = reinterpret_cast<Bars*>(smem + kSmemBar);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -149,7 +245,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     mbar_init(&bars->q_full, 1);
     bars->abort_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tmap_kv);
+    tma_prefetch_desc(&tmap_k);
+    tma_prefetch_desc(&tmap_v);
     tma_prefetch_desc(&tmap_q);
   }
   if (warp == 0) {
@@ -190,8 +287,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       const int qrow = (it.seq_index * prm.S + sq) * prm.H + 64 * (int)rank;   // Q~ rows of this CTA's 64 heads
       if (el) {
         if (rank == 0) mbar_expect_tx(&bars->q_full, 2 * kNumKB * kBlk);
-#pragma unroll
-        for (int db = 0; db < kNumKB; db++) tma_load_2d_2sm(smem + kSmemQ + db * kBlk, &tmap_q, db * 64, qrow, lead_q);
+        for (int grp = 0; grp < kKGroups; grp++) tma_load_3d_2sm(smem + kSmemQ + grp * kKPerGroup * kBlk, &tmap_q, 0, qrow, grp * kKPerGroup, lead_q);
       }
       __syncwarp();
     };
@@ -203,11 +299,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         const uint32_t lead = mapa_u32(smem_u32(&bars->k_full[grp]), 0);
         if (el) {
           if (rank == 0) mbar_expect_tx(&bars->k_full[grp], 2 * kKPerGroup * kBlk);
-#pragma unroll
-          for (int j = 0; j < kKPerGroup; j++) {
-            const int db = grp * kKPerGroup + j;
-            tma_load_2d_2sm(smem + kSmemK + db * kBlk, &tmap_kv, 0, y + db * kPage, lead);
-          }
+          tma_load_2d_2sm(smem + kSmemK + grp * kKPerGroup * kBlk, &tmap_k, 0, y + grp * kKPerGroup * kPage, lead);
         }
         __syncwarp();
       }
@@ -223,8 +315,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         const int blk0 = 4 * nb + 2 * (int)rank;   // this CTA's 128 output dims of block nb = column blocks blk0, blk0 + 1
         if (el) {
           if (rank == 0) mbar_expect_tx(&bars->v_full[u], 4 * kBlk);
-          tma_load_2d_2sm(smem + kSmemV + u * 2 * kBlk, &tmap_kv, 0, y + blk0 * kPage, lead);
-          tma_load_2d_2sm(smem + kSmemV + u * 2 * kBlk + kBlk, &tmap_kv, 0, y + (blk0 + 1) * kPage, lead);
+          tma_load_2d_2sm(smem + kSmemV + u * 2 * kBlk, &tmap_v, 0, y + blk0 * kPage, lead);
         }
         __syncwarp();
       }
@@ -250,6 +341,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       const int npages = cur.page_end - cur.page_begin;
       const int ntiles = (npages + 1) >> 1;
       for (int i = 0; i < ntiles; i++, g++) {
+        if (!has_next && i == max(0, ntiles - kPrefetchTiles) && prm.w_uv_each > 0) {
+          const uint32_t first = (blockIdx.y * gridDim.x + blockIdx.x) * prm.w_uv_each;
+          if (el && first < prm.w_uv_bytes) prefetch_l2(prm.w_uv + first, min(prm.w_uv_each, prm.w_uv_bytes - first));
+          __syncwarp();
+        }
         if (i + 1 < ntiles) {
           load_k(w, i + 1, g + 1);
         } else if (has_next) {
@@ -350,13 +446,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     const int hf = L >> 6;            // token half of the tile (= which CTA's page)
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full), 0);
-    // The partial results (256 KB an item at 128 heads: 17 MB in 64 pieces, 36 MB in 138 items of ranges) wait for the merge while cached
-    // rows stream through L2, and came back from HBM: stored to be evicted last, a step of 64 x 4096 takes 89.2 us instead of 90.5, 40 x
-    // <= 2500 45.2 instead of 46.2, 20 x 16000 94.5 instead of 95.8; shorter ones the same.  They stay while the pool is in use: a program's
-    // own pass over 96 MB behind a step of 64 x 1000 then takes 40 us instead of 37.5 (48 MB: no difference), and no less with a merge that
-    // reads them to be evicted first, which itself takes 1 us longer.  (Cached rows loaded to be evicted first were gone before their second
-    // load, as values: 114 -> 127 us.)
-    const uint64_t evict_last = make_evict_last_policy();
     StreamItem cur = load_item(prm.items + it0);
     int g = 0;
     for (int it = it0; it < it1; ++it) {
@@ -460,45 +549,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       if (hf == 1) bars->lsum[row] = l_run;
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const bool real_head = 64 * (int)rank + row < prm.H;   // padding rows of the tile are not written
-      const size_t prow = (size_t)it * prm.rows_total + (size_t)sq * prm.H + 64 * rank + row;
+      // the pieces of a row lie one behind another where the up-projection reads them, item by item where merge_splits_kernel does
+      const int piece = prm.form != kPartialFloat32 ? cur.first * prm.S + sq * cur.n + (it - cur.first) : it * prm.S + sq;
       if (hf == 0 && real_head) {
+        const size_t prow = (size_t)piece * prm.H + 64 * rank + row;
         prm.part_ml[prow * 2] = ok ? m_used : -INFINITY;
         prm.part_ml[prow * 2 + 1] = ok ? (l_run + bars->lsum[row]) : 0.f;
       }
-      // O leaves through the P tile (free between the item's last PV and the next item's first softmax): a thread holds
-      // one row, so stores straight from its registers put 32 rows into every instruction (6-8 us per item, measured);
-      // staged, 8 lanes write one 128-byte segment of a row.  16-byte chunks are swizzled by the row on both sides.
-      float* obase = prm.part_o + ((size_t)it * prm.rows_total + (size_t)sq * prm.H + 64 * rank) * kDC;   // this CTA's row 0
-      const int heads_here = prm.H - 64 * (int)rank;   // rows [0, heads_here) are real heads
-      uint8_t* stage = smem + kSmemP;
-#pragma unroll 1
-      for (int nb = 0; nb < 2; nb++)
-#pragma unroll 1
-        for (int c = 0; c < 128; c += 32) {
-          uint32_t ov[32];
-          tmem_ld_32x32b_x32(tmem + lane_addr + kTmemO + nb * 128 + c, ov);
-          tmem_ld_wait();
-          if (!ok || m_used == -INFINITY) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) ov[j] = 0u;
-          }
-          uint8_t* srow = stage + (row * 2 + hf) * 128;   // segment (row, hf): columns 256 nb + 128 hf + c .. + 31
-#pragma unroll
-          for (int j = 0; j < 8; j++)
-            *reinterpret_cast<uint4*>(srow + ((j ^ (row & 7)) << 4)) = make_uint4(ov[4 * j], ov[4 * j + 1], ov[4 * j + 2], ov[4 * j + 3]);
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-          for (int k = 0; k < 8; k++) {
-            const int seg = k * 16 + (L >> 3), r = seg >> 1, h2 = seg & 1, j = L & 7;
-            const uint4 v = *reinterpret_cast<const uint4*>(stage + seg * 128 + ((j ^ (r & 7)) << 4));
-            if (r < heads_here) store_hint(obase + (size_t)r * kDC + 256 * nb + 128 * h2 + c + 4 * j, v, evict_last);
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
+      if (64 * (int)rank + 32 * (warp & 1) >= prm.H) {   // none of the warp's rows is a head
+      } else if (prm.form == kPartialHalves) write_partial<kPartialHalves>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, ok);
+      else if (prm.form == kPartialOne) write_partial<kPartialOne>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, ok);
+      else write_partial<kPartialFloat32>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, ok);
       tc_fence_before();   // the O read-out is ordered before this thread's next p_full arrival, which releases the first PV of the next item
       cur = nxt;
     }
   }
+  if (warp < 4) fence_chained_writes();   // the up-projection reads the partial rows by TMA
   tc_fence_before();
   cluster_sync_relaxed();   // nothing is handed over: the pair's barriers and tensor memory outlive what the other CTA does with them
   if (threadIdx.x == 0 && it0 < it1) stamp_end(prm.time);
@@ -552,11 +618,13 @@ int mla_sm100_workers(Pool* p, int q_tokens) {
 }
 
 int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
-                                TimeStamp time) {
+                                int form, TimeStamp time) {
   const relux_pool_params& prm = p->prm;
   if (plan.num_items == 0) return RELUX_OK;   // every sequence is empty: the merge writes zeros
-  CUtensorMap tq;   // the absorbed queries [rows][576], 64 x 64 boxes
-  if (!make_tmap_2d(&tq, (void*)q_abs, (uint64_t)sb.n_seqs * a.q_tokens * a.num_heads, kRow, 64, 64)) {
+  CUtensorMap tq;   // the absorbed queries [rows][576] in boxes of three blocks of 64 columns x 64 rows
+  const uint64_t q_dims[3] = {64, (uint64_t)sb.n_seqs * a.q_tokens * a.num_heads, kNumKB}, q_strides[2] = {kRow, 64};
+  const uint32_t q_box[3] = {64, 64, kKPerGroup};
+  if (!make_tmap_view(&tq, (void*)q_abs, 3, q_dims, q_strides, q_box)) {
     set_error("tensor map for the absorbed queries could not be encoded");
     return RELUX_ERR_CUDA;
   }
@@ -572,16 +640,23 @@ int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_ar
   k.causal = a.causal;
   k.layer_row0 = (int32_t)((int64_t)a.layer * prm.num_pages * kNumKB * kPage);
   k.scale_log2 = a.scale * 1.4426950408889634f;
-  k.part_o = (float*)p->part_o.p;
+  k.form = form;
+  k.part_o = p->part_o.p;
   k.part_ml = (float*)p->part_ml.p;
-  k.rows_total = a.q_tokens * a.num_heads;
   k.H = a.num_heads;
   k.status = p->d_status;
   k.time = time;
+  // Cached rows of more than half of L2 have pushed the weights of the next launch out of it.
+  int64_t cached = 0;
+  for (int i = 0; i < sb.n_seqs; i++) cached += (int64_t)p->h_len[(size_t)a.layer * prm.max_seqs + sb.seq[i]] * kRow * 2;
+  const uint32_t ctas = 2 * plan.num_workers * sx * (a.q_tokens / sx);
+  k.w_uv = (const uint8_t*)a.w_uv;
+  k.w_uv_bytes = (uint32_t)kDC * a.num_heads * a.head_dim * 2;
+  k.w_uv_each = form != kPartialFloat32 && cached > kResidentBytes ? ((k.w_uv_bytes + ctas - 1) / ctas + 127) / 128 * 128 : 0;
   if (int32_t rc = allow_smem(p->dev, mla_decode_sm100_kernel, kSmemTotal)) return rc;
   dim3 grid(2 * plan.num_workers * sx, a.q_tokens / sx);
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, mla_decode_sm100_kernel, grid, dim3(192), (size_t)kSmemTotal,
-                                p->dev->stream, p->tmap_mla, tq, k));
+                                p->dev->stream, p->tmap_mla_3, p->tmap_mla_2, tq, k));
   time_stamp_done(p->attn_times, time);
   return RELUX_OK;
 }

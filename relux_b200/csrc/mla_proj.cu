@@ -1,17 +1,18 @@
-// The two small per-head GEMMs around the absorbed MLA decode, on tensor cores (mma.sync m16n8k16, bf16 in,
-// f32 accumulate):
-//   absorb:  q~[row][h][0:dC]  = q_nope[row][h][:] . W_UK[:, h*Dh:(h+1)*Dh]^T      M = rows, N = dC,  K = Dh
+// The two small per-head GEMMs around the absorbed MLA decode, on tensor cores, bf16 in, f32 accumulate:
+//   absorb:  q~[row][h][0:dC]  = q_nope[row][h][:] . W_UK[:, h*Dh:(h+1)*Dh]^T      M = rows, N = dC,  K = Dh      (mma.sync m16n8k16)
 //            q~[row][h][dC: ]  = q_rope[row][h][:]
-//   up-proj: out[row][h][:]    = O_lat[row][h][:] . W_UV[:, h*Dh:(h+1)*Dh]          M = rows, N = Dh,  K = dC
-// Both are about 1 GFLOP per step at batch 64 (1.5 % of the decode's work) and move ~30 MB; they are written to stay
-// out of the way of the decode kernel, not to chase the tensor peak: one CTA per (head, 128-wide slice, 64 rows),
-// operands staged in shared memory by a few TMA boxes (every load of a CTA in flight at once), fragments through
-// ldmatrix (the up-projection of more than 16 rows runs on tcgen05).  The up-projection also performs the split-KV merge while it
-// builds its operand.
+//   up-proj: out[row][h][:]    = O_lat[row][h][:] . W_UV[:, h*Dh:(h+1)*Dh]          M = Dh, N = pieces of rows, K = dC   (tcgen05)
+// Both are about 1 GFLOP per step at batch 64 (1.5 % of the decode's work) and move ~30 MB; they are written to stay out of the way of
+// the decode kernel, not to chase the tensor peak.  The absorb has one CTA per (head, 128-wide slice, 64 rows), operands staged in shared
+// memory by a few TMA boxes (every load of a CTA in flight at once), fragments through ldmatrix.  The up-projection is also the split-KV
+// merge: it multiplies every piece and adds the products up.
 // Shapes: Dh = 128, dC a multiple of 128.  Other shapes use the scalar kernels in mla_decode.cu.
 #include "common.cuh"
+#include <algorithm>
+
 #include "internal.h"
 #include "prep_parts.cuh"
+#include "splitkv.h"
 #include "umma.cuh"
 
 namespace relux {
@@ -20,8 +21,6 @@ namespace {
 
 constexpr int kDh = 128;
 constexpr int kStride = kDh + 8;  // bf16 elements per shared-memory row (272 B: conflict-free ldmatrix)
-constexpr int kMergeBlk = 8192;   // 64 rows x 64 columns of the merged operand
-constexpr int kMaxChunks = 4;     // the fused merge + up-projection keeps at most 4 x 128 latent columns in shared memory
 
 // 64 rows x 128 latent columns of the absorb for one head, by 128 threads.  W_UK's tile [128 c][128 d] and (bf16) the query
 // tile [64 rows][128 d] come as four TMA boxes from one thread: as 3072 cp.async of 16 bytes they took 2.2 us to issue.  Both
@@ -161,401 +160,243 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ C
   prep_arrive_and_advance(ap, (uint32_t)ap.n_seqs + 1u);
 }
 
-// 16 rows x 16 columns of a warp, over one 128-wide k chunk: A rows at As (kStride), B [128 k][128 n] at Bs as two 64-column
-// blocks with the 128-byte swizzle (n contiguous -> ldmatrix.trans).
-__device__ __forceinline__ void tile_mma_16x16(const uint16_t* As, uint32_t Bs, float (&acc)[2][4], int col0, int lane) {
-  const int m = lane >> 3;
-#pragma unroll
-  for (int ks = 0; ks < 8; ks++) {
-    uint32_t a[4];
-    ldmatrix_x4(a[0], a[1], a[2], a[3], smem_u32(As + ((m & 1) * 8 + (lane & 7)) * kStride + ks * 16 + (m >> 1) * 8));
-    const int krow = ks * 16 + (m & 1) * 8 + (lane & 7);
-    const int col = col0 + (m >> 1) * 8;
-    uint32_t b0, b1, b2, b3;
-    ldmatrix_x4_trans(b0, b1, b2, b3, Bs + (col >> 6) * 16384 + swz128(krow, (col & 63) >> 3));
-    mma_bf16_16816(acc[0], a, b0, b1);
-    mma_bf16_16816(acc[1], a, b2, b3);
-  }
+// Value up-projection of the split-KV partial results, and their sum.  For one head, with the pieces of a row (a sequence's query
+// token) as columns,
+//   D[128 output dims][column] = W_UV^T hi + W_UV^T lo      on tcgen05, W_UV's rows as the M = 128 operand as they lie (MN-major)
+//   out[row] = sum over the row's columns of 2^(m - M) / L * D[:, column]
+// part [piece][H][2 dC]: two bf16 halves of the unnormalised float32 partial (write_partial, mla_decode_generic_kernel), part_ml
+// [piece][H][2] = (max in the log2 domain, sum); the pieces of row (i, q) are [first_i S + q n_i, + n_i), first_i = chunk_off[i], n_i =
+// chunk_off[i + 1] - first_i, so that the columns of neighbouring rows are neighbours.
+// What is summed is 128 float32 outputs a piece instead of 512 latent columns, behind the contraction instead of before it: nothing but TMA
+// touches the partials (2 KB a piece and head), no row is rounded to bf16, and the row's weights are worked out meanwhile.  Adding the
+// partials up first, by ordinary loads, took 15-16 k clocks of a launch at 64 rows of one piece (128 KB a CTA: every row a chain of round
+// trips), rounded the sum to bf16 (the largest part of a latent step's error: 1.7e-3 of 2.4e-3), and multiplied by 3.2 k clocks of MMAs.
+// From the wait to the last output, before -> now, three inputs in turn: 64 x 4096, a piece a row 12.4 -> 4.9 us; 16 x <= 32k, 90 pieces 8.0
+// -> 7.2; 3 x <= 1500, 27 pieces 4.1 -> 3.5; one sequence 3.8 -> 2.4.  Bound: with many pieces what the partials take from L2 (35 bytes a clock
+// and SM), else the round trips of a stage, of 32 MMAs (1.5 k clocks) and of the outputs.
+// An MMA of up to 64 columns takes 40-48 clocks for its 4 KB of weights, so the halves of a block of columns stand side by side as N and the
+// weights are read once for both: 32 MMAs a block.  Rows of one piece each come rounded to bf16 where they were written, without a lo.
+// A launch finds its instructions in no cache, and what is executed once is waited for: clock stamps had 2 k clocks between the wait and the
+// first MMA, 2.4 k for the first outputs, 4 k for the weights of three rows.  So the loops are rolled, and the warps that have nothing to do
+// before the wait go through theirs once, on whatever memory holds, without storing.
+// W_UV's slice of the head (dC x 128 bf16) is fetched by one thread as TMA boxes before chain_wait(): the weights do not depend on the
+// decode kernel, and the launches before it have waited for everything older.
+// grid (H, groups of rows), 512 threads: warp 0 loads, warp 1 issues the MMAs, the others work out the weights, all but those write the outputs.
+constexpr int kVupWarps = 16;
+constexpr int kVupMaxCols = 240;                  // columns of a CTA: two of the 512 tensor-memory columns each, in whole blocks
+constexpr int kVupListed = 256;                   // sequences whose first pieces travel as arguments
+constexpr int kVupRing = 96 << 10, kVupMaxStages = 8;
+static_assert(kVupMaxCols >= kMaxRowItems, "a row's pieces are columns of one CTA");
+struct VupParams {
+  const float* part_ml;
+  const int32_t* chunk_off;
+  void* out;
+  int32_t rows, S, H, nk;
+  int32_t rows_each;                          // rows of a group (the last may have fewer)
+  int32_t halves, n_block, n_kb, n_stages;    // a stage: n_kb times 64 latent columns of n_block columns, [n_kb][hi | lo][n_block][64], one TMA box
+  int32_t tmem_cols;
+  int32_t warm;                               // there are partial results: part_ml may be read, whatever it holds
+  int32_t listed;                             // `first` holds chunk_off
+  int32_t* status;
+  uint16_t first[kVupListed + 1];
+};
+struct VupShared {
+  uint64_t w_full[2], full[kVupMaxStages], empty[kVupMaxStages], done;
+  uint32_t tmem_slot;
+  float4 info[(kVupMaxCols + 16) / 2];        // of a column: first (max, sum), then its weight and, at a row's last, the row's place in `out` (else -1)
+};
+static_assert(131072 + kVupRing + sizeof(VupShared) <= 232448, "more shared memory than a CTA may use");
+
+// Bounded, and out of line: around a loop of its own the issuing warp's operands leave their uniform registers.
+__device__ __noinline__ void vup_wait_slow(uint64_t* bar, uint32_t parity, int32_t* status) {
+  if (!mbar_wait(bar, parity)) set_status(status, RELUX_ERR_TIMEOUT);
+}
+__device__ __forceinline__ void vup_wait(uint64_t* bar, uint32_t parity, int32_t* status) {
+  if (!mbar_try_wait(bar, parity)) vup_wait_slow(bar, parity, status);
+  __syncwarp();
 }
 
-// Merges the split-KV partials of the tile's rows into the bf16 A operand, one warp per row at a time: a lane owns the
-// same 4 of every 128 latent columns, so every load instruction of a warp is 512 contiguous bytes of one partial row
-// (four threads per row with 128 bytes each, the first layout, put 32 different cache lines into every load
-// instruction: the kernel spent most of its time in the load unit's address stage).  The weights of a row's items come
-// from one round trip: lane j reads (max, sum) of item j, the warp reduces.
-// kChunks: 128-column chunks of a warp, 4 / kChunks warps share a row; 16 / kChunks items are in flight per lane.  A call of
-// up to four rows has more warps than rows, and its rows the most items (each worker holds a piece of some sequence).
-// Rows past the batch are zero rows of the MMA tile.  The pointers have come through behind_wait().
-constexpr int kMergeWarps = 16;
-template <int kChunks>
-__device__ __forceinline__ void merge_rows_warp(uint16_t* As, const float* part_o, const float* part_ml, const int32_t* chunk_off,
-                                                int rows, int S, int H, int h, int dC, int nk_all, int rows_total) {
-  constexpr int kParts = kMaxChunks / kChunks, kItems = 16 / kChunks, kRowStep = kMergeWarps / kParts;
-  const int warp = (int)(threadIdx.x >> 5) / kParts, lane = threadIdx.x & 31;   // the warp's first row of the tile
-  const int k0 = (int)(threadIdx.x >> 5) % kParts * kChunks, nk = min(kChunks, nk_all - k0);
-  if (nk <= 0) return;
-  part_o += k0 * 128;
-  As += (size_t)k0 * 16 * kStride;
-  // The item range of a row is the first of two dependent round trips to L2, so it is requested one row ahead.
-  int c0_next = 0, c1_next = 0;
-  if (warp < rows) {
-    const int i = warp / S;
-    c0_next = load_settled(chunk_off + i);
-    c1_next = load_settled(chunk_off + i + 1);
-  }
-  for (int r = warp; r < 16; r += kRowStep) {
-    const int c0 = c0_next, c1 = c1_next;
-    c0_next = c1_next = 0;
-    if (r + kRowStep < rows) {
-      const int i = (r + kRowStep) / S;
-      c0_next = load_settled(chunk_off + i);
-      c1_next = load_settled(chunk_off + i + 1);
-    }
-    float4 acc[kChunks];
-#pragma unroll
-    for (int k = 0; k < kChunks; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < rows) {
-      const size_t prow = (size_t)(r % S) * H + h;
-      // (max, sum) of this lane's item of every group of 32, and at the same time the partial rows of the first
-      // items: one memory round trip serves the common case of a sequence cut into a handful of items
-      const int n_items = c1 - c0;
-      if (n_items <= 0) goto store_row;   // no partial to merge: a zero row
-      float2 ml = make_float2(-INFINITY, 0.f);
-      if (lane < n_items) ml = load_settled(reinterpret_cast<const float2*>(part_ml + ((size_t)(c0 + lane) * rows_total + prow) * 2));
-      float4 x[kItems][kChunks];
-      const int ng0 = min(32, n_items);
-#pragma unroll
-      for (int u = 0; u < kItems; u++) {
-        // a slot past the group's last item stays zero (its weight is zero too): the load unit's data path, 128 bytes
-        // per clock for all 16 warps, is what a row's requests queue on, so no load is spent on padding
-        const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(c0 + u) * rows_total + prow) * dC) + lane;
-#pragma unroll
-        for (int k = 0; k < kChunks; k++)
-          if (k < nk) x[u][k] = load_settled_if(src + k * 32, u < ng0);
-      }
-      // global maximum and normaliser over all items of the sequence
-      float M = ml.x;
-      for (int c = c0 + 32 + lane; c < c1; c += 32) M = fmaxf(M, load_settled(part_ml + ((size_t)c * rows_total + prow) * 2));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-      float L = (ml.x != -INFINITY) ? ml.y * exp2f(ml.x - M) : 0.f;
-      for (int c = c0 + 32 + lane; c < c1; c += 32) {
-        const float2 t = load_settled(reinterpret_cast<const float2*>(part_ml + ((size_t)c * rows_total + prow) * 2));
-        if (t.x != -INFINITY) L += t.y * exp2f(t.x - M);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-      const float inv = (L > 0.f) ? 1.0f / L : 0.f;
-      for (int cb = c0; cb < c1; cb += 32) {
-        // this lane's item of the group of 32: its weight; then kItems at a time, weights by shuffle
-        float w_mine = 0.f;
-        if (cb == c0) {
-          w_mine = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M) * inv;
-        } else if (cb + lane < c1) {
-          const float m = load_settled(part_ml + ((size_t)(cb + lane) * rows_total + prow) * 2);
-          w_mine = (m == -INFINITY) ? 0.f : exp2f(m - M) * inv;
-        }
-        const int ng = min(32, c1 - cb);
-        for (int j = 0; j < ng; j += kItems) {
-          if (cb != c0 || j != 0) {   // the first items of the row are in flight already
-#pragma unroll
-            for (int u = 0; u < kItems; u++) {
-              const float4* src = reinterpret_cast<const float4*>(part_o + ((size_t)(cb + j + u) * rows_total + prow) * dC) + lane;
-#pragma unroll
-              for (int k = 0; k < kChunks; k++)
-                if (k < nk) x[u][k] = load_settled_if(src + k * 32, j + u < ng);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < kItems; u++) {
-            float w = __shfl_sync(0xffffffffu, w_mine, min(j + u, 31));
-            if (j + u >= ng) w = 0.f;
-#pragma unroll
-            for (int k = 0; k < kChunks; k++)
-              if (k < nk) {
-                acc[k].x = fmaf(x[u][k].x, w, acc[k].x);
-                acc[k].y = fmaf(x[u][k].y, w, acc[k].y);
-                acc[k].z = fmaf(x[u][k].z, w, acc[k].z);
-                acc[k].w = fmaf(x[u][k].w, w, acc[k].w);
-              }
-          }
-        }
-      }
-    }
-  store_row:
-#pragma unroll
-    for (int k = 0; k < kChunks; k++)
-      if (k < nk)
-        *reinterpret_cast<uint2*>(As + ((size_t)k * 16 + r) * kStride + lane * 4) =
-            make_uint2(pack_bf16x2(acc[k].x, acc[k].y), pack_bf16x2(acc[k].z, acc[k].w));
-  }
-}
-
-// Split-KV merge fused into the value up-projection, for up to 16 rows and one head: the A operand (the merged, normalised latent
-// output as bf16) is built straight from the per-item partials
-//   part_o [item][S * H][dC] f32 (unnormalised), part_ml [item][S * H][2] = (max in the log2 domain, sum),
-// items of sequence i = [chunk_off[i], chunk_off[i + 1]).
-// All of W_UV's slice for this head (dC x 128 bf16) is fetched by one thread as 2 * nk TMA boxes before chain_wait(): the
-// weights do not depend on the decode kernel, and the launches before it have waited for everything older (as 512 bulk
-// copies of a row each, issued behind the merge's first loads, they took 2-3 us to be accepted).  Eight warps share the MMAs, chunk by
-// chunk as the boxes land.
-// grid (H), 512 threads, row = seq_index * S + query token.  dC = 128 * nk, nk <= 4.
-__global__ void __launch_bounds__(32 * kMergeWarps) mla_merge_vup_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const float* part_o,
-                                                                const float* part_ml, const int32_t* chunk_off,
-                                                                void* __restrict__ out, int out_bf16, int rows, int S, int H, int dC,
-                                                                int32_t* __restrict__ status) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t w_full[kMaxChunks];   // chunk k of W_UV has landed (bytes counted by the TMA loads)
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int nk = dC / 128;
-  const uint32_t Bs = smem_u32(smem);                                       // [nk][2 halves of 64 columns][128][64], swizzled
-  uint16_t* As = reinterpret_cast<uint16_t*>(smem + (size_t)nk * 32768);    // [nk][16][kStride]
-  const int h = blockIdx.x;
+template <bool kOutBf16>
+__global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const __grid_constant__ CUtensorMap tmap_w,
+                                                                          const __grid_constant__ CUtensorMap tmap_p,
+                                                                          const __grid_constant__ VupParams prm) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int nk = prm.nk, H = prm.H, S = prm.S, nb = prm.n_block, blk_bytes = prm.halves * nb * 128, stage_bytes = prm.n_kb * blk_bytes;
+  uint8_t* Ws = smem;                                             // [2 halves of 64 output dims][dC latent rows][64], swizzled
+  uint8_t* ring = smem + nk * 32768;                              // [stage], swizzled
+  VupShared* sh = reinterpret_cast<VupShared*>(ring + prm.n_stages * stage_bytes);
+  float2* info = reinterpret_cast<float2*>(sh->info);
+  const int h = blockIdx.x, r0 = blockIdx.y * prm.rows_each, rows_here = min(prm.rows_each, prm.rows - r0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rows_total = S * H;
+  const int steps_each = (2 * nk + prm.n_kb - 1) / prm.n_kb;      // stages of a block of columns
   chain_release();
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_w);
-    for (int k = 0; k < nk; k++) mbar_init(&w_full[k], 1);
+    if ((smem_u32(smem) & 1023u) != 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);   // the swizzled layouts
+    mbar_init(&sh->w_full[0], 1);
+    mbar_init(&sh->w_full[1], 1);
+    for (int s = 0; s < prm.n_stages; s++) {
+      mbar_init(&sh->full[s], 1);
+      mbar_init(&sh->empty[s], 1);
+    }
+    mbar_init(&sh->done, 1);
     fence_mbar_init();
-    for (int k = 0; k < nk; k++) {
-      mbar_expect_tx(&w_full[k], 32768);
-      tma_load_2d(smem + (size_t)k * 32768, &tmap_w, h * kDh, k * 128, &w_full[k]);
-      tma_load_2d(smem + (size_t)k * 32768 + 16384, &tmap_w, h * kDh + 64, k * 128, &w_full[k]);
+    for (int k = 0; k < nk; k += 2) {   // 256 latent rows (128 where there are no more) in the order of a partial's columns
+      mbar_expect_tx(&sh->w_full[k >> 1], nk == 1 ? 32768 : 65536);
+      tma_load_5d(Ws + k * 16384, &tmap_w, h * kDh, 0, 0, 0, k * 4, &sh->w_full[k >> 1]);
+      tma_load_5d(Ws + nk * 16384 + k * 16384, &tmap_w, h * kDh + 64, 0, 0, 0, k * 4, &sh->w_full[k >> 1]);
     }
-  }
-  chain_wait();   // the partial results come from the kernel before this one
-  part_o = behind_wait(part_o);
-  part_ml = behind_wait(part_ml);
-  chunk_off = behind_wait(chunk_off);
-  if (rows <= 4) merge_rows_warp<1>(As, part_o, part_ml, chunk_off, rows, S, H, h, dC, nk, rows_total);
-  else if (rows <= 8) merge_rows_warp<2>(As, part_o, part_ml, chunk_off, rows, S, H, h, dC, nk, rows_total);
-  else merge_rows_warp<4>(As, part_o, part_ml, chunk_off, rows, S, H, h, dC, nk, rows_total);
-  float acc[2][4];
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-  __syncthreads();   // the merged A tiles are complete, and the barriers visible
-  const int col0 = warp * 16;
-  if (col0 >= kDh) return;
-  for (int k = 0; k < nk; k++) {
-    if (!mbar_wait(&w_full[k], 0)) set_status(status, RELUX_ERR_TIMEOUT);   // bounded: a copy that never lands is reported, not waited for
-    tile_mma_16x16(As + (size_t)k * 16 * kStride, Bs + k * 32768, acc, col0, lane);
-  }
-#pragma unroll
-  for (int hf = 0; hf < 2; hf++) {
-    const int r = hf * 8 + (lane >> 2);
-    if (r >= rows) continue;
-    const size_t off = ((size_t)r * H + h) * kDh + col0 + 2 * (lane & 3);
-#pragma unroll
-    for (int nt = 0; nt < 2; nt++) {
-      const float x = acc[nt][hf * 2], y = acc[nt][hf * 2 + 1];
-      if (out_bf16) *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + off + nt * 8) = pack_bf16x2(x, y);
-      else *reinterpret_cast<float2*>(reinterpret_cast<float*>(out) + off + nt * 8) = make_float2(x, y);
-    }
-  }
-  if (out_bf16) fence_chained_writes();   // a projection's operand
-}
-
-// The same for a tile of up to 64 rows, a warp a row: the item range of the warp's row is requested two rows ahead, (max, sum) of its
-// items one row ahead, and the partial rows, two items at a time, before the ones they follow are added up.  The loop over the rows
-// stays a loop: unrolled, the kernel waited for its own instructions.  Rows past rows_here are left as they are.
-__device__ __forceinline__ void merge_rows_piped(uint8_t* As, const float* part_o, const float* part_ml, const int32_t* chunk_off,
-                                                int r0, int rows_here, int S, int H, int h, int dC, int nk, int rows_total) {
-  constexpr int kChunks = kMaxChunks, kItems = 2, kRowStep = kMergeWarps;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;   // the warp's first row of the tile
-  part_o += lane * 4;
-  struct Row {
-    int c0, n;   // first item, items
-    int pr;      // row of an item's partial block
-  };
-  auto row_at = [&](int row) -> Row {   // a row past the tile has no items
-    Row r{0, 0, 0};
-    if (row < rows_here) {
-      const int i = (r0 + row) / S;
-      r.c0 = load_settled(chunk_off + i);
-      r.n = load_settled(chunk_off + i + 1);   // its end, for now
-      r.pr = (r0 + row) % S * H + h;
-    }
-    return r;
-  };
-  auto ml_of = [&](const Row& r, int j) {
-    return load_settled(reinterpret_cast<const float2*>(part_ml + ((size_t)(r.c0 + j) * rows_total + r.pr) * 2));
-  };
-  float4 x[kItems][kChunks], y[kItems][kChunks];
-  auto fetch = [&](float4 (&z)[kItems][kChunks], const Row& r, int j) {   // a slot past the row's last item stays zero: no load is spent on it
-    const float* src = part_o + ((size_t)(r.c0 + j) * rows_total + r.pr) * dC;
-#pragma unroll
-    for (int u = 0; u < kItems; u++) {
-#pragma unroll
-      for (int k = 0; k < kChunks; k++)
-        if (k < nk) z[u][k] = load_settled_if(reinterpret_cast<const float4*>(src) + k * 32, j + u < r.n);
-      src += (size_t)rows_total * dC;
-    }
-  };
-  Row cur = row_at(warp), nxt = row_at(warp + kRowStep);
-  cur.n -= cur.c0;
-  float2 ml = make_float2(-INFINITY, 0.f);
-  if (lane < cur.n) ml = ml_of(cur, lane);
-  fetch(x, cur, 0);
-#pragma unroll 1
-  for (int row = warp; row < rows_here; row += kRowStep) {
-    nxt.n -= nxt.c0;
-    float2 ml_next = make_float2(-INFINITY, 0.f);
-    if (lane < nxt.n) ml_next = ml_of(nxt, lane);
-    const Row after = row_at(row + 2 * kRowStep);
-    // weights of the row's first 32 items: 2^(m - M) / L
-    float M = ml.x;
-    for (int j = 32 + lane; j < cur.n; j += 32) M = fmaxf(M, ml_of(cur, j).x);
-    M = warp_max(M);
-    float w = (ml.x != -INFINITY) ? exp2f(ml.x - M) : 0.f;
-    float L = ml.y * w;
-    for (int j = 32 + lane; j < cur.n; j += 32) {
-      const float2 m = ml_of(cur, j);
-      if (m.x != -INFINITY) L += m.y * exp2f(m.x - M);
-    }
-    L = warp_sum(L);
-    const float inv = (L > 0.f) ? 1.0f / L : 0.f;
-    w *= inv;
-    float4 acc[kChunks];
-#pragma unroll
-    for (int k = 0; k < kChunks; k++) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int j = 0;
-#pragma unroll 1
-    do {   // a row without items adds up the zeros that fetch left
-      const bool more = j + kItems < cur.n;
-      fetch(y, more ? cur : nxt, more ? j + kItems : 0);
-      if (j > 0 && (j & 31) == 0) {
-        w = 0.f;
-        if (j + lane < cur.n) {
-          const float m = ml_of(cur, j + lane).x;
-          if (m != -INFINITY) w = exp2f(m - M) * inv;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kItems; u++) {
-        const float wu = __shfl_sync(0xffffffffu, w, (j + u) & 31);
-#pragma unroll
-        for (int k = 0; k < kChunks; k++)
-          if (k < nk) {
-            acc[k].x = fmaf(x[u][k].x, wu, acc[k].x);
-            acc[k].y = fmaf(x[u][k].y, wu, acc[k].y);
-            acc[k].z = fmaf(x[u][k].z, wu, acc[k].z);
-            acc[k].w = fmaf(x[u][k].w, wu, acc[k].w);
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < kItems; u++)
-#pragma unroll
-        for (int k = 0; k < kChunks; k++) x[u][k] = y[u][k];
-      j += kItems;
-    } while (j < cur.n);
-#pragma unroll
-    for (int k = 0; k < kChunks; k++)
-      if (k < nk)
-        *reinterpret_cast<uint2*>(As + (k * 2 + (lane >> 4)) * kMergeBlk + swz128(row, (lane & 15) >> 1) + (lane & 1) * 8) =
-            make_uint2(pack_bf16x2(acc[k].x, acc[k].y), pack_bf16x2(acc[k].z, acc[k].w));
-    cur = nxt;
-    nxt = after;
-    ml = ml_next;
-  }
-}
-
-// Split-KV merge fused into the value up-projection, for one head and up to 64 rows: the merged, normalised latent output is built as
-// bf16 straight from the per-item partials
-//   part_o [item][S * H][dC] f32 (unnormalised), part_ml [item][S * H][2] = (max in the log2 domain, sum),
-// items of sequence i = [chunk_off[i], chunk_off[i + 1]),
-// and D[128 output dims x rows] = W_UV^T O on tcgen05: the weights are the M = 128 operand as they lie (MN-major), the rows the N
-// operand (16, 32 or 64, K-major blocks of 64 columns), one tensor-memory column per row.  Rows of the tile past the batch hold
-// whatever shared memory held: their columns of D are not read.
-// Clock stamps at 64 sequences of 4096 tokens, 64 rows of one item each: merge 15-16 k, MMAs 3.2 k, of which their issue is 2.8 k, the
-// outputs 1.5 k.  (With two items a row, the plan of equal ranges: merge 15-16.5 k, 17-22 k with one row's round trips after another; MMAs
-// by mma.sync, whose fragments come from shared memory four times each, 7 k.)  The code runs once and waits for its own instructions: an
-// operand more, for what the rows' rounding leaves, took 2-3 us of the launch, not the 0.4 of its MMAs, and one MMA a turn 3.
-// All of W_UV's slice for this head (dC x 128 bf16) is fetched by one thread as 2 * nk TMA boxes before chain_wait(): the
-// weights do not depend on the decode kernel, and the launches before it have waited for everything older (as 512 bulk
-// copies of a row each, issued behind the merge's first loads, they took 2-3 us to be accepted).
-// grid (H, ceil(rows/64)), 512 threads, row = seq_index * S + query token.  dC = 128 * nk, nk <= 4.
-__global__ void __launch_bounds__(32 * kMergeWarps, 1) mla_merge_vup_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w, const float* part_o,
-                                                                const float* part_ml, const int32_t* chunk_off,
-                                                                void* __restrict__ out, int out_bf16, int rows, int S, int H, int dC,
-                                                                int32_t* __restrict__ status) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t w_full[kMaxChunks], done;   // chunk k of W_UV has landed (bytes counted by the TMA loads); D is complete
-  __shared__ uint32_t tmem_slot;
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int nk = dC / 128;
-  uint8_t* Ws = smem;                           // [nk][2 halves of 64 columns][128][64], swizzled
-  uint8_t* As = smem + (size_t)nk * 32768;      // [2 nk][64 rows][64], swizzled
-  const int h = blockIdx.x, r0 = blockIdx.y * 64;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  chain_release();
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_w);
-    for (int k = 0; k < nk; k++) mbar_init(&w_full[k], 1);
-    mbar_init(&done, 1);
-    fence_mbar_init();
-    for (int k = 0; k < nk; k++) {
-      mbar_expect_tx(&w_full[k], 32768);
-      tma_load_2d(Ws + (size_t)k * 32768, &tmap_w, h * kDh, k * 128, &w_full[k]);
-      tma_load_2d(Ws + (size_t)k * 32768 + 16384, &tmap_w, h * kDh + 64, k * 128, &w_full[k]);
-    }
+    tma_prefetch_desc(&tmap_p);
   }
   if (warp == 1) {
-    tmem_alloc<1>(&tmem_slot, 64);
+    tmem_alloc<1>(&sh->tmem_slot, prm.tmem_cols);
     tmem_relinquish<1>();
   }
-  chain_wait();   // the partial results come from the kernel before this one
-  part_o = behind_wait(part_o);
-  part_ml = behind_wait(part_ml);
-  chunk_off = behind_wait(chunk_off);
-  const int rows_here = min(64, rows - r0), n_tile = rows_here <= 16 ? 16 : rows_here <= 32 ? 32 : 64;
-  merge_rows_piped(As, part_o, part_ml, chunk_off, r0, rows_here, S, H, h, dC, nk, S * H);
-  fence_proxy_async();
   tc_fence_before();
-  __syncthreads();   // the merged rows are complete, the barriers and the tensor memory's address visible
+  __syncthreads();   // the barriers and the tensor memory's address are visible
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-  if (warp == 0) {
+  const uint32_t tmem = sh->tmem_slot;
+  auto first_of = [&](int i) -> int { return prm.listed ? prm.first[i] : load_chained(prm.chunk_off + i); };
+  auto col_of = [&](int row) -> int {   // first column of a row of the call
+    const int i = S == 1 ? row : row / S, q = row - i * S, c0 = first_of(i);
+    return c0 * S + (q == 0 ? 0 : q * (first_of(i + 1) - c0));
+  };
+  if (warp < 2) {
     const bool el = elect_one();
-    const uint32_t idesc = make_idesc_bf16(128, n_tile, true, false);
-    const uint64_t dW = make_desc_mnmajor_sw128(smem_u32(Ws), 16384), dA = make_desc_kmajor_sw128(smem_u32(As));
-    for (int k = 0; k < nk; k++) {
-      if (!mbar_wait(&w_full[k], 0)) set_status(status, RELUX_ERR_TIMEOUT);   // bounded: a copy that never lands is reported, not waited for
-      __syncwarp();
-      if (el) {
-#pragma unroll
-        for (int ks = 0; ks < 8; ks++)
-          umma_ss<1>(tmem, dW + ((uint32_t)(k * 32768 + ks * 2048) >> 4), dA + ((uint32_t)((2 * k + (ks >> 2)) * kMergeBlk + (ks & 3) * 32) >> 4),
-                     idesc, (k | ks) != 0);
-      }
+    chain_wait();   // the partial results come from the kernel before this one
+    const int col0 = col_of(r0), blocks = (col_of(r0 + rows_here) - col0 + nb - 1) / nb;
+    if (warp == 0) {
+#pragma unroll 1
+      for (int b = 0, s = 0, use = 0; b < blocks; b++)
+#pragma unroll 1
+        for (int st = 0; st < steps_each; st++) {
+          if (use > 0) vup_wait(&sh->empty[s], (use - 1) & 1, prm.status);
+          if (el) {
+            mbar_expect_tx(&sh->full[s], stage_bytes);
+            tma_load_5d(ring + s * stage_bytes, &tmap_p, 0, col0 + b * nb, 0, st * prm.n_kb, h, &sh->full[s]);
+          }
+          __syncwarp();
+          if (++s == prm.n_stages) s = 0, use++;
+        }
+    } else {
+      const uint32_t idesc = make_idesc_bf16(128, prm.halves * nb, true, false);
+      const uint64_t dA = make_desc_kmajor_sw128(smem_u32(ring)), dW = make_desc_mnmajor_sw128(smem_u32(Ws), nk * 16384);
+      vup_wait(&sh->w_full[0], 0, prm.status);
+#pragma unroll 1
+      for (int b = 0, s = 0, use = 0; b < blocks; b++)
+#pragma unroll 1
+        for (int st = 0, kb = 0; st < steps_each; st++) {
+          if (kb + prm.n_kb > 4 && nk > 2) vup_wait(&sh->w_full[1], 0, prm.status);
+          vup_wait(&sh->full[s], use & 1, prm.status);
+          const uint64_t a0 = dA + ((uint32_t)(s * stage_bytes) >> 4);
+#pragma unroll 1
+          for (int k = 0; k < prm.n_kb && kb < 2 * nk; k++, kb++)
+            if (el) {
+              const uint64_t a = a0 + ((uint32_t)(k * blk_bytes) >> 4), w = dW + (uint32_t)(kb * 512);
+              umma_ss<1>(tmem + b * prm.halves * nb, w, a, idesc, kb != 0);
+              umma_ss<1>(tmem + b * prm.halves * nb, w + 128, a + 2, idesc, true);
+              umma_ss<1>(tmem + b * prm.halves * nb, w + 256, a + 4, idesc, true);
+              umma_ss<1>(tmem + b * prm.halves * nb, w + 384, a + 6, idesc, true);
+            }
+          if (el) umma_commit<1>(&sh->empty[s]);
+          __syncwarp();
+          if (++s == prm.n_stages) s = 0, use++;
+        }
+      if (el) umma_commit<1>(&sh->done);
       __syncwarp();
     }
-    if (el) umma_commit<1>(&done);
-    __syncwarp();
   }
-  if (!mbar_wait(&done, 0)) set_status(status, RELUX_ERR_TIMEOUT);
-  tc_fence_after();
-  // lane = output dim 32 (warp & 3) + lane, column = row: every store of a warp is 32 neighbouring dims of a row
+  // The others: weights, then outputs, four warps a lane quarter and a quarter of the rows each.
+  // lane = output dim 32 (warp & 3) + lane, column = piece: every store of a warp is 32 neighbouring dims of a row
   const uint32_t tmem_d = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  size_t off = ((size_t)(r0 + (warp >> 2) * 4) * H + h) * kDh + (warp & 3) * 32 + lane;
+  const size_t off0 = ((size_t)r0 * H + h) * kDh + (warp & 3) * 32 + lane;
 #pragma unroll 1
-  for (int g = (warp >> 2) * 4; g < rows_here; g += 16, off += (size_t)16 * H * kDh) {
-    uint32_t v[4];
-    tmem_ld_32x32b_x4(tmem_d + g, v);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (g + j < rows_here) {
-        if (out_bf16) reinterpret_cast<uint16_t*>(out)[off + (size_t)j * H * kDh] = (uint16_t)pack_bf16x2(__uint_as_float(v[j]), 0.f);
-        else reinterpret_cast<float*>(out)[off + (size_t)j * H * kDh] = __uint_as_float(v[j]);
+  for (int pass = warp >= 2 && prm.warm ? 0 : 1; pass < 2; pass++) {
+    const bool real = pass == 1;
+    int col0 = 0, lo = 0, hi = 0;   // first column of the CTA, and columns of the warp's rows
+    if (real) {
+      if (warp >= 2) chain_wait();
+      const int ra = rows_here * (warp >> 2) / 4, rb = rows_here * ((warp >> 2) + 1) / 4;
+      col0 = col_of(r0);
+      lo = col_of(r0 + ra) - col0;
+      hi = col_of(r0 + rb) - col0;
+    }
+    if (warp >= 2) {
+      // the weights of a row's pieces, by 32, 8 or 4 lanes
+      const int lpr = rows_here <= kVupWarps - 2 ? 32 : rows_here <= 4 * (kVupWarps - 2) ? 8 : 4;
+      const int sub = lane & (lpr - 1), per_pass = (kVupWarps - 2) * (32 / lpr), rows_now = real ? rows_here : 1;
+#pragma unroll 1
+      for (int rw = 0; rw < rows_now; rw += per_pass) {
+        const int r = rw + ((warp - 2) * 32 + lane) / lpr;
+        int c = 0, n = 0;
+        if (r < rows_now) {
+          const int i = S == 1 ? r0 + r : (r0 + r) / S, q = r0 + r - i * S, first = first_of(i), pieces = first_of(i + 1) - first;
+          n = real ? pieces : 1;
+          c = real ? first * S + q * n - col0 : 0;
+        }
+        float M = -INFINITY;
+#pragma unroll 1
+        for (int j = sub; j < n; j += lpr) {
+          const float2 ml = load_chained(reinterpret_cast<const float2*>(prm.part_ml + ((size_t)(col0 + c + j) * H + h) * 2));
+          info[c + j] = ml;
+          M = fmaxf(M, ml.x);
+        }
+#pragma unroll 1
+        for (int o = 1; o < lpr; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        float L = 0.f;
+#pragma unroll 1
+        for (int j = sub; j < n; j += lpr) {
+          const float2 ml = info[c + j];
+          if (ml.x != -INFINITY) L += ml.y * exp2f(ml.x - M);
+        }
+#pragma unroll 1
+        for (int o = 1; o < lpr; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        const float inv = (L > 0.f) ? 1.0f / L : 0.f;
+#pragma unroll 1
+        for (int j = sub; j < n; j += lpr) {
+          const float m = info[c + j].x;
+          info[c + j] = make_float2(m == -INFINITY ? 0.f : exp2f(m - M) * inv, __int_as_float(j == n - 1 ? r * H * kDh : -1));
+        }
+        if (r < rows_now && n <= 0)   // an empty sequence
+          for (int d = sub; d < kDh; d += lpr) {
+            const size_t off = ((size_t)(r0 + r) * H + h) * kDh + d;
+            if (kOutBf16) reinterpret_cast<uint16_t*>(prm.out)[off] = 0;
+            else reinterpret_cast<float*>(prm.out)[off] = 0.f;
+          }
       }
+    }
+    if (real) {
+      __syncthreads();   // the weights
+      vup_wait(&sh->done, 0, prm.status);
+      tc_fence_after();
+    }
+    float acc = 0.f;
+#pragma unroll 1
+    for (int c = lo & ~7; c < (real ? hi : 8); c += 8) {
+      uint32_t v[8], w[8];   // the halves' products; a block's lie n_block apart
+      const int b = c >= nb ? c / nb : 0, at = c + (prm.halves - 1) * b * nb;
+      tmem_ld_32x32b_x8(tmem_d + at, v);
+      tmem_ld_32x32b_x8(tmem_d + at + (prm.halves - 1) * nb, w);
+      float4 f[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) f[j] = sh->info[c / 2 + j];
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const float wt = (j & 1) ? f[j >> 1].z : f[j >> 1].x, second = prm.halves == 2 ? __uint_as_float(w[j]) : 0.f;
+        const int r = __float_as_int((j & 1) ? f[j >> 1].w : f[j >> 1].y);
+        const bool mine = c + j >= lo && c + j < hi, last = mine && r >= 0;
+        const float x = fmaf(__uint_as_float(v[j]) + second, wt, acc);
+        acc = mine && wt != 0.f ? x : acc;   // a piece without a visible key may hold anything
+        if (kOutBf16) store_if(reinterpret_cast<uint16_t*>(prm.out) + off0 + r, (uint16_t)pack_bf16x2(acc, 0.f), last);
+        else store_if(reinterpret_cast<float*>(prm.out) + off0 + r, acc, last);
+        acc = last ? 0.f : acc;
+      }
+    }
   }
   tc_fence_before();
-  if (out_bf16) fence_chained_writes();   // a projection's operand
+  if (kOutBf16) fence_chained_writes();   // a projection's operand
   __syncthreads();
-  if (warp == 1) tmem_dealloc<1>(tmem, 64);
+  if (warp == 1) tmem_dealloc<1>(tmem, prm.tmem_cols);
 }
 
 }  // namespace
@@ -598,30 +439,69 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
   return RELUX_OK;
 }
 
-int32_t launch_mla_merge_vup_mma(Device* dev, const float* part_o, const float* part_ml, const int32_t* chunk_off, const uint16_t* W_UV,
-                                 void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
-  CUtensorMap tw;   // W_UV [dC][H * 128], 128 x 64 boxes
-  if (!make_tmap_2d(&tw, (void*)W_UV, (uint64_t)dC, (uint64_t)H * kDh, 64, 128)) {
-    set_error("tensor map for w_uv could not be encoded");
+// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU, more where they do not and every group keeps 32 columns,
+// or where a group would have more columns than it has room for.  A group's columns are one block where a stage of it, 64 latent columns,
+// fits the ring four times, and equal blocks otherwise.
+int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, int form, bool natural, const uint16_t* W_UV,
+                              void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
+  auto col_of = [&](int row) {
+    const int i = row / S, q = row - i * S;
+    return q == 0 ? plan.first[i] * S : plan.first[i] * S + q * (plan.first[i + 1] - plan.first[i]);
+  };
+  const int all = col_of(rows);
+  int groups = std::max(1, std::min({dev->sm_count / H, all / 32, rows}));
+  VupParams k;
+  int most = 0;
+  for (;; groups++) {
+    k.rows_each = (rows + groups - 1) / groups;
+    most = 0;
+    for (int r = 0; r < rows; r += k.rows_each) most = std::max(most, col_of(std::min(rows, r + k.rows_each)) - col_of(r));
+    if (most <= kVupMaxCols || k.rows_each == 1) break;
+  }
+  groups = (rows + k.rows_each - 1) / k.rows_each;
+  const int n_seqs = rows / S;
+  k.listed = n_seqs <= kVupListed && all < 65536;
+  if (k.listed)
+    for (int i = 0; i <= n_seqs; i++) k.first[i] = (uint16_t)plan.first[i];
+  k.halves = form == kPartialHalves ? 2 : 1;
+  const int widest = kVupRing / 4 / (k.halves * 128), blocks = std::max(1, (most + widest - 1) / widest);
+  const int unit = (blocks > 1 ? 32 : 16) / k.halves;   // N is a multiple of 16, and a block begins at a multiple of 32 tensor-memory columns
+  k.n_block = std::max(unit, ((most + blocks - 1) / blocks + unit - 1) / unit * unit);
+  const int blk_bytes = k.halves * k.n_block * 128;
+  k.n_kb = 4;
+  while (k.n_kb > 1 && k.n_kb * blk_bytes > kVupRing / (k.n_kb > 2 ? 2 : 3)) k.n_kb /= 2;
+  k.n_stages = std::min({kVupMaxStages, kVupRing / (k.n_kb * blk_bytes), (dC / 64 + k.n_kb - 1) / k.n_kb * blocks});
+  k.tmem_cols = 32;
+  while (k.tmem_cols < blocks * k.halves * k.n_block) k.tmem_cols *= 2;
+  k.part_ml = part_ml;
+  k.warm = all > 0;
+  k.chunk_off = plan.chunk_off;
+  k.out = out;
+  k.rows = rows;
+  k.S = S;
+  k.H = H;
+  k.nk = dC / 128;
+  k.status = status;
+  // W_UV [dC][H * 128]: latent row 32 b + 8 i + 2 q + e at place 32 b + 8 q + 2 i + e (write_partial), or as it is
+  const uint64_t ld = (uint64_t)H * kDh, di = natural ? 2 : 8, dq = natural ? 8 : 2, lp = (uint64_t)k.halves * dC;
+  const uint64_t w_dims[5] = {ld, 2, 4, 4, (uint64_t)dC / 32}, w_strides[4] = {ld, di * ld, dq * ld, 32 * ld};
+  const uint32_t w_box[5] = {64, 2, 4, 4, dC == 128 ? 4u : 8u};
+  const uint64_t p_dims[5] = {64, (uint64_t)all, (uint64_t)k.halves, (uint64_t)dC / 64, (uint64_t)H}, p_strides[4] = {H * lp, (uint64_t)dC, 64, lp};
+  const uint32_t p_box[5] = {64, (uint32_t)k.n_block, (uint32_t)k.halves, (uint32_t)k.n_kb, 1};
+  CUtensorMap tw, tp;
+  if (!make_tmap_view(&tw, (void*)W_UV, 5, w_dims, w_strides, w_box) || (all > 0 && !make_tmap_view(&tp, (void*)part, 5, p_dims, p_strides, p_box))) {
+    set_error("tensor map for w_uv or the partial results could not be encoded");
     return RELUX_ERR_CUDA;
   }
-  dim3 grid(H, (rows + 63) / 64);
-  // Up to 16 rows a warp has one row, with four items of it in flight, and eight warps' MMAs are short; beyond, rows follow one another
-  // in a warp.  64 rows (64 x 4096): the call takes 98.9 us by mma.sync, 96.7 by tcgen05; 16 rows (16 x <= 32k): 97.7 against 99-102.
-  if (rows > 16) {
-    const size_t smem_tc = (size_t)(dC / 128) * (32768 + 2 * kMergeBlk) + 1024;
-    if (int32_t rc = allow_smem(dev, mla_merge_vup_sm100_kernel, smem_tc)) return rc;
-    RELUX_CUDA_TRY(launch_chained(chained, mla_merge_vup_sm100_kernel, grid, dim3(32 * kMergeWarps), smem_tc, dev->stream, tw, part_o, part_ml, chunk_off,
-                                  out, out_bf16, rows, S, H, dC, status));
+  if (all == 0) tp = tw;   // every sequence is empty: zeros are written
+  const size_t smem = (size_t)k.nk * 32768 + (size_t)k.n_stages * k.n_kb * blk_bytes + sizeof(VupShared);
+  auto launch = [&](auto kern) -> int32_t {
+    if (int32_t rc = allow_smem(dev, kern, smem)) return rc;
+    RELUX_CUDA_TRY(launch_chained(chained, kern, dim3(H, groups), dim3(32 * kVupWarps), smem, dev->stream, tw, tp, k));
     count_launch(dev);
     return RELUX_OK;
-  }
-  const size_t smem = (size_t)(dC / 128) * (32768 + 16 * kStride * 2) + 1024;
-  if (int32_t rc = allow_smem(dev, mla_merge_vup_mma_kernel, smem)) return rc;
-  RELUX_CUDA_TRY(launch_chained(chained, mla_merge_vup_mma_kernel, grid, dim3(32 * kMergeWarps), smem, dev->stream, tw, part_o, part_ml, chunk_off,
-                                out, out_bf16, rows, S, H, dC, status));
-  count_launch(dev);
-  return RELUX_OK;
+  };
+  return out_bf16 ? launch(mla_vup_pieces_kernel<true>) : launch(mla_vup_pieces_kernel<false>);
 }
 
 }  // namespace relux

@@ -131,7 +131,9 @@ __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const Pre
         w.page_begin = cut.begin(c);
         w.page_end = cut.end(c);
         w.tokens = tokens;
-        w.pad[0] = w.pad[1] = w.pad[2] = 0;
+        w.first = c0;
+        w.n = cut.n;
+        w.pad = 0;
         pl.items[c0 + c] = w;
         if (pl.by_item) pl.worker_first[c0 + c] = c0 + c;
         else if (cut.leads(c, at)) pl.worker_first[cut.first + c] = c0 + c;

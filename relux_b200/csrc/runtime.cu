@@ -241,6 +241,17 @@ bool make_tmap_3d(CUtensorMap* m, void* base, uint64_t outer, uint64_t mid, uint
   return r == CUDA_SUCCESS;
 }
 
+bool make_tmap_view(CUtensorMap* m, void* base, int rank, const uint64_t* dims, const uint64_t* stride_elems, const uint32_t* box) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return false;
+  cuuint64_t d[5], strides[4];
+  cuuint32_t b[5], estr[5] = {1, 1, 1, 1, 1};
+  for (int i = 0; i < rank; i++) d[i] = dims[i], b[i] = box[i];
+  for (int i = 0; i + 1 < rank; i++) strides[i] = stride_elems[i] * 2;
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, base, d, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Float32, for stores; box[0] is 16 or 32 columns, the swizzle that of the box's row length.
 bool make_tmap_4d_f32(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]) {
   EncodeTiledFn enc = get_encode();
@@ -983,7 +994,8 @@ API int32_t relux_pool_create(relux_device_t h, const relux_pool_params* prm, re
       // blocked page layout: the whole pool is one [blocks * 64][64] array, every TMA box is one contiguous 8 KB block
       p->mla_blocked = true;
       uint64_t rows = (uint64_t)prm->num_layers * prm->num_pages * (p->row_elems_a / 64) * prm->page_tokens;
-      p->has_tmap = make_tmap_2d(&p->tmap_mla, p->storage, rows, 64, 64, 64);
+      p->has_tmap = make_tmap_2d(&p->tmap_mla, p->storage, rows, 64, 64, 64) && make_tmap_2d(&p->tmap_mla_2, p->storage, rows, 64, 64, 128) &&
+                    make_tmap_2d(&p->tmap_mla_3, p->storage, rows, 64, 64, 192);
     } else if (prm->kind == RELUX_POOL_GQA && prm->gqa_head_dim % 64 == 0) {
       uint64_t rows = (uint64_t)prm->num_layers * 2 * prm->num_pages * prm->gqa_num_kv_heads * prm->page_tokens;
       p->has_tmap = make_tmap_2d(&p->tmap_gqa, p->storage, rows, (uint64_t)prm->gqa_head_dim, 64, 64);

@@ -4,6 +4,7 @@
 // is one work item handled by one CTA (or CTA pair), so a handful of long sequences still fills
 // all SMs.  The list is built on the device from the device-resident lengths; the host computes
 // only the item COUNT from its shadow lengths, so no host->device copy is needed per step.
+#include <algorithm>
 #include <cstdlib>
 #include <vector>
 #include "common.cuh"
@@ -100,8 +101,10 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
     chunk = (chunk + mult - 1) / mult * mult;
     if (max_chunk_pages > 0) chunk = std::min(chunk, max_chunk_pages / mult * mult);
   }
+  while ((max_pages + chunk - 1) / chunk > kMaxRowItems && max_chunk_pages <= 0) chunk += mult;
   int items = 0;
-  for (int i = 0; i < sb.n_seqs; i++) items += (pages[i] + chunk - 1) / chunk;
+  plan->first.assign(1, 0);
+  for (int i = 0; i < sb.n_seqs; i++) plan->first.push_back(items += (pages[i] + chunk - 1) / chunk);
   plan->chunk_pages = chunk;
   plan->num_items = items;
   size_t bytes = sizeof(WorkItem) * (size_t)items + sizeof(int32_t) * ((size_t)sb.n_seqs + 1) + 64;
@@ -168,7 +171,9 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
         w.page_begin = cut.begin(c);
         w.page_end = cut.end(c);
         w.tokens = tokens;
-        w.pad[0] = w.pad[1] = w.pad[2] = 0;
+        w.first = c0;
+        w.n = cut.n;
+        w.pad = 0;
         items[c0 + c] = w;
         if (by_item) worker_first[c0 + c] = c0 + c;
         else if (cut.leads(c, at)) worker_first[cut.first + c] = c0 + c;
@@ -214,7 +219,8 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   StreamShape shape{};
   if (const int chunk = p->tune.get(RELUX_TUNE_CHUNK_PAGES)) {   // tuning knob: ranges of that many pages
     long G = 0;
-    stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, chunk, &G, &shape.workers, &shape.items);
+    const int longest = pages.empty() ? 0 : *std::max_element(pages.begin(), pages.end());
+    stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, std::max(chunk, (longest + kMaxRowItems - 3) / (kMaxRowItems - 2)), &G, &shape.workers, &shape.items);
     shape.G = (int)G;
     shape.room = shape.items;
   } else {
@@ -228,6 +234,12 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   plan->num_items = items;
   plan->room_items = shape.room;
   plan->num_workers = workers;
+  plan->first.assign(1, 0);
+  for (int i = 0, at = 0, sum = 0; i < sb.n_seqs; i++) {
+    const SeqCut cut(shape.by_item, G, shape.start_units, at, pages[i]);
+    at += cut.units;
+    plan->first.push_back(sum += cut.n);
+  }
   const size_t off_chunk = sizeof(StreamItem) * (size_t)shape.room;
   const size_t off_worker = (off_chunk + sizeof(int32_t) * ((size_t)sb.n_seqs + 1) + 15) & ~(size_t)15;
   int32_t rc = grow(p->dev, p->work, off_worker + sizeof(int32_t) * ((size_t)std::max(workers, most_workers) + 1) + 64);

@@ -22,7 +22,8 @@ struct __align__(16) StreamItem {
   int32_t page_begin;
   int32_t page_end;
   int32_t tokens;      // cached length of the sequence + the call's extra tokens
-  int32_t pad[3];
+  int32_t first, n;    // the sequence's first item and how many it has
+  int32_t pad;
 };
 
 struct SplitPlan {
@@ -31,6 +32,7 @@ struct SplitPlan {
   int room_items = 0;           // partials are given room for as many (num_items, where that is more): StreamShape::room
   WorkItem* items = nullptr;    // device
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]
+  std::vector<int32_t> first;   // the same on the host: sequence i has items [first[i], first[i + 1])
   // stream plans only (plan_stream): worker w owns items [worker_first[w], worker_first[w + 1])
   int num_workers = 0;
   // every worker has one item, chunk_pages pages of a sequence; or ranges of chunk_pages units, a sequence's pages (an even number of
@@ -40,6 +42,13 @@ struct SplitPlan {
   StreamItem* stream_items = nullptr;  // device [num_items]
   int32_t* worker_first = nullptr;     // device [num_workers + 1]
 };
+
+// More items than this no sequence is cut into (the projection of the partial results keeps the columns of a row together): only the
+// knob CHUNK_PAGES could ask for more.
+constexpr int kMaxRowItems = 240;
+
+// A row of a latent call's partial results: float32, one bf16 value or two bf16 halves a column (write_partial, mla_decode_sm100.cu).
+enum PartialForm { kPartialFloat32 = 0, kPartialOne = 1, kPartialHalves = 2 };
 
 struct Pool;
 struct SeqBatch;
