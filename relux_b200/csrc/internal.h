@@ -238,7 +238,7 @@ struct StepAppend {
   const void* kr;
   int dtype;
   const int32_t* d_row_off;   // device row offsets of the append batch (nullptr = rows_each rows per sequence)
-  int32_t rows_each = 1;
+  int32_t rows_each = 1, max_rows = 1;   // new rows of a sequence: of each (where there are no offsets), at most
   bool weights_ready = false; // a launch before this one in the call has waited for everything older (launch_mla_prep)
 };
 int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const void* d_q, const void* d_qr,
@@ -264,6 +264,9 @@ void note_append(Pool* p, int layer, int seq, int old_len, int n);
 void note_set_len(Pool* p, int layer, int seq, int old_len, int new_len);
 // Host pointers handed over as device memory must be 16-byte aligned: the kernels read them with vector loads.
 int32_t check_dev_align(const void* ptr, const char* what);
+
+// Whether what the call launches now is recorded in a graph: it then runs with the device's lengths of later moments, not with the host's.
+bool stream_captured(const Device* dev);
 
 // Tensor maps (runtime.cu).  bf16 elements, 128-byte swizzle, no out-of-bounds fill value (zeros); false when the driver
 // entry point is missing or refuses the map.

@@ -808,7 +808,7 @@ int32_t do_mla_layer(Pool* p, const relux_mla_layer_args* a) {
   aa.w_uk = w.w_uk;
   aa.w_uv = w.w_uv;
   aa.mode = a->mode;
-  const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr, 1, mma};   // one row per sequence
+  const StepAppend step{d_c, d_kr, RELUX_DTYPE_F32, nullptr, 1, 1, mma};   // one row per sequence
   const bool o_bf16 = mma && mla_writes_bf16(p, sb, aa);   // the output projection's operand, rounded by the kernel that makes it
   rc = fast ? launch_mla_decode_fast(p, sb, aa, d_qc, d_qr, o_bf16 ? (void*)sc.a_bf16 : d_attn, o_bf16, fused_append ? &step : nullptr)
             : launch_attn_reference_mla(p, sb, aa, (const float*)d_qc, (const float*)d_qr, d_attn);

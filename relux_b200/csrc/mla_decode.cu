@@ -19,7 +19,7 @@
 namespace relux {
 
 int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
-                                int form, TimeStamp time);
+                                const ListedPlan& list, int form, TimeStamp time);
 bool mla_sm100_eligible(const Pool* p, const relux_attn_args& a);
 int mla_sm100_workers(Pool* p, int q_tokens);
 bool mla_proj_mma_eligible(int Dh, int dC);
@@ -288,6 +288,12 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   if (rc) return rc;
   const bool sm100 = mla_sm100_eligible(p, a);
   SplitPlan plan;
+  const bool proj_mma = mla_proj_mma_eligible(Dh, dC);
+  ListedPlan list;                     // read where `listed` says so
+  list.listed = 0;
+  list.new_rows = step ? step->max_rows : 0;
+  plan.captured = stream_captured(p->dev);
+  ListedPlan* const to_list = proj_mma && !plan.captured ? &list : nullptr;   // merge_splits_kernel reads the plan from device memory
   // The stream partition depends on the cached lengths only, the absorb on the queries only: the one-block builder
   // runs on the side stream next to the absorb kernel and is joined before the decode kernel.
   cudaStream_t side = p->dev->side_stream;
@@ -295,7 +301,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   const bool fork = sm100 && side != nullptr && !fused_prep;
   if (fused_prep) {
     // one launch: absorb + the step's append + the stream partition (the host lengths already count the new rows)
-    rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, st, false);
+    rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, st, false, to_list);
     if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
     if (rc) return rc;
     PrepAppend ap;
@@ -319,6 +325,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     ap.dHR = dHR;
     ap.blocked = p->mla_blocked ? 1 : 0;
     PrepPlan pl;
+    pl.listed = list.listed;
     pl.extra = a.extra_tokens;
     pl.G = plan.chunk_pages;
     pl.by_item = plan.by_item ? 1 : 0;
@@ -338,7 +345,6 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     if (rc) return rc;
     RELUX_CUDA_TRY(cudaEventRecord(p->dev->ev_join, side));
   }
-  const bool proj_mma = mla_proj_mma_eligible(Dh, dC);
   if (fused_prep) {
     // absorbed queries, appended rows and the partition are already queued
   } else if (proj_mma) {
@@ -368,7 +374,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     if (rc) return rc;
   }
   // rows of one piece each are rounded where they are written
-  const bool split = !sm100 || plan.num_items > sb.n_seqs || [&] {
+  const bool split = !sm100 || plan.captured || plan.num_items > sb.n_seqs || [&] {
     for (int i = 0; i < sb.n_seqs; i++)
       if (plan.first[i + 1] - plan.first[i] > 1) return true;
     return false;
@@ -378,7 +384,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   const int stride = std::max(1, p->tune.get(RELUX_TUNE_KERNEL_TIMING_STRIDE));
   const bool timed = (p->attn_calls++ % (uint64_t)stride) == 0;
   if (sm100) {
-    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p, form,
+    rc = launch_mla_decode_sm100(p, sb, a, plan, (const uint16_t*)p->q_abs.p, list, form,
                                  timed ? time_stamp_next(p, p->attn_times) : TimeStamp{nullptr, nullptr});
     if (rc) return rc;
   } else {

@@ -119,6 +119,14 @@ __device__ __forceinline__ StreamItem load_item(const StreamItem* p) {
   return it;
 }
 
+// The same from the arguments.
+__device__ __forceinline__ StreamItem listed_item(const ListedItem& l) {
+  StreamItem it;
+  it.seq_index = l.seq_index; it.seq = l.seq; it.page_begin = l.page_begin; it.page_end = l.page_end;
+  it.tokens = l.tokens; it.first = l.first; it.n = l.n; it.pad = 0;
+  return it;
+}
+
 // Page ids of an item as the producer warp holds them: lane l keeps the first pool row (TMA y coordinate) of
 // pages 32 * blk + l (`cur`) and 32 * (blk + 1) + l (`nxt`); positions past the item's last page repeat the last page.
 struct PageWin {
@@ -220,7 +228,7 @@ __device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, vo
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     mla_decode_sm100_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_q,
-                            const __grid_constant__ MlaSm100Params prm) {
+                            const __grid_constant__ MlaSm100Params prm, const __grid_constant__ ListedPlan list) {
   extern __shared__ __align__(1024) uint8_t smem[];
   Bars* bars = reinterpret_cast<Bars*>(smem + kSmemBar);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,12 +265,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
-  chain_wait();   // the ranges, the absorbed queries and the step's new rows come from the kernel before this one
-  int it0 = load_chained(prm.worker_first + worker), it1 = load_chained(prm.worker_first + worker + 1);
+  // The absorbed queries, the step's new rows and (unless they are arguments) the ranges come from the kernel before this one.  The producer
+  // warp waits for them further down, behind its requests for a first tile of older rows: those were complete before the head of this
+  // chain began, like the page table.
+  const bool listed = list.listed != 0;
+  if (warp != 4 || !listed) chain_wait();
+  int it0 = listed ? list.worker_first[worker] : load_chained(prm.worker_first + worker);
+  int it1 = listed ? list.worker_first[worker + 1] : load_chained(prm.worker_first + worker + 1);
   if (sq >= prm.S) it1 = it0;   // an empty range: nothing to do, and the CTA pair still meets at the end
+  auto item_at = [&](int it) { return listed ? listed_item(list.items[it]) : load_item(prm.items + it); };
   if (threadIdx.x == 0 && it0 < it1) stamp_begin(prm.time);
 
   if (it0 >= it1) {
+    if (warp == 4 && listed) chain_wait();
   } else if (warp == 4) {
     // =============================== producer: TMA loads into this CTA's slots ===============================
     // The whole warp stays converged and one elected lane issues: operands that every lane computes identically
@@ -320,20 +335,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         __syncwarp();
       }
     };
-    StreamItem cur = load_item(prm.items + it0);
+    StreamItem cur = item_at(it0);
     PageWin w;
     w.cur = win_load(cur, 0);
     w.nxt = win_load(cur, 1);
     w.blk = 0;
+    // (the first values too, early or behind the queries: no difference)
+    const bool early = listed && (cur.page_begin + 2) * kPage <= cur.tokens - list.new_rows;   // no row of the first tile is new
+    if (early) load_k(w, 0, 0);
+    if (listed) chain_wait();
     load_q(cur);
-    load_k(w, 0, 0);
+    if (!early) load_k(w, 0, 0);
     int g = 0;
     for (int it = it0; it < it1; ++it) {
       const bool has_next = it + 1 < it1;
       StreamItem nxt = cur;
       PageWin wn = w;
       if (has_next) {   // fetched now, used at the end of this item
-        nxt = load_item(prm.items + it + 1);
+        nxt = item_at(it + 1);
         wn.cur = win_load(nxt, 0);
         wn.nxt = win_load(nxt, 1);
         wn.blk = 0;
@@ -414,8 +433,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         __syncwarp();
       };
       auto tiles_of = [&](int it) -> int {
-        const int4 a = load_chained(reinterpret_cast<const int4*>(prm.items + it));
-        return (a.w - a.z + 1) >> 1;
+        const StreamItem a = item_at(it);
+        return (a.page_end - a.page_begin + 1) >> 1;
       };
       int ntiles = tiles_of(it0);
       int g = 0, n = 0;
@@ -446,11 +465,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     const int hf = L >> 6;            // token half of the tile (= which CTA's page)
     const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
     const uint32_t p_full_lead = mapa_u32(smem_u32(&bars->p_full), 0);
-    StreamItem cur = load_item(prm.items + it0);
+    StreamItem cur = item_at(it0);
     int g = 0;
     for (int it = it0; it < it1; ++it) {
       StreamItem nxt = cur;
-      if (it + 1 < it1) nxt = load_item(prm.items + it + 1);   // fetched now, used after this item
+      if (it + 1 < it1) nxt = item_at(it + 1);   // fetched now, used after this item
       const int limit_tok = prm.causal ? (cur.tokens - prm.S + sq + 1) : cur.tokens;   // tokens [0, limit_tok) are visible
       const int tok_end = min(limit_tok, cur.page_end * kPage);
       const int ntiles = (cur.page_end - cur.page_begin + 1) >> 1;
@@ -618,7 +637,7 @@ int mla_sm100_workers(Pool* p, int q_tokens) {
 }
 
 int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_args& a, const SplitPlan& plan, const uint16_t* q_abs,
-                                int form, TimeStamp time) {
+                                const ListedPlan& list, int form, TimeStamp time) {
   const relux_pool_params& prm = p->prm;
   if (plan.num_items == 0) return RELUX_OK;   // every sequence is empty: the merge writes zeros
   CUtensorMap tq;   // the absorbed queries [rows][576] in boxes of three blocks of 64 columns x 64 rows
@@ -656,7 +675,7 @@ int32_t launch_mla_decode_sm100(Pool* p, const SeqBatch& sb, const relux_attn_ar
   if (int32_t rc = allow_smem(p->dev, mla_decode_sm100_kernel, kSmemTotal)) return rc;
   dim3 grid(2 * plan.num_workers * sx, a.q_tokens / sx);
   RELUX_CUDA_TRY(launch_chained(p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0, mla_decode_sm100_kernel, grid, dim3(192), (size_t)kSmemTotal,
-                                p->dev->stream, p->tmap_mla_3, p->tmap_mla_2, tq, k));
+                                p->dev->stream, p->tmap_mla_3, p->tmap_mla_2, tq, k, list));
   time_stamp_done(p->attn_times, time);
   return RELUX_OK;
 }

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const __grid_consta
 }
 
 // The preparation of one MLA decode step in ONE launch: blocks 0 .. n_seqs - 1 append the step's new rows (a sequence
-// each), block n_seqs builds the stream partition, and the blocks after them are the absorb grid (head fastest, then the
+// each), block n_seqs builds the stream partition (unless the decode kernel has it as arguments), and the blocks after them are the absorb grid (head fastest, then the
 // dC / 128 latent slices, then 64 rows each).  The three jobs are independent of one another: the append reads the lengths
 // before it writes, the partition counts every sequence's new rows itself, and the last of those blocks to finish advances
 // the lengths.  They come first because theirs is the longer chain of dependent reads.
@@ -145,11 +145,11 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ C
                                                        uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int weights_ready,
                                                        const __grid_constant__ PrepAppend ap, const __grid_constant__ PrepPlan pl) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  const int e = blockIdx.x;
+  const int e = blockIdx.x, chores = ap.n_seqs + (pl.listed ? 0 : 1);
   if (!weights_ready) chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
   chain_release();
-  if (e > ap.n_seqs) {
-    const int a = e - ap.n_seqs - 1, slices = dC / 128;
+  if (e >= chores) {
+    const int a = e - chores, slices = dC / 128;
     absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, ap.status,
                  true, weights_ready != 0);
     return;
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ C
   if (weights_ready) chain_wait();
   if (e < ap.n_seqs) prep_append_seq(ap, e);
   else prep_build_stream(ap, pl);
-  prep_arrive_and_advance(ap, (uint32_t)ap.n_seqs + 1u);
+  prep_arrive_and_advance(ap, (uint32_t)chores);
 }
 
 // Value up-projection of the split-KV partial results, and their sum.  For one head, with the pieces of a row (a sequence's query
@@ -429,7 +429,7 @@ int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rop
 // One launch: absorb + append of the step's rows + stream partition (see mla_prep_kernel).
 int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows,
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained) {
-  const unsigned blocks = (unsigned)ap.n_seqs + 1u + (unsigned)H * (unsigned)(dC / 128) * (unsigned)((rows + 63) / 64);
+  const unsigned blocks = (unsigned)ap.n_seqs + (pl.listed ? 0u : 1u) + (unsigned)H * (unsigned)(dC / 128) * (unsigned)((rows + 63) / 64);
   CUtensorMap tw, tq;
   if (int32_t rc = absorb_maps(W_UK, q_nope, q_bf16, rows, H, dC, &tw, &tq)) return rc;
   if (int32_t rc = allow_smem(dev, mla_prep_kernel, kAbsorbSmem)) return rc;
@@ -448,19 +448,20 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
     const int i = row / S, q = row - i * S;
     return q == 0 ? plan.first[i] * S : plan.first[i] * S + q * (plan.first[i + 1] - plan.first[i]);
   };
-  const int all = col_of(rows);
+  const int more = plan.captured ? std::max(0, plan.room_items - plan.num_items) * S : 0;   // columns that a graph may find
+  const int all = col_of(rows) + more;
   int groups = std::max(1, std::min({dev->sm_count / H, all / 32, rows}));
   VupParams k;
   int most = 0;
   for (;; groups++) {
     k.rows_each = (rows + groups - 1) / groups;
     most = 0;
-    for (int r = 0; r < rows; r += k.rows_each) most = std::max(most, col_of(std::min(rows, r + k.rows_each)) - col_of(r));
+    for (int r = 0; r < rows; r += k.rows_each) most = std::max(most, col_of(std::min(rows, r + k.rows_each)) - col_of(r) + more);
     if (most <= kVupMaxCols || k.rows_each == 1) break;
   }
   groups = (rows + k.rows_each - 1) / k.rows_each;
   const int n_seqs = rows / S;
-  k.listed = n_seqs <= kVupListed && all < 65536;
+  k.listed = !plan.captured && n_seqs <= kVupListed && all < 65536;
   if (k.listed)
     for (int i = 0; i <= n_seqs; i++) k.first[i] = (uint16_t)plan.first[i];
   k.halves = form == kPartialHalves ? 2 : 1;

@@ -25,6 +25,7 @@ struct PrepAppend {
 };
 
 struct PrepPlan {
+  int32_t listed;              // nothing to build
   int32_t extra, G, workers, by_item, start_units;
   StreamItem* items;
   int32_t* chunk_off;

@@ -252,6 +252,11 @@ bool make_tmap_view(CUtensorMap* m, void* base, int rank, const uint64_t* dims, 
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool stream_captured(const Device* dev) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(dev->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+}
+
 // Float32, for stores; box[0] is 16 or 32 columns, the swizzle that of the box's row length.
 bool make_tmap_4d_f32(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint32_t (&box)[4]) {
   EncodeTiledFn enc = get_encode();
@@ -1406,7 +1411,7 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   }
   // the host lengths count the new rows from here on: the attention call plans with them
   for (int i = 0; i < sb.n_seqs; i++) p->h_len[(size_t)kv->layer * prm.max_seqs + sb.seq[i]] += sb.rows[i];
-  StepAppend step{da, db, kv->dtype, sb.d_row_off, sb.rows_each};
+  StepAppend step{da, db, kv->dtype, sb.d_row_off, sb.rows_each, sb.max_rows};
   rc = do_attention(p, attn, kind, &step);
   if (rc) {
     take_rows_back(p, sb, kv->layer);

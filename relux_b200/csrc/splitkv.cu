@@ -208,8 +208,27 @@ void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_
   *items_out = items;
 }
 
+// The items as build_stream_kernel writes them, into arguments; false where they do not fit.
+static bool list_plan(const SeqBatch& sb, const std::vector<int>& pages, const int32_t* len, int extra, const SplitPlan& plan, ListedPlan* out) {
+  if (plan.num_items > kListedItems || plan.num_workers > kListedWorkers) return false;
+  int at = 0, item = 0;
+  for (int i = 0; i < sb.n_seqs; i++) {
+    const SeqCut cut(plan.by_item, plan.chunk_pages, plan.start_units, at, pages[i]);
+    if (pages[i] > 65535) return false;
+    const int first = item;
+    for (int c = 0; c < cut.n; c++, item++) {
+      out->items[item] = ListedItem{sb.seq[i], len[sb.seq[i]] + extra, (uint16_t)cut.begin(c), (uint16_t)cut.end(c), (uint16_t)i, (uint16_t)first, (uint16_t)cut.n, 0};
+      if (plan.by_item) out->worker_first[item] = (uint16_t)item;
+      else if (cut.leads(c, at)) out->worker_first[cut.first + c] = (uint16_t)item;
+    }
+    at += cut.units;
+  }
+  for (int w = plan.by_item ? item : (at + plan.chunk_pages - 1) / plan.chunk_pages; w <= plan.num_workers; w++) out->worker_first[w] = (uint16_t)item;
+  return true;
+}
+
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
-                    bool launch_builder) {
+                    bool launch_builder, ListedPlan* list) {
   const relux_pool_params& prm = p->prm;
   std::vector<int> pages(sb.n_seqs);
   for (int i = 0; i < sb.n_seqs; i++) {
@@ -240,6 +259,7 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
     at += cut.units;
     plan->first.push_back(sum += cut.n);
   }
+  if (list && (list->listed = list_plan(sb, pages, p->h_len.data() + (size_t)layer * prm.max_seqs, extra, *plan, list))) return RELUX_OK;
   const size_t off_chunk = sizeof(StreamItem) * (size_t)shape.room;
   const size_t off_worker = (off_chunk + sizeof(int32_t) * ((size_t)sb.n_seqs + 1) + 15) & ~(size_t)15;
   int32_t rc = grow(p->dev, p->work, off_worker + sizeof(int32_t) * ((size_t)std::max(workers, most_workers) + 1) + 64);

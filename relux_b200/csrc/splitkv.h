@@ -26,9 +26,24 @@ struct __align__(16) StreamItem {
   int32_t pad;
 };
 
+// A stream plan as kernel arguments, for calls of a few items: the decode kernel then knows its work, and asks for cached rows, before the
+// launch in front of it is complete.
+constexpr int kListedItems = 160, kListedWorkers = 80;
+struct ListedItem {
+  int32_t seq, tokens;
+  uint16_t page_begin, page_end, seq_index, first, n, pad;   // as in StreamItem
+};
+struct ListedPlan {
+  int32_t listed;        // 0: the plan is in device memory
+  int32_t new_rows;      // the call's launches before the decode kernel write the last new_rows of a sequence's tokens, at most
+  uint16_t worker_first[kListedWorkers + 2];
+  ListedItem items[kListedItems];
+};
+
 struct SplitPlan {
   int chunk_pages = 0;                 // of a stream plan: pages of a piece, or units of a range
   int num_items = 0;
+  bool captured = false;        // num_items may have become more (up to room_items) when the launch runs: stream_captured
   int room_items = 0;           // partials are given room for as many (num_items, where that is more): StreamShape::room
   WorkItem* items = nullptr;    // device
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]
@@ -61,8 +76,9 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
 // `st`: the stream the builder kernel is launched on (the pool's main stream, or the device's side stream).
 // launch_builder = false: only the host half (counts, buffers); the caller builds the lists itself (the fused decode-step
 // preparation of mla_proj.cu does it inside its own launch).
+// `list`: where the plan fits there, it is written there and not built on the device.
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
-                    bool launch_builder = true);
+                    bool launch_builder = true, ListedPlan* list = nullptr);
 int32_t launch_build_worklist_raw(cudaStream_t st, const int32_t* len, const int32_t* seq_ids, int n_seqs, int extra, int page_tokens,
                                   int chunk_pages, WorkItem* items, int32_t* chunk_off);
 int32_t launch_merge_raw(cudaStream_t st, const float* part_o, const float* part_ml, const int32_t* chunk_off, int n_seqs, int rows,
