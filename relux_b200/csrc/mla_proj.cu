@@ -1,10 +1,9 @@
 // The two small per-head GEMMs around the absorbed MLA decode, on tensor cores, bf16 in, f32 accumulate:
-//   absorb:  q~[row][h][0:dC]  = q_nope[row][h][:] . W_UK[:, h*Dh:(h+1)*Dh]^T      M = rows, N = dC,  K = Dh      (mma.sync m16n8k16)
+//   absorb:  q~[row][h][0:dC]  = q_nope[row][h][:] . W_UK[:, h*Dh:(h+1)*Dh]^T      M = rows, N = dC,  K = Dh      (M = dC, N = rows on tcgen05)
 //            q~[row][h][dC: ]  = q_rope[row][h][:]
 //   up-proj: out[row][h][:]    = O_lat[row][h][:] . W_UV[:, h*Dh:(h+1)*Dh]          M = Dh, N = pieces of rows, K = dC   (tcgen05)
 // Both are about 1 GFLOP per step at batch 64 (1.5 % of the decode's work) and move ~30 MB; they are written to stay out of the way of
-// the decode kernel, not to chase the tensor peak.  The absorb has one CTA per (head, 128-wide slice, 64 rows), operands staged in shared
-// memory by a few TMA boxes (every load of a CTA in flight at once), fragments through ldmatrix.  The up-projection is also the split-KV
+// the decode kernel, not to chase the tensor peak.  Operands come by a few TMA boxes (every load of a CTA in flight at once).  The up-projection is also the split-KV
 // merge: it multiplies every piece and adds the products up.
 // Shapes: Dh = 128, dC a multiple of 128.  Other shapes use the scalar kernels in mla_decode.cu.
 #include "common.cuh"
@@ -20,36 +19,62 @@ namespace relux {
 namespace {
 
 constexpr int kDh = 128;
-constexpr int kStride = kDh + 8;  // bf16 elements per shared-memory row (272 B: conflict-free ldmatrix)
 
-// 64 rows x 128 latent columns of the absorb for one head, by 128 threads.  W_UK's tile [128 c][128 d] and (bf16) the query
-// tile [64 rows][128 d] come as four TMA boxes from one thread: as 3072 cp.async of 16 bytes they took 2.2 us to issue.  Both
-// lie as two 64-column blocks with the 128-byte swizzle.  Up to 32 rows, the warps share the row groups that hold a row.
-// Measured (the whole preparation launch, before -> now): 3 rows 8.1 -> 4.7 us, 64 rows 12.6 -> 12.0 us.
-// The result leaves through shared memory as 16-byte row-contiguous stores.
-constexpr int kAbsorbSmem = 32768 + 16384 + 1024;
-__device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const void* __restrict__ q_nope,
-                                             const void* __restrict__ q_rope, int q_bf16, uint16_t* __restrict__ q_abs, int rows, int H, int dC,
-                                             int dHR, int bx, int by, int bz, int32_t* status, bool chained, bool wait_for_queries) {
+struct AbsorbParams {
+  const void* q_nope;
+  const void* q_rope;
+  uint16_t* q_abs;
+  int32_t q_bf16, rows, H, dC, dHR, n_chunks;   // n_chunks: 128 latent columns each, of a CTA
+  int32_t* status;
+};
+
+// Up to 32 rows x 128 latent columns of the absorb for one head, by 128 threads on mma.sync.  W_UK's tile [128 c][128 d] and (bf16) the query
+// tile [32 rows][128 d] come as four TMA boxes from one thread: as 3072 cp.async of 16 bytes they took 2.2 us to issue.  Both
+// lie as two 64-column blocks with the 128-byte swizzle; the warps share the row groups that hold a row.  The result leaves through shared
+// memory as 16-byte row-contiguous stores.  Four CTAs an SM: their round trips overlap, which for few rows is all there is to gain, and one
+// CTA of four chunks on tcgen05 takes 0.1-0.3 us longer (1 x 300 19.5 -> 19.7 us, 30 x 1000 layers 253.6 -> 255.9).
+constexpr int kAbsorbMmaThreads = 128, kAbsorbMmaRows = 32;
+constexpr size_t kAbsorbMmaSmem = 32768 + 8192 + 1024;
+constexpr int kStride = kDh + 8;  // bf16 elements per shared-memory row (272 B: conflict-free ldmatrix)
+__device__ __forceinline__ void absorb_block_mma(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const AbsorbParams& prm, int bx,
+                                                 int by, bool chained, bool weights_ready) {
+  const void* const q_nope = prm.q_nope;
+  const void* const q_rope = prm.q_rope;
+  uint16_t* const q_abs = prm.q_abs;
+  const int q_bf16 = prm.q_bf16, H = prm.H, dC = prm.dC, dHR = prm.dHR;
   __shared__ __align__(8) uint64_t landed;
   uint8_t* sm = (uint8_t*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* Bs = sm;             // [2 halves of d][128 c][64], swizzled
-  uint8_t* As = sm + 32768;     // [2 halves of d][64 rows][64], swizzled
-  const int h = bx, c0 = by * 128, r0 = bz * 64;
+  uint8_t* As = sm + 32768;     // [2 halves of d][32 rows][64], swizzled
+  const int h = bx, c0 = by * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rows_here = min(64, rows - r0), groups = rows_here <= 16 ? 1 : rows_here <= 32 ? 2 : 4;
+  const int rows_here = prm.rows, groups = rows_here <= 16 ? 1 : 2;
   if (threadIdx.x == 0) {
     mbar_init(&landed, 1);
     fence_mbar_init();
-    mbar_expect_tx(&landed, 32768 + (q_bf16 ? 16384 : 0));
-    tma_load_2d(Bs, tmap_w, h * kDh, c0, &landed);
-    tma_load_2d(Bs + 16384, tmap_w, h * kDh + 64, c0, &landed);
+    tma_prefetch_desc(tmap_w);
+    tma_prefetch_desc(tmap_q);
+    mbar_expect_tx(&landed, 32768 + (q_bf16 ? 8192 : 0));
   }
-  if (wait_for_queries) chain_wait();
+  auto load_w = [&] {
+    if (threadIdx.x == 0) {
+      tma_load_2d(Bs, tmap_w, h * kDh, c0, &landed);
+      tma_load_2d(Bs + 16384, tmap_w, h * kDh + 64, c0, &landed);
+    }
+  };
+  if (weights_ready) {
+    if (chained) chain_release();
+    load_w();
+  }
+  chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
+  if (!weights_ready) {
+    if (chained) chain_release();
+    load_w();
+  }
   if (q_bf16) {
     if (threadIdx.x == 0) {   // rows past the batch are zero-filled
-      tma_load_2d(As, tmap_q, h * kDh, r0, &landed);
-      tma_load_2d(As + 8192, tmap_q, h * kDh + 64, r0, &landed);
+      tma_load_2d(As, tmap_q, h * kDh, 0, &landed);
+      tma_load_2d(As + 4096, tmap_q, h * kDh + 64, 0, &landed);
     }
   } else {
 #pragma unroll 4
@@ -57,11 +82,11 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
       const int r = e / (kDh / 8), v = e % (kDh / 8);
       uint4 w = make_uint4(0, 0, 0, 0);
       if (r < rows_here) {
-        const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_nope) + ((size_t)(r0 + r) * H + h) * kDh + (size_t)v * 8);
+        const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q_nope) + ((size_t)r * H + h) * kDh + (size_t)v * 8);
         const float4 x = load_chained(s), y = load_chained(s + 1);
         w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
       }
-      *reinterpret_cast<uint4*>(As + (v >> 3) * 8192 + swz128(r, v & 7)) = w;
+      *reinterpret_cast<uint4*>(As + (v >> 3) * 4096 + swz128(r, v & 7)) = w;
     }
   }
   const int roww = dC + dHR;
@@ -69,7 +94,7 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
     const int vecs = dHR / 8;
     for (int e = threadIdx.x; e < rows_here * vecs; e += blockDim.x) {
       const int r = e / vecs, v = e % vecs;
-      const size_t off = ((size_t)(r0 + r) * H + h) * dHR + (size_t)v * 8;
+      const size_t off = ((size_t)r * H + h) * dHR + (size_t)v * 8;
       uint4 w;
       if (q_bf16) w = load_chained(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q_rope) + off));
       else {
@@ -77,26 +102,26 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
         const float4 x = load_chained(s), y = load_chained(s + 1);
         w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
       }
-      *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + dC + (size_t)v * 8) = w;
+      *reinterpret_cast<uint4*>(q_abs + ((size_t)r * H + h) * roww + dC + (size_t)v * 8) = w;
     }
   }
   __syncthreads();   // the barrier and the float32 rows are visible
-  if (!mbar_wait(&landed, 0)) set_status(status, RELUX_ERR_TIMEOUT);   // bounded: a load that never lands is reported
+  if (!mbar_wait(&landed, 0)) set_status(prm.status, RELUX_ERR_TIMEOUT);   // bounded: a load that never lands is reported
   // warp: 16 rows x 32 * groups columns
   const int m = lane >> 3, row_w = (warp % groups) * 16, col_w = (warp / groups) * 32 * groups;
   const uint32_t a_base = smem_u32(As), b_base = smem_u32(Bs);
-  float acc[16][4];
+  float acc[8][4];
 #pragma unroll
-  for (int i = 0; i < 16; i++)
+  for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
 #pragma unroll
   for (int ks = 0; ks < 8; ks++) {
     uint32_t a[4];
     const int ka = ks * 2 + (m >> 1), kb = ks * 2 + (m & 1);   // 16-byte chunk of the row
-    ldmatrix_x4(a[0], a[1], a[2], a[3], a_base + (ka >> 3) * 8192 + swz128(row_w + (m & 1) * 8 + (lane & 7), ka & 7));
+    ldmatrix_x4(a[0], a[1], a[2], a[3], a_base + (ka >> 3) * 4096 + swz128(row_w + (m & 1) * 8 + (lane & 7), ka & 7));
 #pragma unroll
-    for (int n2 = 0; n2 < 8; n2++) {
+    for (int n2 = 0; n2 < 4; n2++) {
       if (n2 >= 2 * groups) break;
       uint32_t b0, b1, b2, b3;
       ldmatrix_x4(b0, b1, b2, b3, b_base + (kb >> 3) * 16384 + swz128(col_w + n2 * 16 + (m >> 1) * 8 + (lane & 7), kb & 7));
@@ -110,7 +135,7 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
   for (int hf = 0; hf < 2; hf++) {
     const int r = row_w + hf * 8 + (lane >> 2);
 #pragma unroll
-    for (int nt = 0; nt < 16; nt++) {
+    for (int nt = 0; nt < 8; nt++) {
       if (nt >= 4 * groups) break;
       *reinterpret_cast<uint32_t*>(Os + r * kStride + col_w + nt * 8 + 2 * (lane & 3)) = pack_bf16x2(acc[nt][hf * 2], acc[nt][hf * 2 + 1]);
     }
@@ -118,46 +143,218 @@ __device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap*
   __syncthreads();
   for (int e = threadIdx.x; e < rows_here * 16; e += blockDim.x) {
     const int r = e / 16, v = e % 16;
-    *reinterpret_cast<uint4*>(q_abs + ((size_t)(r0 + r) * H + h) * roww + c0 + v * 8) = *reinterpret_cast<const uint4*>(Os + r * kStride + v * 8);
+    *reinterpret_cast<uint4*>(q_abs + ((size_t)r * H + h) * roww + c0 + v * 8) = *reinterpret_cast<const uint4*>(Os + r * kStride + v * 8);
   }
   if (chained) fence_chained_writes();
 }
 
-// grid (H, dC/128, ceil(rows/64)), 128 threads.  A plain launch that releases nobody early: the decode kernel reads its rows by TMA
-// behind its end.
-__global__ void __launch_bounds__(128) mla_absorb_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
-                                                             const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
-                                                             uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int32_t* status) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, blockIdx.x, blockIdx.y, blockIdx.z, status, false, false);
+// The absorb of up to 64 rows for one head and 128, 256 or 512 latent columns (n_chunks of 128), on tcgen05: of every chunk
+// D[128 x 128 latent columns] = q W_UK^T, both operands K-major as they lie, in two 64-column blocks with the 128-byte swizzle, by TMA (as 3072
+// cp.async of 16 bytes a chunk took 2.2 us to issue).  The M = 128 rows are the queries' 64 twice over, so that all four warps of a group find rows in
+// the quarter of tensor memory that they can read, and each takes half of the columns.  Warp 8
+// loads and multiplies chunk by chunk, two groups of four warps take the chunks in turn: tensor memory to bf16, through the chunk's own
+// weights' place, out by TMA.
+// CTAs of one chunk each were started one an SM, by their stamps, once the kernel used tensor memory, four by mma.sync: so a CTA has as many
+// chunks as leave no head waiting for a second turn.
+// Bound: W_UK from memory (16.8 MB at 128 heads) behind one round trip.  By mma.sync, four CTAs of one chunk an SM, the launch took 9.3-12
+// us at 64 rows of 128 heads (its products alone 2.8), so 7.1-7.7; steps of 64 x 300 31.8 -> 28.7 us, 64 x 1000 41.0 -> 39.5, 64 x 4096 83.7 -> 81.8.
+constexpr int kAbsorbThreads = 288;
+constexpr int kAbsorbQ = 32768, kAbsorbW = 32768, kAbsorbRows = 64;
+// Unless `weights_ready` the launch is the head of a chain: it releases the next one, and reads W_UK, behind its wait.
+__device__ __forceinline__ void absorb_block(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const CUtensorMap* tmap_out,
+                                             const AbsorbParams& prm, int bx, int by, int bz, bool chained, bool weights_ready) {
+  __shared__ __align__(8) uint64_t landed[4], done[4], q_landed;
+  __shared__ uint32_t tmem_slot;
+  uint8_t* sm = (uint8_t*)(((uintptr_t)sm_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* As = sm;               // [2 halves of d][128 rows][64], swizzled
+  uint8_t* Bs = sm + kAbsorbQ;    // [chunk][2 halves of d][128 c][64], swizzled; then [chunk][2 halves of c][kAbsorbRows rows][64]
+  const int n_chunks = prm.n_chunks, H = prm.H, q_bf16 = prm.q_bf16;
+  const int h = bx, c0 = by * 128 * n_chunks, r0 = bz * 64;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rows_here = min(64, prm.rows - r0);
+  const uint32_t tmem_cols = n_chunks * 128;
+  auto load_w = [&] {
+    for (int i = 0; i < n_chunks; i++) {
+      mbar_expect_tx(&landed[i], kAbsorbW);
+      tma_load_2d(Bs + i * kAbsorbW, tmap_w, h * kDh, c0 + i * 128, &landed[i]);
+      tma_load_2d(Bs + i * kAbsorbW + 16384, tmap_w, h * kDh + 64, c0 + i * 128, &landed[i]);
+    }
+  };
+  // The release stands behind the allocation: a CTA of the up-projection, which allocates ahead of its wait, may share the SM, and must find this
+  // one's columns taken.  Ahead of this launch's own wait it allocates only behind launches that use no tensor memory beside it.
+  auto take_tmem = [&] {
+    tmem_alloc<1>(&tmem_slot, tmem_cols);
+    tmem_relinquish<1>();
+  };
+  if (warp == 8) {
+    if (elect_one()) {
+      tma_prefetch_desc(tmap_w);
+      tma_prefetch_desc(tmap_q);
+      mbar_init(&q_landed, 1);
+      for (int i = 0; i < n_chunks; i++) {
+        mbar_init(&landed[i], 1);
+        mbar_init(&done[i], 1);
+      }
+      fence_mbar_init();
+      if (weights_ready) load_w();
+      tma_prefetch_desc(tmap_out);
+    }
+    if (weights_ready) {
+      take_tmem();
+      if (chained) chain_release();
+    }
+  }
+  chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
+  if (warp == 8) {
+    if (elect_one()) {
+      if (q_bf16) {   // rows past the batch are zero-filled
+        mbar_expect_tx(&q_landed, 32768);
+        for (int r = 0; r < 128; r += kAbsorbRows) {
+          tma_load_2d(As + r * 128, tmap_q, h * kDh, r0, &q_landed);
+          tma_load_2d(As + 16384 + r * 128, tmap_q, h * kDh + 64, r0, &q_landed);
+        }
+      }
+      if (!weights_ready) load_w();
+    }
+    if (!weights_ready) {
+      take_tmem();
+      if (chained) chain_release();
+    }
+    __syncwarp();
+  }
+  if (!q_bf16) {
+#pragma unroll 2
+    for (int e = threadIdx.x; e < rows_here * (kDh / 8); e += blockDim.x) {
+      const int r = e / (kDh / 8), v = e % (kDh / 8);
+      const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(prm.q_nope) + ((size_t)(r0 + r) * H + h) * kDh + (size_t)v * 8);
+      const float4 x = load_chained(s), y = load_chained(s + 1);
+      const uint4 w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
+      for (int k = r; k < 128; k += kAbsorbRows) *reinterpret_cast<uint4*>(As + (v >> 3) * 16384 + swz128(k, v & 7)) = w;
+    }
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();   // the barriers, the tensor memory's address and the float32 rows are visible
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const int roww = prm.dC + prm.dHR;
+  if (warp == 8) {
+    const bool el = elect_one();
+    constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
+    const uint64_t dQ = make_desc_kmajor_sw128(smem_u32(As)), dW = make_desc_kmajor_sw128(smem_u32(Bs));
+    if (q_bf16 && !mbar_wait(&q_landed, 0)) set_status(prm.status, RELUX_ERR_TIMEOUT);   // bounded: a load that never lands is reported
+#pragma unroll 1
+    for (int i = 0; i < n_chunks; i++) {
+      if (!mbar_wait(&landed[i], 0)) set_status(prm.status, RELUX_ERR_TIMEOUT);
+      __syncwarp();
+      if (el) {
+        const uint64_t w = dW + (uint32_t)(i * (kAbsorbW >> 4));
+#pragma unroll
+        for (int ks = 0; ks < 8; ks++)
+          umma_ss<1>(tmem + i * 128, dQ + (((ks >> 2) * 16384 + (ks & 3) * 32) >> 4), w + (((ks >> 2) * 16384 + (ks & 3) * 32) >> 4), idesc, ks != 0);
+        umma_commit<1>(&done[i]);
+      }
+      __syncwarp();
+    }
+  } else {
+    if (by == 0) {   // the rope part of q~ is a copy (with the same rounding when the source is float32)
+      const int vecs = prm.dHR / 8;
+      for (int e = threadIdx.x; e < rows_here * vecs; e += 256) {
+        const int r = e / vecs, v = e % vecs;
+        const size_t off = ((size_t)(r0 + r) * H + h) * prm.dHR + (size_t)v * 8;
+        uint4 w;
+        if (q_bf16) w = load_chained(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(prm.q_rope) + off));
+        else {
+          const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(prm.q_rope) + off);
+          const float4 x = load_chained(s), y = load_chained(s + 1);
+          w = make_uint4(pack_bf16x2(x.x, x.y), pack_bf16x2(x.z, x.w), pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w));
+        }
+        *reinterpret_cast<uint4*>(prm.q_abs + ((size_t)(r0 + r) * H + h) * roww + prm.dC + (size_t)v * 8) = w;
+      }
+    }
+    const int group = warp >> 2, row = (warp & 1) * 32 + lane, first = (warp & 2) * 32;   // this warp's first column of a chunk
+#pragma unroll 1
+    for (int i = group; i < n_chunks; i += 2) {
+      if (!mbar_wait(&done[i], 0)) set_status(prm.status, RELUX_ERR_TIMEOUT);
+      tc_fence_after();
+      uint8_t* Os = Bs + i * kAbsorbW;
+#pragma unroll 1
+      for (int c = first; c < first + 64; c += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + i * 128 + c, v);
+        tmem_ld_wait_for(v);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          uint32_t w[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) w[k] = pack_bf16x2(__uint_as_float(v[8 * j + 2 * k]), __uint_as_float(v[8 * j + 2 * k + 1]));
+          *reinterpret_cast<uint4*>(Os + (c >> 6) * 8192 + swz128(row, ((c & 63) >> 3) + j)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+      fence_proxy_async();
+      asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
+      if ((threadIdx.x & 127) == 0) {   // rows past the batch lie outside the map
+        tma_store_2d(tmap_out, h * roww + c0 + i * 128, r0, Os);
+        tma_store_2d(tmap_out, h * roww + c0 + i * 128 + 64, r0, Os + 8192);
+        tma_store_commit();
+      }
+    }
+    if ((threadIdx.x & 127) == 0) tma_store_wait_all();
+    if (chained) fence_chained_writes();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) tmem_dealloc<1>(tmem, tmem_cols);
 }
 
-// The preparation of one MLA decode step in ONE launch: blocks 0 .. n_seqs - 1 append the step's new rows (a sequence
-// each), block n_seqs builds the stream partition (unless the decode kernel has it as arguments), and the blocks after them are the absorb grid (head fastest, then the
-// dC / 128 latent slices, then 64 rows each).  The three jobs are independent of one another: the append reads the lengths
+// One block of either, a of the grid: head fastest, then the chunks of latent columns, then 64 rows each.
+template <bool kTc>
+__device__ __forceinline__ void absorb_any(uint8_t* sm_raw, const CUtensorMap* tmap_w, const CUtensorMap* tmap_q, const CUtensorMap* tmap_out,
+                                           const AbsorbParams& prm, int a, bool chained, bool weights_ready) {
+  const int slices = prm.dC / 128 / prm.n_chunks;
+  if constexpr (kTc) absorb_block(sm_raw, tmap_w, tmap_q, tmap_out, prm, a % prm.H, a / prm.H % slices, a / prm.H / slices, chained, weights_ready);
+  else absorb_block_mma(sm_raw, tmap_w, tmap_q, prm, a % prm.H, a / prm.H, chained, weights_ready);
+}
+
+// A plain launch.
+template <bool kTc>
+__global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_absorb_mma_kernel(const __grid_constant__ CUtensorMap tmap_w,
+                                                             const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_out,
+                                                             const __grid_constant__ AbsorbParams prm) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  absorb_any<kTc>(smem_raw, &tmap_w, &tmap_q, &tmap_out, prm, blockIdx.x, false, true);
+}
+
+// The preparation of one MLA decode step in ONE launch: the first blocks append the step's new rows (a warp a sequence), the next one builds
+// the stream partition (unless the decode kernel has it as arguments), and the blocks after them are the absorb grid (head fastest, then the
+// chunks of latent columns, then 64 rows each).  The three jobs are independent of one another: the append reads the lengths
 // before it writes, the partition counts every sequence's new rows itself, and the last of those blocks to finish advances
-// the lengths.  They come first because theirs is the longer chain of dependent reads.
+// the lengths (without a partition nobody else reads a sequence's length, and its warp advances it itself).  They come first because theirs is
+// the longer chain of dependent reads.
 // The kernel releases the launches after it only when everything before it is complete (the up-projection fetches its
 // weights without a wait of its own), unless the launches before it in the call have seen to that (weights_ready): its own
 // weights are then fetched ahead of its wait too.
-__global__ void __launch_bounds__(128) mla_prep_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
-                                                       const void* __restrict__ q_nope, const void* __restrict__ q_rope, int q_bf16,
-                                                       uint16_t* __restrict__ q_abs, int rows, int H, int dC, int dHR, int weights_ready,
-                                                       const __grid_constant__ PrepAppend ap, const __grid_constant__ PrepPlan pl) {
+template <bool kTc>
+__global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_prep_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_q,
+                                                       const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ AbsorbParams prm,
+                                                       int weights_ready, const __grid_constant__ PrepAppend ap, const __grid_constant__ PrepPlan pl) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  const int e = blockIdx.x, chores = ap.n_seqs + (pl.listed ? 0 : 1);
-  if (!weights_ready) chain_wait();   // also: the kernel before this one may still be reading what this one overwrites
-  chain_release();
+  constexpr int kWarps = kTc ? 8 : 4;
+  const int appends = (ap.n_seqs + kWarps - 1) / kWarps, chores = appends + (pl.listed ? 0 : 1), e = blockIdx.x;
   if (e >= chores) {
-    const int a = e - chores, slices = dC / 128;
-    absorb_block(smem_raw, &tmap_w, &tmap_q, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, a % H, a / H % slices, a / H / slices, ap.status,
-                 true, weights_ready != 0);
+    absorb_any<kTc>(smem_raw, &tmap_w, &tmap_q, &tmap_out, prm, e - chores, true, weights_ready != 0);
     return;
   }
-  if (weights_ready) chain_wait();
-  if (e < ap.n_seqs) prep_append_seq(ap, e);
-  else prep_build_stream(ap, pl);
-  prep_arrive_and_advance(ap, (uint32_t)chores);
+  if (weights_ready) chain_release();
+  chain_wait();
+  chain_release();
+  if (e < appends) {
+    const int i = e * kWarps + (threadIdx.x >> 5);
+    if (threadIdx.x < 32 * kWarps && i < ap.n_seqs) prep_append_seq(ap, i, pl.listed != 0);
+  } else {
+    prep_build_stream(ap, pl);
+  }
+  if (!pl.listed) prep_arrive_and_advance(ap, (uint32_t)chores);
 }
 
 // Value up-projection of the split-KV partial results, and their sum.  For one head, with the pieces of a row (a sequence's query
@@ -403,40 +600,64 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
 
 bool mla_proj_mma_eligible(int Dh, int dC) { return Dh == kDh && dC % 128 == 0; }
 
-// W_UK [dC][H * 128] in 128 x 64 boxes; bf16 queries [rows][H * 128] in 64 x 64 boxes.
-static int32_t absorb_maps(const uint16_t* W_UK, const void* q_nope, int q_bf16, int rows, int H, int dC, CUtensorMap* tw, CUtensorMap* tq) {
-  if (!make_tmap_2d(tw, (void*)W_UK, (uint64_t)dC, (uint64_t)H * kDh, 64, 128) ||
-      (q_bf16 && !make_tmap_2d(tq, (void*)q_nope, (uint64_t)rows, (uint64_t)H * kDh, 64, 64))) {
+// W_UK [dC][H * 128] in 128 x 64 boxes; bf16 queries [rows][H * 128], and the result [rows][H * (dC + dHR)], in boxes of the kernel's rows.  On tcgen05 a
+// CTA has as many chunks as leave the heads' CTAs one turn on the GPU.
+struct AbsorbSetup {
+  CUtensorMap w, q, out;
+  AbsorbParams prm;
+  bool tc;
+  unsigned ctas;
+  size_t smem;
+};
+static int32_t absorb_setup(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows, int H, int dC,
+                            int dHR, int32_t* status, AbsorbSetup* s) {
+  s->tc = rows > kAbsorbMmaRows;
+  const int n_tile = s->tc ? kAbsorbRows : kAbsorbMmaRows;
+  if (!make_tmap_2d(&s->w, (void*)W_UK, (uint64_t)dC, (uint64_t)H * kDh, 64, 128) ||
+      (s->tc && !make_tmap_2d(&s->out, q_abs, (uint64_t)rows, (uint64_t)H * (dC + dHR), 64, n_tile)) ||
+      (q_bf16 && !make_tmap_2d(&s->q, (void*)q_nope, (uint64_t)rows, (uint64_t)H * kDh, 64, n_tile))) {
     set_error("tensor map for w_uk or the queries could not be encoded");
     return RELUX_ERR_CUDA;
   }
-  if (!q_bf16) *tq = *tw;
+  if (!q_bf16) s->q = s->w;
+  if (!s->tc) s->out = s->w;
+  int n = 1;
+  while (s->tc && n < 4 && dC / 128 % (2 * n) == 0 && H * (dC / 128 / n) > dev->sm_count) n *= 2;
+  s->prm = AbsorbParams{q_nope, q_rope, q_abs, q_bf16, rows, H, dC, dHR, n, status};
+  s->ctas = (unsigned)H * (unsigned)(dC / 128 / n) * (unsigned)((rows + 63) / 64);
+  s->smem = s->tc ? (size_t)kAbsorbQ + (size_t)n * kAbsorbW + 1024 : kAbsorbMmaSmem;
   return RELUX_OK;
 }
+constexpr size_t kAbsorbSmemMost = kAbsorbQ + 4 * kAbsorbW + 1024;
 
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
                               int rows, int H, int dC, int dHR, int32_t* status) {
-  dim3 grid(H, dC / 128, (rows + 63) / 64);
-  CUtensorMap tw, tq;
-  if (int32_t rc = absorb_maps(W_UK, q_nope, q_bf16, rows, H, dC, &tw, &tq)) return rc;
-  if (int32_t rc = allow_smem(dev, mla_absorb_mma_kernel, kAbsorbSmem)) return rc;
-  mla_absorb_mma_kernel<<<grid, 128, kAbsorbSmem, dev->stream>>>(tw, tq, q_nope, q_rope, q_bf16, q_abs, rows, H, dC, dHR, status);
-  RELUX_CUDA_TRY(cudaGetLastError());
-  count_launch(dev);
-  return RELUX_OK;
+  AbsorbSetup s;
+  if (int32_t rc = absorb_setup(dev, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, status, &s)) return rc;
+  auto launch = [&](auto kern, int threads, size_t most) -> int32_t {
+    if (int32_t rc = allow_smem(dev, kern, most)) return rc;
+    kern<<<s.ctas, threads, s.smem, dev->stream>>>(s.w, s.q, s.out, s.prm);
+    RELUX_CUDA_TRY(cudaGetLastError());
+    count_launch(dev);
+    return RELUX_OK;
+  };
+  return s.tc ? launch(mla_absorb_mma_kernel<true>, kAbsorbThreads, kAbsorbSmemMost) : launch(mla_absorb_mma_kernel<false>, kAbsorbMmaThreads, kAbsorbMmaSmem);
 }
 
 // One launch: absorb + append of the step's rows + stream partition (see mla_prep_kernel).
 int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs, int rows,
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained) {
-  const unsigned blocks = (unsigned)ap.n_seqs + (pl.listed ? 0u : 1u) + (unsigned)H * (unsigned)(dC / 128) * (unsigned)((rows + 63) / 64);
-  CUtensorMap tw, tq;
-  if (int32_t rc = absorb_maps(W_UK, q_nope, q_bf16, rows, H, dC, &tw, &tq)) return rc;
-  if (int32_t rc = allow_smem(dev, mla_prep_kernel, kAbsorbSmem)) return rc;
-  RELUX_CUDA_TRY(launch_chained(chained, mla_prep_kernel, dim3(blocks), dim3(128), (size_t)kAbsorbSmem, dev->stream, tw, tq, q_nope, q_rope, q_bf16,
-                                q_abs, rows, H, dC, dHR, weights_ready ? 1 : 0, ap, pl));
-  count_launch(dev);
-  return RELUX_OK;
+  AbsorbSetup s;
+  if (int32_t rc = absorb_setup(dev, q_nope, q_rope, q_bf16, W_UK, q_abs, rows, H, dC, dHR, ap.status, &s)) return rc;
+  auto launch = [&](auto kern, int threads, size_t most) -> int32_t {
+    if (int32_t rc = allow_smem(dev, kern, most)) return rc;
+    const int warps = threads / 64 * 2;   // that append, of a block: 4 of 4, 8 of 9
+    const unsigned blocks = (unsigned)(ap.n_seqs + warps - 1) / (unsigned)warps + (pl.listed ? 0u : 1u) + s.ctas;
+    RELUX_CUDA_TRY(launch_chained(chained, kern, dim3(blocks), dim3(threads), s.smem, dev->stream, s.w, s.q, s.out, s.prm, weights_ready ? 1 : 0, ap, pl));
+    count_launch(dev);
+    return RELUX_OK;
+  };
+  return s.tc ? launch(mla_prep_kernel<true>, kAbsorbThreads, kAbsorbSmemMost) : launch(mla_prep_kernel<false>, kAbsorbMmaThreads, kAbsorbMmaSmem);
 }
 
 // Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU, more where they do not and every group keeps 32 columns,

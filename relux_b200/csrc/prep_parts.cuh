@@ -60,14 +60,25 @@ __device__ __forceinline__ void prep_arrive_and_advance(const PrepAppend& g, uin
   if (threadIdx.x == 0) *g.done = 0u;
 }
 
-// All new rows of sequence i (MLA row = [dC | dHR] fused; 16-byte stores).
-__device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i) {
+// All new rows of sequence i, by a warp (MLA row = [dC | dHR] fused; 16-byte stores).  A row's values do not wait for the length and the page that
+// say where they go.  `advance`: the length is this warp's to advance.
+__device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i, bool advance) {
   const int seq = g.seq_ids ? g.seq_ids[i] : i;
   const int r0 = g.row_off ? g.row_off[i] : i * g.rows_each;
   const int nrows = g.row_off ? g.row_off[i + 1] - r0 : g.rows_each;
+  const int lane = threadIdx.x & 31;
   const int base_len = load_chained(g.len + seq);
   const int row_elems = g.dC + g.dHR, vec_per_row = row_elems / 8, vc = g.dC / 8;
+  auto source = [&](int r, int v) {
+    return (v < vc) ? prep_load8(g.ckv, (size_t)(r0 + r) * g.dC + (size_t)v * 8, g.f32 != 0)
+                    : prep_load8(g.kr, (size_t)(r0 + r) * g.dHR + (size_t)(v - vc) * 8, g.f32 != 0);
+  };
+  constexpr int kHeld = 3;   // vectors of a row that a lane asks for ahead: a row of 512 + 64 columns
   for (int r = 0; r < nrows; r++) {
+    uint4 held[kHeld];
+#pragma unroll
+    for (int k = 0; k < kHeld; k++)
+      if (lane + 32 * k < vec_per_row) held[k] = source(r, lane + 32 * k);
     const int pos = base_len + r;
     const int slot = pos / g.page_tokens;
     int32_t pg;
@@ -76,12 +87,15 @@ __device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i) {
       continue;
     }
     uint16_t* page = g.layer_base + (size_t)pg * g.page_tokens * row_elems;
-    for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
-      const uint4 w = (v < vc) ? prep_load8(g.ckv, (size_t)(r0 + r) * g.dC + (size_t)v * 8, g.f32 != 0)
-                               : prep_load8(g.kr, (size_t)(r0 + r) * g.dHR + (size_t)(v - vc) * 8, g.f32 != 0);
+    auto put = [&](int v, const uint4& w) {
       *reinterpret_cast<uint4*>(page + mla_page_off(g.blocked != 0, g.page_tokens, row_elems, pos % g.page_tokens, v * 8)) = w;
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < kHeld; k++)
+      if (lane + 32 * k < vec_per_row) put(lane + 32 * k, held[k]);
+    for (int v = lane + 32 * kHeld; v < vec_per_row; v += 32) put(v, source(r, v));
   }
+  if (advance && lane == 0) g.len[seq] = base_len + nrows;
   fence_chained_writes();
 }
 
