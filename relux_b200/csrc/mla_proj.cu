@@ -528,12 +528,12 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
         if (r < rows_now) {
           const int i = S == 1 ? r0 + r : (r0 + r) / S, q = r0 + r - i * S, first = first_of(i), pieces = first_of(i + 1) - first;
           n = real ? pieces : 1;
-          c = real ? first * S + q * n - col0 : 0;
+          c = real ? first * S + q * n - col0 : kVupMaxCols + 8;   // no column's place: other warps may be at theirs already
         }
         float M = -INFINITY;
 #pragma unroll 1
         for (int j = sub; j < n; j += lpr) {
-          const float2 ml = load_chained(reinterpret_cast<const float2*>(prm.part_ml + ((size_t)(col0 + c + j) * H + h) * 2));
+          const float2 ml = load_chained(reinterpret_cast<const float2*>(prm.part_ml + ((size_t)((real ? col0 + c : 0) + j) * H + h) * 2));
           info[c + j] = ml;
           M = fmaxf(M, ml.x);
         }
