@@ -38,19 +38,20 @@ struct SeqCut {
   RELUX_HD bool leads(int c, int at) const { return (first + c) * G >= at; }
 };
 
-// What a plan costs, in tiles of two pages (about 2 us): its slowest worker's tiles and two for every item (start and write-out), 0.08 for
-// every partial that a row of the merge adds up, and 0.035 for every partial of the call.  From steps of 1 to 30 short sequences with
-// ranges of one and of two tiles (1 x 1300 tokens 19.9 against 21.5 us, 1 x 2600 21.5 and 21.4, 1 x 6000 26.8 and 24.0, 4 x 1200 24.0 and
-// 23.3, 25 x 200 27.4 and 28.3).
-inline double plan_cost(double worst, int most_items, int items) { return worst + 0.08 * most_items + 0.035 * items; }
+// What a plan costs, in tiles of two pages (1.1 us at 32 heads, 1.3 at 128): its slowest worker's tiles and two for every item (start and
+// write-out); 0.025 for every partial of the call and 0.04 for every one of the longest row (the up-projection's columns); 1.4 where a row has
+// more than one, for then all come as two halves, where single ones are written and read as one; and 0.25 where a worker has several.
+// Fit to forced plans of 49 batches of 1 to 64 sequences at 32, 64 and 128 heads (one query token): the plan taken is on average 0.3 % slower
+// than the best one found, where 0.035, 0.08, 0 and 0 were off by 1.2 % and by up to 11 %.
+inline double plan_cost(double worst, int most_items, int items, bool split, bool shared) {
+  return worst + 0.04 * most_items + 0.025 * items + (split ? 1.4 : 0) + (shared ? 0.25 : 0);
+}
 
 // The cheapest plan of a call: equal ranges of the sequences laid end to end, each counted as its pages and kStartUnits, for a worker
 // that starts it has a second item to start and to write out; or every sequence cut by itself into pieces of 2 t pages, a worker each.
-// Measured, ranges of pages alone -> this, one build: in pieces, 1 x 1300 tokens 21.8 -> 20.2 us, 3 x <= 1500 26.9 -> 22.3, 16 x 300 28.6 ->
-// 25.1, 64 x 300 41.0 -> 40.5, 40 x <= 2500 51.1 -> 45.1, 64 x 4096 93.8 -> 89.4, with 32 heads 64 x 500 42.5 -> 35.7; in ranges, 20 x 16000
-// 97.3 -> 95.5, and no difference beyond the runs' own at 16 x <= 32768 (97) and 64 x 32768 (565-585).  The fit is to one query token and
-// 128 heads; elsewhere: verify of 3 x <= 1500 with 4 tokens 39.1 -> 34.0, 16 x 300 with 2 43.2 -> 37.9, 32 x 1000 with 4 87.6 -> 79.3, 30 x
-// <= 800 with 3 and 32 heads 52.1 -> 46.2, the other way 64 x 300 with 2 and 32 heads 48.5 -> 50.1.
+// Measured, ranges forced -> this, one build: 1 x 1300 tokens 23.3 -> 20.2 us, 3 x <= 1500 24.3 -> 21.7, 16 x 300 26.3 -> 22.3, 64 x 1000 46.3
+// -> 39.4, 64 x 4096 93.2 -> 84, with 32 heads 1 x 1300 18.5 -> 15.1, 64 x 1000 34.5 -> 31.7; no difference beyond the runs' own at 16 x 2000
+// (30.1), 20 x 8000 (64), 16 x <= 32768 and, with 32 heads, 40 x <= 2500 (31.0).
 constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for an item
 struct StreamShape {
   int G, workers, items, start_units;
@@ -85,7 +86,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   }
   r.room = r.items;
   if (live == 0 || live > workers) return r;
-  double best = plan_cost(worst, most, r.items);
+  double best = plan_cost(worst, most, r.items, r.items > live, r.items > r.workers);
   auto items_of = [&](int t) {
     int items = 0;
     for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
@@ -97,9 +98,9 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
     if (items_of(t) <= workers) hi = t;
     else lo = t + 1;
   }
-  for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
-    const int items = items_of(t);
-    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
+  for (int k = 0; k < 4; k++) {   // some more tiles each may leave fewer partials, or one a sequence
+    const int t = k < 3 ? lo + k : (longest + 1) / 2, items = items_of(t);
+    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items, items > live, false);
     r.room = std::max(r.room, items);
     if (cost < best) {
       best = cost;
