@@ -39,9 +39,6 @@ struct Device {
   size_t total_mem = 0;
   char name[256] = {0};
   cudaStream_t stream = nullptr;
-  // side stream for small kernels that do not depend on their predecessor (forked from / joined to `stream` by events)
-  cudaStream_t side_stream = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // copy streams of pipelined calls (RELUX_CALL_PIPELINED): host -> device inputs, device -> host outputs
   cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;
   cudaEvent_t ev_copy_join = nullptr;
@@ -307,6 +304,9 @@ inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 //        - skinny_gemm_sm100_kernel, the weights: the first launch of a layer step or matmul is cast_bf16_kernel, the
 //          second GEMM of a layer follows it, a plain absorb launch, or a cast of its own;
 //        - mla_prep_kernel with weights_ready, W_UK: only behind the projections of the same call (do_mla_layer);
+//        - build_stream_kernel, the lengths (and it writes the plan, which the launches of older calls read): behind an mla_prep_kernel that is
+//          a head, or a plain absorb launch;
+//        - mla_decode_sm100_kernel, tiles without new rows, where it has the plan as arguments: the call's head is before it;
 //        - mla_vup_pieces_kernel, W_UV: the preparation or the plain absorb launch of the same call is before it.  (It also reads part_ml there,
 //          whatever it holds, and makes no use of it: mla_proj.cu.)
 //      A new early read names its head here; a new launch in front of one of these keeps a head between.

@@ -294,16 +294,15 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   list.new_rows = step ? step->max_rows : 0;
   plan.captured = stream_captured(p->dev);
   ListedPlan* const to_list = proj_mma && !plan.captured ? &list : nullptr;   // merge_splits_kernel reads the plan from device memory
-  // The stream partition depends on the cached lengths only, the absorb on the queries only: the one-block builder
-  // runs on the side stream next to the absorb kernel and is joined before the decode kernel.
-  cudaStream_t side = p->dev->side_stream;
   const bool fused_prep = step != nullptr;   // the caller checked mla_step_fusable
-  const bool fork = sm100 && side != nullptr && !fused_prep;
+  const bool chained = p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0;
+  // persistent CTA pairs over a stream partition; ranges are whole 128-token tiles
+  rc = sm100 ? plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, fused_prep ? to_list : nullptr)
+             : plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
+  if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
+  if (rc) return rc;
   if (fused_prep) {
     // one launch: absorb + the step's append + the stream partition (the host lengths already count the new rows)
-    rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, st, false, to_list);
-    if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
-    if (rc) return rc;
     PrepAppend ap;
     ap.table = p->d_table;
     ap.table_stride = prm.max_pages_per_seq;
@@ -335,18 +334,18 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     pl.chunk_off = plan.chunk_off;
     pl.worker_first = plan.worker_first;
     rc = launch_mla_prep(p->dev, d_q, d_qr, a.q_dtype == RELUX_DTYPE_BF16, (const uint16_t*)a.w_uk, (uint16_t*)p->q_abs.p, rows, H, dC, dHR, step->weights_ready, ap,
-                         pl, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
+                         pl, chained);
     if (rc) return rc;
-  }
-  if (fork) {
-    RELUX_CUDA_TRY(cudaEventRecord(p->dev->ev_fork, st));
-    RELUX_CUDA_TRY(cudaStreamWaitEvent(side, p->dev->ev_fork, 0));
-    rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, side);
+  } else if (proj_mma && sm100) {
+    // The preparation without rows to append; the partition's builder, which depends on the cached lengths only, works beside it.  On a second
+    // stream, between two events, a call ended at one of the events' turns, 2.05 us apart: two query tokens of 16 x 300 tokens 32.9 us, now 26.8,
+    // of 24 x 700 37.1 and 31.3, four of 1 x 2600 30.9 and 26.2, of 3 x 1500 33.9 and 29.4.
+    PrepAppend ap{};
+    PrepPlan pl{};
+    ap.status = p->d_status;
+    pl.listed = 1;   // no chores
+    rc = launch_mla_prep(p->dev, d_q, d_qr, a.q_dtype == RELUX_DTYPE_BF16, (const uint16_t*)a.w_uk, (uint16_t*)p->q_abs.p, rows, H, dC, dHR, false, ap, pl, chained);
     if (rc) return rc;
-    RELUX_CUDA_TRY(cudaEventRecord(p->dev->ev_join, side));
-  }
-  if (fused_prep) {
-    // absorbed queries, appended rows and the partition are already queued
   } else if (proj_mma) {
     rc = launch_mla_absorb_mma(p->dev, d_q, d_qr, a.q_dtype == RELUX_DTYPE_BF16, (const uint16_t*)a.w_uk, (uint16_t*)p->q_abs.p, rows, H, dC,
                                dHR, p->d_status);
@@ -360,15 +359,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     RELUX_CUDA_TRY(cudaGetLastError());
     count_launch(p->dev);
   }
-  if (fused_prep) {
-  } else if (fork)
-    RELUX_CUDA_TRY(cudaStreamWaitEvent(st, p->dev->ev_join, 0));
-  else if (sm100)   // persistent CTA pairs over a stream partition; ranges are whole 128-token tiles
-    rc = plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, st);
-  else
-    rc = plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
-  if (rc) return rc;
-  if ((rc = grow_partials(p, plan, rows_total, dC))) return rc;
+  if (sm100 && !fused_prep && (rc = launch_build_stream(p, sb, a.layer, a.extra_tokens, plan, chained))) return rc;
   if (!proj_mma) {   // the unfused path hands the merged latent output to the up-projection through this buffer
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));
     if (rc) return rc;
@@ -423,7 +414,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   if (proj_mma) {
     // the split-KV merge is part of the up-projection: the merged latent output never touches memory
     rc = launch_mla_vup_pieces(p->dev, p->part_o.p, (const float*)p->part_ml.p, plan, form, !sm100, (const uint16_t*)a.w_uv, d_out, out_bf16, rows, S,
-                               H, dC, p->d_status, p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0);
+                               H, dC, p->d_status, chained);
     if (rc) return rc;
   } else {
     rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, (float*)p->o_lat.p);

@@ -732,12 +732,6 @@ API int32_t relux_cuda_device_open(int32_t device_index, relux_device_t* out) {
   snprintf(d->name, sizeof(d->name), "%s", prop.name);
   e = cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete d; return cuda_fail(e, "cudaStreamCreate"); }
-  if (cudaStreamCreateWithFlags(&d->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&d->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&d->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-    (void)cudaGetLastError();   // the side stream is an optimisation: without it the kernels stay on the main stream
-    d->side_stream = nullptr;
-  }
   if (cudaStreamCreateWithFlags(&d->h2d_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&d->d2h_stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&d->ev_copy_join, cudaEventDisableTiming) != cudaSuccess) {
@@ -766,9 +760,6 @@ API int32_t relux_cuda_device_close(relux_device_t h) {
     if (dev->flush_buf) cudaFree(dev->flush_buf);
     if (dev->host_out) cudaFreeHost(dev->host_out);
     if (dev->host_in) cudaFreeHost(dev->host_in);
-    if (dev->side_stream) { cudaStreamSynchronize(dev->side_stream); cudaStreamDestroy(dev->side_stream); }
-    if (dev->ev_fork) cudaEventDestroy(dev->ev_fork);
-    if (dev->ev_join) cudaEventDestroy(dev->ev_join);
     for (cudaStream_t st : {dev->h2d_stream, dev->d2h_stream})
       if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
     if (dev->ev_copy_join) cudaEventDestroy(dev->ev_copy_join);

@@ -145,17 +145,20 @@ __device__ __forceinline__ int block_excl_scan(int v, int32_t* s_warp, int* tota
 // Stream partition (see plan_stream): sequence i occupies pages [start_i, start_i + pages_i) of the stream and
 // is cut at every multiple of G; items are numbered in stream order, so the items of a sequence and the items of
 // a worker are both contiguous.
+// Behind the preparation's absorb it works beside it, and waits at its end only: the lengths and the last plan's readers are older than
+// that head of the chain.
 __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
                                     int page_tokens, int G, int workers, int by_item, int start_units,
                                     StreamItem* __restrict__ items, int32_t* __restrict__ chunk_off, int32_t* __restrict__ worker_first) {
   __shared__ int32_t s_warp[8];
+  chain_release();
   int unit_base = 0, item_base = 0;
   for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
     const int i = i0 + threadIdx.x;
     int seq = 0, pages = 0, tokens = 0;
     if (i < n_seqs) {
       seq = seq_ids ? seq_ids[i] : i;
-      tokens = len[seq] + extra;
+      tokens = load_chained(len + seq) + extra;
       pages = (tokens + page_tokens - 1) / page_tokens;
     }
     int tot_units, tot_items;
@@ -185,6 +188,7 @@ __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32
   if (threadIdx.x == 0) chunk_off[n_seqs] = item_base;
   // ranges past the end of the stream are empty
   for (int w = (by_item ? item_base : (unit_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
+  chain_wait();
 }
 
 // Equal ranges of pages (the tuning knob CHUNK_PAGES, relux_stream_partition): range length G and the counts that follow from it.
@@ -227,8 +231,8 @@ static bool list_plan(const SeqBatch& sb, const std::vector<int>& pages, const i
   return true;
 }
 
-int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
-                    bool launch_builder, ListedPlan* list) {
+int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan,
+                    ListedPlan* list) {
   const relux_pool_params& prm = p->prm;
   std::vector<int> pages(sb.n_seqs);
   for (int i = 0; i < sb.n_seqs; i++) {
@@ -268,11 +272,13 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
   plan->stream_items = (StreamItem*)p->work.p;
   plan->chunk_off = (int32_t*)((char*)p->work.p + off_chunk);
   plan->worker_first = (int32_t*)((char*)p->work.p + off_worker);
-  if (!launch_builder) return RELUX_OK;
-  const int32_t* len = p->d_len + (size_t)layer * prm.max_seqs;
-  build_stream_kernel<<<1, 256, 0, st>>>(len, sb.d_seq_ids, sb.n_seqs, extra, prm.page_tokens, G, workers,
-                                                     plan->by_item ? 1 : 0, plan->start_units, plan->stream_items, plan->chunk_off, plan->worker_first);
-  RELUX_CUDA_TRY(cudaGetLastError());
+  return RELUX_OK;
+}
+
+int32_t launch_build_stream(Pool* p, const SeqBatch& sb, int layer, int extra, const SplitPlan& plan, bool chained) {
+  RELUX_CUDA_TRY(launch_chained(chained, build_stream_kernel, dim3(1), dim3(256), 0, p->dev->stream, p->d_len + (size_t)layer * p->prm.max_seqs, sb.d_seq_ids,
+                                sb.n_seqs, extra, p->prm.page_tokens, plan.chunk_pages, plan.num_workers, plan.by_item ? 1 : 0, plan.start_units,
+                                plan.stream_items, plan.chunk_off, plan.worker_first));
   count_launch(p->dev);
   return RELUX_OK;
 }

@@ -73,12 +73,11 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
 // one item = the part of one sequence inside one range, so a worker meets an item boundary only where a sequence ends inside its
 // range.  Where that is cheaper they are cut sequence by sequence instead, one item a worker (cheapest_plan).  With the tuning knob
 // CHUNK_PAGES: ranges of that many pages, rounded up to `page_multiple`.
-// `st`: the stream the builder kernel is launched on (the pool's main stream, or the device's side stream).
-// launch_builder = false: only the host half (counts, buffers); the caller builds the lists itself (the fused decode-step
-// preparation of mla_proj.cu does it inside its own launch).
+// The host half: counts and buffers.  The lists are built by the fused decode step's preparation (mla_proj.cu), or by
+// launch_build_stream behind a preparation that only absorbs.
 // `list`: where the plan fits there, it is written there and not built on the device.
-int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, cudaStream_t st,
-                    bool launch_builder = true, ListedPlan* list = nullptr);
+int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, ListedPlan* list);
+int32_t launch_build_stream(Pool* p, const SeqBatch& sb, int layer, int extra, const SplitPlan& plan, bool chained);
 int32_t launch_build_worklist_raw(cudaStream_t st, const int32_t* len, const int32_t* seq_ids, int n_seqs, int extra, int page_tokens,
                                   int chunk_pages, WorkItem* items, int32_t* chunk_off);
 int32_t launch_merge_raw(cudaStream_t st, const float* part_o, const float* part_ml, const int32_t* chunk_off, int n_seqs, int rows,
