@@ -79,14 +79,25 @@ struct Tuning {
   int32_t get(int knob) const { return v[knob]; }
 };
 
-// Two device buffers used in turn by pipelined calls.  `ready`: the copy into (inputs) or the kernels writing (outputs)
-// the slot are done; `freed`: whoever read the slot is done with it, so it may be overwritten.
+// Two device buffers used in turn by pipelined calls.  `copied`: the copy into (inputs) or out of (outputs) the slot is done; `reader`: the
+// PipeCalls number of the call whose kernels read an input's slot last.
 struct PipeSlots {
   static constexpr int kSlots = 2;
   GrowBuf buf[kSlots];
-  cudaEvent_t ready[kSlots] = {}, freed[kSlots] = {};
-  bool used[kSlots] = {};
+  cudaEvent_t copied[kSlots] = {};
+  uint64_t reader[kSlots] = {};
+  bool used[kSlots] = {};   // of an output
   uint64_t next = 0;
+};
+
+// The ends of pipelined calls on the compute stream, numbered from 1: one event a call serves all of its buffers.  An event that a later call has
+// recorded again says more than is asked for.
+struct PipeCalls {
+  static constexpr int kEvents = 4;
+  cudaEvent_t done[kEvents] = {};
+  uint64_t last = 0;      // calls recorded
+  uint64_t copies = 0;    // the input copies are behind this one
+  cudaEvent_t of(uint64_t call) const { return done[call % kEvents]; }
 };
 
 // Times of the last kCalls calls.  A call is timed by stamps its kernel writes (one launch: time_stamp_next), or by an
@@ -141,6 +152,7 @@ struct Pool {
   GrowBuf in_a, in_b, out_buf, q_conv;
   GrowBuf expand_buf;  // expanded keys / values of an MLA prompt (+ the sequences' first rows)
   GrowBuf step_rows;   // host-resident new rows of a fused decode step (the attention call uses in_a / in_b for the queries)
+  PipeCalls pipe_calls;
   PipeSlots pipe_in_a, pipe_in_b, pipe_app_a, pipe_app_b, pipe_out;   // the same for pipelined calls
   // attention scratch
   GrowBuf q_abs;     // MLA absorbed queries, bf16 [n][S][H][dC+dHR]
@@ -178,10 +190,13 @@ inline Pool* as_pool(relux_pool_t h) {
 }
 
 int32_t grow(Device* dev, GrowBuf& b, size_t bytes);
-// Pipelined staging: copies a host input into the next slot on the copy stream and makes the compute stream wait for it;
-// pipe_release is called once the kernels that read the slot have been queued.
-int32_t pipe_stage_in(Pool* p, PipeSlots& ps, const void* src, size_t bytes, const void** dptr, int* slot);
-int32_t pipe_release(Pool* p, PipeSlots& ps, int slot);
+// Pipelined staging: copies a host input into the next slot on the copy stream; with `last` the compute stream waits for it, and for the copies
+// before it.  pipe_end is called once the kernels that read a call's slots have been queued, then pipe_release for each of the slots.
+int32_t pipe_stage_in(Pool* p, PipeSlots& ps, const void* src, size_t bytes, bool last, const void** dptr, int* slot);
+int32_t pipe_end(Pool* p);
+inline void pipe_release(Pool* p, PipeSlots& ps, int slot) {
+  if (slot >= 0) ps.reader[slot] = p->pipe_calls.last;
+}
 // Next staging slot (waits for the copy that last used it); call stage_release after the copies are enqueued.
 int32_t stage_acquire(Pool* p, int32_t** slot, int* slot_index);
 int32_t stage_release(Pool* p, int slot_index);

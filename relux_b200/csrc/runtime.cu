@@ -277,9 +277,10 @@ static void pool_free_all(Pool* p) {
   for (PipeSlots* ps : {&p->pipe_in_a, &p->pipe_in_b, &p->pipe_app_a, &p->pipe_app_b, &p->pipe_out})
     for (int i = 0; i < PipeSlots::kSlots; i++) {
       fr(ps->buf[i].p);
-      if (ps->ready[i]) cudaEventDestroy(ps->ready[i]);
-      if (ps->freed[i]) cudaEventDestroy(ps->freed[i]);
+      if (ps->copied[i]) cudaEventDestroy(ps->copied[i]);
     }
+  for (cudaEvent_t e : p->pipe_calls.done)
+    if (e) cudaEventDestroy(e);
   fr(p->storage); fr(p->meta);
   fr(p->in_a.p); fr(p->in_b.p); fr(p->out_buf.p); fr(p->q_abs.p); fr(p->part_o.p); fr(p->part_ml.p); fr(p->work.p); fr(p->stream_done.p); fr(p->seq_list.p);
   fr(p->o_lat.p); fr(p->q_conv.p); fr(p->rope_tab.p); fr(p->layer_buf.p); fr(p->shadow_f32); fr(p->chunk_tab.p); fr(p->step_rows.p); fr(p->expand_buf.p);
@@ -359,9 +360,8 @@ int32_t stage_in(Pool* p, GrowBuf& buf, const void* src, size_t bytes, int mem, 
 
 static size_t dtype_size(int dt) { return dt == RELUX_DTYPE_BF16 ? 2 : 4; }
 
-static int32_t pipe_events(PipeSlots& ps, int slot) {
-  if (!ps.ready[slot]) RELUX_CUDA_TRY(cudaEventCreateWithFlags(&ps.ready[slot], cudaEventDisableTiming));
-  if (!ps.freed[slot]) RELUX_CUDA_TRY(cudaEventCreateWithFlags(&ps.freed[slot], cudaEventDisableTiming));
+static int32_t pipe_event(cudaEvent_t* e) {
+  if (!*e) RELUX_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return RELUX_OK;
 }
 // A slot's buffer may be replaced only when nothing queued on any stream still uses it.
@@ -372,27 +372,37 @@ static int32_t pipe_grow(Pool* p, GrowBuf& b, size_t bytes) {
   if (dev->d2h_stream) RELUX_CUDA_TRY(cudaStreamSynchronize(dev->d2h_stream));
   return grow(dev, b, bytes);
 }
-int32_t pipe_stage_in(Pool* p, PipeSlots& ps, const void* src, size_t bytes, const void** dptr, int* slot) {
+// Small calls are bound by what they queue: with events for each of four inputs and the output a latent step had 20 waits and records, and has 7:
+// 1 x 300 tokens 35.9 -> 31.2 us, 3 x 1500 38.9 -> 28.3, 8 x 1000 33.6 -> 29.3, 24 x 700 with 32 heads 32.1 -> 28.3.
+int32_t pipe_stage_in(Pool* p, PipeSlots& ps, const void* src, size_t bytes, bool last, const void** dptr, int* slot) {
   Device* dev = p->dev;
+  PipeCalls& calls = p->pipe_calls;
   const int s = (int)(ps.next++ % PipeSlots::kSlots);
-  int32_t rc = pipe_events(ps, s);
+  int32_t rc = pipe_event(&ps.copied[s]);
   if (rc) return rc;
   rc = pipe_grow(p, ps.buf[s], bytes);
   if (rc) return rc;
   // the kernels that read this slot two calls ago must be done before the copy overwrites it
-  if (ps.used[s]) RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->h2d_stream, ps.freed[s], 0));
+  if (const uint64_t r = ps.reader[s]; r > calls.copies) {
+    RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->h2d_stream, calls.of(r), 0));
+    calls.copies = calls.last - (calls.last - r) % PipeCalls::kEvents;   // whose end that event is now
+  }
   RELUX_CUDA_TRY(cudaMemcpyAsync(ps.buf[s].p, src, bytes, cudaMemcpyHostToDevice, dev->h2d_stream));
-  RELUX_CUDA_TRY(cudaEventRecord(ps.ready[s], dev->h2d_stream));
-  RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->stream, ps.ready[s], 0));
   dev->copies_in_flight = true;
+  if (last) {
+    RELUX_CUDA_TRY(cudaEventRecord(ps.copied[s], dev->h2d_stream));
+    RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->stream, ps.copied[s], 0));
+  }
   *dptr = ps.buf[s].p;
   *slot = s;
   return RELUX_OK;
 }
-int32_t pipe_release(Pool* p, PipeSlots& ps, int slot) {
-  if (slot < 0) return RELUX_OK;
-  RELUX_CUDA_TRY(cudaEventRecord(ps.freed[slot], p->dev->stream));
-  ps.used[slot] = true;
+int32_t pipe_end(Pool* p) {
+  PipeCalls& calls = p->pipe_calls;
+  const uint64_t call = calls.last + 1;
+  if (int32_t rc = pipe_event(&calls.done[call % PipeCalls::kEvents])) return rc;
+  RELUX_CUDA_TRY(cudaEventRecord(calls.of(call), p->dev->stream));
+  calls.last = call;
   return RELUX_OK;
 }
 // Orders the compute stream after everything queued on the copy streams (used where a caller's event or a full
@@ -466,8 +476,8 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
                                                   : (size_t)sb.total_rows * prm.gqa_num_kv_heads * prm.gqa_head_dim * es;
   const size_t bytes_b = (kind == RELUX_POOL_MLA) ? (size_t)sb.total_rows * prm.mla_dhr * es : bytes_a;
   if (piped) {
-    if ((rc = pipe_stage_in(p, p->pipe_app_a, a->a, bytes_a, &da, &slot_a))) return rc;
-    if ((rc = pipe_stage_in(p, p->pipe_app_b, a->b, bytes_b, &db, &slot_b))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_a, a->a, bytes_a, false, &da, &slot_a))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_b, a->b, bytes_b, true, &db, &slot_b))) return rc;
   } else {
     const void* staged[2];
     stage_small(p, {a->a, a->b}, {bytes_a, bytes_b}, a->mem, staged);
@@ -477,8 +487,9 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
   if (kind == RELUX_POOL_MLA) rc = launch_mla_append(p, sb, a->layer, da, db, a->dtype, a->advance);
   else rc = launch_gqa_append(p, sb, a->layer, da, db, a->dtype, a->layout, a->advance);
   if (rc) return rc;
-  if ((rc = pipe_release(p, p->pipe_app_a, slot_a)) || (rc = pipe_release(p, p->pipe_app_b, slot_b))) return rc;
-  if (rc) return rc;
+  if (piped && (rc = pipe_end(p))) return rc;
+  pipe_release(p, p->pipe_app_a, slot_a);
+  pipe_release(p, p->pipe_app_b, slot_b);
   if (a->advance)
     for (int i = 0; i < sb.n_seqs; i++) {
       int32_t& len = p->h_len[(size_t)a->layer * prm.max_seqs + sb.seq[i]];
@@ -491,6 +502,13 @@ static int32_t do_append(Pool* p, const relux_append_args* a, int kind) {
 // Converts q to the kernels' canonical device form and runs the attention, then delivers `out`.
 int32_t convert_layout(Device* dev, const void* src, void* dst, int n, int S, int H, int D, int src_dtype, int dst_dtype,
                        int src_layout, int dst_layout);
+
+static bool pipes_queries(const Pool* p, const relux_attn_args& a) {
+  return (a.flags & RELUX_CALL_PIPELINED) && p->dev->h2d_stream && p->dev->d2h_stream && a.q_mem == RELUX_MEM_HOST;
+}
+static bool pipes_output(const Pool* p, const relux_attn_args& a) {
+  return (a.flags & RELUX_CALL_PIPELINED) && p->dev->h2d_stream && p->dev->d2h_stream && a.out_mem == RELUX_MEM_HOST;
+}
 
 static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const StepAppend* step = nullptr, const GqaAppend* gstep = nullptr) {
   if (!a) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
@@ -543,12 +561,11 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   const int n = sb.n_seqs, S = a->q_tokens, H = a->num_heads, D = a->head_dim, R = prm.mla_dhr;
   const size_t q_elems = (size_t)n * S * H * D, qr_elems = (size_t)n * S * H * R;
   const void *dq = nullptr, *dqr = nullptr;
-  const bool piped = (a->flags & RELUX_CALL_PIPELINED) != 0 && p->dev->h2d_stream && p->dev->d2h_stream;
-  const bool piped_in = piped && a->q_mem == RELUX_MEM_HOST;
+  const bool piped_in = pipes_queries(p, *a);
   int slot_q = -1, slot_qr = -1;
   if (piped_in) {
-    if ((rc = pipe_stage_in(p, p->pipe_in_a, a->q, q_elems * dtype_size(a->q_dtype), &dq, &slot_q))) return rc;
-    if (kind == RELUX_POOL_MLA && (rc = pipe_stage_in(p, p->pipe_in_b, a->q_rope, qr_elems * dtype_size(a->q_dtype), &dqr, &slot_qr))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_in_a, a->q, q_elems * dtype_size(a->q_dtype), kind != RELUX_POOL_MLA, &dq, &slot_q))) return rc;
+    if (kind == RELUX_POOL_MLA && (rc = pipe_stage_in(p, p->pipe_in_b, a->q_rope, qr_elems * dtype_size(a->q_dtype), true, &dqr, &slot_qr))) return rc;
   } else {
     rc = stage_in(p, p->in_a, a->q, q_elems * dtype_size(a->q_dtype), a->q_mem, &dq);
     if (rc) return rc;
@@ -589,7 +606,7 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   const bool need_conv = a->out_dtype != k_dtype || !out_tm;
   const bool direct = a->out_mem == RELUX_MEM_DEVICE && !need_conv;
   void* kout;
-  const bool piped_out = piped && a->out_mem == RELUX_MEM_HOST;
+  const bool piped_out = pipes_output(p, *a);
   // A small result for host memory: the last kernel writes it to page-locked memory itself (write-only there: the prompt
   // kernels' TMA stores and the reference kernels keep to device memory)
   const size_t out_bytes = out_elems * dtype_size(a->out_dtype);
@@ -602,10 +619,10 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
   else if (piped_out) {
     PipeSlots& po = p->pipe_out;
     slot_out = (int)(po.next++ % PipeSlots::kSlots);
-    if ((rc = pipe_events(po, slot_out))) return rc;
+    if ((rc = pipe_event(&po.copied[slot_out]))) return rc;
     if ((rc = pipe_grow(p, po.buf[slot_out], out_elems * 4 + out_elems * dtype_size(a->out_dtype)))) return rc;
     // the copy that last read this slot (two pipelined calls ago) must have finished before the kernels overwrite it
-    if (po.used[slot_out]) RELUX_CUDA_TRY(cudaStreamWaitEvent(p->dev->stream, po.freed[slot_out], 0));
+    if (po.used[slot_out]) RELUX_CUDA_TRY(cudaStreamWaitEvent(p->dev->stream, po.copied[slot_out], 0));
     out_block = (char*)po.buf[slot_out].p;
     kout = out_block;
   } else {
@@ -626,22 +643,25 @@ static int32_t do_attention(Pool* p, const relux_attn_args* a, int kind, const S
     rc = (kind == RELUX_POOL_MLA) ? launch_mla_decode_fast(p, sb, aa, dq, dqr, kout, k_bf16, step) : launch_gqa_decode_fast(p, sb, aa, dq, kout);
   }
   if (rc) return rc;
-  if ((rc = pipe_release(p, p->pipe_in_a, slot_q)) || (rc = pipe_release(p, p->pipe_in_b, slot_qr))) return rc;
+  const void* src = kout;
   if (!direct) {
-    const void* src = kout;
     if (need_conv) {
       void* dst = (a->out_mem == RELUX_MEM_DEVICE) ? a->out : by_kernel ? p->dev->host_out : out_block + out_elems * 4;
       rc = convert_layout(p->dev, kout, dst, n, S, H, D, RELUX_DTYPE_F32, a->out_dtype, RELUX_LAYOUT_TOKEN_MAJOR, a->out_layout);
       if (rc) return rc;
       src = dst;
     }
+  }
+  if ((piped_in || piped_out) && (rc = pipe_end(p))) return rc;
+  pipe_release(p, p->pipe_in_a, slot_q);
+  pipe_release(p, p->pipe_in_b, slot_qr);
+  if (!direct) {
     if (piped_out) {
       PipeSlots& po = p->pipe_out;
       Device* dev = p->dev;
-      RELUX_CUDA_TRY(cudaEventRecord(po.ready[slot_out], dev->stream));
-      RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->d2h_stream, po.ready[slot_out], 0));
+      RELUX_CUDA_TRY(cudaStreamWaitEvent(dev->d2h_stream, p->pipe_calls.of(p->pipe_calls.last), 0));
       RELUX_CUDA_TRY(cudaMemcpyAsync(a->out, src, out_elems * dtype_size(a->out_dtype), cudaMemcpyDeviceToHost, dev->d2h_stream));
-      RELUX_CUDA_TRY(cudaEventRecord(po.freed[slot_out], dev->d2h_stream));
+      RELUX_CUDA_TRY(cudaEventRecord(po.copied[slot_out], dev->d2h_stream));
       po.used[slot_out] = true;
       dev->copies_in_flight = true;
     } else if (by_kernel) {
@@ -1226,7 +1246,7 @@ API int32_t relux_pool_wait_output(relux_pool_t h, int32_t calls_back) {
     return RELUX_ERR_INVALID_ARG;
   }
   const int slot = (int)((po.next - 1 - (uint64_t)calls_back) % PipeSlots::kSlots);
-  if (po.used[slot]) RELUX_CUDA_TRY(cudaEventSynchronize(po.freed[slot]));
+  if (po.used[slot]) RELUX_CUDA_TRY(cudaEventSynchronize(po.copied[slot]));
   return RELUX_OK;
 }
 
@@ -1291,8 +1311,8 @@ static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_at
   const void *da = kv->a, *db = kv->b;
   int slot_a = -1, slot_b = -1;
   if (piped) {
-    if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes, &da, &slot_a))) return rc;
-    if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes, &db, &slot_b))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes, false, &da, &slot_a))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes, !pipes_queries(p, *attn), &db, &slot_b))) return rc;
   } else if (kv->mem == RELUX_MEM_HOST) {
     // the attention call stages q in in_a: the step's rows get a block of their own
     const size_t off_b = (bytes + 255) & ~(size_t)255;
@@ -1321,7 +1341,9 @@ static int32_t do_gqa_fused(Pool* p, const relux_append_args* kv, const relux_at
     set_error("%s", why);
     return rc;
   }
-  if ((rc = pipe_release(p, p->pipe_app_a, slot_a)) || (rc = pipe_release(p, p->pipe_app_b, slot_b))) return rc;
+  if (piped && !pipes_queries(p, *attn) && !pipes_output(p, *attn) && (rc = pipe_end(p))) return rc;   // else the attention call's end is this one's
+  pipe_release(p, p->pipe_app_a, slot_a);
+  pipe_release(p, p->pipe_app_b, slot_b);
   return RELUX_OK;
 }
 static bool gqa_fuse_args_ok(const Pool* p, const relux_append_args* kv, const relux_attn_args* attn) {
@@ -1385,8 +1407,8 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   const void *da = nullptr, *db = nullptr;
   int slot_a = -1, slot_b = -1;
   if (piped) {
-    if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes_a, &da, &slot_a))) return rc;
-    if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes_b, &db, &slot_b))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes_a, false, &da, &slot_a))) return rc;
+    if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes_b, !pipes_queries(p, *attn), &db, &slot_b))) return rc;
   } else if (kv->mem == RELUX_MEM_HOST) {
     // the attention call stages q / q_rope in in_a / in_b: the step's rows get a block of their own
     if ((rc = grow(p->dev, p->step_rows, bytes_a + bytes_b + 256))) return rc;
@@ -1408,7 +1430,9 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
     take_rows_back(p, sb, kv->layer);
     return rc;
   }
-  if ((rc = pipe_release(p, p->pipe_app_a, slot_a)) || (rc = pipe_release(p, p->pipe_app_b, slot_b))) return rc;
+  if (piped && !pipes_queries(p, *attn) && !pipes_output(p, *attn) && (rc = pipe_end(p))) return rc;   // else the attention call's end is this one's
+  pipe_release(p, p->pipe_app_a, slot_a);
+  pipe_release(p, p->pipe_app_b, slot_b);
   return RELUX_OK;
 }
 API int32_t relux_mla_step(relux_pool_t h, const relux_append_args* kv, const relux_attn_args* attn) {
