@@ -111,12 +111,19 @@ constexpr uint32_t kTmemS = 0, kTmemO = 256;                  // S(g) at kTmemS 
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kPolyPairsOf8 = 2;   // score pairs out of every eight whose exponential runs on the FMA pipe
 
+// What the softmax warps need to know of an item, worked out for them by a read-out warp.  They are the busiest; when all eight worked the next
+// item out for themselves and added a row's four sums up by shuffles, an item's end took them 820 clocks, 28 times in a prompt of 424 k (473 and 88 of
+// them for these two): 8 x 2048 tokens 332.7 -> 326.7 us, 2 x 8192 1058 -> 1044, MLA 4 x 1000 364.6 -> 359.6.
+struct alignas(16) SoftmaxItem {
+  int32_t ntiles, T, pair, more;
+};
 struct Bars {
   uint64_t q_full[2], q_empty[2], k_full[kMaxDepth], k_empty[kMaxDepth], v_full[kMaxDepth], v_empty[kMaxDepth], s_full[2], p_full[2];
   uint64_t o_full[2], o_empty[2], l_full, l_empty, drain;
   uint32_t tmem_base;
   volatile int32_t abort_flag;
-  float lsum[128];                // an item's row sums, handed to the read-out warps
+  alignas(16) float lsum[128][4];   // an item's row sums, of a row's four lanes, handed to the read-out warps
+  SoftmaxItem items[4];           // item n's at n & 3, written by a read-out warp
 };
 static_assert(sizeof(Bars) <= 3072, "barrier block too large");
 
@@ -470,10 +477,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int tq[2] = {row[0] / prm.g, row[1] / prm.g};              // token in block
     const uint64_t scale2 = pack2(prm.scale_log2, prm.scale_log2);
     int g = 0;
-    Walk<kMla> w(prm, worker, n_workers);
-    do {
-      const Item it = w.it;
-      const int n = w.n;
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * (kSoftmaxWarps + 1)) : "memory");   // the first two items are there
+    SoftmaxItem it = bars->items[0];
+    for (int n = 0;; n++) {
       const int t0 = (2 * it.pair + (int)rank) * prm.bq;          // first query token of this CTA's block
       // keys [0, t_eff) are visible to a row; counted from this lane's first key of a tile
       int t_lane[2];
@@ -582,15 +588,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         if (lane == 0) mbar_arrive_cluster(p_full_lead + (g & 1) * 8);
       }
       // ---- end of the item: the row sums go to the read-out warps ----
-#pragma unroll
-      for (int o = 1; o < 4; o <<= 1)
-#pragma unroll
-        for (int k = 0; k < 2; k++) l_run[k] += __shfl_xor_sync(0xffffffffu, l_run[k], o);
       if (n > 0) wait_bar(&bars->l_empty, (n - 1) & 1, bars, prm.status);   // the read-out of the previous item has taken its sums
-      if ((lane & 3) < 2) bars->lsum[row[lane & 1]] = (lane & 1) ? l_run[1] : l_run[0];
+#pragma unroll
+      for (int k = 0; k < 2; k++) bars->lsum[row[k]][lane & 3] = l_run[k];
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->l_full);
-    } while (w.next());
+      if (!it.more || *(volatile uint32_t*)&bars->abort_flag) break;   // after an abort no more items are written
+      it = bars->items[(n + 1) & 3];
+    }
   } else {
     // =============================== read-out: O / l -> out ===============================
     // One warp per TMEM lane quarter; item n's accumulator is O buffer n & 1, handed over by the commit behind the
@@ -606,13 +611,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     constexpr int kOutCols = PL::kOutCols;
     uint8_t* tile = smem + PL::kSmemOut + wq * PL::kOutTile;
     if (lane == 0) tma_prefetch_desc(&tmap_out);
-    Walk<kMla> w(prm, worker, n_workers);
+    Walk<kMla> w(prm, worker, n_workers), ahead = w;   // the first warp also walks for the softmax warps, two items ahead
+    auto put_item = [&] {
+      if (lane == 0) bars->items[ahead.n & 3] = SoftmaxItem{ahead.it.ntiles, ahead.it.T, ahead.it.pair, ahead.more};
+      __syncwarp();
+      ahead.next();
+    };
+    if (wq == 0) {
+      put_item();
+      put_item();
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * (kSoftmaxWarps + 1)) : "memory");
+    }
     do {
       const Item it = w.it;
       const int n = w.n;
       const int t0 = (2 * it.pair + (int)rank) * prm.bq + wq * 32 / prm.g;   // first query token of the warp's rows
       wait_bar(&bars->l_full, n & 1, bars, prm.status);
-      const float l_row = bars->lsum[r];
+      const float4 l4 = *reinterpret_cast<const float4*>(bars->lsum[r]);
+      const float l_row = (l4.x + l4.y) + (l4.z + l4.w);
+      if (wq == 0) put_item();   // of item n + 2, for whoever has waited for l_empty(n)
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->l_empty);
       wait_bar(&bars->o_full[n & 1], (n >> 1) & 1, bars, prm.status);
