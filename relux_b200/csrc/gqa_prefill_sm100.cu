@@ -221,10 +221,10 @@ struct Walk {
 
 // exp2(score * scale - max) for a thread's 2 x 32 scores of a tile (tmem_ld_16x256b_x16: pairs of neighbouring keys of rows a and
 // b in turn): bf16 P values in the order of tmem_st_16x128b_x16; the partial row sums are added to ps2.
-template <bool kPoly>
+template <bool kPoly, int kFrom = 0, int kTo = 32>
 __device__ __forceinline__ void exp_quads(const uint32_t (&sv)[64], uint64_t scale2, const uint64_t (&neg_m2)[2], uint32_t (&pw)[32], uint64_t (&ps2)[2]) {
 #pragma unroll
-  for (int i = 0; i < 32; i++) {   // pair i: row i & 1
+  for (int i = kFrom; i < kTo; i++) {   // pair i: row i & 1, of the eight keys from 8 (i >> 1)
     const uint64_t x2 = fma2(pack2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), scale2, neg_m2[i & 1]);
     uint64_t p2;
     if (kPoly && (i & 7) < kPolyPairsOf8) {
@@ -552,10 +552,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         // P(g), packed to bf16, goes over the first 64 columns of S(g): the rows' scores are in registers, and QK(g+2), which
         // writes this S buffer again, is issued behind PV(g).  kPolyPairsOf8 pairs of every eight take the polynomial; a warp
-        // with a masked key in the tile (the diagonal tiles only) keeps to ex2(-inf) = 0 exactly.
+        // with a masked key in the tile (the diagonal tiles only) keeps to ex2(-inf) = 0 exactly, and leaves the tile's second half out
+        // where none of its rows sees it: 8 x 2048 tokens 325.3 -> 322.1 us, 8 x 100 behind 1500 41.0 -> 40.1, MLA 4 x 1000 356.8 -> 353.9.
         uint32_t pw[32];
         if (whole) exp_quads<true>(sv, scale2, neg_m2, pw, ps2);
-        else exp_quads<false>(sv, scale2, neg_m2, pw, ps2);
+        else {
+          exp_quads<false, 0, 16>(sv, scale2, neg_m2, pw, ps2);
+          if (__any_sync(0xffffffffu, nv1 > kTile / 2)) {
+            exp_quads<false, 16, 32>(sv, scale2, neg_m2, pw, ps2);
+          } else {
+#pragma unroll
+            for (int i = 16; i < 32; i++) pw[i] = 0;
+          }
+        }
         tmem_st_16x128b_x16(tmem_s, pw);
 #pragma unroll
         for (int k = 0; k < 2; k++) {
