@@ -660,10 +660,10 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
   return s.tc ? launch(mla_prep_kernel<true>, kAbsorbThreads, kAbsorbSmemMost) : launch(mla_prep_kernel<false>, kAbsorbMmaThreads, kAbsorbMmaSmem);
 }
 
-// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU, more where they do not and there are more than 40 columns, of
+// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU, more where they do not and there are more than 40 columns (52 where only two groups fit), of
 // about 32 columns each, or where a group would have more columns than it has room for.  (One group -> two of 24 to 32: 32 heads, 16 x 300 tokens 17.9
-// -> 16.5 us, 10 x 600 18.0 -> 16.8, 50 x 600 26.9 -> 25.3, 64 heads, 30 x 800 26.4 -> 25.6; the other way 64 heads, 12 x 900 21.4 -> 22.1; at 36
-// columns, 32 heads, 12 x 300 15.6 -> 17.2.)  A group's columns are one block where a stage of it, 64 latent columns,
+// -> 16.5 us, 10 x 600 18.0 -> 16.8, 50 x 600 26.9 -> 25.3, 64 heads, 30 x 800 26.4 -> 25.6; not at 48 columns of 64 heads, 12 x 900 21.4 -> 22.1, nor
+// at 36 of 32, 12 x 300 15.6 -> 17.2.)  A group's columns are one block where a stage of it, 64 latent columns,
 // fits the ring four times, and equal blocks otherwise.
 int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, int form, bool natural, const uint16_t* W_UV,
                               void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
@@ -673,7 +673,8 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   };
   const int more = plan.captured ? std::max(0, plan.room_items - plan.num_items) * S : 0;   // columns that a graph may find
   const int all = col_of(rows) + more;
-  int groups = std::max(1, std::min({dev->sm_count / H, (all + 23) / 32, rows}));
+  const int fit = dev->sm_count / H;
+  int groups = std::max(1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}));
   VupParams k;
   int most = 0;
   for (;; groups++) {

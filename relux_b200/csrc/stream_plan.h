@@ -39,17 +39,17 @@ struct SeqCut {
 };
 
 // What a plan costs, in tiles of two pages (1.1 us at 32 heads, 1.3 at 128): its slowest worker's tiles and two for every item (start and
-// write-out); 0.025 for every partial of the call and 0.04 for every one of the longest row (the up-projection's columns); 1.4 where a row has
-// more than one, for then all come as two halves, where single ones are written and read as one; and 0.25 where a worker has several.
-// Fit to forced plans of 49 batches of 1 to 64 sequences at 32, 64 and 128 heads (one query token): the plan taken is on average 0.3 % slower
-// than the best one found, where 0.035, 0.08, 0 and 0 were off by 1.2 % and by up to 11 %.
-inline double plan_cost(double worst, int most_items, int items, bool split, bool shared) {
-  return worst + 0.04 * most_items + 0.025 * items + (split ? 1.4 : 0) + (shared ? 0.25 : 0);
-}
+// write-out), 0.035 for every partial of the call and 0.02 for every one of the longest row.  Fit to forced plans of 49 batches of 1 to 64
+// sequences at 32, 64 and 128 heads (one query token); with 0.08 for the longest row's, from when the partials of a row were added up by loads,
+// 1 x 2600 tokens took 21.3 us instead of 21.0, with 32 heads 16.4 instead of 15.3.
+// A call in which every sequence has one piece is 1.4 tiles cheaper than this says (its partials are written and read as one half).  Not counted:
+// P starts from one maximum then, and the sum is rounded, so that such a call is up to 2.4 % further from float64 than the same one in pieces was
+// when those were merged (16 x 300 2.33e-3 -> 2.39e-3; in pieces it is 1.65e-3 now), for 4 to 9 % of a step's time.
+inline double plan_cost(double worst, int most_items, int items) { return worst + 0.02 * most_items + 0.035 * items; }
 
 // The cheapest plan of a call: equal ranges of the sequences laid end to end, each counted as its pages and kStartUnits, for a worker
 // that starts it has a second item to start and to write out; or every sequence cut by itself into pieces of 2 t pages, a worker each.
-// Measured, ranges forced -> this, one build: 1 x 1300 tokens 23.3 -> 20.2 us, 3 x <= 1500 24.3 -> 21.7, 16 x 300 26.3 -> 22.3, 64 x 1000 46.3
+// Measured, ranges forced -> this, one build: 1 x 1300 tokens 23.3 -> 20.2 us, 3 x <= 1500 24.3 -> 21.7, 16 x 300 26.3 -> 23.3, 64 x 1000 46.3
 // -> 39.4, 64 x 4096 93.2 -> 84, with 32 heads 1 x 1300 18.5 -> 15.1, 64 x 1000 34.5 -> 31.7; no difference beyond the runs' own at 16 x 2000
 // (30.1), 20 x 8000 (64), 16 x <= 32768 and, with 32 heads, 40 x <= 2500 (31.0).
 constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for an item
@@ -86,7 +86,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   }
   r.room = r.items;
   if (live == 0 || live > workers) return r;
-  double best = plan_cost(worst, most, r.items, r.items > live, r.items > r.workers);
+  double best = plan_cost(worst, most, r.items);
   auto items_of = [&](int t) {
     int items = 0;
     for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
@@ -98,9 +98,9 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
     if (items_of(t) <= workers) hi = t;
     else lo = t + 1;
   }
-  for (int k = 0; k < 4; k++) {   // some more tiles each may leave fewer partials, or one a sequence
-    const int t = k < 3 ? lo + k : (longest + 1) / 2, items = items_of(t);
-    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items, items > live, false);
+  for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
+    const int items = items_of(t);
+    const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
     r.room = std::max(r.room, items);
     if (cost < best) {
       best = cost;
