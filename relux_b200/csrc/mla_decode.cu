@@ -6,6 +6,7 @@
 //               (mla_decode_sm100.cu when the shape is the tensor-core one, else mla_decode_generic_kernel)
 //   merge the chunks of every sequence                                   (merge_splits_kernel)
 //   out[row][h] = W_UV_h^T O_lat[row][h]                                  (mla_vup_kernel)
+// The tensor-core shapes up-project the chunks as they are and add the results up (mla_vup_pieces_kernel, mla_proj.cu).
 //
 // This replaces the reference's "decompress every cached latent, then attend" (mla.go:323-377): the cache
 // row (dC + dHR values, shared by all heads) is read once per token instead of being expanded to
@@ -412,7 +413,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   }
   count_launch(p->dev);
   if (proj_mma) {
-    // the split-KV merge is part of the up-projection: the merged latent output never touches memory
+    // the up-projection takes the partial results as they are: a merged latent output never exists
     rc = launch_mla_vup_pieces(p->dev, p->part_o.p, (const float*)p->part_ml.p, plan, form, !sm100, (const uint16_t*)a.w_uv, d_out, out_bf16, rows, S,
                                H, dC, p->d_status, chained);
     if (rc) return rc;
