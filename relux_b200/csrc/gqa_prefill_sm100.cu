@@ -36,8 +36,9 @@
 // SM (1024 clocks per tile, as long as the tile's MMAs), so two pairs of every eight take a cubic on the FMA pipe instead
 // (three: the same within 1 %, four: 2 % slower), arithmetic runs two lanes per instruction (fma.f32x2, add.f32x2) and the row
 // maximum takes two scores per instruction (three-input max).
-// What bounds it (clock stamps, 8 x 2048 tokens, 32 heads over 8): a tile takes 1740 clocks, 1000 of them exponentials of two
-// warps per scheduler in step, 330 the maxima, the rest waits and tensor-memory round trips; between two items 1000-2400 more.
+// What bounds it (clock stamps, 8 x 2048 tokens, 32 heads over 8): a tile takes 1690 clocks, 1000 of them exponentials of two
+// warps per scheduler in step, 300 the maxima, the rest waits and tensor-memory round trips; an item's end took 820 more before a
+// read-out warp worked the next one out (SoftmaxItem).
 // Measured, 8 x 2048 GQA and 4 x 1000 MLA tokens (this launch): rows shared by two warps, stored a row per lane 343 and 274 us;
 // output by TMA 317 and 251; 16 rows per warp without a barrier, items walked by digits 307 and 235; the vote before the
 // shuffles and two pairs of eight 303 and 229.  Not kept: the two halves of the softmax warps on alternate tiles, a whole row
@@ -467,7 +468,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   } else if (warp < kSoftmaxWarps) {
     // =============================== softmax / correction ===============================
     // Warp w reads TMEM lanes 32 (w & 3) .. +31 (the hardware's rule), of which warps w and w + 4 take 16 rows each.  The loads
-    // give four lanes a row (two neighbouring keys of every eight each), so a row's maximum and sum meet by shuffles and no warp
+    // give four lanes a row (two neighbouring keys of every eight each), so a row's maximum meets by shuffles, its sum when it is read out, and no warp
     // waits for another: with a row shared by two warps the maxima went through shared memory and a barrier in every tile, and
     // shared memory answers slowly while the MMAs read their operands from it.
     const int r16 = (warp & 3) * 32 + (warp >> 2) * 16;
