@@ -99,7 +99,9 @@ int32_t relux_cuda_device_info(relux_device_t dev, char* name, int32_t name_len,
  * in the reference. */
 int32_t relux_cuda_launch_count(relux_device_t dev, int64_t* count);
 /* The CUDA stream (cudaStream_t) all work of this handle is issued on, for callers that order their own device work
- * with it.  No counterpart in the reference. */
+ * with it.  Where a caller captures calls on it, a launch of the graph runs with, and changes, the lengths that the device has
+ * then; the host's (relux_seq_len, capacity checks) know of the calls alone.  A latent decode, verify or step call on a pool on which a
+ * call that changes lengths has been captured runs with the device's lengths as well.  No counterpart in the reference. */
 int32_t relux_cuda_stream(relux_device_t dev, void** stream);
 
 /* ---- device memory ------------------------------------------------------------------------

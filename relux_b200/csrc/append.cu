@@ -213,6 +213,7 @@ static int32_t launch_append(Pool* p, Kernel kernel, dim3 grid, int threads, Arg
 }
 
 int32_t launch_mla_append(Pool* p, const SeqBatch& sb, int layer, const void* ckv, const void* kr, int dtype, int advance) {
+  if (advance) note_lengths_change(p);
   AppendGeom g = make_geom(p, sb, layer, advance);
   uint16_t* base = p->storage + (size_t)layer * p->layer_elems;
   dim3 grid(sb.n_seqs, row_slices(sb));
@@ -235,6 +236,7 @@ int32_t launch_gqa_append(Pool* p, const SeqBatch& sb, int layer, const void* k,
 }
 
 int32_t launch_set_len(Pool* p, const SeqBatch& sb, int layer0, int layers, const int32_t* new_len) {
+  note_lengths_change(p);
   SetLenParams k;
   k.len = p->d_len + (size_t)layer0 * p->prm.max_seqs;
   k.layers = layers;

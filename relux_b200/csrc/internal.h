@@ -124,6 +124,7 @@ struct Pool {
   int32_t* d_len = nullptr;     // [num_layers][max_seqs]
   int32_t* d_status = nullptr;   // [0] status word, [1] block counter of the append kernels
   std::vector<int32_t> h_table, h_len;
+  bool graph_lengths = false;   // a call that changes lengths was captured: launches of the graph change the device's alone, h_len may be older
   std::vector<int32_t> seq_pages;  // pages reserved per sequence (capacity), 0 = slot not live
   std::vector<uint8_t> seq_owned;  // 1 = table rows were filled by relux_seq_alloc
   bool caller_tables = false;      // relux_pool_set_tables filled the tables: the free list stays unused until a reset
@@ -279,6 +280,10 @@ int32_t check_dev_align(const void* ptr, const char* what);
 
 // Whether what the call launches now is recorded in a graph: it then runs with the device's lengths of later moments, not with the host's.
 bool stream_captured(const Device* dev);
+// Of a call that changes lengths of a latent pool.
+inline void note_lengths_change(Pool* p) {
+  if (p->prm.kind == RELUX_POOL_MLA && !p->graph_lengths && stream_captured(p->dev)) p->graph_lengths = true;
+}
 
 // Tensor maps (runtime.cu).  bf16 elements, 128-byte swizzle, no out-of-bounds fill value (zeros); false when the driver
 // entry point is missing or refuses the map.

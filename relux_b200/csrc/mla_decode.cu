@@ -293,8 +293,9 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   ListedPlan list;                     // read where `listed` says so
   list.listed = 0;
   list.new_rows = step ? step->max_rows : 0;
-  plan.captured = stream_captured(p->dev);
-  ListedPlan* const to_list = proj_mma && !plan.captured ? &list : nullptr;   // merge_splits_kernel reads the plan from device memory
+  if (step) note_lengths_change(p);
+  plan.loose = p->graph_lengths || stream_captured(p->dev);
+  ListedPlan* const to_list = proj_mma && !plan.loose ? &list : nullptr;   // merge_splits_kernel reads the plan from device memory
   const bool fused_prep = step != nullptr;   // the caller checked mla_step_fusable
   const bool chained = p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0;
   // persistent CTA pairs over a stream partition; ranges are whole 128-token tiles
@@ -366,7 +367,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     if (rc) return rc;
   }
   // rows of one piece each are rounded where they are written
-  const bool split = !sm100 || plan.captured || plan.num_items > sb.n_seqs || [&] {
+  const bool split = !sm100 || plan.loose || plan.num_items > sb.n_seqs || [&] {
     for (int i = 0; i < sb.n_seqs; i++)
       if (plan.first[i + 1] - plan.first[i] > 1) return true;
     return false;

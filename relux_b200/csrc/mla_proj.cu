@@ -671,7 +671,7 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
     const int i = row / S, q = row - i * S;
     return q == 0 ? plan.first[i] * S : plan.first[i] * S + q * (plan.first[i + 1] - plan.first[i]);
   };
-  const int more = plan.captured ? std::max(0, plan.room_items - plan.num_items) * S : 0;   // columns that a graph may find
+  const int more = plan.loose ? std::max(0, plan.room_items - plan.num_items) * S : 0;   // columns that the launch may find
   const int all = col_of(rows) + more;
   const int fit = dev->sm_count / H;
   int groups = std::max(1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}));
@@ -685,7 +685,7 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   }
   groups = (rows + k.rows_each - 1) / k.rows_each;
   const int n_seqs = rows / S;
-  k.listed = !plan.captured && n_seqs <= kVupListed && all < 65536;
+  k.listed = !plan.loose && n_seqs <= kVupListed && all < 65536;
   if (k.listed)
     for (int i = 0; i <= n_seqs; i++) k.first[i] = (uint16_t)plan.first[i];
   k.halves = form == kPartialHalves ? 2 : 1;

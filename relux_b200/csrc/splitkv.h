@@ -43,7 +43,8 @@ struct ListedPlan {
 struct SplitPlan {
   int chunk_pages = 0;                 // of a stream plan: pages of a piece, or units of a range
   int num_items = 0;
-  bool captured = false;        // num_items may have become more (up to room_items) when the launch runs: stream_captured
+  bool loose = false;           // made for the host's lengths, but the launches find the device's, which may be others: in a graph, and once a
+                                // graph has changed them (Pool::graph_lengths)
   int room_items = 0;           // partials are given room for as many (num_items, where that is more): StreamShape::room
   WorkItem* items = nullptr;    // device
   int32_t* chunk_off = nullptr; // device [n_seqs + 1]

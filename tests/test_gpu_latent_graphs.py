@@ -1,0 +1,92 @@
+"""Latent calls captured in a graph: its launches run with the lengths that the device has then, and plain calls behind them on the same pool do so
+too, against the same calls, none of them captured, on another pool."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests.test_gpu_attention import dev  # noqa: F401
+from tests.test_gpu_listed_plan import DC, DH, DHR, SCALE, latent_pool
+
+pytestmark = pytest.mark.gpu
+
+
+class Calls:
+    """Steps (S = 1) and decode calls of all sequences of a pool, inputs on the device."""
+
+    def __init__(self, dev, oracle, B, H, S=1):  # noqa: F811
+        from relux_b200 import lib as L
+        rng = np.random.default_rng(B + H)
+        bf = lambda *s: dev.upload(oracle.bf16_from_f32(rng.standard_normal(s).astype(np.float32)))  # noqa: E731
+        self.dev, self.shape, self.S = dev, (B, S, H, DH), S
+        self.q, self.qr, self.c, self.r = bf(B, S, H, DH), bf(B, S, H, DHR), bf(B, DC), bf(B, DHR)
+        self.w = [dev.upload(oracle.bf16_from_f32(rng.standard_normal((DC, H * DH)).astype(np.float32) * 0.02)) for _ in range(2)]
+        self.kw = dict(q_rope=self.qr, w_uk=self.w[0], w_uv=self.w[1], q_dtype=L.DTYPE_BF16, out_dtype=L.DTYPE_F32)
+        self.outs = [dev.upload(np.full(self.shape, np.nan, np.float32)) for _ in range(2)]
+
+    def step(self, pool, k):
+        from relux_b200 import lib as L
+        B, _, H, _ = self.shape
+        pool.step(0, B, self.c, self.r, self.q, self.outs[k], H, DH, SCALE, kv_dtype=L.DTYPE_BF16, **self.kw)
+
+    def decode(self, pool, k):
+        B, _, H, _ = self.shape
+        pool.decode(0, B, self.q, self.outs[k], H, DH, SCALE, q_tokens=self.S, **self.kw)
+
+    def same(self, what):
+        self.dev.sync()
+        want, got = (o.download(self.shape, np.float32) for o in self.outs)
+        # the rounding of a row kept in one half, and of P under another cut of the sequences: a few times 1.7e-3 of the result's size, over all values
+        assert np.isfinite(got).all() and np.max(np.abs(want - got)) <= 2e-2 * np.sqrt(np.mean(want ** 2)), what
+
+    def free(self):
+        for b in [self.q, self.qr, self.c, self.r] + self.w + self.outs:
+            b.free()
+
+
+class Graph:
+    def __init__(self, dev, call):  # noqa: F811
+        from relux_b200 import lib as L
+        self.rt, self.stream, self.graph, self.ready = C.CDLL("libcudart.so.12"), C.c_void_p(), C.c_void_p(), C.c_void_p()
+        L.check(dev.lib.relux_cuda_stream(dev.h, C.byref(self.stream)))
+        assert self.rt.cudaStreamBeginCapture(self.stream, 2) == 0
+        call()
+        assert self.rt.cudaStreamEndCapture(self.stream, C.byref(self.graph)) == 0
+        assert self.rt.cudaGraphInstantiate(C.byref(self.ready), self.graph, C.c_ulonglong(0)) == 0
+
+    def launch(self):
+        assert self.rt.cudaGraphLaunch(self.ready, self.stream) == 0
+
+    def free(self):
+        assert self.rt.cudaGraphExecDestroy(self.ready) == 0 and self.rt.cudaGraphDestroy(self.graph) == 0
+
+
+@pytest.mark.parametrize("captured", ["step", "append"])
+@pytest.mark.parametrize("after", ["step", "decode"])
+def test_a_plain_call_behind_launches_of_a_graph(dev, oracle, captured, after):  # noqa: F811
+    """The host has seen one call captured and none launched: the keys that the graph has appended must be attended to all the same."""
+    from relux_b200 import lib as L
+    ctx, H = [70, 300, 130, 40], 16
+    calls = Calls(dev, oracle, len(ctx), H)
+    plain, graphed = (latent_pool(dev, oracle, ctx, 8) for _ in range(2))
+
+    def once(pool, k):
+        if captured == "step":
+            calls.step(pool, k)
+        else:
+            pool.append(0, calls.c, calls.r, len(ctx), dtype=L.DTYPE_BF16)
+    for k, pool in enumerate((plain, graphed)):
+        once(pool, k)
+        calls.decode(pool, k)
+    graph = Graph(dev, lambda: once(graphed, 1))
+    for _ in range(5):
+        once(plain, 0)
+        graph.launch()
+    for k, pool in enumerate((plain, graphed)):
+        (calls.step if after == "step" else calls.decode)(pool, k)
+    calls.same((captured, after))
+    assert plain.status() == 0 and graphed.status() == 0
+    graph.free()
+    plain.destroy()
+    graphed.destroy()
+    calls.free()
