@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "splitkv.h"
+#include "vup_plan.h"
 #include "prep_parts.cuh"
 
 namespace relux {
@@ -29,8 +30,8 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
                         int H, int dC, int dHR, bool weights_ready, const PrepAppend& ap, const PrepPlan& pl, bool chained);
 int32_t launch_mla_absorb_mma(Device* dev, const void* q_nope, const void* q_rope, int q_bf16, const uint16_t* W_UK, uint16_t* q_abs,
                               int rows, int H, int dC, int dHR, int32_t* status);
-int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, int form, bool natural, const uint16_t* W_UV,
-                              void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
+int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, const VupShape& sh, int form, bool natural,
+                              const uint16_t* W_UV, void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained);
 
 namespace {
 
@@ -303,6 +304,21 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
              : plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
   if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
   if (rc) return rc;
+  // rows of one piece each are rounded where they are written
+  const bool split = !sm100 || plan.loose || plan.num_items > sb.n_seqs || [&] {
+    for (int i = 0; i < sb.n_seqs; i++)
+      if (plan.first[i + 1] - plan.first[i] > 1) return true;
+    return false;
+  }();
+  const int form = !proj_mma ? kPartialFloat32 : split ? kPartialHalves : kPartialOne;
+  VupShape vup{};
+  if (proj_mma) {
+    vup = vup_shape(plan.first, rows, S, p->dev->sm_count / H, form == kPartialHalves ? 2 : 1, dC, plan.loose && sm100 ? plan.num_workers : 0);
+    if (!vup.fits()) {
+      set_error("a sequence of this call is cut into more than %d pieces (tuning knobs)", kVupMaxCols);
+      return RELUX_ERR_UNSUPPORTED;
+    }
+  }
   if (fused_prep) {
     // one launch: absorb + the step's append + the stream partition (the host lengths already count the new rows)
     PrepAppend ap;
@@ -329,6 +345,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     pl.listed = list.listed;
     pl.extra = a.extra_tokens;
     pl.G = plan.chunk_pages;
+    pl.room = plan.room_items;
     pl.by_item = plan.by_item ? 1 : 0;
     pl.start_units = plan.start_units;
     pl.workers = plan.num_workers;
@@ -366,13 +383,6 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
     rc = grow(p->dev, p->o_lat, (size_t)rows * H * dC * sizeof(float));
     if (rc) return rc;
   }
-  // rows of one piece each are rounded where they are written
-  const bool split = !sm100 || plan.loose || plan.num_items > sb.n_seqs || [&] {
-    for (int i = 0; i < sb.n_seqs; i++)
-      if (plan.first[i + 1] - plan.first[i] > 1) return true;
-    return false;
-  }();
-  const int form = !proj_mma ? kPartialFloat32 : split ? kPartialHalves : kPartialOne;
   // the decode kernel is timed on every call, or on every Nth (RELUX_TUNE_KERNEL_TIMING_STRIDE)
   const int stride = std::max(1, p->tune.get(RELUX_TUNE_KERNEL_TIMING_STRIDE));
   const bool timed = (p->attn_calls++ % (uint64_t)stride) == 0;
@@ -415,8 +425,8 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   count_launch(p->dev);
   if (proj_mma) {
     // the up-projection takes the partial results as they are: a merged latent output never exists
-    rc = launch_mla_vup_pieces(p->dev, p->part_o.p, (const float*)p->part_ml.p, plan, form, !sm100, (const uint16_t*)a.w_uv, d_out, out_bf16, rows, S,
-                               H, dC, p->d_status, chained);
+    rc = launch_mla_vup_pieces(p->dev, p->part_o.p, (const float*)p->part_ml.p, plan, vup, form, !sm100, (const uint16_t*)a.w_uv, d_out, out_bf16,
+                               rows, S, H, dC, p->d_status, chained);
     if (rc) return rc;
   } else {
     rc = launch_merge(p, plan, sb.n_seqs, rows_total, dC, (float*)p->o_lat.p);

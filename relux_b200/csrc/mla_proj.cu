@@ -13,6 +13,7 @@
 #include "prep_parts.cuh"
 #include "splitkv.h"
 #include "umma.cuh"
+#include "vup_plan.h"
 
 namespace relux {
 
@@ -380,9 +381,7 @@ __global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_
 // decode kernel, and the launches before it have waited for everything older.
 // grid (H, groups of rows), 512 threads: warp 0 loads, warp 1 issues the MMAs, the others work out the weights, all but those write the outputs.
 constexpr int kVupWarps = 16;
-constexpr int kVupMaxCols = 240;                  // columns of a CTA: two of the 512 tensor-memory columns each, in whole blocks
 constexpr int kVupListed = 256;                   // sequences whose first pieces travel as arguments
-constexpr int kVupRing = 96 << 10, kVupMaxStages = 8;
 static_assert(kVupMaxCols >= kMaxRowItems, "a row's pieces are columns of one CTA");
 struct VupParams {
   const float* part_ml;
@@ -390,8 +389,9 @@ struct VupParams {
   void* out;
   int32_t rows, S, H, nk;
   int32_t rows_each;                          // rows of a group (the last may have fewer)
-  int32_t halves, n_block, n_kb, n_stages;    // a stage: n_kb times 64 latent columns of n_block columns, [n_kb][hi | lo][n_block][64], one TMA box
+  int32_t halves, n_block, n_kb, n_stages;    // VupShape; a stage is one TMA box
   int32_t tmem_cols;
+  int32_t room, all;                          // columns that a CTA has room for, and that there are partial results for
   int32_t warm;                               // there are partial results: part_ml may be read, whatever it holds
   int32_t listed;                             // `first` holds chunk_off
   int32_t* status;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
   uint8_t* ring = smem + nk * 32768;                              // [stage], swizzled
   VupShared* sh = reinterpret_cast<VupShared*>(ring + prm.n_stages * stage_bytes);
   float2* info = reinterpret_cast<float2*>(sh->info);
-  const int h = blockIdx.x, r0 = blockIdx.y * prm.rows_each, rows_here = min(prm.rows_each, prm.rows - r0);
+  const int h = blockIdx.x, r0 = blockIdx.y * prm.rows_each, rows_most = min(prm.rows_each, prm.rows - r0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int steps_each = (2 * nk + prm.n_kb - 1) / prm.n_kb;      // stages of a block of columns
   chain_release();
@@ -457,9 +457,17 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
     const int i = S == 1 ? row : row / S, q = row - i * S, c0 = first_of(i);
     return c0 * S + (q == 0 ? 0 : q * (first_of(i + 1) - c0));
   };
+  // None where the device's lengths have made more columns of them than the launch was sized for.
+  auto rows_now = [&]() -> int {
+    if (prm.listed) return rows_most;
+    const int c0 = col_of(r0), c1 = col_of(r0 + rows_most);
+    return c1 - c0 <= prm.room && c1 <= prm.all ? rows_most : 0;
+  };
   if (warp < 2) {
     const bool el = elect_one();
     chain_wait();   // the partial results come from the kernel before this one
+    const int rows_here = rows_now();
+    if (rows_here == 0 && threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     const int col0 = col_of(r0), blocks = (col_of(r0 + rows_here) - col0 + nb - 1) / nb;
     if (warp == 0) {
 #pragma unroll 1
@@ -509,9 +517,10 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
 #pragma unroll 1
   for (int pass = warp >= 2 && prm.warm ? 0 : 1; pass < 2; pass++) {
     const bool real = pass == 1;
-    int col0 = 0, lo = 0, hi = 0;   // first column of the CTA, and columns of the warp's rows
+    int col0 = 0, lo = 0, hi = 0, rows_here = 1;   // first column of the CTA, and columns of the warp's rows
     if (real) {
       if (warp >= 2) chain_wait();
+      rows_here = rows_now();
       const int ra = rows_here * (warp >> 2) / 4, rb = rows_here * ((warp >> 2) + 1) / 4;
       col0 = col_of(r0);
       lo = col_of(r0 + ra) - col0;
@@ -520,12 +529,12 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
     if (warp >= 2) {
       // the weights of a row's pieces, by 32, 8 or 4 lanes
       const int lpr = rows_here <= kVupWarps - 2 ? 32 : rows_here <= 4 * (kVupWarps - 2) ? 8 : 4;
-      const int sub = lane & (lpr - 1), per_pass = (kVupWarps - 2) * (32 / lpr), rows_now = real ? rows_here : 1;
+      const int sub = lane & (lpr - 1), per_pass = (kVupWarps - 2) * (32 / lpr);
 #pragma unroll 1
-      for (int rw = 0; rw < rows_now; rw += per_pass) {
+      for (int rw = 0; rw < rows_here; rw += per_pass) {
         const int r = rw + ((warp - 2) * 32 + lane) / lpr;
         int c = 0, n = 0;
-        if (r < rows_now) {
+        if (r < rows_here) {
           const int i = S == 1 ? r0 + r : (r0 + r) / S, q = r0 + r - i * S, first = first_of(i), pieces = first_of(i + 1) - first;
           n = real ? pieces : 1;
           c = real ? first * S + q * n - col0 : kVupMaxCols + 8;   // no column's place: other warps may be at theirs already
@@ -553,7 +562,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
           const float m = info[c + j].x;
           info[c + j] = make_float2(m == -INFINITY ? 0.f : exp2f(m - M) * inv, __int_as_float(j == n - 1 ? r * H * kDh : -1));
         }
-        if (r < rows_now && n <= 0)   // an empty sequence
+        if (r < rows_here && n <= 0)   // an empty sequence
           for (int d = sub; d < kDh; d += lpr) {
             const size_t off = ((size_t)(r0 + r) * H + h) * kDh + d;
             if (kOutBf16) reinterpret_cast<uint16_t*>(prm.out)[off] = 0;
@@ -660,44 +669,24 @@ int32_t launch_mla_prep(Device* dev, const void* q_nope, const void* q_rope, int
   return s.tc ? launch(mla_prep_kernel<true>, kAbsorbThreads, kAbsorbSmemMost) : launch(mla_prep_kernel<false>, kAbsorbMmaThreads, kAbsorbMmaSmem);
 }
 
-// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU, more where they do not and there are more than 40 columns (52 where only two groups fit), of
-// about 32 columns each, or where a group would have more columns than it has room for.  (One group -> two of 24 to 32: 32 heads, 16 x 300 tokens 17.9
-// -> 16.5 us, 10 x 600 18.0 -> 16.8, 50 x 600 26.9 -> 25.3, 64 heads, 30 x 800 26.4 -> 25.6; not at 48 columns of 64 heads, 12 x 900 21.4 -> 22.1, nor
-// at 36 of 32, 12 x 300 15.6 -> 17.2.)  A group's columns are one block where a stage of it, 64 latent columns,
-// fits the ring four times, and equal blocks otherwise.
-int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, int form, bool natural, const uint16_t* W_UV,
-                              void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
-  auto col_of = [&](int row) {
-    const int i = row / S, q = row - i * S;
-    return q == 0 ? plan.first[i] * S : plan.first[i] * S + q * (plan.first[i + 1] - plan.first[i]);
-  };
-  const int more = plan.loose ? std::max(0, plan.room_items - plan.num_items) * S : 0;   // columns that the launch may find
-  const int all = col_of(rows) + more;
-  const int fit = dev->sm_count / H;
-  int groups = std::max(1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}));
-  VupParams k;
-  int most = 0;
-  for (;; groups++) {
-    k.rows_each = (rows + groups - 1) / groups;
-    most = 0;
-    for (int r = 0; r < rows; r += k.rows_each) most = std::max(most, col_of(std::min(rows, r + k.rows_each)) - col_of(r) + more);
-    if (most <= kVupMaxCols || k.rows_each == 1) break;
-  }
-  groups = (rows + k.rows_each - 1) / k.rows_each;
+int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_ml, const SplitPlan& plan, const VupShape& sh, int form, bool natural,
+                              const uint16_t* W_UV, void* out, int out_bf16, int rows, int S, int H, int dC, int32_t* status, bool chained) {
+  // columns that there are partial results for
+  const int all = (plan.loose ? std::max(plan.num_items, plan.room_items) : plan.num_items) * S;
   const int n_seqs = rows / S;
+  VupParams k;
+  k.rows_each = sh.rows_each;
   k.listed = !plan.loose && n_seqs <= kVupListed && all < 65536;
   if (k.listed)
     for (int i = 0; i <= n_seqs; i++) k.first[i] = (uint16_t)plan.first[i];
   k.halves = form == kPartialHalves ? 2 : 1;
-  const int widest = kVupRing / 4 / (k.halves * 128), blocks = std::max(1, (most + widest - 1) / widest);
-  const int unit = (blocks > 1 ? 32 : 16) / k.halves;   // N is a multiple of 16, and a block begins at a multiple of 32 tensor-memory columns
-  k.n_block = std::max(unit, ((most + blocks - 1) / blocks + unit - 1) / unit * unit);
+  k.n_block = sh.n_block;
+  k.n_kb = sh.n_kb;
+  k.n_stages = sh.n_stages;
+  k.tmem_cols = sh.tmem_cols;
+  k.room = sh.blocks * sh.n_block;
+  k.all = all;
   const int blk_bytes = k.halves * k.n_block * 128;
-  k.n_kb = 4;
-  while (k.n_kb > 1 && k.n_kb * blk_bytes > kVupRing / (k.n_kb > 2 ? 2 : 3)) k.n_kb /= 2;
-  k.n_stages = std::min({kVupMaxStages, kVupRing / (k.n_kb * blk_bytes), (dC / 64 + k.n_kb - 1) / k.n_kb * blocks});
-  k.tmem_cols = 32;
-  while (k.tmem_cols < blocks * k.halves * k.n_block) k.tmem_cols *= 2;
   k.part_ml = part_ml;
   k.warm = all > 0;
   k.chunk_off = plan.chunk_off;
@@ -722,7 +711,7 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   const size_t smem = (size_t)k.nk * 32768 + (size_t)k.n_stages * k.n_kb * blk_bytes + sizeof(VupShared);
   auto launch = [&](auto kern) -> int32_t {
     if (int32_t rc = allow_smem(dev, kern, smem)) return rc;
-    RELUX_CUDA_TRY(launch_chained(chained, kern, dim3(H, groups), dim3(32 * kVupWarps), smem, dev->stream, tw, tp, k));
+    RELUX_CUDA_TRY(launch_chained(chained, kern, dim3(H, sh.groups), dim3(32 * kVupWarps), smem, dev->stream, tw, tp, k));
     count_launch(dev);
     return RELUX_OK;
   };

@@ -27,6 +27,7 @@ struct PrepAppend {
 struct PrepPlan {
   int32_t listed;              // nothing to build
   int32_t extra, G, workers, by_item, start_units;
+  int32_t room;                // items that `items` and the partial results have room for
   StreamItem* items;
   int32_t* chunk_off;
   int32_t* worker_first;
@@ -120,46 +121,83 @@ __device__ __forceinline__ int prep_block_excl_scan(int v, int32_t* s_warp, int*
   return base + incl - v;
 }
 
-// The stream partition over the lengths AFTER this step's append (the append of the same launch has not advanced them
-// yet: every sequence counts its cached rows + its new rows + extra).  Same arithmetic as build_stream_kernel.
-__device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const PrepPlan& pl) {
+// The stream partition, by a block: sequence i, of the pool's `seq`, has tokens_of(i, seq) tokens and occupies `units` units of the stream from `at`
+// on, where SeqCut cuts it; items are numbered in stream order, so the items of a sequence and the items of a worker are both contiguous.
+// The plan was made for the lengths that the host knows.  Where the device's are others (SplitPlan::loose) and have outgrown its workers or its room,
+// the sequences are cut into equal ranges for as many workers instead, n_seqs + workers - 1 items at most.  That serves all lengths; if it did not, the
+// plan would be empty and the status would say so: nothing is written past its room.
+template <typename Tokens>
+__device__ __forceinline__ void build_stream(const PrepPlan& pl, int n_seqs, const int32_t* seq_ids, int page_tokens, int32_t* status, Tokens tokens_of) {
   __shared__ int32_t s_warp[32];
-  int unit_base = 0, item_base = 0;
-  for (int i0 = 0; i0 < g.n_seqs; i0 += blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    int seq = 0, pages = 0, tokens = 0;
-    if (i < g.n_seqs) {
-      seq = g.seq_ids ? g.seq_ids[i] : i;
-      tokens = load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
-      pages = (tokens + g.page_tokens - 1) / g.page_tokens;
-    }
-    int tot_units, tot_items;
-    const int at = unit_base + prep_block_excl_scan(SeqCut(pl.by_item, pl.G, pl.start_units, 0, pages).units, s_warp, &tot_units);
-    const SeqCut cut(pl.by_item, pl.G, pl.start_units, at, pages);
-    const int c0 = item_base + prep_block_excl_scan(cut.n, s_warp, &tot_items);
-    if (i < g.n_seqs) {
-      pl.chunk_off[i] = c0;
-      for (int c = 0; c < cut.n; c++) {
-        StreamItem w;
-        w.seq_index = i;
-        w.seq = seq;
-        w.page_begin = cut.begin(c);
-        w.page_end = cut.end(c);
-        w.tokens = tokens;
-        w.first = c0;
-        w.n = cut.n;
-        w.pad = 0;
-        pl.items[c0 + c] = w;
-        if (pl.by_item) pl.worker_first[c0 + c] = c0 + c;
-        else if (cut.leads(c, at)) pl.worker_first[cut.first + c] = c0 + c;
+  int by_item = pl.by_item, G = pl.G, start_units = pl.start_units;
+#pragma unroll 1
+  for (int pass = 0;; pass++) {
+    int unit_base = 0, item_base = 0;
+    for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      int seq = 0, pages = 0, tokens = 0;
+      if (i < n_seqs) {
+        seq = seq_ids ? seq_ids[i] : i;
+        tokens = tokens_of(i, seq);
+        pages = (tokens + page_tokens - 1) / page_tokens;
       }
+      int tot_units, tot_items;
+      const int at = unit_base + prep_block_excl_scan(SeqCut(by_item, G, start_units, 0, pages).units, s_warp, &tot_units);
+      const SeqCut cut(by_item, G, start_units, at, pages);
+      const int c0 = item_base + prep_block_excl_scan(cut.n, s_warp, &tot_items);
+      if (i < n_seqs) {
+        pl.chunk_off[i] = c0;
+        for (int c = 0; c < cut.n && c0 + c < pl.room; c++) {
+          StreamItem w;
+          w.seq_index = i;
+          w.seq = seq;
+          w.page_begin = cut.begin(c);
+          w.page_end = cut.end(c);
+          w.tokens = tokens;
+          w.first = c0;
+          w.n = cut.n;
+          w.pad = 0;
+          pl.items[c0 + c] = w;
+          const int worker = by_item ? c0 + c : cut.first + c;
+          if (worker < pl.workers && (by_item || cut.leads(c, at))) pl.worker_first[worker] = c0 + c;
+        }
+      }
+      unit_base += tot_units;
+      item_base += tot_items;
     }
-    unit_base += tot_units;
-    item_base += tot_items;
+    const int used = by_item ? item_base : (unit_base + G - 1) / G;
+    if (used <= pl.workers && item_base <= pl.room) {
+      if (threadIdx.x == 0) pl.chunk_off[n_seqs] = item_base;
+      for (int w = used + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;   // no work
+      return;
+    }
+    __syncthreads();
+    if (pass == 1) {
+      if (threadIdx.x == 0) set_status(status, RELUX_ERR_UNSUPPORTED);
+      for (int w = threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = 0;
+      for (int i = threadIdx.x; i <= n_seqs; i += blockDim.x) pl.chunk_off[i] = 0;
+      return;
+    }
+    int units = 0;
+    for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      int pages = 0, tot;
+      if (i < n_seqs) pages = (tokens_of(i, seq_ids ? seq_ids[i] : i) + page_tokens - 1) / page_tokens;
+      prep_block_excl_scan(SeqCut(0, 1, kStartUnits, 0, pages).units, s_warp, &tot);
+      units += tot;
+    }
+    by_item = 0;
+    start_units = kStartUnits;
+    G = range_units(units, pl.workers);
   }
-  if (threadIdx.x == 0) pl.chunk_off[g.n_seqs] = item_base;
-  // ranges past the end of the stream are empty
-  for (int w = (pl.by_item ? item_base : (unit_base + pl.G - 1) / pl.G) + threadIdx.x; w <= pl.workers; w += blockDim.x) pl.worker_first[w] = item_base;
+}
+
+// The same over the lengths AFTER this step's append (the append of the same launch has not advanced them yet: every sequence counts its cached rows +
+// its new rows + extra).
+__device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const PrepPlan& pl) {
+  build_stream(pl, g.n_seqs, g.seq_ids, g.page_tokens, g.status, [&](int i, int seq) {
+    return load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
+  });
 }
 
 }  // namespace relux

@@ -9,6 +9,7 @@
 #include <vector>
 #include "common.cuh"
 #include "internal.h"
+#include "prep_parts.cuh"
 #include "splitkv.h"
 
 namespace relux {
@@ -121,73 +122,12 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
   return RELUX_OK;
 }
 
-// Exclusive prefix sum over the block (blockDim.x = 256); *total receives the block's sum.
-__device__ __forceinline__ int block_excl_scan(int v, int32_t* s_warp, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  __syncthreads();   // s_warp may still be read from the previous call
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  int base = 0, sum = 0;
-  for (int w = 0; w < 8; w++) {
-    if (w < warp) base += s_warp[w];
-    sum += s_warp[w];
-  }
-  *total = sum;
-  return base + incl - v;
-}
-
-// Stream partition (see plan_stream): sequence i occupies pages [start_i, start_i + pages_i) of the stream and
-// is cut at every multiple of G; items are numbered in stream order, so the items of a sequence and the items of
-// a worker are both contiguous.
 // Behind the preparation's absorb it works beside it, and waits at its end only: the lengths and the last plan's readers are older than
 // that head of the chain.
-__global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
-                                    int page_tokens, int G, int workers, int by_item, int start_units,
-                                    StreamItem* __restrict__ items, int32_t* __restrict__ chunk_off, int32_t* __restrict__ worker_first) {
-  __shared__ int32_t s_warp[8];
+__global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra, int page_tokens,
+                                    const __grid_constant__ PrepPlan pl, int32_t* status) {
   chain_release();
-  int unit_base = 0, item_base = 0;
-  for (int i0 = 0; i0 < n_seqs; i0 += blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    int seq = 0, pages = 0, tokens = 0;
-    if (i < n_seqs) {
-      seq = seq_ids ? seq_ids[i] : i;
-      tokens = load_chained(len + seq) + extra;
-      pages = (tokens + page_tokens - 1) / page_tokens;
-    }
-    int tot_units, tot_items;
-    const int at = unit_base + block_excl_scan(SeqCut(by_item, G, start_units, 0, pages).units, s_warp, &tot_units);
-    const SeqCut cut(by_item, G, start_units, at, pages);
-    const int c0 = item_base + block_excl_scan(cut.n, s_warp, &tot_items);
-    if (i < n_seqs) {
-      chunk_off[i] = c0;
-      for (int c = 0; c < cut.n; c++) {
-        StreamItem w;
-        w.seq_index = i;
-        w.seq = seq;
-        w.page_begin = cut.begin(c);
-        w.page_end = cut.end(c);
-        w.tokens = tokens;
-        w.first = c0;
-        w.n = cut.n;
-        w.pad = 0;
-        items[c0 + c] = w;
-        if (by_item) worker_first[c0 + c] = c0 + c;
-        else if (cut.leads(c, at)) worker_first[cut.first + c] = c0 + c;
-      }
-    }
-    unit_base += tot_units;
-    item_base += tot_items;
-  }
-  if (threadIdx.x == 0) chunk_off[n_seqs] = item_base;
-  // ranges past the end of the stream are empty
-  for (int w = (by_item ? item_base : (unit_base + G - 1) / G) + threadIdx.x; w <= workers; w += blockDim.x) worker_first[w] = item_base;
+  build_stream(pl, n_seqs, seq_ids, page_tokens, status, [&](int, int seq) { return load_chained(len + seq) + extra; });
   chain_wait();
 }
 
@@ -245,7 +185,7 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
     const int longest = pages.empty() ? 0 : *std::max_element(pages.begin(), pages.end());
     stream_partition_shape(pages.data(), sb.n_seqs, workers, page_multiple, std::max(chunk, (longest + kMaxRowItems - 3) / (kMaxRowItems - 2)), &G, &shape.workers, &shape.items);
     shape.G = (int)G;
-    shape.room = shape.items;
+    shape.room = std::max(shape.items, sb.n_seqs + shape.workers - 1);
   } else {
     shape = cheapest_plan(pages, workers);
   }
@@ -276,9 +216,10 @@ int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int worke
 }
 
 int32_t launch_build_stream(Pool* p, const SeqBatch& sb, int layer, int extra, const SplitPlan& plan, bool chained) {
+  const PrepPlan pl{0, extra, plan.chunk_pages, plan.num_workers, plan.by_item ? 1 : 0, plan.start_units, plan.room_items, plan.stream_items, plan.chunk_off,
+                    plan.worker_first};
   RELUX_CUDA_TRY(launch_chained(chained, build_stream_kernel, dim3(1), dim3(256), 0, p->dev->stream, p->d_len + (size_t)layer * p->prm.max_seqs, sb.d_seq_ids,
-                                sb.n_seqs, extra, p->prm.page_tokens, plan.chunk_pages, plan.num_workers, plan.by_item ? 1 : 0, plan.start_units,
-                                plan.stream_items, plan.chunk_off, plan.worker_first));
+                                sb.n_seqs, extra, p->prm.page_tokens, pl, p->d_status));
   count_launch(p->dev);
   return RELUX_OK;
 }

@@ -56,8 +56,13 @@ constexpr int kStartUnits = 4;   // pages, two tiles: what plan_cost counts for 
 struct StreamShape {
   int G, workers, items, start_units;
   bool by_item;
-  int room;   // items of the larger of the plans compared: scratch for as many serves the call on either side of their border
+  int room;   // scratch for as many items serves the call on either side of the plans' border, and every later length of its sequences (build_stream)
 };
+// Length of the equal ranges that share `units` units of sequences, each with its kStartUnits.
+RELUX_HD inline int range_units(int64_t units, int workers) {
+  const int G = (int)((units + workers - 1) / workers + 1) / 2 * 2;
+  return G > 2 * kStartUnits ? G : 2 * kStartUnits;
+}
 inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   int longest = 0, live = 0;
   int64_t units = 0;
@@ -68,7 +73,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   }
   StreamShape r{};
   r.start_units = kStartUnits;
-  r.G = std::max((int)((units + workers - 1) / workers + 1) / 2 * 2, 2 * kStartUnits);
+  r.G = range_units(units, workers);
   r.workers = std::max(1, (int)((units + r.G - 1) / r.G));
   int at = 0, most = 0, of_worker = -1;
   double worst = 0, here = 0;   // of the ranges, walked as the workers walk them
@@ -84,7 +89,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
     r.items += cut.n;
     at += cut.units;
   }
-  r.room = r.items;
+  r.room = std::max(r.items, live + r.workers - 1);
   if (live == 0 || live > workers) return r;
   double best = plan_cost(worst, most, r.items);
   auto items_of = [&](int t) {
@@ -101,7 +106,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   for (int t = lo; t <= lo + 1; t++) {   // one more tile each may leave fewer partials
     const int items = items_of(t);
     const double cost = plan_cost(t + 2, (longest + 2 * t - 1) / (2 * t), items);
-    r.room = std::max(r.room, items);
+    r.room = std::max(r.room, live + items - 1);
     if (cost < best) {
       best = cost;
       r = StreamShape{2 * t, items, items, 0, true, r.room};

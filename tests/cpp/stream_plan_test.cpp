@@ -1,10 +1,12 @@
 // The plan of the persistent latent decode kernel and the items it is cut into, walked as the device builder walks them.
-// With arguments (workers, then pages of every sequence): prints the plan.  Without: random calls.
+// With arguments (workers, then pages of every sequence): prints the plan.  Without: random calls, and random lengths that a plan's launch finds
+// other than those it was made for, with the up-projection's columns for both.
 #include <cstdio>
 #include <cstdlib>
 #include <random>
 
 #include "stream_plan.h"
+#include "vup_plan.h"
 
 using namespace relux;
 
@@ -55,6 +57,56 @@ static bool check(const std::vector<int>& pages, int workers) {
   return true;
 }
 
+// The pieces of every sequence as the device cuts them (build_stream) for a plan made for other lengths; empty where it has no room for them.
+static std::vector<int32_t> device_first(const StreamShape& s, const std::vector<int>& pages) {
+  int by_item = s.by_item, G = s.G, start_units = s.start_units;
+  for (int pass = 0; pass < 2; pass++) {
+    std::vector<int32_t> first(1, 0);
+    int unit = 0;
+    for (int n : pages) {
+      const SeqCut cut(by_item, G, start_units, unit, n);
+      unit += cut.units;
+      first.push_back(first.back() + cut.n);
+    }
+    if ((by_item ? first.back() : (unit + G - 1) / G) <= s.workers && first.back() <= s.room) return first;
+    int64_t units = 0;
+    for (int n : pages) units += SeqCut(0, 1, kStartUnits, 0, n).units;
+    by_item = 0, start_units = kStartUnits, G = range_units(units, s.workers);
+  }
+  return {};
+}
+
+static bool check_columns(const std::vector<int>& pages, int S, int heads, const StreamShape& s, const std::vector<int32_t>& planned, const std::vector<int32_t>& found,
+                          bool loose, int halves) {
+  const int workers = s.workers, rows = (int)pages.size() * S, dC = 512;
+  const VupShape v = vup_shape(planned, rows, S, 148 / heads, halves, dC, loose ? workers : 0);
+  CHECK(v.fits());
+  const int unit = (v.blocks > 1 ? 32 : 16) / halves;
+  CHECK(v.blocks >= 1 && v.n_block % unit == 0 && halves * v.n_block <= 256 && v.blocks * halves * v.n_block <= v.tmem_cols);
+  CHECK(v.tmem_cols >= 32 && v.tmem_cols <= 512 && (v.tmem_cols & (v.tmem_cols - 1)) == 0);
+  CHECK(v.n_stages >= 1 && v.n_stages <= kVupMaxStages && v.n_stages * v.n_kb * halves * v.n_block * 128 <= kVupRing);
+  CHECK(v.groups >= 1 && (v.groups - 1) * v.rows_each < rows && v.groups * v.rows_each >= rows);
+  for (int g = 0; g < v.groups; g++) {
+    const int r = g * v.rows_each, end = std::min(rows, r + v.rows_each);
+    CHECK(vup_col(found, S, end) - vup_col(found, S, r) <= std::min(v.most, v.blocks * v.n_block));
+  }
+  return true;
+}
+
+static bool check_found(std::mt19937& rng, const std::vector<int>& pages, int S, int heads, int resident) {
+  const int workers = S > 8 ? std::min(resident, std::max(1, (2 * resident + S - 1) / S)) : std::max(1, resident / S);
+  const StreamShape s = cheapest_plan(pages, workers);
+  const std::vector<int32_t> planned = device_first(s, pages);
+  CHECK((int)planned.size() == (int)pages.size() + 1 && planned.back() == s.items);   // the host's own lengths are served as planned
+  if (!check_columns(pages, S, heads, s, planned, planned, false, rng() % 2 ? 1 : 2)) return false;
+  std::vector<int> now = pages;
+  const int how = (int)(rng() % 4);
+  for (int& n : now) n = how == 0 ? n + (int)(rng() % 2) : how == 1 ? n + (int)(rng() % 40) : how == 2 ? (int)(rng() % 400) : rng() % 5 ? 0 : (int)(rng() % 2000);
+  const std::vector<int32_t> found = device_first(s, now);
+  CHECK(found.size() == pages.size() + 1);
+  return check_columns(pages, S, heads, s, planned, found, true, 2);
+}
+
 int main(int argc, char** argv) {
   if (argc > 1) {
     std::vector<int> pages;
@@ -73,6 +125,13 @@ int main(int argc, char** argv) {
     for (int& p : pages) p = (int)(rng() % span) * (rng() % 8 != 0) + (rng() % 4 != 0);   // some of them empty
     if (!check(pages, workers)) return 1;
     (cheapest_plan(pages, workers).by_item ? pieces : ranges)++;
+  }
+  const int heads[] = {16, 32, 40, 64, 75, 128};
+  for (int t = 0; t < 60000; t++) {
+    const int S = 1 + (int)(rng() % (rng() % 4 ? 4 : 40)), n = 1 + (int)(rng() % (rng() % 2 ? 8 : 160)), span = spans[rng() % 6];
+    std::vector<int> pages(n);
+    for (int& p : pages) p = 1 + (int)(rng() % span);
+    if (!check_found(rng, pages, S, heads[rng() % 6], rng() % 4 ? 74 : 1 + (int)(rng() % 100))) return 1;
   }
   if (pieces < 1000 || ranges < 1000) return printf("%d pieces, %d ranges\n", pieces, ranges), 1;
   puts("ok");

@@ -90,3 +90,42 @@ def test_a_plain_call_behind_launches_of_a_graph(dev, oracle, captured, after): 
     plain.destroy()
     graphed.destroy()
     calls.free()
+
+
+def _random(n, most, seed):
+    return [int(x) for x in np.random.default_rng(seed).integers(1, most, n)]
+
+
+@pytest.mark.parametrize("ctx,H,later", [
+    ([126] * 37, 16, None),                          # a piece a sequence: six tokens on none fits its worker
+    (_random(65, 3050, 1), 16, None),                # ranges and five groups of heads' CTAs: borders move between the groups
+    (_random(80, 1500, 2), 40, "turned"),
+    ([1000, 64, 2500, 130], 128, "turned"),
+    ([640] * 30, 32, "one"),                         # one sequence of all the length there is, the others almost empty
+])
+def test_a_graph_whose_lengths_have_outgrown_its_plan(dev, oracle, ctx, H, later):  # noqa: F811
+    """Six launches, then lengths that the host sets: what a group of rows has in pieces is not what it had when the call was captured."""
+    B, room = len(ctx), max(ctx)
+    calls = Calls(dev, oracle, B, H)
+    plain, graphed = (latent_pool(dev, oracle, [room] * B, 8) for _ in range(2))
+    for k, pool in enumerate((plain, graphed)):
+        pool.set_len(0, np.asarray(ctx, np.int32))
+        calls.step(pool, k)
+    graph = Graph(dev, lambda: calls.step(graphed, 1))
+    graphed.set_len(0, np.asarray(ctx, np.int32) + 1)   # the host counts the captured call, which did not run
+    for i in range(6):
+        calls.step(plain, 0)
+        graph.launch()
+        calls.same(i)
+    if later:
+        for pool in (plain, graphed):
+            pool.set_len(0, np.asarray(ctx[::-1] if later == "turned" else [room] + [3] * (B - 1), np.int32))
+        for i in range(3):
+            calls.step(plain, 0)
+            graph.launch()
+            calls.same((later, i))
+    assert plain.status() == 0 and graphed.status() == 0
+    graph.free()
+    plain.destroy()
+    graphed.destroy()
+    calls.free()
