@@ -383,6 +383,7 @@ __global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_
 constexpr int kVupWarps = 16;
 constexpr int kVupListed = 256;                   // sequences whose first pieces travel as arguments
 static_assert(kVupMaxCols >= kMaxRowItems, "a row's pieces are columns of one CTA");
+static_assert(kListedItems <= kVupListed && kListedItems < 65536, "a listed plan is listed here too");
 struct VupParams {
   const float* part_ml;
   const int32_t* chunk_off;
@@ -676,7 +677,7 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   const int n_seqs = rows / S;
   VupParams k;
   k.rows_each = sh.rows_each;
-  k.listed = !plan.loose && n_seqs <= kVupListed && all < 65536;
+  k.listed = !plan.loose && n_seqs <= kVupListed && plan.num_items < 65536;   // wherever the plan is (list_plan): chunk_off then does not exist
   if (k.listed)
     for (int i = 0; i <= n_seqs; i++) k.first[i] = (uint16_t)plan.first[i];
   k.halves = form == kPartialHalves ? 2 : 1;

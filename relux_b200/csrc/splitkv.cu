@@ -154,7 +154,7 @@ void stream_partition_shape(const int* pages, int n_seqs, int workers, int page_
 
 // The items as build_stream_kernel writes them, into arguments; false where they do not fit.
 static bool list_plan(const SeqBatch& sb, const std::vector<int>& pages, const int32_t* len, int extra, const SplitPlan& plan, ListedPlan* out) {
-  if (plan.num_items > kListedItems || plan.num_workers > kListedWorkers) return false;
+  if (sb.n_seqs > kListedItems || plan.num_items > kListedItems || plan.num_workers > kListedWorkers) return false;
   int at = 0, item = 0;
   for (int i = 0; i < sb.n_seqs; i++) {
     const SeqCut cut(plan.by_item, plan.chunk_pages, plan.start_units, at, pages[i]);

@@ -54,6 +54,41 @@ def test_a_step_is_append_then_decode(dev, oracle, ctx, new):  # noqa: F811
     wuv.free()
 
 
+def test_a_step_of_prompts(dev, oracle):  # noqa: F811
+    """2048 new rows and query tokens for each of 32 sequences: a plan of few items, 65536 rows of attention."""
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    B, S, pages = 32, 2048, 32
+    rng = np.random.default_rng(3)
+    wuk, wuv = weights(dev, oracle, rng)
+    few = lambda w: np.tile(oracle.bf16_from_f32(rng.standard_normal((1 << 16, w)).astype(np.float32)), (B * S * H // (1 << 16), 1))  # noqa: E731
+    q, qr = dev.upload(few(DH)), dev.upload(few(DHR))
+    c, r = (dev.upload(oracle.bf16_from_f32(rng.standard_normal((B * S, w)).astype(np.float32))) for w in (DC, DHR))
+    n_new, outs = np.full(B, S, np.int32), []
+    for fused in (True, False):
+        pool = rb.Pool(dev, L.POOL_MLA, 1, B * pages, 64, B, pages, dC=DC, dHR=DHR)
+        pool.set_tables(permuted_tables(np.random.default_rng(4), B, pages))
+        pool.tune(L.TUNE_MLA_PROMPT_MIN_TOKENS, 1 << 20)     # by the decode kernel both times
+        out = dev.upload(np.full((B, S, H, DH), 0x7fc0, np.uint16))
+        kw = dict(q_dtype=L.DTYPE_BF16, out_dtype=L.DTYPE_BF16)
+        if fused:
+            ap = pool._append_args(0, c, r, B, None, n_new, L.LAYOUT_TOKEN_MAJOR, True, L.DTYPE_BF16)
+            at = pool._attn_args(0, B, q, qr, out, H, DH, SCALE, S, 0, True, L.ATTN_FAST, wuk, wuv, None, L.LAYOUT_TOKEN_MAJOR, L.LAYOUT_TOKEN_MAJOR,
+                                 L.DTYPE_BF16, L.DTYPE_BF16)
+            L.check(pool.lib.relux_mla_step(pool.h, C.byref(ap), C.byref(at)))
+        else:
+            pool.append(0, c, r, B, n_new=n_new, dtype=L.DTYPE_BF16)
+            pool.decode(0, B, q, out, H, DH, SCALE, q_rope=qr, w_uk=wuk, w_uv=wuv, q_tokens=S, **kw)
+        dev.sync()
+        assert pool.status() == 0
+        outs.append(out.download((B, S, H, DH), np.uint16))
+        pool.destroy()
+        out.free()
+    assert np.array_equal(outs[0], outs[1]) and not (outs[0] == 0x7fc0).any()
+    for b in (q, qr, c, r, wuk, wuv):
+        b.free()
+
+
 def test_a_captured_step_runs_with_the_lengths_of_its_launch(dev, oracle):  # noqa: F811
     from relux_b200 import lib as L
     rt = C.CDLL("libcudart.so.12")
