@@ -203,7 +203,8 @@ int32_t relux_pool_read_rows(relux_pool_t pool, const relux_read_rows_args* args
 
 /* Tuning knobs of relux_pool_tune. */
 #define RELUX_TUNE_MLA_GENERIC 0        /* RELUX_MLA_GENERIC: 1 = MLA decode on the CUDA-core kernels                      */
-#define RELUX_TUNE_MLA_WORKERS 1        /* RELUX_MLA_WORKERS: ranges the stream of pages is cut into (0 = resident pairs)   */
+#define RELUX_TUNE_MLA_WORKERS 1        /* RELUX_MLA_WORKERS: ranges the stream of pages is cut into (0 = resident pairs);
+                                           longer ones for a sequence that would have more than 240 of them                */
 #define RELUX_TUNE_CHUNK_PAGES 2        /* RELUX_CHUNK_PAGES: chunk length of the split-KV planner (0 = chosen per call;
                                            raised for a latent sequence that it would cut into more than 240 chunks)       */
 #define RELUX_TUNE_GEMM_GENERIC 3       /* RELUX_GEMM_GENERIC: 1 = projections on the plain kernel                          */

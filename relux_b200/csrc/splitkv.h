@@ -59,10 +59,6 @@ struct SplitPlan {
   int32_t* worker_first = nullptr;     // device [num_workers + 1]
 };
 
-// More items than this no sequence is cut into (the projection of the partial results keeps the columns of a row together): only the
-// knob CHUNK_PAGES could ask for more.
-constexpr int kMaxRowItems = 240;
-
 // A row of a latent call's partial results: float32, one bf16 value or two bf16 halves a column (write_partial, mla_decode_sm100.cu).
 enum PartialForm { kPartialFloat32 = 0, kPartialOne = 1, kPartialHalves = 2 };
 

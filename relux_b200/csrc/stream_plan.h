@@ -14,6 +14,10 @@
 
 namespace relux {
 
+// More items than this no sequence is cut into: the projection of the partial results keeps the columns of a row together.  Only the tuning knobs
+// (more workers, shorter chunks) could ask for more.
+constexpr int kMaxRowItems = 240;
+
 // The items of a sequence of `pages` pages that begins at unit `at` of the stream: item c is its pages [begin(c), end(c)), and belongs to
 // worker first + c, or (by_item) to a worker of its own.  What the host counts and the device builds from.
 struct SeqCut {
@@ -73,7 +77,8 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
   }
   StreamShape r{};
   r.start_units = kStartUnits;
-  r.G = range_units(units, workers);
+  const int longest2 = (longest + 1) / 2 * 2;
+  r.G = std::max(range_units(units, workers), ((longest2 + kMaxRowItems - 2) / (kMaxRowItems - 1) + 1) / 2 * 2);   // a sequence may begin and end inside ranges
   r.workers = std::max(1, (int)((units + r.G - 1) / r.G));
   int at = 0, most = 0, of_worker = -1;
   double worst = 0, here = 0;   // of the ranges, walked as the workers walk them
@@ -97,7 +102,7 @@ inline StreamShape cheapest_plan(const std::vector<int>& pages, int workers) {
     for (int n : pages) items += (n + 2 * t - 1) / (2 * t);
     return items;
   };
-  int lo = 1, hi = (longest + 1) / 2;   // the smallest t whose pieces find a worker each: one piece a sequence does
+  int lo = (longest + 2 * kMaxRowItems - 1) / (2 * kMaxRowItems), hi = (longest + 1) / 2;   // the smallest t whose pieces find a worker each: one piece a sequence does
   while (lo < hi) {
     const int t = (lo + hi) / 2;
     if (items_of(t) <= workers) hi = t;

@@ -41,7 +41,8 @@ inline VupShape vup_shape(const std::vector<int32_t>& first, int rows, int S, in
     k.most = 0;
     for (int r = 0; r < rows; r += k.rows_each) {
       const int end = std::min(rows, r + k.rows_each), n = end - r;
-      k.most = std::max(k.most, workers > 0 ? n + std::min(S, n) * (workers - 1) : vup_col(first, S, end) - vup_col(first, S, r));
+      const int now = vup_col(first, S, end) - vup_col(first, S, r), later = workers > 0 ? n + std::min(S, n) * (workers - 1) : now;
+      k.most = std::max(k.most, k.rows_each > 1 ? later : std::max(now, std::min(later, kVupMaxCols)));   // one row: the kernel reports what is more
     }
     if (k.most <= kVupMaxCols || k.rows_each == 1) break;
   }

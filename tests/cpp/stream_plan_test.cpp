@@ -36,6 +36,7 @@ static bool check(const std::vector<int>& pages, int workers) {
       items.push_back({i, cut.begin(c), cut.end(c), w});
     }
     CHECK(at == pages[i]);
+    CHECK(cut.n <= kMaxRowItems);
     unit += cut.units;
   }
   CHECK((int)items.size() == s.items);
@@ -125,6 +126,15 @@ int main(int argc, char** argv) {
     for (int& p : pages) p = (int)(rng() % span) * (rng() % 8 != 0) + (rng() % 4 != 0);   // some of them empty
     if (!check(pages, workers)) return 1;
     (cheapest_plan(pages, workers).by_item ? pieces : ranges)++;
+  }
+  for (int t = 0; t < 20000; t++) {   // of the tuning knob: more workers than a row may have pieces
+    std::vector<int> pages(1 + (int)(rng() % (rng() % 2 ? 2 : 30)));
+    for (int& p : pages) p = 1 + (int)(rng() % (rng() % 2 ? 16384 : 300));
+    const int workers = 1 + (int)(rng() % 4096);
+    if (!check(pages, workers)) return 1;
+    const StreamShape s = cheapest_plan(pages, workers);
+    const std::vector<int32_t> planned = device_first(s, pages);
+    if (!check_columns(pages, 1, 16, s, planned, planned, t & 1, 2)) return 1;
   }
   const int heads[] = {16, 32, 40, 64, 75, 128};
   for (int t = 0; t < 60000; t++) {

@@ -49,3 +49,31 @@ def test_pieces_at_the_borders_of_blocks_and_groups(dev, oracle, ctx, H, chunk, 
     pool.destroy()
     d_uk.free()
     d_uv.free()
+
+
+def test_more_workers_than_a_row_may_have_pieces(dev, oracle):  # noqa: F811
+    """The knob MLA_WORKERS asks for 1000 ranges: 4100 pages of one sequence and a short one beside it, against the plan of the call's choice."""
+    from relux_b200 import lib as L
+    import relux_b200 as rb
+    rng = np.random.default_rng(12)
+    ctx, H, pages = [4100 * 64 - 5, 300], 16, 4100
+    pool = rb.Pool(dev, L.POOL_MLA, 1, 2 * pages, 64, 2, pages, dC=DC, dHR=DHR)
+    pool.set_tables(permuted_tables(rng, 2, pages))
+    block = [oracle.bf16_from_f32(rng.standard_normal((4096, w)).astype(np.float32)) for w in (DC, DHR)]
+    for at in range(0, max(ctx), 4096):
+        n = [min(4096, max(0, c - at)) for c in ctx]
+        pool.append(0, *(np.concatenate([x[:k] for k in n]) for x in block), 2, n_new=np.asarray(n, np.int32))
+    q, qr = (oracle.bf16_from_f32(rng.standard_normal((2, 1, H, w)).astype(np.float32)) for w in (DH, DHR))
+    wuk, wuv = (dev.upload(oracle.bf16_from_f32(rng.standard_normal((DC, H * DH)).astype(np.float32) * 0.02)) for _ in range(2))
+    outs = []
+    for workers in (0, 241, 1000, 1 << 20):
+        pool.tune(L.TUNE_MLA_WORKERS, workers)
+        outs.append(np.full((2, 1, H, DH), np.nan, np.float32))
+        pool.decode(0, 2, q, outs[-1], H, DH, (DH + DHR) ** -0.5, q_rope=qr, w_uk=wuk, w_uv=wuv)
+    # P is rounded to 8 bits against other maxima: 2^-9 of a value with a random sign, over the largest of 4096 values
+    for out in outs[1:]:
+        assert np.isfinite(out).all() and np.max(np.abs(out - outs[0])) <= 2e-2 * np.sqrt(np.mean(outs[0] ** 2))
+    assert pool.status() == 0
+    pool.destroy()
+    wuk.free()
+    wuv.free()
