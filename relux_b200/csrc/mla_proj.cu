@@ -393,7 +393,6 @@ struct VupParams {
   int32_t halves, n_block, n_kb, n_stages;    // VupShape; a stage is one TMA box
   int32_t tmem_cols;
   int32_t room, all;                          // columns that a CTA has room for, and that there are partial results for
-  int32_t warm;                               // there are partial results: part_ml may be read, whatever it holds
   int32_t listed;                             // `first` holds chunk_off
   int32_t* status;
   uint16_t first[kVupListed + 1];
@@ -507,6 +506,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
           __syncwarp();
           if (++s == prm.n_stages) s = 0, use++;
         }
+      if (nk > 2) vup_wait(&sh->w_full[1], 0, prm.status);   // no block may have asked for it, and no load may land when the CTA has gone
       if (el) umma_commit<1>(&sh->done);
       __syncwarp();
     }
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
   const uint32_t tmem_d = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   const size_t off0 = ((size_t)r0 * H + h) * kDh + (warp & 3) * 32 + lane;
 #pragma unroll 1
-  for (int pass = warp >= 2 && prm.warm ? 0 : 1; pass < 2; pass++) {
+  for (int pass = warp >= 2 ? 0 : 1; pass < 2; pass++) {
     const bool real = pass == 1;
     int col0 = 0, lo = 0, hi = 0, rows_here = 1;   // first column of the CTA, and columns of the warp's rows
     if (real) {
@@ -689,7 +689,6 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   k.all = all;
   const int blk_bytes = k.halves * k.n_block * 128;
   k.part_ml = part_ml;
-  k.warm = all > 0;
   k.chunk_off = plan.chunk_off;
   k.out = out;
   k.rows = rows;
@@ -704,11 +703,10 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   const uint64_t p_dims[5] = {64, (uint64_t)all, (uint64_t)k.halves, (uint64_t)dC / 64, (uint64_t)H}, p_strides[4] = {H * lp, (uint64_t)dC, 64, lp};
   const uint32_t p_box[5] = {64, (uint32_t)k.n_block, (uint32_t)k.halves, (uint32_t)k.n_kb, 1};
   CUtensorMap tw, tp;
-  if (!make_tmap_view(&tw, (void*)W_UV, 5, w_dims, w_strides, w_box) || (all > 0 && !make_tmap_view(&tp, (void*)part, 5, p_dims, p_strides, p_box))) {
+  if (!make_tmap_view(&tw, (void*)W_UV, 5, w_dims, w_strides, w_box) || !make_tmap_view(&tp, (void*)part, 5, p_dims, p_strides, p_box)) {
     set_error("tensor map for w_uv or the partial results could not be encoded");
     return RELUX_ERR_CUDA;
   }
-  if (all == 0) tp = tw;   // every sequence is empty: zeros are written
   const size_t smem = (size_t)k.nk * 32768 + (size_t)k.n_stages * k.n_kb * blk_bytes + sizeof(VupShared);
   auto launch = [&](auto kern) -> int32_t {
     if (int32_t rc = allow_smem(dev, kern, smem)) return rc;

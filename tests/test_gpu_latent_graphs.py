@@ -129,3 +129,28 @@ def test_a_graph_whose_lengths_have_outgrown_its_plan(dev, oracle, ctx, H, later
     plain.destroy()
     graphed.destroy()
     calls.free()
+
+
+@pytest.mark.parametrize("full", [0, 1, 9])
+def test_a_graph_that_finds_empty_sequences(dev, oracle, full):  # noqa: F811
+    """A captured decode call launched when all, or all but the first few, of its sequences have been emptied: zeros, and CTAs without a column."""
+    B, H = 60, 16
+    calls = Calls(dev, oracle, B, H)
+    plain, graphed = (latent_pool(dev, oracle, [200] * B, 8) for _ in range(2))
+    for k, pool in enumerate((plain, graphed)):
+        calls.decode(pool, k)
+    graph = Graph(dev, lambda: calls.decode(graphed, 1))
+    calls.same("full")
+    graphed.set_len(0, np.asarray([200] * full + [0] * (B - full), np.int32))
+    for _ in range(3):
+        graph.launch()
+    dev.sync()
+    want, got = (o.download(calls.shape, np.float32) for o in calls.outs)
+    assert not got[full:].any()
+    if full:
+        assert np.max(np.abs(want[:full] - got[:full])) <= 2e-2 * np.sqrt(np.mean(want ** 2))
+    assert graphed.status() == 0
+    graph.free()
+    plain.destroy()
+    graphed.destroy()
+    calls.free()
