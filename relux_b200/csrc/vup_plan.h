@@ -35,11 +35,12 @@ struct VupShape {
 inline VupShape vup_shape(const std::vector<int32_t>& first, int rows, int S, int fit, int halves, int dC, int workers) {
   VupShape k;
   const int all = vup_col(first, S, rows);
-  int groups = std::max(1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}));
-  for (;; groups++) {
+  // (a row at a time fewer, from as many groups as the columns need at least: all numbers of groups in turn were quadratic in the rows)
+  int groups = std::max({1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}), workers > 0 ? 1 : std::min(rows, (all + kVupMaxCols - 1) / kVupMaxCols)});
+  for (;; groups = (rows + k.rows_each - 2) / (k.rows_each - 1)) {
     k.rows_each = (rows + groups - 1) / groups;
     k.most = 0;
-    for (int r = 0; r < rows; r += k.rows_each) {
+    for (int r = 0; r < rows && (k.most <= kVupMaxCols || k.rows_each == 1); r += k.rows_each) {
       const int end = std::min(rows, r + k.rows_each), n = end - r;
       const int now = vup_col(first, S, end) - vup_col(first, S, r), later = workers > 0 ? n + std::min(S, n) * (workers - 1) : now;
       k.most = std::max(k.most, k.rows_each > 1 ? later : std::max(now, std::min(later, kVupMaxCols)));   // one row: the kernel reports what is more

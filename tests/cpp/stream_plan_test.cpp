@@ -3,6 +3,7 @@
 // other than those it was made for, with the up-projection's columns for both.
 #include <cstdio>
 #include <cstdlib>
+#include <ctime>
 #include <random>
 
 #include "stream_plan.h"
@@ -143,6 +144,11 @@ int main(int argc, char** argv) {
     for (int& p : pages) p = 1 + (int)(rng() % span);
     if (!check_found(rng, pages, S, heads[rng() % 6], rng() % 4 ? 74 : 1 + (int)(rng() % 100))) return 1;
   }
+  std::vector<int32_t> first(1, 0);   // 131072 rows of one to 60 pieces: groups tried one number after another took 2.6 s
+  for (int i = 0; i < 64; i++) first.push_back(first.back() + 1 + (int)(rng() % 60));
+  const clock_t from = clock();
+  const VupShape many = vup_shape(first, 64 * 2048, 2048, 1, 2, 512, 0);
+  if (!many.fits() || clock() - from > CLOCKS_PER_SEC / 4) return printf("many rows: %d groups, %.3f s\n", many.groups, (double)(clock() - from) / CLOCKS_PER_SEC), 1;
   if (pieces < 1000 || ranges < 1000) return printf("%d pieces, %d ranges\n", pieces, ranges), 1;
   puts("ok");
   return 0;
