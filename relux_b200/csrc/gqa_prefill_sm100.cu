@@ -603,7 +603,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       for (int k = 0; k < 2; k++) bars->lsum[row[k]][lane & 3] = l_run[k];
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->l_full);
-      if (!it.more || *(volatile uint32_t*)&bars->abort_flag) break;   // after an abort no more items are written
+      // After an abort no more items are written.  The warp leaves as one (the tensor-memory loads are its lanes' together), by a vote behind its own wait:
+      // a lane whose wait ran out has raised the flag or seen it.
+      if (__any_sync(0xffffffffu, !it.more || bars->abort_flag != 0)) break;
       it = bars->items[(n + 1) & 3];
     }
   } else {
