@@ -413,7 +413,8 @@ __device__ __forceinline__ void vup_wait(uint64_t* bar, uint32_t parity, int32_t
   __syncwarp();
 }
 
-template <bool kOutBf16>
+// kLoose (SplitPlan): the host has not counted the columns that the device's lengths make.
+template <bool kOutBf16, bool kLoose>
 __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                           const __grid_constant__ CUtensorMap tmap_p,
                                                                           const __grid_constant__ VupParams prm) {
@@ -457,9 +458,8 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
     const int i = S == 1 ? row : row / S, q = row - i * S, c0 = first_of(i);
     return c0 * S + (q == 0 ? 0 : q * (first_of(i + 1) - c0));
   };
-  // None where the device's lengths have made more columns of them than the launch was sized for.
-  auto rows_now = [&]() -> int {
-    if (prm.listed) return rows_most;
+  auto rows_now = [&]() -> int {   // none where they have more columns than the launch was sized for
+    if (!kLoose) return rows_most;
     const int c0 = col_of(r0), c1 = col_of(r0 + rows_most);
     return c1 - c0 <= prm.room && c1 <= prm.all ? rows_most : 0;
   };
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
     const bool el = elect_one();
     chain_wait();   // the partial results come from the kernel before this one
     const int rows_here = rows_now();
-    if (rows_here == 0 && threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
+    if (kLoose && rows_here == 0 && threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     const int col0 = col_of(r0), blocks = (col_of(r0 + rows_here) - col0 + nb - 1) / nb;
     if (warp == 0) {
 #pragma unroll 1
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
           __syncwarp();
           if (++s == prm.n_stages) s = 0, use++;
         }
-      if (nk > 2) vup_wait(&sh->w_full[1], 0, prm.status);   // no block may have asked for it, and no load may land when the CTA has gone
+      if (kLoose && nk > 2) vup_wait(&sh->w_full[1], 0, prm.status);   // without a column nobody has, and no load may land when the CTA has gone
       if (el) umma_commit<1>(&sh->done);
       __syncwarp();
     }
@@ -714,7 +714,8 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
     count_launch(dev);
     return RELUX_OK;
   };
-  return out_bf16 ? launch(mla_vup_pieces_kernel<true>) : launch(mla_vup_pieces_kernel<false>);
+  if (plan.loose) return out_bf16 ? launch(mla_vup_pieces_kernel<true, true>) : launch(mla_vup_pieces_kernel<false, true>);
+  return out_bf16 ? launch(mla_vup_pieces_kernel<true, false>) : launch(mla_vup_pieces_kernel<false, false>);
 }
 
 }  // namespace relux
