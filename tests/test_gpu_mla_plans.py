@@ -78,3 +78,27 @@ def test_a_call_with_an_empty_sequence(dev, oracle):  # noqa: F811
     pool.destroy()
     d_uk.free()
     d_uv.free()
+
+
+@pytest.mark.parametrize("ctx,heads", [([100, 90, 70, 3], 16), ([500] * 40, 32), ([299] * 64, 128)])
+def test_one_piece_is_rounded_once_it_is_an_average(dev, oracle, ctx, heads):  # noqa: F811
+    """All of a sequence's rows are the same, so that its attention is that row, exactly, in bf16: the output is its projection in float32.  Rounded
+    ahead of the division by the number of rows it would be off by 2^-9.  (512 products, summed in float32: 1e-5 of the result's size.)"""
+    from relux_b200 import lib as L
+    import relux_b200 as rb
+    rng = np.random.default_rng(heads)
+    B, pages = len(ctx), (max(ctx) + 63) // 64
+    pool = rb.Pool(dev, L.POOL_MLA, 1, B * pages, 64, B, pages, dC=DC, dHR=DHR)
+    pool.set_tables(permuted_tables(rng, B, pages))
+    c, r = (oracle.bf16_from_f32(rng.standard_normal((B, w)).astype(np.float32)) for w in (DC, DHR))
+    pool.append(0, np.repeat(c, ctx, axis=0), np.repeat(r, ctx, axis=0), B, n_new=np.asarray(ctx, np.int32))
+    q, qr = (oracle.bf16_from_f32(rng.standard_normal((B, 1, heads, w)).astype(np.float32)) for w in (DH, DHR))
+    wuk, wuv = (oracle.bf16_from_f32(rng.standard_normal((DC, heads * DH)).astype(np.float32) * 0.02) for _ in range(2))
+    d_uk, d_uv = dev.upload(wuk), dev.upload(wuv)
+    out = np.full((B, 1, heads, DH), np.nan, np.float32)
+    pool.decode(0, B, q, out, heads, DH, (DH + DHR) ** -0.5, q_rope=qr, w_uk=d_uk, w_uv=d_uv)
+    ref = (oracle.f32_from_bf16(c).astype(np.float64) @ oracle.f32_from_bf16(wuv)).reshape(out.shape)
+    assert np.max(np.abs(out - ref)) <= 1e-5 * np.sqrt(np.mean(ref ** 2))
+    pool.destroy()
+    d_uk.free()
+    d_uv.free()
