@@ -236,7 +236,7 @@ int32_t relux_pool_tune(relux_pool_t pool, int32_t knob, int32_t value);
  * the handle's compute stream: inputs into one of two staging slots on the device, outputs from one of two result
  * slots, with events between the streams.  The call returns as soon as its work is queued, so the copies of the next
  * call overlap the kernels of this one.  Rules for the caller: pass page-locked buffers (relux_cuda_host_alloc) --
- * pageable ones make the copies synchronous --; leave an input buffer unchanged, and an output buffer unread, until
+ * pageable ones make the copies synchronous --; leave an input buffer unchanged (kernels may read it where it is), and an output buffer unread, until
  * relux_pool_wait_output (or relux_cuda_sync) has returned for that call; give calls that may be in flight together
  * different output buffers.  relux_cuda_sync and relux_cuda_event_record cover the copy streams.  The reference has no
  * counterpart: its tensors never leave host memory (internal/alloc/alloc.go:15-18). */

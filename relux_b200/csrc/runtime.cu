@@ -1355,6 +1355,31 @@ static bool gqa_fuse_args_ok(const Pool* p, const relux_append_args* kv, const r
          !(kv->flags & ~RELUX_CALL_PIPELINED) && kv->layer >= 0 && kv->layer < p->prm.num_layers;
 }
 
+// Where the kernels can read a page-locked tensor of the caller's with 16-byte loads; nullptr for other memory.
+static const void* page_locked(const void* ptr) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return at.type == cudaMemoryTypeHost && ((uintptr_t)at.devicePointer & 15u) == 0 ? at.devicePointer : nullptr;
+}
+// A pipelined latent step whose copies outlast its kernels leaves its new rows where they are, for the preparation to read over PCIe: two small copies
+// fewer, which take a turn of the copy engine each (64 sequences, 128 heads: 3.3 MB in by four copies, 2.1 MB out).  Steps of several pools in turn move
+// with the phase of the copies in and out, which slow each other down: 64 x 200 / 300 / 500 / 700 tokens took 97 us while the kernels were 12 us slower, then 105
+// / 103 / 101 / 98, and 84 / 83 / 83 / 90 with rows read in place; 100 x 300 140, 152, 129.  One pool in a loop, copied -> in place: 107 -> 107, 107 -> 107, 110 ->
+// 108, 111 -> 110, 155 -> 156.  Not for fewer bytes (48 x 400, 3.9 MB: 78 -> 72 with several pools, 88 -> 90 with one; 24 x 300 51 -> 54) or more (128 x 300, 10.6 MB:
+// 188 -> 186, one pool 188 -> 193), nor ahead of longer kernels, which wait for the rows (64 x 1000 one pool 110 -> 117, 64 x 4000 107 -> 113, 64 x 32768
+// 625 -> 641).
+static bool rows_in_place(const Pool* p, const SeqBatch& sb, const relux_attn_args& a, int layer, size_t row_bytes) {
+  if (!pipes_queries(p, a) || !pipes_output(p, a)) return false;
+  const size_t rows = (size_t)sb.n_seqs * a.q_tokens * a.num_heads;
+  const size_t copied = row_bytes + rows * (a.head_dim + p->prm.mla_dhr) * dtype_size(a.q_dtype) + rows * a.head_dim * dtype_size(a.out_dtype);
+  size_t cached = 0;
+  for (int i = 0; i < sb.n_seqs; i++) cached += (size_t)p->h_len[(size_t)layer * p->prm.max_seqs + sb.seq[i]] * p->row_elems_a * 2;
+  return copied >= (size_t)9 << 19 && copied <= (size_t)9 << 20 && cached <= 9 * copied && row_bytes <= copied / 16;
+}
+
 static int32_t do_verify(Pool* p, const relux_attn_args* attn, const relux_append_args* kv, int kind) {
   if (!attn || !kv) { set_error("nil argument struct"); return RELUX_ERR_INVALID_ARG; }
   if (kv->advance != 0) { set_error("verify: draft rows must be appended with advance=0"); return RELUX_ERR_INVALID_ARG; }
@@ -1406,7 +1431,8 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   const bool piped = (kv->flags & RELUX_CALL_PIPELINED) && kv->mem == RELUX_MEM_HOST && p->dev->h2d_stream;
   const void *da = nullptr, *db = nullptr;
   int slot_a = -1, slot_b = -1;
-  if (piped) {
+  if (piped && rows_in_place(p, sb, *attn, kv->layer, bytes_a + bytes_b) && (da = page_locked(kv->a)) && (db = page_locked(kv->b))) {
+  } else if (piped) {
     if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes_a, false, &da, &slot_a))) return rc;
     if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes_b, !pipes_queries(p, *attn), &db, &slot_b))) return rc;
   } else if (kv->mem == RELUX_MEM_HOST) {

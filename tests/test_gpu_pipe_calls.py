@@ -65,3 +65,55 @@ def test_calls_of_all_kinds_in_turn(dev, oracle, kind):  # noqa: F811
     assert pools[1].status() == 0
     for p in pools:
         p.destroy()
+
+
+@pytest.mark.parametrize("rows", ["page_locked", "unaligned", "pageable", "one_of_each"])
+def test_large_steps_over_short_sequences(dev, oracle, rows):  # noqa: F811
+    """Steps whose copies outlast their kernels read page-locked new rows where they are, others are copied; a call's inputs are overwritten as soon as its
+    output has landed, two calls are in flight, against ordinary steps."""
+    from relux_b200 import lib as L
+    B, H, D, steps = 64, 128, 128, 5
+    ctx = [3 + (i * 37) % 150 for i in range(B)]
+    pools = [build_mla(dev, oracle, np.random.default_rng(5), ctx, 512, 64)[0] for _ in range(2)]
+    rng = np.random.default_rng(6)
+    bf = lambda *s: oracle.bf16_from_f32(rng.standard_normal(s).astype(np.float32))  # noqa: E731
+    more = dict(w_uk=dev.upload(bf(512, H * D)), w_uv=dev.upload(bf(512, H * D)), q_dtype=L.DTYPE_BF16, out_dtype=L.DTYPE_BF16)
+    held = []
+
+    def pinned(a, shift=0):
+        h = dev.pinned((a.size + 4,), a.dtype)
+        held.append(h)
+        view = h.array[shift:shift + a.size].reshape(a.shape)
+        view[...] = a
+        return view
+
+    def place(a, k):
+        if rows == "pageable" or (rows == "one_of_each" and k):
+            return a.copy()
+        return pinned(a, 1 if rows == "unaligned" else 0)
+    want, got, calls = [], [], []
+    for i in range(steps):
+        new = [rng.standard_normal((B, w)).astype(np.float32) for w in (512, 64)]
+        q, qr, out = bf(B, 1, H, D), bf(B, 1, H, 64), np.zeros((B, 1, H, D), np.uint16)
+        pools[0].step(0, B, *new, q, out, H, D, 0.08, q_rope=qr, **more)
+        want.append(out)
+        mine = [place(new[k], k) for k in range(2)] + [pinned(q), pinned(qr), pinned(np.full_like(out, 0x7fc0))]
+        pools[1].step(0, B, mine[0], mine[1], mine[2], mine[4], H, D, 0.08, q_rope=mine[3], **more, pipelined=True)
+        calls.append(mine)
+        for k in range(2 if i == steps - 1 else 1):
+            if i + k >= 1:
+                pools[1].wait_output(1 - k)
+                got.append(calls[i - 1 + k][4].copy())
+                for a in calls[i - 1 + k][:4]:
+                    a[...] = 3
+    for i in range(steps):
+        assert np.array_equal(got[i], want[i]), i
+    dev.sync()
+    for s in range(0, B, 7):
+        for x, y in zip(*(p.read_rows(0, s, 0, ctx[s] + steps) for p in pools)):
+            assert np.array_equal(x, y)
+    assert pools[1].status() == 0
+    for p in pools:
+        p.destroy()
+    for b in ("w_uk", "w_uv"):
+        more[b].free()
