@@ -206,7 +206,7 @@ int32_t relux_pool_read_rows(relux_pool_t pool, const relux_read_rows_args* args
 #define RELUX_TUNE_MLA_WORKERS 1        /* RELUX_MLA_WORKERS: ranges the stream of pages is cut into (0 = resident pairs);
                                            longer ones for a sequence that would have more than 240 of them                */
 #define RELUX_TUNE_CHUNK_PAGES 2        /* RELUX_CHUNK_PAGES: chunk length of the split-KV planner (0 = chosen per call;
-                                           raised for a latent sequence that it would cut into more than 240 chunks)       */
+                                           raised where a sequence of latents of 128 or more would have more than 240 chunks) */
 #define RELUX_TUNE_GEMM_GENERIC 3       /* RELUX_GEMM_GENERIC: 1 = projections on the plain kernel                          */
 #define RELUX_TUNE_GEMM_SPLIT 4         /* RELUX_GEMM_SPLIT: workers per tile (128 weight columns x a block of rows) of the tcgen05
                                            GEMM (0 = one worker per SM, the split along K chosen per call)                 */

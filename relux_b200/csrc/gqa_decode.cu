@@ -196,7 +196,7 @@ static int32_t launch_gqa_prompt(Pool* p, const SeqBatch& sb, const relux_attn_a
   // every work item becomes groups x kv heads CTAs, so the planner may keep the chunks long: a prompt fills the SMs
   // through its slices, and a CTA that streams many pages amortises its prologue
   SplitPlan plan;
-  int32_t rc = plan_splitkv(p, sb, a.layer, a.extra_tokens, prm.gqa_num_kv_heads * groups, 2, 1, 0, &plan);
+  int32_t rc = plan_splitkv(p, sb, a.layer, a.extra_tokens, prm.gqa_num_kv_heads * groups, 2, 1, 0, 0, &plan);
   if (rc) return rc;
   const int rows_total = per_group * a.num_heads;
   const size_t group_rows = (size_t)plan.num_items * rows_total;

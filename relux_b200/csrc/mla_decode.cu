@@ -301,7 +301,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   const bool chained = p->tune.get(RELUX_TUNE_CHAINED_LAUNCHES) != 0;
   // persistent CTA pairs over a stream partition; ranges are whole 128-token tiles
   rc = sm100 ? plan_stream(p, sb, a.layer, a.extra_tokens, mla_sm100_workers(p, S), 2, &plan, fused_prep ? to_list : nullptr)
-             : plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, &plan);
+             : plan_splitkv(p, sb, a.layer, a.extra_tokens, std::max(1, rows_total / 16), 1, 1, 0, proj_mma ? kMaxRowItems : 0, &plan);
   if (!rc) rc = grow_partials(p, plan, rows_total, dC);   // before the launch that appends: a call without memory leaves the cache as it was
   if (rc) return rc;
   // rows of one piece each are rounded where they are written

@@ -67,7 +67,7 @@ __global__ void build_worklist_kernel(const int32_t* __restrict__ len, const int
 // epilogue (partial write + its share of the merge) of one item.  All candidates are evaluated and the
 // cheapest wins, which avoids a nearly empty last wave (e.g. 4.3 waves costing 5).
 int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas_per_item, int min_chunk_pages, int chunk_multiple,
-                     int max_chunk_pages, SplitPlan* plan) {
+                     int max_chunk_pages, int max_row_items, SplitPlan* plan) {
   const relux_pool_params& prm = p->prm;
   std::vector<int> pages(sb.n_seqs);
   int max_pages = 1;
@@ -102,7 +102,7 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
     chunk = (chunk + mult - 1) / mult * mult;
     if (max_chunk_pages > 0) chunk = std::min(chunk, max_chunk_pages / mult * mult);
   }
-  while ((max_pages + chunk - 1) / chunk > kMaxRowItems && max_chunk_pages <= 0) chunk += mult;
+  while (max_row_items > 0 && (max_pages + chunk - 1) / chunk > max_row_items) chunk += mult;
   int items = 0;
   plan->first.assign(1, 0);
   for (int i = 0; i < sb.n_seqs; i++) plan->first.push_back(items += (pages[i] + chunk - 1) / chunk);

@@ -64,8 +64,9 @@ enum PartialForm { kPartialFloat32 = 0, kPartialOne = 1, kPartialHalves = 2 };
 
 struct Pool;
 struct SeqBatch;
+// `max_row_items`: more chunks than that no sequence is cut into (0: any number).
 int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas_per_item, int min_chunk_pages, int chunk_multiple,
-                     int max_chunk_pages, SplitPlan* plan);
+                     int max_chunk_pages, int max_row_items, SplitPlan* plan);
 // Stream partition for persistent kernels: the sequences of the call, laid end to end, are cut into at most `workers` equal ranges;
 // one item = the part of one sequence inside one range, so a worker meets an item boundary only where a sequence ends inside its
 // range.  Where that is cheaper they are cut sequence by sequence instead, one item a worker (cheapest_plan).  With the tuning knob

@@ -73,3 +73,23 @@ def test_more_workers_than_a_row_may_have_pieces(dev, oracle):  # noqa: F811
     pool.destroy()
     wuk.free()
     wuv.free()
+
+
+def test_chunks_of_other_calls_have_no_such_limit(dev, oracle):  # noqa: F811
+    """A grouped-query prompt in slices takes chunks as short as the knob says over 300 pages as over 60: pieces of one page and of two add up in another
+    order, so that their bits differ."""
+    from relux_b200 import lib as L
+    from tests.test_gpu_attention import build_gqa
+    H, Hkv, D, S = 16, 8, 128, 40
+    for tokens in (60 * 64, 300 * 64):
+        rng = np.random.default_rng(tokens)
+        pool = build_gqa(dev, oracle, rng, [tokens], Hkv, D)[0]
+        pool.tune(L.TUNE_GQA_PROMPT_SLICES, 1)
+        q, outs = rng.standard_normal((1, S, H, D)).astype(np.float32), []
+        for pages in (1, 2, 1):
+            pool.tune(L.TUNE_CHUNK_PAGES, pages)
+            outs.append(np.empty_like(q))
+            pool.decode(0, 1, q, outs[-1], H, D, D ** -0.5, q_tokens=S)
+        assert np.array_equal(outs[0], outs[2]) and not np.array_equal(outs[0], outs[1])
+        assert np.max(np.abs(outs[0] - outs[1])) <= 1e-2 * np.sqrt(np.mean(outs[0] ** 2)) + 5e-3
+        pool.destroy()
