@@ -210,39 +210,6 @@ __device__ __forceinline__ void fence_chained_writes() { asm volatile("fence.pro
 // while the kernel exists, and which the compiler may move ahead of chain_wait().
 template <typename T>
 __device__ __forceinline__ T load_chained(const T* p) { return __ldcg(p); }
-// The same through L1 and free for the compiler to move among other accesses (the merge of partials lost 1 us of 11 with loads that
-// keep their place between its stores): only on pointers that have come through behind_wait(), which keeps them behind the wait.
-template <typename T>
-__device__ __forceinline__ const T* behind_wait(const T* p) {
-  asm volatile("" : "+l"(p)::"memory");
-  return p;
-}
-__device__ __forceinline__ int32_t load_settled(const int32_t* p) {
-  int32_t v;
-  asm("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
-  return v;
-}
-__device__ __forceinline__ float load_settled(const float* p) {
-  float v;
-  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
-  return v;
-}
-__device__ __forceinline__ float2 load_settled(const float2* p) {
-  float2 v;
-  asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(__cvta_generic_to_global(p)));
-  return v;
-}
-// The float4 at p, or zeros without a load where `there` is false: a predicate, not a branch around every load.
-__device__ __forceinline__ float4 load_settled_if(const float4* p, bool there) {
-  float4 v;
-  asm("{\n\t.reg .pred t;\n\t"
-      "setp.ne.s32 t, %5, 0;\n\t"
-      "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\tmov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-      "@t ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "=&f"(v.x), "=&f"(v.y), "=&f"(v.z), "=&f"(v.w)
-      : "l"(__cvta_generic_to_global(p)), "r"((int)there));
-  return v;
-}
 
 // Stores with an L2 eviction priority: evict_last for what a later launch reads while other data streams through L2.
 __device__ __forceinline__ uint64_t make_evict_last_policy() {

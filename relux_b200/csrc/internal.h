@@ -315,7 +315,7 @@ inline void count_launch(Device* d, int n = 1) { d->launches += n; }
 //   1. Every such kernel calls chain_wait() in the threads that write, and in those that read what a launch of the chain
 //      writes, before they do.  A kernel is complete only when all its threads are, so "the launch before me is complete" holds
 //      back to the first launch of the chain.
-//   2. What a launch of the chain writes is read by load_chained(), by load_settled() or by plain loads of pointers that are not
+//   2. What a launch of the chain writes is read by load_chained() or by plain loads of pointers that are not
 //      const __restrict__, and by TMA only where the writer has called fence_chained_writes().
 //   3. Before its wait a kernel may read what was complete before the HEAD of its chain began.  A head is a plain launch, a launch
 //      behind a copy or an event, or one whose blocks all wait before they release: cast_bf16_kernel, and mla_prep_kernel

@@ -25,18 +25,19 @@ struct VupShape {
   bool fits() const { return most <= kVupMaxCols && tmem_cols <= 512; }
 };
 
-// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU (`fit` groups do), more where they do not and there are more than 40
-// columns (52 where only two groups fit), of about 32 columns each, or where a group would have more columns than it has room for.  (One group -> two of
-// 24 to 32: 32 heads, 16 x 300 tokens 17.9 -> 16.5 us, 10 x 600 18.0 -> 16.8, 50 x 600 26.9 -> 25.3, 64 heads, 30 x 800 26.4 -> 25.6; not at 48 columns
-// of 64 heads, 12 x 900 21.4 -> 22.1, nor at 36 of 32, 12 x 300 15.6 -> 17.2.)  A group's columns are one block where a stage of it, 64 latent columns,
-// fits the ring four times, and equal blocks otherwise.
+// Rows (n_seqs x S) are dealt to groups of CTAs: one where the heads fill the GPU (`fit` groups do), more, of about 32 columns each, where they do not, or where
+// a group would have more columns than it has room for.  The second group comes with 41 columns, or with 53 where no third one would fit.  Steps with one group
+// and with two, us, by columns: 32 heads 33 20.7 / 20.8, 36 17.9 / 17.8, 39 25.0 / 25.2, 42 17.7 / 17.5, 45 19.4 / 18.0, 48 19.7 / 17.7, 51 19.2 / 18.1, 54 23.5 /
+// 22.0, 57 20.9 / 18.5, 60 18.0 / 16.8; 64 heads 41 27.4 / 26.3, 45 24.4 / 24.6, 49 28.9 / 28.9, 53 22.1 / 22.3, 57 22.5 / 22.5, 61 22.3 / 22.4, 65 24.5 / 23.6, 69
+// 34.1 / 33.6.  A group's columns are one block where a stage of it, 64 latent columns, fits the ring four times, and equal blocks otherwise.
 // `first`: the plan's pieces at the host's lengths.  With `workers` the launch may find other lengths, on which the builder cuts at most workers - 1
 // sequences once more each (build_stream): what a group then has at most is its rows, and every cut once for each of its rows of the sequence.
 inline VupShape vup_shape(const std::vector<int32_t>& first, int rows, int S, int fit, int halves, int dC, int workers) {
   VupShape k;
   const int all = vup_col(first, S, rows);
   // (a row at a time fewer, from as many groups as the columns need at least: all numbers of groups in turn were quadratic in the rows)
-  int groups = std::max({1, std::min({fit, (all + (fit > 2 ? 23 : 11)) / 32, rows}), workers > 0 ? 1 : std::min(rows, (all + kVupMaxCols - 1) / kVupMaxCols)});
+  const int second = fit > 2 ? 41 : 53;
+  int groups = std::max({1, std::min({fit, (all + 64 - second) / 32, rows}), workers > 0 ? 1 : std::min(rows, (all + kVupMaxCols - 1) / kVupMaxCols)});
   for (;; groups = (rows + k.rows_each - 2) / (k.rows_each - 1)) {
     k.rows_each = (rows + groups - 1) / groups;
     k.most = 0;
