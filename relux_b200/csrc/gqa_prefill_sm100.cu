@@ -605,7 +605,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       if (lane == 0) mbar_arrive(&bars->l_full);
       // After an abort no more items are written.  The warp leaves as one (the tensor-memory loads are its lanes' together), by a vote behind its own wait:
       // a lane whose wait ran out has raised the flag or seen it.
-      if (__any_sync(0xffffffffu, !it.more || bars->abort_flag != 0)) break;
+      // (With `more` in the vote the kernel took 122 registers instead of 117, and 8 x 2048 tokens 331.4 us instead of 330.4.)
+      if (!it.more) break;
+      if (__any_sync(0xffffffffu, bars->abort_flag != 0)) break;
       it = bars->items[(n + 1) & 3];
     }
   } else {
