@@ -138,13 +138,13 @@ struct PageWin {
 // the order in which a lane holds them, column 8 i + 2 q + e at place 8 q + 2 i + e (mla_vup_pieces_kernel loads W_UV's rows in that
 // order), and a chunk passes through 4 KB of the P tile that belong to the warp, so that its stores are whole lines and no warp waits for
 // another.  Two halves (hi = the upper 16 bits of x, lo = bf16(x - hi), which is off by less than 2^-16 of x) where rows have several
-// pieces.  Where every row has one, that is its whole attention: over its sum (`norm` = 1 / sum) it is the up-projection's operand, and is rounded to bf16
+// pieces.  Where every row has one, that is its whole attention: over its sum (`l_row`) it is the up-projection's operand, and is rounded to bf16
 // here, float32 up to then.  (Rounded ahead of the norm, the error was 0.997-1.002 times as large.)  merge_splits_kernel reads float32.
 // Bound: an SM writes 32 bytes a clock, whether by stores of whole lines (128 KB in 4.0 k clocks, one CTA or all) or by TMA (4.3-5.2 k);
 // stores of 64 bytes a row take twice as long, and so did 64 TMA stores of 2 KB.  An
 // item takes 3.1 us as two halves, as it did in float32, and 1.8 in one.
 template <int kForm>
-__device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, void* part_o, int H, int piece, int head0, float m_used, float norm, bool ok) {
+__device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, void* part_o, int H, int piece, int head0, float m_used, float l_row, bool ok) {
   constexpr int kRowElems = kForm == kPartialOne ? kDC : 2 * kDC;   // bf16 forms
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
   // The partial results (256 KB an item at 128 heads: 17 MB in 64 pieces, 36 MB in 138 items of ranges) wait for the merge while cached
@@ -160,6 +160,12 @@ __device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, vo
   uint32_t v[32];
   auto load = [&](int u) { tmem_ld_16x256b_x8(tmem_o + ((uint32_t)(warp * 32 + (u >> 2) * 16) << 16) + (u & 3) * 64, v); };
   load(0);
+  float norms[4] = {1.f, 1.f, 1.f, 1.f};   // of this lane's rows
+  if constexpr (kForm == kPartialOne) {
+    const float norm = l_row > 0.f ? rcp_normal(l_row) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) norms[k] = __shfl_sync(0xffffffffu, norm, (lane >> 2) + 8 * k);
+  }
 #pragma unroll 1
   for (int u = 0; u < 8; u++) {   // 4 * (half of the rows) + 64-column chunk
     tmem_ld_wait_for(v);
@@ -183,16 +189,15 @@ __device__ __forceinline__ void write_partial(uint8_t* smem, uint32_t tmem_o, vo
       // A row without a visible key may hold anything: the up-projection leaves it out by its maximum.
       uint32_t hi[16], lo[16];   // [row of two][32 columns of two][4]
       float big[4] = {0.f, 0.f, 0.f, 0.f};
-      float norms[2] = {1.f, 1.f};
-      if constexpr (kForm == kPartialOne) {
-        norms[0] = __shfl_sync(0xffffffffu, norm, (u >> 2) * 16 + (lane >> 2));
-        norms[1] = __shfl_sync(0xffffffffu, norm, (u >> 2) * 16 + (lane >> 2) + 8);
-      }
+      const float na = u < 4 ? norms[0] : norms[2], nb = u < 4 ? norms[1] : norms[3];
+      const uint64_t norm2[2] = {pack2(na, na), pack2(nb, nb)};
 #pragma unroll
       for (int w = 0; w < 16; w++) {
         const uint32_t x = v[4 * (w & 7) + 2 * (w >> 3)], y = v[4 * (w & 7) + 2 * (w >> 3) + 1];
         if constexpr (kForm == kPartialOne) {
-          hi[w] = round_bf16x2(__uint_as_float(x) * norms[w >> 3], __uint_as_float(y) * norms[w >> 3]);
+          float a, b;
+          unpack2(mul2(pack2(__uint_as_float(x), __uint_as_float(y)), norm2[w >> 3]), a, b);
+          hi[w] = round_bf16x2(a, b);
         } else {
           hi[w] = __byte_perm(x, y, 0x7632);
           lo[w] = round_bf16x2(__uint_as_float(x) - bf16_hi(x), __uint_as_float(y) - bf16_hi(y));
@@ -573,7 +578,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
       tc_fence_after();
       bars->lsum[L] = l_run;
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float l_row = bars->lsum[row] + bars->lsum[64 + row], norm = l_row > 0.f ? 1.0f / l_row : 0.f;
+      const float l_row = bars->lsum[row] + bars->lsum[64 + row];
       const bool real_head = 64 * (int)rank + row < prm.H;   // padding rows of the tile are not written
       // the pieces of a row lie one behind another where the up-projection reads them, item by item where merge_splits_kernel does
       const int piece = prm.form != kPartialFloat32 ? cur.first * prm.S + sq * cur.n + (it - cur.first) : it * prm.S + sq;
@@ -583,9 +588,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         prm.part_ml[prow * 2 + 1] = !ok ? 0.f : prm.form != kPartialOne ? l_row : l_row > 0.f ? 1.f : 0.f;
       }
       if (64 * (int)rank + 32 * (warp & 1) >= prm.H) {   // none of the warp's rows is a head
-      } else if (prm.form == kPartialHalves) write_partial<kPartialHalves>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, norm, ok);
-      else if (prm.form == kPartialOne) write_partial<kPartialOne>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, norm, ok);
-      else write_partial<kPartialFloat32>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, norm, ok);
+      } else if (prm.form == kPartialHalves) write_partial<kPartialHalves>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, l_row, ok);
+      else if (prm.form == kPartialOne) write_partial<kPartialOne>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, l_row, ok);
+      else write_partial<kPartialFloat32>(smem, tmem + kTmemO, prm.part_o, prm.H, piece, 64 * (int)rank, m_used, l_row, ok);
       tc_fence_before();   // the O read-out is ordered before this thread's next p_full arrival, which releases the first PV of the next item
       cur = nxt;
     }

@@ -344,7 +344,7 @@ __global__ void mla_expand_plan_kernel(const int32_t* __restrict__ len, const in
       rows = (T + kTokTile - 1) / kTokTile * kTokTile;
     }
     int total;
-    const int before = prep_block_excl_scan(rows, s_warp, &total);
+    const int before = prep_block_excl_scan<8>(rows, s_warp, &total);
     if (i < n_seqs) seq_base[i] = base + before;
     base += total;
   }

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_
     const int i = e * kWarps + (threadIdx.x >> 5);
     if (threadIdx.x < 32 * kWarps && i < ap.n_seqs) prep_append_seq(ap, i, pl.listed != 0);
   } else {
-    prep_build_stream(ap, pl);
+    prep_build_stream<(kTc ? kAbsorbThreads : kAbsorbMmaThreads) / 32>(ap, pl);
   }
   if (!pl.listed) prep_arrive_and_advance(ap, (uint32_t)chores);
 }

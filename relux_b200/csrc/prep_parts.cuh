@@ -100,9 +100,10 @@ __device__ __forceinline__ void prep_append_seq(const PrepAppend& g, int i, bool
   fence_chained_writes();
 }
 
-// Exclusive prefix sum over a block of up to 1024 threads; *total receives the block's sum.
+// Exclusive prefix sum over a block of kWarps warps; *total receives the block's sum.
+template <int kWarps>
 __device__ __forceinline__ int prep_block_excl_scan(int v, int32_t* s_warp, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int incl = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -113,7 +114,8 @@ __device__ __forceinline__ int prep_block_excl_scan(int v, int32_t* s_warp, int*
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
   int base = 0, sum = 0;
-  for (int w = 0; w < nw; w++) {
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) {
     if (w < warp) base += s_warp[w];
     sum += s_warp[w];
   }
@@ -126,9 +128,9 @@ __device__ __forceinline__ int prep_block_excl_scan(int v, int32_t* s_warp, int*
 // The plan was made for the lengths that the host knows.  Where the device's are others (SplitPlan::loose) and have outgrown its workers or its room,
 // the sequences are cut into equal ranges for as many workers instead, n_seqs + workers - 1 items at most.  That serves all lengths; if it did not, the
 // plan would be empty and the status would say so: nothing is written past its room.
-template <typename Tokens>
+template <int kWarps, typename Tokens>
 __device__ __forceinline__ void build_stream(const PrepPlan& pl, int n_seqs, const int32_t* seq_ids, int page_tokens, int32_t* status, Tokens tokens_of) {
-  __shared__ int32_t s_warp[32];
+  __shared__ int32_t s_warp[kWarps];
   int by_item = pl.by_item, G = pl.G, start_units = pl.start_units;
 #pragma unroll 1
   for (int pass = 0;; pass++) {
@@ -142,9 +144,9 @@ __device__ __forceinline__ void build_stream(const PrepPlan& pl, int n_seqs, con
         pages = (tokens + page_tokens - 1) / page_tokens;
       }
       int tot_units, tot_items;
-      const int at = unit_base + prep_block_excl_scan(SeqCut(by_item, G, start_units, 0, pages).units, s_warp, &tot_units);
+      const int at = unit_base + prep_block_excl_scan<kWarps>(SeqCut(by_item, G, start_units, 0, pages).units, s_warp, &tot_units);
       const SeqCut cut(by_item, G, start_units, at, pages);
-      const int c0 = item_base + prep_block_excl_scan(cut.n, s_warp, &tot_items);
+      const int c0 = item_base + prep_block_excl_scan<kWarps>(cut.n, s_warp, &tot_items);
       if (i < n_seqs) {
         pl.chunk_off[i] = c0;
         for (int c = 0; c < cut.n && c0 + c < pl.room; c++) {
@@ -183,7 +185,7 @@ __device__ __forceinline__ void build_stream(const PrepPlan& pl, int n_seqs, con
       const int i = i0 + threadIdx.x;
       int pages = 0, tot;
       if (i < n_seqs) pages = (tokens_of(i, seq_ids ? seq_ids[i] : i) + page_tokens - 1) / page_tokens;
-      prep_block_excl_scan(SeqCut(0, 1, kStartUnits, 0, pages).units, s_warp, &tot);
+      prep_block_excl_scan<kWarps>(SeqCut(0, 1, kStartUnits, 0, pages).units, s_warp, &tot);
       units += tot;
     }
     by_item = 0;
@@ -194,8 +196,9 @@ __device__ __forceinline__ void build_stream(const PrepPlan& pl, int n_seqs, con
 
 // The same over the lengths AFTER this step's append (the append of the same launch has not advanced them yet: every sequence counts its cached rows +
 // its new rows + extra).
+template <int kWarps>
 __device__ __forceinline__ void prep_build_stream(const PrepAppend& g, const PrepPlan& pl) {
-  build_stream(pl, g.n_seqs, g.seq_ids, g.page_tokens, g.status, [&](int i, int seq) {
+  build_stream<kWarps>(pl, g.n_seqs, g.seq_ids, g.page_tokens, g.status, [&](int i, int seq) {
     return load_chained(g.len + seq) + (g.row_off ? g.row_off[i + 1] - g.row_off[i] : g.rows_each) + pl.extra;
   });
 }

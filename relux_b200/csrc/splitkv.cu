@@ -127,7 +127,7 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
 __global__ void build_stream_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra, int page_tokens,
                                     const __grid_constant__ PrepPlan pl, int32_t* status) {
   chain_release();
-  build_stream(pl, n_seqs, seq_ids, page_tokens, status, [&](int, int seq) { return load_chained(len + seq) + extra; });
+  build_stream<8>(pl, n_seqs, seq_ids, page_tokens, status, [&](int, int seq) { return load_chained(len + seq) + extra; });
   chain_wait();
 }
 
