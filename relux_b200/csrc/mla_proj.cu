@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kTc ? kAbsorbThreads : kAbsorbMmaThreads) mla_
 // -> 7.2; 3 x <= 1500, 27 pieces 4.1 -> 3.5; one sequence 3.8 -> 2.4.  Bound: with many pieces what the partials take from L2 (35 bytes a clock
 // and SM), else the round trips of a stage, of 32 MMAs (1.5 k clocks) and of the outputs.
 // An MMA of up to 64 columns takes 40-48 clocks for its 4 KB of weights, so the halves of a block of columns stand side by side as N and the
-// weights are read once for both: 32 MMAs a block.  Rows of one piece each come rounded to bf16 where they were written, without a lo.
+// weights are read once for both: 32 MMAs a block.  Rows of one piece each come divided by their sum (their part_ml has 1) and rounded to bf16, without a lo.
 // A launch finds its instructions in no cache, and what is executed once is waited for: clock stamps had 2 k clocks between the wait and the
 // first MMA, 2.4 k for the first outputs, 4 k for the weights of three rows.  So the loops are rolled, and the warps that have nothing to do
 // before the wait go through theirs once, on whatever memory holds, without storing.

@@ -59,7 +59,8 @@ struct SplitPlan {
   int32_t* worker_first = nullptr;     // device [num_workers + 1]
 };
 
-// A row of a latent call's partial results: float32, one bf16 value or two bf16 halves a column (write_partial, mla_decode_sm100.cu).
+// A row of a latent call's partial results: float32, the bf16 value of the row's whole attention or two bf16 halves a column (write_partial,
+// mla_decode_sm100.cu).
 enum PartialForm { kPartialFloat32 = 0, kPartialOne = 1, kPartialHalves = 2 };
 
 struct Pool;
