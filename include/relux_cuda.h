@@ -182,7 +182,8 @@ int32_t relux_seq_len(relux_pool_t pool, int32_t layer, int32_t seq_id, int32_t*
  * such call: its speculative decoder never removes rejected draft rows from the cache (speculative.go:136-156). */
 int32_t relux_seq_set_len(relux_pool_t pool, int32_t layer, int32_t n_seqs, const int32_t* seq_ids,
                           const int32_t* new_len);
-/* Reads the device status word (0, or the first RELUX_ERR_BAD_PAGE / RELUX_ERR_TIMEOUT a kernel recorded)
+/* Reads the device status word (0, or the first RELUX_ERR_BAD_PAGE / RELUX_ERR_TIMEOUT a kernel recorded, or
+ * RELUX_ERR_UNSUPPORTED: a graph found lengths that the scratch of its calls has no room for, and their output is zero or as it was)
  * and clears it.  Synchronises the stream.  No counterpart in the reference (its checks panic on the host). */
 int32_t relux_pool_status(relux_pool_t pool, int32_t* status);
 /* KVCache.View / MLACache.View equivalent used by the bit-exactness tests (kvcache.go:363-380,

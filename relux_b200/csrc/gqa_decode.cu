@@ -411,7 +411,8 @@ extern "C" __attribute__((visibility("default"))) int32_t relux_gqa_decode_noall
   float* d_part_o = d_part_ml + (size_t)items * rows_total * 2;
   cudaStream_t st = dev->stream;
   const int32_t* len = p->d_len + (size_t)a->layer * prm.max_seqs;
-  rc = launch_build_worklist_raw(st, len, sb.d_seq_ids, sb.n_seqs, a->extra_tokens, prm.page_tokens, chunk, d_items, d_chunk_off);
+  rc = launch_build_worklist_raw(st, len, sb.d_seq_ids, sb.n_seqs, a->extra_tokens, prm.page_tokens, chunk, d_items, d_chunk_off,
+                                 (int)items, p->d_status);
   if (rc) return rc;
   count_launch(dev);
   GqaParams k{};

@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(256) mla_decode_generic_kernel(const MlaGenPar
   uint32_t* qsm = smw + kTile * stride_w;            // [kRows][roww/2]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const WorkItem item = prm.items[blockIdx.x];
+  if (item.page_begin >= item.page_end) return;   // of no page: the place of its rows is another's
   const int T = prm.len[item.seq] + prm.extra;
   const int row_base = blockIdx.y * kRows;
   for (int e = threadIdx.x; e < kRows * (roww / 2); e += blockDim.x) {

@@ -15,9 +15,12 @@
 namespace relux {
 
 // One block of 256 threads: every thread counts the chunks of its sequences, a block-wide exclusive scan gives the
-// offsets, then every thread writes the items of its sequences.
+// offsets, then every thread writes the items of its sequences.  There is room for `room` of them, as many as the host counts at its lengths.  In a graph
+// the device's may be others: where there are fewer items the rest are of no page, and where there are more every sequence has none (its attention is
+// zero) and the status word says so.
 __global__ void build_worklist_kernel(const int32_t* __restrict__ len, const int32_t* __restrict__ seq_ids, int n_seqs, int extra,
-                                      int page_tokens, int chunk_pages, WorkItem* __restrict__ items, int32_t* __restrict__ chunk_off) {
+                                      int page_tokens, int chunk_pages, WorkItem* __restrict__ items, int32_t* __restrict__ chunk_off, int room,
+                                      int32_t* status) {
   __shared__ int32_t s_warp[8];
   __shared__ int32_t s_base;
   if (threadIdx.x == 0) s_base = 0;
@@ -45,7 +48,7 @@ __global__ void build_worklist_kernel(const int32_t* __restrict__ len, const int
     const int c0 = s_base + wbase + incl - nc;
     if (i < n_seqs) {
       chunk_off[i] = c0;
-      for (int c = 0; c < nc; c++) {
+      for (int c = 0; c < nc && c0 + c < room; c++) {
         WorkItem w;
         w.seq_index = i;
         w.seq = seq;
@@ -58,7 +61,13 @@ __global__ void build_worklist_kernel(const int32_t* __restrict__ len, const int
     if (threadIdx.x == blockDim.x - 1) s_base = c0 + nc;   // running total after this batch of sequences
     __syncthreads();
   }
-  if (threadIdx.x == 0) chunk_off[n_seqs] = s_base;
+  if (s_base <= room) {
+    if (threadIdx.x == 0) chunk_off[n_seqs] = s_base;
+    for (int c = s_base + threadIdx.x; c < room; c += blockDim.x) items[c] = WorkItem{0, 0, 0, 0};
+    return;
+  }
+  if (threadIdx.x == 0) set_status(status, RELUX_ERR_UNSUPPORTED);
+  for (int i = threadIdx.x; i <= n_seqs; i += blockDim.x) chunk_off[i] = 0;
 }
 
 // Chooses the chunk length.  CTAs are scheduled in waves over the SMs, so the step time is about
@@ -116,7 +125,7 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
   plan->chunk_off = (int32_t*)((char*)p->work.p + off);
   const int32_t* len = p->d_len + (size_t)layer * prm.max_seqs;
   build_worklist_kernel<<<1, 256, 0, p->dev->stream>>>(len, sb.d_seq_ids, sb.n_seqs, extra, prm.page_tokens, chunk, plan->items,
-                                                       plan->chunk_off);
+                                                       plan->chunk_off, items, p->d_status);
   RELUX_CUDA_TRY(cudaGetLastError());
   count_launch(p->dev);
   return RELUX_OK;
@@ -326,8 +335,8 @@ int32_t launch_merge_rows(Pool* p, const SplitPlan& plan, int n_seqs, int rows, 
 
 // Raw launchers on caller-provided buffers (no pool scratch involved).
 int32_t launch_build_worklist_raw(cudaStream_t st, const int32_t* len, const int32_t* seq_ids, int n_seqs, int extra, int page_tokens,
-                                  int chunk_pages, WorkItem* items, int32_t* chunk_off) {
-  build_worklist_kernel<<<1, 256, 0, st>>>(len, seq_ids, n_seqs, extra, page_tokens, chunk_pages, items, chunk_off);
+                                  int chunk_pages, WorkItem* items, int32_t* chunk_off, int room, int32_t* status) {
+  build_worklist_kernel<<<1, 256, 0, st>>>(len, seq_ids, n_seqs, extra, page_tokens, chunk_pages, items, chunk_off, room, status);
   RELUX_CUDA_TRY(cudaGetLastError());
   return RELUX_OK;
 }

@@ -78,7 +78,7 @@ int32_t plan_splitkv(Pool* p, const SeqBatch& sb, int layer, int extra, int ctas
 int32_t plan_stream(Pool* p, const SeqBatch& sb, int layer, int extra, int workers, int page_multiple, SplitPlan* plan, ListedPlan* list);
 int32_t launch_build_stream(Pool* p, const SeqBatch& sb, int layer, int extra, const SplitPlan& plan, bool chained);
 int32_t launch_build_worklist_raw(cudaStream_t st, const int32_t* len, const int32_t* seq_ids, int n_seqs, int extra, int page_tokens,
-                                  int chunk_pages, WorkItem* items, int32_t* chunk_off);
+                                  int chunk_pages, WorkItem* items, int32_t* chunk_off, int room, int32_t* status);
 int32_t launch_merge_raw(cudaStream_t st, const float* part_o, const float* part_ml, const int32_t* chunk_off, int n_seqs, int rows,
                          int width, float* out);
 int32_t launch_merge(Pool* p, const SplitPlan& plan, int n_seqs, int rows, int width, float* out);

@@ -154,3 +154,54 @@ def test_a_graph_that_finds_empty_sequences(dev, oracle, full):  # noqa: F811
     plain.destroy()
     graphed.destroy()
     calls.free()
+
+
+@pytest.mark.parametrize("dc,S", [(64, 1), (128, 1), (128, 3), (64, 2)])
+def test_a_graph_of_the_plain_kernels_whose_chunks_become_fewer_or_more(dev, oracle, dc, S):  # noqa: F811
+    """Latents that the CUDA-core kernels serve.  A decode call captured at ten pages a sequence and launched at one has CTAs without a chunk; captured at
+    one and launched at ten it has more chunks than it has room for: nothing is written past that, zeros, and the status word says so."""
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    B, H, pages = 5, 16, 10
+    rng = np.random.default_rng(dc + S)
+    pool = rb.Pool(dev, L.POOL_MLA, 1, B * pages, 64, B, pages, dC=dc, dHR=DHR)
+    pool.set_tables(np.arange(B * pages, dtype=np.int32).reshape(B, pages))
+    bf = lambda *s: oracle.bf16_from_f32(rng.standard_normal(s).astype(np.float32))  # noqa: E731
+    pool.append(0, bf(B * 640, dc), bf(B * 640, DHR), B, n_new=np.full(B, 640, np.int32))
+    pool.tune(L.TUNE_CHUNK_PAGES, 1)
+    shape = (B, S, H, DH)
+    q, qr, wuk, wuv = (dev.upload(x) for x in (bf(*shape), bf(B, S, H, DHR), bf(dc, H * DH), bf(dc, H * DH)))
+    out = dev.upload(np.full(shape, np.nan, np.float32))
+
+    def call():
+        pool.decode(0, B, q, out, H, DH, 0.01, q_rope=qr, w_uk=wuk, w_uv=wuv, q_tokens=S, q_dtype=L.DTYPE_BF16, out_dtype=L.DTYPE_F32)
+
+    def result():
+        dev.sync()
+        return out.download(shape, np.float32), pool.status()
+
+    def launched(graph, tokens):
+        pool.set_len(0, np.full(B, tokens, np.int32))
+        graph.launch()
+        return result()
+
+    def same(a, b):
+        return np.max(np.abs(a - b)) <= 1e-2 * np.sqrt(np.mean(b ** 2))
+    want, graphs = {}, {}
+    for tokens in (640, 60):
+        pool.set_len(0, np.full(B, tokens, np.int32))
+        call()
+        want[tokens] = result()[0]
+        graphs[tokens] = Graph(dev, call)
+    for at, tokens in ((60, 60), (640, 60), (640, 640), (640, 60)):
+        got, status = launched(graphs[at], tokens)
+        assert status == 0 and same(got, want[tokens]), (at, tokens)
+    got, status = launched(graphs[60], 640)
+    assert status == L.ERR_UNSUPPORTED and not got.any()
+    got, status = launched(graphs[60], 60)
+    assert status == 0 and same(got, want[60])
+    for g in graphs.values():
+        g.free()
+    pool.destroy()
+    for b in (q, qr, wuk, wuv, out):
+        b.free()
