@@ -392,7 +392,7 @@ struct VupParams {
   int32_t rows_each;                          // rows of a group (the last may have fewer)
   int32_t halves, n_block, n_kb, n_stages;    // VupShape; a stage is one TMA box
   int32_t tmem_cols;
-  int32_t room, all;                          // columns that a CTA has room for, and that there are partial results for
+  int32_t n_blocks, room, all;                // blocks and columns that a CTA has room for, and columns that there are partial results for
   int32_t listed;                             // `first` holds chunk_off
   int32_t* status;
   uint16_t first[kVupListed + 1];
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
   uint8_t* ring = smem + nk * 32768;                              // [stage], swizzled
   VupShared* sh = reinterpret_cast<VupShared*>(ring + prm.n_stages * stage_bytes);
   float2* info = reinterpret_cast<float2*>(sh->info);
-  const int h = blockIdx.x, r0 = blockIdx.y * prm.rows_each, rows_most = min(prm.rows_each, prm.rows - r0);
+  const int h = blockIdx.x, r0 = blockIdx.y * prm.rows_each, rows_here = min(prm.rows_each, prm.rows - r0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int steps_each = (2 * nk + prm.n_kb - 1) / prm.n_kb;      // stages of a block of columns
   chain_release();
@@ -458,17 +458,14 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
     const int i = S == 1 ? row : row / S, q = row - i * S, c0 = first_of(i);
     return c0 * S + (q == 0 ? 0 : q * (first_of(i + 1) - c0));
   };
-  auto rows_now = [&]() -> int {   // none where they have more columns than the launch was sized for
-    if (!kLoose) return rows_most;
-    const int c0 = col_of(r0), c1 = col_of(r0 + rows_most);
-    return c1 - c0 <= prm.room && c1 <= prm.all ? rows_most : 0;
-  };
+  auto beyond = [&](int c0, int n) { return kLoose && (n > prm.room || c0 + n > prm.all); };   // columns that the launch was not sized for
   if (warp < 2) {
     const bool el = elect_one();
     chain_wait();   // the partial results come from the kernel before this one
-    const int rows_here = rows_now();
-    if (kLoose && rows_here == 0 && threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
-    const int col0 = col_of(r0), blocks = (col_of(r0 + rows_here) - col0 + nb - 1) / nb;
+    const int col0 = col_of(r0), cols = col_of(r0 + rows_here) - col0;
+    int blocks = (cols + nb - 1) / nb;
+    if (kLoose) blocks = min(blocks, prm.n_blocks);
+    if (beyond(col0, cols) && threadIdx.x == 0) set_status(prm.status, RELUX_ERR_UNSUPPORTED);
     if (warp == 0) {
 #pragma unroll 1
       for (int b = 0, s = 0, use = 0; b < blocks; b++)
@@ -518,27 +515,28 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
 #pragma unroll 1
   for (int pass = warp >= 2 ? 0 : 1; pass < 2; pass++) {
     const bool real = pass == 1;
-    int col0 = 0, lo = 0, hi = 0, rows_here = 1;   // first column of the CTA, and columns of the warp's rows
+    int col0 = 0, lo = 0, hi = 0;   // first column of the CTA, and columns of the warp's rows
     if (real) {
       if (warp >= 2) chain_wait();
-      rows_here = rows_now();
       const int ra = rows_here * (warp >> 2) / 4, rb = rows_here * ((warp >> 2) + 1) / 4;
       col0 = col_of(r0);
       lo = col_of(r0 + ra) - col0;
       hi = col_of(r0 + rb) - col0;
+      if (beyond(col0, hi)) hi = lo;
     }
     if (warp >= 2) {
       // the weights of a row's pieces, by 32, 8 or 4 lanes
       const int lpr = rows_here <= kVupWarps - 2 ? 32 : rows_here <= 4 * (kVupWarps - 2) ? 8 : 4;
-      const int sub = lane & (lpr - 1), per_pass = (kVupWarps - 2) * (32 / lpr);
+      const int sub = lane & (lpr - 1), per_pass = (kVupWarps - 2) * (32 / lpr), rows_now = real ? rows_here : 1;
 #pragma unroll 1
-      for (int rw = 0; rw < rows_here; rw += per_pass) {
+      for (int rw = 0; rw < rows_now; rw += per_pass) {
         const int r = rw + ((warp - 2) * 32 + lane) / lpr;
         int c = 0, n = 0;
-        if (r < rows_here) {
+        if (r < rows_now) {
           const int i = S == 1 ? r0 + r : (r0 + r) / S, q = r0 + r - i * S, first = first_of(i), pieces = first_of(i + 1) - first;
           n = real ? pieces : 1;
           c = real ? first * S + q * n - col0 : kVupMaxCols + 8;   // no column's place: other warps may be at theirs already
+          if (real && beyond(col0, c + n)) n = 0;
         }
         float M = -INFINITY;
 #pragma unroll 1
@@ -563,7 +561,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
           const float m = info[c + j].x;
           info[c + j] = make_float2(m == -INFINITY ? 0.f : exp2f(m - M) * inv, __int_as_float(j == n - 1 ? r * H * kDh : -1));
         }
-        if (r < rows_here && n <= 0)   // an empty sequence
+        if (r < rows_now && n <= 0)   // an empty sequence
           for (int d = sub; d < kDh; d += lpr) {
             const size_t off = ((size_t)(r0 + r) * H + h) * kDh + d;
             if (kOutBf16) reinterpret_cast<uint16_t*>(prm.out)[off] = 0;
@@ -685,7 +683,8 @@ int32_t launch_mla_vup_pieces(Device* dev, const void* part, const float* part_m
   k.n_kb = sh.n_kb;
   k.n_stages = sh.n_stages;
   k.tmem_cols = sh.tmem_cols;
-  k.room = sh.blocks * sh.n_block;
+  k.n_blocks = sh.blocks;
+  k.room = std::min(sh.blocks * sh.n_block, kVupMaxCols);
   k.all = all;
   const int blk_bytes = k.halves * k.n_block * 128;
   k.part_ml = part_ml;

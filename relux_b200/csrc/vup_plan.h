@@ -19,7 +19,7 @@ inline int vup_col(const std::vector<int32_t>& first, int S, int row) {
 
 struct VupShape {
   int groups, rows_each;                          // rows of a group of CTAs, one for each head (the last group may have fewer)
-  int most;                                       // columns that a group may find
+  int planned, most;                              // columns that a group has at the host's lengths, and may find
   int blocks, n_block, n_kb, n_stages;            // a stage: n_kb times 64 latent columns of n_block columns, [n_kb][hi | lo][n_block][64]
   int tmem_cols;
   bool fits() const { return most <= kVupMaxCols && tmem_cols <= 512; }
@@ -40,19 +40,25 @@ inline VupShape vup_shape(const std::vector<int32_t>& first, int rows, int S, in
   int groups = std::max({1, std::min({fit, (all + 64 - second) / 32, rows}), workers > 0 ? 1 : std::min(rows, (all + kVupMaxCols - 1) / kVupMaxCols)});
   for (;; groups = (rows + k.rows_each - 2) / (k.rows_each - 1)) {
     k.rows_each = (rows + groups - 1) / groups;
-    k.most = 0;
+    k.planned = k.most = 0;
     for (int r = 0; r < rows && (k.most <= kVupMaxCols || k.rows_each == 1); r += k.rows_each) {
       const int end = std::min(rows, r + k.rows_each), n = end - r;
       const int now = vup_col(first, S, end) - vup_col(first, S, r), later = workers > 0 ? n + std::min(S, n) * (workers - 1) : now;
+      k.planned = std::max(k.planned, now);
       k.most = std::max(k.most, k.rows_each > 1 ? later : std::max(now, std::min(later, kVupMaxCols)));   // one row: the kernel reports what is more
     }
     if (k.most <= kVupMaxCols || k.rows_each == 1) break;
   }
   k.groups = (rows + k.rows_each - 1) / k.rows_each;
+  // As wide as the host's lengths need, and as many as others may; as wide as those need where that would be more tensor memory than there is.
   const int widest = kVupRing / 4 / (halves * 128);
-  k.blocks = std::max(1, (k.most + widest - 1) / widest);
-  const int unit = (k.blocks > 1 ? 32 : 16) / halves;   // N is a multiple of 16, and a block begins at a multiple of 32 tensor-memory columns
-  k.n_block = std::max(unit, ((k.most + k.blocks - 1) / k.blocks + unit - 1) / unit * unit);
+  for (int wide : {k.planned, k.most}) {
+    const int n = std::max(1, (wide + widest - 1) / widest), unit = (k.most > wide || n > 1 ? 32 : 16) / halves;
+    // N is a multiple of 16, and a block begins at a multiple of 32 tensor-memory columns
+    k.n_block = std::max(unit, ((wide + n - 1) / n + unit - 1) / unit * unit);
+    k.blocks = std::max(1, (k.most + k.n_block - 1) / k.n_block);
+    if (k.blocks * k.n_block * halves <= 512) break;
+  }
   const int blk_bytes = halves * k.n_block * 128;
   k.n_kb = 4;
   while (k.n_kb > 1 && k.n_kb * blk_bytes > kVupRing / (k.n_kb > 2 ? 2 : 3)) k.n_kb /= 2;
