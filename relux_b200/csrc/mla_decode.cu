@@ -314,7 +314,7 @@ int32_t launch_mla_decode_fast(Pool* p, const SeqBatch& sb, const relux_attn_arg
   const int form = !proj_mma ? kPartialFloat32 : split ? kPartialHalves : kPartialOne;
   VupShape vup{};
   if (proj_mma) {
-    vup = vup_shape(plan.first, rows, S, p->dev->sm_count / H, form == kPartialHalves ? 2 : 1, dC, plan.loose && sm100 ? plan.num_workers : 0);
+    vup = vup_shape(plan.first, rows, S, p->dev->sm_count / H, form == kPartialHalves ? 2 : 1, dC, !plan.loose ? 0 : sm100 ? plan.num_workers : kVupAnyChunks);
     if (!vup.fits()) {
       set_error("a sequence of this call is cut into more than %d pieces (tuning knobs)", kVupMaxCols);
       return RELUX_ERR_UNSUPPORTED;

@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(32 * kVupWarps, 1) mla_vup_pieces_kernel(const
       col0 = col_of(r0);
       lo = col_of(r0 + ra) - col0;
       hi = col_of(r0 + rb) - col0;
-      if (beyond(col0, hi)) hi = lo;
+      if (beyond(col0, hi)) lo = hi = 0;   // (not from `lo` on: a lane's eight columns would be beyond it too)
     }
     if (warp >= 2) {
       // the weights of a row's pieces, by 32, 8 or 4 lanes

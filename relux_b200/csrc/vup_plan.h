@@ -31,19 +31,23 @@ struct VupShape {
 // 22.0, 57 20.9 / 18.5, 60 18.0 / 16.8; 64 heads 41 27.4 / 26.3, 45 24.4 / 24.6, 49 28.9 / 28.9, 53 22.1 / 22.3, 57 22.5 / 22.5, 61 22.3 / 22.4, 65 24.5 / 23.6, 69
 // 34.1 / 33.6.  A group's columns are one block where a stage of it, 64 latent columns, fits the ring four times, and equal blocks otherwise.
 // `first`: the plan's pieces at the host's lengths.  With `workers` the launch may find other lengths, on which the builder cuts at most workers - 1
-// sequences once more each (build_stream): what a group then has at most is its rows, and every cut once for each of its rows of the sequence.
+// sequences once more each (build_stream): what a group then has at most is its rows, and every cut once for each of its rows of the sequence.  With
+// kVupAnyChunks it may find any chunks, as many as were planned in all (build_worklist_kernel): one group may have them all.
+constexpr int kVupAnyChunks = -1;
 inline VupShape vup_shape(const std::vector<int32_t>& first, int rows, int S, int fit, int halves, int dC, int workers) {
   VupShape k;
   const int all = vup_col(first, S, rows);
   // (a row at a time fewer, from as many groups as the columns need at least: all numbers of groups in turn were quadratic in the rows)
   const int second = fit > 2 ? 41 : 53;
   int groups = std::max({1, std::min({fit, (all + 64 - second) / 32, rows}), workers > 0 ? 1 : std::min(rows, (all + kVupMaxCols - 1) / kVupMaxCols)});
+  if (workers == kVupAnyChunks && all > kVupMaxCols) groups = rows;
   for (;; groups = (rows + k.rows_each - 2) / (k.rows_each - 1)) {
     k.rows_each = (rows + groups - 1) / groups;
     k.planned = k.most = 0;
     for (int r = 0; r < rows && (k.most <= kVupMaxCols || k.rows_each == 1); r += k.rows_each) {
       const int end = std::min(rows, r + k.rows_each), n = end - r;
-      const int now = vup_col(first, S, end) - vup_col(first, S, r), later = workers > 0 ? n + std::min(S, n) * (workers - 1) : now;
+      const int now = vup_col(first, S, end) - vup_col(first, S, r);
+      const int later = workers > 0 ? n + std::min(S, n) * (workers - 1) : workers == kVupAnyChunks ? all : now;
       k.planned = std::max(k.planned, now);
       k.most = std::max(k.most, k.rows_each > 1 ? later : std::max(now, std::min(later, kVupMaxCols)));   // one row: the kernel reports what is more
     }

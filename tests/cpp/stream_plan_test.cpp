@@ -95,6 +95,25 @@ static bool check_columns(const std::vector<int>& pages, int S, int heads, const
   return true;
 }
 
+// Chunks of a graph's decode call on the CUDA-core kernel, dealt to the sequences anew: as many as were planned at most, wherever they lie.
+static bool check_chunks(std::mt19937& rng, int n, int S, int heads) {
+  const int span = rng() % 2 ? 6 : 40;
+  std::vector<int32_t> planned(1, 0), found(1, 0);
+  for (int i = 0; i < n; i++) planned.push_back(planned.back() + 1 + (int)(rng() % span));
+  for (int i = 0; i < n; i++) {
+    const int left = planned.back() - found.back(), most = std::min(left, kMaxRowItems);
+    found.push_back(found.back() + (i == n / 2 || rng() % 8 == 0 ? most : (int)(rng() % (std::min(most, span) + 1))));
+  }
+  const int rows = n * S;
+  const VupShape v = vup_shape(planned, rows, S, 148 / heads, 2, 512, kVupAnyChunks);
+  int widest = 0;
+  for (const std::vector<int32_t>* first : {&planned, &found})
+    for (int r = 0; r < rows; r += v.rows_each) widest = std::max(widest, vup_col(*first, S, std::min(rows, r + v.rows_each)) - vup_col(*first, S, r));
+  if (v.fits() && widest <= std::min({v.most, v.blocks * v.n_block, kVupMaxCols})) return true;
+  printf("chunks: %d rows in groups of %d, %d columns of %d x %d\n", rows, v.rows_each, widest, v.blocks, v.n_block);
+  return false;
+}
+
 static bool check_found(std::mt19937& rng, const std::vector<int>& pages, int S, int heads, int resident) {
   const int workers = S > 8 ? std::min(resident, std::max(1, (2 * resident + S - 1) / S)) : std::max(1, resident / S);
   const StreamShape s = cheapest_plan(pages, workers);
@@ -144,6 +163,8 @@ int main(int argc, char** argv) {
     for (int& p : pages) p = 1 + (int)(rng() % span);
     if (!check_found(rng, pages, S, heads[rng() % 6], rng() % 4 ? 74 : 1 + (int)(rng() % 100))) return 1;
   }
+  for (int t = 0; t < 20000; t++)
+    if (!check_chunks(rng, 1 + (int)(rng() % (rng() % 2 ? 8 : 60)), 1 + (int)(rng() % 4), t % 3 ? 8 : 16)) return 1;
   std::vector<int32_t> first(1, 0);   // 131072 rows of one to 60 pieces: groups tried one number after another took 2.6 s
   for (int i = 0; i < 64; i++) first.push_back(first.back() + 1 + (int)(rng() % 60));
   const clock_t from = clock();

@@ -205,3 +205,40 @@ def test_a_graph_of_the_plain_kernels_whose_chunks_become_fewer_or_more(dev, ora
     pool.destroy()
     for b in (q, qr, wuk, wuv, out):
         b.free()
+
+
+@pytest.mark.parametrize("dc,H,S", [(128, 16, 1), (256, 16, 2), (512, 8, 1)])
+def test_a_graph_of_the_plain_kernels_whose_chunks_move(dev, oracle, dc, H, S):  # noqa: F811
+    """As many chunks as at capture, in other sequences: one group of rows of the up-projection has those of two."""
+    import relux_b200 as rb
+    from relux_b200 import lib as L
+    B, pages = 24, 10
+    rng = np.random.default_rng(dc + S)
+    pool = rb.Pool(dev, L.POOL_MLA, 1, B * pages, 64, B, pages, dC=dc, dHR=DHR)
+    pool.set_tables(np.arange(B * pages, dtype=np.int32).reshape(B, pages))
+    bf = lambda *s: oracle.bf16_from_f32(rng.standard_normal(s).astype(np.float32))  # noqa: E731
+    pool.append(0, bf(B * 640, dc), bf(B * 640, DHR), B, n_new=np.full(B, 640, np.int32))
+    pool.tune(L.TUNE_CHUNK_PAGES, 1)
+    shape = (B, S, H, DH)
+    q, qr, wuk, wuv = (dev.upload(x) for x in (bf(*shape), bf(B, S, H, DHR), bf(dc, H * DH), bf(dc, H * DH)))
+    outs = [dev.upload(np.full(shape, np.nan, np.float32)) for _ in range(2)]
+
+    def call(k):
+        pool.decode(0, B, q, outs[k], H, DH, 0.01, q_rope=qr, w_uk=wuk, w_uv=wuv, q_tokens=S, q_dtype=L.DTYPE_BF16, out_dtype=L.DTYPE_F32)
+
+    def lengths(longest):
+        pool.set_len(0, np.asarray([630 if i in longest else 50 for i in range(B)], np.int32))
+    lengths((0, 1, 22, 23))
+    call(1)
+    graph = Graph(dev, lambda: call(1))
+    for longest in ((0, 1, 22, 23), (20, 21, 22, 23), (0, 1, 2, 3), (11, 12)):
+        lengths(longest)
+        call(0)
+        graph.launch()
+        dev.sync()
+        want, got = (o.download(shape, np.float32) for o in outs)
+        assert pool.status() == 0 and np.max(np.abs(want - got)) <= 1e-2 * np.sqrt(np.mean(want ** 2)), longest
+    graph.free()
+    pool.destroy()
+    for b in [q, qr, wuk, wuv] + outs:
+        b.free()
