@@ -1355,14 +1355,19 @@ static bool gqa_fuse_args_ok(const Pool* p, const relux_append_args* kv, const r
          !(kv->flags & ~RELUX_CALL_PIPELINED) && kv->layer >= 0 && kv->layer < p->prm.num_layers;
 }
 
-// Where the kernels can read a page-locked tensor of the caller's with 16-byte loads; nullptr for other memory.
-static const void* page_locked(const void* ptr) {
-  cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return nullptr;
+// Where the kernels can read a page-locked tensor of the caller's with 16-byte loads; nullptr for other memory, and for a tensor that is page-locked in part.
+static const void* page_locked(const void* ptr, size_t bytes) {
+  const char* at[2];
+  for (size_t i = 0; i < 2; i++) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, (const char*)ptr + i * (bytes - 1)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    if (attr.type != cudaMemoryTypeHost || !attr.devicePointer) return nullptr;
+    at[i] = (const char*)attr.devicePointer;
   }
-  return at.type == cudaMemoryTypeHost && ((uintptr_t)at.devicePointer & 15u) == 0 ? at.devicePointer : nullptr;
+  return ((uintptr_t)at[0] & 15u) == 0 && (size_t)(at[1] - at[0]) == bytes - 1 ? at[0] : nullptr;
 }
 // A pipelined latent step whose copies outlast its kernels leaves its new rows where they are, for the preparation to read over PCIe: two small copies
 // fewer, which take a turn of the copy engine each (64 sequences, 128 heads: 3.3 MB in by four copies, 2.1 MB out).  Steps of several pools in turn move
@@ -1431,7 +1436,7 @@ static int32_t do_step(Pool* p, const relux_append_args* kv, const relux_attn_ar
   const bool piped = (kv->flags & RELUX_CALL_PIPELINED) && kv->mem == RELUX_MEM_HOST && p->dev->h2d_stream;
   const void *da = nullptr, *db = nullptr;
   int slot_a = -1, slot_b = -1;
-  if (piped && rows_in_place(p, sb, *attn, kv->layer, bytes_a + bytes_b) && (da = page_locked(kv->a)) && (db = page_locked(kv->b))) {
+  if (piped && rows_in_place(p, sb, *attn, kv->layer, bytes_a + bytes_b) && (da = page_locked(kv->a, bytes_a)) && (db = page_locked(kv->b, bytes_b))) {
   } else if (piped) {
     if ((rc = pipe_stage_in(p, p->pipe_app_a, kv->a, bytes_a, false, &da, &slot_a))) return rc;
     if ((rc = pipe_stage_in(p, p->pipe_app_b, kv->b, bytes_b, !pipes_queries(p, *attn), &db, &slot_b))) return rc;
