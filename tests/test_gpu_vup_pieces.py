@@ -40,6 +40,10 @@ def test_pieces_at_the_borders_of_blocks_and_groups(dev, oracle, ctx, H, chunk, 
         ref = oracle.mla_attend(ragged_to_padded(c, ctx, (DC,)), ragged_to_padded(r, ctx, (DHR,)), ctx, oracle.f32_from_bf16(q),
                                 oracle.f32_from_bf16(qr), wuk, wuv, scale, absorbed=True)
     got = oracle.f32_from_bf16(out) if out_bf16 else out
+    for b in range(B):
+        if ctx[b] == 0:
+            assert not got[b].any()
+            ref[b] = 0.0
     check_attention(got, ref, "pieces of %d sequences, %d heads" % (B, H), bf16_output=out_bf16, max_tol=EDGE_MAX, mean_tol=EDGE_MEAN)
     assert pool.status() == 0
     pool.destroy()
